@@ -5,6 +5,8 @@
 Produces, next to this file:
     librfk.so         the kernel library behind include/rfk.h (CUDA runtime only)
     librfk_layers.so  layer boundaries, render session (include/rfk_layers.h; cuBLAS + librfk.so)
+    librfk_io.so      weight, scene and image files (include/rfk_io.h)
+    _native.so        the operators of librfk.so as Python callables (compiled against the installed torch)
 
 nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine.
 """
@@ -92,6 +94,22 @@ def cudnn_include() -> str:
     return os.path.join(sysconfig.get_paths()["purelib"], "nvidia", "cudnn", "include")
 
 
+def build_binding(force: bool, verbose: bool) -> Path:
+    """_native.so, a Python extension module: g++ against the headers of this interpreter and of its torch, whose
+    libraries are in the process already when it is imported."""
+    import sysconfig
+    out, src = PKG / "_native.so", CSRC / "ops_binding.cpp"
+    if force or not _newer(out, [src, INCLUDE / "rfk.h"]):
+        torch_dir = Path(sysconfig.get_paths()["purelib"]) / "torch"
+        cuda_include = Path(nvcc()).resolve().parent.parent / "include"
+        _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wno-unused-function",
+              f"-I{INCLUDE}", f"-I{sysconfig.get_paths()['include']}", f"-isystem{torch_dir / 'include'}",
+              f"-isystem{torch_dir / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-isystem{cuda_include}",
+              str(src), "-o", str(out), f"-L{PKG}", "-lrfk", "-Wl,-rpath,$ORIGIN", f"-L{torch_dir / 'lib'}",
+              "-lc10", "-lc10_cuda", "-ltorch_python", "-ltorch_cpu"], verbose)
+    return out
+
+
 def build_all(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> dict[str, Path]:
     libs = {"rfk": build_library("rfk", KERNEL_SOURCES, [], force, verbose, ptxas_info)}
     # layer boundaries + session + DPT head: cuBLAS for the fallback GEMMs, cuDNN for the head's convolutions,
@@ -100,6 +118,7 @@ def build_all(force: bool = False, verbose: bool = False, ptxas_info: bool = Fal
         "rfk_layers", LAYER_SOURCES,
         ["-lcublas", "-lcudnn", f"-L{PKG}", "-lrfk", "-Xlinker", "-rpath=$ORIGIN"], force, verbose, ptxas_info)
     libs["rfk_io"] = build_library("rfk_io", IO_SOURCES, ["-lz"], force, verbose, False)
+    libs["native"] = build_binding(force, verbose)
     return libs
 
 

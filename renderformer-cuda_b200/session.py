@@ -314,6 +314,9 @@ class RenderSession:
 
     def render_frame(self, c2w, fov_rad: float):
         """c2w: 16 floats (row-major 4x4, host: list / numpy / CPU tensor)."""
+        if (isinstance(c2w, torch.Tensor) and c2w.dtype == torch.float32 and not c2w.is_cuda and c2w.is_contiguous()
+                and c2w.numel() == 16):
+            return self.render_frame_raw(c2w.data_ptr(), fov_rad)   # the call copies the camera before it returns
         arr = (ctypes.c_float * 16)(*[float(v) for v in (c2w.reshape(-1).tolist() if hasattr(c2w, "reshape") else c2w)])
         _check("rfk_session_render_frame", _lib().rfk_session_render_frame(self.h, arr, ctypes.c_float(fov_rad)))
 
