@@ -25,6 +25,8 @@ __device__ __forceinline__ float silu_fast(float a) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const T* a, const T* __restrict__ b, T* out, long long n, int vec) {
+    pdl_wait();
+    pdl_trigger();
     const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i0 >= n) return;
     if (vec && i0 + 8 <= n) {
@@ -44,6 +46,8 @@ silu_mul_kernel(const T* a, const T* __restrict__ b, T* out, long long n, int ve
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const __half* gate_up, __half* out, long long rows, int hidden,
               long long out_pitch, int vec) {  // out may alias the gate half of gate_up
+    pdl_wait();
+    pdl_trigger();
     const int cpr = (hidden + 7) / 8;
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= rows * cpr) return;
@@ -74,6 +78,8 @@ __device__ __forceinline__ float elu_ref(float v, float alpha) {
 template <int OP, typename TI, typename TO>
 __global__ void __launch_bounds__(256)
 post_kernel(const TI* x, TO* y, long long n, float alpha, int vec) {
+    pdl_wait();
+    pdl_trigger();
     const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i0 >= n) return;
     auto f = [&](float v) -> float {
@@ -97,7 +103,7 @@ static int launch_post(const TI* x, TO* y, long long n, float alpha, cudaStream_
     if (!x || !y || n < 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     const int vec = aligned16(x) && aligned16(y);
-    post_kernel<OP, TI, TO><<<ceil_div((n + 7) / 8, 256), 256, 0, st>>>(x, y, n, alpha, vec);
+    launch_pdl(post_kernel<OP, TI, TO>, dim3(ceil_div((n + 7) / 8, 256)), dim3(256), 0, st, x, y, n, alpha, vec);
     return launch_status();
 }
 
@@ -110,7 +116,7 @@ extern "C" int rfk_fused_silu_mul(const rfk_half* a, const rfk_half* b, rfk_half
     if (!a || !b || !out || n < 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     const int vec = aligned16(a) && aligned16(b) && aligned16(out);
-    silu_mul_kernel<__half><<<ceil_div((n + 7) / 8, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(silu_mul_kernel<__half>, dim3(ceil_div((n + 7) / 8, 256)), dim3(256), 0, as_stream(stream),
         (const __half*)a, (const __half*)b, (__half*)out, n, vec);
     return launch_status();
 }
@@ -120,7 +126,7 @@ extern "C" int rfk_fused_silu_mul_f32(const float* a, const float* b, float* out
     if (!a || !b || !out || n < 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     const int vec = aligned16(a) && aligned16(b) && aligned16(out);
-    silu_mul_kernel<float><<<ceil_div((n + 7) / 8, 256), 256, 0, as_stream(stream)>>>(a, b, out, n,
+    launch_pdl(silu_mul_kernel<float>, dim3(ceil_div((n + 7) / 8, 256)), dim3(256), 0, as_stream(stream), a, b, out, n,
                                                                                       vec);
     return launch_status();
 }
@@ -131,7 +137,7 @@ extern "C" int rfk_swiglu(const rfk_half* gate_up, rfk_half* out, int rows, int 
     if (rows == 0) return RFK_OK;
     const int vec = hidden % 8 == 0 && aligned16(gate_up) && aligned16(out);
     const long long chunks = (long long)rows * ((hidden + 7) / 8);
-    swiglu_kernel<<<ceil_div(chunks, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(swiglu_kernel, dim3(ceil_div(chunks, 256)), dim3(256), 0, as_stream(stream),
         (const __half*)gate_up, (__half*)out, rows, hidden, hidden, vec);
     return launch_status();
 }
@@ -142,7 +148,7 @@ extern "C" int rfk_swiglu_inplace(rfk_half* gate_up, int rows, int hidden, rfk_s
     const int vec = hidden % 8 == 0 && aligned16(gate_up);
     const long long chunks = (long long)rows * ((hidden + 7) / 8);
     // every thread overwrites exactly the gate elements it has just read
-    swiglu_kernel<<<ceil_div(chunks, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(swiglu_kernel, dim3(ceil_div(chunks, 256)), dim3(256), 0, as_stream(stream),
         (const __half*)gate_up, (__half*)gate_up, rows, hidden, 2LL * hidden, vec);
     return launch_status();
 }

@@ -20,6 +20,8 @@ template <bool BIAS, bool SILU, bool RES>
 __global__ void __launch_bounds__(256)
 bias_act_residual_nhwc_kernel(__half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ res,
                               long long chunks, int c8 /* C / 8 */) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= chunks) return;
     float f[8];
@@ -49,6 +51,8 @@ bias_act_residual_nhwc_kernel(__half* __restrict__ x, const __half* __restrict__
 
 __global__ void __launch_bounds__(256)
 silu_nhwc_kernel(const __half* __restrict__ x, __half* __restrict__ y, long long chunks) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= chunks) return;
     float f[8];
@@ -65,6 +69,8 @@ silu_nhwc_kernel(const __half* __restrict__ x, __half* __restrict__ y, long long
 __global__ void __launch_bounds__(256)
 bilinear_upsample_nhwc_kernel(const __half* __restrict__ in, __half* __restrict__ out, int H_in, int W_in, int H_out, int W_out,
                               int c8) {
+    pdl_wait();
+    pdl_trigger();
     const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (unsigned)W_out * (unsigned)c8) return;
     const int w_out = (int)(idx / (unsigned)c8), cc = (int)(idx % (unsigned)c8);
@@ -93,6 +99,8 @@ bilinear_upsample_nhwc_kernel(const __half* __restrict__ in, __half* __restrict_
 __global__ void __launch_bounds__(256)
 depth_to_space_bias_nhwc_kernel(const __half* __restrict__ in, const __half* __restrict__ bias, __half* __restrict__ out,
                                 long long chunks, int H, int W, int c8, int f) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // over the OUTPUT, 8 channels each
     if (i >= chunks) return;
     const int cc = (int)(i % c8);
@@ -117,6 +125,8 @@ depth_to_space_bias_nhwc_kernel(const __half* __restrict__ in, const __half* __r
 // [N, HW, C] -> [N, C, HW] for small C (the head's last layer: C = 3): one thread per output element
 __global__ void __launch_bounds__(256)
 permute_nhwc_to_nchw_kernel(const __half* __restrict__ in, __half* __restrict__ out, long long total, long long HW, int C) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const long long hw = i % HW;
@@ -135,6 +145,8 @@ template <int COUT>
 __global__ void __launch_bounds__(256)
 pointwise_to_planar_kernel(const __half* __restrict__ in, const __half* __restrict__ w, const __half* __restrict__ bias,
                            __half* __restrict__ out, long long HW, long long total, int c_in) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float sw[];  // [COUT][c_in]
     for (int i = threadIdx.x; i < COUT * c_in; i += blockDim.x) sw[i] = __half2float(w[i]);
     __syncthreads();
@@ -177,7 +189,7 @@ permute_filter_kernel(const __half* __restrict__ w, __half* __restrict__ out, in
 
 template <bool BIAS, bool SILU, bool RES>
 static int launch_bar(__half* x, const __half* bias, const __half* res, long long chunks, int c8, cudaStream_t st) {
-    bias_act_residual_nhwc_kernel<BIAS, SILU, RES><<<(unsigned)ceil_div(chunks, 256), 256, 0, st>>>(x, bias, res, chunks, c8);
+    launch_pdl(bias_act_residual_nhwc_kernel<BIAS, SILU, RES>, dim3((unsigned)ceil_div(chunks, 256)), dim3(256), 0, st, x, bias, res, chunks, c8);
     return launch_status();
 }
 
@@ -212,7 +224,7 @@ extern "C" int rfk_silu(const rfk_half* x, rfk_half* y, long long n, rfk_stream_
     if (!x || !y || n < 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     if (n % 8 || !aligned16(x) || !aligned16(y)) return RFK_EUNSUPPORTED;
-    silu_nhwc_kernel<<<(unsigned)ceil_div(n / 8, 256), 256, 0, as_stream(stream)>>>((const __half*)x, (__half*)y, n / 8);
+    launch_pdl(silu_nhwc_kernel, dim3((unsigned)ceil_div(n / 8, 256)), dim3(256), 0, as_stream(stream), (const __half*)x, (__half*)y, n / 8);
     return launch_status();
 }
 
@@ -224,7 +236,7 @@ extern "C" int rfk_bilinear_upsample_nhwc(const rfk_half* in, rfk_half* out, int
     const long long per_row = (long long)W_out * (C / 8);
     if (per_row > 0x7fffffffLL || H_out > 65535 || N > 65535) return RFK_EUNSUPPORTED;
     dim3 grid((unsigned)ceil_div(per_row, 256), (unsigned)H_out, (unsigned)N);
-    bilinear_upsample_nhwc_kernel<<<grid, 256, 0, as_stream(stream)>>>((const __half*)in, (__half*)out, H_in, W_in, H_out, W_out,
+    launch_pdl(bilinear_upsample_nhwc_kernel, dim3(grid), dim3(256), 0, as_stream(stream), (const __half*)in, (__half*)out, H_in, W_in, H_out, W_out,
                                                                       C / 8);
     return launch_status();
 }
@@ -236,7 +248,7 @@ extern "C" int rfk_depth_to_space_bias_nhwc(const rfk_half* in, const rfk_half* 
     if (C % 8 || !aligned16(in) || !aligned16(out) || (bias && !aligned16(bias))) return RFK_EUNSUPPORTED;
     const long long chunks = (long long)N * H * f * W * f * (C / 8);
     if (chunks > 0x7fffffffLL * 256) return RFK_EUNSUPPORTED;
-    depth_to_space_bias_nhwc_kernel<<<(unsigned)ceil_div(chunks, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(depth_to_space_bias_nhwc_kernel, dim3((unsigned)ceil_div(chunks, 256)), dim3(256), 0, as_stream(stream),
         (const __half*)in, (const __half*)bias, (__half*)out, chunks, H, W, C / 8, f);
     return launch_status();
 }
@@ -246,7 +258,7 @@ extern "C" int rfk_permute_nhwc_to_nchw(const rfk_half* in, rfk_half* out, int N
     const long long total = (long long)N * HW * C;
     if (total == 0) return RFK_OK;
     if (total > 0x7fffffffLL * 256) return RFK_EUNSUPPORTED;
-    permute_nhwc_to_nchw_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, as_stream(stream)>>>((const __half*)in, (__half*)out,
+    launch_pdl(permute_nhwc_to_nchw_kernel, dim3((unsigned)ceil_div(total, 256)), dim3(256), 0, as_stream(stream), (const __half*)in, (__half*)out,
                                                                                                total, HW, C);
     return launch_status();
 }
@@ -273,10 +285,10 @@ extern "C" int rfk_pointwise_conv_to_planar(const rfk_half* in, const rfk_half* 
     const __half *pi = (const __half*)in, *pw = (const __half*)weight, *pb = (const __half*)bias;
     __half* po = (__half*)out;
     switch (C_out) {
-        case 1: pointwise_to_planar_kernel<1><<<grid, 256, smem, st>>>(pi, pw, pb, po, HW, total, C_in); break;
-        case 2: pointwise_to_planar_kernel<2><<<grid, 256, smem, st>>>(pi, pw, pb, po, HW, total, C_in); break;
-        case 3: pointwise_to_planar_kernel<3><<<grid, 256, smem, st>>>(pi, pw, pb, po, HW, total, C_in); break;
-        default: pointwise_to_planar_kernel<4><<<grid, 256, smem, st>>>(pi, pw, pb, po, HW, total, C_in); break;
+        case 1: launch_pdl(pointwise_to_planar_kernel<1>, dim3(grid), dim3(256), smem, st, pi, pw, pb, po, HW, total, C_in); break;
+        case 2: launch_pdl(pointwise_to_planar_kernel<2>, dim3(grid), dim3(256), smem, st, pi, pw, pb, po, HW, total, C_in); break;
+        case 3: launch_pdl(pointwise_to_planar_kernel<3>, dim3(grid), dim3(256), smem, st, pi, pw, pb, po, HW, total, C_in); break;
+        default: launch_pdl(pointwise_to_planar_kernel<4>, dim3(grid), dim3(256), smem, st, pi, pw, pb, po, HW, total, C_in); break;
     }
     return launch_status();
 }

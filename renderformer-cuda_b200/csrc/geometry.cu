@@ -45,6 +45,8 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <typename T>
 __global__ void __launch_bounds__(256)
 world_to_cam_kernel(const float* __restrict__ c2w, T* tri, T* vn, int n_verts) {
+    pdl_wait();
+    pdl_trigger();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     if (idx >= n_verts) return;
@@ -74,6 +76,8 @@ world_to_cam_kernel(const float* __restrict__ c2w, T* tri, T* vn, int n_verts) {
 // is bound by load latency). A thread whose vertices straddle two batch entries looks the camera up per vertex.
 __global__ void __launch_bounds__(256)
 world_to_cam_vec8_kernel(const float* __restrict__ c2w, __half* tri, __half* vn, int n_verts, long long n_groups) {
+    pdl_wait();
+    pdl_trigger();
     const long long gidx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gidx >= n_groups) return;
     const long long v0 = gidx * 8;
@@ -109,6 +113,8 @@ view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ t
                      __half* __restrict__ vvn, __half* __restrict__ vpos,
                      __half* __restrict__ k_cos, __half* __restrict__ k_sin, int n_tris, int nr,
                      int seq_pad, int num_freqs, int head_dim) {
+    pdl_wait();
+    pdl_trigger();
     const int cpt = head_dim / 16;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= seq_pad * cpt) return;
@@ -197,12 +203,12 @@ extern "C" int rfk_world_to_cam(const float* c2w, rfk_half* tri, rfk_half* vn, i
     const long long total = (long long)batch * n_verts;
     if (total >= 8 * 256 * (long long)kNumSMs && total % 8 == 0 && aligned16(tri) && (!vn || aligned16(vn))) {
         const long long n_groups = total / 8;
-        world_to_cam_vec8_kernel<<<ceil_div(n_groups, 256), 256, 0, as_stream(stream)>>>(c2w, (__half*)tri, (__half*)vn,
+        launch_pdl(world_to_cam_vec8_kernel, dim3(ceil_div(n_groups, 256)), dim3(256), 0, as_stream(stream), c2w, (__half*)tri, (__half*)vn,
                                                                                           n_verts, n_groups);
         return launch_status();
     }
     dim3 grid(ceil_div(n_verts, 256), batch);
-    world_to_cam_kernel<__half><<<grid, 256, 0, as_stream(stream)>>>(c2w, (__half*)tri,
+    launch_pdl(world_to_cam_kernel<__half>, dim3(grid), dim3(256), 0, as_stream(stream), c2w, (__half*)tri,
                                                                      (__half*)vn, n_verts);
     return launch_status();
 }
@@ -213,7 +219,7 @@ extern "C" int rfk_world_to_cam_f32(const float* c2w, float* verts, float* norma
     if (batch == 0 || n_verts == 0) return RFK_OK;
     if (batch > 65535) return RFK_EUNSUPPORTED;
     dim3 grid(ceil_div(n_verts, 256), batch);
-    world_to_cam_kernel<float><<<grid, 256, 0, as_stream(stream)>>>(c2w, verts, normals, n_verts);
+    launch_pdl(world_to_cam_kernel<float>, dim3(grid), dim3(256), 0, as_stream(stream), c2w, verts, normals, n_verts);
     return launch_status();
 }
 
@@ -232,7 +238,7 @@ extern "C" int rfk_view_geometry(const float* c2w, const rfk_half* tri_world,
         return RFK_EUNSUPPORTED;
     if (seq_pad == 0) return RFK_OK;
     const long long n = (long long)seq_pad * (head_dim / 16);
-    view_geometry_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(view_geometry_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream),
         c2w, (const __half*)tri_world, (const __half*)vn_world, world_center, learned_freqs,
         (__half*)vtri, (__half*)vvn, (__half*)vpos, (__half*)k_cos, (__half*)k_sin, n_tris,
         n_register, seq_pad, num_freqs, head_dim);

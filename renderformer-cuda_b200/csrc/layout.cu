@@ -31,6 +31,8 @@ template <int OP>
 __global__ void __launch_bounds__(256)
 ew_kernel(typename EwTypes<OP>::A* a, const typename EwTypes<OP>::B* __restrict__ b, long long n,
           int vec) {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i0 = t * 8;
     if (i0 >= n) return;
@@ -61,12 +63,14 @@ static int launch_ew(typename EwTypes<OP>::A* a, const typename EwTypes<OP>::B* 
     if (!a || !b || n < 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     const int vec = aligned16(a) && aligned16(b);
-    ew_kernel<OP><<<ceil_div((n + 7) / 8, 256), 256, 0, st>>>(a, b, n, vec);
+    launch_pdl(ew_kernel<OP>, dim3(ceil_div((n + 7) / 8, 256)), dim3(256), 0, st, a, b, n, vec);
     return launch_status();
 }
 
 __global__ void __launch_bounds__(256)
 broadcast_add_kernel(__half* out, const __half* __restrict__ bc, long long n, int dim, int vec) {
+    pdl_wait();
+    pdl_trigger();
     const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i0 >= n) return;
     if (vec && i0 + 8 <= n) {
@@ -140,6 +144,8 @@ template <typename MAP, bool ACCUM>
 __global__ void __launch_bounds__(256)
 chunk_copy_kernel(const __half* __restrict__ in, __half* out, long long nchunks, int cpr,
                   MAP map) {
+    pdl_wait();
+    pdl_trigger();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
     size_t src, dst;
@@ -160,6 +166,8 @@ chunk_copy_kernel(const __half* __restrict__ in, __half* out, long long nchunks,
 template <typename MAP, bool ACCUM>
 __global__ void __launch_bounds__(256)
 elem_copy_kernel(const __half* __restrict__ in, __half* out, long long n, int inner, MAP map) {
+    pdl_wait();
+    pdl_trigger();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     // reuse the chunk maps with "chunks" of one row and add the in-row offset
@@ -174,6 +182,8 @@ elem_copy_kernel(const __half* __restrict__ in, __half* out, long long n, int in
 
 __global__ void __launch_bounds__(256)
 patchify_kernel(const __half* __restrict__ in, __half* __restrict__ out, long long n, PatchMap map) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     size_t src, dst;
@@ -188,11 +198,11 @@ static int launch_rows(const __half* in, __half* out, long long n_rows, int inne
     if (inner % 8 == 0 && aligned16(in) && aligned16(out)) {
         const int cpr = inner / 8;
         const long long nchunks = n_rows * cpr;
-        chunk_copy_kernel<MAP, ACCUM><<<ceil_div(nchunks, 256), 256, 0, st>>>(in, out, nchunks, cpr,
+        launch_pdl(chunk_copy_kernel<MAP, ACCUM>, dim3(ceil_div(nchunks, 256)), dim3(256), 0, st, in, out, nchunks, cpr,
                                                                               map);
     } else {
         const long long n = n_rows * inner;
-        elem_copy_kernel<MAP, ACCUM><<<ceil_div(n, 256), 256, 0, st>>>(in, out, n, inner, map);
+        launch_pdl(elem_copy_kernel<MAP, ACCUM>, dim3(ceil_div(n, 256)), dim3(256), 0, st, in, out, n, inner, map);
     }
     return launch_status();
 }
@@ -222,7 +232,7 @@ extern "C" int rfk_broadcast_add(rfk_half* out, const rfk_half* bc, long long n,
     if (!out || !bc || n < 0 || dim <= 0) return RFK_EINVAL;
     if (n == 0) return RFK_OK;
     const int vec = aligned16(out) && aligned16(bc) && dim % 8 == 0;
-    broadcast_add_kernel<<<ceil_div((n + 7) / 8, 256), 256, 0, as_stream(stream)>>>(
+    launch_pdl(broadcast_add_kernel, dim3(ceil_div((n + 7) / 8, 256)), dim3(256), 0, as_stream(stream),
         (__half*)out, (const __half*)bc, n, dim, vec);
     return launch_status();
 }
@@ -283,7 +293,7 @@ extern "C" int rfk_patchify(const rfk_half* in, rfk_half* out, int H, int W, int
         return RFK_EINVAL;
     PatchMap m{H, W, C, ps};
     const long long n = (long long)H * W * C;
-    patchify_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>((const __half*)in,
+    launch_pdl(patchify_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream), (const __half*)in,
                                                                      (__half*)out, n, m);
     return launch_status();
 }

@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(kPeThreads)
 nerf_pe_tile_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long rows,
                     int rows_per_block, int in_dim, int num_freqs, int include_input,
                     const __grid_constant__ FreqTable ft, FastDiv div_in, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) __half s_out[];
     const int per_row = in_dim * num_freqs;
     const int off = include_input ? in_dim : 0;
@@ -100,6 +102,8 @@ __global__ void __launch_bounds__(kPeThreads)
 nerf_pe_tile_nf_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long rows,
                        int rows_per_block, int in_dim, int include_input,
                        const __grid_constant__ FreqTable ft, FastDiv div_in, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) __half s_out[];
     const int per_row = in_dim * NF;
     const int off = include_input ? in_dim : 0;
@@ -160,6 +164,8 @@ template <typename TI, int IN_DIM, int NF, bool DOUBLING, bool INCLUDE>
 __global__ void __launch_bounds__(kPeRowThreads)
 nerf_pe_rows1_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long rows,
                     const __grid_constant__ FreqTable ft, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int PER_ROW = IN_DIM * NF, OFF = INCLUDE ? IN_DIM : 0, OUT_DIM = 2 * PER_ROW + OFF;
     __shared__ __align__(16) __half s_out[kPeRowThreads * OUT_DIM];
     __shared__ TI s_in[kPeRowThreads * IN_DIM];
@@ -218,6 +224,8 @@ template <typename TI, int IN_DIM, int NF, bool DOUBLING, bool INCLUDE>
 __global__ void __launch_bounds__(kPeRowThreads)
 nerf_pe_rows_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long rows,
                     const __grid_constant__ FreqTable ft, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int PER_ROW = IN_DIM * NF, OFF = INCLUDE ? IN_DIM : 0, OUT_DIM = 2 * PER_ROW + OFF;
     constexpr int kRows = 2 * kPeRowThreads;
     __shared__ __align__(16) __half s_out[kRows * OUT_DIM];
@@ -285,6 +293,8 @@ __global__ void __launch_bounds__(256)
 nerf_pe_flat_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long total,
                     int in_dim, int num_freqs, int out_dim, int include_input,
                     const __grid_constant__ FreqTable ft) {
+    pdl_wait();
+    pdl_trigger();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     const long long row = e / out_dim;
@@ -333,22 +343,22 @@ static int launch_nerf_pe(const TI* input, __half* output, int batch, int seq_le
 #define RFK_PE_NF(NF)                                                                                              \
     do {                                                                                                           \
         if (doubling)                                                                                              \
-            nerf_pe_tile_nf_kernel<TI, NF, true><<<grid, kPeThreads, smem, st>>>(input, output, rows, rpb, in_dim, \
+            launch_pdl(nerf_pe_tile_nf_kernel<TI, NF, true>, dim3(grid), dim3(kPeThreads), smem, st, input, output, rows, rpb, in_dim, \
                                                                                  inc, ft, FastDiv((unsigned)in_dim), vec); \
         else                                                                                                       \
-            nerf_pe_tile_nf_kernel<TI, NF, false><<<grid, kPeThreads, smem, st>>>(input, output, rows, rpb, in_dim, \
+            launch_pdl(nerf_pe_tile_nf_kernel<TI, NF, false>, dim3(grid), dim3(kPeThreads), smem, st, input, output, rows, rpb, in_dim, \
                                                                                   inc, ft, FastDiv((unsigned)in_dim), vec); \
     } while (0)
         const unsigned row_grid = ceil_div(rows, 2 * kPeRowThreads), row1_grid = ceil_div(rows, kPeRowThreads);
 #define RFK_PE_ROWS1(IN, NF)                                                                                  \
     do {                                                                                                      \
-        if (doubling) nerf_pe_rows1_kernel<TI, IN, NF, true, true><<<row1_grid, kPeRowThreads, 0, st>>>(input, output, rows, ft, vec); \
-        else nerf_pe_rows1_kernel<TI, IN, NF, false, true><<<row1_grid, kPeRowThreads, 0, st>>>(input, output, rows, ft, vec);         \
+        if (doubling) launch_pdl(nerf_pe_rows1_kernel<TI, IN, NF, true, true>, dim3(row1_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec); \
+        else launch_pdl(nerf_pe_rows1_kernel<TI, IN, NF, false, true>, dim3(row1_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec);         \
     } while (0)
 #define RFK_PE_ROWS(IN, NF)                                                                                   \
     do {                                                                                                      \
-        if (doubling) nerf_pe_rows_kernel<TI, IN, NF, true, true><<<row_grid, kPeRowThreads, 0, st>>>(input, output, rows, ft, vec); \
-        else nerf_pe_rows_kernel<TI, IN, NF, false, true><<<row_grid, kPeRowThreads, 0, st>>>(input, output, rows, ft, vec);         \
+        if (doubling) launch_pdl(nerf_pe_rows_kernel<TI, IN, NF, true, true>, dim3(row_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec); \
+        else launch_pdl(nerf_pe_rows_kernel<TI, IN, NF, false, true>, dim3(row_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec);         \
     } while (0)
         if (num_freqs == 6 && in_dim == 3 && inc) RFK_PE_ROWS(3, 6);
         else if (num_freqs == 6 && in_dim == 9 && inc) RFK_PE_ROWS1(9, 6);
@@ -356,14 +366,14 @@ static int launch_nerf_pe(const TI* input, __half* output, int batch, int seq_le
         else if (num_freqs == 4) RFK_PE_NF(4);
         else if (num_freqs == 10) RFK_PE_NF(10);
         else
-            nerf_pe_tile_kernel<TI><<<grid, kPeThreads, smem, st>>>(
+            launch_pdl(nerf_pe_tile_kernel<TI>, dim3(grid), dim3(kPeThreads), smem, st,
                 input, output, rows, rpb, in_dim, num_freqs, inc, ft, FastDiv((unsigned)in_dim), vec);
 #undef RFK_PE_NF
 #undef RFK_PE_ROWS
 #undef RFK_PE_ROWS1
     } else {
         const long long total = rows * out_dim;
-        nerf_pe_flat_kernel<TI><<<ceil_div(total, 256), 256, 0, st>>>(
+        launch_pdl(nerf_pe_flat_kernel<TI>, dim3(ceil_div(total, 256)), dim3(256), 0, st,
             input, output, total, in_dim, num_freqs, (int)out_dim, include_input ? 1 : 0, ft);
     }
     return launch_status();

@@ -52,6 +52,8 @@ template <int PATCH, int ROWS, int COALESCE = 0>
 __global__ void __launch_bounds__(256)
 ray_gen_vec_kernel(const float* __restrict__ c2w, const float* __restrict__ fov,
                    float* __restrict__ rays_o, __half* __restrict__ out, int batch, int res) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) unsigned char s_stage[COALESCE ? 8 * 1536 : 16];
     const int groups_per_row = res / 8;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -127,6 +129,8 @@ __global__ void __launch_bounds__(256)
 ray_gen_generic_kernel(const float* __restrict__ c2w, const float* __restrict__ fov,
                        float* __restrict__ rays_o, __half* __restrict__ out, int batch, int res,
                        int ps) {
+    pdl_wait();
+    pdl_trigger();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long per_image = (long long)res * res;
     if (idx >= per_image * batch) return;
@@ -168,14 +172,14 @@ static int launch_ray_gen(const float* c2w, const float* fov, float* rays_o, __h
         const bool strips = res % 4 == 0 && (long long)batch * res * (res / 8) >= 4LL * kNumSMs * 2048;
         const long long n = (long long)batch * (res / (strips ? 4 : 1)) * (res / 8);
         const unsigned grid = ceil_div(n, 256);
-        if (ps && strips) ray_gen_vec_kernel<1, 4><<<grid, 256, 0, st>>>(c2w, fov, rays_o, out, batch, res);
-        else if (ps) ray_gen_vec_kernel<1, 1><<<grid, 256, 0, st>>>(c2w, fov, rays_o, out, batch, res);
-        else if (strips && res % 256 == 0) ray_gen_vec_kernel<0, 4, 1><<<grid, 256, 0, st>>>(c2w, fov, rays_o, out, batch, res);
-        else if (strips) ray_gen_vec_kernel<0, 4><<<grid, 256, 0, st>>>(c2w, fov, rays_o, out, batch, res);
-        else ray_gen_vec_kernel<0, 1><<<grid, 256, 0, st>>>(c2w, fov, rays_o, out, batch, res);
+        if (ps && strips) launch_pdl(ray_gen_vec_kernel<1, 4>, dim3(grid), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res);
+        else if (ps) launch_pdl(ray_gen_vec_kernel<1, 1>, dim3(grid), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res);
+        else if (strips && res % 256 == 0) launch_pdl(ray_gen_vec_kernel<0, 4, 1>, dim3(grid), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res);
+        else if (strips) launch_pdl(ray_gen_vec_kernel<0, 4>, dim3(grid), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res);
+        else launch_pdl(ray_gen_vec_kernel<0, 1>, dim3(grid), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res);
     } else {
         const long long n = (long long)batch * res * res;
-        ray_gen_generic_kernel<<<ceil_div(n, 256), 256, 0, st>>>(c2w, fov, rays_o, out, batch, res,
+        launch_pdl(ray_gen_generic_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st, c2w, fov, rays_o, out, batch, res,
                                                                  ps);
     }
     return launch_status();

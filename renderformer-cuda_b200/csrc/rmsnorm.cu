@@ -127,6 +127,8 @@ template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
 __global__ void __launch_bounds__(256)
 rmsnorm_generic_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
                        const float* __restrict__ gamma, TY* y, int dim, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[8];
     const size_t base = (size_t)blockIdx.x * dim;
     auto value = [&](int i) -> float {
@@ -174,7 +176,7 @@ static int launch_variant(const TH* x, TH* xw, const TR* r, const float* gamma, 
         else RFK_RMS_LAUNCH(2, 4);
 #undef RFK_RMS_LAUNCH
     } else {
-        rmsnorm_generic_kernel<TH, TR, TY, HAS_RES, WRITE_H><<<rows, 256, 0, st>>>(
+        launch_pdl(rmsnorm_generic_kernel<TH, TR, TY, HAS_RES, WRITE_H>, dim3(rows), dim3(256), 0, st,
             x, xw, r, gamma, y, dim, eps);
     }
     return launch_status();

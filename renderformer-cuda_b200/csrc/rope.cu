@@ -25,6 +25,8 @@ __global__ void __launch_bounds__(256)
 rope_table_vec_kernel(const __half* __restrict__ pos, const float* __restrict__ freqs,
                       __half* __restrict__ out_cos, __half* __restrict__ out_sin,
                       long long tokens, int num_freqs, int head_dim) {
+    pdl_wait();
+    pdl_trigger();
     const int cpt = head_dim / 16;  // chunks per token (first half)
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= tokens * cpt) return;
@@ -55,6 +57,8 @@ __global__ void __launch_bounds__(256)
 rope_table_generic_kernel(const __half* __restrict__ pos, const float* __restrict__ freqs,
                           __half* __restrict__ out_cos, __half* __restrict__ out_sin,
                           long long tokens, int num_freqs, int head_dim) {
+    pdl_wait();
+    pdl_trigger();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= tokens * head_dim) return;
     const long long tok = idx / head_dim;
@@ -152,6 +156,8 @@ rope_apply_generic_kernel(const T* src0, T* dst0, const T* src1, T* dst1,
                           int seq_len, int rows_total, int head_dim, long long src_rows,
                           long long dst_rows, long long src_bstride, long long dst_bstride,
                           long long tab_bstride) {
+    pdl_wait();
+    pdl_trigger();
     const int half_d = head_dim / 2;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long total = (long long)batch * num_heads * rows_total * half_d;
@@ -227,7 +233,7 @@ static int launch_rope(const T* src0, T* dst0, const T* src1, T* dst1, const __h
 #undef RFK_ROPE
     } else {
         const long long total = (long long)batch * num_heads * rows_total * (head_dim / 2);
-        rope_apply_generic_kernel<T, NT><<<ceil_div(total, 256), 256, 0, st>>>(
+        launch_pdl(rope_apply_generic_kernel<T, NT>, dim3(ceil_div(total, 256)), dim3(256), 0, st,
             src0, dst0, src1, dst1, cos_vals, sin_vals, batch, num_heads, seq_len, rows_total,
             head_dim, src_rows, dst_rows, src_bstride, dst_bstride, tab_bstride);
     }
@@ -382,12 +388,12 @@ extern "C" int rfk_triangle_rope_freqs(const rfk_half* pos, const float* learned
     cudaStream_t st = as_stream(stream);
     if (head_dim % 16 == 0 && aligned16(out_cos) && aligned16(out_sin)) {
         const long long n = tokens * (head_dim / 16);
-        rope_table_vec_kernel<<<ceil_div(n, 256), 256, 0, st>>>(
+        launch_pdl(rope_table_vec_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st,
             (const __half*)pos, learned_freqs, (__half*)out_cos, (__half*)out_sin, tokens,
             num_freqs, head_dim);
     } else {
         const long long n = tokens * head_dim;
-        rope_table_generic_kernel<<<ceil_div(n, 256), 256, 0, st>>>(
+        launch_pdl(rope_table_generic_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st,
             (const __half*)pos, learned_freqs, (__half*)out_cos, (__half*)out_sin, tokens,
             num_freqs, head_dim);
     }

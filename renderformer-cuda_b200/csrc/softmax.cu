@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(256)
 softmax_row_kernel(const float* in, TOut* out, const uint8_t* __restrict__ mask, MaskMap mm,
                    int cols, long long in_stride, long long out_stride, long long out_pitch,
                    float scale_log2e, int vec_in, int vec_out, int vec_mask) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float s_max[8];
     __shared__ float s_sum[8];
     const int tid = threadIdx.x;
@@ -139,6 +141,8 @@ __global__ void __launch_bounds__(256)
 softmax_small_kernel(const float* in, TOut* out, const uint8_t* __restrict__ mask, MaskMap mm,
                      long long rows, int cols, long long in_stride, long long out_stride,
                      long long out_pitch, float scale_log2e, int vec_in, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
     const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const int gl = threadIdx.x % G;
     const bool live = gid < rows;
@@ -218,6 +222,8 @@ __global__ void __launch_bounds__(1024)
 softmax_long_kernel(const float* in, TOut* out, const uint8_t* __restrict__ mask, MaskMap mm,
                     int cols, long long in_stride, long long out_stride, long long out_pitch,
                     float scale_log2e) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float s_red[32];
     __shared__ float s_bcast;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
@@ -287,7 +293,7 @@ static int launch_softmax(const float* in, TOut* out, const uint8_t* mask, MaskM
         const int vec_out = ((reinterpret_cast<uintptr_t>(out) % (4 * osz)) == 0) &&
                             (out_pitch % 4 == 0);
 #define RFK_SM_SMALL(G, N)                                                                    \
-    softmax_small_kernel<TOut, G, N, MASK><<<ceil_div(rows * G, 256), 256, 0, st>>>(          \
+    launch_pdl(softmax_small_kernel<TOut, G, N, MASK>, dim3(ceil_div(rows * G, 256)), dim3(256), 0, st,           \
         in, out, mask, mm, rows, cols, in_stride, out_stride, out_pitch, sl2, vec_in, vec_out)
         if (span <= 32) RFK_SM_SMALL(8, 1);
         else if (span <= 64) RFK_SM_SMALL(16, 1);
@@ -304,7 +310,7 @@ static int launch_softmax(const float* in, TOut* out, const uint8_t* mask, MaskM
         const int threads = chunks <= 128 ? 128 : 256;
         const int nch = (chunks + threads - 1) / threads;
 #define RFK_SM_ROW(N)                                                                         \
-    softmax_row_kernel<TOut, N, MASK><<<(unsigned)rows, threads, 0, st>>>(                    \
+    launch_pdl(softmax_row_kernel<TOut, N, MASK>, dim3((unsigned)rows), dim3(threads), 0, st,                     \
         in, out, mask, mm, cols, in_stride, out_stride, out_pitch, sl2, vec_in, vec_out, vec_mask)
         switch (nch) {
             case 1: RFK_SM_ROW(1); break;
@@ -316,7 +322,7 @@ static int launch_softmax(const float* in, TOut* out, const uint8_t* mask, MaskM
         return launch_status();
     }
     if (registers_only) return RFK_EUNSUPPORTED;  // the streaming tier re-reads its input
-    softmax_long_kernel<TOut, MASK><<<(unsigned)rows, 1024, 0, st>>>(
+    launch_pdl(softmax_long_kernel<TOut, MASK>, dim3((unsigned)rows), dim3(1024), 0, st,
         in, out, mask, mm, cols, in_stride, out_stride, out_pitch, sl2);
     return launch_status();
 }
