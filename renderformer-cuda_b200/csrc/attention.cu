@@ -470,7 +470,7 @@ extern std::atomic<int> g_attn_split;
 size_t attention_tc_workspace_bytes();
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
-                        int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
+                        int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
                         int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared);
 
 }  // namespace rfk
@@ -488,9 +488,9 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     cudaStream_t st = as_stream(stream);
     const long long kvs = (long long)Sk * D;
     const int path = g_attn_path.load(std::memory_order_relaxed);
-    if (D == 64 && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
+    if ((D == 64 || D == 128) && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
         const int rc = launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk,
-                                           n_keys, o_bshd, scale, st, nullptr, 0, 0, 0.0f, nullptr, 0, 0);
+                                           n_keys, D, o_bshd, scale, st, nullptr, 0, 0, 0.0f, nullptr, 0, 0);
         if (rc != RFK_EUNSUPPORTED || path == 2) return rc;
     }
     if (D == 64)
@@ -511,10 +511,10 @@ extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, cons
     if (q_row_ss && (ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
     if (workspace && workspace_bytes < attention_tc_workspace_bytes()) return RFK_EINVAL;
     if (B == 0 || Sq == 0) return RFK_OK;
-    if (D != 64 || (long long)B * H > 65535 || g_attn_path.load(std::memory_order_relaxed) == 1) return RFK_EUNSUPPORTED;
+    if ((D != 64 && D != 128) || (long long)B * H > 65535 || g_attn_path.load(std::memory_order_relaxed) == 1) return RFK_EUNSUPPORTED;
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
-    return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, o_bshd,
-                               scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared != 0);
+    return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D,
+                               o_bshd, scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared != 0);
 }
 
 extern "C" size_t rfk_flash_attention_workspace_bytes(void) { return attention_tc_workspace_bytes(); }

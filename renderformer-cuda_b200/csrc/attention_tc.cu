@@ -54,7 +54,7 @@ __device__ int g_attn_tc_error = 0;  // first time-out / failure code seen by an
 
 namespace tcattn {
 
-constexpr int BM = 128, BN = 64, HD = 64;
+constexpr int BM = 128, BN = 64;
 constexpr int kBlocks = 2;                     // 128-query blocks per CTA, sharing the K/V ring
 constexpr int kThreads = 512;                  // warps 0-7 softmax (block = warp / 4), 8 producer, 9-10 PV, 11-12 QK issuers, 13-15 none
 // Registers: the CTA starts with 128 per thread. The two warpgroups that only issue copies and products (warps 8-15)
@@ -62,26 +62,33 @@ constexpr int kThreads = 512;                  // warps 0-7 softmax (block = war
 // compiler keep both halves of a score tile and their exponentials in flight without reusing registers early
 // (measured: 3 % off the kernel's time). 256 * 40 + 256 * 216 = 65536, the register file.
 constexpr int kRegsIssue = 40, kRegsSoftmax = 216;
-constexpr int kStages = 6;
-constexpr int kQBytes = BM * HD * 2;           // 16 KB
-constexpr int kKBytes = BN * HD * 2;           // 8 KB; a stage is K then V
-constexpr int kStageBytes = 2 * kKBytes;
-constexpr int kSBufs = 3;                      // score buffers in tensor memory
-constexpr int kTmemCols = 512;                 // per block: S0, S1, S2 at +0, +64, +128; O at +192
+constexpr int kTmemCols = 512;                 // 256 per block: the score buffers (64 columns each), then O
+// Per head size. A row of the operand tiles is HD / 64 swizzle rows of 128 bytes: the tiles are kept as HD / 64
+// sub-tiles of 64 columns, each fetched by its own TMA box.
+template <int HD> struct Cfg {
+    static constexpr int kSub = HD / 64;
+    static constexpr int kQSub = BM * 128, kQBytes = kSub * kQSub;     // 16 KB per 64 columns
+    static constexpr int kKSub = BN * 128, kKBytes = kSub * kKSub;     // 8 KB per 64 columns; a stage is K then V
+    static constexpr int kStageBytes = 2 * kKBytes;
+    static constexpr int kStages = HD == 64 ? 6 : 4;
+    // O takes HD of a block's 256 tensor-memory columns, score buffers the rest: three at 64, two at 128
+    static constexpr int kSBufs = (256 - HD) / 64;
+    // The shared-memory window is declared 1024-byte aligned (swizzled tiles need it) and the kernel checks it.
+    static constexpr int kSmemBytes = kBlocks * kQBytes + kStages * kStageBytes + 512;
+    static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
+};
+constexpr int kMaxStages = 6, kMaxSBufs = 3;
 
 struct __align__(8) Ctrl {
-    uint64_t q_full, kv_full[kStages], kv_empty[kStages], s_full[kBlocks][kSBufs], p_full[kBlocks][kSBufs],
-        pv_done[kBlocks][kSBufs];
+    uint64_t q_full, kv_full[kMaxStages], kv_empty[kMaxStages], s_full[kBlocks][kMaxSBufs], p_full[kBlocks][kMaxSBufs],
+        pv_done[kBlocks][kMaxSBufs];
     uint64_t drain[2 * kBlocks];  // abort path only, one per issuing thread: completes once that thread's products have finished
     uint32_t tmem_base;
     int abort;
     int merge;  // set by thread 0 of a split unit's last piece: this CTA merges the unit
 };
 
-// The shared-memory window is declared 1024-byte aligned (swizzled tiles need it) and the kernel checks it.
-constexpr int kSmemBytes = kBlocks * kQBytes + kStages * kStageBytes + 512;
 static_assert(sizeof(Ctrl) <= 512, "control block");
-static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
 
 enum : int { kErrTimeout = 1, kErrSmemAlign = 2 };
 
@@ -100,7 +107,7 @@ struct WorkList {
 constexpr int kUnitRows = kBlocks * BM;
 constexpr size_t kWsCounterBytes = 1024;
 constexpr size_t kWsMlBytes = (size_t)kMaxPieces * kUnitRows * 2 * sizeof(float);
-constexpr size_t kWsOBytes = (size_t)kMaxPieces * kUnitRows * HD * sizeof(float);
+constexpr size_t kWsOBytes = (size_t)kMaxPieces * kUnitRows * 128 * sizeof(float);  // for the larger head size
 constexpr size_t kWsBytes = kWsCounterBytes + kWsMlBytes + kWsOBytes;
 
 __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue)); }
@@ -225,11 +232,14 @@ __device__ __forceinline__ void store_row_half(__half* dst, const uint32_t (&v)[
     }
 }
 
+template <int HD>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, __half* __restrict__ O, int H, int Sq, int n_keys,
                     int o_bshd, float scale_log2e_all, const float* __restrict__ row_ss, int ss_tiles, float inv_norm_dim,
                     float norm_eps, unsigned char* __restrict__ ws, int v_heads, const __grid_constant__ WorkList work) {
+    using C = Cfg<HD>;
+    constexpr int kStages = C::kStages, kSBufs = C::kSBufs, kQBytes = C::kQBytes, kKBytes = C::kKBytes, kStageBytes = C::kStageBytes;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = tc::smem_addr(smem_raw);
     if (base & 1023u) {  // uniform over the CTA, nothing allocated yet
@@ -284,15 +294,22 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (lane == 0) {
             tc::prefetch_tensormap(&map_q); tc::prefetch_tensormap(&map_k); tc::prefetch_tensormap(&map_v);
             tc::mbar_arrive_expect_tx(&ctrl->q_full, kBlocks * kQBytes);
-            for (int k = 0; k < kBlocks; ++k) tc::tma_load_3d(sQ + k * kQBytes, &map_q, 0, q0 + k * BM, bh, &ctrl->q_full);
+            for (int k = 0; k < kBlocks; ++k)
+                for (int x = 0; x < C::kSub; ++x)
+                    tc::tma_load_3d(sQ + k * kQBytes + x * C::kQSub, &map_q, x * 64, q0 + k * BM, bh, &ctrl->q_full);
             int issued = 0;
             for (int j = 0; j < n_tiles; ++j) {
                 const int s = j % kStages;
                 // stage s was last read by the products of tile j - kStages (phase j / kStages - 1 of kv_empty[s])
                 if (j >= kStages && !tc::mbar_wait(&ctrl->kv_empty[s], ((j / kStages) + 1) & 1, abort_flag)) break;
                 tc::mbar_arrive_expect_tx(&ctrl->kv_full[s], kStageBytes);
-                tc::tma_load_3d(sKV + s * kStageBytes, &map_k, 0, (t0 + j) * BN, bh, &ctrl->kv_full[s]);
-                tc::tma_load_3d(sKV + s * kStageBytes + kKBytes, &map_v, 0, (t0 + j) * BN, bh % v_heads, &ctrl->kv_full[s]);
+#pragma unroll
+                for (int x = 0; x < C::kSub; ++x)
+                    tc::tma_load_3d(sKV + s * kStageBytes + x * C::kKSub, &map_k, x * 64, (t0 + j) * BN, bh, &ctrl->kv_full[s]);
+#pragma unroll
+                for (int x = 0; x < C::kSub; ++x)
+                    tc::tma_load_3d(sKV + s * kStageBytes + kKBytes + x * C::kKSub, &map_v, x * 64, (t0 + j) * BN, bh % v_heads,
+                                    &ctrl->kv_full[s]);
                 issued = j + 1;
             }
             if (*abort_flag) {
@@ -313,7 +330,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // tile j: score buffer j % kSBufs (its use number j / kSBufs gives the barrier phase), ring stage j % kStages
         if (lane == 0) {
             constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
-            const uint32_t v_lo = tc::umma_desc_lo(sKV + kKBytes);
+            // MN-major operand: the leading byte offset is the distance between its 64-column sub-tiles
+            const uint32_t v_lo = ((sKV + kKBytes) >> 4 & 0x3fffu) | ((HD == 64 ? 1u : (uint32_t)(C::kKSub >> 4)) << 16);
             bool ok = true;
             int buf = 0, buf_par = 0, st = 0;
             for (int j = 0; ok && j < n_tiles; ++j) {
@@ -352,8 +370,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_fence_after();
                 const uint32_t kt_lo = k_lo + st * (kStageBytes >> 4);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)  // 16 head-dim elements = 32 bytes along a row
-                    tc::umma_f16_lo(tmem + buf * 64, q_lo + ks * 2, kt_lo + ks * 2, idesc_qk, ks > 0);
+                for (int ks = 0; ks < HD / 16; ++ks)  // 16 head-dim elements = 32 bytes along a row of a sub-tile
+                    tc::umma_f16_lo(tmem + buf * 64, q_lo + (ks / 4) * (C::kQSub >> 4) + (ks % 4) * 2,
+                                    kt_lo + (ks / 4) * (C::kKSub >> 4) + (ks % 4) * 2, idesc_qk, ks > 0);
                 tc::umma_commit(&ctrl->s_full[blk][buf]);
                 if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
                 if (++st == kStages) { st = 0; st_par ^= 1; }
@@ -455,13 +474,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             if (j > 0 && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
                 // O belongs to the tensor core until the previous tile's P V is done. Having seen s_full of tile j,
-                // P V of tile j - 4 (the previous phase of this barrier) is known complete: the parity is unambiguous.
+                // P V of tile j - 1 - kSBufs (the previous phase of this barrier) is known complete: the parity is unambiguous.
                 const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
                 ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after();
 #pragma unroll
-                for (int hc = 0; hc < 2; ++hc) {
+                for (int hc = 0; hc < HD / 32; ++hc) {
                     tc::tmem_ld32(tO + hc * 32, vb);
                     tc::tc_wait_ld(vb);
 #pragma unroll
@@ -490,7 +509,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_fence_after();
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
 #pragma unroll
-                for (int hc = 0; hc < 2; ++hc) {
+                for (int hc = 0; hc < HD / 32; ++hc) {
                     tc::tmem_ld32(tO + hc * 32, va);
                     tc::tc_wait_ld(va);
                     if (q < Sq) store_row_half(dst + hc * 32, va, inv);
@@ -505,7 +524,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_fence_after();
                 uint4* po = reinterpret_cast<uint4*>(ws_o) + (size_t)split_slot * (HD / 4) * kUnitRows + row;
 #pragma unroll
-                for (int hc = 0; hc < 2; ++hc) {
+                for (int hc = 0; hc < HD / 32; ++hc) {
                     tc::tmem_ld32(tO + hc * 32, va);
                     tc::tc_wait_ld(va);
 #pragma unroll
@@ -535,27 +554,32 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int p = 0; p < split_count; ++p)
                     m_all = fmaxf(m_all, __ldcg(ws_ml + ((size_t)(split_first + p) * kUnitRows + row) * 2));
                 float l_all = 0.0f;
-                float* acc = reinterpret_cast<float*>(va);  // va, vb: this row's 64 merged outputs
-                float* acc2 = reinterpret_cast<float*>(vb);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) { acc[i] = 0.0f; acc2[i] = 0.0f; }
                 for (int p = 0; p < split_count; ++p) {  // in slot order, whichever CTA merges: the sum is reproducible
-                    const size_t pr = (size_t)(split_first + p) * kUnitRows + row;
-                    const float2 ml = __ldcg(reinterpret_cast<const float2*>(ws_ml + pr * 2));
-                    const float w = fast_exp2(ml.x - m_all);
-                    l_all += w * ml.y;
-                    const float4* src = reinterpret_cast<const float4*>(ws_o) + (size_t)(split_first + p) * (HD / 4) * kUnitRows + row;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float4 a = __ldcg(src + c * kUnitRows), b = __ldcg(src + (8 + c) * kUnitRows);
-                        acc[4 * c] += w * a.x; acc[4 * c + 1] += w * a.y; acc[4 * c + 2] += w * a.z; acc[4 * c + 3] += w * a.w;
-                        acc2[4 * c] += w * b.x; acc2[4 * c + 1] += w * b.y; acc2[4 * c + 2] += w * b.z; acc2[4 * c + 3] += w * b.w;
-                    }
+                    const float2 ml = __ldcg(reinterpret_cast<const float2*>(ws_ml + ((size_t)(split_first + p) * kUnitRows + row) * 2));
+                    l_all += fast_exp2(ml.x - m_all) * ml.y;
                 }
                 const float inv = l_all > 0.0f ? 1.0f / l_all : 0.0f;
-                if (q < Sq) {
-                    store_row_half(dst, va, inv);
-                    store_row_half(dst + 32, vb, inv);
+#pragma unroll 1
+                for (int x = 0; x < C::kSub; ++x) {  // 64 merged outputs of this row at a time, in va and vb
+                    float* acc = reinterpret_cast<float*>(va);
+                    float* acc2 = reinterpret_cast<float*>(vb);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) { acc[i] = 0.0f; acc2[i] = 0.0f; }
+                    for (int p = 0; p < split_count; ++p) {
+                        const float w = fast_exp2(__ldcg(ws_ml + ((size_t)(split_first + p) * kUnitRows + row) * 2) - m_all);
+                        const float4* src = reinterpret_cast<const float4*>(ws_o) +
+                                            ((size_t)(split_first + p) * (HD / 4) + x * 16) * kUnitRows + row;
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            const float4 a = __ldcg(src + c * kUnitRows), b = __ldcg(src + (8 + c) * kUnitRows);
+                            acc[4 * c] += w * a.x; acc[4 * c + 1] += w * a.y; acc[4 * c + 2] += w * a.z; acc[4 * c + 3] += w * a.w;
+                            acc2[4 * c] += w * b.x; acc2[4 * c + 1] += w * b.y; acc2[4 * c + 2] += w * b.z; acc2[4 * c + 3] += w * b.w;
+                        }
+                    }
+                    if (q < Sq) {
+                        store_row_half(dst + x * 64, va, inv);
+                        store_row_half(dst + x * 64 + 32, vb, inv);
+                    }
                 }
             }
         }
@@ -595,13 +619,13 @@ EncodeTiledFn tensor_map_encoder() {
     return fn;
 }
 
-// fp16 tensor [n_heads][rows][64], contiguous; boxes of box_rows x 64 in the 128-byte-swizzled layout,
+// fp16 tensor [n_heads][rows][hd], contiguous; boxes of box_rows x 64 in the 128-byte-swizzled layout,
 // rows past the end of a head read as zeros
-bool make_map(CUtensorMap* m, const void* base, long long n_heads, long long rows, int box_rows) {
+bool make_map(CUtensorMap* m, const void* base, long long n_heads, long long rows, int hd, int box_rows) {
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return false;
-    const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)n_heads};
-    const cuuint64_t strides[2] = {128, (cuuint64_t)rows * 128};  // bytes, dimensions 1 and 2
+    const cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)rows, (cuuint64_t)n_heads};
+    const cuuint64_t strides[2] = {(cuuint64_t)hd * 2, (cuuint64_t)rows * hd * 2};  // bytes, dimensions 1 and 2
     const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -668,12 +692,11 @@ int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, i
     return RFK_OK;
 }
 
-// Launches the tcgen05 kernel; the caller has validated pointers, alignment and sizes (D == 64). v_shared: V is
-// [H, Sk, D], one set of values for every batch element (views of one scene). ws (may be NULL):
-// attention_tc_workspace_bytes() bytes whose first 1024 are zero, for the key split.
-int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
-                        int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared) {
+namespace {
+template <int HD>
+int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
+              int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
+              int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared) {
     // per-device "kernel attributes set" marks; setting them twice from racing threads is harmless
     static std::atomic<bool> configured[64];
     static std::atomic<int> sm_count[64];
@@ -681,12 +704,11 @@ int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __hal
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    constexpr auto kernel = tcattn::attention_tc_kernel<HD>;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(tcattn::attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tcattn::kSmemBytes);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcattn::Cfg<HD>::kSmemBytes);
         if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(tcattn::attention_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return (int)e;
         int sms = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -695,8 +717,8 @@ int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __hal
         configured[dev].store(true, std::memory_order_release);
     }
     CUtensorMap mq, mk, mv;
-    if (!make_map(&mq, Q, (long long)B * H, Sq, tcattn::BM) || !make_map(&mk, K, (long long)B * H, Sk, tcattn::BN) ||
-        !make_map(&mv, V, v_shared ? (long long)H : (long long)B * H, Sk, tcattn::BN))
+    if (!make_map(&mq, Q, (long long)B * H, Sq, HD, tcattn::BM) || !make_map(&mk, K, (long long)B * H, Sk, HD, tcattn::BN) ||
+        !make_map(&mv, V, v_shared ? (long long)H : (long long)B * H, Sk, HD, tcattn::BN))
         return RFK_EUNSUPPORTED;
     tcattn::WorkList work;
     work.q_blocks = ceil_div(Sq, tcattn::kUnitRows);
@@ -705,10 +727,21 @@ int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __hal
     const bool split = ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
     plan_work(work, units, ceil_div(n_keys, tcattn::BN), sm_count[dev].load(std::memory_order_relaxed), split);
     dim3 grid((unsigned)(work.whole_units + work.n_pieces));
-    launch_pdl(tcattn::attention_tc_kernel, grid, dim3(tcattn::kThreads), tcattn::kSmemBytes, st, mq, mk, mv, O, H, Sq, n_keys,
+    launch_pdl(kernel, grid, dim3(tcattn::kThreads), tcattn::Cfg<HD>::kSmemBytes, st, mq, mk, mv, O, H, Sq, n_keys,
                o_bshd, scale * 1.4426950408889634f, row_ss, ss_tiles, norm_dim > 0 ? 1.0f / (float)norm_dim : 0.0f, norm_eps,
                static_cast<unsigned char*>(ws), v_shared ? H : B * H, work);
     return launch_status();
+}
+}  // namespace
+
+// Launches the tcgen05 kernel; the caller has validated pointers, alignment and sizes (D 64 or 128). v_shared: V is
+// [H, Sk, D], one set of values for every batch element (views of one scene). ws (may be NULL):
+// attention_tc_workspace_bytes() bytes whose first 1024 are zero, for the key split.
+int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
+                        int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared) {
+    return (D == 64 ? launch_hd<64> : launch_hd<128>)(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles,
+                                                      norm_dim, norm_eps, ws, ws_bytes, v_shared);
 }
 
 }  // namespace rfk

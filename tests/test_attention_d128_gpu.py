@@ -1,0 +1,94 @@
+"""tcgen05 attention with 128-wide heads (two swizzle sub-tiles per operand row, two score buffers): tile edges, padded
+keys, the key split and its merge, row statistics, and a running reference that turns out wrong. Oracle: torch fp32
+attention on the same fp16 inputs. Tolerance: probabilities and outputs are rounded to fp16 (2^-11 each) and up to 2^8 of
+reference slack does not change a relative rounding, so an output of magnitude up to 4 is within 4e-3 + 4e-3 |want|."""
+import pytest
+import torch
+
+import renderformer_cuda_b200 as pkg
+
+pytestmark = pytest.mark.gpu
+D = 128
+
+
+@pytest.fixture(autouse=True)
+def tc_path():
+    pkg.ops.flash_attention_error(clear=True)
+    pkg.ops.flash_attention_set_path(2)      # the tcgen05 kernel or an error
+    yield
+    pkg.ops.flash_attention_set_path(0)
+    torch.cuda.synchronize()
+    assert pkg.ops.flash_attention_error(clear=True) == 0
+
+
+def _qkv(B, Hh, Sq, Sk, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(Sq * 31 + Sk)
+    return tuple((torch.randn(B, Hh, n, D, device="cuda", generator=g) * s).half() for n, s in ((Sq, scale), (Sk, scale), (Sk, 1.0)))
+
+
+def _close(got, want, what):
+    err = (got.float() - want.float()).abs()
+    assert torch.isfinite(got.float()).all(), what
+    assert (err <= 4e-3 + 4e-3 * want.float().abs()).all(), f"{what}: max error {err.max().item():.2e}"
+    assert err.mean() < 5e-4, f"{what}: mean error {err.mean().item():.2e}"
+
+
+def _want(Q, K, V, n_keys):
+    return torch.nn.functional.scaled_dot_product_attention(Q.float(), K[:, :, :n_keys].float(), V[:, :, :n_keys].float())
+
+
+@pytest.mark.parametrize("B,Hh,Sq,Sk,n_keys,scale", [
+    (1, 1, 128, 64, 64, 1.0), (1, 2, 129, 128, 65, 1.0), (1, 1, 1, 5, 3, 1.0), (2, 3, 300, 1000, 993, 1.0),
+    (1, 2, 256, 384, 384, 1.0), (1, 8, 512, 2048, 2041, 2.0)])
+def test_matches_fp32_attention(B, Hh, Sq, Sk, n_keys, scale):
+    Q, K, V = _qkv(B, Hh, Sq, Sk, scale)
+    O = torch.full_like(Q, 7.0)
+    pkg.ops.flash_attention(Q, K, V, O, B, Hh, Sq, Sk, n_keys, D)
+    _close(O, _want(Q, K, V, n_keys), "whole units")
+    O2 = torch.full((B, Sq, Hh * D), 7.0, device="cuda", dtype=torch.float16)
+    pkg.ops.flash_attention(Q, K, V, O2, B, Hh, Sq, Sk, n_keys, D, o_bshd=True)
+    assert torch.equal(O2.view(B, Sq, Hh, D).permute(0, 2, 1, 3), O)
+
+
+@pytest.mark.parametrize("B,Hh,Sq,Sk,n_keys", [(1, 1, 256, 4096, 4096), (1, 8, 700, 3000, 2995), (3, 2, 256, 2600, 2593)])
+def test_key_split_merges_and_repeats(B, Hh, Sq, Sk, n_keys):
+    Q, K, V = _qkv(B, Hh, Sq, Sk)
+    ws = pkg.ops.flash_attention_workspace()
+    outs = []
+    for _ in range(2):
+        O = torch.full_like(Q, 7.0)
+        pkg.ops.flash_attention_ex(Q, K, V, O, B, Hh, Sq, Sk, n_keys, D, workspace=ws)
+        outs.append(O)
+    _close(outs[0], _want(Q, K, V, n_keys), "split")
+    assert torch.equal(outs[0], outs[1]) and not ws[:1024].any()
+
+
+def test_row_statistics_and_shared_values():
+    B, Hh, Sq, Sk, n_keys = 2, 2, 320, 500, 491
+    Q, K, V = _qkv(B, Hh, Sq, Sk)
+    Q = (Q.float() * 3).half()
+    dim = Hh * D
+    rows = Q.permute(0, 2, 1, 3).reshape(B * Sq, dim).float()
+    ss = torch.stack([rows[:, :128].pow(2).sum(-1), rows[:, 128:].pow(2).sum(-1)], -1).contiguous()
+    O = torch.empty_like(Q)
+    pkg.ops.flash_attention_ex(Q, K, V[0].contiguous(), O, B, Hh, Sq, Sk, n_keys, D, q_row_ss=ss, ss_tiles=2, norm_dim=dim,
+                               v_shared=True)
+    rinv = torch.rsqrt(ss.sum(-1) / dim + pkg.ops.K_EPS_FP16).view(B, 1, Sq, 1)
+    _close(O, _want(Q.float() * rinv, K, V[:1].expand(B, -1, -1, -1), n_keys), "row statistics")
+
+
+@pytest.mark.parametrize("boost", [60.0, 250.0])
+def test_running_reference_is_wrong(boost):
+    """Keys that beat the running reference by far (2^65) and by more than fp32's range (2^128), in columns of both
+    exponential paths, and scores that rise along all keys."""
+    B, Hh, Sq, Sk = 1, 2, 256, 1024
+    Q, K, V = _qkv(B, Hh, Sq, Sk)
+    d = torch.nn.functional.normalize(Q.float().mean(2, keepdim=True), dim=-1)
+    Q = (Q.float() + 6.0 * d).half()
+    Kf = K.float() + 40.0 * torch.linspace(0.0, 1.0, Sk, device="cuda").view(1, 1, Sk, 1) * d
+    Kf[:, :, 64 * 3 + 8, :] += boost * d[:, :, 0, :]
+    Kf[:, :, 64 * 9 + 3, :] += 1.5 * boost * d[:, :, 0, :]
+    K = Kf.half()
+    O = torch.full_like(Q, 7.0)
+    pkg.ops.flash_attention(Q, K, V, O, B, Hh, Sq, Sk, Sk, D)
+    _close(O, _want(Q, K, V, Sk), "wrong reference")
