@@ -39,9 +39,8 @@
 // pieces (it may cross a unit boundary), a piece is one CTA over a range of key tiles. A piece writes its un-normalised
 // O, running maximum and sum to the workspace and increments its unit's counter; the CTA that finds the counter
 // complete (no CTA ever waits for another) merges the unit's pieces, writes the output and zeroes the counter for the
-// next launch. A piece costs about 10 us beyond its tiles (pipeline fill, publishing, merging), which is why grids
-// that already fill the SMs once or more are left whole: measured, cutting the last partial round of a 256-unit grid
-// gains nothing.
+// next launch. A piece costs about 10 us beyond its tiles (pipeline fill, publishing, merging), so the last, partial
+// round of a larger grid is cut the same way only when few units are left for it (plan_work).
 #include <algorithm>
 #include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
 #define RFK_TC_WAIT_INLINE  // this kernel re-partitions its registers (setmaxnreg)
@@ -633,19 +632,25 @@ bool make_map(CUtensorMap* m, const void* base, long long n_heads, long long row
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Fills `w` for `units` units of `n_tiles` key tiles each on a device with `sms` SMs (see "Key split" above).
-// split = false, or the estimate says it does not pay: every unit whole.
+// Fills `w` for `units` units of `n_tiles` key tiles each on a device with `sms` SMs (see "Key split" above): full rounds
+// of units run whole, and the units of the last, partial round are cut when the estimate says it pays.
+// split = false: every unit whole.
 void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool split) {
     using tcattn::Piece;
     constexpr int kPieceCostTiles = 12;  // what a piece costs beyond its tiles (fill, publishing, merging), in tile times
     w.whole_units = (int)units;
     w.n_pieces = 0;
-    if (!split || sms <= 0 || units <= 0 || units >= sms || units > 256 || n_tiles > 65535) return;  // 256 unit counters
-    const long long tiles = units * n_tiles;
+    if (!split || sms <= 0 || units <= 0 || n_tiles > 65535 || units > 65535) return;
+    const int rounds = (int)(units / sms), rest = (int)(units % sms);
+    if (rest == 0 || rest > 256) return;  // 256 unit counters
+    const long long tiles = (long long)rest * n_tiles;
     constexpr int kMaxPiecesPerUnit = 8;  // the CTA that merges a unit reads its pieces one after the other
-    const int shares = (int)std::min<long long>(std::min(sms, tcattn::kMaxPieces / 2), units * kMaxPiecesPerUnit);
-    // whole: one round of n_tiles; split: a share's tiles plus the piece overhead. Cut only for a clear gain.
-    if ((tiles + shares - 1) / shares + kPieceCostTiles > (long long)n_tiles * 4 / 5) return;
+    const int shares = (int)std::min<long long>(std::min(sms, tcattn::kMaxPieces / 2), (long long)rest * kMaxPiecesPerUnit);
+    // whole: one more round of n_tiles; split: a share's tiles plus the piece overhead. Cut only for a clear gain: a fifth of
+    // the launch. (Measured where the estimate gives 7 %, 256 units of 89 tiles on 148 SMs: nothing gained. 184 units of 89
+    // tiles, estimate 31 %: 187 -> 143 us at head size 128; 208 units, estimate 23 %: 141 -> 116 us at head size 64.)
+    if (((long long)rounds * n_tiles + (tiles + shares - 1) / shares + kPieceCostTiles) * 5 > (long long)(rounds + 1) * n_tiles * 4) return;
+    const int whole = rounds * sms;
     Piece* pc = w.pieces;
     int n = 0;
     for (int s = 0; s < shares; ++s) {
@@ -653,7 +658,7 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
         const long long e = tiles * (s + 1) / shares;
         while (b < e) {  // at most twice: a share is shorter than a unit
             const long long u = b / n_tiles, pe = std::min(e, (u + 1) * n_tiles);
-            pc[n].unit = (uint16_t)u;
+            pc[n].unit = (uint16_t)(whole + u);
             pc[n].t0 = (uint16_t)(b - u * n_tiles);
             pc[n].nt = (uint16_t)(pe - b);
             pc[n].slot = (uint16_t)n;
@@ -669,7 +674,7 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     }
     // longest first: in-order dispatch then hands the short pieces to the SMs that finish their long ones first
     std::stable_sort(pc, pc + n, [](const Piece& a, const Piece& b) { return a.nt > b.nt; });
-    w.whole_units = 0;
+    w.whole_units = whole;
     w.n_pieces = n;
 }
 

@@ -50,7 +50,7 @@ def test_matches_fp32_attention(B, Hh, Sq, Sk, n_keys, scale):
     assert torch.equal(O2.view(B, Sq, Hh, D).permute(0, 2, 1, 3), O)
 
 
-@pytest.mark.parametrize("B,Hh,Sq,Sk,n_keys", [(1, 1, 256, 4096, 4096), (1, 8, 700, 3000, 2995), (3, 2, 256, 2600, 2593)])
+@pytest.mark.parametrize("B,Hh,Sq,Sk,n_keys", [(1, 1, 256, 4096, 4096), (1, 8, 700, 3000, 2995), (3, 2, 256, 2600, 2593), (1, 8, 4672, 3000, 2995)])
 def test_key_split_merges_and_repeats(B, Hh, Sq, Sk, n_keys):
     Q, K, V = _qkv(B, Hh, Sq, Sk)
     ws = pkg.ops.flash_attention_workspace()

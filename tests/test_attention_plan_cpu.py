@@ -61,3 +61,15 @@ def test_plan_rejects_bad_arguments():
     assert lib.rfk_flash_attention_plan(4, 8, 0, ctypes.byref(w), ctypes.byref(n), None, 0) == -1
     assert lib.rfk_flash_attention_plan(4, 8, 148, None, ctypes.byref(n), None, 0) == -1
     assert lib.rfk_flash_attention_plan(64, 89, 148, ctypes.byref(w), ctypes.byref(n), None, 0) == 0 and n.value > 0   # count only
+
+
+@pytest.mark.parametrize("units,n_tiles,sms", [(184, 89, 148), (208, 89, 148), (149, 200, 148), (301, 500, 148), (20, 64, 16)])
+def test_last_round_is_cut_behind_whole_rounds(units, n_tiles, sms):
+    whole, pieces = _plan(units, n_tiles, sms)
+    assert whole == units // sms * sms and pieces
+    seen = [[0] * n_tiles for _ in range(units)]
+    for unit, t0, nt, first, count, slot in pieces:
+        assert unit >= whole and first <= slot < first + count <= len(pieces)
+        for t in range(t0, t0 + nt):
+            seen[unit][t] += 1
+    assert all(c == 1 for u in seen[whole:] for c in u)
