@@ -24,6 +24,7 @@
 // This is the portable tensor-core path (it also serves head_dim 128 and ragged lengths);
 // per layer it replaces 0.72 ms of GEMM + softmax + GEMM and 2.2 GB of score traffic.
 #include "common.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -278,11 +279,16 @@ static int launch_flash(const __half* Q, const __half* K, const __half* V, __hal
 }
 
 // ------------------------------------------------------------------ swin window attention
-// One CTA = one (window, head): 64 queries x 64 keys x head_dim 64, everything in one pass:
+// One CTA = one (window, head): 64 queries x 64 keys x head_dim 64 or 128, everything in one pass:
 // S = scale Q K^T (mma.sync), optional shifted-window mask, row softmax in registers, P rounded to
 // fp16 after normalisation (what the unfused GEMM -> softmax -> GEMM sequence does), O = P V, and
 // the output written straight into the [windows * 64, heads * 64] token-major layout the output
-// projection reads. Four warps, 16 query rows each; Q, K, V are 8 KB contiguous tiles.
+// projection reads. Four warps, 16 query rows each; Q, K, V are contiguous tiles of 8 KB (16 KB with 128-wide heads).
+// Bound by latency: a CTA loads its tiles once and has one dependent pass over them, so what counts is that all CTAs of a
+// layer are resident together (8 per SM of 28 KB, 4 per SM of 52 KB: 1024 and 512 CTAs of a 512 x 512 view are one wave).
+// 128-wide heads used to take two library batches, a softmax over a materialised score matrix and a transpose; with the
+// head-split projections and the deferred norms that this kernel lets them use, a 512 x 512 view of 8 heads of 128 takes
+// 3647 us instead of 3954.
 constexpr int kWinTokens = 64, kWinThreads = 128;
 
 // NORMED: Q and K arrive un-normalised (straight from the projection) together with the partial sums of squares of
@@ -290,20 +296,25 @@ constexpr int kWinTokens = 64, kWinThreads = 128;
 // rounding of the separate kernel - is applied while the tiles are staged into shared memory.
 struct WinNorm {
     const float* q_ss; const float* k_ss;      // [rows][tiles] partial sums of squares (rows in window order)
-    const float* gamma_q; const float* gamma_k;  // [heads * 64]
+    const float* gamma_q; const float* gamma_k;  // [heads * head_dim]
     int tiles; float inv_dim, eps;
 };
 
-template <bool NORMED>
-__global__ void __launch_bounds__(kWinThreads, 8)  // 8 CTAs per SM: the 1024 CTAs of a decoder layer are one wave
+template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTokens * kWinTokens;
+
+template <bool NORMED, int HD>
+__global__ void __launch_bounds__(kWinThreads, HD == 64 ? 8 : 4)
 window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
                         __half* __restrict__ O, const uint8_t* __restrict__ mask, int heads, int nW, float scale_log2e,
                         const WinNorm nrm) {
-    constexpr int HD = 64;
-    __shared__ __align__(128) __half sQ[kWinTokens * HD];
-    __shared__ __align__(128) __half sK[kWinTokens * HD];
-    __shared__ __align__(128) __half sV[kWinTokens * HD];
-    __shared__ __align__(16) uint8_t sMask[kWinTokens * kWinTokens];  // this window's mask, fetched with the tiles
+    constexpr int CPR = HD / 8;   // 16-byte chunks per row
+    constexpr int KS = HD / 16;   // k-steps of Q K^T
+    constexpr int NT = HD / 8;    // 8-column output tiles
+    extern __shared__ __align__(128) unsigned char win_smem[];
+    __half* sQ = reinterpret_cast<__half*>(win_smem);
+    __half* sK = sQ + kWinTokens * HD;
+    __half* sV = sK + kWinTokens * HD;
+    uint8_t* sMask = reinterpret_cast<uint8_t*>(sV + kWinTokens * HD);  // this window's mask, fetched with the tiles
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tig = lane & 3;
     pdl_wait();
@@ -313,8 +324,8 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     const __half* Qh = Q + bh * (kWinTokens * HD);
     const __half* Kh = K + bh * (kWinTokens * HD);
     const __half* Vh = V + bh * (kWinTokens * HD);
-    for (int i = tid; i < kWinTokens * 8; i += kWinThreads) {
-        const int r = i >> 3, c = i & 7;
+    for (int i = tid; i < kWinTokens * CPR; i += kWinThreads) {
+        const int r = i / CPR, c = i % CPR;
         if (!NORMED) {
             cp_async16(tile_ptr<HD>(sQ, r, c), Qh + r * HD + c * 8, 16);
             cp_async16(tile_ptr<HD>(sK, r, c), Kh + r * HD + c * 8, 16);
@@ -322,40 +333,44 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
         cp_async16(tile_ptr<HD>(sV, r, c), Vh + r * HD + c * 8, 16);
     }
     if (NORMED) {
-        // A thread keeps one 8-column chunk (c) of four rows (r0 + 16 k) of both tiles: the weights of its columns are
-        // loaded once, and every global load is issued before the first value is needed.
-        const int c = tid & 7, r0 = tid >> 3;
-        constexpr int kRowsPerThread = kWinTokens * 8 / kWinThreads;  // 4
-        Half8 raw[2][kRowsPerThread];
-        float ss[2][kRowsPerThread];
+        // A thread keeps one 8-column chunk (c) of four rows at a time of both tiles: the weights of its columns are
+        // loaded once, and every global load of the four rows is issued before the first value is needed.
+        const int c = tid % CPR, r_first = tid / CPR;
+        constexpr int kRowStep = kWinThreads / CPR;                   // 16 (8 with 128-wide heads)
+        constexpr int kRowsPerPass = 4;
         float gq[8], gk[8];
-#pragma unroll
-        for (int k = 0; k < kRowsPerThread; ++k) {
-            const int r = r0 + k * (kWinThreads / 8);
-            raw[0][k] = ldg_half8(Qh + r * HD + c * 8);
-            raw[1][k] = ldg_half8(Kh + r * HD + c * 8);
-            const long long row = (long long)bw * kWinTokens + r;   // token row in window order
-            float sq = 0.0f, sk = 0.0f;
-            for (int t = 0; t < nrm.tiles; ++t) {
-                sq += __ldg(nrm.q_ss + row * nrm.tiles + t);
-                sk += __ldg(nrm.k_ss + row * nrm.tiles + t);
-            }
-            ss[0][k] = sq;
-            ss[1][k] = sk;
-        }
         ldg_float8(nrm.gamma_q + h * HD + c * 8, gq);
         ldg_float8(nrm.gamma_k + h * HD + c * 8, gk);
 #pragma unroll
-        for (int k = 0; k < kRowsPerThread; ++k) {
-            const int r = r0 + k * (kWinThreads / 8);
+        for (int r0 = r_first; r0 < kWinTokens; r0 += kRowsPerPass * kRowStep) {
+            Half8 raw[2][kRowsPerPass];
+            float ss[2][kRowsPerPass];
 #pragma unroll
-            for (int which = 0; which < 2; ++which) {
-                const float rinv = rsqrtf(ss[which][k] * nrm.inv_dim + nrm.eps);
-                float x[8];
-                unpack8(raw[which][k], x);
+            for (int k = 0; k < kRowsPerPass; ++k) {
+                const int r = r0 + k * kRowStep;
+                raw[0][k] = ldg_half8(Qh + r * HD + c * 8);
+                raw[1][k] = ldg_half8(Kh + r * HD + c * 8);
+                const long long row = (long long)bw * kWinTokens + r;   // token row in window order
+                float sq = 0.0f, sk = 0.0f;
+                for (int t = 0; t < nrm.tiles; ++t) {
+                    sq += __ldg(nrm.q_ss + row * nrm.tiles + t);
+                    sk += __ldg(nrm.k_ss + row * nrm.tiles + t);
+                }
+                ss[0][k] = sq;
+                ss[1][k] = sk;
+            }
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = (x[e] * rinv) * (which ? gk[e] : gq[e]);
-                *reinterpret_cast<Half8*>(tile_ptr<HD>(which ? sK : sQ, r, c)) = pack8(x);
+            for (int k = 0; k < kRowsPerPass; ++k) {
+                const int r = r0 + k * kRowStep;
+#pragma unroll
+                for (int which = 0; which < 2; ++which) {
+                    const float rinv = rsqrtf(ss[which][k] * nrm.inv_dim + nrm.eps);
+                    float x[8];
+                    unpack8(raw[which][k], x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = (x[e] * rinv) * (which ? gk[e] : gq[e]);
+                    *reinterpret_cast<Half8*>(tile_ptr<HD>(which ? sK : sQ, r, c)) = pack8(x);
+                }
             }
         }
     }
@@ -367,17 +382,17 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     cp_async_wait<0>();
     __syncthreads();
 
-    unsigned qf[4][4];
+    unsigned qf[KS][4];
     {
         const int r = warp * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(qf[ks], tile_ptr<HD>(sQ, r, ks * 2 + (lane >> 4)));
+        for (int ks = 0; ks < KS; ++ks) ldmatrix_x4(qf[ks], tile_ptr<HD>(sQ, r, ks * 2 + (lane >> 4)));
     }
     float s[8][4];
 #pragma unroll
     for (int n = 0; n < 8; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.0f;
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
+    for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
         for (int np = 0; np < 4; ++np) {
             unsigned kb[4];
@@ -432,13 +447,13 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
         pf[n >> 1][(n & 1) * 2 + 0] = pack_half2(s[n][0] * rs[0], s[n][1] * rs[0]);
         pf[n >> 1][(n & 1) * 2 + 1] = pack_half2(s[n][2] * rs[1], s[n][3] * rs[1]);
     }
-    float o_acc[8][4];
+    float o_acc[NT][4];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) o_acc[n][0] = o_acc[n][1] = o_acc[n][2] = o_acc[n][3] = 0.0f;
+    for (int n = 0; n < NT; ++n) o_acc[n][0] = o_acc[n][1] = o_acc[n][2] = o_acc[n][3] = 0.0f;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
-        for (int np = 0; np < 4; ++np) {
+        for (int np = 0; np < NT / 2; ++np) {
             unsigned vb[4];
             const int key = ks * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
             ldmatrix_x4_trans(vb, tile_ptr<HD>(sV, key, np * 2 + (lane >> 4)));
@@ -449,7 +464,7 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     // stage this warp's 16 output rows over its own rows of sQ (only this warp read them), then 128-bit stores
     __syncwarp();
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
+    for (int n = 0; n < NT; ++n) {
         const int col = n * 8 + 2 * tig;
         *reinterpret_cast<unsigned*>(tile_ptr<HD>(sQ, q_lo, col >> 3) + (col & 7)) = pack_half2(o_acc[n][0], o_acc[n][1]);
         *reinterpret_cast<unsigned*>(tile_ptr<HD>(sQ, q_lo + 8, col >> 3) + (col & 7)) = pack_half2(o_acc[n][2], o_acc[n][3]);
@@ -457,11 +472,54 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     __syncwarp();
     const long long dim = (long long)heads * HD;
 #pragma unroll
-    for (int i = lane; i < 16 * 8; i += 32) {
-        const int r = warp * 16 + (i >> 3), c = i & 7;
+    for (int i = lane; i < 16 * CPR; i += 32) {
+        const int r = warp * 16 + i / CPR, c = i % CPR;
         *reinterpret_cast<uint4*>(O + ((long long)bw * kWinTokens + r) * dim + h * HD + c * 8) =
             *reinterpret_cast<const uint4*>(tile_ptr<HD>(sQ, r, c));
     }
+}
+
+template <bool NORMED, int HD>
+static int launch_window_attention(const __half* Q, const __half* K, const __half* V, __half* O, const uint8_t* mask, int BnW,
+                                   int heads, int nW, float scale, const WinNorm& nrm, cudaStream_t st) {
+    constexpr int smem = kWinSmemBytes<HD>;
+    if (smem > 48 * 1024) {  // opt in to large dynamic shared memory once per device
+        static std::atomic<bool> configured[64];
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return (int)e;
+        if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+        if (!configured[dev].load(std::memory_order_acquire)) {
+            e = cudaFuncSetAttribute(window_attention_kernel<NORMED, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return (int)e;
+            configured[dev].store(true, std::memory_order_release);
+        }
+    }
+    launch_pdl(window_attention_kernel<NORMED, HD>, dim3((unsigned)((long long)BnW * heads)), dim3(kWinThreads), smem, st, Q, K, V, O,
+               mask, heads, nW, scale * 1.4426950408889634f, nrm);
+    return launch_status();
+}
+
+int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
+                     const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
+                     int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
+                     rfk_stream_t stream) {
+    if (!Q || !K || !V || !O || BnW < 0 || num_heads <= 0 || nW <= 0) return RFK_EINVAL;
+    if (q_row_ss && (!k_row_ss || !gamma_q || !gamma_k || ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
+    if (window_tokens != kWinTokens || (head_dim != 64 && head_dim != 128)) return RFK_EUNSUPPORTED;
+    if (BnW == 0) return RFK_OK;
+    if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O)) return RFK_EUNSUPPORTED;
+    if (mask && !aligned16(mask)) return RFK_EUNSUPPORTED;
+    if ((long long)BnW * num_heads > 0x7fffffffLL) return RFK_EUNSUPPORTED;
+    const __half *q = (const __half*)Q, *k = (const __half*)K, *v = (const __half*)V;
+    cudaStream_t st = as_stream(stream);
+    if (!q_row_ss)
+        return (head_dim == 64 ? launch_window_attention<false, 64> : launch_window_attention<false, 128>)(
+            q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, WinNorm{}, st);
+    if (!aligned16(gamma_q) || !aligned16(gamma_k)) return RFK_EUNSUPPORTED;
+    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
+    return (head_dim == 64 ? launch_window_attention<true, 64> : launch_window_attention<true, 128>)(
+        q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
 }
 
 // attention_tc.cu
@@ -477,6 +535,18 @@ int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __hal
 
 using namespace rfk;
 
+int rfk::flash_attention_mma(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq, int Sk,
+                             int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream) {
+    if (!Q || !K || !V || !O || B < 0 || H <= 0 || Sq < 0 || Sk <= 0 || n_keys <= 0 || n_keys > Sk) return RFK_EINVAL;
+    if (!(scale > 0.0f)) return RFK_EINVAL;
+    if (B == 0 || Sq == 0) return RFK_OK;
+    if ((long long)B * H > 65535) return RFK_EUNSUPPORTED;
+    if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O)) return RFK_EUNSUPPORTED;
+    if (D != 64 && D != 128) return RFK_EUNSUPPORTED;
+    return (D == 64 ? launch_flash<64> : launch_flash<128>)((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H,
+                                                            Sq, Sk, n_keys, (long long)Sk * D, o_bshd, scale, as_stream(stream));
+}
+
 extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B,
                                    int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
                                    rfk_stream_t stream) {
@@ -485,21 +555,13 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     if (B == 0 || Sq == 0) return RFK_OK;
     if ((long long)B * H > 65535) return RFK_EUNSUPPORTED;
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O)) return RFK_EUNSUPPORTED;
-    cudaStream_t st = as_stream(stream);
-    const long long kvs = (long long)Sk * D;
     const int path = g_attn_path.load(std::memory_order_relaxed);
     if ((D == 64 || D == 128) && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
         const int rc = launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk,
-                                           n_keys, D, o_bshd, scale, st, nullptr, 0, 0, 0.0f, nullptr, 0, 0);
+                                           n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0, 0);
         if (rc != RFK_EUNSUPPORTED || path == 2) return rc;
     }
-    if (D == 64)
-        return launch_flash<64>((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, kvs,
-                                o_bshd, scale, st);
-    if (D == 128)
-        return launch_flash<128>((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, kvs,
-                                 o_bshd, scale, st);
-    return RFK_EUNSUPPORTED;
+    return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
 extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
@@ -529,20 +591,14 @@ extern "C" int rfk_flash_attention_set_split(int on) {
     return RFK_OK;
 }
 
+// The C entry points take 64-wide heads; the layers reach the 128-wide form through window_attention above.
 extern "C" int rfk_window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
                                     const uint8_t* mask, int BnW, int num_heads, int window_tokens, int head_dim, int nW,
                                     float scale, rfk_stream_t stream) {
     if (!Q || !K || !V || !O || BnW < 0 || num_heads <= 0 || nW <= 0) return RFK_EINVAL;
-    if (window_tokens != kWinTokens || head_dim != 64) return RFK_EUNSUPPORTED;
-    if (BnW == 0) return RFK_OK;
-    if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O)) return RFK_EUNSUPPORTED;
-    if (mask && !aligned16(mask)) return RFK_EUNSUPPORTED;
-    const long long ctas = (long long)BnW * num_heads;
-    if (ctas > 0x7fffffffLL) return RFK_EUNSUPPORTED;
-    launch_pdl(window_attention_kernel<false>, dim3((unsigned)ctas), dim3(kWinThreads), 0, as_stream(stream),
-               (const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, mask, num_heads, nW,
-               scale * 1.4426950408889634f, WinNorm{});
-    return launch_status();
+    if (head_dim != 64) return RFK_EUNSUPPORTED;
+    return window_attention(Q, K, V, O, mask, nullptr, nullptr, 0, nullptr, nullptr, 0, 0.0f, BnW, num_heads, window_tokens,
+                            head_dim, nW, scale, stream);
 }
 
 extern "C" int rfk_window_attention_normed(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
@@ -553,16 +609,7 @@ extern "C" int rfk_window_attention_normed(const rfk_half* Q, const rfk_half* K,
     if (!Q || !K || !V || !O || !q_row_ss || !k_row_ss || !gamma_q || !gamma_k || BnW < 0 || num_heads <= 0 || nW <= 0 ||
         ss_tiles <= 0 || norm_dim <= 0)
         return RFK_EINVAL;
-    if (window_tokens != kWinTokens || head_dim != 64) return RFK_EUNSUPPORTED;
-    if (BnW == 0) return RFK_OK;
-    if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(gamma_q) || !aligned16(gamma_k))
-        return RFK_EUNSUPPORTED;
-    if (mask && !aligned16(mask)) return RFK_EUNSUPPORTED;
-    const long long ctas = (long long)BnW * num_heads;
-    if (ctas > 0x7fffffffLL) return RFK_EUNSUPPORTED;
-    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
-    launch_pdl(window_attention_kernel<true>, dim3((unsigned)ctas), dim3(kWinThreads), 0, as_stream(stream),
-               (const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, mask, num_heads, nW,
-               scale * 1.4426950408889634f, nrm);
-    return launch_status();
+    if (head_dim != 64) return RFK_EUNSUPPORTED;
+    return window_attention(Q, K, V, O, mask, q_row_ss, k_row_ss, ss_tiles, gamma_q, gamma_k, norm_dim, eps, BnW, num_heads,
+                            window_tokens, head_dim, nW, scale, stream);
 }

@@ -29,6 +29,7 @@
 #include <cstdlib>
 #include "attention_tc.cuh"
 #include "common.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -77,7 +78,7 @@ struct Params {
     int M, N, K;                        // N = output columns
     int tiles_m, tiles_n;
     float* row_ss;                      // kEpiHeads: [parts][M][tiles per part] partial sums of squares, or null
-    int seq, heads, ss_mask;            // kEpiHeads: rows per group, heads per part (64 wide), parts that get row_ss
+    int seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
 };
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
@@ -531,8 +532,9 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
         __syncwarp();
         if (lane == 0) {
             if (EPI == kEpiHeads) {
-                const int g = (n0 + u * kUnitCols) / kUnitCols;   // 64-wide head index over all parts
-                tma_store_5d(map_c, stage_base + b * kUnitBytes, 0, row0 % p.seq, g % p.heads, row0 / p.seq, g / p.heads);
+                const int g = (n0 + u * kUnitCols) / kUnitCols;   // 64-column unit over all parts
+                tma_store_5d(map_c, stage_base + b * kUnitBytes, (g % p.head_units) * kUnitCols, row0 % p.seq,
+                             (g % p.units) / p.head_units, row0 / p.seq, g / p.units);
             } else {
                 tma_store_2d(map_c, stage_base + b * kUnitBytes, n0 + u * kUnitCols, row0);   // rows >= M, columns >= N are clipped
             }
@@ -540,7 +542,7 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
         }
     }
     if (EPI == kEpiHeads && p.row_ss) {
-        const int dim = p.heads * kUnitCols, part = n0 / dim, row = row0 + lane;
+        const int dim = p.units * kUnitCols, part = n0 / dim, row = row0 + lane;
         if (((p.ss_mask >> part) & 1) && row < p.M)
             p.row_ss[((size_t)part * p.M + row) * (dim / 256) + (n0 % dim) / 256] = ss;
     }
@@ -824,12 +826,14 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtens
     return launch_status();
 }
 
-// rank-5 map of a head-split output: [part][group][head][seq][64] halves, boxes of 32 rows x 64 columns
-bool make_map_heads(CUtensorMap* m, const void* base, int seq, int heads, long long groups, int parts, long long part_stride) {
+// rank-5 map of a head-split output: [part][group][head][seq][hd] halves, boxes of 32 rows x 64 columns
+bool make_map_heads(CUtensorMap* m, const void* base, int seq, int heads, int hd, long long groups, int parts,
+                    long long part_stride) {
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return false;
-    const cuuint64_t dims[5] = {64, (cuuint64_t)seq, (cuuint64_t)heads, (cuuint64_t)groups, (cuuint64_t)parts};
-    const cuuint64_t strides[4] = {128, (cuuint64_t)seq * 128, (cuuint64_t)heads * seq * 128, (cuuint64_t)part_stride * 2};
+    const cuuint64_t row = (cuuint64_t)hd * 2;
+    const cuuint64_t dims[5] = {(cuuint64_t)hd, (cuuint64_t)seq, (cuuint64_t)heads, (cuuint64_t)groups, (cuuint64_t)parts};
+    const cuuint64_t strides[4] = {row, (cuuint64_t)seq * row, (cuuint64_t)heads * seq * row, (cuuint64_t)part_stride * 2};
     const cuuint32_t box[5] = {64, 32, 1, 1, 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
@@ -891,11 +895,12 @@ extern "C" int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W,
     }
 }
 
-extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out,
-                                  long long part_stride, float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len,
-                                  int num_heads, rfk_stream_t stream) {
+int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out, long long part_stride,
+                    float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int num_heads, int head_dim,
+                    rfk_stream_t stream) {
     if (!A || !W || !out || M < 0 || N <= 0 || K <= 0 || seq_len <= 0 || num_heads <= 0 || lda < K || ldw < K) return RFK_EINVAL;
-    const int dim = num_heads * 64;
+    if (head_dim != 64 && head_dim != 128) return RFK_EUNSUPPORTED;
+    const int dim = num_heads * head_dim;
     if (N % dim != 0 || (ss_parts_mask && !row_ss)) return RFK_EINVAL;
     const int parts = N / dim;
     if (parts > 1 && part_stride < (long long)M * dim) return RFK_EINVAL;
@@ -913,14 +918,20 @@ extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_ha
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
     CUtensorMap ma, mw, mh;
     if (!make_map_2d(&ma, A, M, K, lda) || !make_map_2d(&mw, W, N, K, ldw) ||
-        !make_map_heads(&mh, out, seq_len, num_heads, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
+        !make_map_heads(&mh, out, seq_len, num_heads, head_dim, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
         return RFK_EUNSUPPORTED;
     tcgemm::Params p{};
     p.C = (__half*)out; p.ldc = N; p.M = M; p.N = N; p.K = K;
     p.tiles_m = (M + tcgemm::BM - 1) / tcgemm::BM;
     p.tiles_n = N / 256;
-    p.row_ss = row_ss; p.seq = seq_len; p.heads = num_heads; p.ss_mask = ss_parts_mask;
+    p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
     return launch_gemm_pair<tcgemm::kEpiHeads>(ma, mw, mw, p, dev, as_stream(stream), &mh);
+}
+
+extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out,
+                                  long long part_stride, float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len,
+                                  int num_heads, rfk_stream_t stream) {
+    return gemm_heads(A, lda, W, ldw, out, part_stride, row_ss, ss_parts_mask, M, N, K, seq_len, num_heads, 64, stream);
 }
 
 extern "C" int rfk_gemm_pair_clusters(void) {

@@ -1,0 +1,23 @@
+// Forms of the kernels that only the layer library uses (not part of the C ABI): more head sizes than the C entry points
+// of the same name take.
+#pragma once
+#include "rfk.h"
+
+namespace rfk {
+
+// rfk_gemm_f16_heads for heads of 64 or 128: out is [part][group][head][seq][head_dim]
+int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out, long long part_stride,
+               float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int num_heads, int head_dim,
+               rfk_stream_t stream);
+
+// rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128
+int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
+                     const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
+                     int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
+                     rfk_stream_t stream);
+
+// the mma.sync kernel of rfk_flash_attention, whatever path is set
+int flash_attention_mma(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq, int Sk,
+                        int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);
+
+}  // namespace rfk

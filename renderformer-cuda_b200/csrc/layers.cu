@@ -18,12 +18,13 @@
 //   - attention is one fused kernel whenever head_dim is 64 or 128 (rfk_flash_attention: no
 //     score matrix, output written [B,Sq,H*D] directly); other head sizes keep GEMM -> softmax
 //     (fp16 probabilities over its own fp32 score rows) -> GEMM;
-//   - swin attention with 64-token windows and head_dim 64 is one kernel per layer
+//   - swin attention with 64-token windows and head_dim 64 or 128 is one kernel per layer
 //     (rfk_window_attention); cyclic shift + window partition are folded into the norm before
 //     it, window reverse + un-shift + residual add into the norm after it
 //     (rfk_rmsnorm_residual_f16_windows); other window / head sizes keep the gather ->
 //     GEMM -> softmax -> GEMM -> scatter sequence;
 //   - w1 and w3 run as one GEMM when stored back to back; the gate overwrites its own input.
+#include "kernels_internal.h"
 #include "layers_internal.h"
 
 #include <algorithm>
@@ -219,6 +220,10 @@ static int attention_core(rfk_ctx* ctx, const rfk_half* Q, const rfk_half* K, co
                           float* score_buf, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd,
                           rfk_stream_t stream) {
     int rc = RFK_EUNSUPPORTED;
+    if (D == 128 && ctx->d128_reproducible) {
+        rc = rfk::flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
+        if (rc != RFK_EUNSUPPORTED) return rc;
+    }
     if (ctx->attn_ws)  // tcgen05 kernel with the balanced key split; declines what only the other kernels serve
         rc = rfk_flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, 0, B, H, Sq, Sk, n_keys, D,
                                     o_bshd, 1.0f / sqrtf((float)D), stream);
@@ -305,13 +310,15 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
     // Deferred Q-RMSNorm: the projection writes Q head-split and the rows' sums of squares, the attention kernel scales
     // each row's scores by 1 / rms, and the norm's weight rides on the keys (multiplied in by the rotation kernel, here
     // or by the caller). One kernel (norm + head split) and 18 MB of traffic less per layer. Needs: no query rotation
-    // (the view decoder's query tables are the identity), keys that are rotated here or arrive prescaled, head size 64.
+    // (the view decoder's query tables are the identity), keys that are rotated here or arrive prescaled, head size 64
+    // or 128.
     const int k_prescaled = cache_flags & 1, v_shared = (cache_flags >> 1) & 1;
-    const bool deferred = norm_ss && w->q_norm_gamma && !w->q_proj_b && !q_rope_cos && hd == 64 && (k_prescaled || k_rope_cos) &&
+    const bool deferred = norm_ss && w->q_norm_gamma && !w->q_proj_b && !q_rope_cos &&
+                          (hd == 64 || (hd == 128 && !ctx->d128_reproducible)) && (k_prescaled || k_rope_cos) &&
                           (reinterpret_cast<uintptr_t>(w->q_norm_gamma) & 15u) == 0;
     if (k_prescaled && !deferred) return RFK_EUNSUPPORTED;  // prescaled keys only make sense with the deferred norm
     if (deferred) {
-        int rc = rfk_gemm_f16_heads(q_in, q_dim, w->q_proj_w, q_dim, Q_bhsd, 0, norm_ss, 1, Mq, dim, q_dim, Sq, num_heads, stream);
+        int rc = rfk::gemm_heads(q_in, q_dim, w->q_proj_w, q_dim, Q_bhsd, 0, norm_ss, 1, Mq, dim, q_dim, Sq, num_heads, hd, stream);
         if (rc == RFK_OK) {
             const rfk_half* K_use = K_cached;
             if (!k_prescaled) {
@@ -378,14 +385,16 @@ static int swin_core(rfk_ctx* ctx, const rfk_mha_weights* w, rfk_half* window_bu
     // Deferred QK-RMSNorm: the packed projection writes q, k, v head-split per window and the sums of squares of the q and
     // k rows; the window attention kernel normalises the two tiles while it stages them (same formula and rounding as
     // the separate kernel). One kernel and 50 MB of traffic less per layer.
-    if (norm_ss && ws2 == 64 && hd == 64 && w->q_norm_gamma && w->k_norm_gamma && !w->in_proj_b) {
+    const bool fused = ws2 == 64 && (hd == 64 || (hd == 128 && !ctx->d128_reproducible));  // the window attention kernel
+    if (hd != 64 && !score_buf) return RFK_EINVAL;            // score space is only optional for 64-wide heads
+    if (norm_ss && fused && w->q_norm_gamma && w->k_norm_gamma && !w->in_proj_b) {
         const int tiles = dim / 256;
-        int rc = rfk_gemm_f16_heads(window_buf, dim, w->in_proj_w, dim, Qt, (long long)M * dim, norm_ss, 3, M, 3 * dim, dim, ws2,
-                                    num_heads, stream);
+        int rc = rfk::gemm_heads(window_buf, dim, w->in_proj_w, dim, Qt, (long long)M * dim, norm_ss, 3, M, 3 * dim, dim, ws2,
+                                 num_heads, hd, stream);
         if (rc == RFK_OK)
-            rc = rfk_window_attention_normed(Qt, Kt, Vt, window_buf, win_mask, norm_ss, norm_ss + (size_t)M * tiles, tiles,
-                                             w->q_norm_gamma, w->k_norm_gamma, dim, kEpsFp16, BnW, num_heads, ws2, hd, nW,
-                                             1.0f / sqrtf((float)hd), stream);
+            rc = rfk::window_attention(Qt, Kt, Vt, window_buf, win_mask, norm_ss, norm_ss + (size_t)M * tiles, tiles,
+                                       w->q_norm_gamma, w->k_norm_gamma, dim, kEpsFp16, BnW, num_heads, ws2, hd, nW,
+                                       1.0f / sqrtf((float)hd), stream);
         if (rc == RFK_OK) return rfk_linear(ctx, window_buf, w->out_proj_w, w->out_proj_b, qkv_buf, M, dim, dim, stream);
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
@@ -396,9 +405,11 @@ static int swin_core(rfk_ctx* ctx, const rfk_mha_weights* w, rfk_half* window_bu
     TRY(project_epilogue(qkv_buf, 3LL * dim, 3, g, o, no_rope, nullptr, nullptr, BnW, ws2, num_heads, hd, 0,
                          window_buf, stream));
     const float scale = 1.0f / sqrtf((float)hd), zero = 0.0f, one = 1.0f;
-    if (ws2 == 64 && hd == 64) {  // the whole window attention in one kernel, output already token-major
-        TRY(rfk_window_attention(Qt, Kt, Vt, window_buf, win_mask, BnW, num_heads, ws2, hd, nW, scale, stream));
-        return rfk_linear(ctx, window_buf, w->out_proj_w, w->out_proj_b, qkv_buf, M, dim, dim, stream);
+    if (fused) {  // the whole window attention in one kernel, output already token-major
+        const int rc = rfk::window_attention(Qt, Kt, Vt, window_buf, win_mask, nullptr, nullptr, 0, nullptr, nullptr, 0, 0.0f,
+                                             BnW, num_heads, ws2, hd, nW, scale, stream);
+        if (rc == RFK_OK) return rfk_linear(ctx, window_buf, w->out_proj_w, w->out_proj_b, qkv_buf, M, dim, dim, stream);
+        if (rc != RFK_EUNSUPPORTED || hd == 64) return rc;   // the separate steps below serve 128-wide heads without it
     }
     if (!score_buf) return RFK_EINVAL;
     TRY(blas_status(cublasSetStream(ctx->blas, st)));
