@@ -564,10 +564,10 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
-extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
-                                      const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
-                                      size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
-                                      int o_bshd, float scale, rfk_stream_t stream) {
+extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
+                                           const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
+                                           size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
+                                           int o_bshd, float scale, rfk_stream_t stream) {
     if (!Q || !K || !V || !O || B < 0 || H <= 0 || Sq < 0 || Sk <= 0 || n_keys <= 0 || n_keys > Sk || !(scale > 0.0f))
         return RFK_EINVAL;
     if (q_row_ss && (ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
@@ -577,6 +577,16 @@ extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, cons
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
     return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D,
                                o_bshd, scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared != 0);
+}
+
+// The public form takes 64-wide heads, as its header says.
+extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
+                                      const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
+                                      size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
+                                      int o_bshd, float scale, rfk_stream_t stream) {
+    const int rc = rfk_flash_attention_ex_wide(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared,
+                                               D == 64 || B < 0 ? B : 0, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
+    return rc == RFK_OK && D != 64 && B > 0 && Sq != 0 ? RFK_EUNSUPPORTED : rc;
 }
 
 extern "C" size_t rfk_flash_attention_workspace_bytes(void) { return attention_tc_workspace_bytes(); }

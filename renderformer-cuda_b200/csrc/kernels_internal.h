@@ -21,3 +21,9 @@ int flash_attention_mma(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
                         int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);
 
 }  // namespace rfk
+
+// rfk_flash_attention_ex for heads of 64 or 128
+extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
+                                           const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
+                                           size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
+                                           int o_bshd, float scale, rfk_stream_t stream);

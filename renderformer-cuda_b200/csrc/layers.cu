@@ -225,7 +225,7 @@ static int attention_core(rfk_ctx* ctx, const rfk_half* Q, const rfk_half* K, co
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
     if (ctx->attn_ws)  // tcgen05 kernel with the balanced key split; declines what only the other kernels serve
-        rc = rfk_flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, 0, B, H, Sq, Sk, n_keys, D,
+        rc = rfk_flash_attention_ex_wide(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, 0, B, H, Sq, Sk, n_keys, D,
                                     o_bshd, 1.0f / sqrtf((float)D), stream);
     if (rc == RFK_EUNSUPPORTED)
         rc = rfk_flash_attention(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
@@ -328,7 +328,7 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
                 K_use = K_rot;
             }
             if (rc == RFK_OK)
-                rc = rfk_flash_attention_ex(Q_bhsd, K_use, V_cached, Q, norm_ss, dim / 256, dim, kEpsFp16, ctx->attn_ws,
+                rc = rfk_flash_attention_ex_wide(Q_bhsd, K_use, V_cached, Q, norm_ss, dim / 256, dim, kEpsFp16, ctx->attn_ws,
                                             ctx->attn_ws_bytes, v_shared, B, num_heads, Sq, Sk, n_keys, hd, 1,
                                             1.0f / sqrtf((float)hd), stream);
         }

@@ -2,10 +2,13 @@
 keys, the key split and its merge, row statistics, and a running reference that turns out wrong. Oracle: torch fp32
 attention on the same fp16 inputs. Tolerance: probabilities and outputs are rounded to fp16 (2^-11 each) and up to 2^8 of
 reference slack does not change a relative rounding, so an output of magnitude up to 4 is within 4e-3 + 4e-3 |want|."""
+import ctypes
+
 import pytest
 import torch
 
 import renderformer_cuda_b200 as pkg
+from renderformer_cuda_b200 import _abi
 
 pytestmark = pytest.mark.gpu
 D = 128
@@ -33,6 +36,18 @@ def _close(got, want, what):
     assert err.mean() < 5e-4, f"{what}: mean error {err.mean().item():.2e}"
 
 
+def _ex(q, k, v, o, B, Hh, Sq, Sk, n_keys, D, q_row_ss=None, ss_tiles=0, norm_dim=0, workspace=None, v_shared=False):
+    """What the layers call: flash_attention_ex for both head sizes (the public form takes 64-wide heads)."""
+    lib = _abi.load("rfk.h")
+    fn = lib.rfk_flash_attention_ex_wide
+    fn.argtypes, fn.restype = lib.rfk_flash_attention_ex.argtypes, ctypes.c_int
+    p = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
+    rc = fn(p(q), p(k), p(v), p(o), p(q_row_ss), ss_tiles, norm_dim, pkg.ops.K_EPS_FP16, p(workspace),
+            0 if workspace is None else workspace.numel(), int(v_shared), B, Hh, Sq, Sk, n_keys, D, 0, D ** -0.5,
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, rc
+
+
 def _want(Q, K, V, n_keys):
     return torch.nn.functional.scaled_dot_product_attention(Q.float(), K[:, :, :n_keys].float(), V[:, :, :n_keys].float())
 
@@ -57,7 +72,7 @@ def test_key_split_merges_and_repeats(B, Hh, Sq, Sk, n_keys):
     outs = []
     for _ in range(2):
         O = torch.full_like(Q, 7.0)
-        pkg.ops.flash_attention_ex(Q, K, V, O, B, Hh, Sq, Sk, n_keys, D, workspace=ws)
+        _ex(Q, K, V, O, B, Hh, Sq, Sk, n_keys, D, workspace=ws)
         outs.append(O)
     _close(outs[0], _want(Q, K, V, n_keys), "split")
     assert torch.equal(outs[0], outs[1]) and not ws[:1024].any()
@@ -71,7 +86,7 @@ def test_row_statistics_and_shared_values():
     rows = Q.permute(0, 2, 1, 3).reshape(B * Sq, dim).float()
     ss = torch.stack([rows[:, :128].pow(2).sum(-1), rows[:, 128:].pow(2).sum(-1)], -1).contiguous()
     O = torch.empty_like(Q)
-    pkg.ops.flash_attention_ex(Q, K, V[0].contiguous(), O, B, Hh, Sq, Sk, n_keys, D, q_row_ss=ss, ss_tiles=2, norm_dim=dim,
+    _ex(Q, K, V[0].contiguous(), O, B, Hh, Sq, Sk, n_keys, D, q_row_ss=ss, ss_tiles=2, norm_dim=dim,
                                v_shared=True)
     rinv = torch.rsqrt(ss.sum(-1) / dim + pkg.ops.K_EPS_FP16).view(B, 1, Sq, 1)
     _close(O, _want(Q.float() * rinv, K, V[:1].expand(B, -1, -1, -1), n_keys), "row statistics")
