@@ -270,9 +270,10 @@ extern "C" int rfk_precompute_cross_kv(rfk_ctx* ctx, const rfk_cross_attn_weight
     TRY(rfk_linear(ctx, ctx_normed, w->k_proj_w, w->k_proj_b, Kp, Mk, dim, kv_dim, stream));
     TRY(rfk_linear(ctx, ctx_normed, w->v_proj_w, w->v_proj_b, Vp, Mk, dim, kv_dim, stream));
     if (Sk_pad != Sk) {
-        const size_t bytes = (size_t)B * num_heads * Sk_pad * hd * 2;
-        cudaError_t e = cudaMemsetAsync(K_out, 0, bytes, (cudaStream_t)stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(V_out, 0, bytes, (cudaStream_t)stream);
+        // only the rows behind the last key of each head; every other element is written below
+        const size_t pitch = (size_t)Sk_pad * hd * 2, width = (size_t)(Sk_pad - Sk) * hd * 2, heads = (size_t)B * num_heads;
+        cudaError_t e = cudaMemset2DAsync(K_out + (size_t)Sk * hd, pitch, 0, width, heads, (cudaStream_t)stream);
+        if (e == cudaSuccess) e = cudaMemset2DAsync(V_out + (size_t)Sk * hd, pitch, 0, width, heads, (cudaStream_t)stream);
         if (e != cudaSuccess) return (int)e;
     }
     const float* g[1] = {w->k_norm_gamma};

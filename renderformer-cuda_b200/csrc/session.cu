@@ -62,12 +62,55 @@ StateLayout state_layout(const rfk_model& m, int n_tris) {
     return L;
 }
 
-// last `last_n` channels of each row: v <- half(log10f(float(v) + 1))   (render_session.cu:33-38)
-__global__ void log_encode_kernel(__half* data, int N, int C, int last_n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N * last_n) return;
-    const int n = i / last_n, idx = n * C + (C - last_n) + (i % last_n);
-    data[idx] = __float2half(log10f(__half2float(data[idx]) + 1.0f));
+// ---- scene encoding, the geometry ahead of the encoder. The centre was summed on the host and the register positions were
+// built there: two round trips in which the device stood still for 0.5 ms. Two short kernels instead, and nothing waits for
+// the host until the call's end.
+
+// One element each of the geometry kept for every view (fp16, render_session.cu:301-304), of the encoder's positions behind
+// the register tokens (render_session.cu:342-350), and of the texture, whose last `last_n` channels become
+// half(log10f(v + 1)) (render_session.cu:33-38).
+__global__ void scene_inputs_kernel(const float* __restrict__ tri, const float* __restrict__ vn, const __half* __restrict__ tex,
+                                    __half* __restrict__ tri16, __half* __restrict__ vn16, __half* __restrict__ pos,
+                                    __half* __restrict__ tex_out, int N, int C, int last_n) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (long long)N * 9) {
+        const __half t = __float2half(tri[i]);
+        tri16[i] = t;
+        pos[i] = t;
+        vn16[i] = __float2half(vn[i]);
+    }
+    if (i < (long long)N * C)
+        tex_out[i] = (int)(i % C) >= C - last_n ? __float2half(log10f(__half2float(tex[i]) + 1.0f)) : tex[i];
+}
+
+// Scene centre = mean of all 3N fp16 vertices (render_session.cu:62-70), summed in double precision: every partial sum of
+// fp16 values below 2^29 is exact, so the order does not matter. One CTA: 1023 threads, a multiple of three, so that a
+// thread stays on one axis. Then the register tokens' positions, the centre three times over (render_session.cu:91-97).
+__global__ void __launch_bounds__(1024)
+scene_centre_kernel(const __half* __restrict__ tri16, float* __restrict__ centre, __half* __restrict__ reg_pos, int N, int nr) {
+    __shared__ double part[3][32];
+    __shared__ float c[3];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long n = (long long)N * 9;
+    double sum = 0.0;
+    if (tid < 1023) {
+#pragma unroll 8
+        for (long long i = tid; i < n; i += 1023) sum += (double)__half2float(tri16[i]);
+    }
+    for (int a = 0; a < 3; ++a) {
+        double v = (tid < 1023 && tid % 3 == a) ? sum : 0.0;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) part[a][warp] = v;
+    }
+    __syncthreads();
+    if (tid < 3) {
+        double v = 0.0;
+        for (int w = 0; w < 32; ++w) v += part[tid][w];
+        c[tid] = (float)(v / (3.0 * N));
+        centre[tid] = c[tid];
+    }
+    __syncthreads();
+    for (int i = tid; i < nr * 9; i += 1024) reg_pos[i] = __float2half(c[i % 3]);
 }
 
 // out = a + b + float(c[i % dim])   (render_session.cu:39-43)
@@ -142,6 +185,7 @@ struct rfk_session {
     long long frames = 0;  // frames submitted so far
     int graph_nodes = 0, kernels_per_view = 0;
     bool finalized = false;
+    char* encode_block = nullptr;  // work buffers of the scene encoding, allocated by the first one (see EncodeBuffers)
 
     rfk_half* kvK(int layer) const { return (rfk_half*)(state + L.kv_off + (size_t)(2 * layer) * L.kv_layer_bytes); }
     // rotated keys: [dec_layers][V][heads][Se_pad][hd], so that a layer's keys are one [V * heads, Se_pad, hd] batch
@@ -381,17 +425,50 @@ extern "C" int rfk_session_destroy(rfk_session* d) {
     return RFK_OK;
 }
 
-// Scratch allocations of the one-time scene encoding (freed on every exit path).
-struct Scratch {
-    std::vector<void*> ptrs;
-    ~Scratch() { for (void* p : ptrs) cudaFree(p); }
-    template <typename T> int get(T** p, size_t count) {
-        void* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, std::max<size_t>(count * sizeof(T), 256));
-        if (e != cudaSuccess) return (int)e;
-        ptrs.push_back(d);
-        *p = (T*)d;
-        return RFK_OK;
+// Carves 256-byte aligned pieces out of one block; with base NULL it only adds up what they need.
+struct Carver {
+    char* base;
+    size_t used = 0;
+    template <typename T> void get(T** p, size_t count) {
+        *p = base ? (T*)(base + used) : nullptr;
+        used += align_up(std::max<size_t>(count * sizeof(T), 256), 256);
+    }
+};
+
+// Work buffers of the scene encoding. They are one block that the session keeps (174 MB at 5633 triangles): 19 cudaMalloc
+// and as many cudaFree a call, and the host work above, took 6.7 of 12.7 ms (5633 triangles; now 6.0). The embeddings and the K/V
+// projections lie in the layers' qkv buffer, which is idle before the first and after the last encoder layer.
+struct EncodeBuffers {
+    rfk_half *tex, *vn_pe, *pos, *cos, *sin, *temp, *qkv, *ffn;
+    rfk_half* emb16;                            // inside qkv, before the encoder; fp32 beside it:
+    float *vn_n, *tex_n;
+    rfk_half *ctx16, *ctx_normed, *kv_proj;     // inside qkv, after it
+    float *seq, *score;
+    size_t plan(const rfk_session& d, char* base) {
+        const rfk_model& m = d.m;
+        const size_t Se = d.Se, N = d.N, dim = m.dim;
+        Carver c{base};
+        c.get(&tex, N * m.texture_channels);
+        c.get(&vn_pe, N * (9 + 9 * m.vn_pe_num_freqs * 2));
+        c.get(&pos, Se * 9);
+        c.get(&cos, Se * d.hd);
+        c.get(&sin, Se * d.hd);
+        c.get(&seq, Se * dim);
+        c.get(&temp, Se * dim);
+        c.get(&qkv, std::max(6 * align_up(Se * dim, 128), 2 * Se * (size_t)m.ffn_hidden));
+        c.get(&ffn, Se * std::max(dim, (size_t)m.ffn_hidden));
+        score = nullptr;
+        if (!(d.hd == 64 || d.hd == 128)) c.get(&score, (size_t)m.num_heads * Se * d.Se_pad);
+        if (base) {
+            const size_t piece = align_up(Se * dim, 128);   // halves, so that every piece is 256-byte aligned
+            emb16 = qkv;
+            vn_n = (float*)(qkv + piece);
+            tex_n = (float*)(qkv + 3 * piece);
+            ctx16 = qkv;
+            ctx_normed = qkv + piece;
+            kv_proj = qkv + 2 * piece;                      // two pieces
+        }
+        return c.used;
     }
 };
 
@@ -403,86 +480,43 @@ extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const 
     const int vn_pe_dim = 9 + 9 * m.vn_pe_num_freqs * 2;
     cudaStream_t st = d->stream;
     rfk_stream_t s = (rfk_stream_t)st;
-    Scratch sc;
+    EncodeBuffers b{};
+    if (!d->encode_block) TRY(d->alloc(&d->encode_block, b.plan(*d, nullptr)));
+    b.plan(*d, d->encode_block);
 
-    // texture: log-encode the last 3 channels (render_session.cu:297-299)
-    rfk_half* tex_buf; TRY(sc.get(&tex_buf, (size_t)N * C));
-    TRY_CUDA(cudaMemcpyAsync(tex_buf, tex, (size_t)N * C * sizeof(rfk_half), cudaMemcpyDeviceToDevice, st));
-    log_encode_kernel<<<blocks_for((long long)N * 3), 256, 0, st>>>((__half*)tex_buf, N, C, 3);
-    // fp16 copies of the geometry kept for every view (render_session.cu:301-304)
-    TRY(rfk_cast_fp32_to_fp16(tri, d->tri16(), (long long)N * 9, s));
-    TRY(rfk_cast_fp32_to_fp16(vn, d->vn16(), (long long)N * 9, s));
-    // Scene centre = mean of all 3N fp16 vertices, summed on the host in double precision (the
-    // reference's centroid is the same quantity, src/pipeline/render_session.cu:62-70).
-    std::vector<__half> h_tri((size_t)N * 9);
-    TRY_CUDA(cudaMemcpyAsync(h_tri.data(), d->tri16(), h_tri.size() * sizeof(__half), cudaMemcpyDeviceToHost, st));
-    TRY_CUDA(cudaStreamSynchronize(st));
-    double axis_sum[3] = {0.0, 0.0, 0.0};
-    for (size_t v = 0; v < (size_t)N * 3; ++v)
-        for (int a = 0; a < 3; ++a) axis_sum[a] += (double)__half2float(h_tri[v * 3 + a]);
-    float c[3];
-    for (int a = 0; a < 3; ++a) c[a] = (float)(axis_sum[a] / (3.0 * N));
-    TRY_CUDA(cudaMemcpyAsync(d->center(), c, sizeof(c), cudaMemcpyHostToDevice, st));
-
+    scene_inputs_kernel<<<blocks_for((long long)N * std::max(9, C)), 256, 0, st>>>(
+        tri, vn, (const __half*)tex, (__half*)d->tri16(), (__half*)d->vn16(), (__half*)b.pos + (size_t)nr * 9, (__half*)b.tex, N, C, 3);
+    scene_centre_kernel<<<1, 1024, 0, st>>>((const __half*)d->tri16(), d->center(), (__half*)b.pos, N, nr);
+    TRY(rfk_triangle_rope_freqs(b.pos, m.enc_rope_freqs, b.cos, b.sin, 1, Se, m.rope_num_freqs, hd, s));
     // normals: NeRF PE -> linear -> fp32 RMSNorm (render_session.cu:310-318)
-    rfk_half *vn_pe, *emb16; float *vn_n, *tex_n, *seq;
-    TRY(sc.get(&vn_pe, (size_t)N * vn_pe_dim));
-    TRY(sc.get(&emb16, (size_t)N * dim));
-    TRY(sc.get(&vn_n, (size_t)N * dim));
-    TRY(sc.get(&tex_n, (size_t)N * dim));
-    TRY(sc.get(&seq, (size_t)Se * dim));
-    TRY(rfk_nerf_pe_f32(vn, vn_pe, 1, N, 9, m.vn_pe_num_freqs, 0.0f, (float)(m.vn_pe_num_freqs - 1), 1, s));
-    TRY(rfk_linear(d->ctx, vn_pe, m.vn_proj_w, m.vn_proj_b, emb16, N, dim, vn_pe_dim, s));
-    TRY(rfk_cast_fp16_to_fp32(emb16, vn_n, (long long)N * dim, s));
-    TRY(rfk_rmsnorm_f32(vn_n, m.vn_enc_norm, vn_n, N, dim, kEpsFp16, s));
+    TRY(rfk_nerf_pe_f32(vn, b.vn_pe, 1, N, 9, m.vn_pe_num_freqs, 0.0f, (float)(m.vn_pe_num_freqs - 1), 1, s));
+    TRY(rfk_linear(d->ctx, b.vn_pe, m.vn_proj_w, m.vn_proj_b, b.emb16, N, dim, vn_pe_dim, s));
+    TRY(rfk_cast_fp16_to_fp32(b.emb16, b.vn_n, (long long)N * dim, s));
+    TRY(rfk_rmsnorm_f32(b.vn_n, m.vn_enc_norm, b.vn_n, N, dim, kEpsFp16, s));
     // texture: linear -> fp32 RMSNorm (render_session.cu:321-327)
-    TRY(rfk_linear(d->ctx, tex_buf, m.tex_enc_w, m.tex_enc_b, emb16, N, dim, C, s));
-    TRY(rfk_cast_fp16_to_fp32(emb16, tex_n, (long long)N * dim, s));
-    TRY(rfk_rmsnorm_f32(tex_n, m.tex_enc_norm, tex_n, N, dim, kEpsFp16, s));
+    TRY(rfk_linear(d->ctx, b.tex, m.tex_enc_w, m.tex_enc_b, b.emb16, N, dim, C, s));
+    TRY(rfk_cast_fp16_to_fp32(b.emb16, b.tex_n, (long long)N * dim, s));
+    TRY(rfk_rmsnorm_f32(b.tex_n, m.tex_enc_norm, b.tex_n, N, dim, kEpsFp16, s));
     // sequence = [register tokens | texture + normal + triangle token] in fp32 (render_session.cu:330-339)
-    TRY(rfk_cast_fp16_to_fp32(m.reg_tokens, seq, (long long)nr * dim, s));
-    add3_bc_kernel<<<blocks_for((long long)N * dim), 256, 0, st>>>(seq + (size_t)nr * dim, tex_n, vn_n,
+    TRY(rfk_cast_fp16_to_fp32(m.reg_tokens, b.seq, (long long)nr * dim, s));
+    add3_bc_kernel<<<blocks_for((long long)N * dim), 256, 0, st>>>(b.seq + (size_t)nr * dim, b.tex_n, b.vn_n,
                                                                    (const __half*)m.tri_token, (long long)N * dim, dim);
-    // encoder positions: world centroid for the register tokens, then the triangles (render_session.cu:91-97,342-350)
-    rfk_half *enc_pos, *enc_cos, *enc_sin;
-    TRY(sc.get(&enc_pos, (size_t)Se * 9));
-    TRY(sc.get(&enc_cos, (size_t)Se * hd));
-    TRY(sc.get(&enc_sin, (size_t)Se * hd));
-    std::vector<__half> h_reg((size_t)nr * 9);
-    for (int r = 0; r < nr; ++r)
-        for (int k = 0; k < 9; ++k) h_reg[(size_t)r * 9 + k] = __float2half(c[k % 3]);
-    TRY_CUDA(cudaMemcpyAsync(enc_pos, h_reg.data(), h_reg.size() * sizeof(__half), cudaMemcpyHostToDevice, st));
-    TRY_CUDA(cudaMemcpyAsync(enc_pos + (size_t)nr * 9, d->tri16(), (size_t)N * 9 * sizeof(rfk_half), cudaMemcpyDeviceToDevice, st));
-    TRY(rfk_triangle_rope_freqs(enc_pos, m.enc_rope_freqs, enc_cos, enc_sin, 1, Se,
-                                m.rope_num_freqs, hd, s));
-    TRY_CUDA(cudaStreamSynchronize(st));  // h_reg goes out of use
 
     // encoder (render_session.cu:356-371)
-    rfk_half *temp, *qkvb, *ffnb; float* score;
-    TRY(sc.get(&temp, (size_t)Se * dim));
-    TRY(sc.get(&qkvb, (size_t)Se * std::max(6 * dim, 2 * ffn)));
-    TRY(sc.get(&ffnb, (size_t)Se * std::max(dim, ffn)));
-    score = nullptr;
-    if (!(hd == 64 || hd == 128)) TRY(sc.get(&score, (size_t)nh * Se * Se_pad));
     const rfk_half* pending = nullptr;
     for (int i = 0; i < m.enc_layers; ++i) {
         const rfk_half* next = nullptr;
-        TRY(rfk_encoder_layer_forward_mixed(d->ctx, &m.enc[i], seq, pending, i + 1 < m.enc_layers ? &next : nullptr,
-                                            temp, qkvb, ffnb, score, 1, Se, dim, nh, ffn,
-                                            enc_cos, enc_sin, s));
+        TRY(rfk_encoder_layer_forward_mixed(d->ctx, &m.enc[i], b.seq, pending, i + 1 < m.enc_layers ? &next : nullptr,
+                                            b.temp, b.qkv, b.ffn, b.score, 1, Se, dim, nh, ffn, b.cos, b.sin, s));
         pending = next;
     }
     // context in fp16, then per decoder layer: kv-norm, K/V projections, padded head-major cache
     // (render_session.cu:377-416)
-    rfk_half *ctx16, *ctx_normed, *kv_proj;
-    TRY(sc.get(&ctx16, (size_t)Se * dim));
-    TRY(sc.get(&ctx_normed, (size_t)Se * dim));
-    TRY(sc.get(&kv_proj, (size_t)2 * Se * dim));
-    TRY(rfk_cast_fp32_to_fp16(seq, ctx16, (long long)Se * dim, s));
+    TRY(rfk_cast_fp32_to_fp16(b.seq, b.ctx16, (long long)Se * dim, s));
     for (int i = 0; i < m.dec_layers; ++i) {
-        TRY(rfk_rmsnorm(ctx16, m.dec[i].kv_norm_gamma, ctx_normed, Se, dim, kEpsFp16, s));
-        TRY(rfk_precompute_cross_kv(d->ctx, &m.dec[i].cross_attn, ctx_normed, d->kvK(i),
-                                    d->kvV(i), kv_proj, 1, Se, Se_pad, dim, dim, nh, s));
+        TRY(rfk_rmsnorm(b.ctx16, m.dec[i].kv_norm_gamma, b.ctx_normed, Se, dim, kEpsFp16, s));
+        TRY(rfk_precompute_cross_kv(d->ctx, &m.dec[i].cross_attn, b.ctx_normed, d->kvK(i),
+                                    d->kvV(i), b.kv_proj, 1, Se, Se_pad, dim, dim, nh, s));
     }
     TRY_CUDA(cudaStreamSynchronize(st));
     TRY_CUDA(cudaGetLastError());

@@ -1,0 +1,65 @@
+"""Scene encoding: the geometry kernels (fp16 copies, centre) at sizes around a thread's stride, and a session that encodes
+several scenes with its one block of work buffers. Oracle: fp16 casts and a double-precision mean on the host, exact - every
+partial sum of the fp16 vertices is exact in double precision."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(n, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    tri = ((torch.rand(n, 3, 3, device="cuda", generator=g) * 2 - 1) * scale).contiguous()
+    vn = torch.nn.functional.normalize(torch.randn(n, 3, 3, device="cuda", generator=g), dim=-1).contiguous()
+    return tri, vn, torch.rand(n, 13, device="cuda", generator=g).half().contiguous()
+
+
+def _session(n, heads=4, dim=256):
+    import renderformer_cuda_b200  # noqa: F401
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=2, dim=dim, num_heads=heads, ffn_hidden=2 * dim, enc_layers=1, dec_layers=1,
+                                 num_register_tokens=5)
+    return session.RenderSession(model, n, 64)
+
+
+def _geometry(s, n):
+    """(fp16 triangles, fp16 normals, fp32 centre): the last three pieces of the scene state, 256-byte aligned each."""
+    up = lambda v: (v + 255) // 256 * 256
+    raw = s.scene_state.cpu().numpy().view(np.uint8)
+    size = up(n * 18)
+    start = raw.size - 256 - 2 * size
+    f16 = lambda o: raw[o:o + n * 18].view(np.float16).reshape(n * 3, 3)
+    return f16(start), f16(start + size), raw[start + 2 * size:start + 2 * size + 12].view(np.float32)
+
+
+@pytest.mark.parametrize("n,scale", [(1, 1.0), (113, 1.0), (114, 300.0), (341, 1.0), (1365, 0.01), (5633, 20.0)])
+def test_geometry_of_the_scene_state(n, scale):
+    s = _session(n)
+    tri, vn, tex = _scene(n, n, scale)
+    s.encode_scene(tri, vn, tex)
+    t16, v16, centre = _geometry(s, n)
+    want = tri.half().cpu().numpy().reshape(n * 3, 3)
+    assert np.array_equal(t16.view(np.uint16), want.view(np.uint16))
+    assert np.array_equal(v16.view(np.uint16), vn.half().cpu().numpy().reshape(n * 3, 3).view(np.uint16))
+    assert np.array_equal(centre, (want.astype(np.float64).sum(0) / (3.0 * n)).astype(np.float32))
+    s.close()
+
+
+@pytest.mark.parametrize("heads", [4, 2, 8])
+def test_a_session_encodes_scene_after_scene(heads):
+    """64-, 128- and 32-wide heads (the last with a materialised score matrix among the work buffers)."""
+    n = 61
+    a, b = _session(n, heads), _session(n, heads)
+    first, second = _scene(n, 1), _scene(n, 2)
+    a.encode_scene(*first)
+    one = a.scene_state.clone()
+    a.encode_scene(*second)
+    assert not torch.equal(a.scene_state, one)
+    b.encode_scene(*second)
+    assert torch.equal(a.scene_state, b.scene_state)
+    a.encode_scene(*first)
+    assert torch.equal(a.scene_state, one)
+    kv = one[:2 * 72 * 256 * 2].view(torch.float16).view(2, heads, 72, 256 // heads)
+    assert torch.isfinite(kv).all() and (kv[:, :, 66:] == 0).all() and (kv[:, :, :66] != 0).any(-1).all()
+    a.close(); b.close()
