@@ -46,12 +46,17 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 #define RFK_TC_SLOW_PATH static __device__ __noinline__
 #endif
 RFK_TC_SLOW_PATH bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort) {
+    // The time limit counts from two readings taken apart, as signed differences: one reading of the 64-bit timer that is off
+    // must not end a wait.
     const uint64_t t0 = global_timer_ns();
+    uint64_t first = 0;
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((it & 63u) == 63u) {
             if (*abort) return false;
-            if (global_timer_ns() - t0 > kWaitLimitNs) break;
+            const uint64_t now = global_timer_ns();
+            if (first == 0) first = now;   // a second start, should t0 itself be off
+            if ((int64_t)(now - t0) > (int64_t)kWaitLimitNs && (int64_t)(now - first) > (int64_t)kWaitLimitNs) break;
         }
         __nanosleep(32);
     }

@@ -361,6 +361,7 @@ constexpr int kMaxStages = 6;
 
 struct __align__(8) Ctrl {
     uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], drain;
+    uint64_t started;          // one phase only: the products of the CTA's first K block are complete
     uint64_t res_full[4][4];   // residual epilogue: [epilogue warp][unit], completes when that unit's residual box has landed
     uint32_t tmem_base;
     int abort;
@@ -574,6 +575,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
         for (int a = 0; a < 2; ++a) { tc::mbar_init(&ctrl->acc_full[a], 1); tc::mbar_init(&ctrl->acc_empty[a], 8); }
         tc::mbar_init(&ctrl->drain, 1);
+        tc::mbar_init(&ctrl->started, 1);
         for (int w = 0; w < 4; ++w)
             for (int u = 0; u < 4; ++u) tc::mbar_init(&ctrl->res_full[w][u], 1);
         ctrl->abort = 0;
@@ -648,6 +650,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     for (int ks = 0; ks < BK / 16; ++ks)
                         umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb > 0) || (ks > 0));
                     umma_pair_commit(&ctrl->empty[s]);
+                    if (EPI == RFK_GEMM_EPI_RESIDUAL && it == 0) umma_pair_commit(&ctrl->started);
                 }
                 if (ok) umma_pair_commit(&ctrl->acc_full[acc]);
                 if (tl == 0) RFK_STAMP(3);       // all products of the first tile issued
@@ -672,8 +675,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int row0 = m0 + lane_grp * 32;
             if (lane == 0) {
                 // The residual boxes of the CTA's first tile are asked for only once the first K block has been consumed
-                // (first multicast commit): issued at kernel start they delay the first operand tiles by ~0.5 us.
-                if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->empty[0], 0, abort_flag);
+                // (a multicast commit): issued at kernel start they delay the first operand tiles by ~0.5 us. The barrier has one
+                // phase, so a warp that comes late cannot miss it; empty[0] goes on to other phases.
+                if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
                 epilogue_prefetch_residual<EPI>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
