@@ -325,61 +325,66 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     } else if (warp == 9 || warp == 10) {
         const int blk = warp - 9;
         const uint32_t tmem = tmem_cta + blk * 256, tmem_O = tmem + kSBufs * 64;
-        // ------------------------------------------------------------ issuer of O += P V (one thread)
+        // ------------------------------------------------------------ issuer of O += P V (the warp's elected lane)
+        // The whole warp runs the loop and one lane issues (elect_one): with a single thread's loop the issue of a tile's
+        // products, not the tensor pipe, paced the 128-wide heads (8 x 4096 x 5665: 96 -> 84 us, 1.13 PFLOP/s; with 64-wide
+        // heads, which the softmax warps pace, 142 -> 139 us).
         // tile j: score buffer j % kSBufs (its use number j / kSBufs gives the barrier phase), ring stage j % kStages
-        if (lane == 0) {
-            constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
-            // MN-major operand: the leading byte offset is the distance between its 64-column sub-tiles
-            const uint32_t v_lo = ((sKV + kKBytes) >> 4 & 0x3fffu) | ((HD == 64 ? 1u : (uint32_t)(C::kKSub >> 4)) << 16);
-            bool ok = true;
-            int buf = 0, buf_par = 0, st = 0;
-            for (int j = 0; ok && j < n_tiles; ++j) {
-                ok = tc::mbar_wait(&ctrl->p_full[blk][buf], buf_par, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after();
+        const bool leader = tc::elect_one();
+        constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
+        // MN-major operand: the leading byte offset is the distance between its 64-column sub-tiles
+        const uint32_t v_lo = ((sKV + kKBytes) >> 4 & 0x3fffu) | ((HD == 64 ? 1u : (uint32_t)(C::kKSub >> 4)) << 16);
+        bool ok = true;
+        int buf = 0, buf_par = 0, st = 0;
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            ok = tc::mbar_wait_warp(&ctrl->p_full[blk][buf], buf_par, abort_flag);
+            if (!ok) break;
+            tc::tc_fence_after();
+            if (leader) {
                 const uint32_t p_tmem = tmem + buf * 64, vt_lo = v_lo + st * (kStageBytes >> 4);
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks)  // P: 16 keys = 8 columns; V: 16 keys = 16 rows of 128 bytes
                     tc::umma_f16_ts_lo(tmem_O, p_tmem + ks * 8, vt_lo + ks * (2048 >> 4), idesc_pv, (j > 0) || (ks > 0));
                 tc::umma_commit(&ctrl->kv_empty[st]);  // K of this stage was consumed before its scores could be read
                 tc::umma_commit(&ctrl->pv_done[blk][buf]);
-                if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
-                if (++st == kStages) st = 0;
             }
-            if (*abort_flag) {  // giving up: let this thread's products finish before tensor memory is freed
-                tc::umma_commit(&ctrl->drain[blk]);
-                tc::mbar_wait_drain(&ctrl->drain[blk], 0);
-            }
+            if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
+            if (++st == kStages) st = 0;
+        }
+        if (leader && *abort_flag) {  // giving up: let this lane's products finish before tensor memory is freed
+            tc::umma_commit(&ctrl->drain[blk]);
+            tc::mbar_wait_drain(&ctrl->drain[blk], 0);
         }
         __syncwarp();
     } else if (warp == 11 || warp == 12) {
         const int blk = warp - 11;
         const uint32_t tmem = tmem_cta + blk * 256;
-        // ------------------------------------------------------------ issuer of S = Q K^T (one thread)
-        if (lane == 0) {
-            constexpr uint32_t idesc_qk = tc::umma_idesc_f16(BM, BN, 0);  // B = K tile, K-major
-            const uint32_t q_lo = tc::umma_desc_lo(sQ + blk * kQBytes), k_lo = tc::umma_desc_lo(sKV);
-            bool ok = tc::mbar_wait(&ctrl->q_full, 0, abort_flag);
-            int buf = 0, buf_par = 0, st = 0, st_par = 0;
-            for (int j = 0; ok && j < n_tiles; ++j) {
-                ok = tc::mbar_wait(&ctrl->kv_full[st], st_par, abort_flag);
-                // the buffer still holds P of tile j - kSBufs until that tile's P V is complete
-                if (ok && j >= kSBufs) ok = tc::mbar_wait(&ctrl->pv_done[blk][buf], buf_par ^ 1, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after();
+        // ------------------------------------------------------------ issuer of S = Q K^T (the warp's elected lane)
+        const bool leader = tc::elect_one();
+        constexpr uint32_t idesc_qk = tc::umma_idesc_f16(BM, BN, 0);  // B = K tile, K-major
+        const uint32_t q_lo = tc::umma_desc_lo(sQ + blk * kQBytes), k_lo = tc::umma_desc_lo(sKV);
+        bool ok = tc::mbar_wait_warp(&ctrl->q_full, 0, abort_flag);
+        int buf = 0, buf_par = 0, st = 0, st_par = 0;
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            ok = tc::mbar_wait_warp(&ctrl->kv_full[st], st_par, abort_flag);
+            // the buffer still holds P of tile j - kSBufs until that tile's P V is complete
+            if (ok && j >= kSBufs) ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][buf], buf_par ^ 1, abort_flag);
+            if (!ok) break;
+            tc::tc_fence_after();
+            if (leader) {
                 const uint32_t kt_lo = k_lo + st * (kStageBytes >> 4);
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks)  // 16 head-dim elements = 32 bytes along a row of a sub-tile
                     tc::umma_f16_lo(tmem + buf * 64, q_lo + (ks / 4) * (C::kQSub >> 4) + (ks % 4) * 2,
                                     kt_lo + (ks / 4) * (C::kKSub >> 4) + (ks % 4) * 2, idesc_qk, ks > 0);
                 tc::umma_commit(&ctrl->s_full[blk][buf]);
-                if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
-                if (++st == kStages) { st = 0; st_par ^= 1; }
             }
-            if (*abort_flag) {
-                tc::umma_commit(&ctrl->drain[kBlocks + blk]);
-                tc::mbar_wait_drain(&ctrl->drain[kBlocks + blk], 0);
-            }
+            if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
+            if (++st == kStages) { st = 0; st_par ^= 1; }
+        }
+        if (leader && *abort_flag) {
+            tc::umma_commit(&ctrl->drain[kBlocks + blk]);
+            tc::mbar_wait_drain(&ctrl->drain[kBlocks + blk], 0);
         }
         __syncwarp();
     }  // warps 13-15 have no role beyond handing their registers back together with warp 12

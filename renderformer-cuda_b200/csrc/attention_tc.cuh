@@ -100,6 +100,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     if ((threadIdx.x & 31) == 0) ok = mbar_wait_slow(bar, parity, abort);
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
+// One lane of a fully active warp, the same on every call. A role that runs its loop as a whole warp and issues under this
+// predicate keeps its addresses in uniform registers; inside `if (lane == 0)` each operand of an issued instruction is moved
+// there first.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // make generic-proxy writes to shared memory (st.shared, cp.async) visible to the tensor core's async proxy
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
