@@ -323,6 +323,222 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------
+// The same product on small tiles, one per CTA, for calls that do not fill the machine: a view of 256 tokens gives the pair
+// kernel below four tiles for its 74 pairs, and a 4096-wide K then runs 64 K blocks of 0.3 us one after the other. Here a
+// tile is 64 or 128 rows by 32 to 128 accumulator columns, so that there are many and each takes few operand bytes per K
+// block (one SM takes them at about 110 GB/s). K is not split: every output is summed over the K blocks in the same order
+// as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
+// must equal the views one by one).
+//   A stage is two K blocks: one wait, one announcement and one commit for eight products. And the issuing warp runs its loop
+//   as a whole, one elected lane issuing, so that descriptors and counters live in uniform registers. With one block per
+//   stage and a single thread's loop a K block took 0.30 us on every tile size, the cost of issuing and not of the operands;
+//   together the two took the 64 x 32 tile to 0.16 us.
+//   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
+//   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
+// The epilogue's threads store their own rows: a tile row is 32 to 256 bytes, one to eight whole sectors.
+namespace small {
+
+constexpr int kSub = 2;                  // K blocks per stage
+template <int BM_, int BN_> struct Cfg {
+    static constexpr int kBlockBytes = (BM_ + BN_) * BK * 2;      // operands of one K block
+    static constexpr int kStageBytes = kSub * kBlockBytes;
+    static constexpr int kStages = 192 * 1024 / kStageBytes;      // 8 to 3: a lone CTA waits for memory, so as deep as fits
+    static constexpr int kSmemBytes = kStages * kStageBytes + 256;
+    static_assert(kStages >= 2 && kStages <= 8 && kSmemBytes + 1024 <= 227 * 1024, "control block, shared memory of an SM");
+};
+
+struct __align__(8) Ctrl {
+    uint64_t full[8], empty[8], acc_full, drain;
+    uint32_t tmem_base;
+    int abort;
+};
+static_assert(sizeof(Ctrl) <= 256, "control block");
+
+template <int EPI, int BM_, int BN_>
+__global__ void __launch_bounds__(kThreads)
+gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
+                     const __grid_constant__ CUtensorMap map_w1, const Params p) {
+    constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
+    constexpr int kStages = Cfg<BM_, BN_>::kStages, kStage = Cfg<BM_, BN_>::kStageBytes, kBlock = Cfg<BM_, BN_>::kBlockBytes;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const uint32_t base = tc::smem_addr(smem_raw);
+    if (base & 1023u) {  // uniform over the CTA, nothing allocated yet
+        if (threadIdx.x == 0) atomicCAS(&g_gemm_tc_error, 0, kErrSmemAlign);
+        return;
+    }
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + kStages * kStage);
+    volatile int* abort_flag = &ctrl->abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int num_st = (p.K + kSub * BK - 1) / (kSub * BK);   // stages of K; a second block beyond K arrives as zeros
+    const int m0 = (blockIdx.x % p.tiles_m) * BM_, n0 = (blockIdx.x / p.tiles_m) * BN_OUT;
+
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
+        tc::mbar_init(&ctrl->acc_full, 1);
+        tc::mbar_init(&ctrl->drain, 1);
+        ctrl->abort = 0;
+        tc::fence_barrier_init();
+    }
+    if (warp == 0) {
+        tc::tmem_alloc(&ctrl->tmem_base, BN_);
+        tc::tmem_relinquish();
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem_cta = ctrl->tmem_base;
+    pdl_wait();      // set-up above is on-chip only; the operands are another kernel's output
+    pdl_trigger();
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ producer (one thread)
+        if (lane == 0) {
+            int it = 0;
+            for (; it < num_st; ++it) {
+                const int s = it % kStages;
+                if (it >= kStages && !tc::mbar_wait(&ctrl->empty[s], ((it / kStages) + 1) & 1, abort_flag)) break;
+                tc::mbar_arrive_expect_tx(&ctrl->full[s], kStage);
+#pragma unroll
+                for (int h = 0; h < kSub; ++h) {
+                    const uint32_t sA = base + s * kStage + h * kBlock, sW = sA + BM_ * BK * 2;
+                    const int x = (it * kSub + h) * BK;
+                    tma_load_2d(sA, &map_a, x, m0, &ctrl->full[s]);
+                    tma_load_2d(sW, &map_w0, x, n0, &ctrl->full[s]);
+                    if (kGate) tma_load_2d(sW + BN_OUT * BK * 2, &map_w1, x, n0, &ctrl->full[s]);
+                }
+            }
+            if (*abort_flag) {   // giving up: wait (bounded) for the last copy of each stage before the CTA exits
+                for (int s = 0; s < kStages && s < it; ++s) {
+                    const int last = ((it - 1 - s) / kStages) * kStages + s;
+                    tc::mbar_wait_drain(&ctrl->full[s], (last / kStages) & 1);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ issuer of the products (the warp's elected lane)
+        constexpr uint32_t idesc = tc::umma_idesc_f16(BM_, BN_, 0);  // A and B both K-major
+        const bool leader = tc::elect_one();
+        bool ok = true;
+        for (int it = 0; it < num_st; ++it) {
+            const int s = it % kStages;
+            ok = tc::mbar_wait_warp(&ctrl->full[s], (it / kStages) & 1, abort_flag);
+            if (!ok) break;
+            tc::tc_fence_after();
+            if (leader) {
+#pragma unroll
+                for (int h = 0; h < kSub; ++h) {
+                    const uint32_t a_lo = tc::umma_desc_lo(base + s * kStage + h * kBlock);
+                    const uint32_t b_lo = tc::umma_desc_lo(base + s * kStage + h * kBlock + BM_ * BK * 2);
+#pragma unroll
+                    for (int ks = 0; ks < BK / 16; ++ks)  // 16 halves = 32 bytes along a swizzled row
+                        tc::umma_f16_lo(tmem_cta, a_lo + ks * 2, b_lo + ks * 2, idesc, (it > 0) || (h > 0) || (ks > 0));
+                }
+                tc::umma_commit(&ctrl->empty[s]);
+            }
+        }
+        if (leader) {
+            if (ok) tc::umma_commit(&ctrl->acc_full);
+            if (*abort_flag) {  // giving up: let this lane's products finish before tensor memory is freed
+                tc::umma_commit(&ctrl->drain);
+                tc::mbar_wait_drain(&ctrl->drain, 0);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------ epilogue, warps 2-5
+        const int lane_grp = warp & 3;                        // a warp reaches tensor-memory lanes [32 * (warp % 4), +32)
+        const int row = m0 + (BM_ == 64 ? lane_grp * 16 + lane : lane_grp * 32 + lane);
+        const bool row_ok = row < p.M && (BM_ == 128 || lane < 16);
+        const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
+        __half* crow = p.C + (size_t)(row_ok ? row : 0) * p.ldc + n0;
+        constexpr int kChunk = BN_OUT < 32 ? BN_OUT : 32;     // output columns per step
+        uint4 res[EPI == RFK_GEMM_EPI_RESIDUAL ? BN_OUT / 8 : 1];
+        if (EPI == RFK_GEMM_EPI_RESIDUAL) {                   // the row's residual arrives while the products run
+            const __half* rrow = p.R + (size_t)(row_ok ? row : 0) * p.ldr + n0;
+#pragma unroll
+            for (int q = 0; q < BN_OUT / 8; ++q)
+                res[q] = (row_ok && n0 + q * 8 < p.N) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
+        }
+        if (tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag)) {
+            tc::tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < BN_OUT / kChunk; ++c) {
+                if (n0 + c * kChunk >= p.N) break;            // uniform over the CTA: the tile's tail lies beyond N
+                uint32_t v[32], o[kChunk / 2];
+                tc::tmem_ld32(t_acc + c * 32, v);
+                if (kGate) {
+                    uint32_t u[32];
+                    if (kChunk == 32) {
+                        tc::tmem_ld32(t_acc + BN_OUT + c * 32, u);
+                        tc::tc_wait_ld(v);
+                        tc::tc_wait_ld(u);
+                    } else {                                  // 16 gate and 16 up columns in one load
+                        tc::tc_wait_ld(v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) u[i] = v[16 + i];
+                    }
+#pragma unroll
+                    for (int i = 0; i < kChunk; i += 2) {
+                        const float g0 = __uint_as_float(v[i]), g1 = __uint_as_float(v[i + 1]);
+                        // silu(g) * u = g * u / (1 + 2^(-g log2 e))
+                        const float s0 = g0 * fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * g0));
+                        const float s1 = g1 * fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * g1));
+                        o[i >> 1] = pack_half2(s0 * __uint_as_float(u[i]), s1 * __uint_as_float(u[i + 1]));
+                    }
+                } else {
+                    tc::tc_wait_ld(v);
+                    if (p.bias) {
+#pragma unroll
+                        for (int i = 0; i < kChunk; i += 2) {
+                            const int col = n0 + c * 32 + i;
+                            if (col < p.N) {
+                                const float2 b = unpack_half2(__ldg(reinterpret_cast<const uint32_t*>(p.bias + col)));
+                                // the unfused path rounds the product to fp16 before the bias is added (linear.cu:15-25)
+                                v[i] = __float_as_uint(round_half(__uint_as_float(v[i])) + b.x);
+                                v[i + 1] = __float_as_uint(round_half(__uint_as_float(v[i + 1])) + b.y);
+                            }
+                        }
+                    }
+                    if (EPI == RFK_GEMM_EPI_RESIDUAL) {
+#pragma unroll
+                        for (int i = 0; i < kChunk / 2; ++i) {
+                            const uint4 w = res[EPI == RFK_GEMM_EPI_RESIDUAL ? c * 4 + i / 4 : 0];
+                            const float2 rr = unpack_half2(i % 4 == 0 ? w.x : i % 4 == 1 ? w.y : i % 4 == 2 ? w.z : w.w);
+                            o[i] = pack_half2(__uint_as_float(v[2 * i]) + rr.x, __uint_as_float(v[2 * i + 1]) + rr.y);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < kChunk / 2; ++i) o[i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                    }
+                }
+                if (row_ok) {
+#pragma unroll
+                    for (int q = 0; q < kChunk / 8; ++q) {
+                        const int col = n0 + c * kChunk + q * 8;
+                        if (col < p.N)
+                            *reinterpret_cast<uint4*>(crow + c * kChunk + q * 8) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+
+    // ---- teardown: every path (normal or aborted) arrives here with no divergence inside a warp
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem_cta, BN_);
+    }
+    if (tid == 0 && ctrl->abort) atomicCAS(&g_gemm_tc_error, 0, kErrTimeout);
+}
+
+}  // namespace small
+
+// ------------------------------------------------------------------------------------------------
 // The same product on CTA pairs: a cluster of two CTAs (two SMs of one TPC) owns a tile of 256 rows x 256
 // accumulator columns and one thread of the pair's first CTA issues tcgen05.mma.cta_group::2 (M = 256):
 // each CTA stages only ITS 128 rows of A and ITS half of the weight tile (128 of the 256 accumulator
@@ -845,11 +1061,74 @@ bool make_map_heads(CUtensorMap* m, const void* base, int seq, int heads, int hd
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// path 0 / 2: CTA pairs, the single-CTA kernel if pairs are unavailable; path 3: the single-CTA kernel
+int sm_count(int dev) {
+    static std::atomic<int> count[64];
+    int n = count[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); return 0; }
+        count[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// ---- small tiles: their launch, and the rule that chooses them
+template <int EPI, int BM_, int BN_>
+int launch_gemm_small(const void* A, long long lda, const void* W, const void* W_up, long long ldw, tcgemm::Params p, int dev,
+                      cudaStream_t st) {
+    constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
+    constexpr int smem = tcgemm::small::Cfg<BM_, BN_>::kSmemBytes;
+    CUtensorMap ma, mw0, mw1;
+    if (!make_map_2d(&ma, A, p.M, p.K, lda, BM_) || !make_map_2d(&mw0, W, p.N, p.K, ldw, BN_OUT)) return RFK_EUNSUPPORTED;
+    if (!kGate) mw1 = mw0;
+    else if (!make_map_2d(&mw1, W_up, p.N, p.K, ldw, BN_OUT)) return RFK_EUNSUPPORTED;
+    static std::atomic<bool> configured[64];
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        cudaError_t e = cudaFuncSetAttribute(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    p.tiles_m = (p.M + BM_ - 1) / BM_;
+    p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
+    launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, dim3((unsigned)(p.tiles_m * p.tiles_n)), dim3(tcgemm::kThreads),
+               smem, st, ma, mw0, mw1, p);
+    return launch_status();
+}
+
+// The smallest tile whose tiles all run at once, one per SM; 0: none of them, the pair kernel. Smaller tiles take fewer
+// operand bytes per K block and CTA, and a second round costs as much as the first. Measured on both sides of the line
+// (us, small tile / pair kernel, weights from HBM): 256 x 1024 x 4096 10.9 / 24.5 (64 x 32), 1024 x 1024 x 1024 5.5 / 10.5
+// (128 x 64), 2304 x 1024 x 4096 18.8 / 24.6 (128 x 128, 144 tiles); 3136 x 1024 x 4096 35.3 / 26.3 (200 tiles),
+// 576 x 8192 x 1024 21.0 / 15.4 (320 tiles).
+int small_tile(int M, int acc_cols, int sms) {
+    constexpr int kTiles[4][2] = {{64, 32}, {64, 64}, {128, 64}, {128, 128}};   // rows, accumulator columns
+    for (int i = 0; i < 4; ++i)
+        if ((long long)ceil_div(M, kTiles[i][0]) * ceil_div(acc_cols, kTiles[i][1]) <= sms) return i + 1;
+    return 0;
+}
+
+// path 0 / 2: small tiles or CTA pairs, the single-CTA kernel if pairs are unavailable; path 3: the single-CTA kernel
 template <int EPI>
-int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, const tcgemm::Params& p, int dev,
+int launch_gemm(const void* A, long long lda, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev,
                 cudaStream_t st) {
-    if (g_gemm_path.load(std::memory_order_relaxed) != 3) {
+    constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    const int path = g_gemm_path.load(std::memory_order_relaxed);
+    if (path != 3) {
+        int rc = RFK_EUNSUPPORTED;
+        switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
+            case 1: rc = launch_gemm_small<EPI, 64, 32>(A, lda, W, W_up, ldw, p, dev, st); break;
+            case 2: rc = launch_gemm_small<EPI, 64, 64>(A, lda, W, W_up, ldw, p, dev, st); break;
+            case 3: rc = launch_gemm_small<EPI, 128, 64>(A, lda, W, W_up, ldw, p, dev, st); break;
+            case 4: rc = launch_gemm_small<EPI, 128, 128>(A, lda, W, W_up, ldw, p, dev, st); break;
+        }
+        if (rc != RFK_EUNSUPPORTED) return rc;
+    }
+    CUtensorMap ma, mw0, mw1;
+    if (!make_map_2d(&ma, A, p.M, p.K, lda) || !make_map_2d(&mw0, W, p.N, p.K, ldw) ||
+        !make_map_2d(&mw1, kGate ? W_up : W, p.N, p.K, ldw))
+        return RFK_EUNSUPPORTED;
+    if (path != 3) {
         const int rc = launch_gemm_pair<EPI>(ma, mw0, mw1, p, dev, st);
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
@@ -881,11 +1160,7 @@ extern "C" int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W,
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
-    CUtensorMap ma, mw0, mw1;
     const bool swiglu = epilogue == RFK_GEMM_EPI_SWIGLU;
-    if (!make_map_2d(&ma, A, M, K, lda) || !make_map_2d(&mw0, W, N, K, ldw) ||
-        !make_map_2d(&mw1, swiglu ? W_up : W, N, K, ldw))
-        return RFK_EUNSUPPORTED;
     tcgemm::Params p{};
     p.C = (__half*)C; p.ldc = ldc; p.R = (const __half*)R; p.ldr = ldr; p.bias = (const __half*)bias;
     p.M = M; p.N = N; p.K = K;
@@ -893,9 +1168,9 @@ extern "C" int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W,
     p.tiles_n = (N + (swiglu ? 128 : 256) - 1) / (swiglu ? 128 : 256);
     cudaStream_t st = as_stream(stream);
     switch (epilogue) {
-        case RFK_GEMM_EPI_NONE: return launch_gemm<RFK_GEMM_EPI_NONE>(ma, mw0, mw1, p, dev, st);
-        case RFK_GEMM_EPI_RESIDUAL: return launch_gemm<RFK_GEMM_EPI_RESIDUAL>(ma, mw0, mw1, p, dev, st);
-        default: return launch_gemm<RFK_GEMM_EPI_SWIGLU>(ma, mw0, mw1, p, dev, st);
+        case RFK_GEMM_EPI_NONE: return launch_gemm<RFK_GEMM_EPI_NONE>(A, lda, W, W_up, ldw, p, dev, st);
+        case RFK_GEMM_EPI_RESIDUAL: return launch_gemm<RFK_GEMM_EPI_RESIDUAL>(A, lda, W, W_up, ldw, p, dev, st);
+        default: return launch_gemm<RFK_GEMM_EPI_SWIGLU>(A, lda, W, W_up, ldw, p, dev, st);
     }
 }
 

@@ -1,0 +1,67 @@
+"""Small output tiles of the projection kernel (64 x 32 to 128 x 128, one per CTA) at the edges of tiles, stages and of the
+rule that chooses them. Oracle: the single-CTA kernel on the same operands, bit for bit - the K blocks are added in the
+same order on every tile - and torch fp32 for the sizes themselves (fp16 operands, fp32 sums, one rounding: 2^-11 relative,
+plus the fp32 sum of at most 4096 products of magnitude 1 / sqrt(K))."""
+import pytest
+import torch
+
+import renderformer_cuda_b200 as pkg
+
+pytestmark = pytest.mark.gpu
+ops = pkg.ops
+
+
+@pytest.fixture(autouse=True)
+def _paths():
+    ops.gemm_error(clear=True)
+    yield
+    ops.gemm_set_path(0)
+    torch.cuda.synchronize()
+    assert ops.gemm_error(clear=True) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 8), (63, 40, 64), (64, 32, 128), (65, 33 * 8, 136), (129, 1024, 200), (256, 1024, 1024), (256, 1024, 4096),
+    (576, 1024, 1024), (577, 1000, 1096), (1024, 1024, 1024), (1025, 1032, 328), (1600, 1024, 1024), (2304, 1024, 264),
+    (2368, 1024, 64), (2369, 1024, 64)])
+@pytest.mark.parametrize("epilogue", ["none", "bias", "residual", "in_place", "swiglu"])
+def test_same_bits_as_the_large_tiles(M, N, K, epilogue):
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    a, w = rnd(M, K).half(), (rnd(N, K) * K ** -0.5).half()
+    kw = {}
+    if epilogue == "bias":
+        kw["bias"] = rnd(N).half()
+    if epilogue == "swiglu":
+        kw["w_up"] = (rnd(N, K) * K ** -0.5).half()
+    r = rnd(M, N).half()
+    got = []
+    for path in (0, 3):
+        ops.gemm_set_path(path)
+        c = r.clone() if epilogue == "in_place" else torch.full((M, N), 7.0, device="cuda", dtype=torch.float16)
+        if epilogue in ("residual", "in_place"):
+            kw["residual"] = c if epilogue == "in_place" else r
+        ops.gemm_f16(a, w, c, M, N, K, **kw)
+        got.append(c)
+    assert torch.equal(got[0], got[1])
+    want = a.float() @ w.float().t()
+    if epilogue == "bias":
+        want = want.half().float() + kw["bias"].float()
+    if epilogue in ("residual", "in_place"):
+        want = want + r.float()
+    if epilogue == "swiglu":
+        want = torch.nn.functional.silu(want) * (a.float() @ kw["w_up"].float().t())
+    assert ((got[0].float() - want).abs() <= 2e-3 + 2e-3 * want.abs()).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 48, 72), (300, 96, 256)])
+def test_pitches_larger_than_the_rows(M, N, K):
+    """Only the output's own columns are written, operands of a wider matrix are read in place."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    big_a = torch.randn(M, K + 24, device="cuda", generator=g).half()
+    big_w = torch.randn(N, K + 8, device="cuda", generator=g).half()
+    out = torch.full((M, N + 16), 7.0, device="cuda", dtype=torch.float16)
+    ops.gemm_f16(big_a, big_w, out, M, N, K, lda=K + 24, ldw=K + 8, ldc=N + 16)
+    want = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    ops.gemm_f16(big_a[:, :K].contiguous(), big_w[:, :K].contiguous(), want, M, N, K)
+    assert torch.equal(out[:, :N], want) and (out[:, N:] == 7.0).all()
