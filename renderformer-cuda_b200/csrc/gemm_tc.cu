@@ -78,6 +78,7 @@ struct Params {
     int M, N, K;                        // N = output columns
     int tiles_m, tiles_n;
     float* row_ss;                      // kEpiHeads: [parts][M][tiles per part] partial sums of squares, or null
+    long long part_stride;              // kEpiHeads on small tiles, which store without a tensor map: halves between parts
     int seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
 };
 
@@ -322,6 +323,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (tid == 0 && ctrl->abort) atomicCAS(&g_gemm_tc_error, 0, kErrTimeout);
 }
 
+// ---- clusters
+namespace pair {
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// shared::cluster address of the location `smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+}  // namespace pair
+
 // ------------------------------------------------------------------------------------------------
 // The same product on small tiles, one per CTA, for calls that do not fill the machine: a view of 256 tokens gives the pair
 // kernel below four tiles for its 74 pairs, and a 4096-wide K then runs 64 K blocks of 0.3 us one after the other. Here a
@@ -371,7 +390,12 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     volatile int* abort_flag = &ctrl->abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int num_st = (p.K + kSub * BK - 1) / (kSub * BK);   // stages of K; a second block beyond K arrives as zeros
-    const int m0 = (blockIdx.x % p.tiles_m) * BM_, n0 = (blockIdx.x / p.tiles_m) * BN_OUT;
+    // rows fastest, so that the tiles running together share weights; the heads form runs columns fastest, because the tiles
+    // of 256 columns are one cluster
+    const int m0 = (EPI == kEpiHeads ? blockIdx.x / p.tiles_n : blockIdx.x % p.tiles_m) * BM_;
+    const int n0 = (EPI == kEpiHeads ? blockIdx.x % p.tiles_n : blockIdx.x / p.tiles_m) * BN_OUT;
+    const bool want_ss = EPI == kEpiHeads && p.row_ss && ((p.ss_mask >> (n0 / (p.units * 64))) & 1);   // uniform over a cluster
+    bool acc_ok = false;
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
@@ -461,7 +485,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             for (int q = 0; q < BN_OUT / 8; ++q)
                 res[q] = (row_ok && n0 + q * 8 < p.N) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
         }
-        if (tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag)) {
+        acc_ok = tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag);
+        if (EPI != kEpiHeads && acc_ok) {
             tc::tc_fence_after();
 #pragma unroll
             for (int c = 0; c < BN_OUT / kChunk; ++c) {
@@ -524,6 +549,67 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
         }
         __syncwarp();
+    }
+
+    if (EPI == kEpiHeads) {
+        // ------------------------------------------------------------ epilogue of the head-split form
+        // [part][group][head][seq][hd] by plain stores. The row statistic has the bits of the pair kernel's: one thread adds
+        // a row's 256 squares in column order. So the cluster's tiles are gathered in its first CTA's ring, which is idle
+        // once every CTA has its accumulator (first barrier), and summed there (second barrier).
+        constexpr int kPitch = 512 + 16;                      // bytes per gathered row; the odd 16 bytes spread the banks
+        static_assert(BM_ * kPitch <= kStages * kStage, "the gathered rows lie in the ring");
+        const int lane_grp = warp & 3;
+        const int local = BM_ == 64 ? lane_grp * 16 + lane : lane_grp * 32 + lane, row = m0 + local;
+        const bool mine = warp >= 2 && (BM_ == 128 || lane < 16), row_ok = mine && row < p.M;
+        if (want_ss) pair::cluster_sync();
+        if (warp >= 2 && acc_ok) {
+            tc::tc_fence_after();
+            const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
+            const int hd = p.head_units * 64, heads = p.units / p.head_units;
+            const size_t rows_off = ((size_t)(row / p.seq) * heads * p.seq + row % p.seq) * hd;
+            const uint32_t gather = pair::map_to_cta(base, 0) + local * kPitch + (n0 % 256) * 2;
+#pragma unroll
+            for (int c = 0; c < BN_ / 32; ++c) {
+                uint32_t v[32];
+                tc::tmem_ld32(t_acc + c * 32, v);
+                tc::tc_wait_ld(v);
+                const int g = (n0 + c * 32) / 64, u = g % p.units;   // 64-column unit over all parts, and within its part
+                __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + rows_off + (size_t)(u / p.head_units) * p.seq * hd +
+                              (u % p.head_units) * 64 + (c & 1) * 32;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[i] = pack_half2(__uint_as_float(v[8 * q + 2 * i]), __uint_as_float(v[8 * q + 2 * i + 1]));
+                    if (row_ok) *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+                    if (want_ss && mine)
+                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(gather + c * 64 + q * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                }
+            }
+        }
+        if (want_ss) {
+            __syncwarp();
+            pair::cluster_sync();
+            if (pair::cluster_rank() == 0 && row_ok) {
+                const uint4* src = reinterpret_cast<const uint4*>(smem_raw + local * kPitch);
+                float ss = 0.0f;
+#pragma unroll 8
+                for (int q = 0; q < 32; ++q) {
+                    const uint4 w = src[q];
+                    const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 r2 = unpack_half2(x[i]);
+                        ss = fmaf(r2.x, r2.x, ss);
+                        ss = fmaf(r2.y, r2.y, ss);
+                    }
+                }
+                const int dim = p.units * 64, part = n0 / dim;
+                p.row_ss[((size_t)part * p.M + row) * (dim / 256) + (n0 % dim) / 256] = ss;
+            }
+            __syncwarp();
+        }
     }
 
     // ---- teardown: every path (normal or aborted) arrives here with no divergence inside a warp
@@ -597,20 +683,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 // waits until at most N of this thread's committed store groups still READ their shared-memory source
 template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// shared::cluster address of the location `smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
@@ -1091,8 +1163,21 @@ int launch_gemm_small(const void* A, long long lda, const void* W, const void* W
     }
     p.tiles_m = (p.M + BM_ - 1) / BM_;
     p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
-    launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, dim3((unsigned)(p.tiles_m * p.tiles_n)), dim3(tcgemm::kThreads),
-               smem, st, ma, mw0, mw1, p);
+    const dim3 grid((unsigned)(p.tiles_m * p.tiles_n));
+    if (EPI != tcgemm::kEpiHeads) {
+        launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, grid, dim3(tcgemm::kThreads), smem, st, ma, mw0, mw1, p);
+        return launch_status();
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 256 / BN_; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid; cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, ma, mw0, mw1, p);
+    if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
 
@@ -1195,15 +1280,27 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    tcgemm::Params p{};
+    p.C = (__half*)out; p.ldc = N; p.M = M; p.N = N; p.K = K;
+    p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
+    p.part_stride = part_stride;
+    {
+        // The rule of the other epilogues over tiles of at least 64 columns; a cluster of four needs its SMs within one GPC,
+        // which leaves about an eighth of them over.
+        const int sms = sm_count(dev), tile = small_tile(M, N, sms - sms / 8);
+        int rc = RFK_EUNSUPPORTED;
+        cudaStream_t st = as_stream(stream);
+        if (tile == 1 || tile == 2) rc = launch_gemm_small<tcgemm::kEpiHeads, 64, 64>(A, lda, W, nullptr, ldw, p, dev, st);
+        if (tile == 3) rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 64>(A, lda, W, nullptr, ldw, p, dev, st);
+        if (tile == 4) rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 128>(A, lda, W, nullptr, ldw, p, dev, st);
+        if (rc != RFK_EUNSUPPORTED) return rc;
+    }
     CUtensorMap ma, mw, mh;
     if (!make_map_2d(&ma, A, M, K, lda) || !make_map_2d(&mw, W, N, K, ldw) ||
         !make_map_heads(&mh, out, seq_len, num_heads, head_dim, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
         return RFK_EUNSUPPORTED;
-    tcgemm::Params p{};
-    p.C = (__half*)out; p.ldc = N; p.M = M; p.N = N; p.K = K;
     p.tiles_m = (M + tcgemm::BM - 1) / tcgemm::BM;
     p.tiles_n = N / 256;
-    p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
     return launch_gemm_pair<tcgemm::kEpiHeads>(ma, mw, mw, p, dev, as_stream(stream), &mh);
 }
 

@@ -65,3 +65,24 @@ def test_pitches_larger_than_the_rows(M, N, K):
     want = torch.empty(M, N, device="cuda", dtype=torch.float16)
     ops.gemm_f16(big_a[:, :K].contiguous(), big_w[:, :K].contiguous(), want, M, N, K)
     assert torch.equal(out[:, :N], want) and (out[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M,seq,heads,parts,K,mask", [
+    (32, 32, 4, 1, 72, 1), (64, 64, 16, 3, 1024, 3), (96, 32, 8, 3, 200, 2), (256, 256, 16, 1, 1024, 1),
+    (256, 64, 16, 3, 1024, 3), (576, 64, 16, 3, 1024, 3), (960, 320, 4, 1, 136, 1), (1600, 1600, 16, 1, 1024, 1)])
+def test_head_split_form_has_the_bits_of_the_pair_kernel(M, seq, heads, parts, K, mask):
+    """The same rows as the head of a call that is large enough for the pair kernel: values and row statistics."""
+    dim = heads * 64
+    N = parts * dim
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    groups = -(-9600 // seq)
+    a = torch.randn(groups * seq, K, device="cuda", generator=g).half()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).half()
+    got = []
+    for rows in (M, groups * seq):
+        out = torch.full((parts, rows * dim), 7.0, device="cuda", dtype=torch.float16)
+        ss = torch.full((parts, rows, dim // 256), -1.0, device="cuda", dtype=torch.float32)
+        ops.gemm_f16_heads(a[:rows].contiguous(), w, out, ss, mask, rows, N, K, seq, heads, part_stride=rows * dim)
+        got.append((out[:, :M * dim], ss[:, :M]))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert all(bool((got[0][1][p] >= 0).all()) == bool(mask >> p & 1) for p in range(parts))
