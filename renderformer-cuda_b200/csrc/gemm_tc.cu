@@ -79,7 +79,7 @@ struct Params {
     int tiles_m, tiles_n;
     float* row_ss;                      // kEpiHeads: [parts][M][tiles per part] partial sums of squares, or null
     long long part_stride;              // kEpiHeads on small tiles, which store without a tensor map: halves between parts
-    int seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
+    int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
 };
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
@@ -566,7 +566,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             tc::tc_fence_after();
             const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
             const int hd = p.head_units * 64, heads = p.units / p.head_units;
-            const size_t rows_off = ((size_t)(row / p.seq) * heads * p.seq + row % p.seq) * hd;
+            const size_t rows_off = ((size_t)(row / p.seq) * heads * p.out_seq + row % p.seq) * hd;
             const uint32_t gather = pair::map_to_cta(base, 0) + local * kPitch + (n0 % 256) * 2;
 #pragma unroll
             for (int c = 0; c < BN_ / 32; ++c) {
@@ -574,7 +574,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 tc::tmem_ld32(t_acc + c * 32, v);
                 tc::tc_wait_ld(v);
                 const int g = (n0 + c * 32) / 64, u = g % p.units;   // 64-column unit over all parts, and within its part
-                __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + rows_off + (size_t)(u / p.head_units) * p.seq * hd +
+                __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + rows_off + (size_t)(u / p.head_units) * p.out_seq * hd +
                               (u % p.head_units) * 64 + (c & 1) * 32;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -1119,13 +1119,13 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtens
 }
 
 // rank-5 map of a head-split output: [part][group][head][seq][hd] halves, boxes of 32 rows x 64 columns
-bool make_map_heads(CUtensorMap* m, const void* base, int seq, int heads, int hd, long long groups, int parts,
+bool make_map_heads(CUtensorMap* m, const void* base, int seq, int out_seq, int heads, int hd, long long groups, int parts,
                     long long part_stride) {
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return false;
     const cuuint64_t row = (cuuint64_t)hd * 2;
     const cuuint64_t dims[5] = {(cuuint64_t)hd, (cuuint64_t)seq, (cuuint64_t)heads, (cuuint64_t)groups, (cuuint64_t)parts};
-    const cuuint64_t strides[4] = {row, (cuuint64_t)seq * row, (cuuint64_t)heads * seq * row, (cuuint64_t)part_stride * 2};
+    const cuuint64_t strides[4] = {row, (cuuint64_t)out_seq * row, (cuuint64_t)heads * out_seq * row, (cuuint64_t)part_stride * 2};
     const cuuint32_t box[5] = {64, 32, 1, 1, 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
@@ -1260,8 +1260,8 @@ extern "C" int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W,
 }
 
 int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out, long long part_stride,
-                    float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int num_heads, int head_dim,
-                    rfk_stream_t stream) {
+                    float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int out_seq, int num_heads,
+                    int head_dim, rfk_stream_t stream) {
     if (!A || !W || !out || M < 0 || N <= 0 || K <= 0 || seq_len <= 0 || num_heads <= 0 || lda < K || ldw < K) return RFK_EINVAL;
     if (head_dim != 64 && head_dim != 128) return RFK_EUNSUPPORTED;
     const int dim = num_heads * head_dim;
@@ -1272,7 +1272,8 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     const int path = g_gemm_path.load(std::memory_order_relaxed);
     if (path == 1 || path == 3) return RFK_EUNSUPPORTED;   // pair kernel only
     // a 256-column tile must lie inside one part, a 32-row store box inside one group
-    if (dim % 256 != 0 || seq_len % 32 != 0 || M % seq_len != 0) return RFK_EUNSUPPORTED;
+    if (dim % 256 != 0 || M % seq_len != 0) return RFK_EUNSUPPORTED;
+    if (out_seq < seq_len || (M != seq_len && (seq_len % 32 != 0 || out_seq != seq_len))) return RFK_EUNSUPPORTED;
     if ((lda | ldw | part_stride) % 8 != 0 || K % 8 != 0 || !aligned16(A) || !aligned16(W) || !aligned16(out) ||
         (row_ss && !aligned16(row_ss)))
         return RFK_EUNSUPPORTED;
@@ -1283,7 +1284,7 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     tcgemm::Params p{};
     p.C = (__half*)out; p.ldc = N; p.M = M; p.N = N; p.K = K;
     p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
-    p.part_stride = part_stride;
+    p.part_stride = part_stride; p.out_seq = out_seq;
     {
         // The rule of the other epilogues over tiles of at least 64 columns; a cluster of four needs its SMs within one GPC,
         // which leaves about an eighth of them over.
@@ -1297,7 +1298,7 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     }
     CUtensorMap ma, mw, mh;
     if (!make_map_2d(&ma, A, M, K, lda) || !make_map_2d(&mw, W, N, K, ldw) ||
-        !make_map_heads(&mh, out, seq_len, num_heads, head_dim, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
+        !make_map_heads(&mh, out, seq_len, out_seq, num_heads, head_dim, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
         return RFK_EUNSUPPORTED;
     p.tiles_m = (M + tcgemm::BM - 1) / tcgemm::BM;
     p.tiles_n = N / 256;
@@ -1307,7 +1308,9 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
 extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out,
                                   long long part_stride, float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len,
                                   int num_heads, rfk_stream_t stream) {
-    return gemm_heads(A, lda, W, ldw, out, part_stride, row_ss, ss_parts_mask, M, N, K, seq_len, num_heads, 64, stream);
+    const int out_seq = seq_len % 32 == 0 ? seq_len : 0;   // 0: refused, as the header says
+    return gemm_heads(A, lda, W, ldw, out, part_stride, row_ss, ss_parts_mask, M, N, K, seq_len, out_seq, num_heads, 64,
+                      stream);
 }
 
 extern "C" int rfk_gemm_pair_clusters(void) {

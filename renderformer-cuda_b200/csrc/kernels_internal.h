@@ -5,10 +5,11 @@
 
 namespace rfk {
 
-// rfk_gemm_f16_heads for heads of 64 or 128: out is [part][group][head][seq][head_dim]
+// rfk_gemm_f16_heads for heads of 64 or 128: out is [part][group][head][out_seq][head_dim], of which the first seq_len rows of
+// each head are written. out_seq other than seq_len, and a seq_len that is not a multiple of 32, need one group (M == seq_len).
 int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out, long long part_stride,
-               float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int num_heads, int head_dim,
-               rfk_stream_t stream);
+               float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int out_seq, int num_heads,
+               int head_dim, rfk_stream_t stream);
 
 // rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,

@@ -268,7 +268,6 @@ extern "C" int rfk_precompute_cross_kv(rfk_ctx* ctx, const rfk_cross_attn_weight
     rfk_half* Kp = proj_buf;
     rfk_half* Vp = proj_buf + (size_t)Mk * dim;
     TRY(rfk_linear(ctx, ctx_normed, w->k_proj_w, w->k_proj_b, Kp, Mk, dim, kv_dim, stream));
-    TRY(rfk_linear(ctx, ctx_normed, w->v_proj_w, w->v_proj_b, Vp, Mk, dim, kv_dim, stream));
     if (Sk_pad != Sk) {
         // only the rows behind the last key of each head; every other element is written below
         const size_t pitch = (size_t)Sk_pad * hd * 2, width = (size_t)(Sk_pad - Sk) * hd * 2, heads = (size_t)B * num_heads;
@@ -282,6 +281,14 @@ extern "C" int rfk_precompute_cross_kv(rfk_ctx* ctx, const rfk_cross_attn_weight
     // K and V cannot share a launch: they live in two separate [Mk, dim] projections
     TRY(project_epilogue(Kp, dim, 1, g, o, no_rope, nullptr, nullptr, B, Sk, num_heads, hd, Sk_pad,
                          nullptr, stream));
+    // V has no norm: its projection is stored head-split by the GEMM when the shape allows (one batch element, no bias); a
+    // transposing pass less per layer (scene of 300 triangles 983 -> 965 us, of 1500 triangles 1650 -> 1628 us)
+    int rc = RFK_EUNSUPPORTED;
+    if (B == 1 && !w->v_proj_b && (hd == 64 || hd == 128))
+        rc = rfk::gemm_heads(ctx_normed, kv_dim, w->v_proj_w, kv_dim, V_out, 0, nullptr, 0, Mk, dim, kv_dim, Sk, Sk_pad, num_heads, hd,
+                             stream);
+    if (rc != RFK_EUNSUPPORTED) return rc;
+    TRY(rfk_linear(ctx, ctx_normed, w->v_proj_w, w->v_proj_b, Vp, Mk, dim, kv_dim, stream));
     g[0] = nullptr; o[0] = V_out;
     return project_epilogue(Vp, dim, 1, g, o, no_rope, nullptr, nullptr, B, Sk, num_heads, hd, Sk_pad,
                             nullptr, stream);
@@ -319,7 +326,9 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
                           (reinterpret_cast<uintptr_t>(w->q_norm_gamma) & 15u) == 0;
     if (k_prescaled && !deferred) return RFK_EUNSUPPORTED;  // prescaled keys only make sense with the deferred norm
     if (deferred) {
-        int rc = rfk::gemm_heads(q_in, q_dim, w->q_proj_w, q_dim, Q_bhsd, 0, norm_ss, 1, Mq, dim, q_dim, Sq, num_heads, hd, stream);
+        int rc = RFK_EUNSUPPORTED;
+        if (Sq % 32 == 0)
+            rc = rfk::gemm_heads(q_in, q_dim, w->q_proj_w, q_dim, Q_bhsd, 0, norm_ss, 1, Mq, dim, q_dim, Sq, Sq, num_heads, hd, stream);
         if (rc == RFK_OK) {
             const rfk_half* K_use = K_cached;
             if (!k_prescaled) {
@@ -391,7 +400,7 @@ static int swin_core(rfk_ctx* ctx, const rfk_mha_weights* w, rfk_half* window_bu
     if (norm_ss && fused && w->q_norm_gamma && w->k_norm_gamma && !w->in_proj_b) {
         const int tiles = dim / 256;
         int rc = rfk::gemm_heads(window_buf, dim, w->in_proj_w, dim, Qt, (long long)M * dim, norm_ss, 3, M, 3 * dim, dim, ws2,
-                                 num_heads, hd, stream);
+                                 ws2, num_heads, hd, stream);
         if (rc == RFK_OK)
             rc = rfk::window_attention(Qt, Kt, Vt, window_buf, win_mask, norm_ss, norm_ss + (size_t)M * tiles, tiles,
                                        w->q_norm_gamma, w->k_norm_gamma, dim, kEpsFp16, BnW, num_heads, ws2, hd, nW,

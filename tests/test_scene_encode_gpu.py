@@ -63,3 +63,31 @@ def test_a_session_encodes_scene_after_scene(heads):
     kv = one[:2 * 72 * 256 * 2].view(torch.float16).view(2, heads, 72, 256 // heads)
     assert torch.isfinite(kv).all() and (kv[:, :, 66:] == 0).all() and (kv[:, :, :66] != 0).any(-1).all()
     a.close(); b.close()
+
+
+@pytest.mark.parametrize("Sk,heads,hd,kv_dim", [(1, 4, 64, 256), (33, 2, 128, 256), (120, 4, 64, 72), (333, 16, 64, 1024), (4700, 4, 64, 256)])
+def test_values_of_the_cache_are_the_plain_projection_head_split(Sk, heads, hd, kv_dim):
+    """V stored head-split by its projection, with pad rows behind each head: the plain product transposed, bit for bit,
+    on small and on large tiles, and zeros behind it."""
+    import ctypes
+    import renderformer_cuda_b200 as pkg
+    from renderformer_cuda_b200 import _abi, session
+    L, VP = _abi.load("rfk_layers.h"), ctypes.c_void_p
+    dim, pad = heads * hd, (Sk + 7) // 8 * 8
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).half()
+    model = session.Model.random(seed=1, dim=dim, num_heads=heads, ffn_hidden=256, enc_layers=0, dec_layers=1)
+    w = model.decoder_record(0).cross_attn
+    x, wv, wk = rnd(Sk, kv_dim), rnd(dim, kv_dim), rnd(dim, kv_dim)
+    w.v_proj_w, w.k_proj_w = wv.data_ptr(), wk.data_ptr()
+    K, V = (torch.full((heads, pad, hd), 7.0, device="cuda", dtype=torch.float16) for _ in range(2))
+    proj, want = torch.empty(2 * Sk, dim, device="cuda", dtype=torch.float16), torch.empty(Sk, dim, device="cuda", dtype=torch.float16)
+    ctx = session.Ctx()
+    rc = L.rfk_precompute_cross_kv(ctx.h, ctypes.byref(w), VP(x.data_ptr()), VP(K.data_ptr()), VP(V.data_ptr()), VP(proj.data_ptr()),
+                                   1, Sk, pad, kv_dim, dim, heads, VP(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, rc
+    pkg.ops.gemm_f16(x, wv, want, Sk, dim, kv_dim)
+    torch.cuda.synchronize()
+    assert torch.equal(V[:, :Sk], want.view(Sk, heads, hd).permute(1, 0, 2))
+    assert (V[:, Sk:] == 0).all() and (K[:, Sk:] == 0).all() and torch.isfinite(K.float()).all()
+    ctx.close()
