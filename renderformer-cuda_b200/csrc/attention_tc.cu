@@ -18,13 +18,15 @@
 //                so row maximum and row sum are thread-local (no shuffles). The 64 scores come to
 //                registers with tcgen05.ld; the common tile exponentiates them against the running
 //                reference right away and checks afterwards that this was admissible (the exact path,
-//                with the tile's maximum first, runs for the first tile, a padded last tile and a
-//                failed check); P = exp2(...) is rounded to fp16 and stored back with
-//                tcgen05.st over the first 32 columns of the same score buffer, from where
+//                with the tile's maximum first, runs for the first tile, a padded last tile, a
+//                failed check and every tile of 128-wide heads); P = exp2(...) is rounded to fp16
+//                and stored back with tcgen05.st over the first 32 columns of the same score
+//                buffer, from where
 //   warps 9-10   one thread per block issues O += P V with P as the A operand from tensor memory
 //                and V (MN-major) from shared memory: P never passes through shared memory. The
 //                output accumulator O (128 x 64 fp32 per block) is rescaled in place only when a
-//                row's running maximum has grown by more than 2^8 (the factor cancels in O / l).
+//                row's running maximum has grown by more than 2^8 (the factor cancels in O / l; at
+//                all with 128-wide heads).
 // A stage of the ring is free again when both blocks' P V products of its tile are complete
 // (kv_empty counts two arrivals). The products have separate issuing threads because one thread's
 // instruction stream (8 products, 3 commits and 2-3 waits per tile, all dependent) takes about as
@@ -155,19 +157,21 @@ __device__ __forceinline__ float2 exp2_poly(float2 x) {
 
 // 32 raw scores -> 32 probabilities exp2(s * c - mc), packed two fp16 per word into pk[0..16); their
 // fp32 sums are added to acc0 / acc1 (two lanes each).
-// Packed fp32x2 multiply-adds and adds halve the instruction count around the exponentials. The
-// special-function unit (16 exponentials per clock and SM) is the scarcest resource of this kernel,
-// so of every four pairs, those selected by kPolyMask take the polynomial path instead.
+// Packed fp32x2 multiply-adds and adds halve the instruction count around the exponentials. With 64-wide heads the
+// special-function unit (16 exponentials per clock and SM) is the scarcest resource of this kernel, so of every four
+// pairs those selected by the mask take the polynomial path instead. With 128-wide heads there are half as many
+// exponentials per product and every one comes from the special-function unit, as in flash_attention_kernel (the
+// polynomial was 5 us of 95 on 8 x 4096 x 5665, and 0.4 % of the result's distance from 64 bits).
 #ifndef RFK_ATTN_POLY_MASK
 #define RFK_ATTN_POLY_MASK 0x1
 #endif
-constexpr int kPolyMask = RFK_ATTN_POLY_MASK;
-
 #ifndef RFK_ATTN_POLY_PERIOD
 #define RFK_ATTN_POLY_PERIOD 4
 #endif
-__device__ __forceinline__ constexpr bool poly_pair(int pair) { return (kPolyMask >> (pair % RFK_ATTN_POLY_PERIOD)) & 1; }
+template <int HD> constexpr int kPolyMask = HD == 64 ? RFK_ATTN_POLY_MASK : 0;
+template <int HD> __device__ __forceinline__ constexpr bool poly_pair(int pair) { return (kPolyMask<HD> >> (pair % RFK_ATTN_POLY_PERIOD)) & 1; }
 
+template <int HD>
 __device__ __forceinline__ void exp_half(uint32_t (&v)[32], uint32_t* pk /* may alias v */, float c, float mc, float2& acc0,
                                          float2& acc1, float& poly_max) {
     const float2 c2 = make_float2(c, c), nm2 = make_float2(-mc, -mc);
@@ -181,13 +185,13 @@ __device__ __forceinline__ void exp_half(uint32_t (&v)[32], uint32_t* pk /* may 
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        if (poly_pair(i >> 1)) continue;  // this pair takes the polynomial path below
+        if (poly_pair<HD>(i >> 1)) continue;  // this pair takes the polynomial path below
         v[i] = __float_as_uint(fast_exp2(__uint_as_float(v[i])));
     }
-    if (kPolyMask) {
+    if (kPolyMask<HD>) {
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-            if (poly_pair(i >> 1)) {
+            if (poly_pair<HD>(i >> 1)) {
                 // the polynomial path is only good for exponents below 128: the caller checks the largest it was given
                 poly_max = fmax3(poly_max, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
                 const float2 p = exp2_poly(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])));
@@ -392,9 +396,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         regs_take();
         // ------------------------------------------------------------ softmax, warps 0-7 (query block = warp / 4)
         constexpr unsigned kFull = 0xffffffffu;
-        constexpr float kSumLimit = 256.0f;  // 2^kRescaleThreshold
+        constexpr float kSumLimit = 256.0f;  // 2^8, the threshold below
         constexpr uint32_t kNegInf = 0xff800000u;
-        constexpr float kRescaleThreshold = 8.0f;  // in exponent units: P stays below 2^8, well inside fp16
+        // In exponent units: P stays below 2^8, well inside fp16. With 128-wide heads the reference is the row's exact running
+        // maximum, as in flash_attention_kernel: a row's largest probabilities are then exactly 1 or round on the finer half
+        // of their binade. Against 64 bits the deferred reference was 3 % further off than that kernel on unit-variance
+        // scores and 19 to 21 % on scores of two and three times that; with the exact one the two agree to 1e-4 (8 x 4096 x
+        // 5665: 95 us deferred, 115 us exact, 362 us flash_attention_kernel).
+        constexpr bool kExactMax = HD == 128;
+        constexpr float kRescaleThreshold = kExactMax ? 0.0f : 8.0f;
         const int blk = warp >> 2;
         const int r = (warp & 3) * 32 + lane;                       // query row within the block = its tensor-memory lane
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;  // a warp reaches lanes [32 * (warp % 4), +32)
@@ -440,7 +450,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // tile) the scores are read again, the maximum is taken and the same code runs once more.
             float2 acc0, acc1;
             float m_new = m_run, alpha = 1.0f;
-            bool any_move = false, need_max = j == 0 || n_valid != BN;
+            bool any_move = false, need_max = kExactMax || j == 0 || n_valid != BN;
 #pragma unroll 1
             for (;;) {
                 acc0 = make_float2(0.0f, 0.0f);
@@ -465,9 +475,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 // the 32 packed words end up in va, which is what the store below takes
                 const float mc = m_new * scale_log2e;
                 float poly_max = -INFINITY;
-                exp_half(va, va, scale_log2e, mc, acc0, acc1, poly_max);
+                exp_half<HD>(va, va, scale_log2e, mc, acc0, acc1, poly_max);
                 tc::tc_wait_ld(vb);
-                exp_half(vb, va + 16, scale_log2e, mc, acc0, acc1, poly_max);
+                exp_half<HD>(vb, va + 16, scale_log2e, mc, acc0, acc1, poly_max);
                 if (need_max) break;
                 const float sum = (acc0.x + acc0.y) + (acc1.x + acc1.y);
                 if (!__any_sync(kFull, !(sum <= kSumLimit) || poly_max > kRescaleThreshold)) break;
