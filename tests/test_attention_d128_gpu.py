@@ -136,3 +136,23 @@ def test_no_further_from_64_bits_than_the_mma_kernel(B, Hh, Sq, Sk, n_keys, scal
     got, mma = _distance(O, Q, K, V, n_keys), _distance(M, Q, K, V, n_keys)
     print(f"distance from 64 bits: {got:.4e}, mma.sync kernel {mma:.4e}, ratio {got / mma:.4f}")
     assert got <= 1.002 * mma, (got, mma)
+
+
+@pytest.mark.parametrize("split", [False, True], ids=["whole", "split"])
+@pytest.mark.parametrize("n_out", [1, 64, 100, 640, 4096])
+def test_keys_with_a_score_of_minus_infinity(n_out, split):
+    """Keys switched off through an operand column (1 in every query, -inf in the key): none of a tile, whole tiles from the
+    first on, every piece of a unit, every key of a head (output 0, as from the mma.sync kernel)."""
+    B, Hh, Sq, Sk = 1, 2, 130, 4096
+    Q, K, V = _qkv(B, Hh, Sq, Sk)
+    Q[..., -1] = 1.0
+    K[..., -1] = 0.0
+    K[:, 0, :n_out, -1] = -float("inf")
+    O, M = torch.full_like(Q, 7.0), torch.full_like(Q, 7.0)
+    _ex(Q, K, V, O, B, Hh, Sq, Sk, Sk, D, workspace=pkg.ops.flash_attention_workspace() if split else None)
+    pkg.ops.flash_attention_set_path(1)
+    pkg.ops.flash_attention(Q, K, V, M, B, Hh, Sq, Sk, Sk, D)
+    assert torch.isfinite(M.float()).all()
+    _close(O, M, "keys at -inf")
+    if n_out == Sk:
+        assert not O[:, 0].any()
