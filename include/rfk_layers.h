@@ -325,8 +325,10 @@ int rfk_session_create(const rfk_model* model, int n_tris, int img_res, void* sc
  * scene, each with its own camera, that go through the decoder as one batch (rfk_session_render_frames). Throughput
  * mode: the projections see views_per_frame times the rows and the cross-attention that many times the work units,
  * which is what fills all SMs evenly (four views at 512 x 512: 1024 units on 148 SMs instead of 256); a frame's
- * results are the views' results back to back, bit-identical to rendering them one by one. Needs the fused attention
- * route (head size 64, dim % 256 == 0, QK-norm weights present): RFK_EUNSUPPORTED otherwise. No reference counterpart
+ * results are the views' results back to back, bit-identical to rendering them one by one wherever a view alone is not cut
+ * along its keys (rfk_flash_attention_plan: never from 148 units on, with 16 heads from 320 x 320 up at any number of
+ * triangles, below that up to 2112 (256 x 256), 1664 (192 x 192) or 1152 keys); where it is, that view and the same view in
+ * a frame are sums of the same terms in another order and differ by rounding. Needs the fused attention route (head size 64, dim % 256 == 0, QK-norm weights present): RFK_EUNSUPPORTED otherwise. No reference counterpart
  * (the reference renders one view at a time, render_session.cu:501-548). */
 int rfk_session_create_batched(const rfk_model* model, int n_tris, int img_res, void* scene_state, int flags,
                                int views_per_frame, rfk_session** out);

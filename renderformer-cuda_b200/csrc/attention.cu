@@ -529,7 +529,7 @@ size_t attention_tc_workspace_bytes();
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared);
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared);
 
 }  // namespace rfk
 
@@ -558,16 +558,16 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     const int path = g_attn_path.load(std::memory_order_relaxed);
     if ((D == 64 || D == 128) && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
         const int rc = launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk,
-                                           n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0, 0);
+                                           n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0, false, 0);
         if (rc != RFK_EUNSUPPORTED || path == 2) return rc;
     }
     return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
-extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
-                                           const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
-                                           size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
-                                           int o_bshd, float scale, rfk_stream_t stream) {
+int rfk::flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss,
+                            int ss_tiles, int norm_dim, float eps, void* workspace, size_t workspace_bytes, AttnCut cut,
+                            int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
+                            rfk_stream_t stream) {
     if (!Q || !K || !V || !O || B < 0 || H <= 0 || Sq < 0 || Sk <= 0 || n_keys <= 0 || n_keys > Sk || !(scale > 0.0f))
         return RFK_EINVAL;
     if (q_row_ss && (ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
@@ -575,8 +575,17 @@ extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K,
     if (B == 0 || Sq == 0) return RFK_OK;
     if ((D != 64 && D != 128) || (long long)B * H > 65535 || g_attn_path.load(std::memory_order_relaxed) == 1) return RFK_EUNSUPPORTED;
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
-    return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D,
-                               o_bshd, scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared != 0);
+    return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D, o_bshd,
+                               scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes,
+                               cut == AttnCut::kLastRound, v_shared != 0);
+}
+
+extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
+                                           const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
+                                           size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
+                                           int o_bshd, float scale, rfk_stream_t stream) {
+    return flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, AttnCut::kLastRound,
+                              v_shared, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
 // The public form takes 64-wide heads, as its header says.

@@ -650,16 +650,17 @@ bool make_map(CUtensorMap* m, const void* base, long long n_heads, long long row
 }
 
 // Fills `w` for `units` units of `n_tiles` key tiles each on a device with `sms` SMs (see "Key split" above): full rounds
-// of units run whole, and the units of the last, partial round are cut when the estimate says it pays.
-// split = false: every unit whole.
-void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool split) {
+// of units run whole, and the units of the last, partial round are cut when the estimate says it pays. split = false: every
+// unit whole; cut_last_round = false: every unit of a grid of one round or more whole. A cut changes the order of the sums, so
+// whether a unit is cut, and where, must not depend on what else is in the launch where the caller promises equal bits.
+void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool split, bool cut_last_round) {
     using tcattn::Piece;
     constexpr int kPieceCostTiles = 12;  // what a piece costs beyond its tiles (fill, publishing, merging), in tile times
     w.whole_units = (int)units;
     w.n_pieces = 0;
     if (!split || sms <= 0 || units <= 0 || n_tiles > 65535 || units > 65535) return;
     const int rounds = (int)(units / sms), rest = (int)(units % sms);
-    if (rest == 0 || rest > 256) return;  // 256 unit counters
+    if (rest == 0 || rest > 256 || (rounds > 0 && !cut_last_round)) return;  // 256 unit counters
     const long long tiles = (long long)rest * n_tiles;
     constexpr int kMaxPiecesPerUnit = 8;  // the CTA that merges a unit reads its pieces one after the other
     const int shares = (int)std::min<long long>(std::min(sms, tcattn::kMaxPieces / 2), (long long)rest * kMaxPiecesPerUnit);
@@ -703,7 +704,7 @@ size_t attention_tc_workspace_bytes() { return tcattn::kWsBytes; }
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces) {
     if (units < 0 || n_tiles <= 0 || sms <= 0 || !whole_units || !n_pieces || max_pieces < 0 || (max_pieces && !pieces)) return RFK_EINVAL;
     tcattn::WorkList w;
-    plan_work(w, units, n_tiles, sms, true);
+    plan_work(w, units, n_tiles, sms, true, true);
     *whole_units = w.whole_units;
     *n_pieces = w.n_pieces;
     for (int i = 0; i < w.n_pieces && i < max_pieces; ++i) {
@@ -718,7 +719,7 @@ namespace {
 template <int HD>
 int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
               int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-              int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared) {
+              int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared) {
     // per-device "kernel attributes set" marks; setting them twice from racing threads is harmless
     static std::atomic<bool> configured[64];
     static std::atomic<int> sm_count[64];
@@ -747,7 +748,8 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
     const long long units = (long long)B * H * work.q_blocks;
     if (units > 0x7fffffffLL) return RFK_EUNSUPPORTED;
     const bool split = ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
-    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sm_count[dev].load(std::memory_order_relaxed), split);
+    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sm_count[dev].load(std::memory_order_relaxed), split,
+              cut_last_round);
     dim3 grid((unsigned)(work.whole_units + work.n_pieces));
     launch_pdl(kernel, grid, dim3(tcattn::kThreads), tcattn::Cfg<HD>::kSmemBytes, st, mq, mk, mv, O, H, Sq, n_keys,
                o_bshd, scale * 1.4426950408889634f, row_ss, ss_tiles, norm_dim > 0 ? 1.0f / (float)norm_dim : 0.0f, norm_eps,
@@ -761,9 +763,9 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
 // attention_tc_workspace_bytes() bytes whose first 1024 are zero, for the key split.
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, int v_shared) {
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared) {
     return (D == 64 ? launch_hd<64> : launch_hd<128>)(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles,
-                                                      norm_dim, norm_eps, ws, ws_bytes, v_shared);
+                                                      norm_dim, norm_eps, ws, ws_bytes, cut_last_round, v_shared);
 }
 
 }  // namespace rfk

@@ -225,8 +225,8 @@ static int attention_core(rfk_ctx* ctx, const rfk_half* Q, const rfk_half* K, co
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
     if (ctx->attn_ws)  // tcgen05 kernel with the balanced key split; declines what only the other kernels serve
-        rc = rfk_flash_attention_ex_wide(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, 0, B, H, Sq, Sk, n_keys, D,
-                                    o_bshd, 1.0f / sqrtf((float)D), stream);
+        rc = rfk::flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, rfk::AttnCut::kLastRound, 0,
+                                     B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
     if (rc == RFK_EUNSUPPORTED)
         rc = rfk_flash_attention(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
     if (rc != RFK_EUNSUPPORTED) return rc;
@@ -337,10 +337,13 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
                                               w->q_norm_gamma, 0, stream);
                 K_use = K_rot;
             }
+            // With 64-wide heads a view is rendered alone or in a frame of several and must have the same bits: a view alone
+            // that fills the SMs (208 units at 448 x 448) stays whole, as it is among the units of a frame. 128-wide heads have
+            // no such frames.
             if (rc == RFK_OK)
-                rc = rfk_flash_attention_ex_wide(Q_bhsd, K_use, V_cached, Q, norm_ss, dim / 256, dim, kEpsFp16, ctx->attn_ws,
-                                            ctx->attn_ws_bytes, v_shared, B, num_heads, Sq, Sk, n_keys, hd, 1,
-                                            1.0f / sqrtf((float)hd), stream);
+                rc = rfk::flash_attention_ex(Q_bhsd, K_use, V_cached, Q, norm_ss, dim / 256, dim, kEpsFp16, ctx->attn_ws,
+                                             ctx->attn_ws_bytes, hd == 64 ? rfk::AttnCut::kBelowOneRound : rfk::AttnCut::kLastRound,
+                                             v_shared, B, num_heads, Sq, Sk, n_keys, hd, 1, 1.0f / sqrtf((float)hd), stream);
         }
         if (rc != RFK_OK && rc != RFK_EUNSUPPORTED) return rc;
         if (rc == RFK_EUNSUPPORTED && (k_prescaled || (v_shared && B > 1))) return rc;  // only the fused route serves these

@@ -91,3 +91,23 @@ def test_batched_session_refuses_models_without_the_fused_route():
     with pytest.raises(session.RfkLayersError):
         session.RenderSession(model, 20, 128, views_per_frame=2)
     session.RenderSession(model, 20, 128).close()                      # one view per frame still works
+
+
+@pytest.mark.parametrize("res,n_tris,V", [(448, 5000, 4), (320, 7200, 3)])
+def test_equality_where_a_cut_would_pay(res, n_tris, V):
+    """Views whose attention has enough keys for a cut to pay. 448 x 448: a view alone has 208 units of work on 148 SMs, 60 in
+    its last round, its frame of four 832. 320 x 320: alone 112 units, left whole, a frame of three 336, 40 in the last
+    round. One cut along the keys and the other whole would differ in the order of their sums."""
+    session, cases = _mods()
+    model = session.Model.random(seed=9, dim=1024, num_heads=16, ffn_hidden=256, enc_layers=0, dec_layers=1)
+    c2w, fov = cases.look_at_c2w(np.random.default_rng(3), V)
+    one = session.RenderSession(model, n_tris, res)
+    one.encode_scene(*_scene(n_tris)); one.finalize()
+    many = session.RenderSession(model, n_tris, res, scene_state=one.scene_state, views_per_frame=V)
+    many.finalize()
+    many.render_frames(torch.as_tensor(np.asarray(c2w, dtype=np.float32)), torch.as_tensor(np.asarray(fov, dtype=np.float32)))
+    got = many.download()
+    for v in range(V):
+        one.render_frame(c2w[v], float(fov[v]))
+        assert torch.equal(got[v], one.download()), f"view {v}"
+    many.close(); one.close()
