@@ -220,13 +220,13 @@ static int attention_core(rfk_ctx* ctx, const rfk_half* Q, const rfk_half* K, co
                           float* score_buf, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd,
                           rfk_stream_t stream) {
     int rc = RFK_EUNSUPPORTED;
-    if (D == 128 && ctx->d128_reproducible) {
+    if (D == 128 && ctx->reproducible) {
         rc = rfk::flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
     if (ctx->attn_ws)  // tcgen05 kernel with the balanced key split; declines what only the other kernels serve
-        rc = rfk::flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes, rfk::AttnCut::kLastRound, 0,
-                                     B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
+        rc = rfk::flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, ctx->attn_ws, ctx->attn_ws_bytes,
+                                     ctx->reproducible ? rfk::AttnCut::kBelowOneRound : rfk::AttnCut::kLastRound, 0, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
     if (rc == RFK_EUNSUPPORTED)
         rc = rfk_flash_attention(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, 1.0f / sqrtf((float)D), stream);
     if (rc != RFK_EUNSUPPORTED) return rc;
@@ -322,7 +322,7 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
     // or 128.
     const int k_prescaled = cache_flags & 1, v_shared = (cache_flags >> 1) & 1;
     const bool deferred = norm_ss && w->q_norm_gamma && !w->q_proj_b && !q_rope_cos &&
-                          (hd == 64 || (hd == 128 && !ctx->d128_reproducible)) && (k_prescaled || k_rope_cos) &&
+                          (hd == 64 || (hd == 128 && !ctx->reproducible)) && (k_prescaled || k_rope_cos) &&
                           (reinterpret_cast<uintptr_t>(w->q_norm_gamma) & 15u) == 0;
     if (k_prescaled && !deferred) return RFK_EUNSUPPORTED;  // prescaled keys only make sense with the deferred norm
     if (deferred) {
@@ -398,7 +398,7 @@ static int swin_core(rfk_ctx* ctx, const rfk_mha_weights* w, rfk_half* window_bu
     // Deferred QK-RMSNorm: the packed projection writes q, k, v head-split per window and the sums of squares of the q and
     // k rows; the window attention kernel normalises the two tiles while it stages them (same formula and rounding as
     // the separate kernel). One kernel and 50 MB of traffic less per layer.
-    const bool fused = ws2 == 64 && (hd == 64 || (hd == 128 && !ctx->d128_reproducible));  // the window attention kernel
+    const bool fused = ws2 == 64 && (hd == 64 || (hd == 128 && !ctx->reproducible));  // the window attention kernel
     if (hd != 64 && !score_buf) return RFK_EINVAL;            // score space is only optional for 64-wide heads
     if (norm_ss && fused && w->q_norm_gamma && w->k_norm_gamma && !w->in_proj_b) {
         const int tiles = dim / 256;

@@ -12,9 +12,10 @@ struct rfk_ctx {
     size_t ws_bytes = 0;
     void* attn_ws = nullptr;  // split workspace of the attention kernel (rfk_ctx_reserve_attention_workspace), else NULL
     size_t attn_ws_bytes = 0;
-    // 128-wide heads on the kernels that images have always been made with: mma.sync attention, GEMM -> softmax -> GEMM in
-    // the windows, a separate query norm. Set for sessions with an image head (rfk_session_create_batched says why).
-    bool d128_reproducible = false;
+    // Every sum in the order that images have always been made with: no key split of grids of one round or more, and 128-wide
+    // heads on mma.sync attention, GEMM -> softmax -> GEMM in the windows and a separate query norm. Set for sessions with an
+    // image head (rfk_session_create_batched says why).
+    bool reproducible = false;
     int device = 0;
 };
 

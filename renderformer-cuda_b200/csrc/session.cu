@@ -328,11 +328,12 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
     if (!rc) rc = rfk_ctx_reserve_attention_workspace(d->ctx);  // all attention launches of a session are on its one stream
     auto fail = [&](int code) { rfk_session_destroy(d); return code; };
     if (rc) return fail(rc);
-    // An image is 10^x of an fp16 head output: a change in the order of one fp32 sum of the decoder flips roundings that come
-    // out as 0.7 to 1.8 % of the image (measured over 20 scenes; the token maps differ by 0.1 %). Sessions with an image head
-    // and 128-wide heads therefore stay on the kernels that earlier versions rendered with, so that an image of
-    // a scene does not change; sessions that end at the token map take the faster ones.
-    d->ctx->d128_reproducible = model->dpt && d->hd == 128;
+    // An image is 10^x of an fp16 head output: a change in the order of one fp32 sum of the encoder or decoder flips roundings
+    // that come out as 0.7 to 1.8 % of the image (measured over 20 scenes; the token maps differ by 0.1 %), though neither
+    // order is further from the exact result. Sessions with an image head therefore keep the kernels and the order that
+    // earlier versions rendered with, so that the image of a scene does not change; sessions that end at the token map take
+    // the faster ones.
+    d->ctx->reproducible = model->dpt != nullptr;
     if (cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) != cudaSuccess) return fail((int)cudaGetLastError());
     if (cudaStreamCreateWithFlags(&d->copy_stream, cudaStreamNonBlocking) != cudaSuccess) return fail((int)cudaGetLastError());
     if (cudaStreamCreateWithFlags(&d->side_stream, cudaStreamNonBlocking) != cudaSuccess) return fail((int)cudaGetLastError());
@@ -368,7 +369,7 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
     {
         // Deferred Q-RMSNorm of the cross-attention (layers.cu): possible when the fused kernels serve the shape and every
         // layer has a norm weight, no query bias and no window-path exclusions; then the key rotation folds the weights in.
-        bool ok = (d->hd == 64 || (d->hd == 128 && !d->ctx->d128_reproducible)) && dim % 256 == 0 && d->nP % 32 == 0 && d->pH % ws == 0 && dim <= 2048;
+        bool ok = (d->hd == 64 || (d->hd == 128 && !d->ctx->reproducible)) && dim % 256 == 0 && d->nP % 32 == 0 && d->pH % ws == 0 && dim <= 2048;
         for (int i = 0; i < model->dec_layers && ok; ++i)
             ok = model->dec[i].cross_attn.q_norm_gamma && !model->dec[i].cross_attn.q_proj_b && !model->dec[i].cross_attn.out_proj_b &&
                  (reinterpret_cast<uintptr_t>(model->dec[i].cross_attn.q_norm_gamma) & 15u) == 0;

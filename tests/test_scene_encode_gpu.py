@@ -91,3 +91,25 @@ def test_values_of_the_cache_are_the_plain_projection_head_split(Sk, heads, hd, 
     assert torch.equal(V[:, :Sk], want.view(Sk, heads, hd).permute(1, 0, 2))
     assert (V[:, Sk:] == 0).all() and (K[:, Sk:] == 0).all() and torch.isfinite(K.float()).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("with_dpt", [True, False])
+def test_cut_of_the_last_round_and_images(with_dpt):
+    """2500 triangles and 16 heads are 160 units of attention work on 148 SMs: a session that ends at the token map cuts the
+    last round's along the keys, one with an image head does not, so that its images stay what they were."""
+    import renderformer_cuda_b200 as pkg
+    from renderformer_cuda_b200 import session
+    n = 2500
+    model = session.Model.random(seed=2, dim=1024, num_heads=16, ffn_hidden=256, enc_layers=1, dec_layers=1, with_dpt=with_dpt,
+                                 dpt_features=64, dpt_out_channels=(32, 64, 128, 128))
+    s = session.RenderSession(model, n, 64)
+    states = []
+    try:
+        for split in (1, 0):
+            pkg.ops.flash_attention_set_split(split)
+            s.encode_scene(*_scene(n, 3))
+            states.append(s.scene_state.clone())
+    finally:
+        pkg.ops.flash_attention_set_split(1)
+    assert torch.equal(*states) == with_dpt
+    s.close()
