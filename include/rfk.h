@@ -348,7 +348,7 @@ int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W, long long 
  * outputs of that row in columns [256 t, 256 t + 256) of part p, written (not accumulated, no zeroing needed, bit-
  * reproducible) for the parts whose bit is set in ss_parts_mask; the consumer adds the entries of a row and applies
  * rsqrt(sum / dim + eps) and the norm weight while it loads (rfk_flash_attention_ex, rfk_window_attention_normed).
- * CTA-pair tcgen05 kernel only: RFK_EUNSUPPORTED (nothing launched) unless num_heads % 4 == 0, seq_len % 32 == 0,
+ * tcgen05 kernels only (small tiles or CTA pairs): RFK_EUNSUPPORTED (nothing launched) unless num_heads % 4 == 0, seq_len % 32 == 0,
  * M % seq_len == 0 and the alignment rules of rfk_gemm_f16 hold; callers then run the projection and
  * rfk_qkv_norm_rope_transpose separately.
  * replaces linear -> (deinterleave_qkv) -> rmsnorm -> transpose_bshd_to_bhsd — src/layers/attention.cu:180-206,336-349,
@@ -356,11 +356,13 @@ int rfk_gemm_f16(const rfk_half* A, long long lda, const rfk_half* W, long long 
 int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out,
                        long long part_stride, float* row_ss, int ss_parts_mask, int M, int N, int K,
                        int seq_len, int num_heads, rfk_stream_t stream);
-/* 0 automatic (the tcgen05 kernel whenever the shape allows: on CTA pairs, tcgen05.mma.cta_group::2,
- * or on single CTAs if the device cannot co-schedule pairs), 1 never (rfk_gemm_f16 returns
- * RFK_EUNSUPPORTED, so the layer functions fall back to their cuBLAS calls: used to time both side
- * by side), 2 as 0, 3 the single-CTA kernel. Process-wide; the environment variable RFK_GEMM_PATH
- * sets the initial value. No reference counterpart. */
+/* 0 automatic (a tcgen05 kernel whenever the shape allows: small tiles, one per CTA, for calls whose
+ * tiles then all run at once; else 256 x 256 tiles on CTA pairs, tcgen05.mma.cta_group::2, or on single
+ * CTAs if the device cannot co-schedule pairs; the result has the same bits on all of them), 1 never
+ * (rfk_gemm_f16 returns RFK_EUNSUPPORTED, so the layer functions fall back to their cuBLAS calls: used
+ * to time both side by side), 2 CTA pairs at every size (single CTAs if pairs are unavailable), 3 the
+ * single-CTA kernel. Process-wide; the environment variable RFK_GEMM_PATH sets the initial value. No
+ * reference counterpart. */
 int rfk_gemm_set_path(int path);
 /* CTA pairs (clusters of two) that the current device runs at once for the pair kernel, as the
  * occupancy query answered at the first launch: 0 before any launch, -1 if pairs cannot be scheduled

@@ -1005,9 +1005,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }  // namespace pair
 }  // namespace tcgemm
 
-// 0 automatic (tcgen05 kernel on CTA pairs when the shape allows), 1 never (callers use their library GEMM), 2 as 0,
-// 3 the single-CTA tcgen05 kernel. The
-// environment variable RFK_GEMM_PATH sets the initial value, for side-by-side runs of an unchanged program.
+// 0 automatic (tcgen05 kernels when the shape allows: small tiles or CTA pairs by the rule of small_tile), 1 never (callers use
+// their library GEMM), 2 CTA pairs whatever the size, 3 the single-CTA tcgen05 kernel. The environment variable RFK_GEMM_PATH
+// sets the initial value, for side-by-side runs of an unchanged program.
 static int initial_gemm_path() {
     const char* e = getenv("RFK_GEMM_PATH");
     return (e && e[0] >= '0' && e[0] <= '3' && e[1] == 0) ? e[0] - '0' : 0;
@@ -1193,13 +1193,13 @@ int small_tile(int M, int acc_cols, int sms) {
     return 0;
 }
 
-// path 0 / 2: small tiles or CTA pairs, the single-CTA kernel if pairs are unavailable; path 3: the single-CTA kernel
+// path 0: small tiles or CTA pairs; path 2: CTA pairs; the single-CTA kernel if pairs are unavailable; path 3: that kernel
 template <int EPI>
 int launch_gemm(const void* A, long long lda, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev,
                 cudaStream_t st) {
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     const int path = g_gemm_path.load(std::memory_order_relaxed);
-    if (path != 3) {
+    if (path == 0) {
         int rc = RFK_EUNSUPPORTED;
         switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
             case 1: rc = launch_gemm_small<EPI, 64, 32>(A, lda, W, W_up, ldw, p, dev, st); break;
@@ -1270,7 +1270,7 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     if (parts > 1 && part_stride < (long long)M * dim) return RFK_EINVAL;
     if (M == 0) return RFK_OK;
     const int path = g_gemm_path.load(std::memory_order_relaxed);
-    if (path == 1 || path == 3) return RFK_EUNSUPPORTED;   // pair kernel only
+    if (path == 1 || path == 3) return RFK_EUNSUPPORTED;   // the single-CTA kernel has no head-split epilogue
     // a 256-column tile must lie inside one part, a 32-row store box inside one group
     if (dim % 256 != 0 || M % seq_len != 0) return RFK_EUNSUPPORTED;
     if (out_seq < seq_len || (M != seq_len && (seq_len % 32 != 0 || out_seq != seq_len))) return RFK_EUNSUPPORTED;
@@ -1285,7 +1285,7 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     p.C = (__half*)out; p.ldc = N; p.M = M; p.N = N; p.K = K;
     p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
     p.part_stride = part_stride; p.out_seq = out_seq;
-    {
+    if (path == 0) {
         // The rule of the other epilogues over tiles of at least 64 columns; a cluster of four needs its SMs within one GPC,
         // which leaves about an eighth of them over.
         const int sms = sm_count(dev), tile = small_tile(M, N, sms - sms / 8);

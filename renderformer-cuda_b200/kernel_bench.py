@@ -347,7 +347,7 @@ def gemm_table(iters: int = 20, nsets: int = 6) -> list[dict]:
                 if epi == "residual":
                     ops.residual_add(c[i], r[i], M * N)
 
-        ops.gemm_set_path(2)
+        ops.gemm_set_path(0)
         t_f = _time_graph(fused, nsets, iters)
         ops.gemm_set_path(3)
         t_s = _time_graph(fused, nsets, iters)

@@ -387,7 +387,8 @@ def gemm_f16_heads(a, w, out, row_ss, ss_parts_mask, M, N, K, seq_len, num_heads
 
 
 def gemm_set_path(path):
-    """0 automatic (tcgen05 kernel on CTA pairs), 1 library GEMM only (rfk_gemm_f16 refuses), 2 as 0, 3 single-CTA kernel."""
+    """0 automatic (tcgen05: small tiles or CTA pairs by size), 1 library GEMM only (rfk_gemm_f16 refuses), 2 CTA pairs at
+    every size, 3 single-CTA kernel."""
     _call("rfk_gemm_set_path", int(path))
 
 

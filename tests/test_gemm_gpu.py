@@ -19,8 +19,8 @@ def _ops():
 
 @pytest.fixture(autouse=True, params=[2, 3], ids=["cta_pair", "single_cta"])
 def _error_word_clear(request):
-    """Every test runs once through the CTA-pair kernel (tcgen05.mma.cta_group::2, the default) and once through
-    the single-CTA kernel."""
+    """Every test runs once through the CTA-pair kernel (tcgen05.mma.cta_group::2) at every size and once through the
+    single-CTA kernel; test_gemm_small_gpu.py compares the small tiles, which serve most small calls, with them."""
     o = _ops()
     o.gemm_error(clear=True)
     o.gemm_set_path(request.param)
@@ -43,7 +43,7 @@ def _rand(g, *shape, scale=1.0):
 
 
 SHAPES = [(128, 256, 64), (128, 256, 1024), (4096, 1024, 1024), (4096, 3072, 1024), (4096, 1024, 4096), (4096, 1024, 192),
-          (5665, 1024, 1024), (300, 264, 200), (1, 8, 8), (77, 1000, 136), (257, 520, 72)]
+          (5665, 1024, 1024), (300, 264, 200), (1, 8, 8), (77, 1000, 136), (257, 520, 72), (2500, 1032, 328)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
@@ -55,7 +55,7 @@ def test_gemm_plain_matches_fp32_product(M, N, K):
     _close(c, a.float() @ w.float().t(), f"gemm {M}x{N}x{K}")
 
 
-@pytest.mark.parametrize("M,N,K", [(4096, 1024, 4096), (300, 264, 200), (4096, 1024, 1024)])
+@pytest.mark.parametrize("M,N,K", [(4096, 1024, 4096), (300, 264, 200), (4096, 1024, 1024), (2500, 1032, 328)])
 def test_gemm_bias_and_residual_epilogues(M, N, K):
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a, w = _rand(g, M, K), _rand(g, N, K, scale=K ** -0.5)

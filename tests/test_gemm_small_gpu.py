@@ -86,3 +86,30 @@ def test_head_split_form_has_the_bits_of_the_pair_kernel(M, seq, heads, parts, K
         got.append((out[:, :M * dim], ss[:, :M]))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert all(bool((got[0][1][p] >= 0).all()) == bool(mask >> p & 1) for p in range(parts))
+
+
+def test_pair_path_serves_small_calls_with_the_pair_kernel():
+    """In a fresh process: the pair kernel's occupancy query has run after one small call on path 2, and not after the same
+    call on path 0, which goes to the small tiles."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    code = """
+import sys, torch, renderformer_cuda_b200 as pkg
+from renderformer_cuda_b200 import _abi
+o, lib = pkg.ops, _abi.load("rfk.h")
+a = torch.randn(77, 136, device="cuda").half(); w = torch.randn(1000, 136, device="cuda").half()
+h = torch.randn(64, 64, device="cuda").half(); wh = torch.randn(256, 64, device="cuda").half()
+out = torch.empty(77, 1000, device="cuda", dtype=torch.float16); outh = torch.empty(4, 64, 64, device="cuda", dtype=torch.float16)
+o.gemm_set_path(int(sys.argv[1]))
+if sys.argv[2] == "plain": o.gemm_f16(a, w, out, 77, 1000, 136)
+else: o.gemm_f16_heads(h, wh, outh, None, 0, 64, 256, 64, 64, 4)
+torch.cuda.synchronize()
+print(lib.rfk_gemm_pair_clusters())
+"""
+    root = Path(__file__).resolve().parent.parent
+    for form in ("plain", "heads"):
+        for path in ("0", "2"):
+            r = subprocess.run([sys.executable, "-c", code, path, form], capture_output=True, text=True, cwd=root)
+            assert r.returncode == 0, r.stderr
+            assert (int(r.stdout.split()[-1]) > 0) == (path == "2"), (form, path, r.stdout)
