@@ -368,6 +368,10 @@ int rfk_gemm_set_path(int path);
  * occupancy query answered at the first launch: 0 before any launch, -1 if pairs cannot be scheduled
  * (the single-CTA kernel then serves every call). Diagnostic. No reference counterpart. */
 int rfk_gemm_pair_clusters(void);
+/* The tile rfk_gemm_f16_heads takes for M rows and N columns when resident[0..2] CTAs of its tiles of 64 x 64, 128 x 64 and
+ * 128 x 128 run at once (whole clusters of four, four and two; 0: the device cannot place one): 1, 2 or 3, or 0 for the
+ * CTA-pair kernel. Host only: touches no device. Diagnostic. No reference counterpart. */
+int rfk_gemm_heads_tile(int M, int N, const int* resident);
 /* Reads (and with clear != 0 resets) the current device's error word of the GEMM kernel: 0 none,
  * 1 a bounded wait ran out, 2 shared memory window not 1024-byte aligned. Synchronises the device.
  * No reference counterpart. */

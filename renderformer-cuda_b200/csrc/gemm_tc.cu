@@ -1143,7 +1143,34 @@ int sm_count(int dev) {
     return n;
 }
 
-// ---- small tiles: their launch, and the rule that chooses them
+// ---- small tiles: their launch, and the rules that choose them
+// CTAs of the head-split form on this tile that the device runs at once, in whole clusters of 256 columns (a cluster needs its
+// SMs within one GPC): the occupancy query's answer, asked once per device. 0: it cannot place such a cluster at all. At most
+// seven eighths of the SMs: the query gives 132 of 148 for clusters of four and all 148 for clusters of two, but a grid that
+// takes every SM is no faster than CTA pairs (2304 x 1024 x 1024, 144 tiles of 128 x 128: 11.7 us, pairs 11.3).
+template <int BM_, int BN_>
+int heads_resident(int dev) {
+    static std::atomic<int> asked[64];   // the answer + 1
+    int n = asked[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+        constexpr auto kernel = tcgemm::small::gemm_tc_small_kernel<tcgemm::kEpiHeads, BM_, BN_>;
+        constexpr int smem = tcgemm::small::Cfg<BM_, BN_>::kSmemBytes, size = 256 / BN_;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(size * std::max(1, sm_count(dev))); cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = smem;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int clusters = 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+        if (e != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+        n = std::min(std::max(clusters, 0) * size, sm_count(dev) - sm_count(dev) / 8) + 1;
+        asked[dev].store(n, std::memory_order_release);
+    }
+    return n - 1;
+}
+
 template <int EPI, int BM_, int BN_>
 int launch_gemm_small(const void* A, long long lda, const void* W, const void* W_up, long long ldw, tcgemm::Params p, int dev,
                       cudaStream_t st) {
@@ -1190,6 +1217,15 @@ int small_tile(int M, int acc_cols, int sms) {
     constexpr int kTiles[4][2] = {{64, 32}, {64, 64}, {128, 64}, {128, 128}};   // rows, accumulator columns
     for (int i = 0; i < 4; ++i)
         if ((long long)ceil_div(M, kTiles[i][0]) * ceil_div(acc_cols, kTiles[i][1]) <= sms) return i + 1;
+    return 0;
+}
+
+// The same rule for the head-split form, over its tiles of at least 64 columns: resident[i] CTAs of tile i run at once
+// (heads_resident; 0: that tile cannot run). 1 to 3: the tile, 0: the pair kernel.
+int heads_tile(int M, int N, const int* resident) {
+    constexpr int kTiles[3][2] = {{64, 64}, {128, 64}, {128, 128}};
+    for (int i = 0; i < 3; ++i)
+        if ((long long)ceil_div(M, kTiles[i][0]) * ceil_div(N, kTiles[i][1]) <= resident[i]) return i + 1;
     return 0;
 }
 
@@ -1286,14 +1322,14 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
     p.row_ss = row_ss; p.seq = seq_len; p.units = dim / 64; p.head_units = head_dim / 64; p.ss_mask = ss_parts_mask;
     p.part_stride = part_stride; p.out_seq = out_seq;
     if (path == 0) {
-        // The rule of the other epilogues over tiles of at least 64 columns; a cluster of four needs its SMs within one GPC,
-        // which leaves about an eighth of them over.
-        const int sms = sm_count(dev), tile = small_tile(M, N, sms - sms / 8);
+        const int resident[3] = {heads_resident<64, 64>(dev), heads_resident<128, 64>(dev), heads_resident<128, 128>(dev)};
+        const cudaStream_t st = as_stream(stream);
         int rc = RFK_EUNSUPPORTED;
-        cudaStream_t st = as_stream(stream);
-        if (tile == 1 || tile == 2) rc = launch_gemm_small<tcgemm::kEpiHeads, 64, 64>(A, lda, W, nullptr, ldw, p, dev, st);
-        if (tile == 3) rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 64>(A, lda, W, nullptr, ldw, p, dev, st);
-        if (tile == 4) rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 128>(A, lda, W, nullptr, ldw, p, dev, st);
+        switch (heads_tile(M, N, resident)) {
+            case 1: rc = launch_gemm_small<tcgemm::kEpiHeads, 64, 64>(A, lda, W, nullptr, ldw, p, dev, st); break;
+            case 2: rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 64>(A, lda, W, nullptr, ldw, p, dev, st); break;
+            case 3: rc = launch_gemm_small<tcgemm::kEpiHeads, 128, 128>(A, lda, W, nullptr, ldw, p, dev, st); break;
+        }
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
     CUtensorMap ma, mw, mh;
@@ -1311,6 +1347,10 @@ extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_ha
     const int out_seq = seq_len % 32 == 0 ? seq_len : 0;   // 0: refused, as the header says
     return gemm_heads(A, lda, W, ldw, out, part_stride, row_ss, ss_parts_mask, M, N, K, seq_len, out_seq, num_heads, 64,
                       stream);
+}
+
+extern "C" int rfk_gemm_heads_tile(int M, int N, const int* resident) {
+    return M > 0 && N > 0 && resident ? heads_tile(M, N, resident) : RFK_EINVAL;
 }
 
 extern "C" int rfk_gemm_pair_clusters(void) {
