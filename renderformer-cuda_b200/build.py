@@ -6,7 +6,7 @@ Produces, next to this file:
     librfk.so         the kernel library behind include/rfk.h (CUDA runtime only)
     librfk_layers.so  layer boundaries, render session (include/rfk_layers.h; cuBLAS + librfk.so)
     librfk_io.so      weight, scene and image files (include/rfk_io.h)
-    _native.so        the operators of librfk.so as Python callables (compiled against the installed torch)
+    _native.<abi>.so  the operators of librfk.so as Python callables (compiled against this interpreter and its torch)
 
 nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine.
 """
@@ -94,15 +94,23 @@ def cudnn_include() -> str:
     return os.path.join(sysconfig.get_paths()["purelib"], "nvidia", "cudnn", "include")
 
 
+def binding_built_for() -> str:
+    """What the binding is compiled against and must be imported with (ops.py checks)."""
+    from importlib.metadata import version
+    return f"torch {version('torch')} {sys.implementation.cache_tag}"
+
+
 def build_binding(force: bool, verbose: bool) -> Path:
-    """_native.so, a Python extension module: g++ against the headers of this interpreter and of its torch, whose
-    libraries are in the process already when it is imported."""
+    """_native, a Python extension module: g++ against the headers of this interpreter and of its torch, whose
+    libraries are in the process already when it is imported. Another interpreter looks for another file name; a module that
+    does not carry the installed torch's version is built again."""
     import sysconfig
-    out, src = PKG / "_native.so", CSRC / "ops_binding.cpp"
-    if force or not _newer(out, [src, INCLUDE / "rfk.h"]):
+    out, src, built_for = PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX")), CSRC / "ops_binding.cpp", binding_built_for()
+    if force or not _newer(out, [src, INCLUDE / "rfk.h"]) or built_for.encode() not in out.read_bytes():
         torch_dir = Path(sysconfig.get_paths()["purelib"]) / "torch"
         cuda_include = Path(nvcc()).resolve().parent.parent / "include"
         _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wno-unused-function",
+              f'-DRFK_BUILT_FOR="{built_for}"',
               f"-I{INCLUDE}", f"-I{sysconfig.get_paths()['include']}", f"-isystem{torch_dir / 'include'}",
               f"-isystem{torch_dir / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-isystem{cuda_include}",
               str(src), "-o", str(out), f"-L{PKG}", "-lrfk", "-Wl,-rpath,$ORIGIN", f"-L{torch_dir / 'lib'}",

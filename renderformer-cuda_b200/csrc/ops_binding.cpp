@@ -202,5 +202,8 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", "Operators of librfk
 PyMODINIT_FUNC PyInit__native() {
     op_type = PyType_FromSpec(&op_spec);
     if (!op_type) return nullptr;
-    return PyModule_Create(&module_def);
+    PyObject* module = PyModule_Create(&module_def);
+    // what it was compiled against (build.py); torch's C++ interface is only the same within a version
+    if (module && PyModule_AddStringConstant(module, "built_for", RFK_BUILT_FOR) < 0) Py_CLEAR(module);
+    return module;
 }

@@ -13,6 +13,8 @@ from __future__ import annotations
 import ctypes
 import functools
 import inspect
+import sys
+import warnings
 
 import torch
 
@@ -59,10 +61,27 @@ def _failed(symbol: str, status: int):
     raise RfkError(symbol, status)
 
 
+@functools.cache
+def _binding():
+    """The compiled binding, or None (said once) where it is not built or was built for another torch."""
+    why = "not built (python renderformer-cuda_b200/build.py)"
+    try:
+        from . import _native as binding
+        want = f"torch {torch.__version__} {sys.implementation.cache_tag}"
+        if binding.built_for == want:
+            return binding
+        why = f"built for {binding.built_for}, this is {want}"
+    except ImportError as e:
+        why = f"{why}: {e}"
+    warnings.warn(f"operators are called through ctypes, 4 to 6 us a call slower: the compiled binding is {why}", RuntimeWarning, stacklevel=4)
+    return None
+
+
 def _native(checked):
     """Operators whose parameters are those of `rfk_<name>` in the same order are called through the compiled binding
     (csrc/ops_binding.cpp), which is bound at the first call and then takes the function's place in this module; the
-    decorated function stays behind it for the arguments the binding does not take and for the argument errors."""
+    decorated function stays behind it for the arguments the binding does not take and for the argument errors, and serves
+    every call where there is no binding: the same kernels, called through ctypes."""
     symbol = "rfk_" + checked.__name__
     op = None
 
@@ -71,9 +90,9 @@ def _native(checked):
         nonlocal op
         if op is None:
             _lib()   # raises if the libraries are not built
-            from . import _native as binding
+            binding = _binding()
             defaults = tuple(p.default for p in inspect.signature(checked).parameters.values() if p.default is not p.empty)
-            op = functools.update_wrapper(binding.bind(symbol, checked, _failed, defaults), checked)
+            op = functools.update_wrapper(binding.bind(symbol, checked, _failed, defaults), checked) if binding else checked
             globals()[checked.__name__] = op
         return op(*args, **kwargs)
 
