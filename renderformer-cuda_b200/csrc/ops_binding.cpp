@@ -156,6 +156,11 @@ void op_dealloc(PyObject* self) {
     Py_TYPE(self)->tp_free(self);
 }
 
+// An operator is copied and pickled as the module's function that it stands for: by name.
+PyObject* op_reduce(PyObject* self, PyObject*) { return PyObject_GetAttrString(self, "__qualname__"); }
+
+PyMethodDef op_methods[] = {{"__reduce__", op_reduce, METH_NOARGS, "the operator's name in its module"},
+                            {nullptr, nullptr, 0, nullptr}};
 PyMemberDef op_members[] = {
     {"__dictoffset__", T_PYSSIZET, offsetof(Op, dict), READONLY, nullptr},
     {"__vectorcalloffset__", T_PYSSIZET, offsetof(Op, vectorcall), READONLY, nullptr},
@@ -166,7 +171,7 @@ PyType_Slot op_slots[] = {
     {Py_tp_dealloc, reinterpret_cast<void*>(op_dealloc)}, {Py_tp_traverse, reinterpret_cast<void*>(op_traverse)},
     {Py_tp_clear, reinterpret_cast<void*>(op_clear)},     {Py_tp_call, reinterpret_cast<void*>(PyVectorcall_Call)},
     {Py_tp_members, op_members},                          {Py_tp_getset, op_getset},
-    {0, nullptr}};
+    {Py_tp_methods, op_methods},                          {0, nullptr}};
 PyType_Spec op_spec = {"rfk.Op", sizeof(Op), 0,
                        Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_HAVE_VECTORCALL | Py_TPFLAGS_DISALLOW_INSTANTIATION,
                        op_slots};

@@ -1,5 +1,8 @@
 """CPU tests of the operators' compiled binding: where it is missing or was built for another torch, the checked function behind
-an operator serves it (and its argument errors), and this is said once."""
+an operator serves it (and its argument errors), and this is said once. A bound operator is copied and pickled like the function
+it stands for."""
+import copy
+import pickle
 import sys
 import warnings
 
@@ -49,3 +52,13 @@ def test_binding_of_this_torch_is_used(unbound):
         warnings.simplefilter("error")
         _refused(unbound)
     assert type(ops.silu).__name__ == "Op"
+
+
+@pytest.mark.parametrize("bound", [False, True])
+def test_operators_are_copied_and_pickled_by_name(bound):
+    """A program keeps an operator in an object that it copies, or hands it to another process."""
+    if bound:
+        _refused(ops.silu)
+    assert (type(ops.silu).__name__ == "Op") >= bound
+    assert pickle.loads(pickle.dumps(ops.silu)) is ops.silu
+    assert copy.deepcopy({"act": ops.silu})["act"] is ops.silu and copy.copy(ops.silu) is ops.silu
