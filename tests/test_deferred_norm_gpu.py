@@ -103,12 +103,12 @@ def test_heads_projection_refuses_shapes_it_cannot_tile():
     assert e.value.status == -1
 
 
-@pytest.mark.parametrize("layers,heads,rows,pad", [(1, 12, 1537, 1600), (3, 4, 200, 256), (11, 6, 64, 64)])
-def test_rotation_with_folded_norm_weight(layers, heads, rows, pad):
+@pytest.mark.parametrize("layers,heads,rows,pad,hd", [(1, 12, 1537, 1600, 64), (3, 4, 200, 256, 64), (11, 6, 64, 64, 64),
+                                                      (1, 8, 1537, 1600, 128), (11, 2, 200, 208, 128)])
+def test_rotation_with_folded_norm_weight(layers, heads, rows, pad, hd):
     """dst[l] = half(rotate(src[l]) * gamma[l]) with one shared table: fp32 torch evaluation, half an fp16 step of
     slack for the fused multiply-add order."""
     o = _ops()
-    hd = 64
     g = torch.Generator(device="cuda").manual_seed(layers * 100 + rows)
     src = _rand(g, layers, 2, heads, pad, hd)                       # [layer][K|V][heads][rows][hd]: the key slabs
     ang = torch.rand(pad, hd // 2, device="cuda", generator=g) * 6.28
