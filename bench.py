@@ -428,7 +428,7 @@ def attention_roofline(n_tris, nr, heads, n_tokens, head_dim, views=1, iters=12)
     alg_bytes = 2 * (2 * V * heads * n_tokens * head_dim + (V + 1) * heads * Se_pad * head_dim)   # Q, O, K per view; V once
     del sets, ws
     torch.cuda.empty_cache()
-    name = "attention_tc_kernel (tcgen05)" if head_dim == 64 else f"flash_attention_kernel<{head_dim}> (mma.sync)"
+    name = "attention_tc_kernel (tcgen05)" if head_dim == 64 else f"attention_tc_kernel<{head_dim}> (tcgen05)"
     err = pkg.ops.flash_attention_error(clear=False)
     if err:
         raise RuntimeError(f"tcgen05 attention kernel reported error word {err}")

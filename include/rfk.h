@@ -264,7 +264,7 @@ int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
                         int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
                         rfk_stream_t stream);
 
-/* rfk_flash_attention with two optional extensions; tcgen05 kernel only (D = 64: RFK_EUNSUPPORTED otherwise).
+/* rfk_flash_attention with three optional extensions; tcgen05 kernel only, D = 64 (RFK_EUNSUPPORTED otherwise).
  * (1) Queries that come un-normalised out of rfk_gemm_f16_heads (q_row_ss != NULL): q_row_ss [B*Sq][ss_tiles] holds the
  * partial sums of squares of each token's whole projection row (all heads); the kernel multiplies a row's scores by
  * rsqrt(sum / norm_dim + eps), which is what normalising the query first would do up to rounding. The norm's
@@ -272,7 +272,8 @@ int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
  * (2) Key split (workspace != NULL): the kernel's units of work are 256 queries of one head; a grid with fewer units
  * than SMs (a 256 x 256 view has 64) leaves most of the machine idle, so with a workspace - and when the launcher's
  * estimate says it pays - the units' key ranges are cut into one share per SM and merged by the CTA that finishes a
- * unit last (nobody waits). workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
+ * unit last (nobody waits); of a larger grid the units of the last, partial round are, when that saves a fifth of the
+ * launch. Which units are cut, and with it the order of their sums, depends on B * H and Sq. workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
  * bytes zero before the first launch (the kernel leaves them zero); launches that may overlap in time need separate
  * workspaces. The result differs from the unsplit kernel's only by rounding (fp32 merge; fp16 probabilities relative to
  * each piece's own maximum) and is bit-reproducible from launch to launch.
@@ -294,9 +295,9 @@ int rfk_flash_attention_plan(long long units, int n_tiles, int sms, int* whole_u
  * it cuts where that pays. Process-wide. No reference counterpart. */
 int rfk_flash_attention_set_split(int on);
 
-/* Which kernel serves rfk_flash_attention at D = 64: 0 automatic (the tcgen05 / tensor-memory
- * kernel; the mma.sync kernel only if the driver cannot encode tensor maps), 1 the mma.sync kernel,
- * 2 the tcgen05 kernel or RFK_EUNSUPPORTED. Process-wide; D = 128 always takes the mma.sync kernel.
+/* Which kernel serves rfk_flash_attention: 0 automatic (the tcgen05 / tensor-memory kernel; the
+ * mma.sync kernel only if the driver cannot encode tensor maps), 1 the mma.sync kernel, 2 the tcgen05
+ * kernel or RFK_EUNSUPPORTED. Process-wide; at D = 128 both are equally far from the exact result.
  * No reference counterpart (the reference leaves the choice to cuDNN's heuristics,
  * src/layers/attention.cu:100-140). */
 int rfk_flash_attention_set_path(int path);

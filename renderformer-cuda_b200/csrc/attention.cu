@@ -21,8 +21,9 @@
 //     shuffles per tile;
 //   - the output tile is normalised, staged through shared memory and written with 128-bit
 //     stores, either [B,H,Sq,D] or directly [B,Sq,H*D] (what the output projection reads).
-// This is the portable tensor-core path (it also serves head_dim 128 and ragged lengths);
-// per layer it replaces 0.72 ms of GEMM + softmax + GEMM and 2.2 GB of score traffic.
+// This is the fallback of the tcgen05 kernel (attention_tc.cu), path 1, and the attention of sessions
+// with an image head and 128-wide heads (whose images keep the order of their sums); per layer it
+// replaces 0.72 ms of GEMM + softmax + GEMM and 2.2 GB of score traffic.
 #include "common.cuh"
 #include "kernels_internal.h"
 
@@ -564,15 +565,22 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
-int rfk::flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss,
-                            int ss_tiles, int norm_dim, float eps, void* workspace, size_t workspace_bytes, AttnCut cut,
-                            int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
-                            rfk_stream_t stream) {
+static int check_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, const rfk_half* O,
+                                    const float* q_row_ss, int ss_tiles, int norm_dim, const void* workspace,
+                                    size_t workspace_bytes, int B, int H, int Sq, int Sk, int n_keys, float scale) {
     if (!Q || !K || !V || !O || B < 0 || H <= 0 || Sq < 0 || Sk <= 0 || n_keys <= 0 || n_keys > Sk || !(scale > 0.0f))
         return RFK_EINVAL;
     if (q_row_ss && (ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
     if (workspace && workspace_bytes < attention_tc_workspace_bytes()) return RFK_EINVAL;
-    if (B == 0 || Sq == 0) return RFK_OK;
+    return RFK_OK;
+}
+
+int rfk::flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss,
+                            int ss_tiles, int norm_dim, float eps, void* workspace, size_t workspace_bytes, AttnCut cut,
+                            int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
+                            rfk_stream_t stream) {
+    const int rc = check_flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, workspace, workspace_bytes, B, H, Sq, Sk, n_keys, scale);
+    if (rc != RFK_OK || B == 0 || Sq == 0) return rc;
     if ((D != 64 && D != 128) || (long long)B * H > 65535 || g_attn_path.load(std::memory_order_relaxed) == 1) return RFK_EUNSUPPORTED;
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
     return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D, o_bshd,
@@ -588,14 +596,17 @@ extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K,
                               v_shared, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
-// The public form takes 64-wide heads, as its header says.
+// The public form takes 64-wide heads, as its header says (arguments are checked first: a bad one is RFK_EINVAL, an empty
+// problem a success at any head size).
 extern "C" int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
                                       const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
                                       size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
                                       int o_bshd, float scale, rfk_stream_t stream) {
-    const int rc = rfk_flash_attention_ex_wide(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, v_shared,
-                                               D == 64 || B < 0 ? B : 0, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
-    return rc == RFK_OK && D != 64 && B > 0 && Sq != 0 ? RFK_EUNSUPPORTED : rc;
+    const int rc = check_flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, workspace, workspace_bytes, B, H, Sq, Sk, n_keys, scale);
+    if (rc != RFK_OK || B == 0 || Sq == 0) return rc;
+    if (D != 64) return RFK_EUNSUPPORTED;
+    return flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, AttnCut::kLastRound,
+                              v_shared, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
 extern "C" size_t rfk_flash_attention_workspace_bytes(void) { return attention_tc_workspace_bytes(); }

@@ -1,4 +1,5 @@
-// Fused attention on the 5th-generation tensor cores (tcgen05 + tensor memory + TMA), head_dim 64.
+// Fused attention on the 5th-generation tensor cores (tcgen05 + tensor memory + TMA), head_dim 64 and 128 (sizes below: 64,
+// with 128 in brackets where it differs).
 //
 // Same function as flash_attention_kernel (attention.cu): O = softmax(scale * Q K^T) V over
 // the first n_keys keys, fp16 operands, fp32 accumulation, probabilities rounded to fp16.
@@ -10,10 +11,10 @@
 //   warp 8       producer: one thread issues TMA tile loads (both Q blocks once, then K and V tiles
 //                through a ring of kStages shared-memory stages); the copies land in the tensor
 //                core's 128-byte-swizzled layout and complete on mbarriers, no thread touches the bytes.
-//   warps 11-12  one thread per block issues S = Q K^T (tcgen05.mma M128 N64 K16 x 4) into one of
-//                the block's three score buffers in tensor memory, as soon as the P V product that
-//                read that buffer's previous contents is complete: the softmax warps find their
-//                next two tiles ready and never wait for a product.
+//   warps 11-12  one warp per block, whose elected lane issues S = Q K^T (tcgen05.mma M128 N64 K16
+//                x 4 [8]) into one of the block's three [two] score buffers in tensor memory, as
+//                soon as the P V product that read that buffer's previous contents is complete:
+//                the softmax warps find their next two [one] tiles ready.
 //   warps 0-7    softmax (block = warp / 4): a thread owns one query row = its tensor-memory lane,
 //                so row maximum and row sum are thread-local (no shuffles). The 64 scores come to
 //                registers with tcgen05.ld; the common tile exponentiates them against the running
@@ -22,17 +23,17 @@
 //                failed check and every tile of 128-wide heads); P = exp2(...) is rounded to fp16
 //                and stored back with tcgen05.st over the first 32 columns of the same score
 //                buffer, from where
-//   warps 9-10   one thread per block issues O += P V with P as the A operand from tensor memory
-//                and V (MN-major) from shared memory: P never passes through shared memory. The
-//                output accumulator O (128 x 64 fp32 per block) is rescaled in place only when a
+//   warps 9-10   one warp per block, whose elected lane issues O += P V with P as the A operand
+//                from tensor memory and V (MN-major) from shared memory: P never passes through
+//                shared memory. The output accumulator O (128 x 64 [128] fp32 per block) is rescaled in place only when a
 //                row's running maximum has grown by more than 2^8 (the factor cancels in O / l; at
 //                all with 128-wide heads).
 // A stage of the ring is free again when both blocks' P V products of its tile are complete
-// (kv_empty counts two arrivals). The products have separate issuing threads because one thread's
+// (kv_empty counts two arrivals). The products have separate issuing warps because one warp's
 // instruction stream (8 products, 3 commits and 2-3 waits per tile, all dependent) takes about as
 // long as the softmax of a tile; the order between them is kept by mbarriers, not by issue order.
-// Tensor memory: all 512 columns (per block S0, S1, S2, O: 64 each); shared memory 32 KB (Q) +
-// kStages x 16 KB; one CTA per SM. Every mbarrier wait is bounded; on a time-out the CTA raises an
+// Tensor memory: all 512 columns (per block S0, S1, S2, O: 64 each [S0, S1: 64, O: 128]); shared
+// memory 32 [64] KB (Q) + 6 x 16 KB [4 x 32 KB]; one CTA per SM. Every mbarrier wait is bounded; on a time-out the CTA raises an
 // error word, frees its tensor memory and returns.
 //
 // Key split for grids that do not fill the machine. A unit = 256 queries of one head over all keys = one CTA. With few
@@ -83,7 +84,7 @@ constexpr int kMaxStages = 6, kMaxSBufs = 3;
 struct __align__(8) Ctrl {
     uint64_t q_full, kv_full[kMaxStages], kv_empty[kMaxStages], s_full[kBlocks][kMaxSBufs], p_full[kBlocks][kMaxSBufs],
         pv_done[kBlocks][kMaxSBufs];
-    uint64_t drain[2 * kBlocks];  // abort path only, one per issuing thread: completes once that thread's products have finished
+    uint64_t drain[2 * kBlocks];  // abort path only, one per issuing lane: completes once that lane's products have finished
     uint32_t tmem_base;
     int abort;
     int merge;  // set by thread 0 of a split unit's last piece: this CTA merges the unit
@@ -104,7 +105,7 @@ struct WorkList {
     Piece pieces[kMaxPieces];
 };
 // Workspace: 256 counters (one per split unit, zero between launches), then per slot 256 x {m, l}, then per slot the
-// un-normalised output as [16 groups of 4 columns][256 rows] float4 (a warp's 32 rows of one group are contiguous).
+// un-normalised output as [16 or 32 groups of 4 columns][256 rows] float4 (a warp's 32 rows of one group are contiguous).
 constexpr int kUnitRows = kBlocks * BM;
 constexpr size_t kWsCounterBytes = 1024;
 constexpr size_t kWsMlBytes = (size_t)kMaxPieces * kUnitRows * 2 * sizeof(float);
@@ -613,7 +614,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
 }  // namespace tcattn
 
-std::atomic<int> g_attn_path{0};  // 0 automatic, 1 mma.sync kernel, 2 tcgen05 kernel (head_dim 64 only)
+std::atomic<int> g_attn_path{0};  // 0 automatic, 1 mma.sync kernel, 2 tcgen05 kernel
 std::atomic<int> g_attn_split{1};  // 0: never split keys, even with a workspace (to time both side by side)
 
 namespace {

@@ -371,7 +371,7 @@ def window_attention_normed(q, k, v, o, mask, q_row_ss, k_row_ss, ss_tiles, gamm
 
 
 def flash_attention_set_path(path):
-    """0 automatic, 1 mma.sync kernel, 2 tcgen05 kernel (head_dim 64)."""
+    """0 automatic, 1 mma.sync kernel, 2 tcgen05 kernel."""
     _call("rfk_flash_attention_set_path", int(path))
 
 
