@@ -162,7 +162,7 @@ __device__ __forceinline__ float2 exp2_poly(float2 x) {
 // special-function unit (16 exponentials per clock and SM) is the scarcest resource of this kernel, so of every four
 // pairs those selected by the mask take the polynomial path instead. With 128-wide heads there are half as many
 // exponentials per product and every one comes from the special-function unit, as in flash_attention_kernel (the
-// polynomial was 5 us of 95 on 8 x 4096 x 5665, and 0.4 % of the result's distance from 64 bits).
+// polynomial was worth 5 % of the kernel's time while the reference trailed, for 0.4 % of the result's distance from 64 bits).
 #ifndef RFK_ATTN_POLY_MASK
 #define RFK_ATTN_POLY_MASK 0x1
 #endif
@@ -332,8 +332,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const uint32_t tmem = tmem_cta + blk * 256, tmem_O = tmem + kSBufs * 64;
         // ------------------------------------------------------------ issuer of O += P V (the warp's elected lane)
         // The whole warp runs the loop and one lane issues (elect_one): with a single thread's loop the issue of a tile's
-        // products, not the tensor pipe, paced the 128-wide heads (8 x 4096 x 5665: 96 -> 84 us, 1.13 PFLOP/s; with 64-wide
-        // heads, which the softmax warps pace, 142 -> 139 us).
+        // products, not the tensor pipe, paced the 128-wide heads (8 x 4096 x 5665: 96 -> 84 us with the trailing reference they
+        // had then; with the exact one the softmax warps pace them, 105 us = 0.91 PFLOP/s; 64-wide heads 142 -> 139 us).
         // tile j: score buffer j % kSBufs (its use number j / kSBufs gives the barrier phase), ring stage j % kStages
         const bool leader = tc::elect_one();
         constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
@@ -403,7 +403,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // maximum, as in flash_attention_kernel: a row's largest probabilities are then exactly 1 or round on the finer half
         // of their binade. Against 64 bits the deferred reference was 3 % further off than that kernel on unit-variance
         // scores and 19 to 21 % on scores of two and three times that; with the exact one the two agree to 1e-4 (8 x 4096 x
-        // 5665: 95 us deferred, 115 us exact, 362 us flash_attention_kernel).
+        // 5665: 81 us deferred, 105 us exact, 361 us flash_attention_kernel).
         constexpr bool kExactMax = HD == 128;
         constexpr float kRescaleThreshold = kExactMax ? 0.0f : 8.0f;
         const int blk = warp >> 2;
@@ -667,7 +667,8 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     const int shares = (int)std::min<long long>(std::min(sms, tcattn::kMaxPieces / 2), (long long)rest * kMaxPiecesPerUnit);
     // whole: one more round of n_tiles; split: a share's tiles plus the piece overhead. Cut only for a clear gain: a fifth of
     // the launch. (Measured where the estimate gives 7 %, 256 units of 89 tiles on 148 SMs: nothing gained. 184 units of 89
-    // tiles, estimate 31 %: 187 -> 143 us at head size 128; 208 units, estimate 23 %: 141 -> 116 us at head size 64.)
+    // tiles, estimate 31 %: 200 -> 153 us at head size 128; 208 units, estimate 23 %: 139 -> 114 us and 160 units of 40 tiles,
+    // 29 %: 68 -> 52 us at head size 64.)
     if (((long long)rounds * n_tiles + (tiles + shares - 1) / shares + kPieceCostTiles) * 5 > (long long)(rounds + 1) * n_tiles * 4) return;
     const int whole = rounds * sms;
     Piece* pc = w.pieces;

@@ -338,7 +338,8 @@ static int cross_attention_impl(rfk_ctx* ctx, const rfk_cross_attn_weights* w,
                 K_use = K_rot;
             }
             // With 64-wide heads a view is rendered alone or in a frame of several and must have the same bits: a view alone
-            // that fills the SMs (208 units at 448 x 448) stays whole, as it is among the units of a frame. 128-wide heads have
+            // that fills the SMs (208 units at 448 x 448) stays whole, as it is among the units of a frame (139 us where the cut
+            // would take 114). 128-wide heads have
             // no such frames.
             if (rc == RFK_OK)
                 rc = rfk::flash_attention_ex(Q_bhsd, K_use, V_cached, Q, norm_ss, dim / 256, dim, kEpsFp16, ctx->attn_ws,
