@@ -399,6 +399,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         constexpr unsigned kFull = 0xffffffffu;
         constexpr float kSumLimit = 256.0f;  // 2^8, the threshold below
         constexpr uint32_t kNegInf = 0xff800000u;
+        constexpr float kNoMax = -1.0e30f;  // a score is at most 65504^2 * HD
         // In exponent units: P stays below 2^8, well inside fp16. With 128-wide heads the reference is the row's exact running
         // maximum, as in flash_attention_kernel: a row's largest probabilities are then exactly 1 or round on the finer half
         // of their binade. Against 64 bits the deferred reference was 3 % further off than that kernel on unit-variance
@@ -450,7 +451,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // 2^threshold, none of them exceeded it and the tile is done. Otherwise (and for the first and the last
             // tile) the scores are read again, the maximum is taken and the same code runs once more.
             float2 acc0, acc1;
-            float m_new = m_run, m_ref = m_run, alpha = 1.0f;
+            float m_new = m_run, alpha = 1.0f;
             bool any_move = false, need_max = kExactMax || j == 0 || n_valid != BN;
 #pragma unroll 1
             for (;;) {
@@ -468,14 +469,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     }
                     const float m_tile = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
                     const bool move = (m_tile - m_run) * scale_log2e > kRescaleThreshold;  // first tile: m_run = -inf
-                    m_new = move ? m_tile : m_run;
-                    m_ref = m_new == -INFINITY ? 0.0f : m_new;  // every score of the row so far is -inf: P = 0, no difference of infinities
+                    // A row whose scores so far are all -inf has no maximum: a reference far below every finite score, and
+                    // still finite, makes their P 0 instead of the exponential of a difference of infinities; the first
+                    // finite score fails the check below and moves it.
+                    m_new = fmaxf(move ? m_tile : m_run, kNoMax);
                     any_move = __any_sync(kFull, move);
                     if (any_move && move) alpha = fast_exp2((m_run - m_new) * scale_log2e);  // first tile: 0
                 }
                 // P = exp2(scale * log2e * (S - max)), two fp16 per 32-bit column: keys 2i, 2i+1 in column i;
                 // the 32 packed words end up in va, which is what the store below takes
-                const float mc = m_ref * scale_log2e;
+                const float mc = m_new * scale_log2e;
                 float poly_max = -INFINITY;
                 exp_half<HD>(va, va, scale_log2e, mc, acc0, acc1, poly_max);
                 tc::tc_wait_ld(vb);
@@ -569,7 +572,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 float m_all = -INFINITY;
                 for (int p = 0; p < split_count; ++p)
                     m_all = fmaxf(m_all, __ldcg(ws_ml + ((size_t)(split_first + p) * kUnitRows + row) * 2));
-                if (m_all == -INFINITY) m_all = 0.0f;  // a row without a finite score: every weight below is 0, as is the output
                 float l_all = 0.0f;
                 for (int p = 0; p < split_count; ++p) {  // in slot order, whichever CTA merges: the sum is reproducible
                     const float2 ml = __ldcg(reinterpret_cast<const float2*>(ws_ml + ((size_t)(split_first + p) * kUnitRows + row) * 2));

@@ -156,3 +156,21 @@ def test_keys_with_a_score_of_minus_infinity(n_out, split):
     _close(O, M, "keys at -inf")
     if n_out == Sk:
         assert not O[:, 0].any()
+
+
+@pytest.mark.parametrize("n_out", [64, 640, 1024])
+def test_keys_with_a_score_of_minus_infinity_on_64_wide_heads(n_out):
+    """The same in the kernel's other form, whose common tile does not take the maximum first."""
+    g = torch.Generator(device="cuda").manual_seed(n_out)
+    Q, K, V = (torch.randn(1, 2, n, 64, device="cuda", generator=g).half() for n in (130, 1024, 1024))
+    Q[..., -1] = 1.0
+    K[..., -1] = 0.0
+    K[:, 0, :n_out, -1] = -float("inf")
+    outs = []
+    for path in (2, 1):
+        pkg.ops.flash_attention_set_path(path)
+        outs.append(torch.full_like(Q, 7.0))
+        pkg.ops.flash_attention(Q, K, V, outs[-1], 1, 2, 130, 1024, 1024, 64)
+    assert torch.isfinite(outs[1].float()).all()
+    _close(outs[0], outs[1], "keys at -inf")
+    assert n_out < 1024 or not outs[0][:, 0].any()
