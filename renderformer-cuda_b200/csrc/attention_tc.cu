@@ -333,7 +333,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // ------------------------------------------------------------ issuer of O += P V (the warp's elected lane)
         // The whole warp runs the loop and one lane issues (elect_one): with a single thread's loop the issue of a tile's
         // products, not the tensor pipe, paced the 128-wide heads (8 x 4096 x 5665: 96 -> 84 us with the trailing reference they
-        // had then; with the exact one the softmax warps pace them, 105 us = 0.91 PFLOP/s; 64-wide heads 142 -> 139 us).
+        // had then; with the exact one the softmax warps pace them, 102 us = 0.93 PFLOP/s; 64-wide heads 142 -> 139 us).
         // tile j: score buffer j % kSBufs (its use number j / kSBufs gives the barrier phase), ring stage j % kStages
         const bool leader = tc::elect_one();
         constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
@@ -399,12 +399,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         constexpr unsigned kFull = 0xffffffffu;
         constexpr float kSumLimit = 256.0f;  // 2^8, the threshold below
         constexpr uint32_t kNegInf = 0xff800000u;
-        constexpr float kNoMax = -1.0e30f;  // a score is at most 65504^2 * HD
+        // The reference ahead of a row's first finite score: far below every such score (at most 65504^2 * HD), so that the
+        // first one moves it, and finite, so that scores of -inf give P = 0 and not the exponential of a difference of
+        // infinities.
+        constexpr float kNoMax = -1.0e30f;
         // In exponent units: P stays below 2^8, well inside fp16. With 128-wide heads the reference is the row's exact running
         // maximum, as in flash_attention_kernel: a row's largest probabilities are then exactly 1 or round on the finer half
         // of their binade. Against 64 bits the deferred reference was 3 % further off than that kernel on unit-variance
         // scores and 19 to 21 % on scores of two and three times that; with the exact one the two agree to 1e-4 (8 x 4096 x
-        // 5665: 81 us deferred, 105 us exact, 361 us flash_attention_kernel).
+        // 5665: 81 us deferred, 102 us exact, 361 us flash_attention_kernel).
         constexpr bool kExactMax = HD == 128;
         constexpr float kRescaleThreshold = kExactMax ? 0.0f : 8.0f;
         const int blk = warp >> 2;
@@ -423,7 +426,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int t = 0; t < ss_tiles; ++t) ss += __ldg(sp + t);
             scale_log2e *= rsqrtf(ss * inv_norm_dim + norm_eps);
         }
-        float m_run = -INFINITY, l_run = 0.0f;
+        float m_run = kNoMax, l_run = 0.0f;
         uint32_t va[32], vb[32];
         bool ok = true;
         int buf = 0, buf_par = 0;  // score buffer of tile j and the phase parity of its barriers
@@ -468,11 +471,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         m3 = fmax3(m3, __uint_as_float(vb[i + 2]), __uint_as_float(vb[i + 3]));
                     }
                     const float m_tile = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-                    const bool move = (m_tile - m_run) * scale_log2e > kRescaleThreshold;  // first tile: m_run = -inf
-                    // A row whose scores so far are all -inf has no maximum: a reference far below every finite score, and
-                    // still finite, makes their P 0 instead of the exponential of a difference of infinities; the first
-                    // finite score fails the check below and moves it.
-                    m_new = fmaxf(move ? m_tile : m_run, kNoMax);
+                    const bool move = (m_tile - m_run) * scale_log2e > kRescaleThreshold;  // first tile: always, with a finite score
+                    m_new = move ? m_tile : m_run;
                     any_move = __any_sync(kFull, move);
                     if (any_move && move) alpha = fast_exp2((m_run - m_new) * scale_log2e);  // first tile: 0
                 }
