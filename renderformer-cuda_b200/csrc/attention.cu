@@ -21,8 +21,7 @@
 //     shuffles per tile;
 //   - the output tile is normalised, staged through shared memory and written with 128-bit
 //     stores, either [B,H,Sq,D] or directly [B,Sq,H*D] (what the output projection reads).
-// This is the fallback of the tcgen05 kernel (attention_tc.cu), path 1, and the attention of sessions
-// with an image head and 128-wide heads (whose images keep the order of their sums); per layer it
+// This is the fallback of the tcgen05 kernel (attention_tc.cu), path 1; per layer it
 // replaces 0.72 ms of GEMM + softmax + GEMM and 2.2 GB of score traffic.
 #include "common.cuh"
 #include "kernels_internal.h"
@@ -530,7 +529,7 @@ size_t attention_tc_workspace_bytes();
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared);
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared);
 
 }  // namespace rfk
 
@@ -559,7 +558,8 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     const int path = g_attn_path.load(std::memory_order_relaxed);
     if ((D == 64 || D == 128) && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
         const int rc = launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk,
-                                           n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0, false, 0);
+                                           n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0,
+                                           AttnCut::kLastRound, 0);
         if (rc != RFK_EUNSUPPORTED || path == 2) return rc;
     }
     return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
@@ -585,7 +585,7 @@ int rfk::flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
     return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D, o_bshd,
                                scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes,
-                               cut == AttnCut::kLastRound, v_shared != 0);
+                               cut, v_shared != 0);
 }
 
 extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
@@ -594,6 +594,11 @@ extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K,
                                            int o_bshd, float scale, rfk_stream_t stream) {
     return flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes, AttnCut::kLastRound,
                               v_shared, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
+}
+
+extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq,
+                                           int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream) {
+    return flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, nullptr, 0, AttnCut::kNone, 0, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
 }
 
 // The public form takes 64-wide heads, as its header says (arguments are checked first: a bad one is RFK_EINVAL, an empty

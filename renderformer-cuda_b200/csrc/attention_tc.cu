@@ -44,11 +44,19 @@
 // complete (no CTA ever waits for another) merges the unit's pieces, writes the output and zeroes the counter for the
 // next launch. A piece costs about 10 us beyond its tiles (pipeline fill, publishing, merging), so the last, partial
 // round of a larger grid is cut the same way only when few units are left for it (plan_work).
+//
+// One block per CTA. Two blocks share a CTA so that they share the K/V tiles; their softmax warps then share the SM's
+// schedulers and special-function unit (a tile of one block alone takes 1020 clocks, of two together 1410, 64-wide heads).
+// Where all blocks of 128 queries find an SM of their own, each gets one (BLOCKS = 1): 16 x 576 x 4607, 48 units of 256 queries,
+// 62 -> 47 us; 16 x 1100 x 5665 72 -> 53 us; 8 x 1600 x 4607 x 128 84 -> 62 us. Past that line the blocks without an SM would be
+// a second round, and two rounds of one block take longer than one round of two (2 x 1020 against 1410).
+// A row's arithmetic does not depend on its block's company: both forms have the same bits.
 #include <algorithm>
 #include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
 #define RFK_TC_WAIT_INLINE  // this kernel re-partitions its registers (setmaxnreg)
 #include "attention_tc.cuh"
 #include "common.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -57,7 +65,7 @@ __device__ int g_attn_tc_error = 0;  // first time-out / failure code seen by an
 namespace tcattn {
 
 constexpr int BM = 128, BN = 64;
-constexpr int kBlocks = 2;                     // 128-query blocks per CTA, sharing the K/V ring
+constexpr int kBlocks = 2;                     // 128-query blocks per CTA, sharing the K/V ring (at most; see "One block per CTA")
 constexpr int kThreads = 512;                  // warps 0-7 softmax (block = warp / 4), 8 producer, 9-10 PV, 11-12 QK issuers, 13-15 none
 // Registers: the CTA starts with 128 per thread. The two warpgroups that only issue copies and products (warps 8-15)
 // hand theirs back down to kRegsIssue and the softmax warpgroups (warps 0-7) grow to kRegsSoftmax, which lets the
@@ -67,16 +75,17 @@ constexpr int kRegsIssue = 40, kRegsSoftmax = 216;
 constexpr int kTmemCols = 512;                 // 256 per block: the score buffers (64 columns each), then O
 // Per head size. A row of the operand tiles is HD / 64 swizzle rows of 128 bytes: the tiles are kept as HD / 64
 // sub-tiles of 64 columns, each fetched by its own TMA box.
-template <int HD> struct Cfg {
+template <int HD, int BLOCKS> struct Cfg {
     static constexpr int kSub = HD / 64;
     static constexpr int kQSub = BM * 128, kQBytes = kSub * kQSub;     // 16 KB per 64 columns
     static constexpr int kKSub = BN * 128, kKBytes = kSub * kKSub;     // 8 KB per 64 columns; a stage is K then V
     static constexpr int kStageBytes = 2 * kKBytes;
-    static constexpr int kStages = HD == 64 ? 6 : 4;
-    // O takes HD of a block's 256 tensor-memory columns, score buffers the rest: three at 64, two at 128
-    static constexpr int kSBufs = (256 - HD) / 64;
+    static constexpr int kStages = HD == 64 || BLOCKS == 1 ? 6 : 4;
+    // O takes HD of a block's 256 tensor-memory columns, score buffers the rest: three at 64, two at 128; a block that has the
+    // CTA to itself always has three
+    static constexpr int kSBufs = BLOCKS == 1 ? 3 : (256 - HD) / 64;
     // The shared-memory window is declared 1024-byte aligned (swizzled tiles need it) and the kernel checks it.
-    static constexpr int kSmemBytes = kBlocks * kQBytes + kStages * kStageBytes + 512;
+    static constexpr int kSmemBytes = BLOCKS * kQBytes + kStages * kStageBytes + 512;
     static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
 };
 constexpr int kMaxStages = 6, kMaxSBufs = 3;
@@ -157,7 +166,8 @@ __device__ __forceinline__ float2 exp2_poly(float2 x) {
 }
 
 // 32 raw scores -> 32 probabilities exp2(s * c - mc), packed two fp16 per word into pk[0..16); their
-// fp32 sums are added to acc0 / acc1 (two lanes each).
+// fp32 sums are added to acc0 / acc1 (two lanes each). ORDERED: the four lanes are the partial sums of the four threads that
+// share a row in flash_attention_kernel (columns 8n + 2t and 8n + 2t + 1, in that order), so that the row sum has its bits.
 // Packed fp32x2 multiply-adds and adds halve the instruction count around the exponentials. With 64-wide heads the
 // special-function unit (16 exponentials per clock and SM) is the scarcest resource of this kernel, so of every four
 // pairs those selected by the mask take the polynomial path instead. With 128-wide heads there are half as many
@@ -172,7 +182,7 @@ __device__ __forceinline__ float2 exp2_poly(float2 x) {
 template <int HD> constexpr int kPolyMask = HD == 64 ? RFK_ATTN_POLY_MASK : 0;
 template <int HD> __device__ __forceinline__ constexpr bool poly_pair(int pair) { return (kPolyMask<HD> >> (pair % RFK_ATTN_POLY_PERIOD)) & 1; }
 
-template <int HD>
+template <int HD, bool ORDERED>
 __device__ __forceinline__ void exp_half(uint32_t (&v)[32], uint32_t* pk /* may alias v */, float c, float mc, float2& acc0,
                                          float2& acc1, float& poly_max) {
     const float2 c2 = make_float2(c, c), nm2 = make_float2(-mc, -mc);
@@ -200,6 +210,19 @@ __device__ __forceinline__ void exp_half(uint32_t (&v)[32], uint32_t* pk /* may 
                 v[i + 1] = __float_as_uint(p.y);
             }
         }
+    }
+    if (ORDERED) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+            float e[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) e[j] = __uint_as_float(v[i + j]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) pk[(i >> 1) + j] = pack_half2(e[2 * j], e[2 * j + 1]);
+            acc0 = __fadd2_rn(acc0, __fadd2_rn(make_float2(e[0], e[2]), make_float2(e[1], e[3])));
+            acc1 = __fadd2_rn(acc1, __fadd2_rn(make_float2(e[4], e[6]), make_float2(e[5], e[7])));
+        }
+        return;
     }
     // four independent chains of packed adds (with two, the adds of a half waited on each other: -3 % with four), the
     // packing written ahead of the adds (the compiler keeps this order; -1 %)
@@ -236,13 +259,18 @@ __device__ __forceinline__ void store_row_half(__half* dst, const uint32_t (&v)[
     }
 }
 
-template <int HD>
+// ORDERED (128-wide heads): the row sums in the order of flash_attention_kernel. The products of both kernels sum in the same
+// order (mma.sync and tcgen05.mma add 16 products at a time, with the same bits, which the tests compare), the running maximum is
+// exact in both, so that whole units then have the bits of that kernel at a third of its time: 8 x 1600 x 4607 148 -> 62 us (one
+// block per CTA), 8 x 4096 x 5665 363 -> 105 us. It costs 2 %: the packed sums follow the register pairs of the exponents otherwise.
+template <int HD, int BLOCKS, bool ORDERED>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, __half* __restrict__ O, int H, int Sq, int n_keys,
                     int o_bshd, float scale_log2e_all, const float* __restrict__ row_ss, int ss_tiles, float inv_norm_dim,
                     float norm_eps, unsigned char* __restrict__ ws, int v_heads, const __grid_constant__ WorkList work) {
-    using C = Cfg<HD>;
+    using C = Cfg<HD, BLOCKS>;
+    constexpr int kRows = BLOCKS * BM;  // queries of a unit
     constexpr int kStages = C::kStages, kSBufs = C::kSBufs, kQBytes = C::kQBytes, kKBytes = C::kKBytes, kStageBytes = C::kStageBytes;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = tc::smem_addr(smem_raw);
@@ -250,8 +278,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (threadIdx.x == 0) atomicCAS(&g_attn_tc_error, 0, kErrSmemAlign);
         return;
     }
-    const uint32_t sQ = base, sKV = base + kBlocks * kQBytes;
-    Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + kBlocks * kQBytes + kStages * kStageBytes);
+    const uint32_t sQ = base, sKV = base + BLOCKS * kQBytes;
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + BLOCKS * kQBytes + kStages * kStageBytes);
     volatile int* abort_flag = &ctrl->abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -261,17 +289,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const Piece& pc = work.pieces[blockIdx.x - work.whole_units];
         unit = pc.unit; t0 = pc.t0; n_tiles = pc.nt; split_count = pc.count; split_first = pc.first; split_slot = pc.slot;
     }
-    const int q0 = (unit % work.q_blocks) * kUnitRows;
+    const int q0 = (unit % work.q_blocks) * kRows;
     const int bh = unit / work.q_blocks;
 
     if (tid == 0) {
         tc::mbar_init(&ctrl->q_full, 1);
-        for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->kv_full[s], 1); tc::mbar_init(&ctrl->kv_empty[s], kBlocks); }
-        for (int k = 0; k < kBlocks; ++k)
+        for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->kv_full[s], 1); tc::mbar_init(&ctrl->kv_empty[s], BLOCKS); }
+        for (int k = 0; k < BLOCKS; ++k)
             for (int b = 0; b < kSBufs; ++b) {
                 tc::mbar_init(&ctrl->s_full[k][b], 1); tc::mbar_init(&ctrl->p_full[k][b], 4); tc::mbar_init(&ctrl->pv_done[k][b], 1);
             }
-        for (int k = 0; k < 2 * kBlocks; ++k) tc::mbar_init(&ctrl->drain[k], 1);
+        for (int k = 0; k < 2 * BLOCKS; ++k) tc::mbar_init(&ctrl->drain[k], 1);
         ctrl->abort = 0;
         ctrl->merge = 0;
         tc::fence_barrier_init();
@@ -291,14 +319,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // The register hand-over: every warp of a warpgroup executes the same setmaxnreg instruction (warpgroups 2 and 3 the
     // release, 0 and 1 the take), as the first statement of a branch that does not meet the other again before the
     // teardown - placed ahead of the branch, the compiler bound every role by the smaller budget.
-    if (warp >= 8) {
+    if (warp >= 4 * BLOCKS) {
     regs_release();
     if (warp == 8) {
         // ------------------------------------------------------------ producer (one thread)
         if (lane == 0) {
             tc::prefetch_tensormap(&map_q); tc::prefetch_tensormap(&map_k); tc::prefetch_tensormap(&map_v);
-            tc::mbar_arrive_expect_tx(&ctrl->q_full, kBlocks * kQBytes);
-            for (int k = 0; k < kBlocks; ++k)
+            tc::mbar_arrive_expect_tx(&ctrl->q_full, BLOCKS * kQBytes);
+            for (int k = 0; k < BLOCKS; ++k)
                 for (int x = 0; x < C::kSub; ++x)
                     tc::tma_load_3d(sQ + k * kQBytes + x * C::kQSub, &map_q, x * 64, q0 + k * BM, bh, &ctrl->q_full);
             int issued = 0;
@@ -327,7 +355,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
         }
         __syncwarp();
-    } else if (warp == 9 || warp == 10) {
+    } else if (warp == 9 || (BLOCKS == 2 && warp == 10)) {
         const int blk = warp - 9;
         const uint32_t tmem = tmem_cta + blk * 256, tmem_O = tmem + kSBufs * 64;
         // ------------------------------------------------------------ issuer of O += P V (the warp's elected lane)
@@ -361,7 +389,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tc::mbar_wait_drain(&ctrl->drain[blk], 0);
         }
         __syncwarp();
-    } else if (warp == 11 || warp == 12) {
+    } else if (warp == 11 || (BLOCKS == 2 && warp == 12)) {
         const int blk = warp - 11;
         const uint32_t tmem = tmem_cta + blk * 256;
         // ------------------------------------------------------------ issuer of S = Q K^T (the warp's elected lane)
@@ -388,8 +416,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (++st == kStages) { st = 0; st_par ^= 1; }
         }
         if (leader && *abort_flag) {
-            tc::umma_commit(&ctrl->drain[kBlocks + blk]);
-            tc::mbar_wait_drain(&ctrl->drain[kBlocks + blk], 0);
+            tc::umma_commit(&ctrl->drain[BLOCKS + blk]);
+            tc::mbar_wait_drain(&ctrl->drain[BLOCKS + blk], 0);
         }
         __syncwarp();
     }  // warps 13-15 have no role beyond handing their registers back together with warp 12
@@ -427,6 +455,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             scale_log2e *= rsqrtf(ss * inv_norm_dim + norm_eps);
         }
         float m_run = kNoMax, l_run = 0.0f;
+        float2 l01 = make_float2(0.0f, 0.0f), l23 = l01;  // ORDERED: the row sum in its four parts (exp_half)
         uint32_t va[32], vb[32];
         bool ok = true;
         int buf = 0, buf_par = 0;  // score buffer of tile j and the phase parity of its barriers
@@ -471,7 +500,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         m3 = fmax3(m3, __uint_as_float(vb[i + 2]), __uint_as_float(vb[i + 3]));
                     }
                     const float m_tile = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-                    const bool move = (m_tile - m_run) * scale_log2e > kRescaleThreshold;  // first tile: always, with a finite score
+                    // first tile: always, with a finite score
+                    const bool move = kExactMax ? m_tile > m_run : (m_tile - m_run) * scale_log2e > kRescaleThreshold;
                     m_new = move ? m_tile : m_run;
                     any_move = __any_sync(kFull, move);
                     if (any_move && move) alpha = fast_exp2((m_run - m_new) * scale_log2e);  // first tile: 0
@@ -480,9 +510,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 // the 32 packed words end up in va, which is what the store below takes
                 const float mc = m_new * scale_log2e;
                 float poly_max = -INFINITY;
-                exp_half<HD>(va, va, scale_log2e, mc, acc0, acc1, poly_max);
+                exp_half<HD, ORDERED>(va, va, scale_log2e, mc, acc0, acc1, poly_max);
                 tc::tc_wait_ld(vb);
-                exp_half<HD>(vb, va + 16, scale_log2e, mc, acc0, acc1, poly_max);
+                exp_half<HD, ORDERED>(vb, va + 16, scale_log2e, mc, acc0, acc1, poly_max);
                 if (need_max) break;
                 const float sum = (acc0.x + acc0.y) + (acc1.x + acc1.y);
                 if (!__any_sync(kFull, !(sum <= kSumLimit) || poly_max > kRescaleThreshold)) break;
@@ -507,7 +537,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     tc::tmem_st32(tO + hc * 32, vb);
                 }
             }
-            l_run = (any_move ? l_run * alpha : l_run) + ((acc0.x + acc0.y) + (acc1.x + acc1.y));
+            if (ORDERED) {
+                const float2 a2 = make_float2(alpha, alpha);
+                l01 = __ffma2_rn(l01, a2, acc0);
+                l23 = __ffma2_rn(l23, a2, acc1);
+            } else {
+                l_run = (any_move ? l_run * alpha : l_run) + ((acc0.x + acc0.y) + (acc1.x + acc1.y));
+            }
             m_run = m_new;
             tc::tmem_st32(tS, va);    // P over the first 32 columns of this thread's own lane of S
             tc::tc_wait_st();
@@ -516,6 +552,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (lane == 0) tc::mbar_arrive(&ctrl->p_full[blk][buf]);
             if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
         }
+        if (ORDERED) l_run = (l01.x + l01.y) + (l23.x + l23.y);
         // ---- epilogue: O / l -> fp16 -> global, one 128-byte row per thread
         if (ok) {  // buf / buf_par have moved on to tile n_tiles: step back to the last tile
             const int lbuf = buf == 0 ? kSBufs - 1 : buf - 1, lbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;
@@ -523,7 +560,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         const int q = q0 + blk * BM + r;
         __half* dst = o_bshd ? O + (((size_t)(bh / H) * Sq + q) * H + bh % H) * HD : O + ((size_t)bh * Sq + q) * HD;
-        if (split_count == 1) {
+        if (BLOCKS == 1 || split_count == 1) {
             if (ok) {
                 tc::tc_fence_after();
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
@@ -700,6 +737,10 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     w.n_pieces = n;
 }
 
+// Whether a grid without cut units runs with one block of 128 queries per CTA (see "One block per CTA" above): when each block
+// finds an SM of its own.
+bool one_block_per_cta(int n_pieces, long long blocks, int sms) { return n_pieces == 0 && blocks <= sms; }
+
 }  // namespace
 
 size_t attention_tc_workspace_bytes() { return tcattn::kWsBytes; }
@@ -720,28 +761,41 @@ int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, i
 }
 
 namespace {
-template <int HD>
-int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
-              int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-              int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared) {
+template <int HD, int BLOCKS, bool ORDERED>
+int launch_units(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, __half* O, int H, int Sq, int n_keys, int o_bshd,
+                 float scale, cudaStream_t st, const float* row_ss, int ss_tiles, int norm_dim, float norm_eps, void* ws, int v_heads,
+                 const tcattn::WorkList& work, int dev) {
+    constexpr auto kernel = tcattn::attention_tc_kernel<HD, BLOCKS, ORDERED>;
+    constexpr int smem = tcattn::Cfg<HD, BLOCKS>::kSmemBytes;
     // per-device "kernel attributes set" marks; setting them twice from racing threads is harmless
     static std::atomic<bool> configured[64];
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return (int)e;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    launch_pdl(kernel, dim3((unsigned)(work.whole_units + work.n_pieces)), dim3(tcattn::kThreads), smem, st, mq, mk, mv, O, H, Sq, n_keys,
+               o_bshd, scale * 1.4426950408889634f, row_ss, ss_tiles, norm_dim > 0 ? 1.0f / (float)norm_dim : 0.0f, norm_eps,
+               static_cast<unsigned char*>(ws), v_heads, work);
+    return launch_status();
+}
+
+template <int HD, bool ORDERED>
+int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
+              int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
+              int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared) {
     static std::atomic<int> sm_count[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
-    constexpr auto kernel = tcattn::attention_tc_kernel<HD>;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcattn::Cfg<HD>::kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return (int)e;
-        int sms = 0;
+    int sms = sm_count[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return (int)e;
         sm_count[dev].store(sms, std::memory_order_relaxed);
-        configured[dev].store(true, std::memory_order_release);
     }
     CUtensorMap mq, mk, mv;
     if (!make_map(&mq, Q, (long long)B * H, Sq, HD, tcattn::BM) || !make_map(&mk, K, (long long)B * H, Sk, HD, tcattn::BN) ||
@@ -751,14 +805,15 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
     work.q_blocks = ceil_div(Sq, tcattn::kUnitRows);
     const long long units = (long long)B * H * work.q_blocks;
     if (units > 0x7fffffffLL) return RFK_EUNSUPPORTED;
-    const bool split = ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
-    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sm_count[dev].load(std::memory_order_relaxed), split,
-              cut_last_round);
-    dim3 grid((unsigned)(work.whole_units + work.n_pieces));
-    launch_pdl(kernel, grid, dim3(tcattn::kThreads), tcattn::Cfg<HD>::kSmemBytes, st, mq, mk, mv, O, H, Sq, n_keys,
-               o_bshd, scale * 1.4426950408889634f, row_ss, ss_tiles, norm_dim > 0 ? 1.0f / (float)norm_dim : 0.0f, norm_eps,
-               static_cast<unsigned char*>(ws), v_shared ? H : B * H, work);
-    return launch_status();
+    const bool split = cut != AttnCut::kNone && ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
+    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sms, split, cut == AttnCut::kLastRound);
+    const int v_heads = v_shared ? H : B * H;
+    if (one_block_per_cta(work.n_pieces, (long long)B * H * ceil_div(Sq, tcattn::BM), sms)) {
+        work.q_blocks = ceil_div(Sq, tcattn::BM);
+        work.whole_units = B * H * work.q_blocks;
+        return launch_units<HD, 1, ORDERED>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
+    }
+    return launch_units<HD, 2, ORDERED>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
 }
 }  // namespace
 
@@ -767,9 +822,9 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
 // attention_tc_workspace_bytes() bytes whose first 1024 are zero, for the key split.
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, bool cut_last_round, int v_shared) {
-    return (D == 64 ? launch_hd<64> : launch_hd<128>)(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles,
-                                                      norm_dim, norm_eps, ws, ws_bytes, cut_last_round, v_shared);
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared) {
+    const auto launch = D == 64 ? launch_hd<64, false> : cut == AttnCut::kNone ? launch_hd<128, true> : launch_hd<128, false>;
+    return launch(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, ws_bytes, cut, v_shared);
 }
 
 }  // namespace rfk

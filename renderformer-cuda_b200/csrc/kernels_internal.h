@@ -17,9 +17,10 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
                      int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
                      rfk_stream_t stream);
 
-// Which grids a workspace may cut along the keys (plan_work in attention_tc.cu): those of less than one round of the SMs, or
-// the last, partial round of larger ones too.
-enum class AttnCut { kBelowOneRound, kLastRound };
+// Which grids a workspace may cut along the keys (plan_work in attention_tc.cu): none, those of less than one round of the SMs,
+// or the last, partial round of larger ones too. kNone also takes the row sums of 128-wide heads in the order of
+// flash_attention_mma, whose bits the result then has.
+enum class AttnCut { kNone, kBelowOneRound, kLastRound };
 
 // rfk_flash_attention_ex for heads of 64 or 128
 int flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss, int ss_tiles,
@@ -32,8 +33,11 @@ int flash_attention_mma(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
 
 }  // namespace rfk
 
-// The same with AttnCut::kLastRound, for the tests of the 128-wide kernel, which reach the library through its C symbols.
+// The same with AttnCut::kLastRound, and with kNone, for the tests of the 128-wide kernel, which reach the library through its C
+// symbols.
 extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,
                                            const float* q_row_ss, int ss_tiles, int norm_dim, float eps, void* workspace,
                                            size_t workspace_bytes, int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D,
                                            int o_bshd, float scale, rfk_stream_t stream);
+extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq,
+                                           int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);

@@ -13,8 +13,8 @@ struct rfk_ctx {
     void* attn_ws = nullptr;  // split workspace of the attention kernel (rfk_ctx_reserve_attention_workspace), else NULL
     size_t attn_ws_bytes = 0;
     // Every sum in the order that images have always been made with: no key split of grids of one round or more, and 128-wide
-    // heads on mma.sync attention, GEMM -> softmax -> GEMM in the windows and a separate query norm. Set for sessions with an
-    // image head (rfk_session_create_batched says why).
+    // heads on attention with the mma.sync kernel's bits, GEMM -> softmax -> GEMM in the windows and a separate query norm. Set
+    // for sessions with an image head (rfk_session_create_batched says why).
     bool reproducible = false;
     int device = 0;
 };

@@ -174,3 +174,46 @@ def test_keys_with_a_score_of_minus_infinity_on_64_wide_heads(n_out):
     assert torch.isfinite(outs[1].float()).all()
     _close(outs[0], outs[1], "keys at -inf")
     assert n_out < 1024 or not outs[0][:, 0].any()
+
+
+def _ordered(q, k, v, o, B, Hh, Sq, Sk, n_keys):
+    lib = _abi.load("rfk.h")
+    fn = lib.rfk_flash_attention_ordered
+    fn.argtypes, fn.restype = [ctypes.c_void_p] * 4 + [ctypes.c_int] * 7 + [ctypes.c_float, ctypes.c_void_p], ctypes.c_int
+    rc = fn(*(ctypes.c_void_p(t.data_ptr()) for t in (q, k, v, o)), B, Hh, Sq, Sk, n_keys, D, 0, D ** -0.5,
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, rc
+
+
+@pytest.mark.parametrize("B,Hh,Sq,Sk,n_keys,scale", [
+    (1, 1, 1, 5, 3, 1.0), (1, 2, 129, 128, 65, 1.0), (1, 2, 64, 64, 64, 1.0), (2, 3, 300, 1000, 993, 2.0), (1, 8, 1600, 1408, 1407, 1.0),
+    (1, 8, 4096, 584, 581, 3.0), (3, 40, 257, 300, 290, 1.0)])
+def test_ordered_form_has_the_bits_of_the_mma_sync_kernel(B, Hh, Sq, Sk, n_keys, scale):
+    """Sessions with an image head keep the bits of the mma.sync kernel: grids of one and of two blocks per CTA, ragged
+    queries and keys, references that move in every tile (scores rising along the keys), a row without a finite score."""
+    Q, K, V = _qkv(B, Hh, Sq, Sk, scale)
+    d = torch.nn.functional.normalize(Q.float().mean(2, keepdim=True), dim=-1)
+    K = (K.float() + 4.0 * torch.linspace(0.0, 1.0, Sk, device="cuda").view(1, 1, Sk, 1) * d).half()
+    Q[0, 0, Sq // 2] = -float("inf")
+    K[0, 0] = K[0, 0].abs() + 0.01
+    got, want = torch.full_like(Q, 7.0), torch.full_like(Q, 9.0)
+    _ordered(Q, K, V, got, B, Hh, Sq, Sk, n_keys)
+    pkg.ops.flash_attention_set_path(1)
+    pkg.ops.flash_attention(Q, K, V, want, B, Hh, Sq, Sk, n_keys, D)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("Sq,Sk", [(1, 64), (128, 333), (300, 1000)])
+def test_one_block_per_cta_has_the_bits_of_two(hd, Sq, Sk):
+    """A call whose blocks of 128 queries all find an SM runs one per CTA; the same heads among copies of themselves share
+    theirs."""
+    g = torch.Generator(device="cuda").manual_seed(Sq)
+    Q, K, V = (torch.randn(1, 2, n, hd, device="cuda", generator=g).half() * s for n, s in ((Sq, 4.0), (Sk, 1.0), (Sk, 1.0)))
+    alone = torch.empty_like(Q)
+    pkg.ops.flash_attention(Q, K, V, alone, 1, 2, Sq, Sk, Sk, hd)
+    copies = 100
+    Qm, Km, Vm = (t.expand(copies, -1, -1, -1).contiguous() for t in (Q, K, V))
+    many = torch.empty_like(Qm)
+    pkg.ops.flash_attention(Qm, Km, Vm, many, copies, 2, Sq, Sk, Sk, hd)
+    assert torch.equal(many, alone.expand(copies, -1, -1, -1))
