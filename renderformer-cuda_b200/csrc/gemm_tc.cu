@@ -348,10 +348,13 @@ __device__ __forceinline__ void cluster_sync() {
 // block (one SM takes them at about 110 GB/s). K is not split: every output is summed over the K blocks in the same order
 // as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
 // must equal the views one by one).
-//   A stage is two K blocks: one wait, one announcement and one commit for eight products. And the issuing warp runs its loop
-//   as a whole, one elected lane issuing, so that descriptors and counters live in uniform registers. With one block per
-//   stage and a single thread's loop a K block took 0.30 us on every tile size, the cost of issuing and not of the operands;
-//   together the two took the 64 x 32 tile to 0.16 us.
+//   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing warp and the producer run
+//   their loops as a whole, one elected lane issuing, so that descriptors, coordinates and counters live in uniform registers.
+//   With one block per stage and single threads' loops a K block took 0.30 us on every tile size, the cost of issuing and not of
+//   the operands; two blocks and the elected issuer took the 64 x 32 tile to 0.14 us, the elected producer to 0.12 us (256 x 1024 x
+//   4096 10.96 -> 9.95 us, weights from HBM; the tensor pipe alone would take 0.05 us). Half the ring costs 7 % (the copies in flight cover
+//   their latency); one copy per operand and stage instead of two, and weights asked for ahead of the kernel's wait for its
+//   predecessor, changed nothing or cost (320 x 320 views +4 %).
 //   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
 //   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
 // The epilogue's threads store their own rows: a tile row is 32 to 256 bytes, one to eight whole sectors.
@@ -416,12 +419,12 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_trigger();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ producer (one thread)
-        if (lane == 0) {
-            int it = 0;
-            for (; it < num_st; ++it) {
-                const int s = it % kStages;
-                if (it >= kStages && !tc::mbar_wait(&ctrl->empty[s], ((it / kStages) + 1) & 1, abort_flag)) break;
+        // ------------------------------------------------------------ producer (the warp's elected lane)
+        const bool leader = tc::elect_one();
+        int it = 0, s = 0, par = 1;   // stage of `it`, and the parity of its barrier's previous phase
+        for (; it < num_st; ++it) {
+            if (it >= kStages && !tc::mbar_wait_warp(&ctrl->empty[s], par, abort_flag)) break;
+            if (leader) {
                 tc::mbar_arrive_expect_tx(&ctrl->full[s], kStage);
 #pragma unroll
                 for (int h = 0; h < kSub; ++h) {
@@ -432,11 +435,12 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     if (kGate) tma_load_2d(sW + BN_OUT * BK * 2, &map_w1, x, n0, &ctrl->full[s]);
                 }
             }
-            if (*abort_flag) {   // giving up: wait (bounded) for the last copy of each stage before the CTA exits
-                for (int s = 0; s < kStages && s < it; ++s) {
-                    const int last = ((it - 1 - s) / kStages) * kStages + s;
-                    tc::mbar_wait_drain(&ctrl->full[s], (last / kStages) & 1);
-                }
+            if (++s == kStages) { s = 0; par ^= 1; }
+        }
+        if (leader && *abort_flag) {   // giving up: wait (bounded) for the last copy of each stage before the CTA exits
+            for (int t = 0; t < kStages && t < it; ++t) {
+                const int last = ((it - 1 - t) / kStages) * kStages + t;
+                tc::mbar_wait_drain(&ctrl->full[t], (last / kStages) & 1);
             }
         }
         __syncwarp();
