@@ -288,7 +288,8 @@ static int launch_flash(const __half* Q, const __half* K, const __half* V, __hal
 // layer are resident together (8 per SM of 28 KB, 4 per SM of 52 KB: 1024 and 512 CTAs of a 512 x 512 view are one wave).
 // 128-wide heads used to take two library batches, a softmax over a materialised score matrix and a transpose; with the
 // head-split projections and the deferred norms that this kernel lets them use, a 512 x 512 view of 8 heads of 128 takes
-// 3647 us instead of 3954.
+// 3647 us instead of 3954. Sessions with an image head keep the bits of
+// those steps: kWinSteps has their arithmetic in the one kernel (a 320 x 320 image 2781 -> 2653 us).
 constexpr int kWinTokens = 64, kWinThreads = 128;
 
 // NORMED: Q and K arrive un-normalised (straight from the projection) together with the partial sums of squares of
@@ -302,11 +303,20 @@ struct WinNorm {
 
 template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTokens * kWinTokens;
 
-template <bool NORMED, int HD>
+// How the softmax is taken. kWinFused: the scale rides in the exponent, a row's sum is the sum of its four threads' sums.
+// kWinSteps: the arithmetic of the separate steps - scores rounded after the scale (the library product's alpha), the sums of
+// softmax_small_kernel (16 chunks of four columns, then a butterfly over the chunks) - so that the result has their bits; the
+// products need nothing, mma.sync and the library's kernels add K in the same order.
+enum WinForm { kWinFused, kWinNormed, kWinSteps };
+
+template <WinForm FORM, int HD>
 __global__ void __launch_bounds__(kWinThreads, HD == 64 ? 8 : 4)
 window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
-                        __half* __restrict__ O, const uint8_t* __restrict__ mask, int heads, int nW, float scale_log2e,
+                        __half* __restrict__ O, const uint8_t* __restrict__ mask, int heads, int nW, float scale,
                         const WinNorm nrm) {
+    constexpr bool NORMED = FORM == kWinNormed;
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float scale_log2e = scale * kLog2e;
     constexpr int CPR = HD / 8;   // 16-byte chunks per row
     constexpr int KS = HD / 16;   // k-steps of Q K^T
     constexpr int NT = HD / 8;    // 8-column output tiles
@@ -410,7 +420,12 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
         const int c = n * 8 + 2 * tig;
-        s[n][0] *= scale_log2e; s[n][1] *= scale_log2e; s[n][2] *= scale_log2e; s[n][3] *= scale_log2e;
+        if (FORM == kWinSteps) {   // rounded here: not to be fused with the subtraction of the maximum
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[n][i] = __fmul_rn(s[n][i], scale);
+        } else {
+            s[n][0] *= scale_log2e; s[n][1] *= scale_log2e; s[n][2] *= scale_log2e; s[n][3] *= scale_log2e;
+        }
         if (mask) {
             const unsigned a = *reinterpret_cast<const unsigned short*>(m0 + c);
             const unsigned b = *reinterpret_cast<const unsigned short*>(m1 + c);
@@ -428,18 +443,38 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
     }
+    if (FORM == kWinSteps) {
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-        s[n][0] = fast_exp2(s[n][0] - mx[0]); s[n][1] = fast_exp2(s[n][1] - mx[0]);
-        s[n][2] = fast_exp2(s[n][2] - mx[1]); s[n][3] = fast_exp2(s[n][3] - mx[1]);
-        rs[0] += s[n][0] + s[n][1];
-        rs[1] += s[n][2] + s[n][3];
-    }
+        for (int r = 0; r < 2; ++r) {
+            if (mx[r] == -INFINITY) mx[r] = 0.0f;
+            float c[8];   // this thread pair's chunk of four columns in each 8-column tile: ((e0 + e1) + e2) + e3
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 1);
-        rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 2);
-        rs[r] = 1.0f / rs[r];
+            for (int n = 0; n < 8; ++n) {
+                const float a = s[n][2 * r] = fast_exp2((s[n][2 * r] - mx[r]) * kLog2e);
+                const float b = s[n][2 * r + 1] = fast_exp2((s[n][2 * r + 1] - mx[r]) * kLog2e);
+                const float first = __shfl_xor_sync(0xffffffffu, a + b, 1);   // of columns 0 and 1, at the odd threads
+                c[n] = (first + a) + b;                                       // and so complete there
+            }
+            // the chunk of tile n is number 2n (thread 1) or 2n + 1 (thread 3): partners 8, 4, 2 and 1 numbers away
+            const float sum = ((c[0] + c[4]) + (c[2] + c[6])) + ((c[1] + c[5]) + (c[3] + c[7]));
+            const float both = sum + __shfl_xor_sync(0xffffffffu, sum, 2);
+            const float l = __shfl_sync(0xffffffffu, both, lane | 1);
+            rs[r] = l > 0.0f ? 1.0f / l : 0.0f;
+        }
+    } else {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            s[n][0] = fast_exp2(s[n][0] - mx[0]); s[n][1] = fast_exp2(s[n][1] - mx[0]);
+            s[n][2] = fast_exp2(s[n][2] - mx[1]); s[n][3] = fast_exp2(s[n][3] - mx[1]);
+            rs[0] += s[n][0] + s[n][1];
+            rs[1] += s[n][2] + s[n][3];
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 1);
+            rs[r] += __shfl_xor_sync(0xffffffffu, rs[r], 2);
+            rs[r] = 1.0f / rs[r];
+        }
     }
     unsigned pf[4][4];  // normalised P as A fragments: 4 k-steps of 16 keys
 #pragma unroll
@@ -479,7 +514,7 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     }
 }
 
-template <bool NORMED, int HD>
+template <WinForm FORM, int HD>
 static int launch_window_attention(const __half* Q, const __half* K, const __half* V, __half* O, const uint8_t* mask, int BnW,
                                    int heads, int nW, float scale, const WinNorm& nrm, cudaStream_t st) {
     constexpr int smem = kWinSmemBytes<HD>;
@@ -490,13 +525,13 @@ static int launch_window_attention(const __half* Q, const __half* K, const __hal
         if (e != cudaSuccess) return (int)e;
         if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
         if (!configured[dev].load(std::memory_order_acquire)) {
-            e = cudaFuncSetAttribute(window_attention_kernel<NORMED, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = cudaFuncSetAttribute(window_attention_kernel<FORM, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return (int)e;
             configured[dev].store(true, std::memory_order_release);
         }
     }
-    launch_pdl(window_attention_kernel<NORMED, HD>, dim3((unsigned)((long long)BnW * heads)), dim3(kWinThreads), smem, st, Q, K, V, O,
-               mask, heads, nW, scale * 1.4426950408889634f, nrm);
+    launch_pdl(window_attention_kernel<FORM, HD>, dim3((unsigned)((long long)BnW * heads)), dim3(kWinThreads), smem, st, Q, K, V, O,
+               mask, heads, nW, scale, nrm);
     return launch_status();
 }
 
@@ -514,12 +549,23 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
     const __half *q = (const __half*)Q, *k = (const __half*)K, *v = (const __half*)V;
     cudaStream_t st = as_stream(stream);
     if (!q_row_ss)
-        return (head_dim == 64 ? launch_window_attention<false, 64> : launch_window_attention<false, 128>)(
+        return (head_dim == 64 ? launch_window_attention<kWinFused, 64> : launch_window_attention<kWinFused, 128>)(
             q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, WinNorm{}, st);
     if (!aligned16(gamma_q) || !aligned16(gamma_k)) return RFK_EUNSUPPORTED;
     const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
-    return (head_dim == 64 ? launch_window_attention<true, 64> : launch_window_attention<true, 128>)(
+    return (head_dim == 64 ? launch_window_attention<kWinNormed, 64> : launch_window_attention<kWinNormed, 128>)(
         q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
+}
+
+int window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask, int BnW,
+                           int num_heads, int window_tokens, int head_dim, int nW, float scale, rfk_stream_t stream) {
+    if (!Q || !K || !V || !O || BnW < 0 || num_heads <= 0 || nW <= 0) return RFK_EINVAL;
+    if (window_tokens != kWinTokens || head_dim != 128) return RFK_EUNSUPPORTED;
+    if (BnW == 0) return RFK_OK;
+    if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || (mask && !aligned16(mask))) return RFK_EUNSUPPORTED;
+    if ((long long)BnW * num_heads > 0x7fffffffLL) return RFK_EUNSUPPORTED;
+    return launch_window_attention<kWinSteps, 128>((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, mask, BnW, num_heads,
+                                                   nW, scale, WinNorm{}, as_stream(stream));
 }
 
 // attention_tc.cu
@@ -647,4 +693,9 @@ extern "C" int rfk_window_attention_normed(const rfk_half* Q, const rfk_half* K,
     if (head_dim != 64) return RFK_EUNSUPPORTED;
     return window_attention(Q, K, V, O, mask, q_row_ss, k_row_ss, ss_tiles, gamma_q, gamma_k, norm_dim, eps, BnW, num_heads,
                             window_tokens, head_dim, nW, scale, stream);
+}
+
+extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
+                                          int BnW, int num_heads, int nW, float scale, rfk_stream_t stream) {
+    return window_attention_steps(Q, K, V, O, mask, BnW, num_heads, kWinTokens, 128, nW, scale, stream);
 }

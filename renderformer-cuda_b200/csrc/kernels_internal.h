@@ -17,6 +17,11 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
                      int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
                      rfk_stream_t stream);
 
+// The same for heads of 128 with the bits of the separate steps: library Q K^T with the scale as its alpha,
+// rfk_swin_softmax_probs_inplace, library P V, rfk_transpose_bhsd_to_bsd
+int window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask, int BnW,
+                           int num_heads, int window_tokens, int head_dim, int nW, float scale, rfk_stream_t stream);
+
 // Which grids a workspace may cut along the keys (plan_work in attention_tc.cu): none, those of less than one round of the SMs,
 // or the last, partial round of larger ones too. kNone also takes the row sums of 128-wide heads in the order of
 // flash_attention_mma, whose bits the result then has.
@@ -41,3 +46,6 @@ extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K,
                                            int o_bshd, float scale, rfk_stream_t stream);
 extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq,
                                            int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);
+// window_attention_steps, for its test
+extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
+                                          int BnW, int num_heads, int nW, float scale, rfk_stream_t stream);

@@ -217,3 +217,29 @@ def test_one_block_per_cta_has_the_bits_of_two(hd, Sq, Sk):
     many = torch.empty_like(Qm)
     pkg.ops.flash_attention(Qm, Km, Vm, many, copies, 2, Sq, Sk, Sk, hd)
     assert torch.equal(many, alone.expand(copies, -1, -1, -1))
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("windows,heads", [(1, 1), (4, 8), (25, 3)])
+def test_window_attention_of_128_wide_heads_has_the_bits_of_the_separate_steps(windows, heads, masked):
+    """Sessions with an image head: library Q K^T with the scale as its alpha, swin softmax over the score matrix, library P V
+    and a transpose, against the one kernel. Rows of large scores, a window whose mask leaves single keys, a row of nothing."""
+    g = torch.Generator(device="cuda").manual_seed(windows * 10 + heads)
+    BH, scale = windows * heads, D ** -0.5
+    Q, K, V = (torch.randn(BH, 64, D, device="cuda", generator=g).half() for _ in range(3))
+    Q[:, 10:20] *= 8
+    mask = None
+    if masked:
+        mask = (torch.rand(windows, 64, 64, device="cuda", generator=g) < 0.5).to(torch.uint8)
+        mask[0] = torch.eye(64, device="cuda", dtype=torch.uint8)
+        mask[0, 5] = 0
+    scores = (torch.bmm(Q, K.transpose(1, 2), out_dtype=torch.float32) * scale).contiguous()
+    pkg.ops.swin_softmax_probs_inplace(scores, mask, windows, heads, 64, windows)
+    P = scores.view(torch.float16).view(BH, 64, 128)[:, :, :64].contiguous()
+    want = torch.bmm(P, V).view(windows, heads, 64, D).permute(0, 2, 1, 3).reshape(windows * 64, heads * D)
+    got = torch.full_like(want, 7.0)
+    fn = _abi.load("rfk.h").rfk_window_attention_steps
+    fn.argtypes, fn.restype = [ctypes.c_void_p] * 5 + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_void_p], ctypes.c_int
+    rc = fn(*(ctypes.c_void_p(0 if t is None else t.data_ptr()) for t in (Q, K, V, got, mask)), windows, heads, windows, scale,
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0 and torch.equal(got, want)
