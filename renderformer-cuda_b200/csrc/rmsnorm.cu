@@ -47,7 +47,9 @@ struct WinRows {
 // TH: hidden-state storage, TR: residual storage, TY: normalised output storage.
 // MAP: 0 all operands in token order; 1 y is written in window order; 2 r is read in window order.
 // W: warps per row (1, 2 or 4); NCH: 8-element chunks per lane (dim <= NCH * W * 256).
-template <typename TH, typename TR, typename TY, int NCH, int W, bool HAS_RES, bool WRITE_H, int MAP = 0>
+// SUMS: 1, or the number of warps (256-element chunks) whose partial sums a lone warp adds as W warps would, so that a row has
+// the same bits either way.
+template <typename TH, typename TR, typename TY, int NCH, int W, bool HAS_RES, bool WRITE_H, int MAP = 0, int SUMS = 1>
 __global__ void __launch_bounds__(kRmsThreads)
 rmsnorm_row_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
                    const float* __restrict__ gamma, TY* y,  // x, xw, y may alias
@@ -91,15 +93,32 @@ rmsnorm_row_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
         }
     }
     float ss = 0.0f;
+    if (SUMS > 1) {
+        static_assert(SUMS == 1 || (W == 1 && SUMS == NCH), "one chunk per warp of the other form");
+        float part[NCH];
 #pragma unroll
-    for (int k = 0; k < NCH; ++k) {
-        const int off = (wir * 32 + lane + k * W * 32) * 8;
-        if (off < dim) {
+        for (int k = 0; k < NCH; ++k) {
+            part[k] = 0.0f;
+            if ((lane + k * 32) * 8 < dim) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(v[k][i], v[k][i], ss);
+                for (int i = 0; i < 8; ++i) part[k] = fmaf(v[k][i], v[k][i], part[k]);
+            }
         }
+#pragma unroll
+        for (int k = 0; k < NCH; ++k) part[k] = warp_sum(part[k]);
+#pragma unroll
+        for (int k = 0; k < NCH; ++k) ss += part[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < NCH; ++k) {
+            const int off = (wir * 32 + lane + k * W * 32) * 8;
+            if (off < dim) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) ss = fmaf(v[k][i], v[k][i], ss);
+            }
+        }
+        ss = warp_sum(ss);
     }
-    ss = warp_sum(ss);
     if (W > 1) {
         if (lane == 0) s_part[warp] = ss;
         __syncthreads();
@@ -159,6 +178,18 @@ rmsnorm_generic_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
     }
 }
 
+// Whether fp16 rows of 513 to 1024 elements go to one warp each (four chunks per lane) instead of four warps. They are the
+// decoder's, which the kernel before has left in L2: at 4096 rows the four-warp form is 1.7 rounds of CTAs of which each waits once
+// for memory, the one-warp form a single round with four times the loads in flight. Both have the same bits. Measured
+// (us, four warps / one, 1024 wide; plain, to windows, from windows with residual): 1024 rows 2.1 / 2.4, 2.7 / 2.9, 2.9 / 3.8;
+// 1600 rows 2.2 / 2.6, 4.0 / 3.0, 4.7 / 3.9; 2304 rows 2.8 / 2.7, 4.4 / 3.2, 4.9 / 4.2; 4096 rows 4.8 / 4.0, 6.6 / 4.7, 7.5 / 5.9;
+// 16384 rows 17.6 / 11.0, 22.4 / 12.5, 25.7 / 26.7 - the last is 134 MB of traffic, more than L2, and stays with four.
+static bool one_warp_per_row(int rows, int dim, bool windows, bool residual) {
+    if (dim <= 512 || dim > 1024) return false;
+    if (residual && (long long)rows * dim * 8 > (96ll << 20)) return false;
+    return rows >= (windows ? 1280 : 2048);
+}
+
 template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
 static int launch_variant(const TH* x, TH* xw, const TR* r, const float* gamma, TY* y,
                           int rows, int dim, float eps, cudaStream_t st) {
@@ -170,6 +201,11 @@ static int launch_variant(const TH* x, TH* xw, const TR* r, const float* gamma, 
     launch_pdl(rmsnorm_row_kernel<TH, TR, TY, N, WW, HAS_RES, WRITE_H, 0>,                             \
                dim3(ceil_div(rows, (kRmsThreads / 32) / WW)), dim3(kRmsThreads), 0, st, x, xw, r, gamma, y, \
                rows, dim, eps, WinRows{})
+        if (IsHalf<TH>::value && IsHalf<TY>::value && one_warp_per_row(rows, dim, false, HAS_RES)) {
+            launch_pdl(rmsnorm_row_kernel<TH, TR, TY, 4, 1, HAS_RES, WRITE_H, 0, 4>, dim3(ceil_div(rows, kRmsThreads / 32)), dim3(kRmsThreads),
+                       0, st, x, xw, r, gamma, y, rows, dim, eps, WinRows{});
+            return launch_status();
+        }
         if (dim <= 256) RFK_RMS_LAUNCH(1, 1);
         else if (dim <= 512) RFK_RMS_LAUNCH(1, 2);
         else if (dim <= 1024) RFK_RMS_LAUNCH(1, 4);
@@ -239,20 +275,21 @@ extern "C" int rfk_rmsnorm_residual_f16_windows(rfk_half* x, const rfk_half* r, 
     const WinRows wr{H, W, window_size, shift_size};
     cudaStream_t st = as_stream(stream);
     __half* xh = (__half*)x;
-#define RFK_RMS_WIN(N, WW, M)                                                                                   \
+#define RFK_RMS_WIN(N, WW, M, SUMS)                                                                             \
     if (r)                                                                                                      \
-        launch_pdl(rmsnorm_row_kernel<__half, __half, __half, N, WW, true, true, M>,                             \
+        launch_pdl(rmsnorm_row_kernel<__half, __half, __half, N, WW, true, true, M, SUMS>,                       \
                    dim3(ceil_div(rows, (kRmsThreads / 32) / WW)), dim3(kRmsThreads), 0, st, (const __half*)xh, xh, \
                    (const __half*)r, gamma, (__half*)y, rows, dim, eps, wr);                                     \
     else                                                                                                        \
-        launch_pdl(rmsnorm_row_kernel<__half, __half, __half, N, WW, false, false, 1>,                           \
+        launch_pdl(rmsnorm_row_kernel<__half, __half, __half, N, WW, false, false, 1, SUMS>,                     \
                    dim3(ceil_div(rows, (kRmsThreads / 32) / WW)), dim3(kRmsThreads), 0, st, (const __half*)xh, xh, \
                    (const __half*)nullptr, gamma, (__half*)y, rows, dim, eps, wr)
-#define RFK_RMS_WIN_DIM(M)                            \
-    if (dim <= 256) { RFK_RMS_WIN(1, 1, M); }         \
-    else if (dim <= 512) { RFK_RMS_WIN(1, 2, M); }    \
-    else if (dim <= 1024) { RFK_RMS_WIN(1, 4, M); }   \
-    else { RFK_RMS_WIN(2, 4, M); }
+#define RFK_RMS_WIN_DIM(M)                               \
+    if (one_warp_per_row(rows, dim, true, r != nullptr)) { RFK_RMS_WIN(4, 1, M, 4); } \
+    else if (dim <= 256) { RFK_RMS_WIN(1, 1, M, 1); }    \
+    else if (dim <= 512) { RFK_RMS_WIN(1, 2, M, 1); }    \
+    else if (dim <= 1024) { RFK_RMS_WIN(1, 4, M, 1); }   \
+    else { RFK_RMS_WIN(2, 4, M, 1); }
     if (windowed_operand == 1) { RFK_RMS_WIN_DIM(1); } else { RFK_RMS_WIN_DIM(2); }
 #undef RFK_RMS_WIN_DIM
 #undef RFK_RMS_WIN

@@ -119,3 +119,43 @@ def test_rmsnorm_residual_with_window_ordered_operand_equals_the_separate_kernel
     ops.rmsnorm_residual_f16_windows(xb, r, gamma, yb, B, Hh, W, dim, ws, shift, 2)
     torch.cuda.synchronize()
     assert torch.equal(xa, xb) and torch.equal(ya, yb)
+
+
+@pytest.mark.parametrize("dim", [520, 768, 1024])
+@pytest.mark.parametrize("side", [36, 40, 48])
+def test_rmsnorm_one_warp_per_row_has_the_bits_of_four(side, dim):
+    """Many fp16 rows go to one warp each, few to four: the same rows in one call and a few at a time, plain, with a residual, to
+    windows and from windows."""
+    import torch
+    import renderformer_cuda_b200 as pkg
+    ops = pkg.ops
+    g = torch.Generator(device="cuda").manual_seed(dim + side)
+    copies = 2
+    rows = copies * side * side
+    gamma = 1 + 0.1 * torch.randn(dim, device="cuda", generator=g)
+    x0 = torch.randn(rows, dim, device="cuda", generator=g).half()
+    r0 = torch.randn(rows, dim, device="cuda", generator=g).half()
+    for res in (None, r0):
+        x, y, xs, ys = x0.clone(), torch.empty_like(x0), x0.clone(), torch.empty_like(x0)
+        ops.rmsnorm_residual_f16(x, res, gamma, y, rows, dim)
+        for i in range(0, rows, 300):
+            n = min(300, rows - i)
+            ops.rmsnorm_residual_f16(xs[i:i + n], None if res is None else res[i:i + n], gamma, ys[i:i + n], n, dim)
+        assert torch.equal(x, xs) and torch.equal(y, ys)
+        if side % 8:
+            continue
+        for operand in ([1] if res is None else [1, 2]):
+            xw, yw = x0.clone(), torch.empty_like(x0)
+            ops.rmsnorm_residual_f16_windows(xw, res, gamma, yw, copies, side, side, dim, 8, 4, operand)
+            def to_win(t):
+                t = torch.roll(t.view(copies, side, side, dim), (4, 4), (1, 2)).view(copies, side // 8, 8, side // 8, 8, dim)
+                return t.permute(0, 1, 3, 2, 4, 5).reshape(rows, dim).contiguous()
+            def from_win(t):
+                t = t.view(copies, side // 8, side // 8, 8, 8, dim).permute(0, 1, 3, 2, 4, 5).reshape(copies, side, side, dim)
+                return torch.roll(t, (-4, -4), (1, 2)).reshape(rows, dim).contiguous()
+            xs, ys = x0.clone(), torch.empty_like(x0)
+            rs = None if res is None else (from_win(res) if operand == 2 else res)
+            for i in range(0, rows, 300):
+                n = min(300, rows - i)
+                ops.rmsnorm_residual_f16(xs[i:i + n], None if rs is None else rs[i:i + n], gamma, ys[i:i + n], n, dim)
+            assert torch.equal(xw, xs) and torch.equal(yw, to_win(ys) if operand == 1 else ys)
