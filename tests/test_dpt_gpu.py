@@ -250,3 +250,15 @@ def test_pointwise_convolution_to_planes(C_in, C_out):
     with pytest.raises(o.RfkError) as e:
         o.pointwise_conv_to_planar(x, w, b, out, N, HW, C_in, 5)
     assert e.value.status == -2
+
+
+@pytest.mark.parametrize("N,C,Hi,Wi,Ho,Wo", [(1, 256, 64, 64, 128, 128), (2, 64, 40, 33, 203, 199), (1, 8, 3, 400, 2, 131072), (1, 128, 90, 40, 88, 300)])
+def test_channels_last_upsample_of_many_rows_per_thread_equals_the_nchw_operator(N, C, Hi, Wi, Ho, Wo):
+    """Large maps: eight output rows per thread, the last group short; enlarging, shrinking, more and fewer rows than sources."""
+    o = _ops()
+    g = torch.Generator(device="cuda").manual_seed(Ho)
+    x = torch.randn(N, C, Hi, Wi, device="cuda", generator=g).half()
+    want, got = torch.empty(N, C, Ho, Wo, device="cuda", dtype=H16), torch.empty(N, Ho, Wo, C, device="cuda", dtype=H16)
+    o.bilinear_upsample(x, want, N, C, Hi, Wi, Ho, Wo)
+    o.bilinear_upsample_nhwc(_nhwc(x), got, N, Hi, Wi, Ho, Wo, C)
+    assert torch.equal(got, _nhwc(want))
