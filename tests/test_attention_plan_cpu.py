@@ -73,3 +73,12 @@ def test_last_round_is_cut_behind_whole_rounds(units, n_tiles, sms):
         for t in range(t0, t0 + nt):
             seen[unit][t] += 1
     assert all(c == 1 for u in seen[whole:] for c in u)
+
+
+@pytest.mark.parametrize("units,n_tiles,cut", [(368, 89, True), (464, 113, True), (224, 55, True), (232, 113, True), (256, 89, False),
+                                               (320, 79, True), (300, 40, False), (160, 14, False), (112, 89, False)])
+def test_last_round_of_a_full_chip_is_cut_for_a_tenth(units, n_tiles, cut):
+    """Behind whole rounds, and where every SM gets a share; a grid of less than a round keeps the line of a fifth."""
+    whole, pieces = _plan(units, n_tiles)
+    assert bool(pieces) == cut
+    assert whole == (units // 148 * 148 if cut else units)
