@@ -11,6 +11,11 @@ int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ld
                float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int out_seq, int num_heads,
                int head_dim, rfk_stream_t stream);
 
+// rfk_qkv_norm_rope_transpose behind gemm_heads: parts [heads][seq_len][head_dim] normalised over the row (all heads) and rotated in
+// place, with that kernel's bits
+int qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts, const rfk_half* cos_vals,
+                       const rfk_half* sin_vals, int seq_len, int num_heads, int head_dim, float eps, rfk_stream_t stream);
+
 // rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                      const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,

@@ -15,6 +15,7 @@
 // once, and the in-place update is race-free by construction. The cos/sin chunk is
 // loaded once per thread and reused across the heads the thread walks.
 #include "common.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -253,7 +254,9 @@ struct QkvParts {
 // head h = p / (D/16), chunk j = p % (D/16). With WPR > 1 the sum of squares crosses the warps
 // of a row through shared memory; rows past the end are clamped (and not stored) so that every
 // thread reaches the barrier.
-template <int NPAIR, int WPR>
+// HEADS: the projection has stored its parts head-split already (gemm_heads): each is normalised and rotated in place, x is not
+// read. A thread reads and writes the same chunks.
+template <int NPAIR, int WPR, bool HEADS = false>
 __global__ void __launch_bounds__(128, NPAIR == 1 ? 8 : 1)
 qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
                     const __grid_constant__ QkvParts parts,
@@ -276,6 +279,7 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
     const __half* xr = x + row * row_stride + (long long)part * dim;
     const float* gamma = parts.gamma[part];
     __half* out = parts.out[part];
+    auto out_at = [&](int p) { return (((size_t)b * num_heads + p / cpt) * out_seq_stride + s) * head_dim + (p % cpt) * 8; };
 
     // every load of the row is issued before the first use: the row itself (streamed), the norm weights
     // and the rotation tables (both shared by all rows, L2-resident)
@@ -286,9 +290,9 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
     for (int k = 0; k < NPAIR; ++k) {
         const int p = lane + 32 * WPR * k;
         if (p < npairs) {
-            const int o = (p / cpt) * head_dim + (p % cpt) * 8;
-            xl[k] = ldcs_half8(xr + o);
-            xh[k] = ldcs_half8(xr + o + half_d);
+            const __half* src = HEADS ? out + out_at(p) : xr + (p / cpt) * head_dim + (p % cpt) * 8;
+            xl[k] = HEADS ? ld_half8(src) : ldcs_half8(src);
+            xh[k] = HEADS ? ld_half8(src + half_d) : ldcs_half8(src + half_d);
         }
     }
 #pragma unroll
@@ -354,7 +358,6 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
     for (int k = 0; k < NPAIR; ++k) {
         const int p = lane + 32 * WPR * k;
         if (p < npairs) {
-            const int h = p / cpt, j = p % cpt;
             if (rope) {
                 float cl[8], sl[8], ch[8], sh[8];
                 unpack8(cl8[k], cl);
@@ -363,7 +366,7 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
                 unpack8(sh8[k], sh);
                 rotate8(lo[k], hi[k], cl, sl, ch, sh);
             }
-            const size_t oo = (((size_t)b * num_heads + h) * out_seq_stride + s) * head_dim + j * 8;
+            const size_t oo = out_at(p);
             if (live) {
                 store8(out + oo, lo[k]);
                 store8(out + oo + half_d, hi[k]);
@@ -375,6 +378,33 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
 }  // namespace rfk
 
 using namespace rfk;
+
+int rfk::qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts_io, const rfk_half* cos_vals,
+                            const rfk_half* sin_vals, int seq_len, int num_heads, int head_dim, float eps, rfk_stream_t stream) {
+    if (!gamma || !parts_io || n_parts < 1 || n_parts > 3 || seq_len < 0 || num_heads <= 0 || head_dim <= 0) return RFK_EINVAL;
+    const long long dim = (long long)num_heads * head_dim;
+    if (head_dim % 16 != 0 || dim > 2048) return RFK_EUNSUPPORTED;
+    QkvParts parts{};
+    for (int p = 0; p < n_parts; ++p) {
+        if (!parts_io[p]) return RFK_EINVAL;
+        if (!aligned16(parts_io[p]) || (gamma[p] && !aligned16(gamma[p]))) return RFK_EUNSUPPORTED;
+        parts.gamma[p] = gamma[p];
+        parts.out[p] = (__half*)parts_io[p];
+        parts.use_rope[p] = cos_vals != nullptr;
+    }
+    if (cos_vals && (!sin_vals || !aligned16(cos_vals) || !aligned16(sin_vals))) return RFK_EINVAL;
+    if (seq_len == 0) return RFK_OK;
+    const int npairs = (int)(dim / 16);
+#define RFK_QK_HEADS(N, W)                                                                                   \
+    launch_pdl(qkv_epilogue_kernel<N, W, true>, dim3(ceil_div(seq_len, 4 / W), n_parts), dim3(128), 0, as_stream(stream), \
+               (const __half*)nullptr, 0LL, parts, (const __half*)cos_vals, (const __half*)sin_vals, 1, seq_len, num_heads, \
+               head_dim, eps, (long long)seq_len)
+    if (npairs <= 32) RFK_QK_HEADS(1, 1);
+    else if (npairs <= 64) RFK_QK_HEADS(1, 2);
+    else RFK_QK_HEADS(2, 2);
+#undef RFK_QK_HEADS
+    return launch_status();
+}
 
 extern "C" int rfk_triangle_rope_freqs(const rfk_half* pos, const float* learned_freqs,
                                        rfk_half* out_cos, rfk_half* out_sin, int batch,

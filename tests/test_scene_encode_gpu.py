@@ -113,3 +113,36 @@ def test_cut_of_the_last_round_and_images(with_dpt):
         pkg.ops.flash_attention_set_split(1)
     assert torch.equal(*states) == with_dpt
     s.close()
+
+
+@pytest.mark.parametrize("S,heads,hd", [(1, 4, 64), (33, 4, 64), (300, 2, 128), (1100, 16, 64), (4700, 4, 64), (64, 8, 32)])
+@pytest.mark.parametrize("rope", [True, False])
+def test_head_split_projection_has_the_bits_of_the_separate_epilogue(S, heads, hd, rope):
+    """Self-attention of one batch element: q, k, v stored head-split by their projection, q and k normalised and rotated in
+    place, against the packed projection and its epilogue kernel, which a projection with a bias (here of zeros) takes."""
+    import ctypes
+    from renderformer_cuda_b200 import _abi, session
+    L, VP = _abi.load("rfk_layers.h"), ctypes.c_void_p
+    dim = heads * hd
+    g = torch.Generator(device="cuda").manual_seed(S + hd)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, wi, wo = rnd(S, dim).half(), (rnd(3 * dim, dim) / dim ** 0.5).half(), (rnd(dim, dim) / dim ** 0.5).half()
+    gq, gk = 1 + 0.1 * rnd(dim), 1 + 0.1 * rnd(dim)
+    ang = rnd(S, hd // 2)
+    cos, sin = (torch.cat([f(ang)] * 2, -1).half().contiguous() for f in (torch.cos, torch.sin))
+    zero = torch.zeros(3 * dim, device="cuda", dtype=torch.float16)
+    ctx, outs = session.Ctx(), []
+    score = torch.empty(heads * S * ((S + 7) // 8 * 8), device="cuda") if hd == 32 else None
+    for bias in (None, zero):
+        w = session.MhaW(wi.data_ptr(), None if bias is None else bias.data_ptr(), wo.data_ptr(), None, gq.data_ptr(), gk.data_ptr())
+        out = torch.full((S, dim), 7.0, device="cuda", dtype=torch.float16)
+        buf = torch.full((6 * S * dim,), 7.0, device="cuda", dtype=torch.float16)
+        rc = L.rfk_self_attention(ctx.h, ctypes.byref(w), VP(x.data_ptr()), VP(out.data_ptr()), VP(buf.data_ptr()),
+                                  VP(score.data_ptr() if score is not None else 0), 1, S, dim, heads,
+                                  VP(cos.data_ptr() if rope else 0), VP(sin.data_ptr() if rope else 0),
+                                  VP(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, rc
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
+    ctx.close()
