@@ -103,9 +103,12 @@ world_to_cam_vec8_kernel(const float* __restrict__ c2w, __half* tri, __half* vn,
     if (vn) transform(vn, false);
 }
 
-// thread -> (token t in [0, seq_pad), table chunk j in [0, head_dim/16)).
+// thread -> (token t in [0, seq_pad), chunk j of PER table angles in the first half of head_dim).
 // Every thread rebuilds the token's 9 camera-space coordinates (27 FMAs); the j == 0
-// thread also stores the geometry outputs.
+// thread also stores the geometry outputs. cosf and sinf are long dependent chains, and 5665 tokens of eight-angle threads are
+// five warps an SM: with two angles a thread 4.9 -> 3.8 us (333 tokens 4.6 -> 2.8; 64-wide heads). With twice the angles, 5665
+// tokens of 128-wide heads, there are threads enough and the rebuilt coordinates count: eight 5.5, two 6.6 us.
+template <int PER>
 __global__ void __launch_bounds__(256)
 view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ tri_world,
                      const __half* __restrict__ vn_world, const float* __restrict__ world_center,
@@ -115,7 +118,7 @@ view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ t
                      int seq_pad, int num_freqs, int head_dim) {
     pdl_wait();
     pdl_trigger();
-    const int cpt = head_dim / 16;
+    const int cpt = head_dim / (2 * PER);
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= seq_pad * cpt) return;
     const int t = idx / cpt, j = idx % cpt;
@@ -164,12 +167,12 @@ view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ t
 #pragma unroll
         for (int i = 0; i < 9; ++i) vpos[(size_t)t * 9 + i] = p[i];
     }
-    // RoPE table chunk: l = j*8 + i within the first half of head_dim
+    // RoPE table angles: l = j * PER + i within the first half of head_dim
     const int freq_dim = 9 * num_freqs;
-    float cs[8], sn[8];
+    float cs[PER], sn[PER];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int l = j * 8 + i;
+    for (int i = 0; i < PER; ++i) {
+        const int l = j * PER + i;
         float val = 0.0f;
         if (l < freq_dim) {
             const int coord = l / num_freqs;
@@ -182,12 +185,17 @@ view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ t
         cs[i] = cosf(val);
         sn[i] = sinf(val);
     }
-    const size_t o = (size_t)t * head_dim + j * 8;
-    const Half8 hc = pack8(cs), hs = pack8(sn);
-    st_half8(k_cos + o, hc);
-    st_half8(k_cos + o + head_dim / 2, hc);
-    st_half8(k_sin + o, hs);
-    st_half8(k_sin + o + head_dim / 2, hs);
+    const size_t o = (size_t)t * head_dim + j * PER;
+    struct __align__(2 * PER) Chunk { __half2 v[PER / 2]; } hc, hs;
+#pragma unroll
+    for (int i = 0; i < PER / 2; ++i) {
+        hc.v[i] = __floats2half2_rn(cs[2 * i], cs[2 * i + 1]);
+        hs.v[i] = __floats2half2_rn(sn[2 * i], sn[2 * i + 1]);
+    }
+    *reinterpret_cast<Chunk*>(k_cos + o) = hc;
+    *reinterpret_cast<Chunk*>(k_cos + o + head_dim / 2) = hc;
+    *reinterpret_cast<Chunk*>(k_sin + o) = hs;
+    *reinterpret_cast<Chunk*>(k_sin + o + head_dim / 2) = hs;
 }
 
 }  // namespace rfk
@@ -237,8 +245,9 @@ extern "C" int rfk_view_geometry(const float* c2w, const rfk_half* tri_world,
     if (head_dim <= 0 || head_dim % 16 || !aligned16(k_cos) || !aligned16(k_sin))
         return RFK_EUNSUPPORTED;
     if (seq_pad == 0) return RFK_OK;
-    const long long n = (long long)seq_pad * (head_dim / 16);
-    launch_pdl(view_geometry_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream),
+    const bool many = (long long)seq_pad * (head_dim / 4) > 100000;
+    const long long n = (long long)seq_pad * (head_dim / (many ? 16 : 4));
+    launch_pdl(many ? view_geometry_kernel<8> : view_geometry_kernel<2>, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream),
         c2w, (const __half*)tri_world, (const __half*)vn_world, world_center, learned_freqs,
         (__half*)vtri, (__half*)vvn, (__half*)vpos, (__half*)k_cos, (__half*)k_sin, n_tris,
         n_register, seq_pad, num_freqs, head_dim);

@@ -217,6 +217,54 @@ nerf_pe_rows1_kernel(const TI* __restrict__ input, __half* __restrict__ output, 
     }
 }
 
+// The same with a thread per (row, coordinate), for calls whose rows alone do not give every SM's schedulers several warps: the
+// normals of one scene, 5633 rows of 9, are 45 CTAs of 128 rows, in which each thread walks nine dependent chains one after the
+// other. Tiles of 32 rows: 177 CTAs of nine warps, 3.2 -> 1.8 us (301 rows 3.0 -> 1.5, 45064 rows 4.9 -> 4.1; at 360512 rows 20.4
+// against 21.8, so many rows keep a thread each). Directions, three wide: 4096 rows 2.7 -> 1.6 us, 36864 2.8 -> 2.0, 102400 3.8 against
+// 4.0, 262144 5.9 against 9.3.
+constexpr int kPeCoordRows = 32;
+template <typename TI, int IN_DIM, int NF, bool DOUBLING>
+__global__ void __launch_bounds__(kPeCoordRows * IN_DIM)
+nerf_pe_coords_kernel(const TI* __restrict__ input, __half* __restrict__ output, long long rows,
+                      const __grid_constant__ FreqTable ft, int vec_out) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int PER_ROW = IN_DIM * NF, OUT_DIM = 2 * PER_ROW + IN_DIM, kThreads = kPeCoordRows * IN_DIM;
+    __shared__ __align__(16) __half s_out[kPeCoordRows * OUT_DIM];
+    const long long r0 = (long long)blockIdx.x * kPeCoordRows;
+    const int nrows = (int)min((long long)kPeCoordRows, rows - r0);
+    const int r = threadIdx.x / IN_DIM, d = threadIdx.x % IN_DIM;
+    if (r < nrows) {
+        __half* o = s_out + r * OUT_DIM;
+        const float x = (float)input[r0 * IN_DIM + threadIdx.x];
+        o[d] = __float2half(x);
+        float sn, cs;
+        if (DOUBLING) sincos_fast(x * ft.f[0], sn, cs);
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+            if (!DOUBLING) sincos_fast(x * ft.f[k], sn, cs);
+            o[IN_DIM + d * NF + k] = __float2half(sn);
+            o[IN_DIM + PER_ROW + d * NF + k] = __float2half(cs);
+            if (DOUBLING) {
+                const float s2 = 2.0f * sn * cs;
+                cs = fmaf(-2.0f * sn, sn, 1.0f);
+                sn = s2;
+            }
+        }
+    }
+    __syncthreads();
+    const int n_out = nrows * OUT_DIM;
+    __half* dst = output + r0 * OUT_DIM;  // kPeCoordRows * OUT_DIM halves per tile: a multiple of 16 bytes
+    if (vec_out) {
+        const int nvec = n_out / 8;
+        for (int v = threadIdx.x; v < nvec; v += kThreads)
+            __stcs(reinterpret_cast<uint4*>(dst) + v, reinterpret_cast<const uint4*>(s_out)[v]);
+        for (int e = nvec * 8 + threadIdx.x; e < n_out; e += kThreads) dst[e] = s_out[e];
+    } else {
+        for (int e = threadIdx.x; e < n_out; e += kThreads) dst[e] = s_out[e];
+    }
+}
+
 // A thread owns two adjacent rows: their 2 * OUT_DIM halves start on a 4-byte boundary whatever the parity
 // of OUT_DIM (39 and 117 are odd), so the values leave the registers as packed pairs: half as many
 // shared-memory stores as with one row per thread.
@@ -360,7 +408,16 @@ static int launch_nerf_pe(const TI* input, __half* output, int batch, int seq_le
         if (doubling) launch_pdl(nerf_pe_rows_kernel<TI, IN, NF, true, true>, dim3(row_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec); \
         else launch_pdl(nerf_pe_rows_kernel<TI, IN, NF, false, true>, dim3(row_grid), dim3(kPeRowThreads), 0, st, input, output, rows, ft, vec);         \
     } while (0)
-        if (num_freqs == 6 && in_dim == 3 && inc) RFK_PE_ROWS(3, 6);
+        const bool few = rows <= (1 << 16);
+#define RFK_PE_COORDS(IN, NF)                                                                                 \
+    do {                                                                                                      \
+        const dim3 g(ceil_div(rows, kPeCoordRows)), b(kPeCoordRows * IN);                                      \
+        if (doubling) launch_pdl(nerf_pe_coords_kernel<TI, IN, NF, true>, g, b, 0, st, input, output, rows, ft, vec);  \
+        else launch_pdl(nerf_pe_coords_kernel<TI, IN, NF, false>, g, b, 0, st, input, output, rows, ft, vec); \
+    } while (0)
+        if (num_freqs == 6 && in_dim == 3 && inc && few) RFK_PE_COORDS(3, 6);
+        else if (num_freqs == 6 && in_dim == 3 && inc) RFK_PE_ROWS(3, 6);
+        else if (num_freqs == 6 && in_dim == 9 && inc && few) RFK_PE_COORDS(9, 6);
         else if (num_freqs == 6 && in_dim == 9 && inc) RFK_PE_ROWS1(9, 6);
         else if (num_freqs == 6) RFK_PE_NF(6);
         else if (num_freqs == 4) RFK_PE_NF(4);
@@ -371,6 +428,7 @@ static int launch_nerf_pe(const TI* input, __half* output, int batch, int seq_le
 #undef RFK_PE_NF
 #undef RFK_PE_ROWS
 #undef RFK_PE_ROWS1
+#undef RFK_PE_COORDS
     } else {
         const long long total = rows * out_dim;
         launch_pdl(nerf_pe_flat_kernel<TI>, dim3(ceil_div(total, 256)), dim3(256), 0, st,

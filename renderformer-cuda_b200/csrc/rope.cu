@@ -21,23 +21,27 @@ namespace rfk {
 
 // ---------------------------------------------------------------- tables
 
-// thread -> (token, chunk j of the first half); writes both halves (they are equal)
+// thread -> (token, chunk of PER angles of the first half); writes both halves (they are equal). One scene's tables are short work
+// of a long dependent chain each (cosf and sinf with their reductions), so what counts is how many run side by side: with eight
+// angles a thread the tables of 5633 triangles took 3.5 us, with two 2.1 (301 triangles 3.3 and 1.8; 64-wide heads). Eight keep
+// the wider stores where threads abound: 45064 triangles and 128-wide heads, 1.4 million threads of two, 11.8 against 13.5 us.
+template <int PER>
 __global__ void __launch_bounds__(256)
 rope_table_vec_kernel(const __half* __restrict__ pos, const float* __restrict__ freqs,
                       __half* __restrict__ out_cos, __half* __restrict__ out_sin,
                       long long tokens, int num_freqs, int head_dim) {
     pdl_wait();
     pdl_trigger();
-    const int cpt = head_dim / 16;  // chunks per token (first half)
+    const int cpt = head_dim / (2 * PER);  // chunks per token (first half)
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= tokens * cpt) return;
     const long long tok = idx / cpt;
     const int j = (int)(idx % cpt);
     const int freq_dim = 9 * num_freqs;
-    float c[8], s[8];
+    float c[PER], s[PER];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int l = j * 8 + i;
+    for (int i = 0; i < PER; ++i) {
+        const int l = j * PER + i;
         float val = 0.0f;
         if (l < freq_dim) {
             const float p = __half2float(pos[tok * 9 + l / num_freqs]);
@@ -46,12 +50,17 @@ rope_table_vec_kernel(const __half* __restrict__ pos, const float* __restrict__ 
         c[i] = cosf(val);
         s[i] = sinf(val);
     }
-    const size_t o = (size_t)tok * head_dim + j * 8;
-    const Half8 hc = pack8(c), hs = pack8(s);
-    st_half8(out_cos + o, hc);
-    st_half8(out_cos + o + head_dim / 2, hc);
-    st_half8(out_sin + o, hs);
-    st_half8(out_sin + o + head_dim / 2, hs);
+    const size_t o = (size_t)tok * head_dim + j * PER;
+    struct __align__(2 * PER) Chunk { __half2 v[PER / 2]; } hc, hs;
+#pragma unroll
+    for (int i = 0; i < PER / 2; ++i) {
+        hc.v[i] = __floats2half2_rn(c[2 * i], c[2 * i + 1]);
+        hs.v[i] = __floats2half2_rn(s[2 * i], s[2 * i + 1]);
+    }
+    *reinterpret_cast<Chunk*>(out_cos + o) = hc;
+    *reinterpret_cast<Chunk*>(out_cos + o + head_dim / 2) = hc;
+    *reinterpret_cast<Chunk*>(out_sin + o) = hs;
+    *reinterpret_cast<Chunk*>(out_sin + o + head_dim / 2) = hs;
 }
 
 __global__ void __launch_bounds__(256)
@@ -417,8 +426,9 @@ extern "C" int rfk_triangle_rope_freqs(const rfk_half* pos, const float* learned
     if (tokens == 0) return RFK_OK;
     cudaStream_t st = as_stream(stream);
     if (head_dim % 16 == 0 && aligned16(out_cos) && aligned16(out_sin)) {
-        const long long n = tokens * (head_dim / 16);
-        launch_pdl(rope_table_vec_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st,
+        const bool many = tokens * (head_dim / 4) > (1 << 20);
+        const long long n = tokens * (head_dim / (many ? 16 : 4));
+        launch_pdl(many ? rope_table_vec_kernel<8> : rope_table_vec_kernel<2>, dim3(ceil_div(n, 256)), dim3(256), 0, st,
             (const __half*)pos, learned_freqs, (__half*)out_cos, (__half*)out_sin, tokens,
             num_freqs, head_dim);
     } else {

@@ -159,3 +159,59 @@ def test_rmsnorm_one_warp_per_row_has_the_bits_of_four(side, dim):
                 n = min(300, rows - i)
                 ops.rmsnorm_residual_f16(xs[i:i + n], None if rs is None else rs[i:i + n], gamma, ys[i:i + n], n, dim)
             assert torch.equal(xw, xs) and torch.equal(yw, to_win(ys) if operand == 1 else ys)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("n", [1, 61, 3000])
+def test_rope_tables_and_view_geometry_have_the_same_bits_for_many_and_few_tokens(n, hd):
+    """Few tokens take two angles a thread, many eight: the same tokens in a small call and repeated in a large one."""
+    import math
+    import torch
+    import renderformer_cuda_b200 as pkg
+    from renderformer_cuda_b200 import _abi
+    import ctypes
+    ops, L, VP = pkg.ops, _abi.load("rfk.h"), ctypes.c_void_p
+    g = torch.Generator(device="cuda").manual_seed(n)
+    nf = min(6, hd // 2 // 9)
+    freqs = torch.tensor([math.pi * 10000.0 ** (-i / nf) for i in range(nf)], device="cuda")
+    pos = (torch.rand(n, 9, device="cuda", generator=g) * 4 - 2).half()
+    tables = lambda t, m: [torch.empty(m, hd, device="cuda", dtype=torch.float16) for _ in range(2)]
+    few = tables(pos, n)
+    ops.triangle_rope_freqs(pos, freqs, *few, 1, n, nf, hd)
+    copies = (1 << 20) // (hd // 4) // n + 1
+    many = tables(pos, copies * n)
+    ops.triangle_rope_freqs(pos.repeat(copies, 1).contiguous(), freqs, *many, 1, copies * n, nf, hd)
+    for a, b in zip(few, many):
+        assert torch.equal(b.view(copies, n, hd), a.expand(copies, n, hd))
+    vn = torch.randn(n, 9, device="cuda", generator=g).half()
+    c2w = torch.eye(4, device="cuda")
+    c2w[:3, :] = torch.randn(3, 4, device="cuda", generator=g)
+    centre = torch.zeros(3, device="cuda")
+    def geometry(tri, normals, m):
+        out = [torch.empty_like(tri), torch.empty_like(tri), torch.empty(m, 9, device="cuda", dtype=torch.float16), *tables(tri, m)]
+        rc = L.rfk_view_geometry(*(VP(t.data_ptr()) for t in (c2w, tri, normals, centre, freqs, *out)), m, 0, m, nf, hd,
+                                 VP(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        return out
+    copies = 100000 // (hd // 4) // n + 1
+    for a, b in zip(geometry(pos, vn, n), geometry(pos.repeat(copies, 1).contiguous(), vn.repeat(copies, 1).contiguous(), copies * n)):
+        assert torch.equal(b.view(copies, n, -1), a.expand(copies, n, -1))
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+@pytest.mark.parametrize("in_dim", [3, 9])
+@pytest.mark.parametrize("rows,exps", [(1, (0.0, 5.0)), (31, (0.0, 5.0)), (33, (0.0, 4.0)), (1000, (0.0, 5.0))])
+def test_nerf_pe_has_the_same_bits_for_many_and_few_rows(rows, exps, in_dim, dtype):
+    """Few rows take a thread per coordinate, many a thread per row or two: octaves (doubling) and other bands, ragged tiles."""
+    import torch
+    import renderformer_cuda_b200 as pkg
+    dt = getattr(torch, dtype)
+    fn = pkg.ops.nerf_pe if dt == torch.float16 else pkg.ops.nerf_pe_f32
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, in_dim, device="cuda", generator=g).to(dt)
+    few = torch.empty(rows, in_dim * 13, device="cuda", dtype=torch.float16)
+    fn(x, few, 1, rows, in_dim, 6, *exps, True)
+    copies = (1 << 16) // rows + 1
+    many = torch.empty(copies * rows, in_dim * 13, device="cuda", dtype=torch.float16)
+    fn(x.repeat(copies, 1).contiguous(), many, 1, copies * rows, in_dim, 6, *exps, True)
+    assert torch.equal(many.view(copies, rows, -1), few.expand(copies, rows, -1))
