@@ -1,0 +1,489 @@
+// 3x3 convolution, stride 1, padding 1, channels-last fp16, as an implicit GEMM on CTA pairs (tcgen05 + tensor memory + TMA), with the
+// element-wise steps that follow it in the DPT head as its epilogue:
+//   out = act(half(conv(x, w)) + bias) (+ residual), every intermediate rounded to fp16 as by the separate operators;
+//   and, if asked, silu(out) beside it, the operand of the residual unit that follows.
+// Reference boundary: rf::conv2d and the residual units of rf::dpt_forward, src/layers/dpt.cu:100-178, :397-409 of
+// BANANASJIM/renderformer-cuda.
+//
+// A pair of CTAs owns 256 output pixels (two boxes of 16 x 8, one per CTA) x BN output channels (256 or 128). The GEMM's rows are
+// pixels and its K index is (tap, input channel): a K block is 64 channels of one tap, and its A tile is the box of input pixels
+// shifted by the tap, which one TMA copy of a rank-4 map [n][y][x][c] brings in the tensor core's swizzled layout; pixels beyond
+// the image arrive as zeros, which is the padding. So no patch matrix exists, and the nine shifted reads of a box come from L2.
+// Otherwise the kernel is the projection kernel's (gemm_tc.cu: pair tiles, ring of operand stages filled by per-CTA copies that
+// count on CTA 0's barrier, two accumulators so that a tile's epilogue runs under the next tile's products, staged TMA stores).
+//
+// Order of the sums. The library kernels that this replaces add the K blocks in one of two orders, and images rest on the bits:
+//   taps inside  for each 64 input channels: the nine taps        (its implicit-GEMM kernels)
+//   rows outside for each row of taps: for each 64 channels: the three taps of that row   (its weight-stationary kernels)
+// The caller names the order; both cost the same here.
+// Bound: tensor pipe and the operands' way from L2 (32 KB a K block and SM for 256 channels), as the projections: 1.37 PFLOP/s for
+// 256 -> 256 channels at 256 x 256 with bias and SiLU (56 us; library 61 and 12 for the pass behind it), 1.10 for 256 -> 128 at
+// 512 x 512 (140 us; 171 and 16), whose tiles of 128 channels read 24 KB a K block for half the products.
+#include <algorithm>
+#include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
+#include "common.cuh"
+#include "dpt_math.cuh"
+#include "kernels_internal.h"
+#include "tc_pair.cuh"
+
+namespace rfk {
+
+__device__ int g_conv_tc_error = 0;  // first time-out / failure code seen by any CTA since load
+
+namespace tcconv {
+using namespace pair_ptx;
+
+constexpr int BM = 128, BK = 64, kBoxX = 16, kBoxY = 8;
+static_assert(kBoxX * kBoxY == BM, "a CTA's rows are one box of pixels");
+constexpr int kThreads = 192;                    // warp 0 producer, warp 1 issuer of the products, warps 2-5 epilogue
+constexpr int kTmemCols = 512;                   // all of it: both CTAs of a pair then have the same addresses
+constexpr int kABytes = BM * BK * 2;             // 16 KB
+constexpr int kUnitBytes = 32 * 64 * 2;          // one epilogue warp's 32 pixels x 64 channels, 4 KB
+template <int BN> struct Cfg {
+    static constexpr int kWBytes = BN / 2 * BK * 2;          // this CTA's half of the weight tile
+    static constexpr int kStageBytes = kABytes + kWBytes;
+    static constexpr int kUnits = BN / 64;                   // 64-channel units per tile, one staging buffer each
+    static constexpr int kStagingBytes = 4 * kUnits * kUnitBytes;
+    static constexpr int kStages = BN == 256 ? 5 : 7;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 512;
+    static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
+};
+
+struct __align__(8) Ctrl {
+    uint64_t full[7], empty[7], acc_full[2], acc_empty[2], drain;
+    uint64_t started;          // one phase only: the products of the CTA's first K block are complete
+    uint64_t res_full[4][4];   // [epilogue warp][unit]: that unit's residual box has landed
+    uint32_t tmem_base;
+    int abort;
+};
+static_assert(sizeof(Ctrl) <= 512, "control block");
+
+enum : int { kErrTimeout = 1, kErrSmemAlign = 2 };
+
+struct Params {
+    const __half* bias;
+    int tiles, tiles_x, tiles_img;    // boxes in all images, per row of an image, per image
+    int tiles_m, tiles_n;             // pairs of boxes, blocks of BN output channels
+    int c_in, cb;                     // input channels, blocks of 64 of them
+    int rows_outside, silu, has_res, dual;
+};
+
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* map, int c, int x, int y, int n, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int c, int x, int y, int n, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(tc::smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int c, int x, int y, int n) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                 ::"l"(map), "r"(src), "r"(c), "r"(x), "r"(y), "r"(n) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+    __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ float2 unpack_half2(uint32_t w) { return __half22float2(*reinterpret_cast<__half2*>(&w)); }
+
+struct Box { int x, y, n; };   // first pixel of a CTA's box, and its image
+__device__ __forceinline__ Box box_of(const Params& p, int tile) {
+    const int n = tile / p.tiles_img, r = tile - n * p.tiles_img, ty = r / p.tiles_x;
+    return {(r - ty * p.tiles_x) * kBoxX, ty * kBoxY, n};
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                    const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r,
+                    const __grid_constant__ CUtensorMap map_s, const Params p) {
+    using C = Cfg<BN>;
+    constexpr int kStages = C::kStages, kUnits = C::kUnits;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const uint32_t base = tc::smem_addr(smem_raw);
+    const uint32_t rank = cluster_rank();            // 0: issues the products for the pair; 1: its peer
+    unsigned char* staging = smem_raw + kStages * C::kStageBytes;
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(staging + C::kStagingBytes);
+    volatile int* abort_flag = &ctrl->abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int num_kb = 9 * p.cb;
+    const int num_tiles = p.tiles_m * p.tiles_n;
+    const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+    const bool aligned = (base & 1023u) == 0;        // the same in both CTAs (same kernel, same shared-memory layout)
+
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { tc::mbar_init(&ctrl->acc_full[a], 1); tc::mbar_init(&ctrl->acc_empty[a], 8); }
+        tc::mbar_init(&ctrl->drain, 1);
+        tc::mbar_init(&ctrl->started, 1);
+        for (int w = 0; w < 4; ++w)
+            for (int u = 0; u < 4; ++u) tc::mbar_init(&ctrl->res_full[w][u], 1);
+        ctrl->abort = 0;
+        tc::fence_barrier_init();
+    }
+    if (warp == 0 && aligned) {  // each CTA allocates its own tensor memory
+        tc::tmem_alloc(&ctrl->tmem_base, kTmemCols);
+        tc::tmem_relinquish();
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    cluster_sync();              // both CTAs' barriers are initialised before either signals the other
+    tc::tc_fence_after();
+    if (!aligned) {
+        if (tid == 0) atomicCAS(&g_conv_tc_error, 0, kErrSmemAlign);
+        return;
+    }
+    const uint32_t tmem_cta = ctrl->tmem_base;
+    pdl_wait();      // set-up above is on-chip only; the operands are another kernel's output
+    pdl_trigger();
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ producer (the warp's elected lane, one per CTA)
+        const bool leader = tc::elect_one();
+        int s = 0, par = 1, filled = 0;   // stage, parity of its previous phase, stages filled once
+        bool ok = true;
+        for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
+            const Box b = box_of(p, 2 * (t % p.tiles_m) + (int)rank);   // a box beyond the last one reads as zeros
+            const int nw = (t / p.tiles_m) * BN + (int)rank * (BN / 2);
+            int c = 0, ty = 0, tx = 0;    // channel block and tap of the K block
+            for (int kb = 0; kb < num_kb; ++kb) {
+                if (filled == kStages) ok = tc::mbar_wait_warp(&ctrl->empty[s], par, abort_flag);
+                else ++filled;
+                if (!ok) break;
+                if (leader) {
+                    const uint32_t sA = base + s * C::kStageBytes;
+                    const uint32_t full0 = map_to_cta(tc::smem_addr(&ctrl->full[s]), 0);
+                    // CTA 0 announces the bytes of both CTAs' copies on its own barrier; CTA 1's may land before that: the phase
+                    // cannot complete without the announcement's arrival
+                    if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->full[s], 2 * C::kStageBytes);
+                    tma_load_4d_pair(sA, &map_x, c * BK, b.x + tx - 1, b.y + ty - 1, b.n, full0);
+                    tma_load_2d_pair(sA + kABytes, &map_w, (ty * 3 + tx) * p.c_in + c * BK, nw, full0);
+                }
+                if (++tx == 3) {
+                    tx = 0;
+                    if (p.rows_outside) { if (++c == p.cb) { c = 0; ++ty; } }
+                    else if (++ty == 3) { ty = 0; ++c; }
+                }
+                if (++s == kStages) { s = 0; par ^= 1; }
+            }
+        }
+        if (leader && *abort_flag) drain_pause();   // this CTA's copies count on CTA 0's barriers: give them time to land
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ issuer of the pair's products (elected lane of CTA 0)
+        if (rank == 0) {
+            constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BN, 0);
+            const bool leader = tc::elect_one();
+            int s = 0, par = 0, tl = 0;
+            bool ok = true;
+            for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
+                const int acc = tl & 1;
+                if (tl >= 2) ok = tc::mbar_wait_warp(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1, abort_flag);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint32_t d_tmem = tmem_cta + acc * BN;
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    ok = tc::mbar_wait_warp(&ctrl->full[s], par, abort_flag);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    if (leader) {
+                        const uint32_t a_lo = tc::umma_desc_lo(base + s * C::kStageBytes);
+                        const uint32_t b_lo = tc::umma_desc_lo(base + s * C::kStageBytes + kABytes);
+#pragma unroll
+                        for (int ks = 0; ks < BK / 16; ++ks)
+                            umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb > 0) || (ks > 0));
+                        umma_pair_commit(&ctrl->empty[s]);
+                        if (tl == 0 && kb == 0) umma_pair_commit(&ctrl->started);
+                    }
+                    if (++s == kStages) { s = 0; par ^= 1; }
+                }
+                if (ok && leader) umma_pair_commit(&ctrl->acc_full[acc]);
+            }
+            if (leader && *abort_flag) {
+                umma_pair_commit(&ctrl->drain);
+                tc::mbar_wait_drain(&ctrl->drain, 0);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------ epilogue, warps 2-5 of both CTAs
+        const int lane_grp = warp & 3;                        // a warp reaches tensor-memory lanes [32 * (warp % 4), +32)
+        const uint32_t lane_off = (uint32_t)(lane_grp * 32) << 16;
+        unsigned char* my_stage = staging + lane_grp * kUnits * kUnitBytes;
+        const uint32_t stage_base = tc::smem_addr(my_stage);
+        uint64_t* my_res = ctrl->res_full[lane_grp];
+        bool ok = true;
+        int tl = 0;
+        for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
+            const int acc = tl & 1;
+            const Box b = box_of(p, 2 * (t % p.tiles_m) + (int)rank);
+            const int y0 = b.y + 2 * lane_grp, n0 = (t / p.tiles_m) * BN;   // this warp's 32 pixels: two rows of the box
+            const bool live = 2 * (t % p.tiles_m) + (int)rank < p.tiles;
+            if (lane == 0) {
+                bulk_wait_read<0>();   // the previous tile's stores have read the buffers
+                if (p.has_res) {
+                    // of the first tile only once its first K block has been consumed, so that the operands are not held up;
+                    // the barrier has one phase, which a late warp cannot miss
+                    if (tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
+#pragma unroll
+                    for (int u = 0; u < kUnits; ++u) {
+                        tc::mbar_arrive_expect_tx(&my_res[u], kUnitBytes);
+                        tma_load_4d(stage_base + u * kUnitBytes, &map_r, n0 + u * 64, b.x, y0, b.n, &my_res[u]);
+                    }
+                }
+            }
+            __syncwarp();
+            // Lane l holds channels 2l and 2l + 1 of a unit's bias, fetched a unit ahead (each thread reading the 64 of them itself
+            // was 8 us of load latencies a tile)
+            const uint32_t* bias_lane = reinterpret_cast<const uint32_t*>(p.bias + n0) + lane;
+            uint32_t bias_next = p.bias ? __ldg(bias_lane) : 0;
+            ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
+            if (!ok) break;
+            tc::tc_fence_after();
+            const uint32_t t_acc = tmem_cta + lane_off + acc * BN;
+#pragma unroll 1
+            for (int u = 0; u < kUnits; ++u) {
+                const uint32_t bias_u = bias_next;
+                if (p.bias && u + 1 < kUnits) bias_next = __ldg(bias_lane + (u + 1) * 32);
+                unsigned char* buf = my_stage + u * kUnitBytes;
+                if (p.has_res) ok = tc::mbar_wait_warp(&my_res[u], tl & 1, abort_flag);
+                if (!ok) break;
+                uint32_t second[32];      // silu(out), if asked
+#pragma unroll
+                for (int hc = 0; hc < 2; ++hc) {
+                    uint32_t v[32], o[16];
+                    tc::tmem_ld32(t_acc + u * 64 + hc * 32, v);
+                    uint4 res[4];
+                    if (p.has_res) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) res[q] = *reinterpret_cast<const uint4*>(buf + staged(lane, hc * 4 + q));
+                    }
+                    tc::tc_wait_ld(v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                    if (p.bias) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 y = unpack_half2(o[i]), bb = unpack_half2(__shfl_sync(0xffffffffu, bias_u, hc * 16 + i));
+                            o[i] = pack_half2(y.x + bb.x, y.y + bb.y);
+                        }
+                    }
+                    if (p.silu) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 y = unpack_half2(o[i]);
+                            o[i] = pack_half2(silu_sfu(y.x), silu_sfu(y.y));
+                        }
+                    }
+                    if (p.has_res) {
+                        const uint32_t* rw = reinterpret_cast<const uint32_t*>(res);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 y = unpack_half2(o[i]), rr = unpack_half2(rw[i]);
+                            o[i] = pack_half2(y.x + rr.x, y.y + rr.y);
+                        }
+                    }
+                    if (p.dual) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 z = unpack_half2(o[i]);
+                            second[hc * 16 + i] = pack_half2(silu_sfu(z.x), silu_sfu(z.y));
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        *reinterpret_cast<uint4*>(buf + staged(lane, hc * 4 + q)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                }
+                tc::fence_proxy_async();                      // the copy engine reads what the threads just wrote
+                __syncwarp();
+                if (lane == 0 && live) {
+                    tma_store_4d(&map_o, stage_base + u * kUnitBytes, n0 + u * 64, b.x, y0, b.n);   // pixels beyond the image are clipped
+                    bulk_commit();
+                }
+                if (p.dual) {                                 // the same buffer again, once that store has read it
+                    if (lane == 0) bulk_wait_read<0>();
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        *reinterpret_cast<uint4*>(buf + staged(lane, q)) =
+                            make_uint4(second[4 * q], second[4 * q + 1], second[4 * q + 2], second[4 * q + 3]);
+                    tc::fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0 && live) {
+                        tma_store_4d(&map_s, stage_base + u * kUnitBytes, n0 + u * 64, b.x, y0, b.n);
+                        bulk_commit();
+                    }
+                }
+            }
+            if (!ok) break;
+            // every tcgen05.ld of this warp has completed: hand the accumulator back
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) remote_arrive(map_to_cta(tc::smem_addr(&ctrl->acc_empty[acc]), 0));
+        }
+        if (lane == 0) {
+            if (*abort_flag) drain_pause();
+            bulk_wait_read<0>();   // the stores complete with the grid; shared memory only has to outlive their reads
+        }
+        __syncwarp();
+    }
+
+    // ---- teardown: neither CTA leaves while the other may still signal its barriers or read its shared memory
+    tc::tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    if (warp == 0) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem_cta, kTmemCols);
+    }
+    if (tid == 0 && ctrl->abort) atomicCAS(&g_conv_tc_error, 0, kErrTimeout);
+}
+
+}  // namespace tcconv
+
+namespace {
+
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// cuTensorMapEncodeTiled, taken from the driver the runtime already has loaded (no link against libcuda)
+EncodeTiledFn tensor_map_encoder() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// fp16 tensor of 2 to 4 dimensions, innermost first, dense; boxes in the 128-byte-swizzled layout, elements outside read as zeros
+bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint32_t* box) {
+    EncodeTiledFn enc = tensor_map_encoder();
+    if (!enc) return false;
+    cuuint64_t strides[3], bytes = 2;
+    for (int i = 0; i + 1 < rank; ++i) strides[i] = bytes *= dims[i];
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// [N][H][W][C]; boxes of 64 channels x kBoxX x rows pixels of one image
+bool make_map_pixels(CUtensorMap* m, const void* base, int N, int H, int W, int C, int rows) {
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint32_t box[4] = {64, (cuuint32_t)tcconv::kBoxX, (cuuint32_t)rows, 1};
+    return make_map(m, base, 4, dims, box);
+}
+
+template <int BN> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(tcconv::kThreads); cfg.dynamicSmemBytes = tcconv::Cfg<BN>::kSmemBytes; cfg.stream = st;
+    cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
+    return cfg;
+}
+
+// CTA pairs of the kernel that the device runs at once (asked once per device; 0: it cannot place them)
+template <int BN> int resident_pairs(int dev) {
+    static std::atomic<int> asked[64];   // the answer + 1
+    int n = asked[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+        cudaLaunchAttribute attr[2];
+        cudaLaunchConfig_t cfg = pair_config<BN>(attr, nullptr);
+        int sms = 0, pairs = 0;
+        cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tcconv::conv3x3_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcconv::Cfg<BN>::kSmemBytes);
+        cfg.gridDim = dim3(2 * std::max(1, sms / 2));
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&pairs, tcconv::conv3x3_pair_kernel<BN>, &cfg);
+        if (e != cudaSuccess) { cudaGetLastError(); pairs = 0; }
+        n = std::min(std::max(pairs, 0), sms / 2) + 1;
+        asked[dev].store(n, std::memory_order_release);
+    }
+    return n - 1;
+}
+
+template <int BN>
+int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap& mr, const CUtensorMap& ms, const __half* w, int Cout,
+                tcconv::Params p, int dev, cudaStream_t st) {
+    CUtensorMap mw;
+    const cuuint64_t dims[2] = {(cuuint64_t)9 * p.c_in, (cuuint64_t)Cout};
+    const cuuint32_t box[2] = {64, BN / 2};
+    if (!make_map(&mw, w, 2, dims, box)) return RFK_EUNSUPPORTED;
+    const int pairs = resident_pairs<BN>(dev);
+    if (pairs <= 0) return RFK_EUNSUPPORTED;
+    p.tiles_n = Cout / BN;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = pair_config<BN>(attr, st);
+    cfg.gridDim = dim3(2 * std::min(p.tiles_m * p.tiles_n, pairs));
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcconv::conv3x3_pair_kernel<BN>, mx, mw, mo, mr, ms, p);
+    if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
+    return launch_status();
+}
+
+// shapes and alignments that the kernel takes
+bool conv_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, const rfk_half* out,
+                 const rfk_half* out_silu, int C_in, int C_out) {
+    return C_in % 64 == 0 && C_out % 128 == 0 && aligned16(x) && aligned16(w) && aligned16(out) && (!residual || aligned16(residual)) &&
+           (!out_silu || aligned16(out_silu)) && (!bias || (reinterpret_cast<uintptr_t>(bias) & 3u) == 0);
+}
+
+}  // namespace
+}  // namespace rfk
+
+using namespace rfk;
+
+extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
+                                       const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out) {
+    int dev = 0;
+    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out) || !tensor_map_encoder()) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    return (C_out % 256 == 0 ? resident_pairs<256>(dev) : resident_pairs<128>(dev)) > 0;
+}
+
+extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
+                                rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside,
+                                rfk_stream_t stream) {
+    if (!x || !w || !out || N < 0 || H <= 0 || W <= 0 || C_in <= 0 || C_out <= 0) return RFK_EINVAL;
+    if (x == out || x == out_silu || out == out_silu) return RFK_EINVAL;   // a pixel is read by its neighbours' tiles
+    if (N == 0) return RFK_OK;
+    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out)) return RFK_EUNSUPPORTED;
+    const long long tx = ceil_div(W, tcconv::kBoxX), ty = ceil_div(H, tcconv::kBoxY);
+    if (tx * ty * N * (C_out / 128) > 0x3fffffffLL || 9LL * C_in > 0x7fffffffLL) return RFK_EUNSUPPORTED;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    CUtensorMap mx, mo, mr, ms;
+    if (!make_map_pixels(&mx, x, N, H, W, C_in, tcconv::kBoxY) || !make_map_pixels(&mo, out, N, H, W, C_out, 2) ||
+        !make_map_pixels(&mr, residual ? residual : out, N, H, W, C_out, 2) ||
+        !make_map_pixels(&ms, out_silu ? out_silu : out, N, H, W, C_out, 2))
+        return RFK_EUNSUPPORTED;
+    tcconv::Params p{};
+    p.bias = (const __half*)bias;
+    p.tiles_x = (int)tx; p.tiles_img = (int)(tx * ty); p.tiles = p.tiles_img * N;
+    p.tiles_m = (p.tiles + 1) / 2;
+    p.c_in = C_in; p.cb = C_in / 64;
+    p.rows_outside = rows_outside != 0; p.silu = silu != 0; p.has_res = residual != nullptr; p.dual = out_silu != nullptr;
+    return (C_out % 256 == 0 ? launch_conv<256> : launch_conv<128>)(mx, mo, mr, ms, (const __half*)w, C_out, p, dev, as_stream(stream));
+}
+
+extern "C" int rfk_conv_error(int* code, int clear) {
+    if (!code) return RFK_EINVAL;
+    cudaError_t e = cudaMemcpyFromSymbol(code, g_conv_tc_error, sizeof(int));
+    if (e != cudaSuccess) return (int)e;
+    if (clear) {
+        const int zero = 0;
+        e = cudaMemcpyToSymbol(g_conv_tc_error, &zero, sizeof(int));
+        if (e != cudaSuccess) return (int)e;
+    }
+    return RFK_OK;
+}

@@ -7,14 +7,16 @@
 //     they are (handed NCHW tensors they convert every operand on the way in and out: 69 conversion launches, 35 % of
 //     the head's time when it ran that way); a 1x1 convolution is a row-major GEMM and goes to rfk_linear, i.e. the
 //     tcgen05 projection kernel with the bias in its epilogue; the two transposed convolutions (kernel = stride) are that
-//     same GEMM followed by a depth-to-space scatter. Only the 3x3 convolutions remain library (cuDNN) calls. Filters
-//     are re-laid out once, at plan time.
-//   - bias, SiLU and residual adds that follow a convolution are one pass (rfk_bias_act_residual_nhwc), bit-identical
+//     same GEMM followed by a depth-to-space scatter. The large 3x3 convolutions of a single view are the tcgen05 kernel of
+//     conv_tc.cu, the others library (cuDNN) calls (own_conv says where the line lies). Filters are re-laid out once, at plan time.
+//   - bias, SiLU and residual adds that follow a convolution, and the SiLU that the next residual unit starts with, are the
+//     epilogue of that kernel, or one pass behind the library (rfk_bias_act_residual_nhwc), bit-identical
 //     to the separate operators; the copy the reference's in-place SiLU forces before a residual unit is gone.
 //   - nothing is allocated on the launch path. The reference calls cudaMallocAsync / cudaFreeAsync for every
 //     intermediate inside dpt_forward (and so inside its captured graph); here rfk_dpt_create sizes every intermediate
 //     once, picks the cuDNN algorithms, allocates one workspace, and records the whole head as a list of steps over
 //     fixed buffers. rfk_dpt_forward only walks that list, so it can be captured.
+#include "kernels_internal.h"
 #include "layers_internal.h"
 
 #include <cudnn.h>
@@ -35,6 +37,16 @@ namespace {
         int rc_ = (expr);               \
         if (rc_ != RFK_OK) return rc_;  \
     } while (0)
+
+// Which 3x3 convolutions (stride 1) the tcgen05 kernel of conv_tc.cu takes from the library: those of one view with more than 2^31
+// multiply-adds a tap, where its tiles of 256 pixels fill the SMs about twice. Measured with bias and SiLU (us, library and its pass / this
+// kernel): 256 -> 256 channels at 256^2 73 / 56, 160^2 28.6 / 31.7, 128^2 21 / 22, 64^2 9.7 / 19.6; 256 -> 128 at 512^2 187 / 140, 320^2
+// 55.6 / 55.9; 512 -> 256 at 128^2 31.7 / 32.7. A head over several views keeps the library, which chooses the order of its sums anew
+// for every batch size.
+bool own_conv(int B, int H, int W, int Cin, int Cout) { return B == 1 && (long long)H * W * Cin * Cout > (1LL << 31); }
+// The order in which it then adds (conv_tc.cu): the library's for that size, bit for bit (compared for every map of 64 x 64 to
+// 512 x 512 images), so that images stay what they were.
+int sums_rows_outside(int H, int W, int Cout) { return (long long)H * W >= (Cout >= 256 ? 65536 : 200704); }
 
 using Step = std::function<int(const rfk_half* const* feats, cudaStream_t st)>;
 
@@ -87,9 +99,10 @@ struct rfk_dpt {
     }
 
     // o [B, Ho, Wo, Cout] = conv(in [B, H, W, Cin], weight [Cout, Cin, k, k] as the reference stores it) + bias, then SiLU
-    // if silu, then + residual if given. in == nullptr: the step reads feature tap `tap` ([B, pH*pW, dim] is [B, pH, pW, dim]).
+    // if silu, then + residual if given; o_silu (3x3, may be null) = SiLU of that.
+    // in == nullptr: the step reads feature tap `tap` ([B, pH*pW, dim] is [B, pH, pW, dim]).
     int add_conv(const rfk_half* in, int tap, const rfk_half* weight, const rfk_half* bias, rfk_half* o, int Cin, int H, int W,
-                 int Cout, int k, int stride, int pad, bool silu = false, const rfk_half* residual = nullptr) {
+                 int Cout, int k, int stride, int pad, bool silu = false, const rfk_half* residual = nullptr, rfk_half* o_silu = nullptr) {
         const int Ho = (H + 2 * pad - k) / stride + 1, Wo = (W + 2 * pad - k) / stride + 1;
         const long long rows_out = (long long)B * Ho * Wo;
         ++n_convs;
@@ -109,6 +122,14 @@ struct rfk_dpt {
         rfk_half* wk = alloc((size_t)Cout * Cin * k * k);  // [Cout, k, k, Cin]
         if (!wk) return (int)cudaErrorMemoryAllocation;
         TRY(rfk_permute_filter(weight, wk, Cout, Cin, k * k, 0, nullptr));
+        if (k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout) &&
+            rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout)) {
+            const int Bn = B, rows_outside = sums_rows_outside(H, W, Cout);
+            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
+                return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
+            });
+            return RFK_OK;
+        }
         cudnnTensorDescriptor_t xd = tensor(B, Cin, H, W), yd = tensor(B, Cout, Ho, Wo);
         cudnnFilterDescriptor_t fd = filter(Cout, Cin, k, k);
         cudnnConvolutionDescriptor_t cd = conv(pad, stride);
@@ -129,7 +150,8 @@ struct rfk_dpt {
             const float one = 1.0f, zero = 0.0f;
             DNN_TRY(cudnnSetStream(self->dnn, st));
             DNN_TRY(cudnnConvolutionForward(self->dnn, &one, xd, in, fd, wk, cd, algo, self->workspace, ws, &zero, yd, o));
-            if (bias || silu || residual) return rfk_bias_act_residual_nhwc(o, bias, residual, rows_out, Cout, silu, (rfk_stream_t)st);
+            if (bias || silu || residual) TRY(rfk_bias_act_residual_nhwc(o, bias, residual, rows_out, Cout, silu, (rfk_stream_t)st));
+            if (o_silu) return rfk_silu(o, o_silu, rows_out * Cout, (rfk_stream_t)st);
             return RFK_OK;
         });
         return RFK_OK;
@@ -157,32 +179,44 @@ struct rfk_dpt {
         return RFK_OK;
     }
 
-    // residual convolution unit (src/layers/dpt.cu:397-409): *result <- conv2(silu(conv1(silu(x)))) + x; x is left as it was
-    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, int F, int H, int W, rfk_half** result) {
+    // residual convolution unit (src/layers/dpt.cu:397-409): *result <- conv2(silu(conv1(x_silu))) + x with x_silu = silu(x), which
+    // whatever made x has left beside it; x is left as it was
+    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, const rfk_half* x_silu, int F, int H, int W, rfk_half** result) {
         const long long n = (long long)B * F * H * W;
         rfk_half* t0 = alloc((size_t)n);
         rfk_half* t1 = alloc((size_t)n);
         if (!t0 || !t1) return (int)cudaErrorMemoryAllocation;
-        program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int { return rfk_silu(x, t0, n, (rfk_stream_t)st); });
-        TRY(add_conv(t0, -1, r.conv1_w, r.conv1_b, t1, F, H, W, F, 3, 1, 1, /*silu=*/true));
+        TRY(add_conv(x_silu, -1, r.conv1_w, r.conv1_b, t1, F, H, W, F, 3, 1, 1, /*silu=*/true));
         TRY(add_conv(t1, -1, r.conv2_w, r.conv2_b, t0, F, H, W, F, 3, 1, 1, /*silu=*/false, /*residual=*/x));
         *result = t0;
         return RFK_OK;
     }
 
-    // feature fusion block (src/layers/dpt.cu:411-426); returns the [B, th, tw, F] result buffer in *result
-    int add_refinenet(int i, rfk_half* path_in, rfk_half* lr, int ph, int pw, int th, int tw, rfk_half** result) {
+    // feature fusion block (src/layers/dpt.cu:411-426); returns the [B, th, tw, F] result buffer in *result. path_silu and lr_silu:
+    // SiLU of path_in and lr, where they are a residual unit's first operand as they come (path_silu may be null)
+    int add_refinenet(int i, rfk_half* path_in, const rfk_half* path_silu, const rfk_half* lr, const rfk_half* lr_silu, int ph, int pw,
+                      int th, int tw, rfk_half** result) {
         const int F = w.features_dim;
         const rfk_ffb_weights& f = w.refinenet[i];
+        const long long n = (long long)B * F * ph * pw;
         if (f.has_resconv1) {
             if (!lr) return RFK_EINVAL;
             rfk_half* r1 = nullptr;
-            TRY(add_rcu(f.rcu1, lr, F, ph, pw, &r1));
-            const long long n = (long long)B * F * ph * pw;
-            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int { return rfk_residual_add(path_in, r1, n, (rfk_stream_t)st); });
+            TRY(add_rcu(f.rcu1, lr, lr_silu, F, ph, pw, &r1));
+            rfk_half* s = alloc((size_t)n);
+            if (!s) return (int)cudaErrorMemoryAllocation;
+            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
+                return rfk_residual_add_silu_nhwc(path_in, r1, s, n, (rfk_stream_t)st);
+            });
+            path_silu = s;
+        } else if (!path_silu) {
+            rfk_half* s = alloc((size_t)n);
+            if (!s) return (int)cudaErrorMemoryAllocation;
+            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int { return rfk_silu(path_in, s, n, (rfk_stream_t)st); });
+            path_silu = s;
         }
         rfk_half* r2 = nullptr;
-        TRY(add_rcu(f.rcu2, path_in, F, ph, pw, &r2));
+        TRY(add_rcu(f.rcu2, path_in, path_silu, F, ph, pw, &r2));
         rfk_half* up = alloc((size_t)B * F * th * tw);
         rfk_half* res = alloc((size_t)B * F * th * tw);
         if (!up || !res) return (int)cudaErrorMemoryAllocation;
@@ -220,18 +254,20 @@ struct rfk_dpt {
                 TRY(add_conv(projected, -1, w.resize_w[i], w.resize_b[i], resized[i], C, pH, pW, C, 3, 2, 1));
             }
         }
-        rfk_half* layer_rn[4];
+        rfk_half *layer_rn[4], *rn_silu[4];
         for (int i = 0; i < 4; ++i) {
             layer_rn[i] = alloc((size_t)B * F * rh[i] * rw[i]);
-            if (!layer_rn[i]) return (int)cudaErrorMemoryAllocation;
-            TRY(add_conv(resized[i], -1, w.layer_rn_w[i], nullptr, layer_rn[i], w.out_channels[i], rh[i], rw[i], F, 3, 1, 1));
+            rn_silu[i] = alloc((size_t)B * F * rh[i] * rw[i]);
+            if (!layer_rn[i] || !rn_silu[i]) return (int)cudaErrorMemoryAllocation;
+            TRY(add_conv(resized[i], -1, w.layer_rn_w[i], nullptr, layer_rn[i], w.out_channels[i], rh[i], rw[i], F, 3, 1, 1, false, nullptr,
+                         rn_silu[i]));
         }
         rfk_half *path4, *path3, *path2, *path1;
-        TRY(add_refinenet(3, layer_rn[3], nullptr, rh[3], rw[3], rh[2], rw[2], &path4));
-        TRY(add_refinenet(2, path4, layer_rn[2], rh[2], rw[2], rh[1], rw[1], &path3));
-        TRY(add_refinenet(1, path3, layer_rn[1], rh[1], rw[1], rh[0], rw[0], &path2));
+        TRY(add_refinenet(3, layer_rn[3], rn_silu[3], nullptr, nullptr, rh[3], rw[3], rh[2], rw[2], &path4));
+        TRY(add_refinenet(2, path4, nullptr, layer_rn[2], rn_silu[2], rh[2], rw[2], rh[1], rw[1], &path3));
+        TRY(add_refinenet(1, path3, nullptr, layer_rn[1], rn_silu[1], rh[1], rw[1], rh[0], rw[0], &path2));
         const int oh = rh[0] * 2, ow = rw[0] * 2;
-        TRY(add_refinenet(0, path2, layer_rn[0], rh[0], rw[0], oh, ow, &path1));
+        TRY(add_refinenet(0, path2, nullptr, layer_rn[0], rn_silu[0], rh[0], rw[0], oh, ow, &path1));
         // output head (src/layers/dpt.cu:440-460)
         const int fh = F / 2, full_h = pH * ps, full_w = pW * ps;
         rfk_half* oc1 = alloc((size_t)B * fh * oh * ow);

@@ -12,6 +12,7 @@
 // intermediate is still rounded to fp16, so the values are bit-identical to the unfused sequence.
 #include "common.cuh"
 #include "dpt_math.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -60,6 +61,24 @@ silu_nhwc_kernel(const __half* __restrict__ x, __half* __restrict__ y, long long
 #pragma unroll
     for (int k = 0; k < 8; ++k) f[k] = silu_sfu(f[k]);
     store8(y + i * 8, f);
+}
+
+// y += r, and silu of the sum beside it: the operand of the residual unit that follows the addition
+__global__ void __launch_bounds__(256)
+residual_add_silu_nhwc_kernel(__half* __restrict__ y, const __half* __restrict__ r, __half* __restrict__ s, long long chunks) {
+    pdl_wait();
+    pdl_trigger();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= chunks) return;
+    float f[8], g[8];
+    load8(y + i * 8, f);
+    load8(r + i * 8, g);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] = round_half(f[k] + g[k]);
+    store8(y + i * 8, f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] = silu_sfu(f[k]);
+    store8(s + i * 8, f);
 }
 
 // out[n, ho, wo, :] from in[n, :, :, :], align_corners = true; a thread owns 8 channels of one output column in ROWS
@@ -255,6 +274,15 @@ extern "C" int rfk_silu(const rfk_half* x, rfk_half* y, long long n, rfk_stream_
     if (n == 0) return RFK_OK;
     if (n % 8 || !aligned16(x) || !aligned16(y)) return RFK_EUNSUPPORTED;
     launch_pdl(silu_nhwc_kernel, dim3((unsigned)ceil_div(n / 8, 256)), dim3(256), 0, as_stream(stream), (const __half*)x, (__half*)y, n / 8);
+    return launch_status();
+}
+
+extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream) {
+    if (!y || !r || !y_silu || n < 0) return RFK_EINVAL;
+    if (n == 0) return RFK_OK;
+    if (n % 8 || !aligned16(y) || !aligned16(r) || !aligned16(y_silu) || n / 8 > 0x7fffffffLL) return RFK_EUNSUPPORTED;
+    launch_pdl(residual_add_silu_nhwc_kernel, dim3((unsigned)ceil_div(n / 8, 256)), dim3(256), 0, as_stream(stream), (__half*)y,
+               (const __half*)r, (__half*)y_silu, n / 8);
     return launch_status();
 }
 

@@ -54,3 +54,19 @@ extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K,
 // window_attention_steps, for its test
 extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                                           int BnW, int num_heads, int nW, float scale, rfk_stream_t stream);
+
+// 3x3 convolution of the DPT head (conv_tc.cu): x [N,H,W,C_in], w [C_out,3,3,C_in], stride 1, padding 1;
+// out [N,H,W,C_out] = act(half(conv) + bias) (+ residual), act SiLU if silu, every intermediate rounded to fp16; out_silu (may be
+// NULL) = silu(out). bias and residual may be NULL; out and out_silu must not be x or one another. rows_outside: the order of the
+// sums (see conv_tc.cu). C_in % 64 == 0, C_out % 128 == 0, else RFK_EUNSUPPORTED.
+extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
+                                rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside,
+                                rfk_stream_t stream);
+// whether it takes these operands on the current device
+extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
+                                       const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out);
+// the convolution's time-out word, as rfk_gemm_error
+extern "C" int rfk_conv_error(int* code, int clear);
+
+// y += r in fp16, and silu(y) beside it: rfk_residual_add and rfk_silu in one pass; n % 8 == 0, 16-byte aligned
+extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);

@@ -19,6 +19,7 @@
 //     the input bit for bit, so the query rotation is skipped;
 //   - the DPT convolution head and the image post-process are outside this library: the frame
 //     result is the decoder's final token map plus the four feature taps a DPT head reads.
+#include "kernels_internal.h"
 #include "layers_internal.h"
 
 #include <algorithm>
@@ -531,6 +532,8 @@ static int check_attention_error() {
     TRY(rfk_flash_attention_error(&code, 0));
     if (code) return RFK_EKERNEL;
     TRY(rfk_gemm_error(&code, 0));  // the tcgen05 GEMM kernel reports the same way
+    if (code) return RFK_EKERNEL;
+    TRY(rfk_conv_error(&code, 0));  // and the convolution
     return code ? RFK_EKERNEL : RFK_OK;
 }
 
