@@ -16,6 +16,11 @@ int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ld
 int qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts, const rfk_half* cos_vals,
                        const rfk_half* sin_vals, int seq_len, int num_heads, int head_dim, float eps, rfk_stream_t stream);
 
+// out = rmsnorm_f32(a) + rmsnorm_f32(b) + c, fp32, in one pass with the bits of the separate steps; a, b fp16 [rows, dim], c fp16 [dim];
+// dim % 8 == 0, dim <= 1024, 16-byte aligned, else RFK_EUNSUPPORTED
+int norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c, float* out,
+                  int rows, int dim, float eps, rfk_stream_t stream);
+
 // rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                      const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
@@ -70,3 +75,7 @@ extern "C" int rfk_conv_error(int* code, int clear);
 
 // y += r in fp16, and silu(y) beside it: rfk_residual_add and rfk_silu in one pass; n % 8 == 0, 16-byte aligned
 extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);
+
+// norm_pair_add, for its test
+extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,
+                                 float* out, int rows, int dim, float eps, rfk_stream_t stream);

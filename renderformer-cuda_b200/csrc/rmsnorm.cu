@@ -20,6 +20,7 @@
 // 16 CTAs per SM) retire and get replaced continuously, so loads of new rows overlap the
 // stores of finished ones. The W partial sums meet through 16 bytes of shared memory.
 #include "common.cuh"
+#include "kernels_internal.h"
 
 namespace rfk {
 
@@ -141,6 +142,56 @@ rmsnorm_row_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
     }
 }
 
+// out = norm(a) + norm(b) + c in fp32, a and b fp16, c one fp16 row for all: the two embeddings of a scene's triangles and the
+// triangle token, with the bits of two casts to fp32, two fp32 norms and the sum (same chunks, same order of the partial sums as
+// rmsnorm_row_kernel with W warps a row). One pass over 46 MB at 5633 x 1024 where the five took 185.
+template <int W>
+__global__ void __launch_bounds__(kRmsThreads)
+norm_pair_add_kernel(const __half* __restrict__ a, const float* __restrict__ gamma_a, const __half* __restrict__ b,
+                     const float* __restrict__ gamma_b, const __half* __restrict__ c, float* __restrict__ out, int rows, int dim, float eps) {
+    constexpr int kWarps = kRmsThreads / 32;
+    __shared__ float s_part[2][kWarps];
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long row = (long long)blockIdx.x * (kWarps / W) + warp / W;
+    const bool live = row < rows;
+    if (!live) row = rows - 1;  // idle warps shadow the last row and never store
+    const int off = ((warp % W) * 32 + lane) * 8;
+    const bool in = off < dim;
+    float v[2][8], ss[2] = {0.0f, 0.0f};
+    if (in) {
+        load8(a + (size_t)row * dim + off, v[0]);
+        load8(b + (size_t)row * dim + off, v[1]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss[t] = fmaf(v[t][i], v[t][i], ss[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) ss[t] = warp_sum(ss[t]);
+    if (W > 1) {
+        if (lane == 0) { s_part[0][warp] = ss[0]; s_part[1][warp] = ss[1]; }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            ss[t] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < W; ++i) ss[t] += s_part[t][(warp / W) * W + i];
+        }
+    }
+    if (!live || !in) return;
+    float ga[8], gb[8], cc[8], o[8];
+    ldg_float8(gamma_a + off, ga);
+    ldg_float8(gamma_b + off, gb);
+    load8(c + off, cc);
+    const float ra = rsqrtf(ss[0] * (1.0f / (float)dim) + eps), rb = rsqrtf(ss[1] * (1.0f / (float)dim) + eps);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)   // each term rounded as it was when it was stored
+        o[i] = __fadd_rn(__fadd_rn(__fmul_rn(__fmul_rn(v[0][i], ra), ga[i]), __fmul_rn(__fmul_rn(v[1][i], rb), gb[i])), cc[i]);
+    store8(out + (size_t)row * dim + off, o);
+}
+
 // Any dim / any alignment: one CTA per row, scalar accesses, the row is re-read.
 template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
 __global__ void __launch_bounds__(256)
@@ -227,9 +278,27 @@ static int launch_rmsnorm(const TH* x, TH* xw, const TR* r, const float* gamma, 
     return launch_variant<TH, TR, TY, false, false>(x, xw, r, gamma, y, rows, dim, eps, st);
 }
 
+int norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c, float* out,
+                  int rows, int dim, float eps, rfk_stream_t stream) {
+    if (!a || !gamma_a || !b || !gamma_b || !c || !out || rows < 0 || dim <= 0) return RFK_EINVAL;
+    if (dim % 8 || dim > 1024 || !aligned16(a) || !aligned16(gamma_a) || !aligned16(b) || !aligned16(gamma_b) || !aligned16(c) || !aligned16(out))
+        return RFK_EUNSUPPORTED;
+    if (rows == 0) return RFK_OK;
+    const int w = dim <= 256 ? 1 : dim <= 512 ? 2 : 4;
+    launch_pdl(w == 1 ? norm_pair_add_kernel<1> : w == 2 ? norm_pair_add_kernel<2> : norm_pair_add_kernel<4>,
+               dim3(ceil_div(rows, (kRmsThreads / 32) / w)), dim3(kRmsThreads), 0, as_stream(stream), (const __half*)a, gamma_a,
+               (const __half*)b, gamma_b, (const __half*)c, out, rows, dim, eps);
+    return launch_status();
+}
+
 }  // namespace rfk
 
 using namespace rfk;
+
+extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,
+                                 float* out, int rows, int dim, float eps, rfk_stream_t stream) {
+    return norm_pair_add(a, gamma_a, b, gamma_b, c, out, rows, dim, eps, stream);
+}
 
 extern "C" int rfk_rmsnorm(const rfk_half* x, const float* gamma, rfk_half* y, int rows, int dim,
                            float eps, rfk_stream_t stream) {

@@ -442,7 +442,7 @@ struct Carver {
 // projections lie in the layers' qkv buffer, which is idle before the first and after the last encoder layer.
 struct EncodeBuffers {
     rfk_half *tex, *vn_pe, *pos, *cos, *sin, *temp, *qkv, *ffn;
-    rfk_half* emb16;                            // inside qkv, before the encoder; fp32 beside it:
+    rfk_half *vn_emb16, *tex_emb16;             // inside qkv, before the encoder; fp32 beside them:
     float *vn_n, *tex_n;
     rfk_half *ctx16, *ctx_normed, *kv_proj;     // inside qkv, after it
     float *seq, *score;
@@ -463,9 +463,10 @@ struct EncodeBuffers {
         if (!(d.hd == 64 || d.hd == 128)) c.get(&score, (size_t)m.num_heads * Se * d.Se_pad);
         if (base) {
             const size_t piece = align_up(Se * dim, 128);   // halves, so that every piece is 256-byte aligned
-            emb16 = qkv;
-            vn_n = (float*)(qkv + piece);
-            tex_n = (float*)(qkv + 3 * piece);
+            vn_emb16 = qkv;
+            tex_emb16 = qkv + piece;
+            vn_n = (float*)(qkv + 2 * piece);
+            tex_n = (float*)(qkv + 4 * piece);
             ctx16 = qkv;
             ctx_normed = qkv + piece;
             kv_proj = qkv + 2 * piece;                      // two pieces
@@ -492,17 +493,23 @@ extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const 
     TRY(rfk_triangle_rope_freqs(b.pos, m.enc_rope_freqs, b.cos, b.sin, 1, Se, m.rope_num_freqs, hd, s));
     // normals: NeRF PE -> linear -> fp32 RMSNorm (render_session.cu:310-318)
     TRY(rfk_nerf_pe_f32(vn, b.vn_pe, 1, N, 9, m.vn_pe_num_freqs, 0.0f, (float)(m.vn_pe_num_freqs - 1), 1, s));
-    TRY(rfk_linear(d->ctx, b.vn_pe, m.vn_proj_w, m.vn_proj_b, b.emb16, N, dim, vn_pe_dim, s));
-    TRY(rfk_cast_fp16_to_fp32(b.emb16, b.vn_n, (long long)N * dim, s));
-    TRY(rfk_rmsnorm_f32(b.vn_n, m.vn_enc_norm, b.vn_n, N, dim, kEpsFp16, s));
+    TRY(rfk_linear(d->ctx, b.vn_pe, m.vn_proj_w, m.vn_proj_b, b.vn_emb16, N, dim, vn_pe_dim, s));
     // texture: linear -> fp32 RMSNorm (render_session.cu:321-327)
-    TRY(rfk_linear(d->ctx, b.tex, m.tex_enc_w, m.tex_enc_b, b.emb16, N, dim, C, s));
-    TRY(rfk_cast_fp16_to_fp32(b.emb16, b.tex_n, (long long)N * dim, s));
-    TRY(rfk_rmsnorm_f32(b.tex_n, m.tex_enc_norm, b.tex_n, N, dim, kEpsFp16, s));
+    TRY(rfk_linear(d->ctx, b.tex, m.tex_enc_w, m.tex_enc_b, b.tex_emb16, N, dim, C, s));
     // sequence = [register tokens | texture + normal + triangle token] in fp32 (render_session.cu:330-339)
     TRY(rfk_cast_fp16_to_fp32(m.reg_tokens, b.seq, (long long)nr * dim, s));
-    add3_bc_kernel<<<blocks_for((long long)N * dim), 256, 0, st>>>(b.seq + (size_t)nr * dim, b.tex_n, b.vn_n,
-                                                                   (const __half*)m.tri_token, (long long)N * dim, dim);
+    float* tri_seq = b.seq + (size_t)nr * dim;
+    const int rc = rfk::norm_pair_add(b.tex_emb16, m.tex_enc_norm, b.vn_emb16, m.vn_enc_norm, m.tri_token, tri_seq, N, dim, kEpsFp16, s);
+    if (rc == RFK_EUNSUPPORTED) {   // other widths: step by step
+        TRY(rfk_cast_fp16_to_fp32(b.vn_emb16, b.vn_n, (long long)N * dim, s));
+        TRY(rfk_rmsnorm_f32(b.vn_n, m.vn_enc_norm, b.vn_n, N, dim, kEpsFp16, s));
+        TRY(rfk_cast_fp16_to_fp32(b.tex_emb16, b.tex_n, (long long)N * dim, s));
+        TRY(rfk_rmsnorm_f32(b.tex_n, m.tex_enc_norm, b.tex_n, N, dim, kEpsFp16, s));
+        add3_bc_kernel<<<blocks_for((long long)N * dim), 256, 0, st>>>(tri_seq, b.tex_n, b.vn_n, (const __half*)m.tri_token,
+                                                                       (long long)N * dim, dim);
+    } else if (rc != RFK_OK) {
+        return rc;
+    }
 
     // encoder (render_session.cu:356-371)
     const rfk_half* pending = nullptr;

@@ -146,3 +146,27 @@ def test_head_split_projection_has_the_bits_of_the_separate_epilogue(S, heads, h
         outs.append(out)
     assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
     ctx.close()
+
+
+@pytest.mark.parametrize("dim", [8, 256, 264, 512, 768, 1024])
+@pytest.mark.parametrize("rows", [1, 5, 300])
+def test_embedding_norms_and_sum_have_the_bits_of_the_separate_steps(rows, dim):
+    import ctypes
+    import renderformer_cuda_b200 as pkg
+    from renderformer_cuda_b200 import _abi
+    ops, VP = pkg.ops, ctypes.c_void_p
+    g = torch.Generator(device="cuda").manual_seed(rows + dim)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    a, b, c, ga, gb = rnd(rows, dim).half(), rnd(rows, dim).half(), rnd(dim).half(), 1 + 0.1 * rnd(dim), 1 + 0.1 * rnd(dim)
+    norms = []
+    for x, gamma in ((a, ga), (b, gb)):
+        f = torch.empty(rows, dim, device="cuda")
+        ops.cast_fp16_to_fp32(x, f, rows * dim)
+        ops.rmsnorm_f32(f, gamma, f, rows, dim, ops.K_EPS_FP16)
+        norms.append(f)
+    want, got = (norms[0] + norms[1]) + c.float(), torch.empty(rows, dim, device="cuda")
+    fn = _abi.load("rfk.h").rfk_norm_pair_add
+    fn.argtypes, fn.restype = [VP] * 6 + [ctypes.c_int] * 2 + [ctypes.c_float, VP], ctypes.c_int
+    assert fn(*(VP(t.data_ptr()) for t in (a, ga, b, gb, c, got)), rows, dim, ops.K_EPS_FP16,
+              VP(torch.cuda.current_stream().cuda_stream)) == 0
+    assert torch.equal(got, want)
