@@ -363,7 +363,8 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
                 raw[1][k] = ldg_half8(Kh + r * HD + c * 8);
                 const long long row = (long long)bw * kWinTokens + r;   // token row in window order
                 float sq = 0.0f, sk = 0.0f;
-                if (nrm.four) {   // dim 1024, both aligned: one load each instead of four (64 windows x 16 heads 9.6 -> 8.9 us, 4 x 16 4.5 -> 3.9)
+                if (nrm.four) {   // dim 1024, both aligned: one load each instead of four (operands in L2 as behind the projection: 64 windows x
+                    // 16 heads 9.6 -> 8.9 us, 4 x 16 4.5 -> 3.9; operands from HBM 13.2 either way)
                     const float4 a = __ldg(reinterpret_cast<const float4*>(nrm.q_ss) + row), b = __ldg(reinterpret_cast<const float4*>(nrm.k_ss) + row);
                     sq = ((a.x + a.y) + a.z) + a.w;
                     sk = ((b.x + b.y) + b.z) + b.w;
