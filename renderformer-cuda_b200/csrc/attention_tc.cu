@@ -704,15 +704,13 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     const long long tiles = (long long)rest * n_tiles;
     constexpr int kMaxPiecesPerUnit = 8;  // the CTA that merges a unit reads its pieces one after the other
     const int shares = (int)std::min<long long>(std::min(sms, tcattn::kMaxPieces / 2), (long long)rest * kMaxPiecesPerUnit);
-    // whole: one more round of n_tiles; split: a share's tiles plus the piece overhead. Cut only for a clear gain: a fifth of the
-    // launch, or a tenth where whole rounds go ahead and every SM of a full chip gets a share (grids of less than a round keep the
-    // line: frames and images rest on where those are cut; slices of a chip were not measured).
-    // Measured where the estimate gives 7 %, 256 units of 89 tiles on 148 SMs: nothing gained. 368 units of 89 tiles, estimate
-    // 12 %: 209 -> 189 us, 464 of 113, 19 %: 343 -> 291 us, 224 of 55, 13 %: 95 -> 85 us at head size 64; 232 of 113, 16 %: 264 -> 237 us,
-    // 184 of 89, 31 %: 200 -> 153 us at head size 128.
-    const long long cut = (long long)rounds * n_tiles + (tiles + shares - 1) / shares + kPieceCostTiles, uncut = (long long)(rounds + 1) * n_tiles;
-    const bool full_chip = sms >= 100 && rest * kMaxPiecesPerUnit >= sms;
-    if (cut * 5 > uncut * 4 && !(rounds > 0 && full_chip && cut * 10 <= uncut * 9)) return;
+    // whole: one more round of n_tiles; split: a share's tiles plus the piece overhead. Cut only for a clear gain: a fifth of
+    // the launch. (Measured where the estimate gives 7 %, 256 units of 89 tiles on 148 SMs: nothing gained. 184 units of 89
+    // tiles, estimate 31 %: 200 -> 153 us at head size 128; 208 units, estimate 23 %: 139 -> 114 us and 160 units of 40 tiles,
+    // 29 %: 68 -> 52 us at head size 64.) A line of a tenth gains too (368 units of 89 tiles, estimate 12 %: 209 -> 189 us at head
+    // size 64), but it moves the sums, and so the K/V cache and every view, of scenes that this line leaves whole: the line is
+    // part of what rfk_flash_attention_ex and the sessions promise, and stays.
+    if (((long long)rounds * n_tiles + (tiles + shares - 1) / shares + kPieceCostTiles) * 5 > (long long)(rounds + 1) * n_tiles * 4) return;
     const int whole = rounds * sms;
     Piece* pc = w.pieces;
     int n = 0;

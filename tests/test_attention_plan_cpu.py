@@ -75,10 +75,8 @@ def test_last_round_is_cut_behind_whole_rounds(units, n_tiles, sms):
     assert all(c == 1 for u in seen[whole:] for c in u)
 
 
-@pytest.mark.parametrize("units,n_tiles,cut", [(368, 89, True), (464, 113, True), (224, 55, True), (232, 113, True), (256, 89, False),
-                                               (320, 79, True), (300, 40, False), (160, 14, False), (112, 89, False)])
-def test_last_round_of_a_full_chip_is_cut_for_a_tenth(units, n_tiles, cut):
-    """Behind whole rounds, and where every SM gets a share; a grid of less than a round keeps the line of a fifth."""
-    whole, pieces = _plan(units, n_tiles)
-    assert bool(pieces) == cut
-    assert whole == (units // 148 * 148 if cut else units)
+@pytest.mark.parametrize("units,n_tiles", [(368, 89), (464, 113), (224, 55), (232, 113)])
+def test_last_round_that_saves_less_than_a_fifth_stays_whole(units, n_tiles):
+    """The line that the header states. The encoder of a scene of 5633 triangles and 16 heads is 368 units of 89 tiles, where a cut is
+    estimated to save 12 %: its sums, and with them the K/V cache and the views, keep their order."""
+    assert _plan(units, n_tiles) == (units, [])
