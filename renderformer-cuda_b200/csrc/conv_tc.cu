@@ -15,7 +15,7 @@
 // Order of the sums. The library kernels that this replaces add the K blocks in one of two orders, and images rest on the bits:
 //   taps inside  for each 64 input channels: the nine taps        (its implicit-GEMM kernels)
 //   rows outside for each row of taps: for each 64 channels: the three taps of that row   (its weight-stationary kernels)
-// The caller names the order; both cost the same here.
+// The caller names the order (dpt.cu finds out, size by size, which the library takes); both cost the same here.
 // Bound: tensor pipe and the operands' way from L2 (32 KB a K block and SM for 256 channels), as the projections: 1.37 PFLOP/s for
 // 256 -> 256 channels at 256 x 256 with bias and SiLU (56 us; library 61 and 12 for the pass behind it), 1.10 for 256 -> 128 at
 // 512 x 512 (140 us; 171 and 16), whose tiles of 128 channels read 24 KB a K block for half the products.

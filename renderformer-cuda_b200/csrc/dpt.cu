@@ -44,9 +44,22 @@ namespace {
 // 55.6 / 55.9; 512 -> 256 at 128^2 31.7 / 32.7. A head over several views keeps the library, which chooses the order of its sums anew
 // for every batch size.
 bool own_conv(int B, int H, int W, int Cin, int Cout) { return B == 1 && (long long)H * W * Cin * Cout > (1LL << 31); }
-// The order in which it then adds (conv_tc.cu): the library's for that size, bit for bit (compared for every map of 64 x 64 to
-// 512 x 512 images), so that images stay what they were.
-int sums_rows_outside(int H, int W, int Cout) { return (long long)H * W >= (Cout >= 256 ? 65536 : 200704); }
+
+// Operands of the plan's comparison of the two (order_of_sums): fp16 in [-1, 1), a hash of the position
+__global__ void fill_hashed_kernel(__half* p, long long n, unsigned seed) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    unsigned h = (unsigned)i * 2654435761u + seed;
+    h = (h ^ (h >> 15)) * 2246822519u;
+    h = (h ^ (h >> 13)) * 3266489917u;
+    h ^= h >> 16;
+    p[i] = __float2half((float)(int)h * (1.0f / 2147483648.0f));
+}
+// *differ becomes 1 unless the n pairs of values at a and b have the same bits
+__global__ void differ_kernel(const unsigned* a, const unsigned* b, long long n, int* differ) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && a[i] != b[i]) *differ = 1;
+}
 
 using Step = std::function<int(const rfk_half* const* feats, cudaStream_t st)>;
 
@@ -65,7 +78,10 @@ struct rfk_dpt {
     size_t ws_bytes = 0;
     std::vector<Step> program;
     rfk_half* out = nullptr;  // [B, out_dim, pH*ps, pW*ps]
-    int n_convs = 0;
+    int n_convs = 0, n_own = 0;      // convolutions in all, and those of the tcgen05 kernel among them
+    bool library_only = false;
+    struct Order { int H, W, Cin, Cout, rows_outside; };
+    std::vector<Order> orders;       // what order_of_sums found
 
     rfk_half* alloc(size_t halves) {
         void* p = nullptr;
@@ -98,6 +114,44 @@ struct rfk_dpt {
         return d;
     }
 
+    // The order in which the tcgen05 kernel has to add (its rows_outside, 0 or 1) for the bits of the library's convolution of this size,
+    // or -1 if neither order has them, and the convolution stays with the library. An image is 10^x of what comes out here, and
+    // images do not change with the kernel that makes them. Which order the library takes is its own choice per size, type of
+    // kernel and version, so it is not written down here but found out: both run once on the same operands when the head is planned, once
+    // for each size of map (about 1 ms for the two of a 512 x 512 image).
+    int order_of_sums(cudnnTensorDescriptor_t xd, cudnnFilterDescriptor_t fd, cudnnConvolutionDescriptor_t cd, cudnnTensorDescriptor_t yd,
+                      cudnnConvolutionFwdAlgo_t algo, size_t ws, int H, int W, int Cin, int Cout) {
+        for (const Order& k : orders)
+            if (k.H == H && k.W == W && k.Cin == Cin && k.Cout == Cout) return k.rows_outside;
+        const size_t nx = (size_t)H * W * Cin, nw = (size_t)Cout * 9 * Cin, ny = (size_t)H * W * Cout;
+        const auto pad = [](size_t halves) { return (halves * sizeof(__half) + 255) / 256 * 256; };
+        int found = -1;
+        char* scratch = nullptr;
+        if (cudaMalloc((void**)&scratch, pad(nx) + pad(nw) + 2 * pad(ny) + 256 + ws) == cudaSuccess) {
+            rfk_half *x = (rfk_half*)scratch, *k = (rfk_half*)((char*)x + pad(nx)), *want = (rfk_half*)((char*)k + pad(nw));
+            rfk_half* got = (rfk_half*)((char*)want + pad(ny));
+            int* differ = (int*)((char*)got + pad(ny));
+            const auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
+            fill_hashed_kernel<<<blocks(nx), 256>>>((__half*)x, (long long)nx, 1);
+            fill_hashed_kernel<<<blocks(nw), 256>>>((__half*)k, (long long)nw, 2);
+            const float one = 1.0f, zero = 0.0f;
+            bool ran = cudnnSetStream(dnn, nullptr) == CUDNN_STATUS_SUCCESS &&
+                       cudnnConvolutionForward(dnn, &one, xd, x, fd, k, cd, algo, (char*)differ + 256, ws, &zero, yd, want) == CUDNN_STATUS_SUCCESS;
+            for (int rows_outside = 0; ran && found < 0 && rows_outside < 2; ++rows_outside) {
+                int other = 1;
+                ran = cudaMemsetAsync(differ, 0, sizeof(int)) == cudaSuccess &&
+                      rfk_conv3x3_nhwc(x, k, nullptr, nullptr, got, nullptr, 1, H, W, Cin, Cout, 0, rows_outside, nullptr) == RFK_OK;
+                if (ran) differ_kernel<<<blocks(ny / 2), 256>>>((const unsigned*)want, (const unsigned*)got, (long long)(ny / 2), differ);
+                ran = ran && cudaMemcpy(&other, differ, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+                if (ran && !other) found = rows_outside;
+            }
+            cudaFree(scratch);
+        }
+        cudaGetLastError();   // whatever failed: the library serves this size
+        orders.push_back({H, W, Cin, Cout, found});
+        return found;
+    }
+
     // o [B, Ho, Wo, Cout] = conv(in [B, H, W, Cin], weight [Cout, Cin, k, k] as the reference stores it) + bias, then SiLU
     // if silu, then + residual if given; o_silu (3x3, may be null) = SiLU of that.
     // in == nullptr: the step reads feature tap `tap` ([B, pH*pW, dim] is [B, pH, pW, dim]).
@@ -122,14 +176,6 @@ struct rfk_dpt {
         rfk_half* wk = alloc((size_t)Cout * Cin * k * k);  // [Cout, k, k, Cin]
         if (!wk) return (int)cudaErrorMemoryAllocation;
         TRY(rfk_permute_filter(weight, wk, Cout, Cin, k * k, 0, nullptr));
-        if (k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout) &&
-            rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout)) {
-            const int Bn = B, rows_outside = sums_rows_outside(H, W, Cout);
-            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
-                return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
-            });
-            return RFK_OK;
-        }
         cudnnTensorDescriptor_t xd = tensor(B, Cin, H, W), yd = tensor(B, Cout, Ho, Wo);
         cudnnFilterDescriptor_t fd = filter(Cout, Cin, k, k);
         cudnnConvolutionDescriptor_t cd = conv(pad, stride);
@@ -144,6 +190,17 @@ struct rfk_dpt {
         const cudnnConvolutionFwdAlgo_t algo = perf[0].algo;
         size_t ws = 0;
         DNN_TRY(cudnnGetConvolutionForwardWorkspaceSize(dnn, xd, fd, cd, yd, algo, &ws));
+        if (!library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout) &&
+            rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout)) {
+            const int Bn = B, rows_outside = order_of_sums(xd, fd, cd, yd, algo, ws, H, W, Cin, Cout);
+            if (rows_outside >= 0) {
+                ++n_own;
+                program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
+                    return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
+                });
+                return RFK_OK;
+            }
+        }
         ws_bytes = std::max(ws_bytes, ws);
         rfk_dpt* self = this;
         program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
@@ -324,8 +381,8 @@ extern "C" int rfk_dpt_destroy(rfk_dpt* d) {
     return RFK_OK;
 }
 
-extern "C" int rfk_dpt_create(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int dim, int patch_h, int patch_w, int patch_size,
-                              rfk_dpt** out) {
+extern "C" int rfk_dpt_create_from(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int dim, int patch_h, int patch_w, int patch_size,
+                                   int library_only, int* own_convolutions, rfk_dpt** out) {
     if (!ctx || !w || !out || B <= 0 || dim <= 0 || patch_h <= 0 || patch_w <= 0 || patch_size <= 0) return RFK_EINVAL;
     if (w->features_dim <= 0 || w->features_dim % 2 || w->out_dim <= 0) return RFK_EINVAL;
     // the channels-last element-wise kernels move 8 channels per access
@@ -336,11 +393,18 @@ extern "C" int rfk_dpt_create(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int
         if (w->out_channels[i] <= 0 || !w->project_w[i] || !w->layer_rn_w[i] || (i != 2 && !w->resize_w[i])) return RFK_EINVAL;
     rfk_dpt* d = new rfk_dpt();
     d->ctx = ctx; d->w = *w; d->B = B; d->dim = dim; d->pH = patch_h; d->pW = patch_w; d->ps = patch_size;
+    d->library_only = library_only != 0;
     if (cudnnCreate(&d->dnn) != CUDNN_STATUS_SUCCESS) { delete d; return 2000; }
     const int rc = d->build();
     if (rc != RFK_OK) { rfk_dpt_destroy(d); return rc; }
+    if (own_convolutions) *own_convolutions = d->n_own;
     *out = d;
     return RFK_OK;
+}
+
+extern "C" int rfk_dpt_create(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int dim, int patch_h, int patch_w, int patch_size,
+                              rfk_dpt** out) {
+    return rfk_dpt_create_from(ctx, w, B, dim, patch_h, patch_w, patch_size, 0, nullptr, out);
 }
 
 extern "C" int rfk_dpt_forward(rfk_dpt* d, const rfk_half* const* features, rfk_half* image_out, rfk_stream_t stream) {

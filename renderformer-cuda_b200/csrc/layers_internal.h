@@ -33,3 +33,8 @@ int decoder_layer_impl(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, rfk_hal
                        const rfk_half* q_rope_cos, const rfk_half* q_rope_sin, const rfk_half* k_rope_cos,
                        const rfk_half* k_rope_sin, int cache_flags, rfk_stream_t stream);
 }  // namespace rfk_layers
+
+// rfk_dpt_create, with every 3x3 convolution left to the library if library_only, for the tests that compare the two;
+// *own_convolutions (may be NULL) = how many the tcgen05 kernel took.
+extern "C" int rfk_dpt_create_from(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int dim, int patch_h, int patch_w, int patch_size,
+                                   int library_only, int* own_convolutions, rfk_dpt** out);

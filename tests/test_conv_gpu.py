@@ -116,3 +116,37 @@ def test_sum_and_its_silu_equal_the_separate_operators(n):
     pkg.ops.silu(want, act, n)
     assert _lib().rfk_residual_add_silu_nhwc(_p(got), _p(r), _p(s), n, _stream()) == 0
     assert torch.equal(got, want) and torch.equal(s, act)
+
+
+def _plan(L, ctx, model, B, pH, pW, library_only):
+    dpt, own = VP(), ctypes.c_int(-1)
+    L.rfk_dpt_create_from.argtypes = [VP] * 2 + [ctypes.c_int] * 6 + [VP, VP]
+    assert L.rfk_dpt_create_from(ctx.h, ctypes.byref(model.dpt_c), B, model.dim, pH, pW, 8, library_only, ctypes.byref(own), ctypes.byref(dpt)) == 0
+    return dpt, own.value
+
+
+@pytest.mark.parametrize("pH,pW,F,B", [(48, 48, 256, 1), (52, 52, 256, 1), (64, 64, 256, 1), (72, 72, 256, 1), (33, 128, 256, 1), (40, 40, 512, 1),
+                                       (52, 52, 256, 2), (16, 16, 256, 1)])
+def test_heads_have_the_bits_of_the_library_convolutions(pH, pW, F, B):
+    """Whole heads, the large convolutions of a view on the kernel and all of them with the library: maps whose order of sums the
+    library changes from one size to the next, oblong ones, more features, images above 512 pixels. Several views and small maps
+    stay with the library."""
+    from renderformer_cuda_b200 import session
+    L = _abi.load("rfk_layers.h")
+    model = session.Model.random(seed=3, dim=256, num_heads=4, ffn_hidden=256, enc_layers=0, dec_layers=1, with_dpt=True, dpt_features=F,
+                                 dpt_out_channels=(256, 512, 1024, 1024))
+    g = torch.Generator(device="cuda").manual_seed(pH)
+    feats = [torch.randn(B, pH * pW, 256, device="cuda", generator=g).half() for _ in range(4)]
+    taps, ctx = (VP * 4)(*[f.data_ptr() for f in feats]), session.Ctx()
+    images = []
+    for library_only in (0, 1):
+        dpt, own = _plan(L, ctx, model, B, pH, pW, library_only)
+        assert (own > 0) == (not library_only and B == 1 and pH > 16)
+        image = torch.full((B, 3, pH * 8, pW * 8), 7.0, device="cuda", dtype=torch.float16)
+        for _ in range(2):   # the buffers of the first pass are those of the second
+            assert L.rfk_dpt_forward(dpt, taps, VP(image.data_ptr()), _stream()) == 0
+        torch.cuda.synchronize()
+        images.append(image)
+        L.rfk_dpt_destroy(dpt)
+    assert torch.isfinite(images[0].float()).all() and torch.equal(*images)
+    ctx.close()
