@@ -76,6 +76,12 @@ extern "C" int rfk_conv_error(int* code, int clear);
 // y += r in fp16, and silu(y) beside it: rfk_residual_add and rfk_silu in one pass; n % 8 == 0, 16-byte aligned
 extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);
 
+// rfk_rmsnorm_residual_f16_windows for operands that the kernels before have just written (the layers' case): the same values, another
+// split of the rows (one_warp_per_row in rmsnorm.cu)
+extern "C" int rfk_rmsnorm_residual_f16_windows_in_l2(rfk_half* x, const rfk_half* r, const float* gamma, rfk_half* y, int B, int H, int W,
+                                                      int dim, int window_size, int shift_size, int windowed_operand, float eps,
+                                                      rfk_stream_t stream);
+
 // norm_pair_add, for its test
 extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,
                                  float* out, int rows, int dim, float eps, rfk_stream_t stream);

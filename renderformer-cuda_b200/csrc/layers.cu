@@ -543,14 +543,14 @@ int rfk_layers::decoder_layer_impl(
             TRY(rfk_cross_attention_cached(ctx, &w->cross_attn, temp, cross_out, proj_buf, cross_score_buf, K_cached, V_cached,
                                            B, Sq, Sk, n_keys, dim, dim, num_heads, q_rope_cos, q_rope_sin, k_rope_cos,
                                            k_rope_sin, stream));
-            TRY(rfk_rmsnorm_residual_f16_windows(x, cross_out, w->self_attn_norm_gamma, window_buf, B, patch_h, patch_w, dim,
-                                                 window_size, shift_size, 1, kEpsFp16, stream));
+            TRY(rfk_rmsnorm_residual_f16_windows_in_l2(x, cross_out, w->self_attn_norm_gamma, window_buf, B, patch_h, patch_w, dim,
+                                                       window_size, shift_size, 1, kEpsFp16, stream));
         }
         const int ws2 = window_size * window_size, nW = (patch_h / window_size) * (patch_w / window_size);
         TRY(swin_core(ctx, &w->self_attn, window_buf, qkv_buf, self_score_buf, proj_buf, B * nW, nW, ws2, dim, num_heads,
                       (shift_mask && shift_size > 0) ? shift_mask : nullptr, stream, swin_ss));
-        TRY(rfk_rmsnorm_residual_f16_windows(x, qkv_buf, w->ffn_norm_gamma, temp, B, patch_h, patch_w, dim, window_size,
-                                             shift_size, 2, kEpsFp16, stream));
+        TRY(rfk_rmsnorm_residual_f16_windows_in_l2(x, qkv_buf, w->ffn_norm_gamma, temp, B, patch_h, patch_w, dim, window_size,
+                                                   shift_size, 2, kEpsFp16, stream));
     } else {
         rfk_half* cross_out = qkv_buf;
         TRY(rfk_cross_attention_cached(ctx, &w->cross_attn, temp, cross_out, proj_buf, cross_score_buf, K_cached, V_cached, B,

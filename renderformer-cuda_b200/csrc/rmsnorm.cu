@@ -229,16 +229,21 @@ rmsnorm_generic_kernel(const TH* x, TH* xw, const TR* __restrict__ r,
     }
 }
 
-// Whether fp16 rows of 513 to 1024 elements go to one warp each (four chunks per lane) instead of four warps. They are the
-// decoder's, which the kernel before has left in L2: at 4096 rows the four-warp form is 1.7 rounds of CTAs of which each waits once
-// for memory, the one-warp form a single round with four times the loads in flight. Both have the same bits. Measured
-// (us, four warps / one, 1024 wide; plain, to windows, from windows with residual): 1024 rows 2.1 / 2.4, 2.7 / 2.9, 2.9 / 3.8;
-// 1600 rows 2.2 / 2.6, 4.0 / 3.0, 4.7 / 3.9; 2304 rows 2.8 / 2.7, 4.4 / 3.2, 4.9 / 4.2; 4096 rows 4.8 / 4.0, 6.6 / 4.7, 7.5 / 5.9;
-// 16384 rows 17.6 / 11.0, 22.4 / 12.5, 25.7 / 26.7 - the last is 134 MB of traffic, more than L2, and stays with four.
-static bool one_warp_per_row(int rows, int dim, bool windows, bool residual) {
+// Whether fp16 rows of 513 to 1024 elements go to one warp each (four chunks per lane) instead of four warps, with the same bits. With
+// four, 4096 rows are 1.7 rounds of CTAs of which each waits once for memory; with one, a single round that has four times the
+// loads in flight - but loads all it loads before it stores anything, which costs where a residual and x come from and go back to HBM.
+// So with a residual only the layers' own call asks for it, whose operands the kernels before have just written. Measured (us, four
+// warps / one, 1024 wide; operands in L2, then from HBM):
+//   plain             2304 rows 2.71 / 2.66, 3.23 / 3.30; 3136 rows 3.68 / 4.04, 4.31 / 4.71; 4096 rows 4.61 / 3.99, 4.96 / 4.86; 16384 rows
+//                     17.5 / 10.0, 17.5 / 12.4 (768 wide at 2304 rows 2.71 / 2.40, 2.87 / 3.40)
+//   with residual     4096 rows 4.86 / 5.38, 6.76 / 8.24; 8192 rows 9.21 / 8.90, 11.7 / 14.5: never
+//   to windows        1024 rows 2.7 / 2.9; 1600 rows 4.14 / 3.02, 4.59 / 3.72; 4096 rows 6.50 / 4.61, 7.06 / 5.53; 16384 rows 22.2 / 11.4, 22.6 / 14.4
+//   windows, residual 1600 rows 4.71 / 3.89, 5.12 / 6.45; 4096 rows 7.42 / 5.84, 8.09 / 8.75; 8192 rows 13.3 / 9.5, 14.0 / 15.3; 16384 rows, 134 MB
+//                     of traffic and more than L2, 25.5 / 26.7
+static bool one_warp_per_row(int rows, int dim, bool windows, bool residual, bool in_l2) {
     if (dim <= 512 || dim > 1024) return false;
-    if (residual && (long long)rows * dim * 8 > (96ll << 20)) return false;
-    return rows >= (windows ? 1280 : 2048);
+    if (residual && (!windows || !in_l2 || (long long)rows * dim * 8 > (96ll << 20))) return false;
+    return rows >= (windows ? 1280 : 4096);
 }
 
 template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
@@ -252,10 +257,12 @@ static int launch_variant(const TH* x, TH* xw, const TR* r, const float* gamma, 
     launch_pdl(rmsnorm_row_kernel<TH, TR, TY, N, WW, HAS_RES, WRITE_H, 0>,                             \
                dim3(ceil_div(rows, (kRmsThreads / 32) / WW)), dim3(kRmsThreads), 0, st, x, xw, r, gamma, y, \
                rows, dim, eps, WinRows{})
-        if (IsHalf<TH>::value && IsHalf<TY>::value && one_warp_per_row(rows, dim, false, HAS_RES)) {
-            launch_pdl(rmsnorm_row_kernel<TH, TR, TY, 4, 1, HAS_RES, WRITE_H, 0, 4>, dim3(ceil_div(rows, kRmsThreads / 32)), dim3(kRmsThreads),
-                       0, st, x, xw, r, gamma, y, rows, dim, eps, WinRows{});
-            return launch_status();
+        if constexpr (IsHalf<TH>::value && IsHalf<TY>::value && !HAS_RES) {
+            if (one_warp_per_row(rows, dim, false, false, false)) {
+                launch_pdl(rmsnorm_row_kernel<TH, TR, TY, 4, 1, false, WRITE_H, 0, 4>, dim3(ceil_div(rows, kRmsThreads / 32)), dim3(kRmsThreads),
+                           0, st, x, xw, r, gamma, y, rows, dim, eps, WinRows{});
+                return launch_status();
+            }
         }
         if (dim <= 256) RFK_RMS_LAUNCH(1, 1);
         else if (dim <= 512) RFK_RMS_LAUNCH(1, 2);
@@ -326,10 +333,8 @@ extern "C" int rfk_rmsnorm_residual_mixed_cast16(float* h, const rfk_half* r, co
                                                  dim, eps, as_stream(stream));
 }
 
-extern "C" int rfk_rmsnorm_residual_f16_windows(rfk_half* x, const rfk_half* r, const float* gamma,
-                                                rfk_half* y, int B, int H, int W, int dim,
-                                                int window_size, int shift_size, int windowed_operand,
-                                                float eps, rfk_stream_t stream) {
+static int rmsnorm_windows(rfk_half* x, const rfk_half* r, const float* gamma, rfk_half* y, int B, int H, int W, int dim, int window_size,
+                           int shift_size, int windowed_operand, float eps, bool in_l2, rfk_stream_t stream) {
     if (!x || !gamma || !y || B < 0 || H <= 0 || W <= 0 || dim <= 0) return RFK_EINVAL;
     if (window_size <= 0 || H % window_size || W % window_size || shift_size < 0) return RFK_EINVAL;
     if (windowed_operand != 1 && windowed_operand != 2) return RFK_EINVAL;
@@ -354,7 +359,7 @@ extern "C" int rfk_rmsnorm_residual_f16_windows(rfk_half* x, const rfk_half* r, 
                    dim3(ceil_div(rows, (kRmsThreads / 32) / WW)), dim3(kRmsThreads), 0, st, (const __half*)xh, xh, \
                    (const __half*)nullptr, gamma, (__half*)y, rows, dim, eps, wr)
 #define RFK_RMS_WIN_DIM(M)                               \
-    if (one_warp_per_row(rows, dim, true, r != nullptr)) { RFK_RMS_WIN(4, 1, M, 4); } \
+    if (one_warp_per_row(rows, dim, true, r != nullptr, in_l2)) { RFK_RMS_WIN(4, 1, M, 4); } \
     else if (dim <= 256) { RFK_RMS_WIN(1, 1, M, 1); }    \
     else if (dim <= 512) { RFK_RMS_WIN(1, 2, M, 1); }    \
     else if (dim <= 1024) { RFK_RMS_WIN(1, 4, M, 1); }   \
@@ -363,6 +368,19 @@ extern "C" int rfk_rmsnorm_residual_f16_windows(rfk_half* x, const rfk_half* r, 
 #undef RFK_RMS_WIN_DIM
 #undef RFK_RMS_WIN
     return launch_status();
+}
+
+extern "C" int rfk_rmsnorm_residual_f16_windows(rfk_half* x, const rfk_half* r, const float* gamma,
+                                                rfk_half* y, int B, int H, int W, int dim,
+                                                int window_size, int shift_size, int windowed_operand,
+                                                float eps, rfk_stream_t stream) {
+    return rmsnorm_windows(x, r, gamma, y, B, H, W, dim, window_size, shift_size, windowed_operand, eps, false, stream);
+}
+
+extern "C" int rfk_rmsnorm_residual_f16_windows_in_l2(rfk_half* x, const rfk_half* r, const float* gamma, rfk_half* y, int B, int H, int W,
+                                                      int dim, int window_size, int shift_size, int windowed_operand, float eps,
+                                                      rfk_stream_t stream) {
+    return rmsnorm_windows(x, r, gamma, y, B, H, W, dim, window_size, shift_size, windowed_operand, eps, true, stream);
 }
 
 extern "C" int rfk_rmsnorm_residual_f16(rfk_half* x, const rfk_half* r, const float* gamma,

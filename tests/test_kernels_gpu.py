@@ -215,3 +215,26 @@ def test_nerf_pe_has_the_same_bits_for_many_and_few_rows(rows, exps, in_dim, dty
     many = torch.empty(copies * rows, in_dim * 13, device="cuda", dtype=torch.float16)
     fn(x.repeat(copies, 1).contiguous(), many, 1, copies * rows, in_dim, 6, *exps, True)
     assert torch.equal(many.view(copies, rows, -1), few.expand(copies, rows, -1))
+
+
+@pytest.mark.parametrize("dim", [520, 1024])
+@pytest.mark.parametrize("copies,side", [(1, 24), (1, 40), (2, 64), (3, 64)])
+def test_window_norm_of_operands_in_l2_has_the_bits_of_the_other_split(copies, side, dim):
+    """The layers' form of the norm to and from windows takes one warp a row from 1280 rows up, the operator four with a residual."""
+    import ctypes
+    import torch
+    import renderformer_cuda_b200 as pkg
+    from renderformer_cuda_b200 import _abi
+    fn = _abi.load("rfk.h").rfk_rmsnorm_residual_f16_windows_in_l2
+    fn.argtypes, fn.restype = [ctypes.c_void_p] * 4 + [ctypes.c_int] * 7 + [ctypes.c_float, ctypes.c_void_p], ctypes.c_int
+    g = torch.Generator(device="cuda").manual_seed(dim + side)
+    rows = copies * side * side
+    gamma = 1 + 0.1 * torch.randn(dim, device="cuda", generator=g)
+    x0, r = (torch.randn(rows, dim, device="cuda", generator=g).half() for _ in range(2))
+    for operand in (1, 2):
+        x, y, xw, yw = x0.clone(), torch.empty_like(x0), x0.clone(), torch.empty_like(x0)
+        pkg.ops.rmsnorm_residual_f16_windows(x, r, gamma, y, copies, side, side, dim, 8, 4, operand)
+        rc = fn(*(ctypes.c_void_p(t.data_ptr()) for t in (xw, r, gamma, yw)), copies, side, side, dim, 8, 4, operand, pkg.ops.K_EPS_FP16,
+                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert rc == 0 and torch.equal(x, xw) and torch.equal(y, yw)
