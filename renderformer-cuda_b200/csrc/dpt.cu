@@ -38,12 +38,20 @@ namespace {
         if (rc_ != RFK_OK) return rc_;  \
     } while (0)
 
-// Which 3x3 convolutions (stride 1) the tcgen05 kernel of conv_tc.cu takes from the library: those of one view with more than 2^31
-// multiply-adds a tap, where its tiles of 256 pixels fill the SMs about twice. Measured with bias and SiLU (us, library and its pass / this
-// kernel): 256 -> 256 channels at 256^2 73 / 56, 160^2 28.6 / 31.7, 128^2 21 / 22, 64^2 9.7 / 19.6; 256 -> 128 at 512^2 187 / 140, 320^2
-// 55.6 / 55.9; 512 -> 256 at 128^2 31.7 / 32.7. A head over several views keeps the library, which chooses the order of its sums anew
-// for every batch size.
-bool own_conv(int B, int H, int W, int Cin, int Cout) { return B == 1 && (long long)H * W * Cin * Cout > (1LL << 31); }
+// Which 3x3 convolutions (stride 1) of a view the tcgen05 kernel of conv_tc.cu takes from the library: those of more than 2^31
+// multiply-adds a tap (smaller ones: 256 -> 256 channels at 128^2 20.4 / 21.1, 64^2 9.7 / 19.6), of which
+//   - maps of 256 channels whose tiles of 256 x 256 fill the pairs of SMs one and a half times, from 256 input channels up, and
+//   - every map beyond 170000 pixels, where the library's kernels take a step (256 -> 128 at 408^2 91.2 / 90.9, at 416^2 139.1 / 95.5).
+// Measured with bias and SiLU, the library and its pass / this kernel, us: 256 -> 256 at 184^2 (1.9 times) 34.5 / 31.5, 200^2 45.2 / 41.1,
+// 224^2 48.3 / 43.7, 256^2 73.5 / 56.3, 288^2 79.2 / 71.3; 512 -> 256 at 136^2 (1.04 times) 33.8 / 51.1, 160^2 (1.35) 46.9 / 51.6, 168^2 (1.57)
+// 55.0 / 52.8, 256^2 131 / 109; 64 -> 256 at 320^2 43.0 / 47.1, 448^2 83.5 / 82.6; 256 -> 128, whose narrow tiles read three quarters of the
+// operands for half the products, at 272^2 38.0 / 39.0, 320^2 54.3 / 55.4, 368^2 75.0 / 76.2, 448^2 152 / 108, 512^2 183 / 140.
+// A head over several views keeps the library, which chooses the order of its sums anew for every batch size.
+bool own_conv(int B, int H, int W, int Cin, int Cout, int sms) {
+    if (B != 1 || (long long)H * W * Cin * Cout <= (1LL << 31)) return false;
+    const long long tiles = ((long long)((H + 7) / 8) * ((W + 15) / 16) + 1) / 2 * (Cout / 256);
+    return (long long)H * W > 170000 || (Cout % 256 == 0 && Cin >= 256 && 2 * tiles > 3 * (sms / 2));
+}
 
 // Operands of the plan's comparison of the two (order_of_sums): fp16 in [-1, 1), a hash of the position
 __global__ void fill_hashed_kernel(__half* p, long long n, unsigned seed) {
@@ -80,6 +88,7 @@ struct rfk_dpt {
     rfk_half* out = nullptr;  // [B, out_dim, pH*ps, pW*ps]
     int n_convs = 0, n_own = 0;      // convolutions in all, and those of the tcgen05 kernel among them
     bool library_only = false;
+    int sms = 0;
     struct Order { int H, W, Cin, Cout, rows_outside; };
     std::vector<Order> orders;       // what order_of_sums found
 
@@ -190,7 +199,7 @@ struct rfk_dpt {
         const cudnnConvolutionFwdAlgo_t algo = perf[0].algo;
         size_t ws = 0;
         DNN_TRY(cudnnGetConvolutionForwardWorkspaceSize(dnn, xd, fd, cd, yd, algo, &ws));
-        if (!library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout) &&
+        if (!library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout, sms) &&
             rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout)) {
             const int Bn = B, rows_outside = order_of_sums(xd, fd, cd, yd, algo, ws, H, W, Cin, Cout);
             if (rows_outside >= 0) {
@@ -394,6 +403,11 @@ extern "C" int rfk_dpt_create_from(rfk_ctx* ctx, const rfk_dpt_weights* w, int B
     rfk_dpt* d = new rfk_dpt();
     d->ctx = ctx; d->w = *w; d->B = B; d->dim = dim; d->pH = patch_h; d->pW = patch_w; d->ps = patch_size;
     d->library_only = library_only != 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        delete d;
+        return (int)cudaGetLastError();
+    }
     if (cudnnCreate(&d->dnn) != CUDNN_STATUS_SUCCESS) { delete d; return 2000; }
     const int rc = d->build();
     if (rc != RFK_OK) { rfk_dpt_destroy(d); return rc; }

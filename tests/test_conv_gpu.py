@@ -150,3 +150,17 @@ def test_heads_have_the_bits_of_the_library_convolutions(pH, pW, F, B):
         L.rfk_dpt_destroy(dpt)
     assert torch.isfinite(images[0].float()).all() and torch.equal(*images)
     ctx.close()
+
+
+@pytest.mark.parametrize("p,own", [(40, 0), (48, 5), (52, 6), (64, 6), (72, 6)])
+def test_convolutions_that_leave_the_library(p, own):
+    """Those that gain by it: the five on the map of four times the grid from 184 pixels up, the one at full resolution beyond 170000
+    pixels; not that one of a 320 x 320 image, nor 512 -> 256 channels at 144 x 144 (81 tiles on 74 pairs)."""
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=3, dim=64, num_heads=1, ffn_hidden=64, enc_layers=0, dec_layers=1, with_dpt=True, dpt_features=256,
+                                 dpt_out_channels=(256, 512, 1024, 1024))
+    L, ctx = _abi.load("rfk_layers.h"), session.Ctx()
+    dpt, n = _plan(L, ctx, model, 1, p, p, 0)
+    L.rfk_dpt_destroy(dpt)
+    ctx.close()
+    assert n == own
