@@ -84,9 +84,8 @@ residual_add_silu_nhwc_kernel(__half* __restrict__ y, const __half* __restrict__
 // out[n, ho, wo, :] from in[n, :, :, :], align_corners = true; a thread owns 8 channels of one output column in ROWS
 // consecutive rows, so every access is 16 bytes, the column's coordinates are computed once, and the two source pixels of a source
 // row are loaded and converted once for all the output rows that lie on it (enlarging by two: five source rows for eight outputs,
-// where a thread per output loaded sixteen). Those loads, not the 134 MB it writes, bound the 256 -> 512 resample of 256 channels:
-// 71 us with a thread per output, 51 with eight rows; 128 -> 256 18.8 -> 12.8. Small maps want the threads more (32 -> 64: 2.6 us with
-// two rows, 4.1 with eight). Grid: x over
+// where a thread per output loads sixteen). Those loads, not the 134 MB it writes, bound the 256 -> 512 resample of 256 channels:
+// 71 us with a thread per output, 51 with eight rows; upsample_rows says which maps take how many. Grid: x over
 // (wo, channel chunk) of one output row, y = groups of rows, z = n: the row arithmetic is uniform over a CTA and the only
 // division left is a 32-bit one (with one thread per flat 64-bit index the three divisions cost more than the loads).
 template <int ROWS>
@@ -101,10 +100,27 @@ bilinear_upsample_nhwc_kernel(const __half* __restrict__ in, __half* __restrict_
     const long long n = blockIdx.z;
     const float h_scale = (H_out > 1) ? (float)(H_in - 1) / (H_out - 1) : 0.0f;
     const float w_scale = (W_out > 1) ? (float)(W_in - 1) / (W_out - 1) : 0.0f;
+    const long long C = (long long)c8 * 8;
+    if (ROWS == 1) {   // nothing to share
+        const int h_out = blockIdx.y;
+        const float h_in_f = __fmul_rn((float)h_out, h_scale), w_in_f = __fmul_rn((float)w_out, w_scale);
+        const int h0 = (int)h_in_f, w0 = (int)w_in_f;
+        const int h1 = min(h0 + 1, H_in - 1), w1 = min(w0 + 1, W_in - 1);
+        const float hf = __fsub_rn(h_in_f, (float)h0), wf = __fsub_rn(w_in_f, (float)w0);
+        const __half* base = in + n * H_in * W_in * C + cc * 8;
+        float v00[8], v01[8], v10[8], v11[8], o[8];
+        unpack8(ldg_half8(base + ((long long)h0 * W_in + w0) * C), v00);
+        unpack8(ldg_half8(base + ((long long)h0 * W_in + w1) * C), v01);
+        unpack8(ldg_half8(base + ((long long)h1 * W_in + w0) * C), v10);
+        unpack8(ldg_half8(base + ((long long)h1 * W_in + w1) * C), v11);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) o[k] = bilerp_ref(v00[k], v01[k], v10[k], v11[k], hf, wf);
+        store8(out + ((n * H_out + h_out) * W_out) * C + (long long)idx * 8, o);
+        return;
+    }
     const float w_in_f = __fmul_rn((float)w_out, w_scale);
     const int w0 = (int)w_in_f, w1 = min(w0 + 1, W_in - 1);
     const float wf = __fsub_rn(w_in_f, (float)w0);   // not contracted with the product: so are the operators this one equals
-    const long long C = (long long)c8 * 8;
     const __half* left = in + (n * H_in * W_in + w0) * C + cc * 8;
     const __half* right = in + (n * H_in * W_in + w1) * C + cc * 8;
     float t0[8], t1[8], b0[8], b1[8];   // the two pixels of source rows h0 and h1
@@ -286,6 +302,16 @@ extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_ha
     return launch_status();
 }
 
+// Output rows a thread: 1, 4 or 8, by the number of CTAs that one row a thread would be. Sharing source rows needs output rows closer
+// together than source rows, and costs threads. Measured (us, one / four / eight rows; 256 channels): 32 -> 64 (512 CTAs) 2.46 / 2.86 / 3.99,
+// 56 -> 112 (1568) 4.71 / 5.12 / 5.02, 64 -> 128 (2048) 5.63 / 5.12 / 5.01, 72 -> 144 (2592) 6.86 / 6.14 / 7.68, 88 -> 176 (3872) 9.52 / 7.88 / 7.88,
+// 128 -> 256 (8192) 18.6 / 14.5 / 12.7, 256 -> 512 70.8 / 58.4 / 50.7; shrinking, 256 -> 230 15.5 / 13.9 / 14.2, 256 -> 200 11.9 / 11.3 / 12.1,
+// 512 -> 256 25.3 / 31.8 / 31.2.
+static int upsample_rows(long long ctas, int H_in, int H_out) {
+    if (8LL * H_out < 7LL * H_in || ctas < 1800) return 1;
+    return ctas < 3800 ? 4 : 8;
+}
+
 extern "C" int rfk_bilinear_upsample_nhwc(const rfk_half* in, rfk_half* out, int N, int H_in, int W_in, int H_out, int W_out,
                                           int C, rfk_stream_t stream) {
     if (!in || !out || N < 0 || C <= 0 || H_in <= 0 || W_in <= 0 || H_out <= 0 || W_out <= 0) return RFK_EINVAL;
@@ -293,10 +319,10 @@ extern "C" int rfk_bilinear_upsample_nhwc(const rfk_half* in, rfk_half* out, int
     if (C % 8 || !aligned16(in) || !aligned16(out)) return RFK_EUNSUPPORTED;
     const long long per_row = (long long)W_out * (C / 8);
     if (per_row > 0x7fffffffLL || H_out > 65535 || N > 65535) return RFK_EUNSUPPORTED;
-    const bool many = per_row * H_out * N >= (1 << 18);   // 16-byte outputs: 64 -> 128 of 256 channels and larger
-    const int rows = many ? 8 : 2;
+    const int rows = upsample_rows(ceil_div(per_row, 256) * H_out * N, H_in, H_out);
     const dim3 grid((unsigned)ceil_div(per_row, 256), (unsigned)ceil_div(H_out, rows), (unsigned)N);
-    launch_pdl(many ? bilinear_upsample_nhwc_kernel<8> : bilinear_upsample_nhwc_kernel<2>, grid, dim3(256), 0, as_stream(stream),
+    launch_pdl(rows == 8 ? bilinear_upsample_nhwc_kernel<8> : rows == 4 ? bilinear_upsample_nhwc_kernel<4> : bilinear_upsample_nhwc_kernel<1>,
+               grid, dim3(256), 0, as_stream(stream),
                (const __half*)in, (__half*)out, H_in, W_in, H_out, W_out, C / 8);
     return launch_status();
 }

@@ -262,3 +262,16 @@ def test_channels_last_upsample_of_many_rows_per_thread_equals_the_nchw_operator
     o.bilinear_upsample(x, want, N, C, Hi, Wi, Ho, Wo)
     o.bilinear_upsample_nhwc(_nhwc(x), got, N, Hi, Wi, Ho, Wo, C)
     assert torch.equal(got, _nhwc(want))
+
+
+@pytest.mark.parametrize("C,Hi,Wi,Ho,Wo", [(256, 128, 128, 256, 256), (64, 70, 300, 203, 600), (64, 100, 200, 199, 400), (256, 36, 36, 72, 72),
+                                           (64, 200, 64, 175, 2048), (64, 200, 64, 174, 2048), (8, 6000, 1, 6553, 4)])
+def test_channels_last_upsample_at_the_lines_of_its_forms(C, Hi, Wi, Ho, Wo):
+    """Eight, four and one output row a thread, last groups short, and both sides of the shrinking that still shares source rows."""
+    o = _ops()
+    g = torch.Generator(device="cuda").manual_seed(Ho)
+    x = torch.randn(1, C, Hi, Wi, device="cuda", generator=g).half()
+    want, got = torch.empty(1, C, Ho, Wo, device="cuda", dtype=H16), torch.full((1, Ho, Wo, C), 7.0, device="cuda", dtype=H16)
+    o.bilinear_upsample(x, want, 1, C, Hi, Wi, Ho, Wo)
+    o.bilinear_upsample_nhwc(_nhwc(x), got, 1, Hi, Wi, Ho, Wo, C)
+    assert torch.equal(got, _nhwc(want))
