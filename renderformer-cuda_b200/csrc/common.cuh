@@ -131,6 +131,17 @@ __device__ __forceinline__ void load8(const __half* p, float (&f)[8]) { unpack8(
 __device__ __forceinline__ void load8(const float* p, float (&f)[8]) { ld_float8(p, f); }
 __device__ __forceinline__ void store8(__half* p, const float (&f)[8]) { st_half8(p, pack8(f)); }
 __device__ __forceinline__ void store8(float* p, const float (&f)[8]) { st_float8(p, f); }
+// The same fp16 values at p and at p + distance, one store each (a struct of __half2 assigned as a whole is stored member by member).
+__device__ __forceinline__ void store_twice(__half* p, const float (&f)[8], int distance) {
+    const Half8 h = pack8(f);
+    st_half8(p, h);
+    st_half8(p + distance, h);
+}
+__device__ __forceinline__ void store_twice(__half* p, const float (&f)[2], int distance) {
+    const __half2 h = __floats2half2_rn(f[0], f[1]);
+    *reinterpret_cast<__half2*>(p) = h;
+    *reinterpret_cast<__half2*>(p + distance) = h;
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

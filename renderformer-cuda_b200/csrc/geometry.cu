@@ -106,8 +106,9 @@ world_to_cam_vec8_kernel(const float* __restrict__ c2w, __half* tri, __half* vn,
 // thread -> (token t in [0, seq_pad), chunk j of PER table angles in the first half of head_dim).
 // Every thread rebuilds the token's 9 camera-space coordinates (27 FMAs); the j == 0
 // thread also stores the geometry outputs. cosf and sinf are long dependent chains, and 5665 tokens of eight-angle threads are
-// five warps an SM: with two angles a thread 4.9 -> 3.8 us (333 tokens 4.6 -> 2.8; 64-wide heads). With twice the angles, 5665
-// tokens of 128-wide heads, there are threads enough and the rebuilt coordinates count: eight 5.5, two 6.6 us.
+// five warps an SM: with two angles a thread 4.8 -> 3.6 us (333 tokens 4.6 -> 2.7; 64-wide heads). With many tokens there are threads
+// enough, and the rebuilt coordinates and the narrower stores count (eight / two angles): 9000 tokens of 64-wide heads, 144000 threads of
+// two, 4.7 / 4.3 us; 12000 tokens, 192000, 5.4 / 6.6; 5665 tokens of 128-wide heads, 181000, 5.3 / 6.7.
 template <int PER>
 __global__ void __launch_bounds__(256)
 view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ tri_world,
@@ -186,16 +187,8 @@ view_geometry_kernel(const float* __restrict__ c2w, const __half* __restrict__ t
         sn[i] = sinf(val);
     }
     const size_t o = (size_t)t * head_dim + j * PER;
-    struct __align__(2 * PER) Chunk { __half2 v[PER / 2]; } hc, hs;
-#pragma unroll
-    for (int i = 0; i < PER / 2; ++i) {
-        hc.v[i] = __floats2half2_rn(cs[2 * i], cs[2 * i + 1]);
-        hs.v[i] = __floats2half2_rn(sn[2 * i], sn[2 * i + 1]);
-    }
-    *reinterpret_cast<Chunk*>(k_cos + o) = hc;
-    *reinterpret_cast<Chunk*>(k_cos + o + head_dim / 2) = hc;
-    *reinterpret_cast<Chunk*>(k_sin + o) = hs;
-    *reinterpret_cast<Chunk*>(k_sin + o + head_dim / 2) = hs;
+    store_twice(k_cos + o, cs, head_dim / 2);
+    store_twice(k_sin + o, sn, head_dim / 2);
 }
 
 }  // namespace rfk
@@ -245,7 +238,7 @@ extern "C" int rfk_view_geometry(const float* c2w, const rfk_half* tri_world,
     if (head_dim <= 0 || head_dim % 16 || !aligned16(k_cos) || !aligned16(k_sin))
         return RFK_EUNSUPPORTED;
     if (seq_pad == 0) return RFK_OK;
-    const bool many = (long long)seq_pad * (head_dim / 4) > 100000;
+    const bool many = (long long)seq_pad * (head_dim / 4) > 150000;   // threads with two angles each
     const long long n = (long long)seq_pad * (head_dim / (many ? 16 : 4));
     launch_pdl(many ? view_geometry_kernel<8> : view_geometry_kernel<2>, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream),
         c2w, (const __half*)tri_world, (const __half*)vn_world, world_center, learned_freqs,

@@ -23,8 +23,9 @@ namespace rfk {
 
 // thread -> (token, chunk of PER angles of the first half); writes both halves (they are equal). One scene's tables are short work
 // of a long dependent chain each (cosf and sinf with their reductions), so what counts is how many run side by side: with eight
-// angles a thread the tables of 5633 triangles took 3.5 us, with two 2.1 (301 triangles 3.3 and 1.8; 64-wide heads). Eight keep
-// the wider stores where threads abound: 45064 triangles and 128-wide heads, 1.4 million threads of two, 11.8 against 13.5 us.
+// angles a thread the tables of 5633 triangles took 3.6 us, with two 2.2 (301 triangles 3.4 and 1.9; 64-wide heads). Eight keep
+// the wider stores where threads abound (eight / two angles, 64-wide heads): 55000 triangles, 0.88 million threads of two, 9.8 / 8.8 us;
+// 70000, 1.12 million, 9.9 / 10.9; 140000 17.0 / 20.3; 45000 with 128-wide heads, 1.44 million, 11.9 / 13.5.
 template <int PER>
 __global__ void __launch_bounds__(256)
 rope_table_vec_kernel(const __half* __restrict__ pos, const float* __restrict__ freqs,
@@ -51,16 +52,8 @@ rope_table_vec_kernel(const __half* __restrict__ pos, const float* __restrict__ 
         s[i] = sinf(val);
     }
     const size_t o = (size_t)tok * head_dim + j * PER;
-    struct __align__(2 * PER) Chunk { __half2 v[PER / 2]; } hc, hs;
-#pragma unroll
-    for (int i = 0; i < PER / 2; ++i) {
-        hc.v[i] = __floats2half2_rn(c[2 * i], c[2 * i + 1]);
-        hs.v[i] = __floats2half2_rn(s[2 * i], s[2 * i + 1]);
-    }
-    *reinterpret_cast<Chunk*>(out_cos + o) = hc;
-    *reinterpret_cast<Chunk*>(out_cos + o + head_dim / 2) = hc;
-    *reinterpret_cast<Chunk*>(out_sin + o) = hs;
-    *reinterpret_cast<Chunk*>(out_sin + o + head_dim / 2) = hs;
+    store_twice(out_cos + o, c, head_dim / 2);
+    store_twice(out_sin + o, s, head_dim / 2);
 }
 
 __global__ void __launch_bounds__(256)
