@@ -336,9 +336,10 @@ namespace pair { using namespace pair_ptx; }
 //   their loops as a whole, one elected lane issuing, so that descriptors, coordinates and counters live in uniform registers.
 //   With one block per stage and single threads' loops a K block took 0.30 us on every tile size, the cost of issuing and not of
 //   the operands; two blocks and the elected issuer took the 64 x 32 tile to 0.14 us, the elected producer to 0.12 us (256 x 1024 x
-//   4096 10.96 -> 9.95 us, weights from HBM; the tensor pipe alone would take 0.05 us). Half the ring costs 7 % (the copies in flight cover
-//   their latency); one copy per operand and stage instead of two, and weights asked for ahead of the kernel's wait for its
-//   predecessor, changed nothing or cost (320 x 320 views +4 %).
+//   4096 10.96 -> 9.95 us, weights from HBM; the tensor pipe alone would take 0.05 us). The 128 x 64 tile keeps a producer of one lane:
+//   1024 x 1024 x 4096 takes 12.0 us with it and 13.3 with the elected one (weights from HBM 12.8 and 13.3), 256 x 3072 x 1024 5.2 and
+//   5.4. Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
+//   weights asked for ahead of the kernel's wait for its predecessor, changed nothing or cost (320 x 320 views +4 %).
 //   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
 //   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
 // The epilogue's threads store their own rows: a tile row is 32 to 256 bytes, one to eight whole sectors.
@@ -403,28 +404,32 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_trigger();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ producer (the warp's elected lane)
-        const bool leader = tc::elect_one();
-        int it = 0, s = 0, par = 1;   // stage of `it`, and the parity of its barrier's previous phase
-        for (; it < num_st; ++it) {
-            if (it >= kStages && !tc::mbar_wait_warp(&ctrl->empty[s], par, abort_flag)) break;
-            if (leader) {
-                tc::mbar_arrive_expect_tx(&ctrl->full[s], kStage);
+        // ------------------------------------------------------------ producer (the warp's elected lane, or lane 0 alone)
+        constexpr bool kWhole = !(BM_ == 128 && BN_ == 64);
+        const bool leader = kWhole ? tc::elect_one() : lane == 0;
+        if (kWhole || leader) {
+            int it = 0, s = 0, par = 1;   // stage of `it`, and the parity of its barrier's previous phase
+            for (; it < num_st; ++it) {
+                if (it >= kStages && !(kWhole ? tc::mbar_wait_warp(&ctrl->empty[s], par, abort_flag) : tc::mbar_wait(&ctrl->empty[s], par, abort_flag)))
+                    break;
+                if (leader) {
+                    tc::mbar_arrive_expect_tx(&ctrl->full[s], kStage);
 #pragma unroll
-                for (int h = 0; h < kSub; ++h) {
-                    const uint32_t sA = base + s * kStage + h * kBlock, sW = sA + BM_ * BK * 2;
-                    const int x = (it * kSub + h) * BK;
-                    tma_load_2d(sA, &map_a, x, m0, &ctrl->full[s]);
-                    tma_load_2d(sW, &map_w0, x, n0, &ctrl->full[s]);
-                    if (kGate) tma_load_2d(sW + BN_OUT * BK * 2, &map_w1, x, n0, &ctrl->full[s]);
+                    for (int h = 0; h < kSub; ++h) {
+                        const uint32_t sA = base + s * kStage + h * kBlock, sW = sA + BM_ * BK * 2;
+                        const int x = (it * kSub + h) * BK;
+                        tma_load_2d(sA, &map_a, x, m0, &ctrl->full[s]);
+                        tma_load_2d(sW, &map_w0, x, n0, &ctrl->full[s]);
+                        if (kGate) tma_load_2d(sW + BN_OUT * BK * 2, &map_w1, x, n0, &ctrl->full[s]);
+                    }
                 }
+                if (++s == kStages) { s = 0; par ^= 1; }
             }
-            if (++s == kStages) { s = 0; par ^= 1; }
-        }
-        if (leader && *abort_flag) {   // giving up: wait (bounded) for the last copy of each stage before the CTA exits
-            for (int t = 0; t < kStages && t < it; ++t) {
-                const int last = ((it - 1 - t) / kStages) * kStages + t;
-                tc::mbar_wait_drain(&ctrl->full[t], (last / kStages) & 1);
+            if (leader && *abort_flag) {   // giving up: wait (bounded) for the last copy of each stage before the CTA exits
+                for (int t = 0; t < kStages && t < it; ++t) {
+                    const int last = ((it - 1 - t) / kStages) * kStages + t;
+                    tc::mbar_wait_drain(&ctrl->full[t], (last / kStages) & 1);
+                }
             }
         }
         __syncwarp();
