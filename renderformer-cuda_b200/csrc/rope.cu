@@ -291,7 +291,9 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
 #pragma unroll
     for (int k = 0; k < NPAIR; ++k) {
         const int p = lane + 32 * WPR * k;
-        if (p < npairs) {
+        if (HEADS && !live) {   // a row past the end only reaches the barrier: its clamped row is being overwritten in place by its own warps
+            xl[k] = xh[k] = Half8{};
+        } else if (p < npairs) {
             const __half* src = HEADS ? out + out_at(p) : xr + (p / cpt) * head_dim + (p % cpt) * 8;
             xl[k] = HEADS ? ld_half8(src) : ldcs_half8(src);
             xh[k] = HEADS ? ld_half8(src + half_d) : ldcs_half8(src + half_d);

@@ -115,7 +115,8 @@ def test_cut_of_the_last_round_and_images(with_dpt):
     s.close()
 
 
-@pytest.mark.parametrize("S,heads,hd", [(1, 4, 64), (33, 4, 64), (300, 2, 128), (1100, 16, 64), (4700, 4, 64), (64, 8, 32)])
+@pytest.mark.parametrize("S,heads,hd", [(1, 4, 64), (33, 4, 64), (300, 2, 128), (1100, 16, 64), (4700, 4, 64), (333, 16, 64), (1, 8, 128),
+                                        (77, 16, 128), (512, 20, 64), pytest.param(64, 8, 32, id="packed_both_times-64-8-32")])
 @pytest.mark.parametrize("rope", [True, False])
 def test_head_split_projection_has_the_bits_of_the_separate_epilogue(S, heads, hd, rope):
     """Self-attention of one batch element: q, k, v stored head-split by their projection, q and k normalised and rotated in
