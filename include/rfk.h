@@ -38,7 +38,8 @@ enum {
     RFK_EINVAL      = -1,  /* null pointer, negative size, unsupported shape */
     RFK_EUNSUPPORTED= -2,  /* shape outside what the kernels implement       */
     RFK_ETOOBIG     = -3,  /* size beyond a documented fixed maximum         */
-    RFK_EKERNEL     = -4   /* a kernel gave up on a bounded device-side wait (rfk_flash_attention_error) */
+    RFK_EKERNEL     = -4   /* a kernel gave up on a bounded device-side wait (rfk_flash_attention_error,
+                             rfk_gemm_error, rfk_conv_error) */
 };
 
 /* Library identification: returns a static string "rfk <version> sm_100a". */
@@ -377,6 +378,10 @@ int rfk_gemm_heads_tile(int M, int N, const int* resident);
  * 1 a bounded wait ran out, 2 shared memory window not 1024-byte aligned. Synchronises the device.
  * No reference counterpart. */
 int rfk_gemm_error(int* code, int clear);
+/* The same for the convolution kernel that rfk_dpt_forward launches (rfk_layers.h) for the large 3x3 convolutions of a
+ * view: code as above; after a non-zero one the images made since the word was last clear are not to be trusted.
+ * Synchronises the device. No reference counterpart. */
+int rfk_conv_error(int* code, int clear);
 
 /* Swin window attention core in one kernel: per (window, head) O = softmax(scale * Q K^T [masked]) V.
  * Q, K, V [BnW, heads, 64, 64] fp16; O [BnW * 64, heads * 64] fp16 (token-major, what the output

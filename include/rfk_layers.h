@@ -265,8 +265,9 @@ int rfk_dpt_destroy(rfk_dpt* dpt);
 /* features: HOST array of 4 device pointers, the decoder feature taps [B, patch_h*patch_w, dim]
  * fp16. Writes the image [B, out_dim, H, W] fp16 (before the ELU / 10^x - 1 post-process) into the
  * plan's own buffer (rfk_dpt_output) and, if image_out != NULL, copies it there. Launch-only:
- * capturable. cuDNN convolutions for k > 1 and the transposed ones, cuBLAS for 1x1 (as the
- * reference), rfk kernels for permute / bias / SiLU / residual / bilinear upsampling.
+ * capturable. The large 3x3 convolutions of a single view run on the library's own tcgen05 kernel (a bounded wait of
+ * its that runs out shows in rfk_conv_error), the other ones of k > 1 are cuDNN calls; 1x1 and transposed convolutions
+ * are projections (rfk_gemm_f16), the rest rfk kernels for bias / SiLU / residual / bilinear upsampling.
  * replaces rf::dpt_forward — src/layers/dpt.h:64-72, src/layers/dpt.cu:322-461 */
 int rfk_dpt_forward(rfk_dpt* dpt, const rfk_half* const* features, rfk_half* image_out,
                     rfk_stream_t stream);
@@ -384,8 +385,9 @@ int rfk_session_download(rfk_session* s, rfk_half* h_out, size_t bytes);
 /* Queues the device->host copy of the last submitted frame's token map on the session's copy
  * stream (h_out should be pinned); it runs as soon as that frame is done, overlapping the
  * next frame. rfk_session_drain waits for every submitted frame and copy and returns RFK_EKERNEL if
- * the fused attention kernel has reported a time-out since its error word was last cleared
- * (rfk_flash_attention_error); rfk_session_finalize makes the same check after its warm-up view. */
+ * an attention, projection or convolution kernel has reported a time-out since its error word was last cleared
+ * (rfk_flash_attention_error, rfk_gemm_error, rfk_conv_error: the words belong to the device, so clear the one that
+ * is set before another session is used); rfk_session_finalize makes the same check after its warm-up view. */
 int rfk_session_download_async(rfk_session* s, rfk_half* h_out, size_t bytes);
 int rfk_session_drain(rfk_session* s);
 /* Timing marks: mark_begin records a CUDA event on the session's render stream; mark_end

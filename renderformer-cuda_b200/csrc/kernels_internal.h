@@ -70,8 +70,6 @@ extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_
 // whether it takes these operands on the current device
 extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
                                        const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out);
-// the convolution's time-out word, as rfk_gemm_error
-extern "C" int rfk_conv_error(int* code, int clear);
 
 // y += r in fp16, and silu(y) beside it: rfk_residual_add and rfk_silu in one pass; n % 8 == 0, 16-byte aligned
 extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);

@@ -419,6 +419,14 @@ def gemm_error(clear=True):
     return code.value
 
 
+def conv_error(clear=True):
+    """Error word of the tcgen05 convolution kernel of the DPT head on the current device (0 = none)."""
+    import ctypes
+    code = ctypes.c_int(-1)
+    _call("rfk_conv_error", ctypes.byref(code), int(clear))
+    return code.value
+
+
 # -------------------------------------------------------------- activations
 
 @_native

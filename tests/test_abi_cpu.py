@@ -134,3 +134,10 @@ void reference_style_caller(half* q, half* k, const float* g, const half* c, con
     proc = subprocess.run(cmd, capture_output=True, text=True)
     assert proc.returncode == 0, proc.stderr
     assert out.exists()
+
+
+def test_every_time_out_word_has_a_public_reader():
+    """A session refuses to go on while one is set, and whoever calls the layers has to be able to see and clear it."""
+    syms = _abi.declared_symbols()["rfk.h"]
+    for word in ("flash_attention_error", "gemm_error", "conv_error"):
+        assert "rfk_" + word in syms and callable(getattr(pkg.ops, word))

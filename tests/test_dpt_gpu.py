@@ -13,6 +13,16 @@ H16 = torch.float16
 VP = ctypes.c_void_p
 
 
+@pytest.fixture(autouse=True)
+def _no_time_out():
+    import renderformer_cuda_b200 as pkg
+    words = (pkg.ops.conv_error, pkg.ops.gemm_error, pkg.ops.flash_attention_error)
+    for word in words:
+        word(clear=True)
+    yield
+    assert [word(clear=True) for word in words] == [0, 0, 0]
+
+
 def _mods():
     from renderformer_cuda_b200 import _abi, session
     return _abi.load("rfk_layers.h"), session

@@ -21,7 +21,7 @@ def _paths():
     ops.gemm_set_path(0)
     ops.flash_attention_set_path(0)
     torch.cuda.synchronize()
-    assert ops.gemm_error() == 0 and ops.flash_attention_error() == 0
+    assert ops.gemm_error() == 0 and ops.flash_attention_error() == 0 and ops.conv_error() == 0
 
 
 def _render(with_dpt):
