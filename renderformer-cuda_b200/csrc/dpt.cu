@@ -245,34 +245,30 @@ struct rfk_dpt {
         return RFK_OK;
     }
 
-    // residual convolution unit (src/layers/dpt.cu:397-409): *result <- conv2(silu(conv1(x_silu))) + x with x_silu = silu(x), which
-    // whatever made x has left beside it; x is left as it was
-    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, const rfk_half* x_silu, int F, int H, int W, rfk_half** result) {
-        const long long n = (long long)B * F * H * W;
-        rfk_half* t0 = alloc((size_t)n);
-        rfk_half* t1 = alloc((size_t)n);
-        if (!t0 || !t1) return (int)cudaErrorMemoryAllocation;
-        TRY(add_conv(x_silu, -1, r.conv1_w, r.conv1_b, t1, F, H, W, F, 3, 1, 1, /*silu=*/true));
-        TRY(add_conv(t1, -1, r.conv2_w, r.conv2_b, t0, F, H, W, F, 3, 1, 1, /*silu=*/false, /*residual=*/x));
-        *result = t0;
+    // residual convolution unit (src/layers/dpt.cu:397-409): y <- conv2(silu(conv1(y))) + x, where y holds silu(x), which whatever made x
+    // has left there; x is left as it was. *spare: a buffer of the same size that nothing needs any more once the unit is done.
+    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, rfk_half* y, int F, int H, int W, rfk_half** spare) {
+        rfk_half* t = alloc((size_t)B * F * H * W);
+        if (!t) return (int)cudaErrorMemoryAllocation;
+        TRY(add_conv(y, -1, r.conv1_w, r.conv1_b, t, F, H, W, F, 3, 1, 1, /*silu=*/true));
+        TRY(add_conv(t, -1, r.conv2_w, r.conv2_b, y, F, H, W, F, 3, 1, 1, /*silu=*/false, /*residual=*/x));
+        *spare = t;
         return RFK_OK;
     }
 
     // feature fusion block (src/layers/dpt.cu:411-426); returns the [B, th, tw, F] result buffer in *result. path_silu and lr_silu:
-    // SiLU of path_in and lr, where they are a residual unit's first operand as they come (path_silu may be null)
-    int add_refinenet(int i, rfk_half* path_in, const rfk_half* path_silu, const rfk_half* lr, const rfk_half* lr_silu, int ph, int pw,
-                      int th, int tw, rfk_half** result) {
+    // SiLU of path_in and lr, where they are a residual unit's first operand as they come (path_silu may be null); both are overwritten
+    int add_refinenet(int i, rfk_half* path_in, rfk_half* path_silu, const rfk_half* lr, rfk_half* lr_silu, int ph, int pw, int th, int tw,
+                      rfk_half** result) {
         const int F = w.features_dim;
         const rfk_ffb_weights& f = w.refinenet[i];
         const long long n = (long long)B * F * ph * pw;
         if (f.has_resconv1) {
             if (!lr) return RFK_EINVAL;
-            rfk_half* r1 = nullptr;
-            TRY(add_rcu(f.rcu1, lr, lr_silu, F, ph, pw, &r1));
-            rfk_half* s = alloc((size_t)n);
-            if (!s) return (int)cudaErrorMemoryAllocation;
+            rfk_half* s = nullptr;
+            TRY(add_rcu(f.rcu1, lr, lr_silu, F, ph, pw, &s));
             program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
-                return rfk_residual_add_silu_nhwc(path_in, r1, s, n, (rfk_stream_t)st);
+                return rfk_residual_add_silu_nhwc(path_in, lr_silu, s, n, (rfk_stream_t)st);
             });
             path_silu = s;
         } else if (!path_silu) {
@@ -281,8 +277,9 @@ struct rfk_dpt {
             program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int { return rfk_silu(path_in, s, n, (rfk_stream_t)st); });
             path_silu = s;
         }
-        rfk_half* r2 = nullptr;
-        TRY(add_rcu(f.rcu2, path_in, path_silu, F, ph, pw, &r2));
+        rfk_half* spare = nullptr;
+        TRY(add_rcu(f.rcu2, path_in, path_silu, F, ph, pw, &spare));
+        const rfk_half* r2 = path_silu;
         rfk_half* up = alloc((size_t)B * F * th * tw);
         rfk_half* res = alloc((size_t)B * F * th * tw);
         if (!up || !res) return (int)cudaErrorMemoryAllocation;
@@ -320,11 +317,12 @@ struct rfk_dpt {
                 TRY(add_conv(projected, -1, w.resize_w[i], w.resize_b[i], resized[i], C, pH, pW, C, 3, 2, 1));
             }
         }
-        rfk_half *layer_rn[4], *rn_silu[4];
+        rfk_half *layer_rn[4], *rn_silu[4] = {};
         for (int i = 0; i < 4; ++i) {
             layer_rn[i] = alloc((size_t)B * F * rh[i] * rw[i]);
-            rn_silu[i] = alloc((size_t)B * F * rh[i] * rw[i]);
-            if (!layer_rn[i] || !rn_silu[i]) return (int)cudaErrorMemoryAllocation;
+            const bool opens_unit = i == 3 || w.refinenet[i].has_resconv1;
+            if (opens_unit) rn_silu[i] = alloc((size_t)B * F * rh[i] * rw[i]);
+            if (!layer_rn[i] || (opens_unit && !rn_silu[i])) return (int)cudaErrorMemoryAllocation;
             TRY(add_conv(resized[i], -1, w.layer_rn_w[i], nullptr, layer_rn[i], w.out_channels[i], rh[i], rw[i], F, 3, 1, 1, false, nullptr,
                          rn_silu[i]));
         }

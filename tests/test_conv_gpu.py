@@ -164,3 +164,29 @@ def test_convolutions_that_leave_the_library(p, own):
     L.rfk_dpt_destroy(dpt)
     ctx.close()
     assert n == own
+
+
+def test_a_head_holds_no_copies_beside_its_maps():
+    """Device memory of a planned head of a 512 x 512 view: the SiLU copies that producers leave are the buffers in which the residual
+    units then build their results, so there is one map per unit beside them. The rounding of allocations to 2 MB and the library's
+    handle and workspace are 18 MB more; copies beside the maps would be 132."""
+    from renderformer_cuda_b200 import session
+    p, F, ch = 64, 256, (256, 512, 1024, 1024)
+    model = session.Model.random(seed=3, dim=64, num_heads=1, ffn_hidden=64, enc_layers=0, dec_layers=1, with_dpt=True, dpt_features=F, dpt_out_channels=ch)
+    L, ctx = _abi.load("rfk_layers.h"), session.Ctx()
+    rn = [(s * p) ** 2 * F for s in (4, 2, 1)] + [(p // 2) ** 2 * F]
+    maps = sum(c * p * p for c in ch) + 2 * sum((c * f * f * p * p) for c, f in ((ch[0], 4), (ch[1], 2))) + ch[3] * (p // 2) ** 2
+    maps += 2 * sum(rn) + 2 * sum(rn[:3]) + rn[3]                                # layer_rn and its SiLU, one more per residual unit
+    maps += 2 * (64 * p * p * F + sum(rn[:3]))                                   # resampled and projected fusion outputs
+    maps += (8 * p) ** 2 * (2 * (F // 2) + 32 + 3 + 3)
+    filters = sum(c * c * f * f for c, f in ((ch[0], 4), (ch[1], 2))) + 9 * (ch[3] ** 2 + sum(ch) * F + 14 * F * F + F * F // 2 + 32 * F // 2)
+    held = []
+    for _ in range(2):   # the first plan of a process also loads the library
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        dpt, _ = _plan(L, ctx, model, 1, p, p, 0)
+        held.append(before - torch.cuda.mem_get_info()[0])
+        L.rfk_dpt_destroy(dpt)
+    ctx.close()
+    print(f"held {held[1] / 1e6:.1f} MB, maps and filters {2 * (maps + filters) / 1e6:.1f} MB")
+    assert held[1] <= 2 * (maps + filters) + (60 << 20)
