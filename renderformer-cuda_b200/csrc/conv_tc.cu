@@ -123,9 +123,9 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         ctrl->abort = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0 && aligned) {  // each CTA allocates its own tensor memory
-        tc::tmem_alloc(&ctrl->tmem_base, kTmemCols);
-        tc::tmem_relinquish();
+    if (warp == 0 && aligned) {  // the same in both CTAs of the pair
+        tmem_alloc_pair(&ctrl->tmem_base, kTmemCols);
+        tmem_relinquish_pair();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -336,7 +336,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     cluster_sync();
     if (warp == 0) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem_cta, kTmemCols);
+        tmem_dealloc_pair(tmem_cta, kTmemCols);
     }
     if (tid == 0 && ctrl->abort) atomicCAS(&g_conv_tc_error, 0, kErrTimeout);
 }

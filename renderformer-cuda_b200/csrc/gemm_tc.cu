@@ -823,9 +823,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         ctrl->abort = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0 && aligned) {  // each CTA allocates its own tensor memory (all 512 columns: both get the same address)
-        tc::tmem_alloc(&ctrl->tmem_base, kTmemCols);
-        tc::tmem_relinquish();
+    if (warp == 0 && aligned) {  // the same in both CTAs of the pair
+        tmem_alloc_pair(&ctrl->tmem_base, kTmemCols);
+        tmem_relinquish_pair();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -950,7 +950,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     cluster_sync();
     if (warp == 0) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem_cta, kTmemCols);
+        tmem_dealloc_pair(tmem_cta, kTmemCols);
     }
     if (tid == 0 && ctrl->abort) atomicCAS(&g_gemm_tc_error, 0, kErrTimeout);
     if (tid == 0) RFK_STAMP(6);   // CTA exit

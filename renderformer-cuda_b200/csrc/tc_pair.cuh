@@ -35,6 +35,18 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* 
         ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
 }
 
+// ---- tensor memory of both CTAs: one whole warp in each of the two issues these together (every tcgen05 instruction of a kernel names
+// the same cta_group); each CTA gets its address in its own shared memory
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_addr(dst_smem)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
 // ---- products and their completion
 __device__ __forceinline__ void umma_pair_f16_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
