@@ -55,7 +55,7 @@ def _conv(x, w, bias, res, silu, rows_outside, second=False):
 
 
 SIZES = [(1, 8, 16, 64, 128), (1, 1, 1, 64, 256), (1, 5, 7, 64, 128), (1, 17, 33, 128, 256), (3, 20, 20, 192, 256), (2, 9, 50, 64, 384),
-         (1, 200, 210, 64, 256)]
+         (1, 200, 210, 64, 256), (1, 250, 250, 64, 128), (1, 135, 203, 128, 768)]   # several tiles a pair, an odd number of boxes
 
 
 @pytest.mark.parametrize("rows_outside", [False, True])
