@@ -299,7 +299,6 @@ struct WinNorm {
     const float* q_ss; const float* k_ss;      // [rows][tiles] partial sums of squares (rows in window order)
     const float* gamma_q; const float* gamma_k;  // [heads * head_dim]
     int tiles; float inv_dim, eps;
-    bool four;                                 // four tiles, 16-byte aligned statistics
 };
 
 template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTokens * kWinTokens;
@@ -310,7 +309,12 @@ template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTo
 // products need nothing, mma.sync and the library's kernels add K in the same order.
 enum WinForm { kWinFused, kWinNormed, kWinSteps };
 
-template <WinForm FORM, int HD>
+// FOURS (kWinNormed): how many loads of four statistics make up a row's (dim 1024: 1, 2048: 2), or 0 for any number, one by one. The
+// statistics of the eight rows that a thread stages are then 8 or 16 loads instead of 32 or 64, all issued ahead of their use
+// (operands in L2 as behind the projection: 64 windows x 16 heads 9.1 -> 8.2 us, 256 x 16 39.3 -> 35.8, 4 x 16 4.3 -> 3.2, 64 x 32
+// 17.6 -> 15.7). A number that is not known to the compiler puts a loop between the loads: 9.1 us again, and the choice between the two
+// inside the kernel cost the others 2 %.
+template <WinForm FORM, int HD, int FOURS = 0>
 __global__ void __launch_bounds__(kWinThreads, HD == 64 ? 8 : 4)
 window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
                         __half* __restrict__ O, const uint8_t* __restrict__ mask, int heads, int nW, float scale,
@@ -363,11 +367,14 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
                 raw[1][k] = ldg_half8(Kh + r * HD + c * 8);
                 const long long row = (long long)bw * kWinTokens + r;   // token row in window order
                 float sq = 0.0f, sk = 0.0f;
-                if (nrm.four) {   // dim 1024, both aligned: one load each instead of four (operands in L2 as behind the projection: 64 windows x
-                    // 16 heads 9.6 -> 8.9 us, 4 x 16 4.5 -> 3.9; operands from HBM 13.2 either way)
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(nrm.q_ss) + row), b = __ldg(reinterpret_cast<const float4*>(nrm.k_ss) + row);
-                    sq = ((a.x + a.y) + a.z) + a.w;
-                    sk = ((b.x + b.y) + b.z) + b.w;
+                if (FOURS > 0) {
+                    const float4 *q4 = reinterpret_cast<const float4*>(nrm.q_ss) + row * FOURS, *k4 = reinterpret_cast<const float4*>(nrm.k_ss) + row * FOURS;
+#pragma unroll
+                    for (int t = 0; t < FOURS; ++t) {
+                        const float4 a = __ldg(q4 + t), b = __ldg(k4 + t);
+                        sq = t == 0 ? ((a.x + a.y) + a.z) + a.w : (((sq + a.x) + a.y) + a.z) + a.w;
+                        sk = t == 0 ? ((b.x + b.y) + b.z) + b.w : (((sk + b.x) + b.y) + b.z) + b.w;
+                    }
                 } else {
                     for (int t = 0; t < nrm.tiles; ++t) {
                         sq += __ldg(nrm.q_ss + row * nrm.tiles + t);
@@ -522,7 +529,7 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     }
 }
 
-template <WinForm FORM, int HD>
+template <WinForm FORM, int HD, int FOURS = 0>
 static int launch_window_attention(const __half* Q, const __half* K, const __half* V, __half* O, const uint8_t* mask, int BnW,
                                    int heads, int nW, float scale, const WinNorm& nrm, cudaStream_t st) {
     constexpr int smem = kWinSmemBytes<HD>;
@@ -533,12 +540,12 @@ static int launch_window_attention(const __half* Q, const __half* K, const __hal
         if (e != cudaSuccess) return (int)e;
         if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
         if (!configured[dev].load(std::memory_order_acquire)) {
-            e = cudaFuncSetAttribute(window_attention_kernel<FORM, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = cudaFuncSetAttribute(window_attention_kernel<FORM, HD, FOURS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return (int)e;
             configured[dev].store(true, std::memory_order_release);
         }
     }
-    launch_pdl(window_attention_kernel<FORM, HD>, dim3((unsigned)((long long)BnW * heads)), dim3(kWinThreads), smem, st, Q, K, V, O,
+    launch_pdl(window_attention_kernel<FORM, HD, FOURS>, dim3((unsigned)((long long)BnW * heads)), dim3(kWinThreads), smem, st, Q, K, V, O,
                mask, heads, nW, scale, nrm);
     return launch_status();
 }
@@ -560,10 +567,15 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
         return (head_dim == 64 ? launch_window_attention<kWinFused, 64> : launch_window_attention<kWinFused, 128>)(
             q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, WinNorm{}, st);
     if (!aligned16(gamma_q) || !aligned16(gamma_k)) return RFK_EUNSUPPORTED;
-    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps,
-                      ss_tiles == 4 && aligned16(q_row_ss) && aligned16(k_row_ss)};
-    return (head_dim == 64 ? launch_window_attention<kWinNormed, 64> : launch_window_attention<kWinNormed, 128>)(
-        q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
+    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
+    const int fours = aligned16(q_row_ss) && aligned16(k_row_ss) && (ss_tiles == 4 || ss_tiles == 8) ? ss_tiles / 4 : 0;
+    const auto launch = head_dim == 64 ? (fours == 1   ? launch_window_attention<kWinNormed, 64, 1>
+                                          : fours == 2 ? launch_window_attention<kWinNormed, 64, 2>
+                                                       : launch_window_attention<kWinNormed, 64>)
+                                       : (fours == 1   ? launch_window_attention<kWinNormed, 128, 1>
+                                          : fours == 2 ? launch_window_attention<kWinNormed, 128, 2>
+                                                       : launch_window_attention<kWinNormed, 128>);
+    return launch(q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
 }
 
 int window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask, int BnW,

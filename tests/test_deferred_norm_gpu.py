@@ -245,3 +245,24 @@ def test_key_split_equals_unsplit_attention(B, Hh, Sq, Sk, n_keys, cut):
         assert torch.equal(off, whole)
     finally:
         o.flash_attention_set_split(True)
+
+
+@pytest.mark.parametrize("tiles", [1, 4, 6, 8, 12])
+def test_window_attention_reads_its_statistics_with_the_same_bits_in_fours_and_one_by_one(tiles):
+    """Four or eight 16-byte aligned statistics a row are read four at a time; the same ones 4 bytes further are not aligned."""
+    o = _ops()
+    BnW, Hh = 3, 2
+    g = torch.Generator(device="cuda").manual_seed(tiles)
+    q, k, v = (torch.randn(BnW, Hh, 64, 64, device="cuda", generator=g).half() for _ in range(3))
+    gq, gk = (1 + 0.1 * torch.randn(Hh * 64, device="cuda", generator=g) for _ in range(2))
+    outs, ss = [], 50 * torch.rand(2, BnW * 64 * tiles, device="cuda", generator=g)
+    for shift in (0, 1):
+        room = torch.empty(2, BnW * 64 * tiles + 4, device="cuda")
+        stats = [r[shift:shift + BnW * 64 * tiles] for r in room]
+        for s, r in zip(stats, ss):
+            s.copy_(r)
+        assert all((s.data_ptr() % 16 == 0) == (shift == 0) for s in stats)
+        out = torch.full((BnW * 64, Hh * 64), 7.0, device="cuda", dtype=torch.float16)
+        o.window_attention_normed(q, k, v, out, None, *stats, tiles, gq, gk, Hh * 64, BnW, Hh, 1)
+        outs.append(out)
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
