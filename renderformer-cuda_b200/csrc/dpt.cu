@@ -127,19 +127,17 @@ struct rfk_dpt {
     // or -1 if neither order has them, and the convolution stays with the library. An image is 10^x of what comes out here, and
     // images do not change with the kernel that makes them. Which order the library takes is its own choice per size, type of
     // kernel and version, so it is not written down here but found out: both run once on the same operands when the head is planned, once
-    // for each size of map (about 1 ms for the two of a 512 x 512 image).
+    // for each size of map (1 to 3 ms of a plan's 50 to 55, most of it the scratch memory). x and y are the step's own buffers,
+    // which hold nothing yet.
     int order_of_sums(cudnnTensorDescriptor_t xd, cudnnFilterDescriptor_t fd, cudnnConvolutionDescriptor_t cd, cudnnTensorDescriptor_t yd,
-                      cudnnConvolutionFwdAlgo_t algo, size_t ws, int H, int W, int Cin, int Cout) {
-        for (const Order& k : orders)
-            if (k.H == H && k.W == W && k.Cin == Cin && k.Cout == Cout) return k.rows_outside;
+                      cudnnConvolutionFwdAlgo_t algo, size_t ws, rfk_half* x, rfk_half* y, int H, int W, int Cin, int Cout) {
         const size_t nx = (size_t)H * W * Cin, nw = (size_t)Cout * 9 * Cin, ny = (size_t)H * W * Cout;
         const auto pad = [](size_t halves) { return (halves * sizeof(__half) + 255) / 256 * 256; };
         int found = -1;
         char* scratch = nullptr;
-        if (cudaMalloc((void**)&scratch, pad(nx) + pad(nw) + 2 * pad(ny) + 256 + ws) == cudaSuccess) {
-            rfk_half *x = (rfk_half*)scratch, *k = (rfk_half*)((char*)x + pad(nx)), *want = (rfk_half*)((char*)k + pad(nw));
-            rfk_half* got = (rfk_half*)((char*)want + pad(ny));
-            int* differ = (int*)((char*)got + pad(ny));
+        if (cudaMalloc((void**)&scratch, pad(nw) + pad(ny) + 256 + ws) == cudaSuccess) {
+            rfk_half *k = (rfk_half*)scratch, *want = (rfk_half*)(scratch + pad(nw));
+            int* differ = (int*)((char*)want + pad(ny));
             const auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
             fill_hashed_kernel<<<blocks(nx), 256>>>((__half*)x, (long long)nx, 1);
             fill_hashed_kernel<<<blocks(nw), 256>>>((__half*)k, (long long)nw, 2);
@@ -149,8 +147,8 @@ struct rfk_dpt {
             for (int rows_outside = 0; ran && found < 0 && rows_outside < 2; ++rows_outside) {
                 int other = 1;
                 ran = cudaMemsetAsync(differ, 0, sizeof(int)) == cudaSuccess &&
-                      rfk_conv3x3_nhwc(x, k, nullptr, nullptr, got, nullptr, 1, H, W, Cin, Cout, 0, rows_outside, nullptr) == RFK_OK;
-                if (ran) differ_kernel<<<blocks(ny / 2), 256>>>((const unsigned*)want, (const unsigned*)got, (long long)(ny / 2), differ);
+                      rfk_conv3x3_nhwc(x, k, nullptr, nullptr, y, nullptr, 1, H, W, Cin, Cout, 0, rows_outside, nullptr) == RFK_OK;
+                if (ran) differ_kernel<<<blocks(ny / 2), 256>>>((const unsigned*)want, (const unsigned*)y, (long long)(ny / 2), differ);
                 ran = ran && cudaMemcpy(&other, differ, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
                 if (ran && !other) found = rows_outside;
             }
@@ -185,6 +183,20 @@ struct rfk_dpt {
         rfk_half* wk = alloc((size_t)Cout * Cin * k * k);  // [Cout, k, k, Cin]
         if (!wk) return (int)cudaErrorMemoryAllocation;
         TRY(rfk_permute_filter(weight, wk, Cout, Cin, k * k, 0, nullptr));
+        const bool may_own = !library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout, sms) &&
+                             rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout);
+        const auto push_own = [&](int rows_outside) {
+            const int Bn = B;
+            ++n_own;
+            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
+                return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
+            });
+            return RFK_OK;
+        };
+        const Order* known = nullptr;
+        for (const Order& q : orders)
+            if (q.H == H && q.W == W && q.Cin == Cin && q.Cout == Cout) known = &q;
+        if (may_own && known && known->rows_outside >= 0) return push_own(known->rows_outside);
         cudnnTensorDescriptor_t xd = tensor(B, Cin, H, W), yd = tensor(B, Cout, Ho, Wo);
         cudnnFilterDescriptor_t fd = filter(Cout, Cin, k, k);
         cudnnConvolutionDescriptor_t cd = conv(pad, stride);
@@ -199,16 +211,9 @@ struct rfk_dpt {
         const cudnnConvolutionFwdAlgo_t algo = perf[0].algo;
         size_t ws = 0;
         DNN_TRY(cudnnGetConvolutionForwardWorkspaceSize(dnn, xd, fd, cd, yd, algo, &ws));
-        if (!library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout, sms) &&
-            rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout)) {
-            const int Bn = B, rows_outside = order_of_sums(xd, fd, cd, yd, algo, ws, H, W, Cin, Cout);
-            if (rows_outside >= 0) {
-                ++n_own;
-                program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
-                    return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
-                });
-                return RFK_OK;
-            }
+        if (may_own && !known) {
+            const int rows_outside = order_of_sums(xd, fd, cd, yd, algo, ws, const_cast<rfk_half*>(in), o, H, W, Cin, Cout);
+            if (rows_outside >= 0) return push_own(rows_outside);
         }
         ws_bytes = std::max(ws_bytes, ws);
         rfk_dpt* self = this;
