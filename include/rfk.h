@@ -274,9 +274,11 @@ int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
  * than SMs (a 256 x 256 view has 64) leaves most of the machine idle, so with a workspace - and when the launcher's
  * estimate says it pays - the units' key ranges are cut into one share per SM and merged by the CTA that finishes a
  * unit last (nobody waits); of a larger grid the units of the last, partial round are, when that saves a fifth of the
- * launch. Which units are cut, and with it the order of their sums, depends on B * H and Sq. workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
+ * launch. Which units are cut, and with it the order of their sums, depends on B * H and Sq. Units of any other grid of more
+ * than one round may be begun by one CTA and finished by another through the workspace, in the order and with the bits of
+ * whole units. workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
  * bytes zero before the first launch (the kernel leaves them zero); launches that may overlap in time need separate
- * workspaces. The result differs from the unsplit kernel's only by rounding (fp32 merge; fp16 probabilities relative to
+ * workspaces. The result of cut units differs from whole ones' only by rounding (fp32 merge; fp16 probabilities relative to
  * each piece's own maximum) and is bit-reproducible from launch to launch.
  * (3) Shared values (v_shared != 0): V is [H, Sk, D], one set for all B batch elements - views of one scene rendered
  * together have their own queries and (rotated) keys but the same values.
@@ -287,13 +289,14 @@ int rfk_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half*
                            int o_bshd, float scale, rfk_stream_t stream);
 size_t rfk_flash_attention_workspace_bytes(void);
 /* The work list rfk_flash_attention_ex would launch for `units` units (256 queries of one head each) of `n_tiles`
- * 64-key tiles on a device with `sms` SMs, given a workspace: units [0, *whole_units) run whole, then *n_pieces pieces
+ * 64-key tiles on a device with `sms` SMs, given a workspace: units [0, *whole_units) run whole (or handed over, which
+ * changes no result), then *n_pieces pieces
  * in launch order, each six values {unit, first tile, tiles, first slot of its unit, pieces of its unit, own slot}
  * written to pieces[6 i ..] for i < max_pieces. Host only: touches no device. Diagnostic; no reference counterpart. */
 int rfk_flash_attention_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces,
                              unsigned short* pieces, int max_pieces);
 /* 0: rfk_flash_attention_ex ignores its workspace (every unit whole), to time both schedules side by side; 1 (default):
- * it cuts where that pays. Process-wide. No reference counterpart. */
+ * it cuts and hands over where that pays. Process-wide. No reference counterpart. */
 int rfk_flash_attention_set_split(int on);
 
 /* Which kernel serves rfk_flash_attention: 0 automatic (the tcgen05 / tensor-memory kernel; the

@@ -45,6 +45,16 @@
 // next launch. A piece costs about 10 us beyond its tiles (pipeline fill, publishing, merging), so the last, partial
 // round of a larger grid is cut the same way only when few units are left for it (plan_work).
 //
+// Hand-over. Any other grid of more than one round (256 units of a 512 x 512 view: 1.73 rounds of 148 SMs) would leave SMs idle in
+// its last round. With a workspace every SM gets the same number of key tiles instead: some units are begun by one CTA, which leaves
+// O, running maximum and row sum as they stand in the workspace, and finished by another, which takes them up and goes on with the
+// next tile (plan_handover). That is the same sequence of operations on every row, so the bits are those of whole units, for every
+// caller. First pieces are the grid's first blocks, second pieces its last, and a first piece waits for nobody: a second piece
+// only ever waits (with the limit of the other waits) for a block that was handed out before it, and by the plan that one has been done for
+// half a round. Measured (us, whole / handed over; estimates agree within 2 %): 16 x 4096 x 5665 x 64 138 / 127, 16 x 5665 x 5665 208 / 180,
+// 448 units of 89 tiles 277 / 221, 149 of 16 33 / 24.5; 128-wide heads 184 of 89 tiles 208 / 148, 256 of 89 217 / 207. Of 137 grids of 149 to 600
+// units and 16 to 113 tiles none lost. It needs a gain of 5 % by the plan's estimate; 256 units of 24 tiles stay whole.
+//
 // One block per CTA. Two blocks share a CTA so that they share the K/V tiles; their softmax warps then share the SM's
 // schedulers and special-function unit (a tile of one block alone takes 1020 clocks, of two together 1410, 64-wide heads).
 // Where all blocks of 128 queries find an SM of their own, each gets one (BLOCKS = 1): 16 x 576 x 4607, 48 units of 256 queries,
@@ -108,9 +118,10 @@ enum : int { kErrTimeout = 1, kErrSmemAlign = 2 };
 struct Piece { uint16_t unit, t0, nt, first, count, slot; };
 constexpr int kMaxPieces = 320;
 struct WorkList {
-    int whole_units;  // CTAs [0, whole_units) take the unit of their index over all keys
-    int n_pieces;     // CTAs [whole_units, whole_units + n_pieces) take pieces[index - whole_units]
+    int whole_units;  // CTAs [heads, heads + whole_units) take the unit of their index, less heads, over all keys
+    int n_pieces;     // the CTAs behind them take pieces[index - whole_units]
     int q_blocks;     // units per head: ceil(Sq / 256)
+    int heads;        // units handed over (else 0): CTAs [0, heads) take their first pieces, pieces[0, heads); n_pieces = 2 * heads
     Piece pieces[kMaxPieces];
 };
 // Workspace: 256 counters (one per split unit, zero between launches), then per slot 256 x {m, l}, then per slot the
@@ -120,10 +131,29 @@ constexpr size_t kWsCounterBytes = 1024;
 constexpr size_t kWsMlBytes = (size_t)kMaxPieces * kUnitRows * 2 * sizeof(float);
 constexpr size_t kWsOBytes = (size_t)kMaxPieces * kUnitRows * 128 * sizeof(float);  // for the larger head size
 constexpr size_t kWsBytes = kWsCounterBytes + kWsMlBytes + kWsOBytes;
+// A unit that is handed over (see "Hand-over") takes its counter, by slot, and two of the output areas: O in 2 * slot, the row sums
+// and the reference in the first two groups of 2 * slot + 1.
+constexpr int kMaxHanded = kMaxPieces / 2;
+static_assert(kMaxHanded * sizeof(int) <= kWsCounterBytes, "a counter each");
 
 __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue)); }
 __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax)); }
 __device__ __forceinline__ void softmax_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }  // warps 0-7 only
+
+// A whole warp waits for the first piece of its unit (a flag in the workspace), with the limits of the other waits.
+__device__ __forceinline__ bool wait_handed(const int* flag, volatile int* abort) {
+    const uint64_t start = tc::global_timer_ns();
+    for (uint32_t it = 0; it < tc::kSpinLimit; ++it) {
+        int set;
+        asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(set) : "l"(flag) : "memory");
+        if (__all_sync(0xffffffffu, set != 0)) return true;
+        if ((it & 63u) == 63u &&
+            __any_sync(0xffffffffu, *abort != 0 || (int64_t)(tc::global_timer_ns() - start) > (int64_t)tc::kWaitLimitNs)) break;
+        __nanosleep(32);
+    }
+    *abort = 1;
+    return false;
+}
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     __half2 h = __floats2half2_rn(lo, hi);
@@ -263,7 +293,7 @@ __device__ __forceinline__ void store_row_half(__half* dst, const uint32_t (&v)[
 // order (mma.sync and tcgen05.mma add 16 products at a time, with the same bits, which the tests compare), the running maximum is
 // exact in both, so that whole units then have the bits of that kernel at a third of its time: 8 x 1600 x 4607 148 -> 62 us (one
 // block per CTA), 8 x 4096 x 5665 363 -> 105 us. It costs 2 %: the packed sums follow the register pairs of the exponents otherwise.
-template <int HD, int BLOCKS, bool ORDERED>
+template <int HD, int BLOCKS, bool ORDERED, bool HAND>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, __half* __restrict__ O, int H, int Sq, int n_keys,
@@ -285,7 +315,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this CTA's work: a whole unit, or a piece of one (n_tiles key tiles from tile t0)
     int unit = blockIdx.x, t0 = 0, n_tiles = (n_keys + BN - 1) / BN, split_count = 1, split_first = 0, split_slot = 0;
-    if ((int)blockIdx.x >= work.whole_units) {
+    bool gives = false, takes = false;  // HAND: the unit's first piece, whose state another CTA takes over; its second piece
+    if (HAND) {
+        const int b = blockIdx.x - work.heads;
+        gives = b < 0;
+        takes = b >= work.whole_units;
+        unit = b;
+        if (gives || takes) {
+            const Piece& pc = work.pieces[gives ? (int)blockIdx.x : b + work.heads - work.whole_units];
+            unit = pc.unit; t0 = pc.t0; n_tiles = pc.nt; split_slot = pc.slot;
+        }
+    } else if ((int)blockIdx.x >= work.whole_units) {
         const Piece& pc = work.pieces[blockIdx.x - work.whole_units];
         unit = pc.unit; t0 = pc.t0; n_tiles = pc.nt; split_count = pc.count; split_first = pc.first; split_slot = pc.slot;
     }
@@ -377,7 +417,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const uint32_t p_tmem = tmem + buf * 64, vt_lo = v_lo + st * (kStageBytes >> 4);
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks)  // P: 16 keys = 8 columns; V: 16 keys = 16 rows of 128 bytes
-                    tc::umma_f16_ts_lo(tmem_O, p_tmem + ks * 8, vt_lo + ks * (2048 >> 4), idesc_pv, (j > 0) || (ks > 0));
+                    tc::umma_f16_ts_lo(tmem_O, p_tmem + ks * 8, vt_lo + ks * (2048 >> 4), idesc_pv, (j > 0) || (ks > 0) || (HAND && takes));
                 tc::umma_commit(&ctrl->kv_empty[st]);  // K of this stage was consumed before its scores could be read
                 tc::umma_commit(&ctrl->pv_done[blk][buf]);
             }
@@ -459,7 +499,31 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         uint32_t va[32], vb[32];
         bool ok = true;
         int buf = 0, buf_par = 0;  // score buffer of tile j and the phase parity of its barriers
-        for (int j = 0; j < n_tiles; ++j) {
+        // HAND: this row's place in the handed-over state, [16 or 32 groups of 4 columns][256 rows] float4 as above
+        uint4* const handed = reinterpret_cast<uint4*>(ws + kWsCounterBytes + kWsMlBytes) + (size_t)split_slot * (2 * HD / 4) * kUnitRows + blk * BM + r;
+        if (HAND && takes) {  // O, the row sum and the reference where the first piece left them
+            ok = wait_handed(reinterpret_cast<const int*>(ws) + split_slot, abort_flag);
+            softmax_warps_sync();  // every softmax warp comes here, whatever its ok; all have seen the flag: ready for the next launch
+            if (tid == 0) reinterpret_cast<int*>(ws)[split_slot] = 0;
+            if (ok) {
+#pragma unroll
+                for (int hc = 0; hc < HD / 32; ++hc) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 w = __ldcg(handed + (hc * 8 + c) * kUnitRows);
+                        va[4 * c] = w.x; va[4 * c + 1] = w.y; va[4 * c + 2] = w.z; va[4 * c + 3] = w.w;
+                    }
+                    tc::tmem_st32(tO + hc * 32, va);
+                }
+                tc::tc_wait_st();
+                const uint4 l = __ldcg(handed + (HD / 4) * kUnitRows), m = __ldcg(handed + (HD / 4 + 1) * kUnitRows);
+                l_run = __uint_as_float(l.x);
+                l01 = make_float2(__uint_as_float(l.x), __uint_as_float(l.y));
+                l23 = make_float2(__uint_as_float(l.z), __uint_as_float(l.w));
+                m_run = __uint_as_float(m.x);
+            }
+        }
+        for (int j = 0; ok && j < n_tiles; ++j) {
             const uint32_t tS = tmem + lane_off + buf * 64;
             ok = tc::mbar_wait_warp(&ctrl->s_full[blk][buf], buf_par, abort_flag);
             if (!ok) break;
@@ -484,7 +548,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // tile) the scores are read again, the maximum is taken and the same code runs once more.
             float2 acc0, acc1;
             float m_new = m_run, alpha = 1.0f;
-            bool any_move = false, need_max = kExactMax || j == 0 || n_valid != BN;
+            bool any_move = false, need_max = kExactMax || (j == 0 && !(HAND && takes)) || n_valid != BN;
 #pragma unroll 1
             for (;;) {
                 acc0 = make_float2(0.0f, 0.0f);
@@ -521,13 +585,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_wait_ld(va);
                 tc::tmem_ld32(tS + 32, vb);
             }
-            if (j > 0 && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
+            if ((j > 0 || (HAND && takes)) && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
                 // O belongs to the tensor core until the previous tile's P V is done. Having seen s_full of tile j,
                 // P V of tile j - 1 - kSBufs (the previous phase of this barrier) is known complete: the parity is unambiguous.
-                const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
-                ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after();
+                if (!HAND || j > 0) {  // ahead of its first tile a taken-over O is this warp's own
+                    const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
+                    ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                }
 #pragma unroll
                 for (int hc = 0; hc < HD / 32; ++hc) {
                     tc::tmem_ld32(tO + hc * 32, vb);
@@ -552,7 +618,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (lane == 0) tc::mbar_arrive(&ctrl->p_full[blk][buf]);
             if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
         }
-        if (ORDERED) l_run = (l01.x + l01.y) + (l23.x + l23.y);
+        if (ORDERED && !(HAND && gives)) l_run = (l01.x + l01.y) + (l23.x + l23.y);
         // ---- epilogue: O / l -> fp16 -> global, one 128-byte row per thread
         if (ok) {  // buf / buf_par have moved on to tile n_tiles: step back to the last tile
             const int lbuf = buf == 0 ? kSBufs - 1 : buf - 1, lbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;
@@ -560,7 +626,27 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         const int q = q0 + blk * BM + r;
         __half* dst = o_bshd ? O + (((size_t)(bh / H) * Sq + q) * H + bh % H) * HD : O + ((size_t)bh * Sq + q) * HD;
-        if (BLOCKS == 1 || split_count == 1) {
+        if (HAND && gives) {
+            // ---- first piece of a unit that is handed over: O, row sum and reference as they stand, then the flag
+            if (ok) {
+                tc::tc_fence_after();
+#pragma unroll
+                for (int hc = 0; hc < HD / 32; ++hc) {
+                    tc::tmem_ld32(tO + hc * 32, va);
+                    tc::tc_wait_ld(va);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        __stcg(handed + (hc * 8 + c) * kUnitRows, make_uint4(va[4 * c], va[4 * c + 1], va[4 * c + 2], va[4 * c + 3]));
+                }
+                __stcg(handed + (HD / 4) * kUnitRows,
+                       ORDERED ? make_uint4(__float_as_uint(l01.x), __float_as_uint(l01.y), __float_as_uint(l23.x), __float_as_uint(l23.y))
+                               : make_uint4(__float_as_uint(l_run), 0, 0, 0));
+                __stcg(handed + (HD / 4 + 1) * kUnitRows, make_uint4(__float_as_uint(m_run), 0, 0, 0));
+                __threadfence();
+            }
+            softmax_warps_sync();  // every softmax warp comes here, whatever its ok
+            if (tid == 0 && !*abort_flag) asm volatile("st.release.gpu.b32 [%0], 1;" ::"l"(reinterpret_cast<int*>(ws) + split_slot) : "memory");
+        } else if (BLOCKS == 1 || HAND || split_count == 1) {
             if (ok) {
                 tc::tc_fence_after();
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
@@ -697,7 +783,7 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     using tcattn::Piece;
     constexpr int kPieceCostTiles = 12;  // what a piece costs beyond its tiles (fill, publishing, merging), in tile times
     w.whole_units = (int)units;
-    w.n_pieces = 0;
+    w.n_pieces = w.heads = 0;
     if (!split || sms <= 0 || units <= 0 || n_tiles > 65535 || units > 65535) return;
     const int rounds = (int)(units / sms), rest = (int)(units % sms);
     if (rest == 0 || rest > 256 || (rounds > 0 && !cut_last_round)) return;  // 256 unit counters
@@ -739,6 +825,51 @@ void plan_work(tcattn::WorkList& w, long long units, int n_tiles, int sms, bool 
     w.n_pieces = n;
 }
 
+// Hand-over (see above) for a grid that plan_work leaves whole: fills the SMs one after the other to the same budget of tile times,
+// each with the first piece of the unit that the SM before it left cut, whole units, and the last keys of one more unit. The
+// hardware hands the blocks out in order: the first pieces, the whole units, then the second pieces, longest first, which
+// comes to the same.
+void plan_handover(tcattn::WorkList& w, long long units, int n_tiles, int sms) {
+    using tcattn::Piece;
+    // Beyond its tiles every CTA costs some (set-up, first scores, last product, output), a hand-over some more on both sides.
+    constexpr int kCtaCost = 5, kGiveCost = 2, kTakeCost = 2, kMinPiece = 4;
+    if (sms <= 0 || sms > tcattn::kMaxHanded || units <= sms || units > 65535 || n_tiles > 65535 || n_tiles < 4 * kMinPiece) return;
+    const int whole = n_tiles + kCtaCost;
+    const long long uncut = (units + sms - 1) / sms * whole;
+    uint16_t tail[tcattn::kMaxHanded];
+    for (long long budget = (units * whole + (sms - 1) * (kCtaCost + kGiveCost + kTakeCost)) / sms; budget * 100 <= uncut * 95; ++budget) {
+        long long left = units;   // units not yet begun
+        int n = 0, open = 0;      // cut units; tiles of the first piece of the last of them, not yet placed
+        for (int s = 0; s < sms && (left > 0 || open > 0); ++s) {
+            long long room = budget;
+            if (open > 0) room -= open + kCtaCost + kGiveCost;
+            open = 0;
+            const long long k = std::min(left, std::max(0LL, room / whole));
+            left -= k;
+            room -= k * whole + kCtaCost + kTakeCost;
+            if (left > 0 && room >= kMinPiece) {
+                tail[n] = (uint16_t)std::min<long long>(room, n_tiles - kMinPiece);
+                open = n_tiles - tail[n++];
+                --left;
+            }
+        }
+        if (left > 0 || open > 0) continue;   // the budget does not hold them
+        if (n == 0) return;
+        w.whole_units = (int)units - n;
+        w.heads = n;
+        w.n_pieces = 2 * n;
+        for (int i = 0; i < n; ++i) {
+            const uint16_t unit = (uint16_t)(w.whole_units + i), t0 = (uint16_t)(n_tiles - tail[i]);
+            w.pieces[i] = Piece{unit, 0, t0, (uint16_t)i, 1, (uint16_t)i};
+            w.pieces[n + i] = Piece{unit, t0, tail[i], (uint16_t)i, 1, (uint16_t)i};
+        }
+        const auto longer = [](const Piece& a, const Piece& b) { return a.nt > b.nt; };
+        std::stable_sort(w.pieces, w.pieces + n, longer);
+        std::stable_sort(w.pieces + n, w.pieces + 2 * n, longer);
+        return;
+    }
+}
+
 // Whether a grid without cut units runs with one block of 128 queries per CTA (see "One block per CTA" above): when each block
 // finds an SM of its own.
 bool one_block_per_cta(int n_pieces, long long blocks, int sms) { return n_pieces == 0 && blocks <= sms; }
@@ -762,12 +893,26 @@ int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, i
     return RFK_OK;
 }
 
+// plan_handover's, the same way: *n_handed units, each three values {unit, tiles of its first piece, slot}, in launch order.
+int attention_tc_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed, unsigned short* first, int max_handed) {
+    if (units < 0 || n_tiles <= 0 || sms <= 0 || !whole_units || !n_handed || max_handed < 0 || (max_handed && !first)) return RFK_EINVAL;
+    tcattn::WorkList w;
+    plan_work(w, units, n_tiles, sms, false, false);
+    plan_handover(w, units, n_tiles, sms);
+    *whole_units = w.whole_units;
+    *n_handed = w.heads;
+    for (int i = 0; i < w.heads && i < max_handed; ++i) {
+        first[3 * i] = w.pieces[i].unit; first[3 * i + 1] = w.pieces[i].nt; first[3 * i + 2] = w.pieces[i].slot;
+    }
+    return RFK_OK;
+}
+
 namespace {
-template <int HD, int BLOCKS, bool ORDERED>
+template <int HD, int BLOCKS, bool ORDERED, bool HAND>
 int launch_units(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, __half* O, int H, int Sq, int n_keys, int o_bshd,
                  float scale, cudaStream_t st, const float* row_ss, int ss_tiles, int norm_dim, float norm_eps, void* ws, int v_heads,
                  const tcattn::WorkList& work, int dev) {
-    constexpr auto kernel = tcattn::attention_tc_kernel<HD, BLOCKS, ORDERED>;
+    constexpr auto kernel = tcattn::attention_tc_kernel<HD, BLOCKS, ORDERED, HAND>;
     constexpr int smem = tcattn::Cfg<HD, BLOCKS>::kSmemBytes;
     // per-device "kernel attributes set" marks; setting them twice from racing threads is harmless
     static std::atomic<bool> configured[64];
@@ -807,15 +952,17 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
     work.q_blocks = ceil_div(Sq, tcattn::kUnitRows);
     const long long units = (long long)B * H * work.q_blocks;
     if (units > 0x7fffffffLL) return RFK_EUNSUPPORTED;
-    const bool split = cut != AttnCut::kNone && ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
-    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sms, split, cut == AttnCut::kLastRound);
+    const bool shared = ws && ws_bytes >= tcattn::kWsBytes && aligned16(ws) && g_attn_split.load(std::memory_order_relaxed);
+    plan_work(work, units, ceil_div(n_keys, tcattn::BN), sms, shared && cut != AttnCut::kNone, cut == AttnCut::kLastRound);
+    if (shared && work.n_pieces == 0) plan_handover(work, units, ceil_div(n_keys, tcattn::BN), sms);
     const int v_heads = v_shared ? H : B * H;
     if (one_block_per_cta(work.n_pieces, (long long)B * H * ceil_div(Sq, tcattn::BM), sms)) {
         work.q_blocks = ceil_div(Sq, tcattn::BM);
         work.whole_units = B * H * work.q_blocks;
-        return launch_units<HD, 1, ORDERED>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
+        return launch_units<HD, 1, ORDERED, false>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
     }
-    return launch_units<HD, 2, ORDERED>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
+    const auto launch = work.heads ? launch_units<HD, 2, ORDERED, true> : launch_units<HD, 2, ORDERED, false>;
+    return launch(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
 }
 }  // namespace
 

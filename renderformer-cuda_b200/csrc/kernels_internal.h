@@ -56,6 +56,13 @@ extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K,
                                            int o_bshd, float scale, rfk_stream_t stream);
 extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq,
                                            int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);
+extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, void* workspace,
+                                              size_t workspace_bytes, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd,
+                                              float scale, rfk_stream_t stream);
+// Which units of a grid that is not cut the launcher hands over from one SM to another (plan_handover in attention_tc.cu): units
+// [0, *whole_units) stay whole, then for each of *n_handed units {unit, key tiles of its first piece, slot} in launch order.
+extern "C" int rfk_flash_attention_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed,
+                                                 unsigned short* first, int max_handed);
 // window_attention_steps, for its test
 extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                                           int BnW, int num_heads, int nW, float scale, rfk_stream_t stream);

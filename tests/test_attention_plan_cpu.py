@@ -1,6 +1,7 @@
 """CPU tests of the attention launcher's work planning (rfk_flash_attention_plan, host only): which grids are cut
 along the keys, and that a cut covers every key tile of every unit exactly once with consistent slot bookkeeping."""
 import ctypes
+import heapq
 
 import pytest
 
@@ -80,3 +81,49 @@ def test_last_round_that_saves_less_than_a_fifth_stays_whole(units, n_tiles):
     """The line that the header states. The encoder of a scene of 5633 triangles and 16 heads is 368 units of 89 tiles, where a cut is
     estimated to save 12 %: its sums, and with them the K/V cache and the views, keep their order."""
     assert _plan(units, n_tiles) == (units, [])
+
+
+def _handover(units, n_tiles, sms=148):
+    fn = _abi.load("rfk.h").rfk_flash_attention_handover_plan
+    fn.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
+                   ctypes.c_void_p, ctypes.c_int]
+    fn.restype = ctypes.c_int
+    whole, n = ctypes.c_int(-1), ctypes.c_int(-1)
+    buf = (ctypes.c_ushort * (3 * 160))()
+    assert fn(units, n_tiles, sms, ctypes.byref(whole), ctypes.byref(n), ctypes.cast(buf, ctypes.c_void_p), 160) == 0
+    return whole.value, [tuple(buf[3 * i + k] for k in range(3)) for i in range(n.value)]
+
+
+@pytest.mark.parametrize("sms", [148, 132, 16, 160])
+def test_handed_over_units_fill_the_last_round(sms):
+    """Every unit is taken once; the first pieces are launched together and wait for nothing, so that a second piece always waits for
+    a block ahead of it; blocks handed out in order finish sooner than whole units by what the plan asks for, and no second piece
+    starts before its first one is done."""
+    cta, give, take = 5, 2, 2
+    planned = 0
+    for units in range(1, 4 * sms, max(1, sms // 12)):
+        for n_tiles in (3, 15, 16, 33, 89, 700):
+            whole, handed = _handover(units, n_tiles, sms)
+            rounds = -(-units // sms) * (n_tiles + cta)
+            if not handed:
+                assert whole == units
+                continue
+            planned += 1
+            assert units > sms and len(handed) < sms
+            assert sorted(u for u, _, _ in handed) == list(range(whole, units)) and sorted(s for _, _, s in handed) == list(range(len(handed)))
+            assert all(4 <= first <= n_tiles - 4 for _, first, _ in handed)
+            free, ready = [0] * sms, {}
+            heapq.heapify(free)
+            for u, first, _ in handed:
+                ready[u] = heapq.heappop(free) + first + cta + give
+                heapq.heappush(free, ready[u])
+            for _ in range(whole):
+                heapq.heappush(free, heapq.heappop(free) + n_tiles + cta)
+            for u, first, _ in sorted(handed, key=lambda h: h[1]):
+                start = heapq.heappop(free)
+                assert start >= ready[u]
+                heapq.heappush(free, start + n_tiles - first + cta + take)
+            assert max(free) <= 0.96 * rounds
+    assert planned > 10
+    assert _handover(sms, 89, sms) == (sms, []) and _handover(2 * sms, 89, sms) == (2 * sms, []) and _handover(70000, 89, sms) == (70000, [])
+    assert _handover(200, 89, 161) == (200, [])          # more SMs than slots
