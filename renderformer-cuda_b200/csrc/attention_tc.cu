@@ -11,7 +11,7 @@
 //   warp 8       producer: one thread issues TMA tile loads (both Q blocks once, then K and V tiles
 //                through a ring of kStages shared-memory stages); the copies land in the tensor
 //                core's 128-byte-swizzled layout and complete on mbarriers, no thread touches the bytes.
-//   warps 11-12  one warp per block, whose elected lane issues S = Q K^T (tcgen05.mma M128 N64 K16
+//   warps 11-12  one warp per block [warp 11 for both], whose elected lane issues S = Q K^T (tcgen05.mma M128 N64 K16
 //                x 4 [8]) into one of the block's three [two] score buffers in tensor memory, as
 //                soon as the P V product that read that buffer's previous contents is complete:
 //                the softmax warps find their next two [one] tiles ready.
@@ -26,8 +26,10 @@
 //   warps 9-10   one warp per block, whose elected lane issues O += P V with P as the A operand
 //                from tensor memory and V (MN-major) from shared memory: P never passes through
 //                shared memory. The output accumulator O (128 x 64 [128] fp32 per block) is rescaled in place only when a
-//                row's running maximum has grown by more than 2^8 (the factor cancels in O / l; at
-//                all with 128-wide heads).
+//                row's running maximum has grown by more than 2^8 (the factor cancels in O / l): by the softmax warps.
+//   [warps 12-15 with 128-wide heads, where O is rescaled whenever a maximum has grown at all: they take each row's factor from
+//                its softmax thread as soon as that has the tile's maximum, wait for the previous P V, rescale, and arrive
+//                beside the softmax warps on the barrier that P V waits for. One block per CTA: warps 4-7.]
 // A stage of the ring is free again when both blocks' P V products of its tile are complete
 // (kv_empty counts two arrivals). The products have separate issuing warps because one warp's
 // instruction stream (8 products, 3 commits and 2-3 waits per tile, all dependent) takes about as
@@ -77,7 +79,7 @@ namespace tcattn {
 constexpr int BM = 128, BN = 64;
 constexpr int kBlocks = 2;                     // 128-query blocks per CTA, sharing the K/V ring (at most; see "One block per CTA")
 constexpr int kThreads = 512;                  // warps 0-7 softmax (block = warp / 4), 8 producer, 9-10 PV, 11-12 QK issuers, 13-15 none
-// Registers: the CTA starts with 128 per thread. The two warpgroups that only issue copies and products (warps 8-15)
+// Registers (64-wide heads): the CTA starts with 128 per thread. The two warpgroups that only issue copies and products (warps 8-15)
 // hand theirs back down to kRegsIssue and the softmax warpgroups (warps 0-7) grow to kRegsSoftmax, which lets the
 // compiler keep both halves of a score tile and their exponentials in flight without reusing registers early
 // (measured: 3 % off the kernel's time). 256 * 40 + 256 * 216 = 65536, the register file.
@@ -94,15 +96,28 @@ template <int HD, int BLOCKS> struct Cfg {
     // O takes HD of a block's 256 tensor-memory columns, score buffers the rest: three at 64, two at 128; a block that has the
     // CTA to itself always has three
     static constexpr int kSBufs = BLOCKS == 1 ? 3 : (256 - HD) / 64;
+    // 128-wide heads follow the exact maximum, which moves in every second tile of a warp's 32 rows: the 128 columns of O are rescaled
+    // by a warpgroup of its own beside the exponentials.
+    // (unit-variance scores: 8 x 4096 x 5665 101.6 -> 92 us, 8 x 1600 x 4607 with one block per CTA 62.2 -> 52.5; where the maxima
+    // hardly move 84.7 -> 80 and 49.4 -> 49.4.) Its latency counts: 16 columns of O at a time 103 us, 32 95.5, 32 fetched under the
+    // multiplication of the 32 before 92, which takes 104 registers. 256 * 160 + 128 * 120 + 128 * 72 = 65536; of the splits that keep
+    // the softmax from spilling this one was the fastest on scenes and views (1 to 2 % ahead of 168 / 120 / 56). With
+    // one block per CTA 128 * 216 + 128 * 104 + 256 * 40 are within the launch's 65536 (softmax with 160: 55 us).
+    static constexpr bool kCorr = HD == 128;
+    static constexpr int kRegSoftmax = !kCorr || BLOCKS == 1 ? kRegsSoftmax : 160, kRegCorr = BLOCKS == 1 ? 104 : 120,
+                         kRegIssue = !kCorr || BLOCKS == 1 ? kRegsIssue : 72;
+    static constexpr int kCorrWarp = !kCorr ? 99 : BLOCKS == 2 ? 12 : 4;   // its first warp
+    static constexpr int kFactorBytes = kCorr ? BLOCKS * kSBufs * BM * 4 : 0;   // behind the control block
+    static constexpr int kQkWarp = 11;                                     // kCorr: one warp issues Q K^T of both blocks
     // The shared-memory window is declared 1024-byte aligned (swizzled tiles need it) and the kernel checks it.
-    static constexpr int kSmemBytes = BLOCKS * kQBytes + kStages * kStageBytes + 512;
+    static constexpr int kSmemBytes = BLOCKS * kQBytes + kStages * kStageBytes + 512 + kFactorBytes;
     static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
 };
 constexpr int kMaxStages = 6, kMaxSBufs = 3;
 
 struct __align__(8) Ctrl {
     uint64_t q_full, kv_full[kMaxStages], kv_empty[kMaxStages], s_full[kBlocks][kMaxSBufs], p_full[kBlocks][kMaxSBufs],
-        pv_done[kBlocks][kMaxSBufs];
+        pv_done[kBlocks][kMaxSBufs], move_full[kBlocks][kMaxSBufs];
     uint64_t drain[2 * kBlocks];  // abort path only, one per issuing lane: completes once that lane's products have finished
     uint32_t tmem_base;
     int abort;
@@ -136,8 +151,8 @@ constexpr size_t kWsBytes = kWsCounterBytes + kWsMlBytes + kWsOBytes;
 constexpr int kMaxHanded = kMaxPieces / 2;
 static_assert(kMaxHanded * sizeof(int) <= kWsCounterBytes, "a counter each");
 
-__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue)); }
-__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax)); }
+template <int N> __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ void softmax_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }  // warps 0-7 only
 
 // A whole warp waits for the first piece of its unit (a flag in the workspace), with the limits of the other waits.
@@ -311,6 +326,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t sQ = base, sKV = base + BLOCKS * kQBytes;
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + BLOCKS * kQBytes + kStages * kStageBytes);
     volatile int* abort_flag = &ctrl->abort;
+    // kCorr: [block][score buffer][row], what a row's O is multiplied by ahead of the tile in that buffer
+    float* const factors = reinterpret_cast<float*>(smem_raw + BLOCKS * kQBytes + kStages * kStageBytes + 512);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this CTA's work: a whole unit, or a piece of one (n_tiles key tiles from tile t0)
@@ -337,7 +354,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->kv_full[s], 1); tc::mbar_init(&ctrl->kv_empty[s], BLOCKS); }
         for (int k = 0; k < BLOCKS; ++k)
             for (int b = 0; b < kSBufs; ++b) {
-                tc::mbar_init(&ctrl->s_full[k][b], 1); tc::mbar_init(&ctrl->p_full[k][b], 4); tc::mbar_init(&ctrl->pv_done[k][b], 1);
+                tc::mbar_init(&ctrl->s_full[k][b], 1); tc::mbar_init(&ctrl->p_full[k][b], C::kCorr ? 8 : 4); tc::mbar_init(&ctrl->pv_done[k][b], 1);
+                tc::mbar_init(&ctrl->move_full[k][b], 4);
             }
         for (int k = 0; k < 2 * BLOCKS; ++k) tc::mbar_init(&ctrl->drain[k], 1);
         ctrl->abort = 0;
@@ -359,8 +377,46 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // The register hand-over: every warp of a warpgroup executes the same setmaxnreg instruction (warpgroups 2 and 3 the
     // release, 0 and 1 the take), as the first statement of a branch that does not meet the other again before the
     // teardown - placed ahead of the branch, the compiler bound every role by the smaller budget.
-    if (warp >= 4 * BLOCKS) {
-    regs_release();
+    if (C::kCorr && warp >= C::kCorrWarp && warp < C::kCorrWarp + 4) {
+        regs_release<C::kRegCorr>();
+        // ------------------------------------------------------------ rescale of O (128-wide heads), a warp for its 32 lanes of every block
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+        const int r = (warp & 3) * 32 + lane;
+        bool ok = true;
+        int buf = 0, buf_par = 0;
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
+            for (int blk = 0; ok && blk < BLOCKS; ++blk) {
+                ok = tc::mbar_wait_warp(&ctrl->move_full[blk][buf], buf_par, abort_flag);
+                if (!ok) break;
+                const float alpha = factors[(blk * kSBufs + buf) * BM + r];
+                if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+                    // O belongs to the tensor core until the previous tile's P V is done (a tile's move_full comes behind its s_full, so
+                    // the parity is unambiguous); ahead of its first tile a taken-over O is the softmax warps'.
+                    if (j > 0) ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint32_t tO = tmem_cta + blk * 256 + kSBufs * 64 + lane_off;
+                    uint32_t v[2][32];
+                    tc::tmem_ld32(tO, v[0]);
+#pragma unroll
+                    for (int hc = 0; hc < HD / 32; ++hc) {
+                        tc::tc_wait_ld(v[hc & 1]);
+                        if (hc + 1 < HD / 32) tc::tmem_ld32(tO + (hc + 1) * 32, v[(hc + 1) & 1]);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[hc & 1][i] = __float_as_uint(__uint_as_float(v[hc & 1][i]) * alpha);
+                        tc::tmem_st32(tO + hc * 32, v[hc & 1]);
+                    }
+                    tc::tc_wait_st();
+                    tc::tc_fence_before();
+                }
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&ctrl->p_full[blk][buf]);
+            }
+            if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
+        }
+    } else if (warp >= 4 * BLOCKS) {
+    regs_release<C::kRegIssue>();
     if (warp == 8) {
         // ------------------------------------------------------------ producer (one thread)
         if (lane == 0) {
@@ -429,40 +485,44 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tc::mbar_wait_drain(&ctrl->drain[blk], 0);
         }
         __syncwarp();
-    } else if (warp == 11 || (BLOCKS == 2 && warp == 12)) {
-        const int blk = warp - 11;
-        const uint32_t tmem = tmem_cta + blk * 256;
+    } else if (warp == C::kQkWarp || (BLOCKS == 2 && !C::kCorr && warp == 12)) {
+        constexpr int kBlks = C::kCorr ? BLOCKS : 1;    // blocks of this warp
+        const int blk0 = warp - C::kQkWarp;
         // ------------------------------------------------------------ issuer of S = Q K^T (the warp's elected lane)
         const bool leader = tc::elect_one();
         constexpr uint32_t idesc_qk = tc::umma_idesc_f16(BM, BN, 0);  // B = K tile, K-major
-        const uint32_t q_lo = tc::umma_desc_lo(sQ + blk * kQBytes), k_lo = tc::umma_desc_lo(sKV);
+        const uint32_t q_lo0 = tc::umma_desc_lo(sQ + blk0 * kQBytes), k_lo = tc::umma_desc_lo(sKV);
         bool ok = tc::mbar_wait_warp(&ctrl->q_full, 0, abort_flag);
         int buf = 0, buf_par = 0, st = 0, st_par = 0;
         for (int j = 0; ok && j < n_tiles; ++j) {
             ok = tc::mbar_wait_warp(&ctrl->kv_full[st], st_par, abort_flag);
-            // the buffer still holds P of tile j - kSBufs until that tile's P V is complete
-            if (ok && j >= kSBufs) ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][buf], buf_par ^ 1, abort_flag);
-            if (!ok) break;
-            tc::tc_fence_after();
-            if (leader) {
-                const uint32_t kt_lo = k_lo + st * (kStageBytes >> 4);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)  // 16 head-dim elements = 32 bytes along a row of a sub-tile
-                    tc::umma_f16_lo(tmem + buf * 64, q_lo + (ks / 4) * (C::kQSub >> 4) + (ks % 4) * 2,
-                                    kt_lo + (ks / 4) * (C::kKSub >> 4) + (ks % 4) * 2, idesc_qk, ks > 0);
-                tc::umma_commit(&ctrl->s_full[blk][buf]);
+            for (int b = 0; b < kBlks; ++b) {
+                const int blk = blk0 + b;
+                // the buffer still holds P of tile j - kSBufs until that tile's P V is complete
+                if (ok && j >= kSBufs) ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][buf], buf_par ^ 1, abort_flag);
+                if (!ok) break;
+                tc::tc_fence_after();
+                if (leader) {
+                    const uint32_t kt_lo = k_lo + st * (kStageBytes >> 4), q_lo = q_lo0 + b * (kQBytes >> 4);
+#pragma unroll
+                    for (int ks = 0; ks < HD / 16; ++ks)  // 16 head-dim elements = 32 bytes along a row of a sub-tile
+                        tc::umma_f16_lo(tmem_cta + blk * 256 + buf * 64, q_lo + (ks / 4) * (C::kQSub >> 4) + (ks % 4) * 2,
+                                        kt_lo + (ks / 4) * (C::kKSub >> 4) + (ks % 4) * 2, idesc_qk, ks > 0);
+                    tc::umma_commit(&ctrl->s_full[blk][buf]);
+                }
             }
             if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
             if (++st == kStages) { st = 0; st_par ^= 1; }
         }
         if (leader && *abort_flag) {
-            tc::umma_commit(&ctrl->drain[BLOCKS + blk]);
-            tc::mbar_wait_drain(&ctrl->drain[BLOCKS + blk], 0);
+            tc::umma_commit(&ctrl->drain[BLOCKS + blk0]);
+            tc::mbar_wait_drain(&ctrl->drain[BLOCKS + blk0], 0);
         }
         __syncwarp();
-    }  // warps 13-15 have no role beyond handing their registers back together with warp 12
+    }  // the other warps have no role beyond handing their registers back together with their warpgroup
     } else {
-        regs_take();
+        regs_take<C::kRegSoftmax>();
         // ------------------------------------------------------------ softmax, warps 0-7 (query block = warp / 4)
         constexpr unsigned kFull = 0xffffffffu;
         constexpr float kSumLimit = 256.0f;  // 2^8, the threshold below
@@ -569,6 +629,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     m_new = move ? m_tile : m_run;
                     any_move = __any_sync(kFull, move);
                     if (any_move && move) alpha = fast_exp2((m_run - m_new) * scale_log2e);  // first tile: 0
+                    if (C::kCorr) {  // the first tile's product overwrites O, unless it was taken over
+                        factors[(blk * kSBufs + buf) * BM + r] = j > 0 || (HAND && takes) ? alpha : 1.0f;
+                        if (HAND && j == 0) tc::tc_fence_before();   // a taken-over O has been stored by this warp
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&ctrl->move_full[blk][buf]);
+                    }
                 }
                 // P = exp2(scale * log2e * (S - max)), two fp16 per 32-bit column: keys 2i, 2i+1 in column i;
                 // the 32 packed words end up in va, which is what the store below takes
@@ -585,7 +651,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_wait_ld(va);
                 tc::tmem_ld32(tS + 32, vb);
             }
-            if ((j > 0 || (HAND && takes)) && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
+            if (!C::kCorr && (j > 0 || (HAND && takes)) && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
                 // O belongs to the tensor core until the previous tile's P V is done. Having seen s_full of tile j,
                 // P V of tile j - 1 - kSBufs (the previous phase of this barrier) is known complete: the parity is unambiguous.
                 if (!HAND || j > 0) {  // ahead of its first tile a taken-over O is this warp's own
