@@ -332,13 +332,14 @@ namespace pair { using namespace pair_ptx; }
 // block (one SM takes them at about 110 GB/s). K is not split: every output is summed over the K blocks in the same order
 // as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
 // must equal the views one by one).
-//   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing warp and the producer run
-//   their loops as a whole, one elected lane issuing, so that descriptors, coordinates and counters live in uniform registers.
-//   With one block per stage and single threads' loops a K block took 0.30 us on every tile size, the cost of issuing and not of
-//   the operands; two blocks and the elected issuer took the 64 x 32 tile to 0.14 us, the elected producer to 0.12 us (256 x 1024 x
-//   4096 10.96 -> 9.95 us, weights from HBM; the tensor pipe alone would take 0.05 us). The 128 x 64 tile keeps a producer of one lane:
-//   1024 x 1024 x 4096 takes 12.0 us with it and 13.3 with the elected one (weights from HBM 12.8 and 13.3), 256 x 3072 x 1024 5.2 and
-//   5.4. Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
+//   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing lane and the producer's are
+//   elected ones (elect.sync), so that descriptors, coordinates and counters live in uniform registers; inside `if (lane == 0)`
+//   each operand is moved there first. With one block per stage and lane 0's loops a K block took 0.30 us on every tile size, the cost
+//   of issuing and not of the operands; two blocks and elected lanes in loops of whole warps took the 64 x 32 tile to 0.12 us, loops of
+//   the elected lanes alone, the others waiting at the warp's barrier, to 0.10 (us, whole warps / lanes alone, weights in L2: 256 x 1024 x
+//   4096 9.63 / 8.23, 256 x 1024 x 1024 3.90 / 3.62, 576 x 1024 x 4096 11.1 / 9.3; 128 x 64 tiles 1024 x 1024 x 4096 12.45 / 12.18; the
+//   tensor pipe alone would take 0.05 us a block). 128 x 128 tiles keep whole warps: 2304 x 1024 x 4096 16.9 / 17.6, 1600 x 1024 x 4096
+//   16.4 / 17.4. Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
 //   weights asked for ahead of the kernel's wait for its predecessor, changed nothing or cost (320 x 320 views +4 %).
 //   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
 //   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(kThreads)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                      const __grid_constant__ CUtensorMap map_w1, const Params p) {
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    constexpr bool kWhole = BM_ == 128 && BN_ == 128;   // producer and issuer run their loops as whole warps
     constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
     constexpr int kStages = Cfg<BM_, BN_>::kStages, kStage = Cfg<BM_, BN_>::kStageBytes, kBlock = Cfg<BM_, BN_>::kBlockBytes;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -404,9 +406,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_trigger();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ producer (the warp's elected lane, or lane 0 alone)
-        constexpr bool kWhole = !(BM_ == 128 && BN_ == 64);
-        const bool leader = kWhole ? tc::elect_one() : lane == 0;
+        // ------------------------------------------------------------ producer (the warp's elected lane)
+        const bool leader = tc::elect_one();
         if (kWhole || leader) {
             int it = 0, s = 0, par = 1;   // stage of `it`, and the parity of its barrier's previous phase
             for (; it < num_st; ++it) {
@@ -438,9 +439,10 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         constexpr uint32_t idesc = tc::umma_idesc_f16(BM_, BN_, 0);  // A and B both K-major
         const bool leader = tc::elect_one();
         bool ok = true;
-        for (int it = 0; it < num_st; ++it) {
+        for (int it = 0; (kWhole || leader) && it < num_st; ++it) {
             const int s = it % kStages;
-            ok = tc::mbar_wait_warp(&ctrl->full[s], (it / kStages) & 1, abort_flag);
+            ok = kWhole ? tc::mbar_wait_warp(&ctrl->full[s], (it / kStages) & 1, abort_flag)
+                        : tc::mbar_wait(&ctrl->full[s], (it / kStages) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
             if (leader) {
@@ -841,8 +843,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (tid == 0) RFK_STAMP(1);   // prologue done (barriers, tensor memory, cluster barrier)
 
     if (warp == 0) {
-        // ------------------------------------------------------------ producer (one thread per CTA)
-        if (lane == 0) {
+        // ------------------------------------------------------------ producer (an elected lane per CTA)
+        if (tc::elect_one()) {
             const void* map_w = rank == 0 ? (const void*)&map_w0 : (const void*)&map_w1;
             tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(map_w); tc::prefetch_tensormap(&map_c);
             if (EPI == RFK_GEMM_EPI_RESIDUAL) tc::prefetch_tensormap(&map_r);
@@ -869,8 +871,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ------------------------------------------------------------ issuer of the pair's products (one thread of CTA 0)
-        if (lane == 0 && rank == 0) {
+        // ------------------------------------------------------------ issuer of the pair's products (an elected lane of CTA 0)
+        // elect.sync keeps descriptors and counters in uniform registers: a K block takes 543 clocks instead of 598 (the tensor pipe's
+        // own time: 512). A loop of the whole warp that issues under the same predicate needs 548, but the epilogue that
+        // followed it took twice as long (4137 clocks for 2086), for a reason that its code does not show.
+        // us, lane 0 / elected lane: 4096 x 1024 x 4096 + residual 27.9 / 26.4, w1|w3 + SwiGLU 48.1 / 46.1, 3072 x 1024 20.5 / 20.2.
+        if (rank == 0 && tc::elect_one()) {
             constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BNACC, 0);
             int it = 0, tl = 0;
             bool ok = true;
