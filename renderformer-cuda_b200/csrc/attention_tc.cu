@@ -362,7 +362,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         ctrl->merge = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0) {  // one warp allocates the CTA's tensor memory and later frees it
+    if (warp == 8 && lane == 0) {  // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
+        tc::prefetch_tensormap(&map_q); tc::prefetch_tensormap(&map_k); tc::prefetch_tensormap(&map_v);
+    }
+    if (warp == 9) {  // beside the barriers
         tc::tmem_alloc(&ctrl->tmem_base, kTmemCols);
         tc::tmem_relinquish();
     }
@@ -420,7 +423,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (warp == 8) {
         // ------------------------------------------------------------ producer (one thread)
         if (lane == 0) {
-            tc::prefetch_tensormap(&map_q); tc::prefetch_tensormap(&map_k); tc::prefetch_tensormap(&map_v);
             tc::mbar_arrive_expect_tx(&ctrl->q_full, BLOCKS * kQBytes);
             for (int k = 0; k < BLOCKS; ++k)
                 for (int x = 0; x < C::kSub; ++x)

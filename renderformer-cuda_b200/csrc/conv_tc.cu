@@ -123,7 +123,11 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         ctrl->abort = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0 && aligned) {  // the same in both CTAs of the pair
+    if (warp == 1 && lane == 0) {   // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
+        tc::prefetch_tensormap(&map_x); tc::prefetch_tensormap(&map_w); tc::prefetch_tensormap(&map_o);
+        if (p.has_res) tc::prefetch_tensormap(&map_r);
+    }
+    if (warp == 2 && aligned) {  // beside the barriers; the same in both CTAs of the pair
         tmem_alloc_pair(&ctrl->tmem_base, kTmemCols);
         tmem_relinquish_pair();
     }

@@ -394,9 +394,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         ctrl->abort = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0) {
+    if (warp == 2) {   // beside the barriers
         tc::tmem_alloc(&ctrl->tmem_base, BN_);
         tc::tmem_relinquish();
+    }
+    if (warp == 1 && lane == 0) {   // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
+        tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(&map_w0);
+        if (kGate) tc::prefetch_tensormap(&map_w1);
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -825,7 +829,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         ctrl->abort = 0;
         tc::fence_barrier_init();
     }
-    if (warp == 0 && aligned) {  // the same in both CTAs of the pair
+    if (warp == 1 && lane == 0) {   // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
+        tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(rank == 0 ? &map_w0 : &map_w1); tc::prefetch_tensormap(&map_c);
+        if (EPI == RFK_GEMM_EPI_RESIDUAL) tc::prefetch_tensormap(&map_r);
+    }
+    if (warp == 2 && aligned) {  // beside the barriers; the same in both CTAs of the pair
         tmem_alloc_pair(&ctrl->tmem_base, kTmemCols);
         tmem_relinquish_pair();
     }
@@ -846,8 +854,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ------------------------------------------------------------ producer (an elected lane per CTA)
         if (tc::elect_one()) {
             const void* map_w = rank == 0 ? (const void*)&map_w0 : (const void*)&map_w1;
-            tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(map_w); tc::prefetch_tensormap(&map_c);
-            if (EPI == RFK_GEMM_EPI_RESIDUAL) tc::prefetch_tensormap(&map_r);
             int it = 0;
             bool ok = true;
             for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
