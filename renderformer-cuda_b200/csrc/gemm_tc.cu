@@ -650,8 +650,9 @@ constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA
 // overwrites the residual in place and is stored from there. Plain / SwiGLU: two buffers per warp in turn.
 constexpr int kUnitCols = 64;
 constexpr int kUnitBytes = 32 * kUnitCols * 2;       // 4 KB
-template <int EPI> struct Cfg {
-    static constexpr int kUnits = (EPI == RFK_GEMM_EPI_SWIGLU) ? 2 : 4;                    // 64-column units per tile
+// BN: accumulator columns of a tile, 256 or 192 (narrow_tile)
+template <int EPI, int BN> struct Cfg {
+    static constexpr int kUnits = (EPI == RFK_GEMM_EPI_SWIGLU) ? 2 : BN / 64;              // 64-column units per tile
     static constexpr int kBufsPerWarp = (EPI == RFK_GEMM_EPI_RESIDUAL) ? 4 : 2;
     static constexpr int kStagingBytes = 4 * kBufsPerWarp * kUnitBytes;                      // 4 epilogue warps
     static constexpr int kStages = (EPI == RFK_GEMM_EPI_RESIDUAL) ? 5 : 6;
@@ -680,13 +681,13 @@ __device__ __forceinline__ void tma_store_5d(const void* tmap, uint32_t src_smem
 }
 // Residual epilogue, before the tile's accumulator is waited for: bring the warp's residual rows of the whole tile
 // into its four staging buffers. Lane 0 only. The buffers were last read by the TMA stores of the previous tile.
-template <int EPI>
+template <int EPI, int BN>
 __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* map_r, uint32_t stage_base, uint64_t* res_full,
                                                            int row0, int n0) {
     if (EPI != RFK_GEMM_EPI_RESIDUAL) return;
     bulk_wait_read<0>();
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {   // units beyond N are loaded too (all zeros): every barrier sees one phase per tile
+    for (int u = 0; u < Cfg<EPI, BN>::kUnits; ++u) {   // units beyond N are loaded too (all zeros): every barrier sees one phase per tile
         tc::mbar_arrive_expect_tx(&res_full[u], kUnitBytes);
         tma_load_2d(stage_base + u * kUnitBytes, map_r, n0 + u * kUnitCols, row0, &res_full[u]);
     }
@@ -694,11 +695,11 @@ __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* ma
 
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
 // t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0.
-template <int EPI>
+template <int EPI, int BN>
 __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, uint32_t t_acc,
                                                      unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
                                                      int row0, int n0, int lane, volatile int* abort_flag) {
-    constexpr int kUnits = Cfg<EPI>::kUnits;
+    constexpr int kUnits = Cfg<EPI, BN>::kUnits;
     const uint32_t stage_base = tc::smem_addr(stage_ptr);
     uint32_t v[32];
     float ss = 0.0f;   // kEpiHeads: this row's sum of squares over the tile
@@ -798,18 +799,20 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     return true;
 }
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                     const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_c,
                     const __grid_constant__ CUtensorMap map_r, const Params p) {
-    constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? 128 : 256;
-    constexpr int kStages = Cfg<EPI>::kStages;
+    static_assert(BN == 256 || (BN == 192 && EPI != RFK_GEMM_EPI_SWIGLU), "whole 64-column units");
+    constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? 128 : BN;
+    constexpr int kTxBytes = kABytes + BN / 2 * BK * 2;   // of a stage, per CTA
+    constexpr int kStages = Cfg<EPI, BN>::kStages;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = tc::smem_addr(smem_raw);
     const uint32_t rank = cluster_rank();            // 0: issues the products for the pair; 1: its peer
     unsigned char* staging = smem_raw + kStages * kStageBytes;   // 1024-byte aligned: the stages are 32 KB each
-    Ctrl* ctrl = reinterpret_cast<Ctrl*>(staging + Cfg<EPI>::kStagingBytes);
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(staging + Cfg<EPI, BN>::kStagingBytes);
     volatile int* abort_flag = &ctrl->abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) RFK_STAMP(0);   // kernel entry
@@ -858,8 +861,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             bool ok = true;
             for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
                 const int m0 = (t % p.tiles_m) * (2 * BM) + (int)rank * BM, n0 = (t / p.tiles_m) * BN_OUT;
-                // this CTA's half of the weight tile: rows n0.. (CTA 0) / n0+128.. (CTA 1) of W, or the gate / up rows
-                const int nw = (EPI == RFK_GEMM_EPI_SWIGLU || rank == 0) ? n0 : n0 + 128;
+                // this CTA's half of the weight tile: rows n0.. (CTA 0) / n0 + BN / 2.. (CTA 1) of W, or the gate / up rows
+                const int nw = (EPI == RFK_GEMM_EPI_SWIGLU || rank == 0) ? n0 : n0 + BN / 2;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % kStages;
                     if (it >= kStages && !wait(&ctrl->empty[s], ((it / kStages) + 1) & 1)) { ok = false; break; }
@@ -868,7 +871,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     // CTA 0 announces the bytes of both CTAs' copies on its own barrier (one local arrival); CTA 1 only
                     // copies. CTA 1's bytes may land before CTA 0's announcement: the phase still cannot complete before
                     // that arrival, and the transaction count balances once it is made.
-                    if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->full[s], 2 * kStageBytes);
+                    if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->full[s], 2 * kTxBytes);
                     tma_load_2d_pair(sA, &map_a, kb * BK, m0, full0);
                     tma_load_2d_pair(sA + kABytes, map_w, kb * BK, nw, full0);
                 }
@@ -883,7 +886,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // followed it took twice as long (4137 clocks for 2086), for a reason that its code does not show.
         // us, lane 0 / elected lane: 4096 x 1024 x 4096 + residual 27.9 / 26.4, w1|w3 + SwiGLU 48.1 / 46.1, 3072 x 1024 20.5 / 20.2.
         if (rank == 0 && tc::elect_one()) {
-            constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BNACC, 0);
+            constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BN, 0);
             int it = 0, tl = 0;
             bool ok = true;
             for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
@@ -919,7 +922,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ------------------------------------------------------------ epilogue, warps 2-5 of both CTAs
         const int lane_grp = warp & 3;                        // a warp reaches tensor-memory lanes [32 * (warp % 4), +32)
         const uint32_t lane_off = (uint32_t)(lane_grp * 32) << 16;
-        unsigned char* my_stage = staging + lane_grp * Cfg<EPI>::kBufsPerWarp * kUnitBytes;
+        unsigned char* my_stage = staging + lane_grp * Cfg<EPI, BN>::kBufsPerWarp * kUnitBytes;
         uint64_t* my_res = ctrl->res_full[lane_grp];
         bool ok = true;
         int tl = 0;
@@ -932,13 +935,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // (a multicast commit): issued at kernel start they delay the first operand tiles by ~0.5 us. The barrier has one
                 // phase, so a warp that comes late cannot miss it; empty[0] goes on to other phases.
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
-                epilogue_prefetch_residual<EPI>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
+                epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(4);   // first tile's accumulator complete
-            ok = epilogue_tile_staged<EPI>(p, &map_c, tmem_cta + lane_off + acc * BNACC, my_stage, my_res, tl & 1, row0, n0,
+            ok = epilogue_tile_staged<EPI, BN>(p, &map_c, tmem_cta + lane_off + acc * BNACC, my_stage, my_res, tl & 1, row0, n0,
                                            lane, abort_flag);
             if (!ok) break;
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(5);   // its epilogue done (stores issued)
@@ -1034,12 +1037,23 @@ int launch_gemm_single(const CUtensorMap& ma, const CUtensorMap& mw0, const CUte
     return launch_status();
 }
 
+int sm_count(int dev) {
+    static std::atomic<int> count[64];
+    int n = count[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); return 0; }
+        count[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 std::atomic<int> g_pair_clusters[64];  // CTA pairs the device can run at once, per device (0 not asked yet, -1 none)
 
 // CTA-pair kernel: clusters of two; returns RFK_EUNSUPPORTED (nothing launched) when the device cannot co-schedule pairs
-template <int EPI>
-int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, tcgemm::Params p, int dev,
-                     cudaStream_t st, const CUtensorMap* heads_map = nullptr) {
+template <int EPI, int BN>
+int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, tcgemm::Params p, int dev,
+                      cudaStream_t st, const CUtensorMap* heads_map) {
+    constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI, BN>;
     // tile maps of the output (stores) and of the residual (loads): boxes of 32 rows x 64 columns, one per epilogue warp
     CUtensorMap mc, mr;
     if (heads_map) mc = *heads_map;
@@ -1047,7 +1061,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtens
         !make_map_2d(&mr, EPI == RFK_GEMM_EPI_RESIDUAL ? (const void*)p.R : (const void*)p.C, p.M, p.N,
                      EPI == RFK_GEMM_EPI_RESIDUAL ? p.ldr : p.ldc, 32))
         return RFK_EUNSUPPORTED;
-    constexpr int kSmem = tcgemm::pair::Cfg<EPI>::kSmemBytes;
+    constexpr int kSmem = tcgemm::pair::Cfg<EPI, BN>::kSmemBytes;
     std::atomic<int>* max_clusters = g_pair_clusters;   // 0 not asked yet, -1 unavailable
     static std::atomic<bool> configured[64];            // per instantiation of the kernel
     cudaLaunchConfig_t cfg{};
@@ -1060,15 +1074,14 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtens
     cfg.attrs = attr; cfg.numAttrs = 1;
     int nc = max_clusters[dev].load(std::memory_order_acquire);
     if (nc == 0 || !configured[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(tcgemm::pair::gemm_tc_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             kSmem);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e != cudaSuccess) return (int)e;
         int sms = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return (int)e;
         cfg.gridDim = dim3(2 * std::max(1, sms / 2));
         int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, tcgemm::pair::gemm_tc_pair_kernel<EPI>, &cfg);
+        e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
         if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
         nc = n > 0 ? std::min(n, sms / 2) : -1;
         max_clusters[dev].store(nc, std::memory_order_release);
@@ -1076,12 +1089,39 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtens
     }
     if (nc < 0) return RFK_EUNSUPPORTED;
     p.tiles_m = (p.M + 2 * tcgemm::BM - 1) / (2 * tcgemm::BM);
+    if (BN != 256) p.tiles_n = (p.N + BN - 1) / BN;
     const int tiles = p.tiles_m * p.tiles_n;
     cfg.gridDim = dim3(2 * std::min(tiles, nc));
     cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::pair::gemm_tc_pair_kernel<EPI>, ma, mw0, mw1, mc, mr, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mw0, mw1, mc, mr, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
+}
+
+// Tiles of 192 accumulator columns instead of 256 where they need no more rounds of the pairs: a K block of them takes three quarters
+// of the products and seven eighths of the copies, and the bits are the same. us, 256 / 192: 2500 x 1024 x 4096 (0.54 and 0.81 rounds) 25.3 / 20.1,
+// 4864 x 1024 x 4096 (1.03, 1.54) 42.8 / 34.7, 5665 x 1024 x 4096 (1.24, 1.86) 43.5 / 38.6, x 1024 14.6 / 12.8, 3136 x 3072 x 1024 (2.11, 2.81)
+// 19.9 / 17.3. One round more loses even where three quarters of the rounds are fewer: 6400 x 3072 x 1024 (5, 6 rounds) 30.9 / 31.4,
+// 3400 x 3072 x 1024 (3, 4) 20.0 / 20.6, 4096 x 1024 x 4096 (1, 2) 25.6 / 33.7, because a round that is not full runs its K blocks faster
+// (0.30 us on few pairs, 0.36 to 0.45 on all).
+bool narrow_tile(int M, int N, int pairs) {
+    const long long rows = ceil_div(M, 2 * tcgemm::BM);
+    const long long wide = ceil_div(rows * ceil_div(N, 256), pairs), narrow = ceil_div(rows * ceil_div(N, 192), pairs);
+    return narrow == wide;
+}
+
+// W (and W_up) as in launch_gemm, for the boxes of the tile width; the head-split form with row statistics needs 256 columns, one sum
+template <int EPI>
+int launch_gemm_pair(const CUtensorMap& ma, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev, cudaStream_t st,
+                     const CUtensorMap* heads_map = nullptr) {
+    constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    CUtensorMap mw0, mw1;
+    if constexpr (!kGate) {
+        if (!(EPI == tcgemm::kEpiHeads && p.row_ss) && narrow_tile(p.M, p.N, sm_count(dev) / 2))
+            return make_map_2d(&mw0, W, p.N, p.K, ldw, 96) ? launch_pair_tiles<EPI, 192>(ma, mw0, mw0, p, dev, st, heads_map) : RFK_EUNSUPPORTED;
+    }
+    if (!make_map_2d(&mw0, W, p.N, p.K, ldw) || (kGate && !make_map_2d(&mw1, W_up, p.N, p.K, ldw))) return RFK_EUNSUPPORTED;
+    return launch_pair_tiles<EPI, 256>(ma, mw0, kGate ? mw1 : mw0, p, dev, st, heads_map);
 }
 
 // rank-5 map of a head-split output: [part][group][head][seq][hd] halves, boxes of 32 rows x 64 columns
@@ -1097,16 +1137,6 @@ bool make_map_heads(CUtensorMap* m, const void* base, int seq, int out_seq, int 
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-int sm_count(int dev) {
-    static std::atomic<int> count[64];
-    int n = count[dev].load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); return 0; }
-        count[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
 }
 
 // ---- small tiles: their launch, and the rules that choose them
@@ -1212,13 +1242,12 @@ int launch_gemm(const void* A, long long lda, const void* W, const void* W_up, l
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
     CUtensorMap ma, mw0, mw1;
-    if (!make_map_2d(&ma, A, p.M, p.K, lda) || !make_map_2d(&mw0, W, p.N, p.K, ldw) ||
-        !make_map_2d(&mw1, kGate ? W_up : W, p.N, p.K, ldw))
-        return RFK_EUNSUPPORTED;
+    if (!make_map_2d(&ma, A, p.M, p.K, lda)) return RFK_EUNSUPPORTED;
     if (path != 3) {
-        const int rc = launch_gemm_pair<EPI>(ma, mw0, mw1, p, dev, st);
+        const int rc = launch_gemm_pair<EPI>(ma, W, W_up, ldw, p, dev, st);
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
+    if (!make_map_2d(&mw0, W, p.N, p.K, ldw) || !make_map_2d(&mw1, kGate ? W_up : W, p.N, p.K, ldw)) return RFK_EUNSUPPORTED;
     return launch_gemm_single<EPI>(ma, mw0, mw1, p, dev, st);
 }
 
@@ -1298,13 +1327,13 @@ int rfk::gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long lo
         }
         if (rc != RFK_EUNSUPPORTED) return rc;
     }
-    CUtensorMap ma, mw, mh;
-    if (!make_map_2d(&ma, A, M, K, lda) || !make_map_2d(&mw, W, N, K, ldw) ||
+    CUtensorMap ma, mh;
+    if (!make_map_2d(&ma, A, M, K, lda) ||
         !make_map_heads(&mh, out, seq_len, out_seq, num_heads, head_dim, M / seq_len, parts, parts > 1 ? part_stride : (long long)M * dim))
         return RFK_EUNSUPPORTED;
     p.tiles_m = (M + tcgemm::BM - 1) / tcgemm::BM;
     p.tiles_n = N / 256;
-    return launch_gemm_pair<tcgemm::kEpiHeads>(ma, mw, mw, p, dev, as_stream(stream), &mh);
+    return launch_gemm_pair<tcgemm::kEpiHeads>(ma, W, nullptr, ldw, p, dev, as_stream(stream), &mh);
 }
 
 extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ldw, rfk_half* out,
