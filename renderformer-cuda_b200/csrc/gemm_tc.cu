@@ -560,40 +560,55 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const int lane_grp = warp & 3;
         const int local = BM_ == 64 ? lane_grp * 16 + lane : lane_grp * 32 + lane, row = m0 + local;
         const bool mine = warp >= 2 && (BM_ == 128 || lane < 16), row_ok = mine && row < p.M;
-        if (want_ss) pair::cluster_sync();
+        // The gathering stores come ahead of the output's: the second barrier's arrival waits for the stores before it, and the output's
+        // are on their way while the cluster meets (256 x 1024 x 1024 6.10 -> 5.68 us, 1600 x 1024 x 1024 9.89 -> 8.91).
+        if (want_ss) pair::cluster_arrive();
+        uint32_t o[BN_ / 2];
         if (warp >= 2 && acc_ok) {
             tc::tc_fence_after();
             const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
-            const int hd = p.head_units * 64, heads = p.units / p.head_units;
-            const size_t rows_off = ((size_t)(row / p.seq) * heads * p.out_seq + row % p.seq) * hd;
-            const uint32_t gather = pair::map_to_cta(base, 0) + local * kPitch + (n0 % 256) * 2;
 #pragma unroll
             for (int c = 0; c < BN_ / 32; ++c) {
                 uint32_t v[32];
                 tc::tmem_ld32(t_acc + c * 32, v);
                 tc::tc_wait_ld(v);
-                const int g = (n0 + c * 32) / 64, u = g % p.units;   // 64-column unit over all parts, and within its part
-                __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + rows_off + (size_t)(u / p.head_units) * p.out_seq * hd +
-                              (u % p.head_units) * 64 + (c & 1) * 32;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint32_t o[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) o[i] = pack_half2(__uint_as_float(v[8 * q + 2 * i]), __uint_as_float(v[8 * q + 2 * i + 1]));
-                    if (row_ok) *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-                    if (want_ss && mine)
-                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(gather + c * 64 + q * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-                }
+                for (int i = 0; i < 16; ++i) o[c * 16 + i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
             }
         }
         if (want_ss) {
             __syncwarp();
-            pair::cluster_sync();
+            pair::cluster_wait();
+            if (mine && acc_ok) {
+                const uint32_t gather = pair::map_to_cta(base, 0) + local * kPitch + (n0 % 256) * 2;
+#pragma unroll
+                for (int q = 0; q < BN_ / 8; ++q)
+                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                 ::"r"(gather + q * 16), "r"(o[4 * q]), "r"(o[4 * q + 1]), "r"(o[4 * q + 2]), "r"(o[4 * q + 3]) : "memory");
+            }
+            __syncwarp();
+            pair::cluster_arrive();
+        }
+        if (row_ok && acc_ok) {
+            const int hd = p.head_units * 64, heads = p.units / p.head_units;
+            const size_t rows_off = ((size_t)(row / p.seq) * heads * p.out_seq + row % p.seq) * hd;
+#pragma unroll
+            for (int c = 0; c < BN_ / 32; ++c) {
+                const int g = (n0 + c * 32) / 64, u = g % p.units;   // 64-column unit over all parts, and within its part
+                __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + rows_off + (size_t)(u / p.head_units) * p.out_seq * hd +
+                              (u % p.head_units) * 64 + (c & 1) * 32;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(o[c * 16 + 4 * q], o[c * 16 + 4 * q + 1], o[c * 16 + 4 * q + 2], o[c * 16 + 4 * q + 3]);
+            }
+        }
+        if (want_ss) {
+            __syncwarp();
+            pair::cluster_wait();
             if (pair::cluster_rank() == 0 && row_ok) {
                 const uint4* src = reinterpret_cast<const uint4*>(smem_raw + local * kPitch);
                 float ss = 0.0f;
-#pragma unroll 8
+#pragma unroll
                 for (int q = 0; q < 32; ++q) {
                     const uint4 w = src[q];
                     const uint32_t x[4] = {w.x, w.y, w.z, w.w};
