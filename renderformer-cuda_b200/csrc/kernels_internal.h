@@ -11,10 +11,10 @@ int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ld
                float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int out_seq, int num_heads,
                int head_dim, rfk_stream_t stream);
 
-// rfk_qkv_norm_rope_transpose behind gemm_heads: parts [heads][seq_len][head_dim] normalised over the row (all heads) and rotated in
-// place, with that kernel's bits
+// rfk_qkv_norm_rope_transpose behind gemm_heads: parts [heads][out_seq][head_dim], of which the first seq_len rows of each head are
+// normalised over the row (all heads) and, unless cos_vals is NULL, rotated in place, with that kernel's bits
 int qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts, const rfk_half* cos_vals,
-                       const rfk_half* sin_vals, int seq_len, int num_heads, int head_dim, float eps, rfk_stream_t stream);
+                       const rfk_half* sin_vals, int seq_len, int out_seq, int num_heads, int head_dim, float eps, rfk_stream_t stream);
 
 // out = rmsnorm_f32(a) + rmsnorm_f32(b) + c, fp32, in one pass with the bits of the separate steps; a, b fp16 [rows, dim], c fp16 [dim];
 // dim % 8 == 0, dim <= 1024, 16-byte aligned, else RFK_EUNSUPPORTED
@@ -87,6 +87,10 @@ extern "C" int rfk_rmsnorm_residual_f16_windows_in_l2(rfk_half* x, const rfk_hal
                                                       int dim, int window_size, int shift_size, int windowed_operand, float eps,
                                                       rfk_stream_t stream);
 
+// qk_norm_rope_heads of q and k, or of q alone (k NULL), for its test
+extern "C" int rfk_qk_norm_rope_heads(rfk_half* q, rfk_half* k, const float* gamma_q, const float* gamma_k, const rfk_half* cos_vals,
+                                      const rfk_half* sin_vals, int seq_len, int out_seq, int num_heads, int head_dim, float eps,
+                                      rfk_stream_t stream);
 // norm_pair_add, for its test
 extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,
                                  float* out, int rows, int dim, float eps, rfk_stream_t stream);

@@ -14,6 +14,7 @@
 // chunk of the second half, so each element is read once (two 128-bit loads), written
 // once, and the in-place update is race-free by construction. The cos/sin chunk is
 // loaded once per thread and reused across the heads the thread walks.
+#include <algorithm>
 #include "common.cuh"
 #include "kernels_internal.h"
 
@@ -379,13 +380,114 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
     }
 }
 
+// The HEADS form for NP parts (q and k, or k alone) that all have a norm, rows of 32 * WPR rotation-pair chunks: a thread keeps its chunk of
+// every part over all of its rows, so that the norm weights are read once, the rotation tables once for both parts, and the next
+// row's loads are in flight while a row is summed. Bound by L2 and that latency: as many CTAs as are resident at once (160
+// registers: three an SM) are the best; us for 5665 rows of q and k, 16 heads of 64: one row a block and part 14.3, two CTAs an SM 13.9,
+// three 10.1, four 12.3 (a second, partial round), eight 11.4; held to 128 registers four 12.6. Same arithmetic, same bits.
+template <int WPR, int NP>
+__global__ void __launch_bounds__(128)
+qk_rows_kernel(const __grid_constant__ QkvParts parts, const __half* __restrict__ cos_vals, const __half* __restrict__ sin_vals,
+               int seq_len, int out_seq, int num_heads, int head_dim, float eps) {
+    constexpr int RPC = 4 / WPR;  // rows per CTA at a time
+    __shared__ float s_part[2][NP][4];
+    pdl_wait();
+    pdl_trigger();
+    const int p = threadIdx.x % (32 * WPR), sub = threadIdx.x / (32 * WPR), w = threadIdx.x >> 5;
+    const int dim = num_heads * head_dim, cpt = head_dim / 16, half_d = head_dim / 2;
+    const int h = p / cpt, j = (p % cpt) * 8;
+    __half* out[NP];
+    float g[NP][2][8];
+#pragma unroll
+    for (int t = 0; t < NP; ++t) {
+        out[t] = parts.out[t] + (size_t)h * out_seq * head_dim + j;
+        ldg_float8(parts.gamma[t] + h * head_dim + j, g[t][0]);
+        ldg_float8(parts.gamma[t] + h * head_dim + j + half_d, g[t][1]);
+    }
+    const bool rope = cos_vals != nullptr;
+    struct Row { Half8 x[NP][2], c[2], s[2]; };
+    auto load = [&](int row, Row& r) {   // a row past the end reads nothing: it may be another thread's, in place
+        if (row >= seq_len) { r = Row{}; return; }
+        const size_t o = (size_t)row * head_dim;
+#pragma unroll
+        for (int t = 0; t < NP; ++t) {
+            r.x[t][0] = ld_half8(out[t] + o);
+            r.x[t][1] = ld_half8(out[t] + o + half_d);
+        }
+        if (rope) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                r.c[e] = ldg_half8(cos_vals + o + j + e * half_d);
+                r.s[e] = ldg_half8(sin_vals + o + j + e * half_d);
+            }
+        }
+    };
+    Row cur, nxt;
+    int base = blockIdx.x * RPC, buf = 0;
+    load(base + sub, cur);
+    for (; base < seq_len; base += gridDim.x * RPC, buf ^= 1) {
+        const int row = base + sub;
+        load(row + gridDim.x * RPC, nxt);
+        float lo[2][8], hi[2][8], ss[NP] = {};
+#pragma unroll
+        for (int t = 0; t < NP; ++t) {
+            unpack8(cur.x[t][0], lo[t]);
+            unpack8(cur.x[t][1], hi[t]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                ss[t] = fmaf(lo[t][i], lo[t][i], ss[t]);
+                ss[t] = fmaf(hi[t][i], hi[t][i], ss[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < NP; ++t) ss[t] = warp_sum(ss[t]);
+        if (WPR > 1) {
+            if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+                for (int t = 0; t < NP; ++t) s_part[buf][t][w] = ss[t];
+            }
+            __syncthreads();   // the buffers take turns: one barrier a row
+            const int w0 = (w / WPR) * WPR;
+#pragma unroll
+            for (int t = 0; t < NP; ++t) {
+                ss[t] = 0.0f;
+#pragma unroll
+                for (int i = 0; i < WPR; ++i) ss[t] += s_part[buf][t][w0 + i];
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < NP; ++t) {
+            const float rinv = rsqrtf(ss[t] / (float)dim + eps);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                // the unfused path stores the normalised value as fp16 before rotating it
+                lo[t][i] = round_half((lo[t][i] * rinv) * g[t][0][i]);
+                hi[t][i] = round_half((hi[t][i] * rinv) * g[t][1][i]);
+            }
+            if (rope) {
+                float cl[8], sl[8], ch[8], sh[8];
+                unpack8(cur.c[0], cl);
+                unpack8(cur.s[0], sl);
+                unpack8(cur.c[1], ch);
+                unpack8(cur.s[1], sh);
+                rotate8(lo[t], hi[t], cl, sl, ch, sh);
+            }
+            if (row < seq_len) {
+                store8(out[t] + (size_t)row * head_dim, lo[t]);
+                store8(out[t] + (size_t)row * head_dim + half_d, hi[t]);
+            }
+        }
+        cur = nxt;
+    }
+}
+
 }  // namespace rfk
 
 using namespace rfk;
 
 int rfk::qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts_io, const rfk_half* cos_vals,
-                            const rfk_half* sin_vals, int seq_len, int num_heads, int head_dim, float eps, rfk_stream_t stream) {
-    if (!gamma || !parts_io || n_parts < 1 || n_parts > 3 || seq_len < 0 || num_heads <= 0 || head_dim <= 0) return RFK_EINVAL;
+                            const rfk_half* sin_vals, int seq_len, int out_seq, int num_heads, int head_dim, float eps, rfk_stream_t stream) {
+    if (!gamma || !parts_io || n_parts < 1 || n_parts > 3 || seq_len < 0 || out_seq < seq_len || num_heads <= 0 || head_dim <= 0) return RFK_EINVAL;
     const long long dim = (long long)num_heads * head_dim;
     if (head_dim % 16 != 0 || dim > 2048) return RFK_EUNSUPPORTED;
     QkvParts parts{};
@@ -399,15 +501,33 @@ int rfk::qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* co
     if (cos_vals && (!sin_vals || !aligned16(cos_vals) || !aligned16(sin_vals))) return RFK_EINVAL;
     if (seq_len == 0) return RFK_OK;
     const int npairs = (int)(dim / 16);
+    if (n_parts <= 2 && gamma[0] && (n_parts == 1 || gamma[1]) && (npairs == 32 || npairs == 64)) {   // wider rows are summed two chunks a thread
+        const int wpr = npairs / 32;
+        const long long resident = (long long)kNumSMs * (n_parts == 2 ? 3 : 4);   // 160 and 116 registers a thread   // 160 and 116 registers a thread
+        const unsigned grid = (unsigned)std::min<long long>(ceil_div(seq_len, 4 / wpr), resident);
+        const auto kernel = n_parts == 2 ? (wpr == 1 ? qk_rows_kernel<1, 2> : qk_rows_kernel<2, 2>)
+                                         : (wpr == 1 ? qk_rows_kernel<1, 1> : qk_rows_kernel<2, 1>);
+        launch_pdl(kernel, dim3(grid), dim3(128), 0, as_stream(stream), parts, (const __half*)cos_vals, (const __half*)sin_vals, seq_len,
+                   out_seq, num_heads, head_dim, eps);
+        return launch_status();
+    }
 #define RFK_QK_HEADS(N, W)                                                                                   \
     launch_pdl(qkv_epilogue_kernel<N, W, true>, dim3(ceil_div(seq_len, 4 / W), n_parts), dim3(128), 0, as_stream(stream), \
                (const __half*)nullptr, 0LL, parts, (const __half*)cos_vals, (const __half*)sin_vals, 1, seq_len, num_heads, \
-               head_dim, eps, (long long)seq_len)
+               head_dim, eps, (long long)out_seq)
     if (npairs <= 32) RFK_QK_HEADS(1, 1);
     else if (npairs <= 64) RFK_QK_HEADS(1, 2);
     else RFK_QK_HEADS(2, 2);
 #undef RFK_QK_HEADS
     return launch_status();
+}
+
+extern "C" int rfk_qk_norm_rope_heads(rfk_half* q, rfk_half* k, const float* gamma_q, const float* gamma_k, const rfk_half* cos_vals,
+                                      const rfk_half* sin_vals, int seq_len, int out_seq, int num_heads, int head_dim, float eps,
+                                      rfk_stream_t stream) {
+    const float* g[2] = {gamma_q, gamma_k};
+    rfk_half* x[2] = {q, k};
+    return qk_norm_rope_heads(k ? 2 : 1, g, x, cos_vals, sin_vals, seq_len, out_seq, num_heads, head_dim, eps, stream);
 }
 
 extern "C" int rfk_triangle_rope_freqs(const rfk_half* pos, const float* learned_freqs,
