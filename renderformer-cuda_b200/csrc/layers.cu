@@ -517,34 +517,41 @@ extern "C" int rfk_self_attention(rfk_ctx* ctx, const rfk_mha_weights* w, const 
 
 // cache_flags: bit 1: V_cached is shared by the B batch elements; bit 0: K_cached is this view's rotated keys already multiplied by the cross-attention query norm's weight
 // (what rfk_session prepares for all layers at once); 0 for keys as the public entry point receives them.
+// x_in: what the layer reads, x or another buffer, which stays as it is; x_out: where its result goes, x or another buffer.
 int rfk_layers::decoder_layer_impl(
-    rfk_ctx* ctx, const rfk_decoder_layer_weights* w, rfk_half* x, const rfk_half* pending_residual,
+    rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const rfk_half* x_in, rfk_half* x, rfk_half* x_out, const rfk_half* pending_residual,
     const rfk_half** pending_out, rfk_half* temp, rfk_half* proj_buf, rfk_half* qkv_buf, rfk_half* ffn_buf,
     rfk_half* window_buf, float* cross_score_buf, float* self_score_buf, const rfk_half* K_cached,
     const rfk_half* V_cached, int B, int Sq, int Sk, int n_keys, int dim, int num_heads, int ffn_hidden,
     int patch_h, int patch_w, int window_size, int shift_size, const uint8_t* shift_mask,
     const rfk_half* q_rope_cos, const rfk_half* q_rope_sin, const rfk_half* k_rope_cos,
     const rfk_half* k_rope_sin, int cache_flags, rfk_stream_t stream) {
-    if (!ctx || !w || !x || !temp || !proj_buf || !qkv_buf || !ffn_buf || !window_buf) return RFK_EINVAL;
+    if (!ctx || !w || !x_in || !x || !x_out || !temp || !proj_buf || !qkv_buf || !ffn_buf || !window_buf) return RFK_EINVAL;
     if (Sq != patch_h * patch_w) return RFK_EINVAL;
     const int Mq = B * Sq;
-    // 1) (deferred residual of the previous layer, if any +) pre-norm -> cached cross-attention
-    TRY(rfk_rmsnorm_residual_f16(x, pending_residual, w->query_norm_gamma, temp, Mq, dim, kEpsFp16, stream));
     // 2) residual + pre-norm -> swin attention -> residual + pre-norm of the FFN. When the fused norm can take an
     //    operand in window order, the cyclic shift / window partition and their inverse cost no launch: the first norm
     //    writes the windows, the second reads the attention output out of them; and the residual add of the
     //    cross-attention is the epilogue of its output projection (x += ...), so the first norm reads x only.
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool win_ok = window_size > 0 && patch_h % window_size == 0 && patch_w % window_size == 0 &&
-                        num_heads > 0 && dim % num_heads == 0 && dim % 8 == 0 && dim <= 2048 && a16(x) && a16(window_buf) &&
+                        num_heads > 0 && dim % num_heads == 0 && dim % 8 == 0 && dim <= 2048 && a16(x_in) && a16(x) && a16(x_out) && a16(window_buf) &&
                         a16(temp) && a16(qkv_buf) && a16(w->self_attn_norm_gamma) && a16(w->ffn_norm_gamma);
+    if (x_in != x && (!win_ok || w->cross_attn.out_proj_b || pending_residual)) {   // the steps below that add onto x itself
+        cudaError_t e = cudaMemcpyAsync(x, x_in, (size_t)Mq * dim * sizeof(rfk_half), cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
+        if (e != cudaSuccess) return (int)e;
+        x_in = x;
+    }
+    // 1) (deferred residual of the previous layer, if any +) pre-norm -> cached cross-attention
+    if (pending_residual) TRY(rfk_rmsnorm_residual_f16(x, pending_residual, w->query_norm_gamma, temp, Mq, dim, kEpsFp16, stream));
+    else TRY(rfk_rmsnorm(x_in, w->query_norm_gamma, temp, Mq, dim, kEpsFp16, stream));
     // Row statistics of the deferred QK-norms live in buffers that are idle while they are needed: window_buf during the
     // cross-attention, temp during the window attention (each holds Mq*dim halves; the statistics need Mq*dim/128 floats).
     float* cross_ss = dim % 256 == 0 ? reinterpret_cast<float*>(window_buf) : nullptr;
     float* swin_ss = dim % 256 == 0 ? reinterpret_cast<float*>(temp) : nullptr;
     if (win_ok) {
         if (!w->cross_attn.out_proj_b) {
-            TRY(cross_attention_impl(ctx, &w->cross_attn, temp, x, x, proj_buf, cross_ss, cache_flags, cross_score_buf, K_cached,
+            TRY(cross_attention_impl(ctx, &w->cross_attn, temp, x, x_in, proj_buf, cross_ss, cache_flags, cross_score_buf, K_cached,
                                      V_cached, B, Sq, Sk, n_keys, dim, dim, num_heads, q_rope_cos, q_rope_sin, k_rope_cos,
                                      k_rope_sin, stream));
             TRY(rfk_rmsnorm_residual_f16_windows(x, nullptr, w->self_attn_norm_gamma, window_buf, B, patch_h, patch_w, dim,
@@ -576,7 +583,7 @@ int rfk_layers::decoder_layer_impl(
     // 3) FFN with its residual add in the epilogue of the W2 product: x is complete when the layer returns and
     //    nothing is left pending for the next layer
     if (!w->ffn.w1 || !w->ffn.w2 || !w->ffn.w3 || ffn_hidden <= 0) return RFK_EINVAL;
-    TRY(ffn_core(ctx, &w->ffn, temp, x, x, qkv_buf, Mq, dim, ffn_hidden, stream));
+    TRY(ffn_core(ctx, &w->ffn, temp, x_out, x, qkv_buf, Mq, dim, ffn_hidden, stream));
     if (pending_out) *pending_out = nullptr;
     return RFK_OK;
 }
@@ -589,7 +596,7 @@ extern "C" int rfk_decoder_layer_forward_cached(
     int patch_h, int patch_w, int window_size, int shift_size, const uint8_t* shift_mask,
     const rfk_half* q_rope_cos, const rfk_half* q_rope_sin, const rfk_half* k_rope_cos,
     const rfk_half* k_rope_sin, rfk_stream_t stream) {
-    return rfk_layers::decoder_layer_impl(ctx, w, x, pending_residual, pending_out, temp, proj_buf, qkv_buf, ffn_buf, window_buf,
+    return rfk_layers::decoder_layer_impl(ctx, w, x, x, x, pending_residual, pending_out, temp, proj_buf, qkv_buf, ffn_buf, window_buf,
                                           cross_score_buf, self_score_buf, K_cached, V_cached, B, Sq, Sk, n_keys, dim, num_heads,
                                           ffn_hidden, patch_h, patch_w, window_size, shift_size, shift_mask, q_rope_cos,
                                           q_rope_sin, k_rope_cos, k_rope_sin, 0, stream);

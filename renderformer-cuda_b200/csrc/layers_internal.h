@@ -25,7 +25,8 @@ constexpr float kEpsFp32 = 1.1920929e-07f;  // 2^-23, the reference's kEpsFp32 (
 
 // rfk_decoder_layer_forward_cached with cache_flags (bit 0: keys arrive rotated and carrying the query norm weight; bit 1:
 // the values are shared by the batch elements; see layers.cu); the session calls this form.
-int decoder_layer_impl(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, rfk_half* x, const rfk_half* pending_residual,
+int decoder_layer_impl(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const rfk_half* x_in, rfk_half* x, rfk_half* x_out,
+                       const rfk_half* pending_residual,
                        const rfk_half** pending_out, rfk_half* temp, rfk_half* proj_buf, rfk_half* qkv_buf, rfk_half* ffn_buf,
                        rfk_half* window_buf, float* cross_score_buf, float* self_score_buf, const rfk_half* K_cached,
                        const rfk_half* V_cached, int B, int Sq, int Sk, int n_keys, int dim, int num_heads, int ffn_hidden,

@@ -257,6 +257,8 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
 
     const int n_keys = (flags & RFK_SESSION_PAD_KEYS_ATTEND) ? Se_pad : Se;
     const rfk_half* pending = nullptr;
+    // A tapped layer's last product writes the tap and the next layer reads it there; the token map that is also a tap is copied.
+    const rfk_half* tokens = rtok;
     const int L4 = std::max(1, m.dec_layers / 4);
     const int cache_flags = (prescale ? 1 : 0) | (V > 1 ? 2 : 0);  // keys rotated + weighted here; values shared by the views
     for (int i = 0; i < m.dec_layers; ++i) {
@@ -267,16 +269,16 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
         // a tapped (or the last) layer finishes x itself; the others leave their FFN residual
         // to the first kernel of the next layer
         if (i < 2) TRY_CUDA(cudaStreamWaitEvent(stream, ev_rot[i], 0));
-        TRY(decoder_layer_impl(ctx, &m.dec[i], rtok, pending, (tap || last) ? nullptr : &next_pending,
+        rfk_half* const out = tap ? taps_out[(i + 1) / L4 - 1] : last ? result_out : rtok;
+        TRY(decoder_layer_impl(ctx, &m.dec[i], tokens, rtok, out, pending, (tap || last) ? nullptr : &next_pending,
                                temp, proj, qkv, ffn, win, score, self_score, kRot(i), kvV(i), V, nP,
                                Se_pad, n_keys, dim, m.num_heads, m.ffn_hidden, pH, pW, m.window_size,
                                shift, shift > 0 ? shift_mask : nullptr, nullptr, nullptr, nullptr, nullptr, cache_flags, s));
         pending = next_pending;
-        if (tap)
-            TRY_CUDA(cudaMemcpyAsync(taps_out[(i + 1) / L4 - 1], rtok, (size_t)rows * dim * sizeof(rfk_half),
-                                     cudaMemcpyDeviceToDevice, stream));
+        tokens = out;
     }
-    TRY_CUDA(cudaMemcpyAsync(result_out, rtok, (size_t)rows * dim * sizeof(rfk_half), cudaMemcpyDeviceToDevice, stream));
+    if (tokens != result_out)
+        TRY_CUDA(cudaMemcpyAsync(result_out, tokens, (size_t)rows * dim * sizeof(rfk_half), cudaMemcpyDeviceToDevice, stream));
     if (dpt) {
         // image head over this frame's taps, then ELU(1e-3) -> fp32 -> 10^x - 1 in one kernel (render_session.cu:239-253)
         TRY(rfk_dpt_forward(dpt, taps_out, nullptr, s));
