@@ -459,7 +459,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // ------------------------------------------------------------ issuer of O += P V (the warp's elected lane)
         // The whole warp runs the loop and one lane issues (elect_one): with a single thread's loop the issue of a tile's
         // products, not the tensor pipe, paced the 128-wide heads (8 x 4096 x 5665: 96 -> 84 us with the trailing reference they
-        // had then; with the exact one the softmax warps pace them, 102 us = 0.93 PFLOP/s; 64-wide heads 142 -> 139 us).
+        // had then; 64-wide heads 142 -> 139 us). The elected lane in a loop of its own is 1 to 4 % slower here.
         // tile j: score buffer j % kSBufs (its use number j / kSBufs gives the barrier phase), ring stage j % kStages
         const bool leader = tc::elect_one();
         constexpr uint32_t idesc_pv = tc::umma_idesc_f16(BM, HD, 1);  // B = V tile, MN-major
@@ -537,7 +537,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // maximum, as in flash_attention_kernel: a row's largest probabilities are then exactly 1 or round on the finer half
         // of their binade. Against 64 bits the deferred reference was 3 % further off than that kernel on unit-variance
         // scores and 19 to 21 % on scores of two and three times that; with the exact one the two agree to 1e-4 (8 x 4096 x
-        // 5665: 81 us deferred, 102 us exact, 361 us flash_attention_kernel).
+        // 5665: 81 us deferred, 102 us exact, 92 with O rescaled by its own warpgroup, 361 us flash_attention_kernel).
         constexpr bool kExactMax = HD == 128;
         constexpr float kRescaleThreshold = kExactMax ? 0.0f : 8.0f;
         const int blk = warp >> 2;
