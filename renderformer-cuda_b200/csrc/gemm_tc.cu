@@ -662,7 +662,10 @@ constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA
 // 2.8 us per tile for the register-to-global epilogue, most of it the scattered stores). With the residual
 // epilogue the same buffers first receive the residual tile by TMA loads issued before the accumulator is ready
 // (one buffer per 64-column unit, so the loads of a whole tile are in flight during its main loop); the sum
-// overwrites the residual in place and is stored from there. Plain / SwiGLU: two buffers per warp in turn.
+// overwrites the residual in place and is stored from there. Plain / SwiGLU / head-split: two buffers per warp in turn, one
+// store after the other, over unit and tile ends alike: a unit may be written once at most one store is still reading, which is then
+// the one before it, of the other buffer. (Counted from each tile's start instead, a tile of an odd number of units - 192 columns, or
+// a tail of N - ends in the buffer that the next one begins with, whose last store may still be reading it.)
 constexpr int kUnitCols = 64;
 constexpr int kUnitBytes = 32 * kUnitCols * 2;       // 4 KB
 // BN: accumulator columns of a tile, 256 or 192 (narrow_tile)
@@ -709,25 +712,26 @@ __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* ma
 }
 
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
-// t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0.
+// t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0. turn: the staging buffer of the
+// next store, kept from tile to tile (not with the residual epilogue).
 template <int EPI, int BN>
 __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, uint32_t t_acc,
                                                      unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
-                                                     int row0, int n0, int lane, volatile int* abort_flag) {
+                                                     int row0, int n0, int lane, int& turn, volatile int* abort_flag) {
     constexpr int kUnits = Cfg<EPI, BN>::kUnits;
     const uint32_t stage_base = tc::smem_addr(stage_ptr);
     uint32_t v[32];
     float ss = 0.0f;   // kEpiHeads: this row's sum of squares over the tile
 #pragma unroll 1
     for (int u = 0; u < kUnits; ++u) {
-        const int b = (EPI == RFK_GEMM_EPI_RESIDUAL) ? u : (u & 1);
+        const int b = (EPI == RFK_GEMM_EPI_RESIDUAL) ? u : turn;
         unsigned char* buf = stage_ptr + b * kUnitBytes;
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                 // this unit's residual box has landed (also for units beyond N)
             if (!tc::mbar_wait_warp(&res_full[u], res_parity, abort_flag)) return false;
         }
 
         if (n0 + u * kUnitCols >= p.N) continue;            // uniform: the tile's tail lies beyond N
-        if (EPI != RFK_GEMM_EPI_RESIDUAL) {                 // the store issued two units ago must have read this buffer
+        if (EPI != RFK_GEMM_EPI_RESIDUAL) {                 // the store before the last one must have read this buffer
             if (lane == 0) bulk_wait_read<1>();
             __syncwarp();
         }
@@ -805,6 +809,7 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
             }
             bulk_commit();
         }
+        turn ^= 1;
     }
     if (EPI == kEpiHeads && p.row_ss) {
         const int dim = p.units * kUnitCols, part = n0 / dim, row = row0 + lane;
@@ -942,7 +947,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const uint32_t lane_off = (uint32_t)(lane_grp * 32) << 16;
         unsigned char* my_stage = staging + lane_grp * Cfg<EPI, BN>::kBufsPerWarp * kUnitBytes;
         uint64_t* my_res = ctrl->res_full[lane_grp];
-        int tl = 0;
+        int tl = 0, turn = 0;
         for (int t = first_tile; t < num_tiles; t += tile_step, ++tl) {
             const bool last = t + tile_step >= num_tiles;
             const int acc = tl & 1;
@@ -960,7 +965,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tc::tc_fence_after();
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(4);   // first tile's accumulator complete
             ok = epilogue_tile_staged<EPI, BN>(p, &map_c, tmem_cta + lane_off + acc * BNACC, my_stage, my_res, tl & 1, row0, n0,
-                                           lane, abort_flag);
+                                           lane, turn, abort_flag);
             if (!ok) break;
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(5);   // its epilogue done (stores issued)
             // every tcgen05.ld of this warp has completed: hand the accumulator back
