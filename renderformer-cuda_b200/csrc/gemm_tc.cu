@@ -339,7 +339,9 @@ namespace pair { using namespace pair_ptx; }
 //   the elected lanes alone, the others waiting at the warp's barrier, to 0.10 (us, whole warps / lanes alone, weights in L2: 256 x 1024 x
 //   4096 9.63 / 8.23, 256 x 1024 x 1024 3.90 / 3.62, 576 x 1024 x 4096 11.1 / 9.3; 128 x 64 tiles 1024 x 1024 x 4096 12.45 / 12.18; the
 //   tensor pipe alone would take 0.05 us a block). 128 x 128 tiles keep whole warps: 2304 x 1024 x 4096 16.9 / 17.6, 1600 x 1024 x 4096
-//   16.4 / 17.4. Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
+//   16.4 / 17.4. The 128 x 64 tile's producer is lane 0 with the plain and residual epilogues (elected / lane 0, issuer elected in both: 2779 x 384 x
+//   4096 13.2 / 12.6, 1115 x 1024 x 4096 12.2 / 11.5, x 1024 4.87 / 4.88) and an elected lane with the others (SwiGLU 1024 x 512 x 1024 5.09 /
+//   5.70, head-split 1024 x 1024 x 4096 12.0 / 12.3). Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
 //   weights asked for ahead of the kernel's wait for its predecessor, changed nothing or cost (320 x 320 views +4 %).
 //   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
 //   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
@@ -368,6 +370,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                      const __grid_constant__ CUtensorMap map_w1, const Params p) {
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     constexpr bool kWhole = BM_ == 128 && BN_ == 128;   // producer and issuer run their loops as whole warps
+    constexpr bool kLane0 = BM_ == 128 && BN_ == 64 && (EPI == RFK_GEMM_EPI_NONE || EPI == RFK_GEMM_EPI_RESIDUAL);   // the producer is lane 0
     constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
     constexpr int kStages = Cfg<BM_, BN_>::kStages, kStage = Cfg<BM_, BN_>::kStageBytes, kBlock = Cfg<BM_, BN_>::kBlockBytes;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -410,8 +413,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_trigger();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ producer (the warp's elected lane)
-        const bool leader = tc::elect_one();
+        // ------------------------------------------------------------ producer (one lane of the warp)
+        const bool leader = kLane0 ? lane == 0 : tc::elect_one();
         if (kWhole || leader) {
             int it = 0, s = 0, par = 1;   // stage of `it`, and the parity of its barrier's previous phase
             for (; it < num_st; ++it) {
