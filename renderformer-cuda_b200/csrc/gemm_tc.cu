@@ -1083,6 +1083,46 @@ int sm_count(int dev) {
 
 std::atomic<int> g_pair_clusters[64];  // CTA pairs the device can run at once, per device (0 not asked yet, -1 none)
 
+template <int EPI, int BN> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = tcgemm::pair::Cfg<EPI, BN>::kSmemBytes; cfg.stream = st;
+    cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
+    return cfg;
+}
+
+// *pairs: how many CTA pairs of this form the device runs at once (asked once per device and form; every form takes a whole SM a CTA);
+// RFK_EUNSUPPORTED where it cannot co-schedule pairs.
+template <int EPI, int BN>
+int resident_pairs(int dev, int* pairs) {
+    static std::atomic<bool> configured[64];
+    int nc = g_pair_clusters[dev].load(std::memory_order_acquire);
+    if (nc == 0 || !configured[dev].load(std::memory_order_acquire)) {
+        constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI, BN>;
+        cudaLaunchAttribute attr[2];
+        cudaLaunchConfig_t cfg = pair_config<EPI, BN>(attr, nullptr);
+        cfg.numAttrs = 1;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        if (e != cudaSuccess) return (int)e;
+        int sms = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return (int)e;
+        const int half = std::max(1, sms / 2);
+        cfg.gridDim = dim3(2 * half);
+        int n = 0;
+        e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+        if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
+        nc = n > 0 ? std::min(n, half) : -1;
+        g_pair_clusters[dev].store(nc, std::memory_order_release);
+        configured[dev].store(true, std::memory_order_release);
+    }
+    *pairs = nc;
+    return nc > 0 ? RFK_OK : RFK_EUNSUPPORTED;
+}
+
 // CTA-pair kernel: clusters of two; returns RFK_EUNSUPPORTED (nothing launched) when the device cannot co-schedule pairs
 template <int EPI, int BN>
 int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, tcgemm::Params p, int dev,
@@ -1095,45 +1135,22 @@ int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUten
         !make_map_2d(&mr, EPI == RFK_GEMM_EPI_RESIDUAL ? (const void*)p.R : (const void*)p.C, p.M, p.N,
                      EPI == RFK_GEMM_EPI_RESIDUAL ? p.ldr : p.ldc, 32))
         return RFK_EUNSUPPORTED;
-    constexpr int kSmem = tcgemm::pair::Cfg<EPI, BN>::kSmemBytes;
-    std::atomic<int>* max_clusters = g_pair_clusters;   // 0 not asked yet, -1 unavailable
-    static std::atomic<bool> configured[64];            // per instantiation of the kernel
-    cudaLaunchConfig_t cfg{};
+    int pairs = 0;
+    const int rc = resident_pairs<EPI, BN>(dev, &pairs);
+    if (rc != RFK_OK) return rc;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = kSmem; cfg.stream = st;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    int nc = max_clusters[dev].load(std::memory_order_acquire);
-    if (nc == 0 || !configured[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-        if (e != cudaSuccess) return (int)e;
-        int sms = 0;
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return (int)e;
-        cfg.gridDim = dim3(2 * std::max(1, sms / 2));
-        int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
-        nc = n > 0 ? std::min(n, sms / 2) : -1;
-        max_clusters[dev].store(nc, std::memory_order_release);
-        configured[dev].store(true, std::memory_order_release);
-    }
-    if (nc < 0) return RFK_EUNSUPPORTED;
+    cudaLaunchConfig_t cfg = pair_config<EPI, BN>(attr, st);
     p.tiles_m = (p.M + 2 * tcgemm::BM - 1) / (2 * tcgemm::BM);
     if (BN != 256) p.tiles_n = (p.N + BN - 1) / BN;
     const int tiles = p.tiles_m * p.tiles_n;
-    cfg.gridDim = dim3(2 * std::min(tiles, nc));
-    cfg.numAttrs = g_pdl_enabled ? 2 : 1;
+    cfg.gridDim = dim3(2 * std::min(tiles, pairs));
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mw0, mw1, mc, mr, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
 
-// Tiles of 192 accumulator columns instead of 256 where they need no more rounds of the pairs: a K block of them takes three quarters
-// of the products and seven eighths of the copies, and the bits are the same. us, 256 / 192: 2500 x 1024 x 4096 (0.54 and 0.81 rounds) 25.3 / 20.1,
+// Tiles of 192 accumulator columns instead of 256 where they need no more rounds of the pairs that the device places (resident_pairs): a
+// K block of them takes three quarters of the products and seven eighths of the copies, and the bits are the same. us, 256 / 192: 2500 x 1024 x 4096 (0.54 and 0.81 rounds) 25.3 / 20.1,
 // 4864 x 1024 x 4096 (1.03, 1.54) 42.8 / 34.7, 5665 x 1024 x 4096 (1.24, 1.86) 43.5 / 38.6, x 1024 14.6 / 12.8, 3136 x 3072 x 1024 (2.11, 2.81)
 // 19.9 / 17.3. One round more loses even where three quarters of the rounds are fewer: 6400 x 3072 x 1024 (5, 6 rounds) 30.9 / 31.4,
 // 3400 x 3072 x 1024 (3, 4) 20.0 / 20.6, 4096 x 1024 x 4096 (1, 2) 25.6 / 33.7, because a round that is not full runs its K blocks faster
@@ -1151,8 +1168,13 @@ int launch_gemm_pair(const CUtensorMap& ma, const void* W, const void* W_up, lon
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     CUtensorMap mw0, mw1;
     if constexpr (!kGate) {
-        if (!(EPI == tcgemm::kEpiHeads && p.row_ss) && narrow_tile(p.M, p.N, sm_count(dev) / 2))
-            return make_map_2d(&mw0, W, p.N, p.K, ldw, 96) ? launch_pair_tiles<EPI, 192>(ma, mw0, mw0, p, dev, st, heads_map) : RFK_EUNSUPPORTED;
+        if (!(EPI == tcgemm::kEpiHeads && p.row_ss)) {
+            int pairs = 0;
+            const int rc = resident_pairs<EPI, 192>(dev, &pairs);
+            if (rc != RFK_OK) return rc;
+            if (narrow_tile(p.M, p.N, pairs))
+                return make_map_2d(&mw0, W, p.N, p.K, ldw, 96) ? launch_pair_tiles<EPI, 192>(ma, mw0, mw0, p, dev, st, heads_map) : RFK_EUNSUPPORTED;
+        }
     }
     if (!make_map_2d(&mw0, W, p.N, p.K, ldw) || (kGate && !make_map_2d(&mw1, W_up, p.N, p.K, ldw))) return RFK_EUNSUPPORTED;
     return launch_pair_tiles<EPI, 256>(ma, mw0, kGate ? mw1 : mw0, p, dev, st, heads_map);
@@ -1380,6 +1402,10 @@ extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_ha
 
 extern "C" int rfk_gemm_heads_tile(int M, int N, const int* resident) {
     return M > 0 && N > 0 && resident ? heads_tile(M, N, resident) : RFK_EINVAL;
+}
+
+extern "C" int rfk_gemm_pair_tile(int M, int N, int pairs) {
+    return M > 0 && N > 0 && pairs > 0 ? (narrow_tile(M, N, pairs) ? 192 : 256) : RFK_EINVAL;
 }
 
 extern "C" int rfk_gemm_pair_clusters(void) {

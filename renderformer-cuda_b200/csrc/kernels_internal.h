@@ -63,6 +63,9 @@ extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half*
 // [0, *whole_units) stay whole, then for each of *n_handed units {unit, key tiles of its first piece, slot} in launch order.
 extern "C" int rfk_flash_attention_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed,
                                                  unsigned short* first, int max_handed);
+// Columns of the pair kernel's tiles, 192 or 256, for a product of M x N on a device that runs `pairs` CTA pairs at once (narrow_tile
+// in gemm_tc.cu), for its test; host only
+extern "C" int rfk_gemm_pair_tile(int M, int N, int pairs);
 // window_attention_steps, for its test
 extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                                           int BnW, int num_heads, int nW, float scale, rfk_stream_t stream);
