@@ -23,8 +23,15 @@ __device__ __forceinline__ void cluster_sync() {
 // its two halves, for work between them; every thread of both CTAs makes each once, whole warps together
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// An arrival on a barrier of the pair's other CTA, and the waiting side's acquire of such arrivals (of a phase that has been waited for and
+// cannot be followed by another yet). Both name the cluster: the default scope is the CTA, which orders nothing between the
+// accumulator reads of one CTA's threads and the products that the other issues into it next.
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void acquire_remote(uint64_t* bar, uint32_t parity) {
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
+                 ::"r"(tc::smem_addr(bar)), "r"(parity) : "memory");
 }
 
 // ---- shared <-> global tile copies
