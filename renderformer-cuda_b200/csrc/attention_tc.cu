@@ -155,15 +155,33 @@ template <int N> __device__ __forceinline__ void regs_release() { asm volatile("
 template <int N> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ void softmax_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }  // warps 0-7 only
 
-// A whole warp waits for the first piece of its unit (a flag in the workspace), with the limits of the other waits.
+// The clock of the wait for a first piece, given a reading of the timer at its start and then now and then. As in mbar_wait_slow the
+// limit counts from two readings, as signed differences, and here it has to be exceeded by two in a row, so that no one reading of
+// the 64-bit timer that is off ends a wait. (In mbar_wait_slow itself, which every wait of this kernel inlines, the same form cost whole
+// units 1.5 to 2 %: 1024 units of 89 tiles 505 -> 516 us.)
+struct WaitClock {
+    uint64_t t0, first = 0;
+    bool over = false;
+    __host__ __device__ explicit WaitClock(uint64_t start) : t0(start) {}
+    __host__ __device__ bool ended(uint64_t now) {
+        if (first == 0) first = now;
+        const bool late = (int64_t)(now - t0) > (int64_t)tc::kWaitLimitNs && (int64_t)(now - first) > (int64_t)tc::kWaitLimitNs, twice = late && over;
+        over = late;
+        return twice;
+    }
+};
+// A whole warp waits for the first piece of its unit (a flag in the workspace). As in mbar_wait_warp every lane polls, which also
+// orders its reads of the state behind the flag, and lane 0 alone keeps the time.
 __device__ __forceinline__ bool wait_handed(const int* flag, volatile int* abort) {
-    const uint64_t start = tc::global_timer_ns();
+    WaitClock clock(tc::global_timer_ns());
     for (uint32_t it = 0; it < tc::kSpinLimit; ++it) {
         int set;
         asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(set) : "l"(flag) : "memory");
         if (__all_sync(0xffffffffu, set != 0)) return true;
-        if ((it & 63u) == 63u &&
-            __any_sync(0xffffffffu, *abort != 0 || (int64_t)(tc::global_timer_ns() - start) > (int64_t)tc::kWaitLimitNs)) break;
+        if ((it & 63u) == 63u) {
+            const int over = (threadIdx.x & 31) == 0 && (*abort != 0 || clock.ended(tc::global_timer_ns()));
+            if (__shfl_sync(0xffffffffu, over, 0)) break;
+        }
         __nanosleep(32);
     }
     *abort = 1;
@@ -973,6 +991,14 @@ int attention_tc_handover_plan(long long units, int n_tiles, int sms, int* whole
         first[3 * i] = w.pieces[i].unit; first[3 * i + 1] = w.pieces[i].nt; first[3 * i + 2] = w.pieces[i].slot;
     }
     return RFK_OK;
+}
+
+int attention_tc_wait_clock(const unsigned long long* readings, int n) {
+    if (n <= 0 || !readings) return RFK_EINVAL;
+    tcattn::WaitClock clock(readings[0]);
+    for (int i = 1; i < n; ++i)
+        if (clock.ended(readings[i])) return i;
+    return 0;
 }
 
 namespace {

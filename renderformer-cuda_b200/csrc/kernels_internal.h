@@ -59,6 +59,9 @@ extern "C" int rfk_flash_attention_ordered(const rfk_half* Q, const rfk_half* K,
 extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, void* workspace,
                                               size_t workspace_bytes, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd,
                                               float scale, rfk_stream_t stream);
+// The clock of the attention's wait for a unit's first piece on a sequence of readings of the timer, in ns, the first at the wait's start: index of the
+// reading that ends the wait, 0 if none does; for its test, host only
+extern "C" int rfk_wait_clock(const unsigned long long* readings, int n);
 // Which units of a grid that is not cut the launcher hands over from one SM to another (plan_handover in attention_tc.cu): units
 // [0, *whole_units) stay whole, then for each of *n_handed units {unit, key tiles of its first piece, slot} in launch order.
 extern "C" int rfk_flash_attention_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed,
