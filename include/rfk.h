@@ -276,9 +276,10 @@ int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V,
  * unit last (nobody waits); of a larger grid the units of the last, partial round are, when that saves a fifth of the
  * launch. Which units are cut, and with it the order of their sums, depends on B * H and Sq. Units of any other grid of more
  * than one round may be begun by one CTA and finished by another through the workspace, in the order and with the bits of
- * whole units. workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
+ * whole units: there a CTA waits for another of its launch, for at most 50 ms, after which it computes the whole unit itself.
+ * workspace: rfk_flash_attention_workspace_bytes() bytes, 16-byte aligned, its first 1024
  * bytes zero before the first launch (the kernel leaves them zero); launches that may overlap in time need separate
- * workspaces. The result of cut units differs from whole ones' only by rounding (fp32 merge; fp16 probabilities relative to
+ * workspaces, or they mix up each other's units. The result of cut units differs from whole ones' only by rounding (fp32 merge; fp16 probabilities relative to
  * each piece's own maximum) and is bit-reproducible from launch to launch.
  * (3) Shared values (v_shared != 0): V is [H, Sk, D], one set for all B batch elements - views of one scene rendered
  * together have their own queries and (rotated) keys but the same values.

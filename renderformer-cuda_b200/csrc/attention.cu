@@ -595,6 +595,7 @@ extern std::atomic<int> g_attn_split;
 size_t attention_tc_workspace_bytes();
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces);
 int attention_tc_wait_clock(const unsigned long long* readings, int n);
+int attention_tc_handover_step(int word, int event, int* next);
 int attention_tc_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed, unsigned short* first, int max_handed);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
@@ -676,6 +677,8 @@ extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half*
     return flash_attention_ex(Q, K, V, O, nullptr, 0, 0, 0.0f, workspace, workspace_bytes, AttnCut::kNone, 0, B, H, Sq, Sk, n_keys, D,
                               o_bshd, scale, stream);
 }
+
+extern "C" int rfk_handover_step(int word, int event, int* next) { return attention_tc_handover_step(word, event, next); }
 
 extern "C" int rfk_wait_clock(const unsigned long long* readings, int n) { return attention_tc_wait_clock(readings, n); }
 

@@ -51,10 +51,11 @@
 // its last round. With a workspace every SM gets the same number of key tiles instead: some units are begun by one CTA, which leaves
 // O, running maximum and row sum as they stand in the workspace, and finished by another, which takes them up and goes on with the
 // next tile (plan_handover). That is the same sequence of operations on every row, so the bits are those of whole units, for every
-// caller. First pieces are the grid's first blocks, second pieces its last, and a first piece waits for nobody: a second piece
-// only ever waits (with the limit of the other waits) for a block that was handed out before it, and by the plan that one has been done for
-// half a round. Measured (us, whole / handed over; estimates agree within 2 %): 16 x 4096 x 5665 x 64 138 / 127, 16 x 5665 x 5665 208 / 180,
-// 448 units of 89 tiles 277 / 221, 149 of 16 33 / 24.5; 128-wide heads 184 of 89 tiles 208 / 148, 256 of 89 217 / 207. Of 137 grids of 149 to 600
+// caller. First pieces are the grid's first blocks, second pieces its last, and a first piece waits for nobody. Blocks are handed out in
+// order, and by the plan a unit's first piece has been done for half a round when its second begins; but nothing promises that order, and
+// nothing depends on it: a second piece that finds no state within 50 ms, or a first piece that failed, takes all of the unit, and a first piece
+// that comes after that leaves it to it (handover.cuh). Measured (us, whole / handed over; estimates agree within 2 %): 16 x 4096 x 5665 x 64 138 / 128, 16 x 5665 x 5665 207 / 182,
+// 448 units of 89 tiles 275 / 220, 149 of 16 32 / 26; 128-wide heads 184 of 89 tiles 181 / 143, 256 of 89 185 / 183. Of 137 grids of 149 to 600
 // units and 16 to 113 tiles none lost. It needs a gain of 5 % by the plan's estimate; 256 units of 24 tiles stay whole.
 //
 // One block per CTA. Two blocks share a CTA so that they share the K/V tiles; their softmax warps then share the SM's
@@ -68,6 +69,7 @@
 #define RFK_TC_WAIT_INLINE  // this kernel re-partitions its registers (setmaxnreg)
 #include "attention_tc.cuh"
 #include "common.cuh"
+#include "handover.cuh"
 #include "kernels_internal.h"
 
 namespace rfk {
@@ -121,7 +123,7 @@ struct __align__(8) Ctrl {
     uint64_t drain[2 * kBlocks];  // abort path only, one per issuing lane: completes once that lane's products have finished
     uint32_t tmem_base;
     int abort;
-    int merge;  // set by thread 0 of a split unit's last piece: this CTA merges the unit
+    int merge;  // set by thread 0 of a split unit's last piece: this CTA merges the unit; of a second piece: it takes up the first one's state
 };
 
 static_assert(sizeof(Ctrl) <= 512, "control block");
@@ -139,7 +141,7 @@ struct WorkList {
     int heads;        // units handed over (else 0): CTAs [0, heads) take their first pieces, pieces[0, heads); n_pieces = 2 * heads
     Piece pieces[kMaxPieces];
 };
-// Workspace: 256 counters (one per split unit, zero between launches), then per slot 256 x {m, l}, then per slot the
+// Workspace: 256 counters (one per split unit, zero between launches, also after one whose waits timed out), then per slot 256 x {m, l}, then per slot the
 // un-normalised output as [16 or 32 groups of 4 columns][256 rows] float4 (a warp's 32 rows of one group are contiguous).
 constexpr int kUnitRows = kBlocks * BM;
 constexpr size_t kWsCounterBytes = 1024;
@@ -157,35 +159,48 @@ __device__ __forceinline__ void softmax_warps_sync() { asm volatile("bar.sync 1,
 
 // The clock of the wait for a first piece, given a reading of the timer at its start and then now and then. As in mbar_wait_slow the
 // limit counts from two readings, as signed differences, and here it has to be exceeded by two in a row, so that no one reading of
-// the 64-bit timer that is off ends a wait. (In mbar_wait_slow itself, which every wait of this kernel inlines, the same form cost whole
-// units 1.5 to 2 %: 1024 units of 89 tiles 505 -> 516 us.)
+// the 64-bit timer that is off ends a wait.
+constexpr uint64_t kHandedLimitNs = 50ull * 1000 * 1000;
 struct WaitClock {
     uint64_t t0, first = 0;
     bool over = false;
     __host__ __device__ explicit WaitClock(uint64_t start) : t0(start) {}
     __host__ __device__ bool ended(uint64_t now) {
         if (first == 0) first = now;
-        const bool late = (int64_t)(now - t0) > (int64_t)tc::kWaitLimitNs && (int64_t)(now - first) > (int64_t)tc::kWaitLimitNs, twice = late && over;
+        const bool late = (int64_t)(now - t0) > (int64_t)kHandedLimitNs && (int64_t)(now - first) > (int64_t)kHandedLimitNs, twice = late && over;
         over = late;
         return twice;
     }
 };
-// A whole warp waits for the first piece of its unit (a flag in the workspace). As in mbar_wait_warp every lane polls, which also
-// orders its reads of the state behind the flag, and lane 0 alone keeps the time.
-__device__ __forceinline__ bool wait_handed(const int* flag, volatile int* abort) {
+// One step of a party on the word (handover.cuh), `seen`: what it probably is. The other party changes it once at most, and so often is
+// the exchange tried again.
+template <typename StepOf> __device__ __forceinline__ int handover_step(int* word, int seen, StepOf step_of) {
+    for (int tries = 0; tries < 8; ++tries) {
+        const handover::Step step = step_of(seen);
+        const int old = atomicCAS(word, seen, step.next);
+        if (old == seen) return step.act;
+        seen = old;
+    }
+    return handover::kWhole;
+}
+// One thread of the second piece waits for the first one. True: its state is there, and is visible to the CTA behind its next barrier.
+// False: the first piece failed, or did not come within the limit; the second one takes all of the unit.
+__device__ __forceinline__ bool wait_handed(int* word) {
+    int found;   // nearly always: the first piece has long been done, one exchange is all
+    asm volatile("atom.acquire.gpu.global.cas.b32 %0, [%1], %2, %3;"
+                 : "=r"(found) : "l"(__cvta_generic_to_global(word)), "n"((int)handover::kReady), "n"(handover::settle(handover::kReady).next) : "memory");
+    if (found == handover::kReady) return true;
     WaitClock clock(tc::global_timer_ns());
     for (uint32_t it = 0; it < tc::kSpinLimit; ++it) {
-        int set;
-        asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(set) : "l"(flag) : "memory");
-        if (__all_sync(0xffffffffu, set != 0)) return true;
-        if ((it & 63u) == 63u) {
-            const int over = (threadIdx.x & 31) == 0 && (*abort != 0 || clock.ended(tc::global_timer_ns()));
-            if (__shfl_sync(0xffffffffu, over, 0)) break;
-        }
+        int seen;
+        asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
+        if (handover::look(seen).act != handover::kWait) break;
+        if ((it & 63u) == 63u && clock.ended(tc::global_timer_ns())) break;
         __nanosleep(32);
     }
-    *abort = 1;
-    return false;
+    const int act = handover_step(word, handover::kReady, [](int w) { return handover::settle(w); });
+    __threadfence();
+    return act == handover::kGo;
 }
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
@@ -350,14 +365,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this CTA's work: a whole unit, or a piece of one (n_tiles key tiles from tile t0)
     int unit = blockIdx.x, t0 = 0, n_tiles = (n_keys + BN - 1) / BN, split_count = 1, split_first = 0, split_slot = 0;
-    bool gives = false, takes = false;  // HAND: the unit's first piece, whose state another CTA takes over; its second piece
+    const bool gives = HAND && (int)blockIdx.x < work.heads;   // the first piece of a unit, whose state another CTA takes over
+    const bool second = HAND && (int)blockIdx.x >= work.heads + work.whole_units;
+    bool takes = false;                                         // a second piece that has the first one's state
     if (HAND) {
-        const int b = blockIdx.x - work.heads;
-        gives = b < 0;
-        takes = b >= work.whole_units;
-        unit = b;
-        if (gives || takes) {
-            const Piece& pc = work.pieces[gives ? (int)blockIdx.x : b + work.heads - work.whole_units];
+        unit = blockIdx.x - work.heads;
+        if (gives || second) {
+            const Piece& pc = work.pieces[gives ? blockIdx.x : blockIdx.x - work.whole_units];
             unit = pc.unit; t0 = pc.t0; n_tiles = pc.nt; split_slot = pc.slot;
         }
     } else if ((int)blockIdx.x >= work.whole_units) {
@@ -394,6 +408,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // everything above touched only this CTA's shared and tensor memory; the operands below are another kernel's output
     pdl_wait();
     pdl_trigger();
+    if (second) {   // ahead of the roles, which then take either the rest of the unit or all of it
+        if (tid == 0) ctrl->merge = wait_handed(reinterpret_cast<int*>(ws) + split_slot);
+        __syncthreads();
+        takes = __any_sync(0xffffffffu, ctrl->merge != 0);   // the same in every lane: by a vote, so that what follows from it takes no registers a thread
+        if (!takes) { t0 = 0; n_tiles = (n_keys + BN - 1) / BN; }
+    }
 
     // The register hand-over: every warp of a warpgroup executes the same setmaxnreg instruction (warpgroups 2 and 3 the
     // release, 0 and 1 the take), as the first statement of a branch that does not meet the other again before the
@@ -580,35 +600,37 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         bool ok = true;
         int buf = 0, buf_par = 0;  // score buffer of tile j and the phase parity of its barriers
         // HAND: this row's place in the handed-over state, [16 or 32 groups of 4 columns][256 rows] float4 as above
-        uint4* const handed = reinterpret_cast<uint4*>(ws + kWsCounterBytes + kWsMlBytes) + (size_t)split_slot * (2 * HD / 4) * kUnitRows + blk * BM + r;
+        auto handed_row = [&](int slot) {
+            return reinterpret_cast<uint4*>(ws + kWsCounterBytes + kWsMlBytes) + (size_t)slot * (2 * HD / 4) * kUnitRows + blk * BM + r;
+        };
         if (HAND && takes) {  // O, the row sum and the reference where the first piece left them
-            ok = wait_handed(reinterpret_cast<const int*>(ws) + split_slot, abort_flag);
-            softmax_warps_sync();  // every softmax warp comes here, whatever its ok; all have seen the flag: ready for the next launch
-            if (tid == 0) reinterpret_cast<int*>(ws)[split_slot] = 0;
-            if (ok) {
+            const uint4* const handed = handed_row(split_slot);
 #pragma unroll
-                for (int hc = 0; hc < HD / 32; ++hc) {
+            for (int hc = 0; hc < HD / 32; ++hc) {
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 w = __ldcg(handed + (hc * 8 + c) * kUnitRows);
-                        va[4 * c] = w.x; va[4 * c + 1] = w.y; va[4 * c + 2] = w.z; va[4 * c + 3] = w.w;
-                    }
-                    tc::tmem_st32(tO + hc * 32, va);
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 w = __ldcg(handed + (hc * 8 + c) * kUnitRows);
+                    va[4 * c] = w.x; va[4 * c + 1] = w.y; va[4 * c + 2] = w.z; va[4 * c + 3] = w.w;
                 }
-                tc::tc_wait_st();
-                const uint4 l = __ldcg(handed + (HD / 4) * kUnitRows), m = __ldcg(handed + (HD / 4 + 1) * kUnitRows);
-                l_run = __uint_as_float(l.x);
-                l01 = make_float2(__uint_as_float(l.x), __uint_as_float(l.y));
-                l23 = make_float2(__uint_as_float(l.z), __uint_as_float(l.w));
-                m_run = __uint_as_float(m.x);
+                tc::tmem_st32(tO + hc * 32, va);
             }
+            tc::tc_wait_st();
+            if (C::kCorr) tc::tc_fence_before();   // the rescaling warps' from here on, by way of move_full
+            const uint4 l = __ldcg(handed + (HD / 4) * kUnitRows), m = __ldcg(handed + (HD / 4 + 1) * kUnitRows);
+            l_run = __uint_as_float(l.x);
+            l01 = make_float2(__uint_as_float(l.x), __uint_as_float(l.y));
+            l23 = make_float2(__uint_as_float(l.z), __uint_as_float(l.w));
+            m_run = __uint_as_float(m.x);
         }
-        for (int j = 0; ok && j < n_tiles; ++j) {
+        // From 1 on for a taken-over unit: tile 0 is where a unit begins. (The tile before its first counts as multiplied: a wait for the
+        // previous phase of a new barrier returns at once.)
+        const int j0 = HAND && takes ? 1 : 0, j_end = n_tiles + j0, j_key = t0 - j0;
+        for (int j = j0; ok && j < j_end; ++j) {
             const uint32_t tS = tmem + lane_off + buf * 64;
             ok = tc::mbar_wait_warp(&ctrl->s_full[blk][buf], buf_par, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
-            const int n_valid = min(BN, n_keys - (t0 + j) * BN);  // real keys among this tile's 64 columns
+            const int n_valid = min(BN, n_keys - (j_key + j) * BN);  // real keys among this tile's 64 columns
             tc::tmem_ld32(tS, va);
             tc::tc_wait_ld(va);
             tc::tmem_ld32(tS + 32, vb);  // in flight during the first half's arithmetic
@@ -628,7 +650,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // tile) the scores are read again, the maximum is taken and the same code runs once more.
             float2 acc0, acc1;
             float m_new = m_run, alpha = 1.0f;
-            bool any_move = false, need_max = kExactMax || (j == 0 && !(HAND && takes)) || n_valid != BN;
+            bool any_move = false, need_max = kExactMax || j == 0 || n_valid != BN;
 #pragma unroll 1
             for (;;) {
                 acc0 = make_float2(0.0f, 0.0f);
@@ -650,8 +672,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     any_move = __any_sync(kFull, move);
                     if (any_move && move) alpha = fast_exp2((m_run - m_new) * scale_log2e);  // first tile: 0
                     if (C::kCorr) {  // the first tile's product overwrites O, unless it was taken over
-                        factors[(blk * kSBufs + buf) * BM + r] = j > 0 || (HAND && takes) ? alpha : 1.0f;
-                        if (HAND && j == 0) tc::tc_fence_before();   // a taken-over O has been stored by this warp
+                        factors[(blk * kSBufs + buf) * BM + r] = j > 0 ? alpha : 1.0f;
                         __syncwarp();
                         if (lane == 0) tc::mbar_arrive(&ctrl->move_full[blk][buf]);
                     }
@@ -671,15 +692,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_wait_ld(va);
                 tc::tmem_ld32(tS + 32, vb);
             }
-            if (!C::kCorr && (j > 0 || (HAND && takes)) && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
+            if (!C::kCorr && j > 0 && any_move) {  // rescale this warp's 32 rows of O (vb is free here)
                 // O belongs to the tensor core until the previous tile's P V is done. Having seen s_full of tile j,
                 // P V of tile j - 1 - kSBufs (the previous phase of this barrier) is known complete: the parity is unambiguous.
-                if (!HAND || j > 0) {  // ahead of its first tile a taken-over O is this warp's own
-                    const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
-                    ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
-                    if (!ok) break;
-                    tc::tc_fence_after();
-                }
+                const int pbuf = buf == 0 ? kSBufs - 1 : buf - 1, pbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;  // of tile j - 1
+                ok = tc::mbar_wait_warp(&ctrl->pv_done[blk][pbuf], pbuf_par, abort_flag);
+                if (!ok) break;
+                tc::tc_fence_after();
 #pragma unroll
                 for (int hc = 0; hc < HD / 32; ++hc) {
                     tc::tmem_ld32(tO + hc * 32, vb);
@@ -704,7 +723,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (lane == 0) tc::mbar_arrive(&ctrl->p_full[blk][buf]);
             if (++buf == kSBufs) { buf = 0; buf_par ^= 1; }
         }
-        if (ORDERED && !(HAND && gives)) l_run = (l01.x + l01.y) + (l23.x + l23.y);
+        if (ORDERED && !gives) l_run = (l01.x + l01.y) + (l23.x + l23.y);
         // ---- epilogue: O / l -> fp16 -> global, one 128-byte row per thread
         if (ok) {  // buf / buf_par have moved on to tile n_tiles: step back to the last tile
             const int lbuf = buf == 0 ? kSBufs - 1 : buf - 1, lbuf_par = buf == 0 ? buf_par ^ 1 : buf_par;
@@ -712,9 +731,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         const int q = q0 + blk * BM + r;
         __half* dst = o_bshd ? O + (((size_t)(bh / H) * Sq + q) * H + bh % H) * HD : O + ((size_t)bh * Sq + q) * HD;
-        if (HAND && gives) {
-            // ---- first piece of a unit that is handed over: O, row sum and reference as they stand, then the flag
+        if (gives) {
+            // ---- first piece of a unit that is handed over: O, row sum and reference as they stand
             if (ok) {
+                uint4* const handed = handed_row(work.pieces[blockIdx.x].slot);
                 tc::tc_fence_after();
 #pragma unroll
                 for (int hc = 0; hc < HD / 32; ++hc) {
@@ -730,8 +750,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 __stcg(handed + (HD / 4 + 1) * kUnitRows, make_uint4(__float_as_uint(m_run), 0, 0, 0));
                 __threadfence();
             }
-            softmax_warps_sync();  // every softmax warp comes here, whatever its ok
-            if (tid == 0 && !*abort_flag) asm volatile("st.release.gpu.b32 [%0], 1;" ::"l"(reinterpret_cast<int*>(ws) + split_slot) : "memory");
         } else if (BLOCKS == 1 || HAND || split_count == 1) {
             if (ok) {
                 tc::tc_fence_after();
@@ -819,6 +837,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (warp == 0) {
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem_cta, kTmemCols);
+    }
+    if (gives && tid == 32) {   // every softmax warp has written its rows of the state, or given up
+        const bool left = *abort_flag == 0;
+        __threadfence();
+        handover_step(reinterpret_cast<int*>(ws) + split_slot, handover::kIdle, [left](int w) { return handover::give(w, left); });
     }
     if (tid == 0 && ctrl->abort) atomicCAS(&g_attn_tc_error, 0, kErrTimeout);
 }
@@ -999,6 +1022,14 @@ int attention_tc_wait_clock(const unsigned long long* readings, int n) {
     for (int i = 1; i < n; ++i)
         if (clock.ended(readings[i])) return i;
     return 0;
+}
+
+int attention_tc_handover_step(int word, int event, int* next) {
+    if (!next || word < 0 || word > handover::kTaken) return RFK_EINVAL;
+    const handover::Step s = event == 0 ? handover::give(word, true) : event == 1 ? handover::give(word, false)
+                             : event == 2 ? handover::look(word) : handover::settle(word);
+    *next = s.next;
+    return s.act;
 }
 
 namespace {

@@ -1,0 +1,32 @@
+// The word through which the two pieces of a handed-over attention unit agree: who does what, and that it is zero again for the next
+// launch whatever becomes of either. Every transition is one atomic step on the word; the steps are plain functions, which the
+// host's test runs in every order.
+#pragma once
+
+namespace rfk {
+namespace handover {
+
+enum Word : int {
+    kIdle = 0,    // before the first piece is done, and once both pieces are done with the word
+    kReady = 1,   // the first piece has left its state
+    kFailed = 2,  // the first piece gave up: there is no state
+    kTaken = 3,   // the second piece has taken all of the unit; the first piece, when it is done, clears the word
+};
+enum Act : int {
+    kGo = 0,      // the second piece takes up the state
+    kWait = 1,    // it goes on waiting
+    kWhole = 2,   // it takes all of the unit
+};
+struct Step { int next, act; };   // what the word becomes, and what the party does
+
+// the first piece is done: `ok` with its state in the workspace
+__host__ __device__ constexpr Step give(int word, bool ok) { return {word == kTaken ? kIdle : ok ? kReady : kFailed, kGo}; }
+// the second piece looks whether its wait is over, and does not change the word
+__host__ __device__ constexpr Step look(int word) { return {word, word == kReady ? kGo : word == kIdle ? kWait : kWhole}; }
+// the second piece is past its wait: it has seen the first piece done, or has run out of time
+__host__ __device__ constexpr Step settle(int word) {
+    return word == kReady ? Step{kIdle, kGo} : Step{word == kFailed ? kIdle : kTaken, kWhole};
+}
+
+}  // namespace handover
+}  // namespace rfk

@@ -62,6 +62,9 @@ extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half*
 // The clock of the attention's wait for a unit's first piece on a sequence of readings of the timer, in ns, the first at the wait's start: index of the
 // reading that ends the wait, 0 if none does; for its test, host only
 extern "C" int rfk_wait_clock(const unsigned long long* readings, int n);
+// One step on the word of a handed-over unit (handover.cuh), for its test, host only: event 0 / 1 the first piece is done / gave up,
+// 2 the second piece looks, 3 it is past its wait. Returns what that piece does next (handover::Act), *next the word.
+extern "C" int rfk_handover_step(int word, int event, int* next);
 // Which units of a grid that is not cut the launcher hands over from one SM to another (plan_handover in attention_tc.cu): units
 // [0, *whole_units) stay whole, then for each of *n_handed units {unit, key tiles of its first piece, slot} in launch order.
 extern "C" int rfk_flash_attention_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed,

@@ -99,3 +99,24 @@ def test_handed_over_units_with_row_statistics_and_shared_values():
         outs.append(torch.full_like(Q, 7.0))
         _call("split", Q, K, V, outs[-1], B, Hh, Sq, Sk, Sk, D, ws, ss=ss, tiles=4, dim=Hh * D, v_shared=True)
     assert torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0].float()).all()
+
+
+@pytest.mark.parametrize("form,D,B,Hh,Sq,Sk", [("split", 64, 1, 50, 700, 1024), ("ordered", 128, 1, 38, 1000, 1536)])
+def test_a_second_piece_without_a_state_takes_the_unit(form, D, B, Hh, Sq, Sk):
+    """The first pieces find that their units have been taken (3) and leave no state, so that each second piece runs into the limit of its
+    wait, 50 ms, and computes all of its unit: the same bits, and no error."""
+    handed, cut = _handed(B * Hh * -(-Sq // 256), -(-Sk // 64))
+    assert handed > 0 and (form == "ordered" or cut == 0)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    Q, K, V = (torch.randn(B, Hh, n, D, device="cuda", generator=g).half() for n in (Sq, Sk, Sk))
+    ws, outs = pkg.ops.flash_attention_workspace(), []
+    for taken in (False, True):
+        ws[:1024].view(torch.int32)[:handed] = 3 if taken else 0
+        outs.append(torch.full_like(Q, 7.0))
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        _call(form, Q, K, V, outs[-1], B, Hh, Sq, Sk, Sk, D, ws)
+        end.record()
+        end.synchronize()
+        assert (start.elapsed_time(end) > 40) == taken
+    assert torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0].float()).all()
