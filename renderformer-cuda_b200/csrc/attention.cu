@@ -596,6 +596,7 @@ size_t attention_tc_workspace_bytes();
 int attention_tc_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_pieces, unsigned short* pieces, int max_pieces);
 int attention_tc_wait_clock(const unsigned long long* readings, int n);
 int attention_tc_handover_step(int word, int event, int* next);
+int attention_tc_arrive(int* counter, int failed, int pieces);
 int attention_tc_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed, unsigned short* first, int max_handed);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
@@ -679,6 +680,8 @@ extern "C" int rfk_flash_attention_ordered_ws(const rfk_half* Q, const rfk_half*
 }
 
 extern "C" int rfk_handover_step(int word, int event, int* next) { return attention_tc_handover_step(word, event, next); }
+
+extern "C" int rfk_piece_arrives(int* counter, int failed, int pieces) { return attention_tc_arrive(counter, failed, pieces); }
 
 extern "C" int rfk_wait_clock(const unsigned long long* readings, int n) { return attention_tc_wait_clock(readings, n); }
 

@@ -783,16 +783,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             softmax_warps_sync();  // every softmax warp comes here, whatever its ok: the barrier cannot be left short
             if (tid == 0) {
-                int merge = 0;
-                if (!*abort_flag) {
-                    int* counter = reinterpret_cast<int*>(ws) + (unit - work.whole_units);
-                    merge = atomicAdd(counter, 1) == split_count - 1;
-                    if (merge) {
-                        *counter = 0;  // every piece of the unit has arrived: ready for the next launch
-                        __threadfence();
-                    }
+                int* counter = reinterpret_cast<int*>(ws) + (unit - work.whole_units);
+                const bool failed = *abort_flag != 0;
+                const handover::Arrival a = handover::arrive(atomicAdd(counter, handover::piece(failed)), failed, split_count);
+                if (a.last) {
+                    *counter = 0;  // every piece of the unit has arrived, or given up: ready for the next launch
+                    __threadfence();
                 }
-                ctrl->merge = merge;
+                ctrl->merge = a.merge;
             }
             softmax_warps_sync();
             if (ctrl->merge && ok) {
@@ -1022,6 +1020,13 @@ int attention_tc_wait_clock(const unsigned long long* readings, int n) {
     for (int i = 1; i < n; ++i)
         if (clock.ended(readings[i])) return i;
     return 0;
+}
+
+int attention_tc_arrive(int* counter, int failed, int pieces) {
+    if (!counter || pieces <= 0) return RFK_EINVAL;
+    const handover::Arrival a = handover::arrive(*counter, failed != 0, pieces);
+    *counter = a.last ? 0 : *counter + handover::piece(failed != 0);
+    return a.merge;
 }
 
 int attention_tc_handover_step(int word, int event, int* next) {

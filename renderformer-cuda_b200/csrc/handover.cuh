@@ -1,5 +1,5 @@
-// The word through which the two pieces of a handed-over attention unit agree: who does what, and that it is zero again for the next
-// launch whatever becomes of either. Every transition is one atomic step on the word; the steps are plain functions, which the
+// The words of the attention's workspace: through one the two pieces of a handed-over unit agree who does what, through another the pieces
+// of a cut unit which of them merges it; and each is zero again for the next launch whatever becomes of a piece. Every transition is one atomic step on the word; the steps are plain functions, which the
 // host's test runs in every order.
 #pragma once
 
@@ -26,6 +26,15 @@ __host__ __device__ constexpr Step look(int word) { return {word, word == kReady
 // the second piece is past its wait: it has seen the first piece done, or has run out of time
 __host__ __device__ constexpr Step settle(int word) {
     return word == kReady ? Step{kIdle, kGo} : Step{word == kFailed ? kIdle : kTaken, kWhole};
+}
+
+// Units whose keys are cut into pieces that nobody waits for: a counter of the pieces that have arrived, in the upper half of those that
+// gave up. The last one zeroes it for the next launch, and merges the pieces if all have left their shares.
+__host__ __device__ constexpr int piece(bool failed) { return failed ? 0x10001 : 1; }   // what a piece adds
+struct Arrival { bool last, merge; };
+__host__ __device__ constexpr Arrival arrive(int before, bool failed, int pieces) {
+    const bool last = (before & 0xffff) == pieces - 1;
+    return {last, last && !failed && before < 0x10000};
 }
 
 }  // namespace handover

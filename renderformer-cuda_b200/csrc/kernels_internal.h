@@ -65,6 +65,8 @@ extern "C" int rfk_wait_clock(const unsigned long long* readings, int n);
 // One step on the word of a handed-over unit (handover.cuh), for its test, host only: event 0 / 1 the first piece is done / gave up,
 // 2 the second piece looks, 3 it is past its wait. Returns what that piece does next (handover::Act), *next the word.
 extern "C" int rfk_handover_step(int word, int event, int* next);
+// A piece of a unit cut into `pieces` arrives at its counter, for its test, host only: 1 if it merges the unit.
+extern "C" int rfk_piece_arrives(int* counter, int failed, int pieces);
 // Which units of a grid that is not cut the launcher hands over from one SM to another (plan_handover in attention_tc.cu): units
 // [0, *whole_units) stay whole, then for each of *n_handed units {unit, key tiles of its first piece, slot} in launch order.
 extern "C" int rfk_flash_attention_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed,

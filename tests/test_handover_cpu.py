@@ -47,3 +47,16 @@ def test_every_order_of_the_steps(first, patience, late_step):
 def test_bad_arguments():
     step = _abi.load("rfk.h").rfk_handover_step
     assert step(0, LOOK, None) == -1 and step(99, LOOK, ctypes.byref(ctypes.c_int())) == -1
+
+
+@pytest.mark.parametrize("pieces", range(1, 9))
+def test_the_counter_of_a_cut_unit_is_zero_after_its_last_piece(pieces):
+    """Whichever pieces give up, in whichever places: the counter is zero behind the last, and a unit is merged once if all arrived."""
+    arrives = _abi.load("rfk.h").rfk_piece_arrives
+    for failures in range(2 ** pieces):
+        counter, merges = ctypes.c_int(0), []
+        for i in range(pieces):
+            assert counter.value != 0 or i == 0
+            merges.append(arrives(ctypes.byref(counter), failures >> i & 1, pieces))
+        assert counter.value == 0
+        assert merges == [0] * (pieces - 1) + [int(failures == 0)]
