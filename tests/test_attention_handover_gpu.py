@@ -120,3 +120,25 @@ def test_a_second_piece_without_a_state_takes_the_unit(form, D, B, Hh, Sq, Sk):
         end.synchronize()
         assert (start.elapsed_time(end) > 40) == taken
     assert torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0].float()).all()
+
+
+def test_two_launches_in_flight_on_two_streams():
+    """Handed-over launches of two streams share the SMs, each with a workspace of its own: the bits of each alone, time after time."""
+    B, Hh, Sq, Sk, D = 1, 50, 700, 1024, 64          # 150 units of 16 tiles
+    assert _handed(150, 16)[0] > 0 and _handed(150, 16)[1] == 0
+    g = torch.Generator(device="cuda").manual_seed(11)
+    sides = []
+    for _ in range(2):
+        q, k, v = (torch.randn(B, Hh, n, D, device="cuda", generator=g).half() for n in (Sq, Sk, Sk))
+        want = torch.empty_like(q)
+        ws = pkg.ops.flash_attention_workspace()
+        _call("split", q, k, v, want, B, Hh, Sq, Sk, Sk, D, ws)
+        sides.append((q, k, v, want, ws, torch.cuda.Stream(), [torch.full_like(q, 7.0) for _ in range(20)]))
+    torch.cuda.synchronize()
+    for i in range(20):
+        for q, k, v, _, ws, stream, outs in sides:
+            with torch.cuda.stream(stream):
+                _call("split", q, k, v, outs[i], B, Hh, Sq, Sk, Sk, D, ws)
+    torch.cuda.synchronize()
+    for _, _, _, want, ws, _, outs in sides:
+        assert all(torch.equal(o, want) for o in outs) and not ws[:1024].any()

@@ -171,3 +171,35 @@ def test_embedding_norms_and_sum_have_the_bits_of_the_separate_steps(rows, dim):
     assert fn(*(VP(t.data_ptr()) for t in (a, ga, b, gb, c, got)), rows, dim, ops.K_EPS_FP16,
               VP(torch.cuda.current_stream().cuda_stream)) == 0
     assert torch.equal(got, want)
+
+
+# on CTA pairs with tiles of 192 columns: 1.2 and 1.9 rounds of 74 pairs, and less than one, with rows that fill neither a tile nor a store box
+@pytest.mark.parametrize("Sk,heads,hd,pad", [(5665, 8, 128, 5672), (5665, 16, 64, 5672), (2501, 8, 128, 2504), (2501, 8, 128, 2600), (4100, 8, 64, 4104)])
+def test_cache_of_large_scenes_has_the_bits_of_the_separate_epilogue(Sk, heads, hd, pad):
+    """K and V stored head-split by their projections, K normalised in place, against the plain projections and their epilogue kernel, which
+    projections with a bias (here of zeros) take."""
+    import ctypes
+    from renderformer_cuda_b200 import _abi, session
+    L, VP = _abi.load("rfk_layers.h"), ctypes.c_void_p
+    dim = heads * hd
+    g = torch.Generator(device="cuda").manual_seed(Sk + hd)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, wk, wv = rnd(Sk, dim).half(), (rnd(dim, dim) / dim ** 0.5).half(), (rnd(dim, dim) / dim ** 0.5).half()
+    zero = torch.zeros(dim, device="cuda", dtype=torch.float16)
+    model = session.Model.random(seed=1, dim=dim, num_heads=heads, ffn_hidden=256, enc_layers=0, dec_layers=1)
+    w = model.decoder_record(0).cross_attn
+    w.k_proj_w, w.v_proj_w = wk.data_ptr(), wv.data_ptr()
+    ctx, outs = session.Ctx(), []
+    for bias in (None, zero):
+        w.k_proj_b = w.v_proj_b = None if bias is None else bias.data_ptr()
+        K, V = (torch.full((heads, pad, hd), 7.0, device="cuda", dtype=torch.float16) for _ in range(2))
+        proj = torch.full((2 * Sk, dim), 7.0, device="cuda", dtype=torch.float16)
+        rc = L.rfk_precompute_cross_kv(ctx.h, ctypes.byref(w), VP(x.data_ptr()), VP(K.data_ptr()), VP(V.data_ptr()), VP(proj.data_ptr()),
+                                       1, Sk, pad, dim, dim, heads, VP(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, rc
+        torch.cuda.synchronize()
+        outs.append((K, V, bool((proj != 7.0).any())))
+    assert not outs[0][2] and outs[1][2]                # one route each
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert (outs[0][0][:, Sk:] == 0).all() and torch.isfinite(outs[0][0].float()).all() and (outs[0][0][:, :Sk] != 0).any(-1).all()
+    ctx.close()
