@@ -272,6 +272,7 @@ extern "C" int rfk_precompute_cross_kv(rfk_ctx* ctx, const rfk_cross_attn_weight
     const int Mk = B * Sk, hd = dim / num_heads;
     rfk_half* Kp = proj_buf;
     rfk_half* Vp = proj_buf + (size_t)Mk * dim;
+    TRY(rfk_linear(ctx, ctx_normed, w->k_proj_w, w->k_proj_b, Kp, Mk, dim, kv_dim, stream));
     if (Sk_pad != Sk) {
         // only the rows behind the last key of each head; every other element is written below
         const size_t pitch = (size_t)Sk_pad * hd * 2, width = (size_t)(Sk_pad - Sk) * hd * 2, heads = (size_t)B * num_heads;
@@ -282,25 +283,14 @@ extern "C" int rfk_precompute_cross_kv(rfk_ctx* ctx, const rfk_cross_attn_weight
     const float* g[1] = {w->k_norm_gamma};
     rfk_half* o[1] = {K_out};
     const int no_rope[1] = {0};
-    // One batch element: K is stored head-split by its projection and normalised in place (5665 rows: 6.2 us
-    // for the transposing norm's 8)
-    int rc = RFK_EUNSUPPORTED;
-    if (B == 1 && !w->k_proj_b && w->k_norm_gamma && (hd == 64 || hd == 128) && dim <= 2048 &&
-        (reinterpret_cast<uintptr_t>(w->k_norm_gamma) & 15u) == 0)
-        rc = rfk::gemm_heads(ctx_normed, kv_dim, w->k_proj_w, kv_dim, K_out, 0, nullptr, 0, Mk, dim, kv_dim, Sk, Sk_pad, num_heads, hd, stream);
-    if (rc == RFK_OK) {
-        TRY(rfk::qk_norm_rope_heads(1, g, o, nullptr, nullptr, Sk, Sk_pad, num_heads, hd, kEpsFp16, stream));
-    } else if (rc == RFK_EUNSUPPORTED) {
-        TRY(rfk_linear(ctx, ctx_normed, w->k_proj_w, w->k_proj_b, Kp, Mk, dim, kv_dim, stream));
-        // K and V cannot share a launch: they live in two separate [Mk, dim] projections
-        TRY(project_epilogue(Kp, dim, 1, g, o, no_rope, nullptr, nullptr, B, Sk, num_heads, hd, Sk_pad,
-                             nullptr, stream));
-    } else {
-        return rc;
-    }
+    // K and V cannot share a launch: they live in two separate [Mk, dim] projections. (K head-split by its projection and normalised in place, as
+    // the encoder's q and k are, was no faster for large scenes and slower for most: us, transposing norm / in place, 16 heads of 64: 33 rows 5.5 / 5.8, 600 rows
+    // 7.4 / 6.9, 1100 rows 8.2 / 9.5, 3300 rows 14.0 / 14.9, 5665 rows 19.0 / 19.0; the head-split store costs its product what the norm gains.)
+    TRY(project_epilogue(Kp, dim, 1, g, o, no_rope, nullptr, nullptr, B, Sk, num_heads, hd, Sk_pad,
+                         nullptr, stream));
     // V has no norm: its projection is stored head-split by the GEMM when the shape allows (one batch element, no bias); a
     // transposing pass less per layer (scene of 300 triangles 983 -> 965 us, of 1500 triangles 1650 -> 1628 us)
-    rc = RFK_EUNSUPPORTED;
+    int rc = RFK_EUNSUPPORTED;
     if (B == 1 && !w->v_proj_b && (hd == 64 || hd == 128))
         rc = rfk::gemm_heads(ctx_normed, kv_dim, w->v_proj_w, kv_dim, V_out, 0, nullptr, 0, Mk, dim, kv_dim, Sk, Sk_pad, num_heads, hd,
                              stream);

@@ -380,16 +380,16 @@ qkv_epilogue_kernel(const __half* __restrict__ x, long long row_stride,
     }
 }
 
-// The HEADS form for NP parts (q and k, or k alone) that all have a norm, rows of 32 * WPR rotation-pair chunks: a thread keeps its chunk of
+// The HEADS form for q and k that both have a norm, rows of 32 * WPR rotation-pair chunks: a thread keeps its chunk of
 // every part over all of its rows, so that the norm weights are read once, the rotation tables once for both parts, and the next
 // row's loads are in flight while a row is summed. Bound by L2 and that latency: as many CTAs as are resident at once (160
 // registers: three an SM) are the best; us for 5665 rows of q and k, 16 heads of 64: one row a block and part 14.3, two CTAs an SM 13.9,
 // three 10.1, four 12.3 (a second, partial round), eight 11.4; held to 128 registers four 12.6. Same arithmetic, same bits.
-template <int WPR, int NP>
+template <int WPR>
 __global__ void __launch_bounds__(128)
 qk_rows_kernel(const __grid_constant__ QkvParts parts, const __half* __restrict__ cos_vals, const __half* __restrict__ sin_vals,
                int seq_len, int out_seq, int num_heads, int head_dim, float eps) {
-    constexpr int RPC = 4 / WPR;  // rows per CTA at a time
+    constexpr int RPC = 4 / WPR, NP = 2;  // rows per CTA at a time; parts
     __shared__ float s_part[2][NP][4];
     pdl_wait();
     pdl_trigger();
@@ -501,14 +501,11 @@ int rfk::qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* co
     if (cos_vals && (!sin_vals || !aligned16(cos_vals) || !aligned16(sin_vals))) return RFK_EINVAL;
     if (seq_len == 0) return RFK_OK;
     const int npairs = (int)(dim / 16);
-    if (n_parts <= 2 && gamma[0] && (n_parts == 1 || gamma[1]) && (npairs == 32 || npairs == 64)) {   // wider rows are summed two chunks a thread
+    if (n_parts == 2 && gamma[0] && gamma[1] && (npairs == 32 || npairs == 64)) {   // wider rows are summed two chunks a thread
         const int wpr = npairs / 32;
-        const long long resident = (long long)kNumSMs * (n_parts == 2 ? 3 : 4);   // 160 and 116 registers a thread   // 160 and 116 registers a thread
-        const unsigned grid = (unsigned)std::min<long long>(ceil_div(seq_len, 4 / wpr), resident);
-        const auto kernel = n_parts == 2 ? (wpr == 1 ? qk_rows_kernel<1, 2> : qk_rows_kernel<2, 2>)
-                                         : (wpr == 1 ? qk_rows_kernel<1, 1> : qk_rows_kernel<2, 1>);
-        launch_pdl(kernel, dim3(grid), dim3(128), 0, as_stream(stream), parts, (const __half*)cos_vals, (const __half*)sin_vals, seq_len,
-                   out_seq, num_heads, head_dim, eps);
+        const unsigned grid = std::min(ceil_div(seq_len, 4 / wpr), 3u * kNumSMs);   // 160 registers a thread
+        launch_pdl(wpr == 1 ? qk_rows_kernel<1> : qk_rows_kernel<2>, dim3(grid), dim3(128), 0, as_stream(stream), parts, (const __half*)cos_vals,
+                   (const __half*)sin_vals, seq_len, out_seq, num_heads, head_dim, eps);
         return launch_status();
     }
 #define RFK_QK_HEADS(N, W)                                                                                   \

@@ -176,8 +176,8 @@ def test_embedding_norms_and_sum_have_the_bits_of_the_separate_steps(rows, dim):
 # on CTA pairs with tiles of 192 columns: 1.2 and 1.9 rounds of 74 pairs, and less than one, with rows that fill neither a tile nor a store box
 @pytest.mark.parametrize("Sk,heads,hd,pad", [(5665, 8, 128, 5672), (5665, 16, 64, 5672), (2501, 8, 128, 2504), (2501, 8, 128, 2600), (4100, 8, 64, 4104)])
 def test_cache_of_large_scenes_has_the_bits_of_the_separate_epilogue(Sk, heads, hd, pad):
-    """K and V stored head-split by their projections, K normalised in place, against the plain projections and their epilogue kernel, which
-    projections with a bias (here of zeros) take."""
+    """V stored head-split by its projection against the plain projection and its epilogue kernel, which a projection with a bias (here of
+    zeros) takes; K's norm with and without one."""
     import ctypes
     from renderformer_cuda_b200 import _abi, session
     L, VP = _abi.load("rfk_layers.h"), ctypes.c_void_p
@@ -198,8 +198,8 @@ def test_cache_of_large_scenes_has_the_bits_of_the_separate_epilogue(Sk, heads, 
                                        1, Sk, pad, dim, dim, heads, VP(torch.cuda.current_stream().cuda_stream))
         assert rc == 0, rc
         torch.cuda.synchronize()
-        outs.append((K, V, bool((proj != 7.0).any())))
-    assert not outs[0][2] and outs[1][2]                # one route each
+        outs.append((K, V, bool((proj[Sk:] != 7.0).any())))
+    assert not outs[0][2] and outs[1][2]                # V's two routes
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     assert (outs[0][0][:, Sk:] == 0).all() and torch.isfinite(outs[0][0].float()).all() and (outs[0][0][:, :Sk] != 0).any(-1).all()
     ctx.close()
