@@ -80,7 +80,7 @@ namespace tcattn {
 
 constexpr int BM = 128, BN = 64;
 constexpr int kBlocks = 2;                     // 128-query blocks per CTA, sharing the K/V ring (at most; see "One block per CTA")
-constexpr int kThreads = 512;                  // warps 0-7 softmax (block = warp / 4), 8 producer, 9-10 PV, 11-12 QK issuers, 13-15 none
+constexpr int kThreads = 512;                  // warps 0-7 softmax (block = warp / 4), 8 producer, 9-10 PV, 11-12 QK issuers, 13-15 none (128-wide heads: see Cfg)
 // Registers (64-wide heads): the CTA starts with 128 per thread. The two warpgroups that only issue copies and products (warps 8-15)
 // hand theirs back down to kRegsIssue and the softmax warpgroups (warps 0-7) grow to kRegsSoftmax, which lets the
 // compiler keep both halves of a score tile and their exponentials in flight without reusing registers early

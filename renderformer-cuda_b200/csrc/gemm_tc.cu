@@ -333,8 +333,7 @@ namespace pair { using namespace pair_ptx; }
 // as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
 // must equal the views one by one).
 //   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing lane and the producer's are
-//   elected ones (elect.sync), so that descriptors, coordinates and counters live in uniform registers; inside `if (lane == 0)`
-//   each operand is moved there first. With one block per stage and lane 0's loops a K block took 0.30 us on every tile size, the cost
+//   elected ones (elect.sync). With one block per stage and lane 0's loops a K block took 0.30 us on every tile size, the cost
 //   of issuing and not of the operands; two blocks and elected lanes in loops of whole warps took the 64 x 32 tile to 0.12 us, loops of
 //   the elected lanes alone, the others waiting at the warp's barrier, to 0.10 (us, whole warps / lanes alone, weights in L2: 256 x 1024 x
 //   4096 9.63 / 8.23, 256 x 1024 x 1024 3.90 / 3.62, 576 x 1024 x 4096 11.1 / 9.3; 128 x 64 tiles 1024 x 1024 x 4096 12.45 / 12.18; the
@@ -642,22 +641,22 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 }  // namespace small
 
 // ------------------------------------------------------------------------------------------------
-// The same product on CTA pairs: a cluster of two CTAs (two SMs of one TPC) owns a tile of 256 rows x 256
+// The same product on CTA pairs: a cluster of two CTAs (two SMs of one TPC) owns a tile of 256 rows x 256 [or 192, narrow_tile]
 // accumulator columns and one thread of the pair's first CTA issues tcgen05.mma.cta_group::2 (M = 256):
-// each CTA stages only ITS 128 rows of A and ITS half of the weight tile (128 of the 256 accumulator
+// each CTA stages only ITS 128 rows of A and ITS half of the weight tile (128 of the 256 [96 of the 192] accumulator
 // columns' rows; with the SwiGLU epilogue CTA 0 holds the gate rows and CTA 1 the up rows), so a K block
-// costs each SM 32 KB of L2 -> shared-memory traffic instead of 48 KB for the same number of products.
+// costs each SM 32 KB [28] of L2 -> shared-memory traffic instead of 48 KB for the same number of products.
 // That traffic, not the tensor pipe, bounds the single-CTA kernel above (the same ~510 ns per K block on
 // every shape = 14 TB/s over 148 SMs). Both accumulator halves live in the two CTAs' tensor memories at the
 // same address; each CTA's epilogue warps drain their own 128 rows.
-//   barriers: full[s] in CTA 0 collects both CTAs' copies (one arrive.expect_tx of 64 KB by CTA 0); empty[s] and
+//   barriers: full[s] in CTA 0 collects both CTAs' copies (one arrive.expect_tx of 64 KB [56] by CTA 0); empty[s] and
 //   acc_full[a] exist in both CTAs and are signalled together by one multicast tcgen05.commit;
 //   acc_empty[a] in CTA 0 counts the 8 epilogue warps of the pair.
 // The copies are ordinary per-CTA TMA loads (no cluster multicast), with the .cta_group::2 form that lets
 // CTA 1's copies count on CTA 0's barrier.
 namespace pair {
 
-constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA
+constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA, of which a tile of 192 columns leaves 4 free
 // The epilogue goes through shared memory both ways: an epilogue warp owns staging buffers of 32 rows x 64 halves
 // (4 KB, the 128-byte-swizzled layout of a TMA box) for its 32 rows of the tile; it writes the finished fp16 values
 // of 64 output columns there and one lane issues a TMA tile store, so the global writes are whole 128-byte lines
@@ -907,8 +906,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ issuer of the pair's products (an elected lane of CTA 0)
-        // elect.sync keeps descriptors and counters in uniform registers: a K block takes 543 clocks instead of 598 (the tensor pipe's
-        // own time: 512). A loop of the whole warp that issues under the same predicate needs 548, but the epilogue that
+        // Under elect.sync a K block takes 543 clocks, inside `if (lane == 0)` 598 (the tensor pipe's own time: 512). A loop of the whole warp that issues under the same predicate needs 548, but the epilogue that
         // followed it took twice as long (4137 clocks for 2086), for a reason that its code does not show.
         // us, lane 0 / elected lane: 4096 x 1024 x 4096 + residual 27.9 / 26.4, w1|w3 + SwiGLU 48.1 / 46.1, 3072 x 1024 20.5 / 20.2.
         if (rank == 0 && tc::elect_one()) {
@@ -978,7 +976,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tc::tc_fence_before();
             __syncwarp();
             // Nobody waits for the last accumulator: the teardown's cluster barrier instead, under the stores' last reads (4096 x 1024 x 1024
-            // 9.9 -> 9.65 us; the arrival's release for the cluster is what cost).
+            // 9.9 -> 9.65 us).
             if (last) {
                 cluster_arrive();
                 left = true;
