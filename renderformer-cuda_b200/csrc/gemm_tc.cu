@@ -915,11 +915,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             bool ok = true;
             for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
                 const int acc = tl & 1;
-                if (tl >= 2) {
-                    ok = wait(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1);
-                    if (!ok) break;
-                    acquire_remote(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1);
-                }
+                if (tl >= 2) ok = wait_remote(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1, abort_flag);
+                if (!ok) break;
                 tc::tc_fence_after();
                 const uint32_t d_tmem = tmem_cta + acc * BNACC;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {

@@ -23,15 +23,29 @@ __device__ __forceinline__ void cluster_sync() {
 // its two halves, for work between them; every thread of both CTAs makes each once, whole warps together
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// An arrival on a barrier of the pair's other CTA, and the waiting side's acquire of such arrivals (of a phase that has been waited for and
-// cannot be followed by another yet). Both name the cluster: the default scope is the CTA, which orders nothing between the
-// accumulator reads of one CTA's threads and the products that the other issues into it next.
+// An arrival on a barrier of the pair's other CTA, and the waiting side's poll for such arrivals. Both name the cluster: the default scope is
+// the CTA, which orders nothing between the accumulator reads of one CTA's threads and the products that the other issues into it next.
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-__device__ __forceinline__ void acquire_remote(uint64_t* bar, uint32_t parity) {
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
-                 ::"r"(tc::smem_addr(bar)), "r"(parity) : "memory");
+__device__ __forceinline__ bool poll_remote(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(tc::smem_addr(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits of one thread and of a whole warp for a phase that other CTAs' threads arrive for and that no other can follow yet: nearly always
+// over, so that one poll is all; behind a wait of the CTA's scope a last poll acquires for the cluster.
+__device__ __forceinline__ bool wait_remote(uint64_t* bar, uint32_t parity, volatile int* abort) {
+    if (poll_remote(bar, parity)) return true;
+    return tc::mbar_wait_slow(bar, parity, abort) && poll_remote(bar, parity);
+}
+__device__ __forceinline__ bool wait_remote_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
+    if (__all_sync(0xffffffffu, poll_remote(bar, parity))) return true;
+    return tc::mbar_wait_warp(bar, parity, abort) && __all_sync(0xffffffffu, poll_remote(bar, parity));
 }
 
 // ---- shared <-> global tile copies
