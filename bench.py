@@ -8,7 +8,7 @@ Prints ONE JSON line on rank 0. For N > 1 launch with
 (one process per GPU; RANK / LOCAL_RANK / WORLD_SIZE are read from the environment).
 
 Workloads
-  views    (default) the view-dependent decoder stack of BASELINE.json's last configuration:
+  views    (default) the view-dependent decoder stack of a 64-camera run:
            random-init weights of renderformer-v1.1-swin-large shapes (dim 1024, 16 heads x 64,
            FFN 4096, 12 + 12 layers, fp16), a 5633-triangle synthetic scene, 64 random look-at
            cameras at 512x512. The scene is encoded once on rank 0 and its state (cross-
@@ -368,7 +368,7 @@ def run_kernels(args, backend, rank, world, peak, peak_src):
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32/f16", "data": "synthetic",
-        "config": {"workload": "kernels: configs 1-4 of BASELINE.json, one launch each per step",
+        "config": {"workload": "kernels: the glue operators at one view's and one scene's sizes, one launch each per step",
                    "l2": "rotating buffer sets > 2x L2 per operator", "impl": backend.name},
         "roofline": {"bound": "hbm", "kernel": dom["kernel"], "achieved": dom["gbs"], "peak": peak,
                      "unit": "GB/s", "frac": round(dom["gbs"] / peak, 3), "peak_source": peak_src,
@@ -589,7 +589,7 @@ def run_views(args, rank, world, peak, peak_src):
         loop(args.warmup, False, 1)
         single = _stats(figure(False, 1, reps=3)[0], world * K)
 
-    # strong scaling of BASELINE configs[4]: its 64 views sharded over the GPUs, the scene-state broadcast included
+    # strong scaling: the 64 views sharded over the GPUs, the scene-state broadcast included
     mine = list(range(rank, N_CAMERAS, world))
     barrier_sync(world)
     tb = time.perf_counter()
@@ -618,7 +618,7 @@ def run_views(args, rank, world, peak, peak_src):
         "unit": "views/s", "n_gpus": world, "steps": K, "warmup": args.warmup,
         "ms_per_step": round(ms_dev / K, 4), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f16", "data": "synthetic",
-        "config": {"workload": "BASELINE configs[4]: decoder stack of renderformer-v1.1-swin-large shapes (dim 1024, 16x64 "
+        "config": {"workload": "decoder stack of renderformer-v1.1-swin-large shapes (dim 1024, 16x64 "
                                "heads, FFN 4096, 12 layers, fp16) per 512x512 view over a 5633-triangle scene, 64 look-at "
                                "cameras; encoder K/V cache computed once on rank 0 and NCCL-broadcast; views sharded "
                                "round-robin, one view per GPU per step (rfk arm: views_per_frame views go through the decoder together "
@@ -640,7 +640,7 @@ def run_views(args, rank, world, peak, peak_src):
                 "scene_state_bytes": bc["bytes"], "scene_encode_s": round(encode_s, 3),
                 "scene_setup_s": round(encode_s + finalize_s, 3),
                 "views64_incl_broadcast": {"ms": round(v64_ms, 2), "views_per_s": round(N_CAMERAS / (v64_ms * 1e-3), 2),
-                                           "note": "the 64 views of configs[4] sharded over the GPUs, one scene-state "
+                                           "note": "the 64 views sharded over the GPUs, one scene-state "
                                                    "broadcast + every frame copied to pinned host memory; strong scaling"},
                 "note": "camera (c2w + fov) from host memory every view; the view's token map [4096x1024] fp16 copied "
                         "to pinned host memory every view"},

@@ -229,7 +229,7 @@ def test_batched_world_to_cam_and_ray_gen_paths_equal_the_single_view_kernels():
 
 
 # ----------------------------------------------------------------------------------------------
-# BASELINE configs[4] at full size: dim 1024, 16 heads x 64, FFN 4096, 12 decoder layers, 5633
+# The benchmark's network at full size: dim 1024, 16 heads x 64, FFN 4096, 12 decoder layers, 5633
 # triangles (5665 keys padded to 5672), 512x512 -> 4096 patch tokens.
 
 def _config5():
