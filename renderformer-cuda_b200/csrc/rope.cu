@@ -91,62 +91,155 @@ __device__ __forceinline__ void rotate8(float (&lo)[8], float (&hi)[8], const fl
     }
 }
 
-// T = __half or float data. NT tensors (1 or 2) share the tables. Each thread walks HP heads.
-// src/dst are [B,H,src_rows,D] / [B,H,dst_rows,D]; rows s >= seq_len (dst only) are copied.
-template <typename T, int NT, int HP>
+// Eight elements as they lie in memory.
+template <typename T> struct Raw8;
+template <> struct Raw8<__half> {
+    Half8 h;
+    __device__ __forceinline__ void load(const __half* p) { h = ld_half8(p); }
+    __device__ __forceinline__ void unpack(float (&f)[8]) const { unpack8(h, f); }
+};
+template <> struct Raw8<float> {
+    float v[8];
+    __device__ __forceinline__ void load(const float* p) { ld_float8(p, v); }
+    __device__ __forceinline__ void unpack(float (&f)[8]) const {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = v[i];
+    }
+};
+
+// The row and chunk of a thread: thread idx of `cpt` chunks a row.
+__device__ __forceinline__ bool row_and_chunk(int cpt, long long rows, long long& s, int& j) {
+    if (rows * cpt <= 0x7fffffffLL) {
+        const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+        s = idx / (unsigned)cpt;
+        j = (int)(idx % (unsigned)cpt);
+    } else {
+        const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        s = idx / cpt;
+        j = (int)(idx % cpt);
+    }
+    return s < rows;
+}
+
+// T = __half or float data. NT tensors (1 or 2) share the tables. src/dst are [B,H,src_rows,D] / [B,H,dst_rows,D]; rows s >= seq_len
+// (dst only) are copied. PLAIN: no such rows, no col_scale.
+// Bound: HBM. A thread has one chunk pair of one head (blockIdx.y, z) of each tensor, and asks for everything it needs before it stores
+// anything: source and destination may be the same, so the compiler keeps a load behind a store that comes before it, and a thread
+// that went from one tensor to the other waited for memory twice. Q and K of 5633 triangles, 47 MB, us from HBM / from L2: 16 heads of 64 11.6 / 9.5
+// that way, 8.5 / 7.6 now (5.5 TB/s); 8 heads of 128 12.1 / 8.9, now 8.9 / 6.3; eight scenes (380 MB) 78, now 58; 60 triangles 2.3, now 1.9. Several heads a
+// thread, which read the tables less often, take 8.8 (two) and 10.8 (four), 256 threads a CTA 9.4.
+template <typename T, int NT, bool PLAIN>
 __global__ void __launch_bounds__(128)
 rope_apply_kernel(const T* src0, T* dst0, const T* src1, T* dst1,
                   const __half* __restrict__ cos_vals, const __half* __restrict__ sin_vals,
-                  int batch, int num_heads, int seq_len, int rows_total, int head_dim,
+                  int num_heads, long long heads_total, int seq_len, int rows_total, int head_dim,
                   long long src_rows, long long dst_rows, long long src_bstride, long long dst_bstride,
                   long long tab_bstride, const float* __restrict__ col_scale, long long scale_bstride) {
     pdl_wait();
     pdl_trigger();
-    const int cpt = head_dim / 16;
-    const int hgroups = num_heads / HP;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = (long long)batch * hgroups * rows_total * cpt;
-    if (idx >= total) return;
-    const int j = (int)(idx % cpt);
-    long long t = idx / cpt;
-    const int s = (int)(t % rows_total);
-    t /= rows_total;
-    const int hg = (int)(t % hgroups);
-    const int b = (int)(t / hgroups);
     const int half_d = head_dim / 2;
-    const bool rotate = s < seq_len;
-
+    long long s;
+    int j;
+    int b = blockIdx.z, h = blockIdx.y;
+    if (heads_total) {   // more heads or batches than a grid has blocks that way: both in y and z
+        const long long bh = (long long)blockIdx.z * gridDim.y + blockIdx.y;
+        if (bh >= heads_total) return;
+        b = (int)(bh / num_heads);
+        h = (int)(bh % num_heads);
+    }
+    if (!row_and_chunk(head_dim / 16, rows_total, s, j)) return;
+    const size_t so = (size_t)b * src_bstride + ((size_t)h * src_rows + s) * head_dim + j * 8;
+    const size_t dofs = (size_t)b * dst_bstride + ((size_t)h * dst_rows + s) * head_dim + j * 8;
+    Raw8<T> lo8[NT], hi8[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        const T* sp = (n == 0 ? src0 : src1) + so;
+        lo8[n].load(sp);
+        hi8[n].load(sp + half_d);
+    }
+    const bool rotate = PLAIN || s < seq_len;
     float cl[8], sl[8], ch[8], sh[8];
     if (rotate) {
         const size_t to = (size_t)b * tab_bstride + (size_t)s * head_dim + j * 8;
-        unpack8(ldg_half8(cos_vals + to), cl);
-        unpack8(ldg_half8(sin_vals + to), sl);
-        unpack8(ldg_half8(cos_vals + to + half_d), ch);
-        unpack8(ldg_half8(sin_vals + to + half_d), sh);
+        const Half8 t0 = ldg_half8(cos_vals + to), t1 = ldg_half8(sin_vals + to), t2 = ldg_half8(cos_vals + to + half_d),
+                    t3 = ldg_half8(sin_vals + to + half_d);
+        unpack8(t0, cl); unpack8(t1, sl); unpack8(t2, ch); unpack8(t3, sh);
     }
 #pragma unroll
-    for (int hh = 0; hh < HP; ++hh) {
-        const int h = hg * HP + hh;
-        const size_t so = (size_t)b * src_bstride + ((size_t)h * src_rows + s) * head_dim + j * 8;
-        const size_t dofs = (size_t)b * dst_bstride + ((size_t)h * dst_rows + s) * head_dim + j * 8;
+    for (int n = 0; n < NT; ++n) {
+        float lo[8], hi[8];
+        lo8[n].unpack(lo);
+        hi8[n].unpack(hi);
+        if (rotate) rotate8(lo, hi, cl, sl, ch, sh);
+        if (!PLAIN && col_scale) {  // per-(head, element) factor applied to the rotated value before the one rounding
+            float g0[8], g1[8];
+            const float* gs = col_scale + (size_t)b * scale_bstride + (size_t)h * head_dim + j * 8;
+            ldg_float8(gs, g0);
+            ldg_float8(gs + half_d, g1);
 #pragma unroll
-        for (int tsel = 0; tsel < NT; ++tsel) {
-            const T* sp = tsel == 0 ? src0 : src1;
-            T* dp = tsel == 0 ? dst0 : dst1;
+            for (int i = 0; i < 8; ++i) { lo[i] *= g0[i]; hi[i] *= g1[i]; }
+        }
+        T* dp = (n == 0 ? dst0 : dst1) + dofs;
+        store8(dp, lo);
+        store8(dp + half_d, hi);
+    }
+}
+
+// The cached keys of several layers by one view's tables, out of place: batches of one tensor that share a table. A thread keeps its part of the
+// tables in registers and walks pairs of heads over all batches, four loads in flight; the stores leave the L2 to others (STREAM)
+// where the result is longer than half of it. Twelve layers, 16 heads of 64, us warm / cold, a thread per four heads of a layer (which read the tables
+// again for each four) and now: 5672 rows (279 MB) 68.8 / 69.9, 52.5 / 57.7; 7232 rows 88.9 / 91.1, 66.1 / 74.0; 1536 rows 19.9 / 22.0, 14.9 / 18.8;
+// 336 rows 6.6 / 7.0, 6.0 / 7.0. Some 2400 CTAs are enough: 600 to 9600 are within 5 %, 300 take 40 % longer.
+template <bool STREAM>
+__global__ void __launch_bounds__(128)
+rope_shared_table_kernel(const __half* src, __half* dst, const __half* __restrict__ cos_vals, const __half* __restrict__ sin_vals,
+                         int pairs, long long pairs_total, int rows, int head_dim, long long src_rows, long long dst_rows,
+                         long long src_bstride, long long dst_bstride, const float* __restrict__ col_scale, long long scale_bstride) {
+    constexpr int UN = 2;
+    pdl_wait();
+    pdl_trigger();
+    const int half_d = head_dim / 2;
+    long long s;
+    int j;
+    if (!row_and_chunk(head_dim / 16, rows, s, j)) return;
+    const size_t at = (size_t)s * head_dim + j * 8;
+    float cl[8], sl[8], ch[8], sh[8];
+    unpack8(ldg_half8(cos_vals + at), cl);
+    unpack8(ldg_half8(sin_vals + at), sl);
+    unpack8(ldg_half8(cos_vals + at + half_d), ch);
+    unpack8(ldg_half8(sin_vals + at + half_d), sh);
+    for (long long g = blockIdx.y; g < pairs_total; g += gridDim.y) {
+        const int b = (int)(g / pairs), h0 = (int)(g % pairs) * UN;
+        const __half* sp = src + (size_t)b * src_bstride + (size_t)h0 * src_rows * head_dim + at;
+        __half* dp = dst + (size_t)b * dst_bstride + (size_t)h0 * dst_rows * head_dim + at;
+        Half8 lo8[UN], hi8[UN];
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            lo8[u] = ldcs_half8(sp + (size_t)u * src_rows * head_dim);
+            hi8[u] = ldcs_half8(sp + (size_t)u * src_rows * head_dim + half_d);
+        }
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
             float lo[8], hi[8];
-            load8(sp + so, lo);
-            load8(sp + so + half_d, hi);
-            if (rotate) rotate8(lo, hi, cl, sl, ch, sh);
-            if (col_scale) {  // per-(head, element) factor applied to the rotated value before the one rounding
+            unpack8(lo8[u], lo);
+            unpack8(hi8[u], hi);
+            rotate8(lo, hi, cl, sl, ch, sh);
+            if (col_scale) {
+                const float* gs = col_scale + (size_t)b * scale_bstride + (size_t)(h0 + u) * head_dim + j * 8;
                 float g0[8], g1[8];
-                const float* gs = col_scale + (size_t)b * scale_bstride + (size_t)h * head_dim + j * 8;
                 ldg_float8(gs, g0);
                 ldg_float8(gs + half_d, g1);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) { lo[i] *= g0[i]; hi[i] *= g1[i]; }
             }
-            store8(dp + dofs, lo);
-            store8(dp + dofs + half_d, hi);
+            __half* d = dp + (size_t)u * dst_rows * head_dim;
+            if (STREAM) {
+                stcs_half8(d, pack8(lo));
+                stcs_half8(d + half_d, pack8(hi));
+            } else {
+                store8(d, lo);
+                store8(d + half_d, hi);
+            }
         }
     }
 }
@@ -215,26 +308,24 @@ static int launch_rope(const T* src0, T* dst0, const T* src1, T* dst1, const __h
                      tab_bstride % 8 == 0 && (!col_scale || (aligned16(col_scale) && scale_bstride % 4 == 0));
     if (col_scale && !vec) return RFK_EUNSUPPORTED;  // the scaled form exists in the vector kernel only
     if (vec) {
-        const int cpt = head_dim / 16;
-        // One head per thread unless the problem is large: at the benchmark size (47 MB) the
-        // kernel lasts ~10 us and is bound by how evenly short-lived CTAs keep loads in
-        // flight (ncu: 24 % DRAM utilisation with 2 heads per thread and 1.6 waves of
-        // 705 CTAs); walking several heads per thread only pays once there are at least two
-        // full waves of threads left (the cos/sin re-reads it saves come from L2 anyway).
-        const long long per_head = (long long)batch * rows_total * cpt;
-        const long long two_waves = 2LL * kNumSMs * 2048;
-        const int hp = (num_heads % 4 == 0 && per_head * (num_heads / 4) >= two_waves) ? 4
-                     : (num_heads % 2 == 0 && per_head * (num_heads / 2) >= two_waves) ? 2 : 1;
-        const long long total = (long long)batch * (num_heads / hp) * rows_total * cpt;
-        const unsigned grid = ceil_div(total, 128);
-#define RFK_ROPE(HPV)                                                                         \
-    launch_pdl(rope_apply_kernel<T, NT, HPV>, dim3(grid), dim3(128), 0, st, src0, dst0, src1, dst1, \
-               cos_vals, sin_vals, batch, num_heads, seq_len, rows_total, head_dim, src_rows,        \
-               dst_rows, src_bstride, dst_bstride, tab_bstride, col_scale, scale_bstride)
-        if (hp == 4) RFK_ROPE(4);
-        else if (hp == 2) RFK_ROPE(2);
-        else RFK_ROPE(1);
-#undef RFK_ROPE
+        const unsigned blocks = ceil_div((long long)rows_total * (head_dim / 16), 128);
+        const long long heads_total = (long long)batch * num_heads;
+        if constexpr (NT == 1 && sizeof(T) == 2) {
+            if (src0 != dst0 && batch > 1 && tab_bstride == 0 && seq_len == rows_total && num_heads % 2 == 0) {
+                const long long pairs_total = heads_total / 2;
+                const unsigned split = (unsigned)std::min<long long>({pairs_total, 65535, (long long)ceil_div(2400, blocks)});
+                const bool out_of_l2 = heads_total * rows_total * head_dim * 2 > (63ll << 20);
+                launch_pdl(out_of_l2 ? rope_shared_table_kernel<true> : rope_shared_table_kernel<false>, dim3(blocks, split), dim3(128), 0, st,
+                           src0, dst0, cos_vals, sin_vals, num_heads / 2, pairs_total, rows_total, head_dim, src_rows, dst_rows,
+                           src_bstride, dst_bstride, col_scale, scale_bstride);
+                return launch_status();
+            }
+        }
+        const bool flat = num_heads > 65535 || batch > 65535;
+        const unsigned gy = flat ? 65535u : num_heads, gz = flat ? ceil_div(heads_total, 65535) : batch;
+        launch_pdl(seq_len == rows_total && !col_scale ? rope_apply_kernel<T, NT, true> : rope_apply_kernel<T, NT, false>, dim3(blocks, gy, gz), dim3(128), 0, st, src0, dst0, src1, dst1, cos_vals, sin_vals,
+                   num_heads, flat ? heads_total : 0, seq_len, rows_total, head_dim, src_rows, dst_rows, src_bstride, dst_bstride,
+                   tab_bstride, col_scale, scale_bstride);
     } else {
         const long long total = (long long)batch * num_heads * rows_total * (head_dim / 2);
         launch_pdl(rope_apply_generic_kernel<T, NT>, dim3(ceil_div(total, 256)), dim3(256), 0, st,
