@@ -319,6 +319,10 @@ size_t rfk_scene_state_bytes(const rfk_model* model, int n_tris);
  * scene_state: caller-owned device buffer of rfk_scene_state_bytes() bytes (filled either by
  * rfk_session_encode_scene on this device or by a broadcast from the device that ran it).
  * Allocates every per-view buffer; runs nothing.
+ * The weights stay the caller's and are read where they lie, except that a session keeps copies, laid out for its kernels, of an image head's
+ * filters and of the cross-attention's query norms (taken when it is created) and, where it ends at the token map and rows are 1024
+ * wide, of the decoder's products behind a norm with the norm's weight multiplied in (24 MB a layer at 4096 hidden; taken by
+ * rfk_session_finalize, and again by every rfk_session_encode_scene after that).
  * replaces the allocation half of rf::RenderSession::create — src/pipeline/render_session.cu:258-295,418-462 */
 int rfk_session_create(const rfk_model* model, int n_tris, int img_res, void* scene_state,
                        int flags, rfk_session** out);

@@ -299,6 +299,7 @@ struct WinNorm {
     const float* q_ss; const float* k_ss;      // [rows][tiles] partial sums of squares (rows in window order)
     const float* gamma_q; const float* gamma_k;  // [heads * head_dim]
     int tiles; float inv_dim, eps;
+    int blocks;                                // the tokens are in blocks, the mask in rows
 };
 
 template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTokens * kWinTokens;
@@ -314,6 +315,7 @@ enum WinForm { kWinFused, kWinNormed, kWinSteps };
 // (operands in L2 as behind the projection: 64 windows x 16 heads 9.1 -> 8.2 us, 256 x 16 39.3 -> 35.8, 4 x 16 4.3 -> 3.2, 64 x 32
 // 17.6 -> 15.7). A number that is not known to the compiler puts a loop between the loads: 9.1 us again, and the choice between the two
 // inside the kernel cost the others 2 %.
+constexpr int kWinEights = 8;   // FOURS: the row's sums in groups of eight (ss_group), summed once per CTA
 template <WinForm FORM, int HD, int FOURS = 0>
 __global__ void __launch_bounds__(kWinThreads, HD == 64 ? 8 : 4)
 window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
@@ -353,6 +355,7 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
         const int c = tid % CPR, r_first = tid / CPR;
         constexpr int kRowStep = kWinThreads / CPR;                   // 16 (8 with 128-wide heads)
         constexpr int kRowsPerPass = 4;
+        __shared__ float s_ss[2][FOURS == kWinEights ? kWinTokens : 1];
         float gq[8], gk[8];
         ldg_float8(nrm.gamma_q + h * HD + c * 8, gq);
         ldg_float8(nrm.gamma_k + h * HD + c * 8, gk);
@@ -367,7 +370,8 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
                 raw[1][k] = ldg_half8(Kh + r * HD + c * 8);
                 const long long row = (long long)bw * kWinTokens + r;   // token row in window order
                 float sq = 0.0f, sk = 0.0f;
-                if (FOURS > 0) {
+                if (FOURS == kWinEights) {
+                } else if (FOURS > 0) {
                     const float4 *q4 = reinterpret_cast<const float4*>(nrm.q_ss) + row * FOURS, *k4 = reinterpret_cast<const float4*>(nrm.k_ss) + row * FOURS;
 #pragma unroll
                     for (int t = 0; t < FOURS; ++t) {
@@ -384,12 +388,23 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
                 ss[0][k] = sq;
                 ss[1][k] = sk;
             }
+            if (FOURS == kWinEights && r0 == r_first) {   // a thread sums one row of one tile for all
+                const int row = tid & (kWinTokens - 1), which = tid / kWinTokens;
+                const float* s = (which ? nrm.k_ss : nrm.q_ss) + ((long long)bw * kWinTokens + row) * nrm.tiles;
+                float sum = 0.0f;
+                for (int t = 0; t < nrm.tiles; t += 8) {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(s + t)), b = __ldg(reinterpret_cast<const float4*>(s + t + 4));
+                    sum += ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+                }
+                s_ss[which][row] = sum;
+                __syncthreads();
+            }
 #pragma unroll
             for (int k = 0; k < kRowsPerPass; ++k) {
                 const int r = r0 + k * kRowStep;
 #pragma unroll
                 for (int which = 0; which < 2; ++which) {
-                    const float rinv = rsqrtf(ss[which][k] * nrm.inv_dim + nrm.eps);
+                    const float rinv = rsqrtf((FOURS == kWinEights ? s_ss[which][r] : ss[which][k]) * nrm.inv_dim + nrm.eps);
                     float x[8];
                     unpack8(raw[which][k], x);
 #pragma unroll
@@ -429,8 +444,11 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     }
     // scores in the exponent's units; masked-out pairs get -FLT_MAX (a fully masked row ends up uniform)
     const int q_lo = warp * 16 + g;  // this thread's rows: q_lo (regs 0, 1) and q_lo + 8 (regs 2, 3)
-    const uint8_t* m0 = sMask + q_lo * kWinTokens;
-    const uint8_t* m1 = m0 + 8 * kWinTokens;
+    const bool blocks = FORM == kWinNormed && nrm.blocks;
+    // token t of a window in blocks -> its place in row order
+    const auto in_rows = [](int t) { return (t & 32) | ((t & 12) << 1) | ((t & 16) >> 2) | (t & 3); };
+    const uint8_t* m0 = sMask + (blocks ? in_rows(q_lo) : q_lo) * kWinTokens;
+    const uint8_t* m1 = sMask + (blocks ? in_rows(q_lo + 8) : q_lo + 8) * kWinTokens;
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
@@ -442,8 +460,9 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
             s[n][0] *= scale_log2e; s[n][1] *= scale_log2e; s[n][2] *= scale_log2e; s[n][3] *= scale_log2e;
         }
         if (mask) {
-            const unsigned a = *reinterpret_cast<const unsigned short*>(m0 + c);
-            const unsigned b = *reinterpret_cast<const unsigned short*>(m1 + c);
+            const int at = blocks ? in_rows(c) : c;   // c is even: a pair stays a pair
+            const unsigned a = *reinterpret_cast<const unsigned short*>(m0 + at);
+            const unsigned b = *reinterpret_cast<const unsigned short*>(m1 + at);
             if ((a & 0xffu) == 0) s[n][0] = -FLT_MAX;
             if ((a >> 8) == 0) s[n][1] = -FLT_MAX;
             if ((b & 0xffu) == 0) s[n][2] = -FLT_MAX;
@@ -553,7 +572,7 @@ static int launch_window_attention(const __half* Q, const __half* K, const __hal
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                      const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
                      int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
-                     rfk_stream_t stream) {
+                     rfk_stream_t stream, int ss_group, bool blocks) {
     if (!Q || !K || !V || !O || BnW < 0 || num_heads <= 0 || nW <= 0) return RFK_EINVAL;
     if (q_row_ss && (!k_row_ss || !gamma_q || !gamma_k || ss_tiles <= 0 || norm_dim <= 0)) return RFK_EINVAL;
     if (window_tokens != kWinTokens || (head_dim != 64 && head_dim != 128)) return RFK_EUNSUPPORTED;
@@ -567,7 +586,12 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
         return (head_dim == 64 ? launch_window_attention<kWinFused, 64> : launch_window_attention<kWinFused, 128>)(
             q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, WinNorm{}, st);
     if (!aligned16(gamma_q) || !aligned16(gamma_k)) return RFK_EUNSUPPORTED;
-    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
+    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps, blocks};
+    if (ss_group == 8) {
+        if (!aligned16(q_row_ss) || !aligned16(k_row_ss) || ss_tiles % 8) return RFK_EUNSUPPORTED;
+        return (head_dim == 64 ? launch_window_attention<kWinNormed, 64, kWinEights> : launch_window_attention<kWinNormed, 128, kWinEights>)(
+            q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
+    }
     const int fours = aligned16(q_row_ss) && aligned16(k_row_ss) && (ss_tiles == 4 || ss_tiles == 8) ? ss_tiles / 4 : 0;
     const auto launch = head_dim == 64 ? (fours == 1   ? launch_window_attention<kWinNormed, 64, 1>
                                           : fours == 2 ? launch_window_attention<kWinNormed, 64, 2>
@@ -600,7 +624,7 @@ int attention_tc_arrive(int* counter, int failed, int pieces);
 int attention_tc_handover_plan(long long units, int n_tiles, int sms, int* whole_units, int* n_handed, unsigned short* first, int max_handed);
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared);
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared, int ss_group);
 
 }  // namespace rfk
 
@@ -630,7 +654,7 @@ extern "C" int rfk_flash_attention(const rfk_half* Q, const rfk_half* K, const r
     if ((D == 64 || D == 128) && path != 1) {  // tcgen05 kernel; in automatic mode the mma.sync kernel takes over if it cannot run
         const int rc = launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk,
                                            n_keys, D, o_bshd, scale, as_stream(stream), nullptr, 0, 0, 0.0f, nullptr, 0,
-                                           AttnCut::kLastRound, 0);
+                                           AttnCut::kLastRound, 0, 1);
         if (rc != RFK_EUNSUPPORTED || path == 2) return rc;
     }
     return flash_attention_mma(Q, K, V, O, B, H, Sq, Sk, n_keys, D, o_bshd, scale, stream);
@@ -649,14 +673,14 @@ static int check_flash_attention_ex(const rfk_half* Q, const rfk_half* K, const 
 int rfk::flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss,
                             int ss_tiles, int norm_dim, float eps, void* workspace, size_t workspace_bytes, AttnCut cut,
                             int v_shared, int B, int H, int Sq, int Sk, int n_keys, int D, int o_bshd, float scale,
-                            rfk_stream_t stream) {
+                            rfk_stream_t stream, int ss_group) {
     const int rc = check_flash_attention_ex(Q, K, V, O, q_row_ss, ss_tiles, norm_dim, workspace, workspace_bytes, B, H, Sq, Sk, n_keys, scale);
     if (rc != RFK_OK || B == 0 || Sq == 0) return rc;
     if ((D != 64 && D != 128) || (long long)B * H > 65535 || g_attn_path.load(std::memory_order_relaxed) == 1) return RFK_EUNSUPPORTED;
     if (!aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(O) || !aligned16(workspace)) return RFK_EUNSUPPORTED;
     return launch_attention_tc((const __half*)Q, (const __half*)K, (const __half*)V, (__half*)O, B, H, Sq, Sk, n_keys, D, o_bshd,
                                scale, as_stream(stream), q_row_ss, ss_tiles, norm_dim, eps, workspace, workspace_bytes,
-                               cut, v_shared != 0);
+                               cut, v_shared != 0, ss_group);
 }
 
 extern "C" int rfk_flash_attention_ex_wide(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O,

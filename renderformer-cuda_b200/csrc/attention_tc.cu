@@ -589,9 +589,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         float scale_log2e = scale_log2e_all;
         if (row_ss) {
             const int q = min(q0 + blk * BM + r, Sq - 1);
-            const float* sp = row_ss + ((size_t)(bh / H) * Sq + q) * ss_tiles;
+            const int sums = ss_tiles < 0 ? -ss_tiles : ss_tiles;
+            const float* sp = row_ss + ((size_t)(bh / H) * Sq + q) * sums;
             float ss = 0.0f;
-            for (int t = 0; t < ss_tiles; ++t) ss += __ldg(sp + t);
+            if (ss_tiles > 0) {
+                for (int t = 0; t < sums; ++t) ss += __ldg(sp + t);
+            } else {   // groups of eight (ss_group)
+                for (int t = 0; t < sums; t += 8) {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(sp + t)), b = __ldg(reinterpret_cast<const float4*>(sp + t + 4));
+                    ss += ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+                }
+            }
             scale_log2e *= rsqrtf(ss * inv_norm_dim + norm_eps);
         }
         float m_run = kNoMax, l_run = 0.0f;
@@ -1101,7 +1109,11 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
 // attention_tc_workspace_bytes() bytes whose first 1024 are zero, for the key split.
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
-                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared) {
+                        int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared, int ss_group) {
+    if (ss_group == 8) {   // the kernel takes it as a negative number of sums
+        if (ss_tiles % 8 || !aligned16(row_ss)) return RFK_EUNSUPPORTED;
+        ss_tiles = -ss_tiles;
+    }
     const auto launch = D == 64 ? launch_hd<64, false> : cut == AttnCut::kNone ? launch_hd<128, true> : launch_hd<128, false>;
     return launch(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, ws_bytes, cut, v_shared);
 }

@@ -71,6 +71,41 @@ __device__ unsigned long long g_timeline[16];
 // statistic of the QK-RMSNorm that follows the projection, so that the consumer can normalise while it loads.
 constexpr int kEpiHeads = 3;
 
+// Folded norms. A projection behind an RMSNorm, C = epilogue((x / rms(x) * gamma) W^T), is rms(x)^-1 * (x (W gamma)^T) a row: with the norm's
+// weight multiplied into W once, the product can take x as it is, and the norm costs a factor a row in the epilogue, from the row's sum
+// of squares, which whoever wrote x has summed beside it. Three launches of a decoder layer's eleven go, and with them 2 to 3 us each of a small
+// view and 5 to 8 of a large one (us a view, separate norms / folded: 128 x 128 pixels 772 / 650, 512 x 512 3902 / 3787, with 128-wide heads
+// 3456 / 3370, frames of four 14460 / 13930); the sums and the reordering cost a product 0.3 to 1.5. Writing x * gamma beside x instead of
+// folding gamma into W cost 36 products of a view 2.4 us each (512 x 512 3863, 128 x 128 680). EPI with this bit: SwiGLU and head-split products whose rows get such a
+// factor; residual products that write the sums of squares of their rows, and may put the rows elsewhere (Grid).
+// The sums lie [row][tiles]: one each 256 columns, or one each 32 where tiles of fewer columns wrote them. Both add the
+// same way - eight squares in column order, four of those in pairs (square_sum), eight of these in order, the 256s in order - so that whoever reads
+// them gets the same bits.
+constexpr int kFold = 8;
+
+// Rows that are the 4 x 4 blocks of a token grid, block by block (16 rows), windows of 2 x 2 blocks one after the other, of a grid that has been
+// shifted by `from` blocks: where they go in a grid shifted by `to` blocks, and where in raster order.
+struct Grid {
+    int bw, bh;       // blocks across and down; 0: rows stay where they are
+    int from, to;
+    __device__ __forceinline__ void block(int k, int& view, int& by, int& bx) const {   // k-th block, in the unshifted grid
+        const int per = bw * bh;
+        view = k / per;
+        const int i = k - view * per, win = i >> 2, ww = bw >> 1;
+        by = (win / ww) * 2 + ((i >> 1) & 1) - from;
+        bx = (win % ww) * 2 + (i & 1) - from;
+        if (by < 0) by += bh;
+        if (bx < 0) bx += bw;
+    }
+    __device__ __forceinline__ int next(int view, int by, int bx) const {   // that block's index in the grid shifted by `to`
+        by += to;
+        bx += to;
+        if (by >= bh) by -= bh;
+        if (bx >= bw) bx -= bw;
+        return view * bw * bh + (((by >> 1) * (bw >> 1) + (bx >> 1)) << 2) + ((by & 1) << 1) + (bx & 1);
+    }
+};
+
 struct Params {
     __half* C; long long ldc;
     const __half* R; long long ldr;     // residual (EPI_RESIDUAL), may alias C
@@ -80,7 +115,27 @@ struct Params {
     float* row_ss;                      // kEpiHeads: [parts][M][tiles per part] partial sums of squares, or null
     long long part_stride;              // kEpiHeads on small tiles, which store without a tensor map: halves between parts
     int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
+    const float* in_ss; int in_tiles, in_group;    // kFold: A's rows' sums of squares, how many a row, and how many of them make up 256 columns
+    float in_inv_dim, in_eps, in_mul;              // the row's factor: in_mul * rsqrt(sum * in_inv_dim + in_eps)
+    int ss_tiles;                                  // kFold: sums a row that row_ss gets, of a part
+    __half* raster;                                // kFold, residual: the rows in raster order too, or alone if C is null; pitch ldc
+    Grid grid;
 };
+
+// a row's factor (kFold)
+__device__ __forceinline__ float row_factor(const Params& p, int row) {
+    const float* s = p.in_ss + (size_t)row * p.in_tiles;
+    float sum = 0.0f;
+    if (p.in_group == 1) {
+        for (int t = 0; t < p.in_tiles; ++t) sum += __ldg(s + t);
+    } else {
+        for (int t = 0; t < p.in_tiles; t += 8) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(s + t)), b = __ldg(reinterpret_cast<const float4*>(s + t + 4));
+            sum += ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+        }
+    }
+    return p.in_mul * rsqrtf(fmaf(sum, p.in_inv_dim, p.in_eps));
+}
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     __half2 h = __floats2half2_rn(lo, hi);
@@ -88,6 +143,22 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 }
 __device__ __forceinline__ float2 unpack_half2(uint32_t w) {
     return __half22float2(*reinterpret_cast<__half2*>(&w));
+}
+
+// The sum of the squares of 32 fp16 values, packed in order; four chains, for their latency
+__device__ __forceinline__ float square_sum(const uint32_t (&o)[16]) {
+    float c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        c[k] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 v = unpack_half2(o[4 * k + i]);
+            c[k] = fmaf(v.x, v.x, c[k]);
+            c[k] = fmaf(v.y, v.y, c[k]);
+        }
+    }
+    return (c[0] + c[1]) + (c[2] + c[3]);
 }
 
 // Tiled copy global -> shared of one box of a rank-2 tensor map (x innermost, in elements; x * 2 bytes
@@ -363,10 +434,12 @@ struct __align__(8) Ctrl {
 };
 static_assert(sizeof(Ctrl) <= 256, "control block");
 
-template <int EPI, int BM_, int BN_>
+template <int EPI_, int BM_, int BN_>
 __global__ void __launch_bounds__(kThreads)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                      const __grid_constant__ CUtensorMap map_w1, const Params p) {
+    constexpr int EPI = EPI_ & 7;
+    constexpr bool FOLD = (EPI_ & kFold) != 0;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     constexpr bool kWhole = BM_ == 128 && BN_ == 128;   // producer and issuer run their loops as whole warps
     constexpr bool kLane0 = BM_ == 128 && BN_ == 64 && (EPI == RFK_GEMM_EPI_NONE || EPI == RFK_GEMM_EPI_RESIDUAL);   // the producer is lane 0
@@ -384,8 +457,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int num_st = (p.K + kSub * BK - 1) / (kSub * BK);   // stages of K; a second block beyond K arrives as zeros
     // rows fastest, so that the tiles running together share weights; the heads form runs columns fastest, because the tiles
     // of 256 columns are one cluster
-    const int m0 = (EPI == kEpiHeads ? blockIdx.x / p.tiles_n : blockIdx.x % p.tiles_m) * BM_;
-    const int n0 = (EPI == kEpiHeads ? blockIdx.x % p.tiles_n : blockIdx.x / p.tiles_m) * BN_OUT;
+    const int m0 = (EPI == kEpiHeads && !FOLD ? blockIdx.x / p.tiles_n : blockIdx.x % p.tiles_m) * BM_;
+    const int n0 = (EPI == kEpiHeads && !FOLD ? blockIdx.x % p.tiles_n : blockIdx.x / p.tiles_m) * BN_OUT;
     const bool want_ss = EPI == kEpiHeads && p.row_ss && ((p.ss_mask >> (n0 / (p.units * 64))) & 1);   // uniform over a cluster
     bool acc_ok = false;
 
@@ -478,6 +551,19 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const bool row_ok = row < p.M && (BM_ == 128 || lane < 16);
         const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
         __half* crow = p.C + (size_t)(row_ok ? row : 0) * p.ldc + n0;
+        __half* rrow2 = nullptr;                              // kFold, residual: the row's place in raster order
+        int ss_row = row;
+        if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && p.grid.bw && row_ok) {
+            int view, by, bx;
+            p.grid.block(row >> 4, view, by, bx);
+            ss_row = p.grid.next(view, by, bx) * 16 + (row & 15);
+            crow = p.C ? p.C + (size_t)ss_row * p.ldc + n0 : nullptr;
+            if (p.raster) {
+                const size_t at = ((size_t)view * p.grid.bh + by) * 4 + ((row >> 2) & 3);
+                rrow2 = p.raster + (at * (p.grid.bw * 4) + bx * 4 + (row & 3)) * p.ldc + n0;
+            }
+        }
+        const float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
         constexpr int kChunk = BN_OUT < 32 ? BN_OUT : 32;     // output columns per step
         uint4 res[EPI == RFK_GEMM_EPI_RESIDUAL ? BN_OUT / 8 : 1];
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                   // the row's residual arrives while the products run
@@ -487,7 +573,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 res[q] = (row_ok && n0 + q * 8 < p.N) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
         }
         acc_ok = tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag);
-        if (EPI != kEpiHeads && acc_ok) {
+        if ((EPI != kEpiHeads || FOLD) && acc_ok) {
             tc::tc_fence_after();
 #pragma unroll
             for (int c = 0; c < BN_OUT / kChunk; ++c) {
@@ -504,6 +590,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         tc::tc_wait_ld(v);
 #pragma unroll
                         for (int i = 0; i < 16; ++i) u[i] = v[16 + i];
+                    }
+                    if (FOLD) {
+#pragma unroll
+                        for (int i = 0; i < kChunk; ++i) {
+                            v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
+                            u[i] = __float_as_uint(__uint_as_float(u[i]) * factor);
+                        }
                     }
 #pragma unroll
                     for (int i = 0; i < kChunk; i += 2) {
@@ -536,15 +629,34 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < kChunk / 2; ++i) o[i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                        for (int i = 0; i < kChunk / 2; ++i)
+                            o[i] = FOLD ? pack_half2(__uint_as_float(v[2 * i]) * factor, __uint_as_float(v[2 * i + 1]) * factor)
+                                        : pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                    }
+                    if (FOLD && p.row_ss && row_ok) {         // the sum of the chunk's squares, as they are stored
+                        const int part = EPI == kEpiHeads ? n0 / (p.units * 64) : 0, col = n0 + c * 32 - part * p.units * 64;
+                        if constexpr (kChunk == 32) {
+                            if (EPI != kEpiHeads || ((p.ss_mask >> part) & 1))
+                                p.row_ss[((size_t)part * p.M + ss_row) * p.ss_tiles + (col >> 5)] = square_sum(o);
+                        }
                     }
                 }
-                if (row_ok) {
+                if (FOLD && EPI == kEpiHeads) {               // [part][group][head][seq][hd]
+                    if (row_ok) {
+                        const int hd = p.head_units * 64, heads = p.units / p.head_units, g = (n0 + c * 32) / 64, u = g % p.units;
+                        __half* dst = p.C + (size_t)(g / p.units) * p.part_stride + ((size_t)(row / p.seq) * heads * p.out_seq + row % p.seq) * hd +
+                                      (size_t)(u / p.head_units) * p.out_seq * hd + (u % p.head_units) * 64 + ((n0 / 32 + c) & 1) * 32;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                    }
+                } else if (row_ok) {
 #pragma unroll
                     for (int q = 0; q < kChunk / 8; ++q) {
                         const int col = n0 + c * kChunk + q * 8;
-                        if (col < p.N)
-                            *reinterpret_cast<uint4*>(crow + c * kChunk + q * 8) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                        const uint4 w = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                        if (col < p.N && (!FOLD || crow)) *reinterpret_cast<uint4*>(crow + c * kChunk + q * 8) = w;
+                        if (FOLD && col < p.N && rrow2) *reinterpret_cast<uint4*>(rrow2 + c * kChunk + q * 8) = w;
                     }
                 }
             }
@@ -552,7 +664,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         __syncwarp();
     }
 
-    if (EPI == kEpiHeads) {
+    if (EPI == kEpiHeads && !FOLD) {
         // ------------------------------------------------------------ epilogue of the head-split form
         // [part][group][head][seq][hd] by plain stores. The row statistic has the bits of the pair kernel's: one thread adds
         // a row's 256 squares in column order. So the cluster's tiles are gathered in its first CTA's ring, which is idle
@@ -671,7 +783,8 @@ constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA, of which a
 constexpr int kUnitCols = 64;
 constexpr int kUnitBytes = 32 * kUnitCols * 2;       // 4 KB
 // BN: accumulator columns of a tile, 256 or 192 (narrow_tile)
-template <int EPI, int BN> struct Cfg {
+template <int EPI_, int BN> struct Cfg {
+    static constexpr int EPI = EPI_ & 7;
     static constexpr int kUnits = (EPI == RFK_GEMM_EPI_SWIGLU) ? 2 : BN / 64;              // 64-column units per tile
     static constexpr int kBufsPerWarp = (EPI == RFK_GEMM_EPI_RESIDUAL) ? 4 : 2;
     static constexpr int kStagingBytes = 4 * kBufsPerWarp * kUnitBytes;                      // 4 epilogue warps
@@ -695,6 +808,10 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src_smem
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
                  ::"l"(tmap), "r"(src_smem), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const void* tmap, uint32_t src_smem, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(tmap), "r"(src_smem), "r"(x), "r"(y), "r"(z) : "memory");
+}
 __device__ __forceinline__ void tma_store_5d(const void* tmap, uint32_t src_smem, int c0, int c1, int c2, int c3, int c4) {
     asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
                  ::"l"(tmap), "r"(src_smem), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
@@ -716,14 +833,23 @@ __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* ma
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
 // t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0. turn: the staging buffer of the
 // next store, kept from tile to tile (not with the residual epilogue).
-template <int EPI, int BN>
-__device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, uint32_t t_acc,
+template <int EPI_, int BN>
+__device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, uint32_t t_acc, float factor,
                                                      unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
                                                      int row0, int n0, int lane, int& turn, volatile int* abort_flag) {
+    constexpr int EPI = EPI_ & 7;
+    constexpr bool FOLD = (EPI_ & kFold) != 0;
     constexpr int kUnits = Cfg<EPI, BN>::kUnits;
     const uint32_t stage_base = tc::smem_addr(stage_ptr);
     uint32_t v[32];
     float ss = 0.0f;   // kEpiHeads: this row's sum of squares over the tile
+    int ss_row = row0 + lane, block[2][3] = {};   // FOLD, residual: where the row's sums go; view and place of the warp's two blocks
+    if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && p.grid.bw) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) p.grid.block((row0 >> 4) + h, block[h][0], block[h][1], block[h][2]);
+        const int h = lane >> 4;
+        ss_row = p.grid.next(h ? block[1][0] : block[0][0], h ? block[1][1] : block[0][1], h ? block[1][2] : block[0][2]) * 16 + (lane & 15);
+    }
 #pragma unroll 1
     for (int u = 0; u < kUnits; ++u) {
         const int b = (EPI == RFK_GEMM_EPI_RESIDUAL) ? u : turn;
@@ -747,6 +873,13 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
                 tc::tmem_ld32(t_acc + 128 + c32 * 32, up);   // up columns of the same hidden units
                 tc::tc_wait_ld(v);
                 tc::tc_wait_ld(up);
+                if (FOLD) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
+                        up[i] = __float_as_uint(__uint_as_float(up[i]) * factor);
+                    }
+                }
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
                     const float g0 = __uint_as_float(v[i]), g1 = __uint_as_float(v[i + 1]);
@@ -784,8 +917,10 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
                     }
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) o[i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-                    if (EPI == kEpiHeads) {   // the norm that follows sees the stored fp16 values
+                    for (int i = 0; i < 16; ++i)
+                        o[i] = FOLD ? pack_half2(__uint_as_float(v[2 * i]) * factor, __uint_as_float(v[2 * i + 1]) * factor)
+                                    : pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                    if (EPI == kEpiHeads && !FOLD) {   // the norm that follows sees the stored fp16 values
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float2 r2 = unpack_half2(o[i]);
@@ -793,6 +928,16 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
                             ss = fmaf(r2.y, r2.y, ss);
                         }
                     }
+                }
+            }
+            if (FOLD && EPI != RFK_GEMM_EPI_SWIGLU) {
+                const float part_ss = square_sum(o);
+                if (BN == 256) {
+                    ss = c32 == 0 ? part_ss : ss + part_ss;
+                } else if (p.row_ss && row0 + lane < p.M) {
+                    const int part = EPI == kEpiHeads ? n0 / (p.units * 64) : 0;
+                    if (EPI != kEpiHeads || ((p.ss_mask >> part) & 1))
+                        p.row_ss[((size_t)part * p.M + ss_row) * p.ss_tiles + (n0 >> 5) + c32 - part * p.units * 2] = part_ss;
                 }
             }
 #pragma unroll
@@ -806,6 +951,17 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
                 const int g = (n0 + u * kUnitCols) / kUnitCols;   // 64-column unit over all parts
                 tma_store_5d(map_c, stage_base + b * kUnitBytes, (g % p.head_units) * kUnitCols, row0 % p.seq,
                              (g % p.units) / p.head_units, row0 / p.seq, g / p.units);
+            } else if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && p.grid.bw) {   // two blocks of 16 rows; M is a whole number of them, 32 at a time
+                if (row0 < p.M) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t src = stage_base + b * kUnitBytes + h * (kUnitBytes / 2);
+                        if (p.C)
+                            tma_store_2d(map_c, src, n0 + u * kUnitCols, p.grid.next(block[h][0], block[h][1], block[h][2]) * 16);
+                        if (p.raster)
+                            tma_store_3d(map_raster, src, n0 + u * kUnitCols, block[h][2] * 4, (block[h][0] * p.grid.bh + block[h][1]) * 4);
+                    }
+                }
             } else {
                 tma_store_2d(map_c, stage_base + b * kUnitBytes, n0 + u * kUnitCols, row0);   // rows >= M, columns >= N are clipped
             }
@@ -813,7 +969,8 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
         }
         turn ^= 1;
     }
-    if (EPI == kEpiHeads && p.row_ss) {
+    if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && BN == 256 && p.row_ss && row0 + lane < p.M) p.row_ss[(size_t)ss_row * p.ss_tiles + n0 / 256] = ss;
+    if (EPI == kEpiHeads && p.row_ss && (!FOLD || BN == 256)) {
         const int dim = p.units * kUnitCols, part = n0 / dim, row = row0 + lane;
         if (((p.ss_mask >> part) & 1) && row < p.M)
             p.row_ss[((size_t)part * p.M + row) * (dim / 256) + (n0 % dim) / 256] = ss;
@@ -821,11 +978,13 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     return true;
 }
 
-template <int EPI, int BN>
+template <int EPI_, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                     const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_c,
                     const __grid_constant__ CUtensorMap map_r, const Params p) {
+    constexpr int EPI = EPI_ & 7;
+    constexpr bool FOLD = (EPI_ & kFold) != 0;
     static_assert(BN == 256 || (BN == 192 && EPI != RFK_GEMM_EPI_SWIGLU), "whole 64-column units");
     constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? 128 : BN;
     constexpr int kTxBytes = kABytes + BN / 2 * BK * 2;   // of a stage, per CTA
@@ -857,7 +1016,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncwarp();
     cluster_arrive();            // this CTA's barriers are initialised; the rest of the set-up runs under the cluster barrier's latency
     if (warp == 1 && lane == 0) {   // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
-        tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(rank == 0 ? &map_w0 : &map_w1); tc::prefetch_tensormap(&map_c);
+        tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(rank == 0 || (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL) ? &map_w0 : &map_w1); tc::prefetch_tensormap(&map_c);
         if (EPI == RFK_GEMM_EPI_RESIDUAL) tc::prefetch_tensormap(&map_r);
     }
     if (warp == 2 && aligned) {  // beside the barriers; the same in both CTAs of the pair
@@ -881,7 +1040,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 0) {
         // ------------------------------------------------------------ producer (an elected lane per CTA)
         if (tc::elect_one()) {
-            const void* map_w = rank == 0 ? (const void*)&map_w0 : (const void*)&map_w1;
+            // (FOLD, residual: map_w1 is the raster output's map)
+            const void* map_w = rank == 0 || (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL) ? (const void*)&map_w0 : (const void*)&map_w1;
             int it = 0;
             bool ok = true;
             for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
@@ -961,11 +1121,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
                 epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
+            const float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(4);   // first tile's accumulator complete
-            ok = epilogue_tile_staged<EPI, BN>(p, &map_c, tmem_cta + lane_off + acc * BNACC, my_stage, my_res, tl & 1, row0, n0,
+            ok = epilogue_tile_staged<EPI_, BN>(p, &map_c, &map_w1, tmem_cta + lane_off + acc * BNACC, factor, my_stage, my_res, tl & 1, row0, n0,
                                            lane, turn, abort_flag);
             if (!ok) break;
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(5);   // its epilogue done (stores issued)
@@ -1122,22 +1283,23 @@ int resident_pairs(int dev, int* pairs) {
 }
 
 // CTA-pair kernel: clusters of two; returns RFK_EUNSUPPORTED (nothing launched) when the device cannot co-schedule pairs
-template <int EPI, int BN>
+template <int EPI_, int BN>
 int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, tcgemm::Params p, int dev,
                       cudaStream_t st, const CUtensorMap* heads_map) {
-    constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI, BN>;
+    constexpr int EPI = EPI_ & 7;
+    constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI_, BN>;
     // tile maps of the output (stores) and of the residual (loads): boxes of 32 rows x 64 columns, one per epilogue warp
     CUtensorMap mc, mr;
     if (heads_map) mc = *heads_map;
-    if ((!heads_map && !make_map_2d(&mc, p.C, p.M, p.N, p.ldc, 32)) ||
+    if ((!heads_map && !make_map_2d(&mc, p.C ? p.C : p.raster, p.M, p.N, p.ldc, p.grid.bw ? 16 : 32)) ||
         !make_map_2d(&mr, EPI == RFK_GEMM_EPI_RESIDUAL ? (const void*)p.R : (const void*)p.C, p.M, p.N,
                      EPI == RFK_GEMM_EPI_RESIDUAL ? p.ldr : p.ldc, 32))
         return RFK_EUNSUPPORTED;
     int pairs = 0;
-    const int rc = resident_pairs<EPI, BN>(dev, &pairs);
+    const int rc = resident_pairs<EPI_, BN>(dev, &pairs);
     if (rc != RFK_OK) return rc;
     cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = pair_config<EPI, BN>(attr, st);
+    cudaLaunchConfig_t cfg = pair_config<EPI_, BN>(attr, st);
     p.tiles_m = (p.M + 2 * tcgemm::BM - 1) / (2 * tcgemm::BM);
     if (BN != 256) p.tiles_n = (p.N + BN - 1) / BN;
     const int tiles = p.tiles_m * p.tiles_n;
@@ -1160,22 +1322,28 @@ bool narrow_tile(int M, int N, int pairs) {
 }
 
 // W (and W_up) as in launch_gemm, for the boxes of the tile width; the head-split form with row statistics needs 256 columns, one sum
-template <int EPI>
-int launch_gemm_pair(const CUtensorMap& ma, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev, cudaStream_t st,
-                     const CUtensorMap* heads_map = nullptr) {
+template <int EPI_>
+int launch_gemm_pair(const CUtensorMap& ma, const void* W, const void* W_up, long long ldw, tcgemm::Params p, int dev, cudaStream_t st,
+                     const CUtensorMap* heads_map = nullptr, const CUtensorMap* raster_map = nullptr, int* ss_tiles = nullptr) {
+    constexpr int EPI = EPI_ & 7;
+    constexpr bool FOLD = (EPI_ & tcgemm::kFold) != 0;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     CUtensorMap mw0, mw1;
     if constexpr (!kGate) {
-        if (!(EPI == tcgemm::kEpiHeads && p.row_ss)) {
+        if (FOLD || !(EPI == tcgemm::kEpiHeads && p.row_ss)) {
             int pairs = 0;
-            const int rc = resident_pairs<EPI, 192>(dev, &pairs);
+            const int rc = resident_pairs<EPI_, 192>(dev, &pairs);
             if (rc != RFK_OK) return rc;
-            if (narrow_tile(p.M, p.N, pairs))
-                return make_map_2d(&mw0, W, p.N, p.K, ldw, 96) ? launch_pair_tiles<EPI, 192>(ma, mw0, mw0, p, dev, st, heads_map) : RFK_EUNSUPPORTED;
+            // (a head-split tile with sums lies inside one part)
+            if (narrow_tile(p.M, p.N, pairs) && !(FOLD && EPI == tcgemm::kEpiHeads && p.row_ss && p.units * 64 != p.N)) {
+                if (FOLD) *ss_tiles = p.ss_tiles = p.N / 32;
+                return make_map_2d(&mw0, W, p.N, p.K, ldw, 96)
+                           ? launch_pair_tiles<EPI_, 192>(ma, mw0, raster_map ? *raster_map : mw0, p, dev, st, heads_map) : RFK_EUNSUPPORTED;
+            }
         }
     }
     if (!make_map_2d(&mw0, W, p.N, p.K, ldw) || (kGate && !make_map_2d(&mw1, W_up, p.N, p.K, ldw))) return RFK_EUNSUPPORTED;
-    return launch_pair_tiles<EPI, 256>(ma, mw0, kGate ? mw1 : mw0, p, dev, st, heads_map);
+    return launch_pair_tiles<EPI_, 256>(ma, mw0, kGate ? mw1 : raster_map ? *raster_map : mw0, p, dev, st, heads_map);
 }
 
 // rank-5 map of a head-split output: [part][group][head][seq][hd] halves, boxes of 32 rows x 64 columns
@@ -1221,9 +1389,11 @@ int heads_resident(int dev) {
     return n - 1;
 }
 
-template <int EPI, int BM_, int BN_>
+template <int EPI_, int BM_, int BN_>
 int launch_gemm_small(const void* A, long long lda, const void* W, const void* W_up, long long ldw, tcgemm::Params p, int dev,
                       cudaStream_t st) {
+    constexpr int EPI = EPI_ & 7;
+    constexpr bool FOLD = (EPI_ & tcgemm::kFold) != 0;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
     constexpr int smem = tcgemm::small::Cfg<BM_, BN_>::kSmemBytes;
@@ -1233,7 +1403,7 @@ int launch_gemm_small(const void* A, long long lda, const void* W, const void* W
     else if (!make_map_2d(&mw1, W_up, p.N, p.K, ldw, BN_OUT)) return RFK_EUNSUPPORTED;
     static std::atomic<bool> configured[64];
     if (!configured[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>,
+        cudaError_t e = cudaFuncSetAttribute(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured[dev].store(true, std::memory_order_release);
@@ -1241,8 +1411,8 @@ int launch_gemm_small(const void* A, long long lda, const void* W, const void* W
     p.tiles_m = (p.M + BM_ - 1) / BM_;
     p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
     const dim3 grid((unsigned)(p.tiles_m * p.tiles_n));
-    if (EPI != tcgemm::kEpiHeads) {
-        launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, grid, dim3(tcgemm::kThreads), smem, st, ma, mw0, mw1, p);
+    if (EPI != tcgemm::kEpiHeads || FOLD) {   // the sums of a folded form need no cluster
+        launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>, grid, dim3(tcgemm::kThreads), smem, st, ma, mw0, mw1, p);
         return launch_status();
     }
     cudaLaunchConfig_t cfg{};
@@ -1253,7 +1423,7 @@ int launch_gemm_small(const void* A, long long lda, const void* W, const void* W
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = grid; cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::small::gemm_tc_small_kernel<EPI, BM_, BN_>, ma, mw0, mw1, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>, ma, mw0, mw1, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
@@ -1397,6 +1567,86 @@ extern "C" int rfk_gemm_f16_heads(const rfk_half* A, long long lda, const rfk_ha
     return gemm_heads(A, lda, W, ldw, out, part_stride, row_ss, ss_parts_mask, M, N, K, seq_len, out_seq, num_heads, 64,
                       stream);
 }
+
+// 3-D map of a token grid in raster order, [height of all views][width][N] halves: boxes of 4 x 4 tokens x 64 columns
+static bool make_map_raster(CUtensorMap* m, const void* base, int n, int width, long long height) {
+    EncodeTiledFn enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)width, (cuuint64_t)height};
+    const cuuint64_t strides[2] = {(cuuint64_t)n * 2, (cuuint64_t)width * n * 2};
+    const cuuint32_t box[3] = {64, 4, 4}, estr[3] = {1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int EPI>
+static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cudaStream_t st, int* ss_tiles) {
+    constexpr int E = EPI | tcgemm::kFold;
+    constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    const int sums = (EPI == tcgemm::kEpiHeads ? p.units * 64 : p.N) / 32;
+    if (g_gemm_path.load(std::memory_order_relaxed) == 0) {
+        int rc = RFK_EUNSUPPORTED;
+        p.ss_tiles = sums;
+        *ss_tiles = sums;
+        switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
+            case 1: rc = launch_gemm_small<E, 64, 32>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
+            case 2: rc = launch_gemm_small<E, 64, 64>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
+            case 3: rc = launch_gemm_small<E, 128, 64>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
+            case 4: rc = launch_gemm_small<E, 128, 128>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
+        }
+        if (rc != RFK_EUNSUPPORTED) return rc;
+    }
+    p.ss_tiles = sums / 8;
+    *ss_tiles = sums / 8;
+    CUtensorMap ma, mh, mraster;
+    if (!make_map_2d(&ma, f.A, p.M, p.K, p.K)) return RFK_EUNSUPPORTED;
+    if (EPI == tcgemm::kEpiHeads &&
+        !make_map_heads(&mh, f.C, p.seq, p.seq, p.units / p.head_units, p.head_units * 64, p.M / p.seq, p.N / (p.units * 64), p.part_stride))
+        return RFK_EUNSUPPORTED;
+    if (p.raster && !make_map_raster(&mraster, p.raster, p.N, p.grid.bw * 4, p.M / (p.grid.bw * 4))) return RFK_EUNSUPPORTED;
+    return launch_gemm_pair<E>(ma, f.W, f.W_up, p.K, p, dev, st, EPI == tcgemm::kEpiHeads ? &mh : nullptr, p.raster ? &mraster : nullptr, ss_tiles);
+}
+
+int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream) {
+    const bool residual = f.R != nullptr, heads = f.num_heads > 0, gate = f.W_up != nullptr;
+    if (!f.A || !f.W || (!f.C && !f.raster) || f.M <= 0 || f.N <= 0 || f.K <= 0 || residual + heads + gate != 1 || !ss_tiles) return RFK_EINVAL;
+    if (!residual && (!f.in_ss || f.in_tiles <= 0)) return RFK_EINVAL;
+    const int path = g_gemm_path.load(std::memory_order_relaxed), dim = heads ? f.num_heads * f.head_dim : f.N;
+    if (path == 1 || path == 3) return RFK_EUNSUPPORTED;
+    if (f.M % 64 || f.K % 256 || f.N % dim || dim % 256) return RFK_EUNSUPPORTED;
+    if (!aligned16(f.A) || !aligned16(f.W) || !aligned16(f.W_up) || !aligned16(f.R) || !aligned16(f.C) || !aligned16(f.raster) ||
+        !aligned16(f.in_ss) || !aligned16(f.out_ss))
+        return RFK_EUNSUPPORTED;
+    if (!residual && f.in_tiles != f.K / 256 && f.in_tiles != f.K / 32) return RFK_EINVAL;
+    if (heads && ((f.head_dim != 64 && f.head_dim != 128) || f.seq <= 0 || f.seq % 32 || f.M % f.seq || (f.N > dim && f.part_stride < (long long)f.M * dim)))
+        return RFK_EUNSUPPORTED;
+    if (f.blocks_across && (!residual || f.blocks_across % 2 || f.blocks_down % 2 || f.blocks_down <= 0 || f.M % (f.blocks_across * f.blocks_down * 16)))
+        return RFK_EUNSUPPORTED;
+    if (!f.blocks_across && (f.raster || !f.C)) return RFK_EINVAL;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    tcgemm::Params p{};
+    p.C = (__half*)f.C; p.ldc = f.N; p.R = (const __half*)f.R; p.ldr = f.N;
+    p.M = f.M; p.N = f.N; p.K = f.K;
+    p.tiles_m = (f.M + tcgemm::BM - 1) / tcgemm::BM;
+    p.tiles_n = (f.N + (gate ? 128 : 256) - 1) / (gate ? 128 : 256);
+    p.in_ss = f.in_ss; p.in_tiles = f.in_tiles; p.in_group = f.in_tiles == f.K / 256 ? 1 : 8;
+    p.in_inv_dim = 1.0f / (float)f.K; p.in_eps = f.eps; p.in_mul = f.in_mul;
+    p.row_ss = f.out_ss;
+    p.raster = (__half*)f.raster;
+    p.grid = tcgemm::Grid{f.blocks_across, f.blocks_down, f.shift_from, f.shift_to};
+    if (heads) {
+        p.seq = p.out_seq = f.seq; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
+        p.part_stride = f.N > dim ? f.part_stride : (long long)f.M * dim;
+    }
+    const cudaStream_t st = as_stream(stream);
+    return gate ? launch_folded<RFK_GEMM_EPI_SWIGLU>(f, p, dev, st, ss_tiles)
+                : heads ? launch_folded<tcgemm::kEpiHeads>(f, p, dev, st, ss_tiles) : launch_folded<RFK_GEMM_EPI_RESIDUAL>(f, p, dev, st, ss_tiles);
+}
+
+extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream) { return f ? rfk::gemm_folded(*f, ss_tiles, stream) : RFK_EINVAL; }
 
 extern "C" int rfk_gemm_heads_tile(int M, int N, const int* resident) {
     return M > 0 && N > 0 && resident ? heads_tile(M, N, resident) : RFK_EINVAL;

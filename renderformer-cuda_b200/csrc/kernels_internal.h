@@ -11,6 +11,35 @@ int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ld
                float* row_ss, int ss_parts_mask, int M, int N, int K, int seq_len, int out_seq, int num_heads,
                int head_dim, rfk_stream_t stream);
 
+// Products of a layer whose norms are folded into them ("Folded norms" in gemm_tc.cu): A [M, K] un-normalised with its rows' sums of squares, W
+// [N, K] with the norm's weight multiplied in. One of: W_up (SwiGLU, C [M, N]), num_heads > 0 (head-split, C as gemm_heads'), R (C = R + A W^T).
+// out_ss (may be NULL; residual and head-split): the sums of squares of the rows written, *ss_tiles a row (of a part). A residual product's
+// rows may be the 4 x 4 blocks of a token grid in window order, of a grid shifted by shift_from blocks; they are then written in the order
+// of a grid shifted by shift_to blocks (C, with out_ss) and in raster order (raster), each where it is not NULL; C is then not R.
+// RFK_EUNSUPPORTED: shapes or a device that these kernels do not serve, nothing launched.
+struct FoldedProduct {
+    const rfk_half *A, *W, *W_up, *R;
+    rfk_half *C, *raster;
+    int M, N, K;
+    const float* in_ss; int in_tiles; float in_mul, eps;    // SwiGLU and head-split: a row's factor is in_mul / sqrt(mean square + eps)
+    float* out_ss; int ss_mask;                             // head-split: parts that get sums
+    long long part_stride; int seq, num_heads, head_dim;
+    int blocks_across, blocks_down, shift_from, shift_to;   // 0: rows stay where they are
+};
+int gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream);
+
+// The tokens that enter a view's folded layers, 1024 wide (else RFK_EUNSUPPORTED): x = half(half(rmsnorm(e) * gamma) + token), with the bits of the
+// separate steps, and its rows' sums of squares row_ss [rows][4]. e is a token grid in raster order, x in the block order of gemm_folded, of
+// the unshifted grid.
+int embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
+                 int blocks_across, int blocks_down, rfk_stream_t stream);
+
+// Weights for gemm_folded: out[i] = half(w[i] * gamma[i][column] * mul[i]) for up to 4 matrices [rows[i]][cols]; out[i] = the largest |gamma[i]|
+// of up to 96 vectors
+int fold_norm_weights(const rfk_half* const* w, rfk_half* const* out, const float* const* gamma, const float* mul, const int* rows, int n, int cols,
+                      rfk_stream_t stream);
+int largest_magnitudes(const float* const* gamma, int n, int dim, float* out, rfk_stream_t stream);
+
 // rfk_qkv_norm_rope_transpose behind gemm_heads: parts [heads][out_seq][head_dim], of which the first seq_len rows of each head are
 // normalised over the row (all heads) and, unless cos_vals is NULL, rotated in place, with that kernel's bits
 int qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* parts, const rfk_half* cos_vals,
@@ -21,11 +50,12 @@ int qk_norm_rope_heads(int n_parts, const float* const* gamma, rfk_half* const* 
 int norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c, float* out,
                   int rows, int dim, float eps, rfk_stream_t stream);
 
-// rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128
+// rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128. ss_group: how many of a row's sums make up 256
+// columns, 1 or 8 (gemm_folded). blocks: a window's tokens are its 4 x 4 blocks one after the other; the mask stays in row order
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                      const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
                      int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
-                     rfk_stream_t stream);
+                     rfk_stream_t stream, int ss_group = 1, bool blocks = false);
 
 // The same for heads of 128 with the bits of the separate steps: library Q K^T with the scale as its alpha,
 // rfk_swin_softmax_probs_inplace, library P V, rfk_transpose_bhsd_to_bsd
@@ -40,7 +70,7 @@ enum class AttnCut { kNone, kBelowOneRound, kLastRound };
 // rfk_flash_attention_ex for heads of 64 or 128
 int flash_attention_ex(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const float* q_row_ss, int ss_tiles,
                        int norm_dim, float eps, void* workspace, size_t workspace_bytes, AttnCut cut, int v_shared, int B, int H,
-                       int Sq, int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream);
+                       int Sq, int Sk, int n_keys, int D, int o_bshd, float scale, rfk_stream_t stream, int ss_group = 1);
 
 // the mma.sync kernel of rfk_flash_attention, whatever path is set
 int flash_attention_mma(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, int B, int H, int Sq, int Sk,
@@ -92,6 +122,10 @@ extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, con
 // y += r in fp16, and silu(y) beside it: rfk_residual_add and rfk_silu in one pass; n % 8 == 0, 16-byte aligned
 extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);
 
+extern "C" int rfk_embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
+                                int blocks_across, int blocks_down, rfk_stream_t stream);   // embed_tokens and fold_norm_weights, for their tests
+extern "C" int rfk_fold_norm_weights(const rfk_half* w, rfk_half* out, const float* gamma, float mul, int rows, int cols, rfk_stream_t stream);
+extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream);   // gemm_folded, for its test
 // rfk_rmsnorm_residual_f16_windows for operands that the kernels before have just written (the layers' case): the same values, another
 // split of the rows (one_warp_per_row in rmsnorm.cu)
 extern "C" int rfk_rmsnorm_residual_f16_windows_in_l2(rfk_half* x, const rfk_half* r, const float* gamma, rfk_half* y, int B, int H, int W,

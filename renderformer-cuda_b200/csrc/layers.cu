@@ -578,6 +578,66 @@ int rfk_layers::decoder_layer_impl(
     return RFK_OK;
 }
 
+// 1024 columns: four sums of squares a row, one 16-byte load, and CTAs of one row (embed_tokens); narrower rows leave less to gain than the launches that
+// are left, and keep their separate norms.
+bool rfk_layers::layer_folds(const rfk_decoder_layer_weights& w, int Sq, int dim, int num_heads, int ffn_hidden, int patch_h, int patch_w,
+                             int window_size, int shift_size) {
+    const auto given = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    return dim == 1024 && num_heads > 0 && (dim == num_heads * 64 || dim == num_heads * 128) && ffn_hidden > 0 && ffn_hidden % 256 == 0 &&
+           window_size == 8 && (shift_size == 0 || shift_size == 4) && patch_h > 0 && patch_w > 0 && patch_h % 8 == 0 && patch_w % 8 == 0 &&
+           Sq == patch_h * patch_w && given(w.query_norm_gamma) && given(w.self_attn_norm_gamma) && given(w.ffn_norm_gamma) &&
+           given(w.cross_attn.q_proj_w) && given(w.cross_attn.out_proj_w) && given(w.cross_attn.q_norm_gamma) && !w.cross_attn.q_proj_b &&
+           !w.cross_attn.out_proj_b && given(w.self_attn.in_proj_w) && given(w.self_attn.out_proj_w) && given(w.self_attn.q_norm_gamma) &&
+           given(w.self_attn.k_norm_gamma) && !w.self_attn.in_proj_b && !w.self_attn.out_proj_b && given(w.ffn.w1) && given(w.ffn.w2) && given(w.ffn.w3);
+}
+
+int rfk_layers::decoder_layer_folded(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const FoldedWeights& f, FoldedBuffers& b, rfk_half* x,
+                                     rfk_half* next, rfk_half* raster, const rfk_half* K_rotated, const rfk_half* V_cached, bool v_shared, int B,
+                                     int Sq, int Sk, int n_keys, int dim, int num_heads, int ffn_hidden, int patch_h, int patch_w, int shift,
+                                     int next_shift, const uint8_t* mask, rfk_stream_t stream) {
+    const int M = B * Sq, hd = dim / num_heads;
+    const auto group = [dim](int tiles) { return tiles == dim / 256 ? 1 : 8; };
+    rfk::FoldedProduct p{};
+    p.M = M;
+    p.eps = kEpsFp16;
+    const auto normed = [&](const rfk_half* W, float mul, rfk_half* C, int N) {   // a product behind a norm
+        rfk::FoldedProduct g = p;
+        g.A = x; g.W = W; g.C = C; g.N = N; g.K = dim; g.in_ss = b.x_ss; g.in_tiles = b.x_tiles; g.in_mul = mul;
+        return g;
+    };
+    const auto onto_x = [&](const rfk_half* A, const rfk_half* W, int K) {        // x += A W^T
+        rfk::FoldedProduct g = p;
+        g.A = A; g.W = W; g.R = x; g.C = x; g.N = dim; g.K = K; g.out_ss = b.x_ss;
+        return g;
+    };
+    int tiles = 0;
+    // cross-attention (its query norm stays deferred: attention applies 1 / rms, the rotated keys carry the weight; the cut along the keys: see cross_attention_impl)
+    rfk::FoldedProduct g = normed(f.q, f.mul_q, b.q, dim);
+    g.num_heads = num_heads; g.head_dim = hd; g.seq = Sq; g.out_ss = b.qk_ss; g.ss_mask = 1;
+    TRY(rfk::gemm_folded(g, &tiles, stream));
+    TRY(rfk::flash_attention_ex(b.q, K_rotated, V_cached, b.attn, b.qk_ss, tiles, dim, kEpsFp16, ctx->attn_ws, ctx->attn_ws_bytes,
+                                hd == 64 ? rfk::AttnCut::kBelowOneRound : rfk::AttnCut::kLastRound, v_shared, B, num_heads, Sq, Sk, n_keys, hd, 1,
+                                1.0f / sqrtf((float)hd), stream, group(tiles)));
+    TRY(rfk::gemm_folded(onto_x(b.attn, w->cross_attn.out_proj_w, dim), &b.x_tiles, stream));
+    // window attention
+    g = normed(f.in, f.mul_in, b.qkv, 3 * dim);
+    g.num_heads = num_heads; g.head_dim = hd; g.seq = 64; g.part_stride = (long long)M * dim; g.out_ss = b.qk_ss; g.ss_mask = 3;
+    TRY(rfk::gemm_folded(g, &tiles, stream));
+    const size_t part = (size_t)M * dim;
+    TRY(rfk::window_attention(b.qkv, b.qkv + part, b.qkv + 2 * part, b.attn, mask, b.qk_ss, b.qk_ss + (size_t)M * tiles, tiles, w->self_attn.q_norm_gamma,
+                              w->self_attn.k_norm_gamma, dim, kEpsFp16, M / 64, num_heads, 64, hd, Sq / 64, 1.0f / sqrtf((float)hd), stream,
+                              group(tiles), true));
+    TRY(rfk::gemm_folded(onto_x(b.attn, w->self_attn.out_proj_w, dim), &b.x_tiles, stream));
+    // FFN; its result leaves in the next layer's order
+    g = normed(f.w1, f.mul_ffn, b.act, ffn_hidden);
+    g.W_up = f.w3;
+    TRY(rfk::gemm_folded(g, &tiles, stream));
+    g = onto_x(b.act, w->ffn.w2, ffn_hidden);
+    g.C = next; g.raster = raster; g.out_ss = next ? b.x_ss : nullptr;
+    g.blocks_across = patch_w / 4; g.blocks_down = patch_h / 4; g.shift_from = shift / 4; g.shift_to = next_shift / 4;
+    return rfk::gemm_folded(g, &b.x_tiles, stream);
+}
+
 extern "C" int rfk_decoder_layer_forward_cached(
     rfk_ctx* ctx, const rfk_decoder_layer_weights* w, rfk_half* x, const rfk_half* pending_residual,
     const rfk_half** pending_out, rfk_half* temp, rfk_half* proj_buf, rfk_half* qkv_buf, rfk_half* ffn_buf,

@@ -33,6 +33,26 @@ int decoder_layer_impl(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const r
                        int patch_h, int patch_w, int window_size, int shift_size, const uint8_t* shift_mask,
                        const rfk_half* q_rope_cos, const rfk_half* q_rope_sin, const rfk_half* k_rope_cos,
                        const rfk_half* k_rope_sin, int cache_flags, rfk_stream_t stream);
+
+// A decoder layer whose norms are folded into its products (gemm_folded): eight launches instead of eleven. The token rows are the 4 x 4 blocks of
+// the grid in the window order of the layer's own shift; x is read there and, where next is not NULL, written in the order of shift
+// next_shift; raster (may be NULL): the result in raster order. The mask's tokens are in row order.
+struct FoldedWeights {
+    rfk_half *q, *in, *w1, *w3;        // the products' weights with the norms' multiplied in, times 1 / mul
+    float mul_q, mul_in, mul_ffn;      // powers of two
+};
+struct FoldedBuffers {                 // work space of a frame of M rows
+    rfk_half *attn, *q, *qkv, *act;    // [M, dim] twice, [3 M, dim] (q may lie in it), [M, ffn_hidden]
+    float *x_ss, *qk_ss;               // M * dim / 32 floats, and twice that
+    int x_tiles;                       // how many sums a row of x has, in and out
+};
+int decoder_layer_folded(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const FoldedWeights& f, FoldedBuffers& b, rfk_half* x, rfk_half* next,
+                         rfk_half* raster, const rfk_half* K_rotated, const rfk_half* V_cached, bool v_shared, int B, int Sq, int Sk, int n_keys,
+                         int dim, int num_heads, int ffn_hidden, int patch_h, int patch_w, int shift, int next_shift, const uint8_t* mask,
+                         rfk_stream_t stream);
+// whether it takes a layer of these sizes and weights
+bool layer_folds(const rfk_decoder_layer_weights& w, int Sq, int dim, int num_heads, int ffn_hidden, int patch_h, int patch_w, int window_size,
+                 int shift_size);
 }  // namespace rfk_layers
 
 // rfk_dpt_create, with every 3x3 convolution left to the library if library_only, for the tests that compare the two;

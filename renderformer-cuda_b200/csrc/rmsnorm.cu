@@ -192,6 +192,84 @@ norm_pair_add_kernel(const __half* __restrict__ a, const float* __restrict__ gam
     store8(out + (size_t)row * dim + off, o);
 }
 
+// The tokens that enter folded layers (gemm_folded), one CTA a row of 1024 (dim): norm, weight, token in one pass, with the bits of rmsnorm_row_kernel
+// and a broadcast add, the row's squares added as gemm_folded's epilogues do, and the row's place in block order. Three launches in one.
+__global__ void __launch_bounds__(kRmsThreads)
+embed_tokens_kernel(const __half* __restrict__ e, const float* __restrict__ gamma, const __half* __restrict__ token, __half* __restrict__ x,
+                    float* __restrict__ row_ss, int dim, float eps, int blocks_across, int blocks_down) {
+    constexpr int W = kRmsThreads / 32;
+    __shared__ float s_part[W];
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, off = threadIdx.x * 8;   // dim = 256 * W
+    float v[8], a[8], t[8], ss = 0.0f;
+    load8(e + (size_t)blockIdx.x * dim + off, v);
+    ldg_float8(gamma + off, a);
+    unpack8(ldg_half8(token + off), t);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+    ss = warp_sum(ss);
+    if (lane == 0) s_part[warp] = ss;
+    __syncthreads();
+    ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < W; ++i) ss += s_part[i];
+    const float rinv = rsqrtf(ss * (1.0f / (float)dim) + eps);
+    float c = 0.0f;   // eight squares in column order
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v[i] = round_half(round_half((v[i] * rinv) * a[i]) + t[i]);
+        c = fmaf(v[i], v[i], c);
+    }
+    const int across = blocks_across * 4, view_rows = across * blocks_down * 4, view = blockIdx.x / view_rows, r = blockIdx.x - view * view_rows;
+    const int y = r / across, z = r - y * across, by = y >> 2, bx = z >> 2;
+    const int row = view * view_rows + ((((by >> 1) * (blocks_across >> 1) + (bx >> 1)) << 2) + ((by & 1) << 1) + (bx & 1)) * 16 + (y & 3) * 4 + (z & 3);
+    store8(x + (size_t)row * dim + off, v);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);   // four of those in pairs
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    float sum = __shfl_sync(0xffffffffu, c, 0);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) sum += __shfl_sync(0xffffffffu, c, 4 * k);
+    if (lane == 0) row_ss[(size_t)row * W + warp] = sum;
+}
+
+// Weights of the folded products (gemm_folded): out = half(w * gamma[column] * mul), a matrix a blockIdx.y
+struct FoldMatrices {
+    const __half* w[4];
+    __half* out[4];
+    const float* gamma[4];
+    float mul[4];
+    int rows[4];
+};
+__global__ void __launch_bounds__(256)
+fold_weights_kernel(const __grid_constant__ FoldMatrices m, int cols) {
+    const int k = blockIdx.y;
+    const long long chunks = (long long)m.rows[k] * (cols / 8);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < chunks; i += (long long)gridDim.x * 256) {
+        float w[8], g[8];
+        unpack8(ldg_half8(m.w[k] + i * 8), w);
+        ldg_float8(m.gamma[k] + (i * 8) % cols, g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] *= g[j] * m.mul[k];
+        store8(m.out[k] + i * 8, w);
+    }
+}
+// the largest magnitude of each of n vectors
+struct GammaList { const float* gamma[96]; };
+__global__ void __launch_bounds__(256)
+largest_magnitude_kernel(const __grid_constant__ GammaList list, float* __restrict__ out, int dim) {
+    __shared__ float part[8];
+    float m = 0.0f;
+    for (int i = threadIdx.x; i < dim; i += 256) m = fmaxf(m, fabsf(list.gamma[blockIdx.x][i]));
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = fmaxf(m, part[w]);
+        out[blockIdx.x] = m;
+    }
+}
+
 // Any dim / any alignment: one CTA per row, scalar accesses, the row is re-read.
 template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
 __global__ void __launch_bounds__(256)
@@ -298,9 +376,51 @@ int norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, co
     return launch_status();
 }
 
+int embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
+                 int blocks_across, int blocks_down, rfk_stream_t stream) {
+    if (!e || !gamma || !token || !x || !row_ss || rows < 0 || blocks_across <= 0 || blocks_down <= 0) return RFK_EINVAL;
+    if (dim != 256 * (kRmsThreads / 32) || !aligned16(e) || !aligned16(gamma) || !aligned16(token) || !aligned16(x) || blocks_across % 2 ||
+        blocks_down % 2 || rows % (blocks_across * blocks_down * 16))
+        return RFK_EUNSUPPORTED;
+    if (rows == 0) return RFK_OK;
+    launch_pdl(embed_tokens_kernel, dim3(rows), dim3(kRmsThreads), 0, as_stream(stream), (const __half*)e, gamma, (const __half*)token, (__half*)x,
+               row_ss, dim, eps, blocks_across, blocks_down);
+    return launch_status();
+}
+
+int fold_norm_weights(const rfk_half* const* w, rfk_half* const* out, const float* const* gamma, const float* mul, const int* rows, int n, int cols,
+                      rfk_stream_t stream) {
+    if (!w || !out || !gamma || !mul || !rows || n < 1 || n > 4 || cols <= 0 || cols % 8) return RFK_EINVAL;
+    FoldMatrices m{};
+    for (int i = 0; i < n; ++i) {
+        if (!w[i] || !out[i] || !gamma[i] || rows[i] < 0) return RFK_EINVAL;
+        if (!aligned16(w[i]) || !aligned16(out[i]) || !aligned16(gamma[i])) return RFK_EUNSUPPORTED;
+        m.w[i] = (const __half*)w[i]; m.out[i] = (__half*)out[i]; m.gamma[i] = gamma[i]; m.mul[i] = mul[i]; m.rows[i] = rows[i];
+    }
+    fold_weights_kernel<<<dim3(2 * kNumSMs, n), 256, 0, as_stream(stream)>>>(m, cols);
+    return launch_status();
+}
+
+int largest_magnitudes(const float* const* gamma, int n, int dim, float* out, rfk_stream_t stream) {
+    if (!gamma || !out || n < 1 || n > 96 || dim <= 0) return RFK_EINVAL;
+    GammaList list{};
+    for (int i = 0; i < n; ++i) list.gamma[i] = gamma[i];
+    largest_magnitude_kernel<<<n, 256, 0, as_stream(stream)>>>(list, out, dim);
+    return launch_status();
+}
+
 }  // namespace rfk
 
 using namespace rfk;
+
+extern "C" int rfk_embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
+                                int blocks_across, int blocks_down, rfk_stream_t stream) {
+    return embed_tokens(e, gamma, token, x, row_ss, rows, dim, eps, blocks_across, blocks_down, stream);
+}
+
+extern "C" int rfk_fold_norm_weights(const rfk_half* w, rfk_half* out, const float* gamma, float mul, int rows, int cols, rfk_stream_t stream) {
+    return fold_norm_weights(&w, &out, &gamma, &mul, &rows, 1, cols, stream);
+}
 
 extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,
                                  float* out, int rows, int dim, float eps, rfk_stream_t stream) {

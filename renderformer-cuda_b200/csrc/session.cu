@@ -170,6 +170,12 @@ struct rfk_session {
     bool prescale = false;         // the rotation multiplies the keys by those weights (deferred Q-RMSNorm, see layers.cu)
     cudaEvent_t ev_fork = nullptr, ev_rot[RFK_MAX_LAYERS]{};
     uint8_t* shift_mask = nullptr;
+    // Views that end at the token map: the decoder with its norms folded into its products (decoder_layer_folded)
+    bool folded = false;
+    FoldedWeights fold[RFK_MAX_LAYERS] = {};
+    FoldedBuffers fbuf{};
+    rfk_half* x_other = nullptr;           // the residual stream's second buffer: a layer's last product reorders the rows
+    float* fold_max = nullptr;
     rfk_half* dft[kSlots][4] = {};  // the four decoder feature taps of each frame slot
     rfk_dpt_weights dptw{};          // copy of the model's DPT record (if any)
     rfk_dpt* dpt = nullptr;          // planned image head; null: the view ends at the token map
@@ -205,6 +211,7 @@ struct rfk_session {
         return RFK_OK;
     }
 
+    int fold_weights();
     int render_view(const float* pinned_cam, rfk_half* result_out, rfk_half* const* taps_out, float* image_out);
 };
 
@@ -251,15 +258,33 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
     for (int v = 0; v < V; ++v)
         TRY(rfk_ray_gen_patchify(id_c2w, cam_gpu + v * kCamStride + 16, nullptr, ray_pat + v * pat_n, 1, res, ps, s));
     const int rows = V * nP;
+    const int n_keys = (flags & RFK_SESSION_PAD_KEYS_ATTEND) ? Se_pad : Se;
+    const int L4 = std::max(1, m.dec_layers / 4);
+    if (folded) {
+        TRY(rfk_linear(ctx, ray_pat, m.ray_enc_w, m.ray_enc_b, x_other, rows, dim, 3 * ps * ps, s));
+        TRY(rfk::embed_tokens(x_other, m.ray_enc_norm, m.ray_map_patch_token, rtok, fbuf.x_ss, rows, dim, kEpsFp16, pW / 4, pH / 4, s));
+        fbuf.x_tiles = dim / 256;
+        rfk_half *x = rtok, *other = x_other, *out = nullptr;
+        for (int i = 0; i < m.dec_layers; ++i) {
+            const bool tap = ((i + 1) % L4 == 0) && ((i + 1) / L4 <= 4), last = i == m.dec_layers - 1;
+            const int shift = i % 2 == 1 ? m.shift_size : 0, next_shift = i % 2 == 0 ? m.shift_size : 0;
+            if (i < 2) TRY_CUDA(cudaStreamWaitEvent(stream, ev_rot[i], 0));
+            out = tap ? taps_out[(i + 1) / L4 - 1] : last ? result_out : nullptr;
+            TRY(decoder_layer_folded(ctx, &m.dec[i], fold[i], fbuf, x, last ? nullptr : other, out, kRot(i), kvV(i), V > 1, V, nP, Se_pad, n_keys,
+                                     dim, m.num_heads, m.ffn_hidden, pH, pW, shift, next_shift, shift > 0 ? shift_mask : nullptr, s));
+            std::swap(x, other);
+        }
+        if (out != result_out)
+            TRY_CUDA(cudaMemcpyAsync(result_out, out, (size_t)rows * dim * sizeof(rfk_half), cudaMemcpyDeviceToDevice, stream));
+        return RFK_OK;
+    }
     TRY(rfk_linear(ctx, ray_pat, m.ray_enc_w, m.ray_enc_b, rtok, rows, dim, 3 * ps * ps, s));
     TRY(rfk_rmsnorm(rtok, m.ray_enc_norm, rtok, rows, dim, kEpsFp16, s));
     TRY(rfk_broadcast_add(rtok, m.ray_map_patch_token, (long long)rows * dim, dim, s));
 
-    const int n_keys = (flags & RFK_SESSION_PAD_KEYS_ATTEND) ? Se_pad : Se;
     const rfk_half* pending = nullptr;
     // A tapped layer's last product writes the tap and the next layer reads it there; the token map that is also a tap is copied.
     const rfk_half* tokens = rtok;
-    const int L4 = std::max(1, m.dec_layers / 4);
     const int cache_flags = (prescale ? 1 : 0) | (V > 1 ? 2 : 0);  // keys rotated + weighted here; values shared by the views
     for (int i = 0; i < m.dec_layers; ++i) {
         const int shift = (i % 2 == 1) ? m.shift_size : 0;
@@ -281,6 +306,38 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
         // image head over this frame's taps, then ELU(1e-3) -> fp32 -> 10^x - 1 in one kernel (render_session.cu:239-253)
         TRY(rfk_dpt_forward(dpt, taps_out, nullptr, s));
         TRY(rfk_post_elu_pow10(rfk_dpt_output(dpt), image_out, (long long)V * dptw.out_dim * res * res, 1e-3f, s));
+    }
+    return RFK_OK;
+}
+
+// The weights of the folded products. The norms' weights are scaled by a power of two to below one first, so that a product of two stays in
+// fp16's range wherever the matrix was; the products' row factors take it back.
+int rfk_session::fold_weights() {
+    const int n = 3 * m.dec_layers, dim = m.dim;
+    std::vector<const float*> gamma(n);
+    for (int i = 0; i < m.dec_layers; ++i) {
+        gamma[3 * i] = m.dec[i].query_norm_gamma;
+        gamma[3 * i + 1] = m.dec[i].self_attn_norm_gamma;
+        gamma[3 * i + 2] = m.dec[i].ffn_norm_gamma;
+    }
+    TRY(rfk::largest_magnitudes(gamma.data(), n, dim, fold_max, (rfk_stream_t)stream));
+    std::vector<float> mul(n);
+    TRY_CUDA(cudaMemcpyAsync(mul.data(), fold_max, n * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    TRY_CUDA(cudaStreamSynchronize(stream));
+    for (float& v : mul) {
+        int e = 0;
+        if (std::isfinite(v) && v > 0.0f) std::frexp(v, &e);
+        v = std::ldexp(1.0f, std::min(std::max(e, -100), 100));
+    }
+    for (int i = 0; i < m.dec_layers; ++i) {
+        FoldedWeights& f = fold[i];
+        f.mul_q = mul[3 * i]; f.mul_in = mul[3 * i + 1]; f.mul_ffn = mul[3 * i + 2];
+        const rfk_half* w[4] = {m.dec[i].cross_attn.q_proj_w, m.dec[i].self_attn.in_proj_w, m.dec[i].ffn.w1, m.dec[i].ffn.w3};
+        rfk_half* out[4] = {f.q, f.in, f.w1, f.w3};
+        const float* g[4] = {gamma[3 * i], gamma[3 * i + 1], gamma[3 * i + 2], gamma[3 * i + 2]};
+        const float by[4] = {1.0f / f.mul_q, 1.0f / f.mul_in, 1.0f / f.mul_ffn, 1.0f / f.mul_ffn};
+        const int rows[4] = {dim, 3 * dim, m.ffn_hidden, m.ffn_hidden};
+        TRY(rfk::fold_norm_weights(w, out, g, by, rows, 4, dim, (rfk_stream_t)stream));
     }
     return RFK_OK;
 }
@@ -380,6 +437,25 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
             if (cudaMemcpy(d->q_gamma_all + (size_t)i * dim, model->dec[i].cross_attn.q_norm_gamma, (size_t)dim * sizeof(float),
                            cudaMemcpyDeviceToDevice) != cudaSuccess)
                 return fail((int)cudaGetLastError());
+    }
+    d->folded = d->prescale && !d->ctx->reproducible && 3 * model->dec_layers <= 96 &&
+                !((reinterpret_cast<uintptr_t>(model->ray_enc_norm) | reinterpret_cast<uintptr_t>(model->ray_map_patch_token)) & 15u);
+    for (int i = 0; i < model->dec_layers && d->folded; ++i)
+        d->folded = layer_folds(model->dec[i], nP, dim, nh, ffn, d->pH, d->pW, ws, model->shift_size);
+    if (d->folded) {
+        const size_t rows = V * nP, per_layer = (size_t)4 * dim * dim + (size_t)2 * ffn * dim;
+        rfk_half* weights = nullptr;
+        if ((rc = d->alloc(&weights, model->dec_layers * per_layer))) return fail(rc);
+        for (int i = 0; i < model->dec_layers; ++i, weights += per_layer)
+            d->fold[i] = FoldedWeights{weights, weights + (size_t)dim * dim, weights + (size_t)4 * dim * dim,
+                                       weights + (size_t)4 * dim * dim + (size_t)ffn * dim, 1.0f, 1.0f, 1.0f};
+        ALLOC(x_other, rows * dim);
+        ALLOC(fold_max, 3 * model->dec_layers);
+        ALLOC(fbuf.x_ss, rows * dim / 32);
+        ALLOC(fbuf.qk_ss, rows * dim / 16);
+        d->fbuf.attn = d->temp;
+        d->fbuf.q = d->fbuf.qkv = d->proj;
+        d->fbuf.act = d->qkv;
     }
     const bool fused_attention = d->hd == 64 || d->hd == 128;  // rfk_flash_attention serves these
     if (!fused_attention) ALLOC(score, V * nh * nP * Se_pad);
@@ -527,6 +603,7 @@ extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const 
         TRY(rfk_precompute_cross_kv(d->ctx, &m.dec[i].cross_attn, b.ctx_normed, d->kvK(i),
                                     d->kvV(i), b.kv_proj, 1, Se, Se_pad, dim, dim, nh, s));
     }
+    if (d->finalized && d->folded) TRY(d->fold_weights());   // should the weights be others now
     TRY_CUDA(cudaStreamSynchronize(st));
     TRY_CUDA(cudaGetLastError());
     return RFK_OK;
@@ -550,12 +627,19 @@ extern "C" int rfk_session_finalize(rfk_session* d) {
     const rfk_model& m = d->m;
     std::vector<uint8_t> mask = build_window_mask(d->pH, d->pW, m.window_size, m.shift_size);
     TRY_CUDA(cudaMemcpy(d->shift_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice));
+    if (d->folded) TRY(d->fold_weights());
     // warm-up view (also lets cuBLAS pick and load its kernels before capture)
     float cam[17] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 3, 0, 0, 0, 1, 0.7f};
     for (int k = 0; k < kSlots; ++k)
         for (int v = 0; v < d->V; ++v) memcpy(d->pin_cam[k] + v * kCamStride, cam, sizeof(cam));
     {
         int rc = d->render_view(d->pin_cam[0], d->result[0], d->dft[0], d->image[0]);
+        if (rc == RFK_EUNSUPPORTED && d->folded) {  // the kernels of the folded layers cannot run here: separate norms instead
+            TRY_CUDA(cudaStreamSynchronize(d->stream));
+            TRY_CUDA(cudaStreamSynchronize(d->side_stream));
+            d->folded = false;
+            rc = d->render_view(d->pin_cam[0], d->result[0], d->dft[0], d->image[0]);
+        }
         if (rc == RFK_EUNSUPPORTED && d->prescale && d->V == 1) {  // the kernels of the deferred norm cannot run here: separate norm instead
             TRY_CUDA(cudaStreamSynchronize(d->stream));
             TRY_CUDA(cudaStreamSynchronize(d->side_stream));
@@ -607,7 +691,14 @@ extern "C" int rfk_session_render_frames(rfk_session* d, const float* h_c2w, con
     }
     TRY_CUDA(cudaEventRecord(d->ev_start[k], d->stream));
     if (d->exec[k]) TRY_CUDA(cudaGraphLaunch(d->exec[k], d->stream));
-    else TRY(d->render_view(d->pin_cam[k], d->result[k], d->dft[k], d->image[k]));
+    else {
+        int rc = d->render_view(d->pin_cam[k], d->result[k], d->dft[k], d->image[k]);
+        if (rc == RFK_EUNSUPPORTED && d->folded) {   // the projections' kernels have been switched off since
+            d->folded = false;
+            rc = d->render_view(d->pin_cam[k], d->result[k], d->dft[k], d->image[k]);
+        }
+        TRY(rc);
+    }
     TRY_CUDA(cudaEventRecord(d->ev_done[k], d->stream));
     d->frames++;
     return RFK_OK;

@@ -1,0 +1,243 @@
+"""Products whose norms are folded into them: rows scaled by their sums of squares, sums written beside the output, rows put in the order of
+another shift or in raster order - on small tiles and CTA pairs, against fp32 torch on the same fp16 operands."""
+import ctypes
+
+import pytest
+import torch
+
+from renderformer_cuda_b200 import _abi
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -10
+
+
+class Product(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("A", "W", "W_up", "R", "C", "raster")] + [(n, ctypes.c_int) for n in ("M", "N", "K")] + [
+        ("in_ss", ctypes.c_void_p), ("in_tiles", ctypes.c_int), ("in_mul", ctypes.c_float), ("eps", ctypes.c_float), ("out_ss", ctypes.c_void_p),
+        ("ss_mask", ctypes.c_int), ("part_stride", ctypes.c_longlong)] + [
+        (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "blocks_across", "blocks_down", "shift_from", "shift_to")]
+
+
+def _run(path=0, **kw):
+    lib = _abi.load("rfk.h")
+    f = Product()
+    f.eps = EPS
+    for k, v in kw.items():
+        setattr(f, k, v.data_ptr() if torch.is_tensor(v) else v)
+    tiles = ctypes.c_int()
+    assert lib.rfk_gemm_set_path(path) == 0
+    try:
+        rc = lib.rfk_gemm_folded(ctypes.byref(f), ctypes.byref(tiles), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    finally:
+        lib.rfk_gemm_set_path(0)
+    assert rc == 0
+    code = ctypes.c_int()
+    assert lib.rfk_gemm_error(ctypes.byref(code), 0) == 0 and code.value == 0
+    return tiles.value
+
+
+def _gen(seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=g) * scale).half()
+
+
+def _near(got, want, terms):
+    # the output's rounding (2^-11 of the value), and fp32 sums of `terms` products in another order
+    tol = want.abs() * 2.0 ** -10 + 2.0 ** -24 * 8 * terms ** 0.5 * want.square().mean().sqrt() + 1e-6
+    assert ((got.float() - want).abs() <= tol).all(), float(((got.float() - want).abs() / tol).max())
+
+
+def _factor(x, mul):
+    return mul * torch.rsqrt(x.float().square().mean(-1, keepdim=True) + EPS)
+
+
+def _check_sums(ss, tiles, x, parts=1):
+    """ss [parts][M][tiles] against the squares of x [M, parts * dim]."""
+    dim = x.shape[1] // parts
+    got = ss.flatten()[: parts * x.shape[0] * tiles].view(parts, x.shape[0], tiles)
+    assert tiles in (dim // 256, dim // 32)
+    want = x.float().square().view(x.shape[0], parts, tiles, -1).sum(-1).permute(1, 0, 2)
+    assert torch.allclose(got, want, rtol=2e-5, atol=1e-6)
+
+
+# 64 rows: 64 x 32 tiles; 1024: 128 x 64; 2304: 128 x 128; 3136 and 5632: pairs of 192 and 256 columns; 4160: a tail of rows
+@pytest.mark.parametrize("M", [64, 256, 1024, 2304, 3136, 4096, 4160, 5632])
+@pytest.mark.parametrize("groups", [1, 8])
+def test_gate_of_scaled_rows(M, groups):
+    rnd = _gen(M)
+    K, N = 256, 512
+    x, w, u = rnd(M, K), rnd(N, K, scale=K ** -0.5), rnd(N, K, scale=K ** -0.5)
+    tiles = K // 256 if groups == 1 else K // 32
+    ss = x.float().square().view(M, tiles, -1).sum(-1).contiguous()
+    out = torch.empty(M, N, device="cuda", dtype=torch.half)
+    _run(A=x, W=w, W_up=u, C=out, M=M, N=N, K=K, in_ss=ss, in_tiles=tiles, in_mul=2.0)
+    f = _factor(x, 2.0)
+    a, b = (x.float() @ w.float().t()) * f, (x.float() @ u.float().t()) * f
+    want = torch.nn.functional.silu(a) * b
+    # the gate's exponential and reciprocal are approximate (2^-22 each), so is the factor's square root; a and b are fp32 sums whose rounding
+    # (some 1e-6 of their terms) the other one multiplies
+    tol = want.abs() * 2.0 ** -10 + 1e-5 * (1 + a.abs()) * (1 + b.abs())
+    assert ((out.float() - want).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("M,seq,parts,hd", [(64, 64, 1, 64), (256, 256, 1, 64), (256, 64, 3, 64), (1024, 512, 1, 128), (2304, 64, 3, 128), (3136, 3136, 1, 64),
+                                            (4096, 4096, 1, 128), (4160, 64, 3, 64)])
+@pytest.mark.parametrize("path", [0, 2])
+def test_heads_of_scaled_rows_with_sums(M, seq, parts, hd, path):
+    rnd = _gen(M + parts)
+    K, dim = 512, 512
+    heads, N = dim // hd, parts * dim
+    x, w = rnd(M, K), rnd(N, K, scale=K ** -0.5)
+    ss = x.float().square().view(M, K // 256, -1).sum(-1).contiguous()
+    out = torch.full((parts, M // seq, heads, seq, hd), float("nan"), device="cuda", dtype=torch.half)
+    sums = torch.full((parts * M * dim // 32,), float("nan"), device="cuda")
+    tiles = _run(path, A=x, W=w, C=out, M=M, N=N, K=K, in_ss=ss, in_tiles=K // 256, in_mul=1.0, out_ss=sums, ss_mask=(1 << parts) - 1,
+                 part_stride=M * dim, seq=seq, num_heads=heads, head_dim=hd)
+    got = out.permute(1, 3, 0, 2, 4).reshape(M, N)
+    _near(got, (x.float() @ w.float().t()) * _factor(x, 1.0), K)
+    _check_sums(sums, tiles, got, parts)
+
+
+def _to_blocks(grid, shift):
+    """[views, H, W, dim] -> rows: the 4 x 4 blocks in window order of the grid shifted by `shift` tokens."""
+    v, h, w, d = grid.shape
+    g = torch.roll(grid, (shift, shift), (1, 2)).view(v, h // 8, 2, 4, w // 8, 2, 4, d)
+    return g.permute(0, 1, 4, 2, 5, 3, 6, 7).reshape(v * h * w, d).contiguous()
+
+
+@pytest.mark.parametrize("views,h,w", [(1, 8, 8), (1, 16, 16), (2, 24, 16), (1, 40, 48), (1, 64, 64), (4, 32, 40)])
+@pytest.mark.parametrize("src,dst", [(0, 4), (4, 0), (0, 0)])
+@pytest.mark.parametrize("path", [0, 2])
+def test_residual_rows_go_to_another_shift_and_to_raster(views, h, w, src, dst, path):
+    rnd = _gen(h * w + src)
+    N, K = 256, 512
+    grid = rnd(views, h, w, N)
+    M = views * h * w
+    r, a, wt = _to_blocks(grid, src), rnd(M, K), rnd(N, K, scale=K ** -0.5)
+    out, raster = (torch.full((M, N), float("nan"), device="cuda", dtype=torch.half) for _ in range(2))
+    sums = torch.full((M * N // 32,), float("nan"), device="cuda")
+    args = dict(A=a, W=wt, R=r, M=M, N=N, K=K, blocks_across=w // 4, blocks_down=h // 4, shift_from=src // 4, shift_to=dst // 4)
+    tiles = _run(path, C=out, raster=raster, out_ss=sums, **args)
+    plain = torch.empty(M, N, device="cuda", dtype=torch.half)
+    _run(path, A=a, W=wt, R=r, C=plain, M=M, N=N, K=K)
+    _near(plain, r.float() + a.float() @ wt.float().t(), K)
+    # the same bits, elsewhere
+    back = _to_blocks(torch.arange(M, device="cuda", dtype=torch.float32).view(views, h, w, 1), src).long().flatten()   # raster row of each row
+    assert torch.equal(raster[back], plain)
+    assert torch.equal(out, _to_blocks(raster.view(views, h, w, N), dst))
+    _check_sums(sums, tiles, out)
+    alone = torch.empty_like(raster)
+    _run(path, C=None, raster=alone, **args)
+    assert torch.equal(alone, raster)
+
+
+def test_sums_have_the_same_bits_from_small_tiles_and_pairs():
+    rnd = _gen(5)
+    M, N, K = 1024, 1024, 512
+    a, w, r = rnd(M, K), rnd(N, K, scale=K ** -0.5), rnd(M, N)
+    res = []
+    for path in (0, 2):
+        out, sums = torch.empty(M, N, device="cuda", dtype=torch.half), torch.empty(M * N // 32, device="cuda")
+        tiles = _run(path, A=a, W=w, R=r, C=out, M=M, N=N, K=K, out_ss=sums)
+        s = sums[: M * tiles].view(M, tiles)
+        if tiles == N // 32:      # eight in order make 256 columns
+            t = s.view(M, N // 256, 8)
+            s = t[..., 0].clone()
+            for i in range(1, 8):
+                s += t[..., i]
+        res.append((out, s))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("views,h,w", [(1, 8, 8), (2, 24, 16), (1, 40, 48), (4, 64, 64)])
+def test_tokens_that_enter_folded_layers(views, h, w):
+    from renderformer_cuda_b200 import ops
+    rnd = _gen(h + w)
+    M, N = views * h * w, 1024
+    rows, norm, token = rnd(M, N), 1 + 0.1 * rnd(N).float(), rnd(N)
+    x, ss = torch.empty(M, N, device="cuda", dtype=torch.half), torch.empty(M, 4, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert _abi.load("rfk.h").rfk_embed_tokens(p(rows), p(norm), p(token), p(x), p(ss), M, N, ctypes.c_float(EPS), w // 4, h // 4,
+                                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want = rows.clone()
+    ops.rmsnorm(want, norm, want, M, N)
+    ops.broadcast_add(want, token, want.numel(), N)
+    assert torch.equal(x, _to_blocks(want.view(views, h, w, N), 0))
+    _check_sums(ss, 4, x)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (33, 264), (3072, 1024)])
+def test_folded_weights(rows, cols):
+    rnd = _gen(rows)
+    w, gamma = rnd(rows, cols), rnd(cols).float()
+    out = torch.empty_like(w)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert _abi.load("rfk.h").rfk_fold_norm_weights(p(w), p(out), p(gamma), ctypes.c_float(0.25), rows, cols,
+                                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert torch.equal(out, (w.float() * (gamma * 0.25)).half())
+
+
+def _scene(n, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    tri = (torch.rand(n, 3, 3, device="cuda", generator=g) * 2 - 1).contiguous()
+    vn = torch.nn.functional.normalize(torch.randn(n, 3, 3, device="cuda", generator=g), dim=-1).contiguous()
+    return tri, vn, torch.rand(n, 13, device="cuda", generator=g).half()
+
+
+def _view(model, scene, res, path=0, **kw):
+    from renderformer_cuda_b200 import session
+    c2w = torch.eye(4)
+    c2w[2, 3] = 3.0
+    s = session.RenderSession(model, scene[0].shape[0], res, **kw)
+    s.encode_scene(*scene)
+    lib = _abi.load("rfk.h")
+    try:
+        lib.rfk_gemm_set_path(path)
+        s.finalize()
+        s.render_frame(c2w, 0.7)
+        return s, s.download()
+    finally:
+        lib.rfk_gemm_set_path(0)
+
+
+@pytest.mark.parametrize("heads,res", [(16, 64), (8, 128), (16, 192)])
+@pytest.mark.parametrize("weights", [1.0, 2.0 ** -6, 37.0])
+def test_views_of_folded_and_separate_norms_agree(heads, res, weights):
+    """1024-wide rows, norm weights of several magnitudes: the folded layers, and with them switched off (the library's products). Twelve roundings
+    of 2^-11 and sums in other orders a layer apart."""
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=3, dim=1024, num_heads=heads, ffn_hidden=512, enc_layers=1, dec_layers=4)
+    for i in range(4):
+        for k in ("query_norm", "self_attn_norm", "ffn_norm"):
+            model.t[f"dec{i}.{k}"].mul_(weights)
+    scene = _scene(60, res)
+    s, got = _view(model, scene, res)
+    few = s.kernels_per_view
+    s.close()
+    s, want = _view(model, scene, res, path=1)
+    assert s.kernels_per_view != few
+    s.close()
+    assert torch.isfinite(got.float()).all()
+    assert (got.float() - want.float()).norm() <= 3e-3 * want.float().norm()
+
+
+def test_weights_changed_in_place_count_from_the_next_encoding():
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=3, dim=1024, num_heads=16, ffn_hidden=512, enc_layers=1, dec_layers=2)
+    scene = _scene(60, 1)
+    s, before = _view(model, scene, 64)
+    other = session.Model.random(seed=4, dim=1024, num_heads=16, ffn_hidden=512, enc_layers=1, dec_layers=2)
+    for k, t in model.t.items():   # all but the query norms of the cross-attention, which a session takes over when it is made
+        if k.endswith("cq_norm"):
+            other.t[k].copy_(t)
+        else:
+            t.copy_(other.t[k])
+    s.encode_scene(*scene)
+    c2w = torch.eye(4)
+    c2w[2, 3] = 3.0
+    s.render_frame(c2w, 0.7)
+    got = s.download().clone()
+    s.close()
+    f, want = _view(other, scene, 64)
+    f.close()
+    assert not torch.equal(before, want) and torch.equal(got, want)
