@@ -299,7 +299,6 @@ struct WinNorm {
     const float* q_ss; const float* k_ss;      // [rows][tiles] partial sums of squares (rows in window order)
     const float* gamma_q; const float* gamma_k;  // [heads * head_dim]
     int tiles; float inv_dim, eps;
-    int blocks;                                // the tokens are in blocks, the mask in rows
 };
 
 template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTokens * kWinTokens;
@@ -308,20 +307,21 @@ template <int HD> constexpr int kWinSmemBytes = 3 * kWinTokens * HD * 2 + kWinTo
 // kWinSteps: the arithmetic of the separate steps - scores rounded after the scale (the library product's alpha), the sums of
 // softmax_small_kernel (16 chunks of four columns, then a butterfly over the chunks) - so that the result has their bits; the
 // products need nothing, mma.sync and the library's kernels add K in the same order.
-enum WinForm { kWinFused, kWinNormed, kWinSteps };
+// kWinBlocks: kWinNormed for windows whose tokens are their 4 x 4 blocks one after the other; the mask is in row order.
+enum WinForm { kWinFused, kWinNormed, kWinSteps, kWinBlocks };
 
 // FOURS (kWinNormed): how many loads of four statistics make up a row's (dim 1024: 1, 2048: 2), or 0 for any number, one by one. The
 // statistics of the eight rows that a thread stages are then 8 or 16 loads instead of 32 or 64, all issued ahead of their use
 // (operands in L2 as behind the projection: 64 windows x 16 heads 9.1 -> 8.2 us, 256 x 16 39.3 -> 35.8, 4 x 16 4.3 -> 3.2, 64 x 32
 // 17.6 -> 15.7). A number that is not known to the compiler puts a loop between the loads: 9.1 us again, and the choice between the two
 // inside the kernel cost the others 2 %.
-constexpr int kWinEights = 8;   // FOURS: the row's sums in groups of eight (ss_group), summed once per CTA
+constexpr int kWinEights = 8;   // FOURS (kWinBlocks): the row's sums in groups of eight (ss_group), summed once per CTA
 template <WinForm FORM, int HD, int FOURS = 0>
 __global__ void __launch_bounds__(kWinThreads, HD == 64 ? 8 : 4)
 window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
                         __half* __restrict__ O, const uint8_t* __restrict__ mask, int heads, int nW, float scale,
                         const WinNorm nrm) {
-    constexpr bool NORMED = FORM == kWinNormed;
+    constexpr bool NORMED = FORM == kWinNormed || FORM == kWinBlocks;
     constexpr float kLog2e = 1.4426950408889634f;
     const float scale_log2e = scale * kLog2e;
     constexpr int CPR = HD / 8;   // 16-byte chunks per row
@@ -444,7 +444,7 @@ window_attention_kernel(const __half* __restrict__ Q, const __half* __restrict__
     }
     // scores in the exponent's units; masked-out pairs get -FLT_MAX (a fully masked row ends up uniform)
     const int q_lo = warp * 16 + g;  // this thread's rows: q_lo (regs 0, 1) and q_lo + 8 (regs 2, 3)
-    const bool blocks = FORM == kWinNormed && nrm.blocks;
+    constexpr bool blocks = FORM == kWinBlocks;
     // token t of a window in blocks -> its place in row order
     const auto in_rows = [](int t) { return (t & 32) | ((t & 12) << 1) | ((t & 16) >> 2) | (t & 3); };
     const uint8_t* m0 = sMask + (blocks ? in_rows(q_lo) : q_lo) * kWinTokens;
@@ -586,12 +586,14 @@ int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rf
         return (head_dim == 64 ? launch_window_attention<kWinFused, 64> : launch_window_attention<kWinFused, 128>)(
             q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, WinNorm{}, st);
     if (!aligned16(gamma_q) || !aligned16(gamma_k)) return RFK_EUNSUPPORTED;
-    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps, blocks};
-    if (ss_group == 8) {
-        if (!aligned16(q_row_ss) || !aligned16(k_row_ss) || ss_tiles % 8) return RFK_EUNSUPPORTED;
-        return (head_dim == 64 ? launch_window_attention<kWinNormed, 64, kWinEights> : launch_window_attention<kWinNormed, 128, kWinEights>)(
-            q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
+    const WinNorm nrm{q_row_ss, k_row_ss, gamma_q, gamma_k, ss_tiles, 1.0f / (float)norm_dim, eps};
+    if (blocks) {
+        if (!aligned16(q_row_ss) || !aligned16(k_row_ss) || (ss_group == 8 ? ss_tiles % 8 : ss_tiles != 4)) return RFK_EUNSUPPORTED;
+        const auto launch = head_dim == 64 ? (ss_group == 8 ? launch_window_attention<kWinBlocks, 64, kWinEights> : launch_window_attention<kWinBlocks, 64, 1>)
+                                           : (ss_group == 8 ? launch_window_attention<kWinBlocks, 128, kWinEights> : launch_window_attention<kWinBlocks, 128, 1>);
+        return launch(q, k, v, (__half*)O, mask, BnW, num_heads, nW, scale, nrm, st);
     }
+    if (ss_group != 1) return RFK_EUNSUPPORTED;
     const int fours = aligned16(q_row_ss) && aligned16(k_row_ss) && (ss_tiles == 4 || ss_tiles == 8) ? ss_tiles / 4 : 0;
     const auto launch = head_dim == 64 ? (fours == 1   ? launch_window_attention<kWinNormed, 64, 1>
                                           : fours == 2 ? launch_window_attention<kWinNormed, 64, 2>

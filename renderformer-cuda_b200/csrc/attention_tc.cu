@@ -341,7 +341,8 @@ __device__ __forceinline__ void store_row_half(__half* dst, const uint32_t (&v)[
 // order (mma.sync and tcgen05.mma add 16 products at a time, with the same bits, which the tests compare), the running maximum is
 // exact in both, so that whole units then have the bits of that kernel at a third of its time: 8 x 1600 x 4607 148 -> 62 us (one
 // block per CTA), 8 x 4096 x 5665 363 -> 105 us. It costs 2 %: the packed sums follow the register pairs of the exponents otherwise.
-template <int HD, int BLOCKS, bool ORDERED, bool HAND>
+// EIGHTS: a row's sums of squares come in groups of eight (ss_group). A form of its own: as a branch of the others it cost them 1 to 3 %.
+template <int HD, int BLOCKS, bool ORDERED, bool HAND, bool EIGHTS>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, __half* __restrict__ O, int H, int Sq, int n_keys,
@@ -589,13 +590,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         float scale_log2e = scale_log2e_all;
         if (row_ss) {
             const int q = min(q0 + blk * BM + r, Sq - 1);
-            const int sums = ss_tiles < 0 ? -ss_tiles : ss_tiles;
-            const float* sp = row_ss + ((size_t)(bh / H) * Sq + q) * sums;
+            const float* sp = row_ss + ((size_t)(bh / H) * Sq + q) * ss_tiles;
             float ss = 0.0f;
-            if (ss_tiles > 0) {
-                for (int t = 0; t < sums; ++t) ss += __ldg(sp + t);
-            } else {   // groups of eight (ss_group)
-                for (int t = 0; t < sums; t += 8) {
+            if constexpr (!EIGHTS) {
+                for (int t = 0; t < ss_tiles; ++t) ss += __ldg(sp + t);
+            } else {
+                for (int t = 0; t < ss_tiles; t += 8) {
                     const float4 a = __ldg(reinterpret_cast<const float4*>(sp + t)), b = __ldg(reinterpret_cast<const float4*>(sp + t + 4));
                     ss += ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
                 }
@@ -1046,11 +1046,11 @@ int attention_tc_handover_step(int word, int event, int* next) {
 }
 
 namespace {
-template <int HD, int BLOCKS, bool ORDERED, bool HAND>
+template <int HD, int BLOCKS, bool ORDERED, bool HAND, bool EIGHTS>
 int launch_units(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, __half* O, int H, int Sq, int n_keys, int o_bshd,
                  float scale, cudaStream_t st, const float* row_ss, int ss_tiles, int norm_dim, float norm_eps, void* ws, int v_heads,
                  const tcattn::WorkList& work, int dev) {
-    constexpr auto kernel = tcattn::attention_tc_kernel<HD, BLOCKS, ORDERED, HAND>;
+    constexpr auto kernel = tcattn::attention_tc_kernel<HD, BLOCKS, ORDERED, HAND, EIGHTS>;
     constexpr int smem = tcattn::Cfg<HD, BLOCKS>::kSmemBytes;
     // per-device "kernel attributes set" marks; setting them twice from racing threads is harmless
     static std::atomic<bool> configured[64];
@@ -1067,7 +1067,7 @@ int launch_units(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
     return launch_status();
 }
 
-template <int HD, bool ORDERED>
+template <int HD, bool ORDERED, bool EIGHTS>
 int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
               int n_keys, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
               int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared) {
@@ -1097,9 +1097,9 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
     if (one_block_per_cta(work.n_pieces, (long long)B * H * ceil_div(Sq, tcattn::BM), sms)) {
         work.q_blocks = ceil_div(Sq, tcattn::BM);
         work.whole_units = B * H * work.q_blocks;
-        return launch_units<HD, 1, ORDERED, false>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
+        return launch_units<HD, 1, ORDERED, false, EIGHTS>(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
     }
-    const auto launch = work.heads ? launch_units<HD, 2, ORDERED, true> : launch_units<HD, 2, ORDERED, false>;
+    const auto launch = work.heads ? launch_units<HD, 2, ORDERED, true, EIGHTS> : launch_units<HD, 2, ORDERED, false, EIGHTS>;
     return launch(mq, mk, mv, O, H, Sq, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, v_heads, work, dev);
 }
 }  // namespace
@@ -1110,11 +1110,10 @@ int launch_hd(const __half* Q, const __half* K, const __half* V, __half* O, int 
 int launch_attention_tc(const __half* Q, const __half* K, const __half* V, __half* O, int B, int H, int Sq, int Sk,
                         int n_keys, int D, int o_bshd, float scale, cudaStream_t st, const float* row_ss, int ss_tiles,
                         int norm_dim, float norm_eps, void* ws, size_t ws_bytes, AttnCut cut, int v_shared, int ss_group) {
-    if (ss_group == 8) {   // the kernel takes it as a negative number of sums
-        if (ss_tiles % 8 || !aligned16(row_ss)) return RFK_EUNSUPPORTED;
-        ss_tiles = -ss_tiles;
-    }
-    const auto launch = D == 64 ? launch_hd<64, false> : cut == AttnCut::kNone ? launch_hd<128, true> : launch_hd<128, false>;
+    if (ss_group == 8 && (ss_tiles % 8 || !aligned16(row_ss) || (D != 64 && cut == AttnCut::kNone))) return RFK_EUNSUPPORTED;
+    const auto launch = ss_group == 8 ? (D == 64 ? launch_hd<64, false, true> : launch_hd<128, false, true>)
+                        : D == 64     ? launch_hd<64, false, false>
+                        : cut == AttnCut::kNone ? launch_hd<128, true, false> : launch_hd<128, false, false>;
     return launch(Q, K, V, O, B, H, Sq, Sk, n_keys, o_bshd, scale, st, row_ss, ss_tiles, norm_dim, norm_eps, ws, ws_bytes, cut, v_shared);
 }
 

@@ -51,7 +51,8 @@ int norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, co
                   int rows, int dim, float eps, rfk_stream_t stream);
 
 // rfk_window_attention (q_row_ss NULL) / rfk_window_attention_normed for heads of 64 or 128. ss_group: how many of a row's sums make up 256
-// columns, 1 or 8 (gemm_folded). blocks: a window's tokens are its 4 x 4 blocks one after the other; the mask stays in row order
+// columns, 1 or 8 (gemm_folded). blocks (rows of 1024): a window's tokens are its 4 x 4 blocks one after the other, the mask stays in row
+// order; only that form takes groups of 8
 int window_attention(const rfk_half* Q, const rfk_half* K, const rfk_half* V, rfk_half* O, const uint8_t* mask,
                      const float* q_row_ss, const float* k_row_ss, int ss_tiles, const float* gamma_q, const float* gamma_k,
                      int norm_dim, float eps, int BnW, int num_heads, int window_tokens, int head_dim, int nW, float scale,
