@@ -117,6 +117,7 @@ struct Params {
     int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
     const float* in_ss; int in_tiles, in_group;    // kFold: A's rows' sums of squares, how many a row, and how many of them make up 256 columns
     float in_inv_dim, in_eps, in_mul;              // the row's factor: in_mul * rsqrt(sum * in_inv_dim + in_eps)
+    const float* part_mul;                         // kEpiHeads: if not null, another factor for each part
     int ss_tiles;                                  // kFold: sums a row that row_ss gets, of a part
     __half* raster;                                // kFold, residual: the rows in raster order too, or alone if C is null; pitch ldc
     Grid grid;
@@ -579,7 +580,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 rrow2 = p.raster + (at * (p.grid.bw * 4) + bx * 4 + (row & 3)) * p.ldc + n0;
             }
         }
-        const float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
+        float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
+        if (FOLD && EPI == kEpiHeads && p.part_mul) factor *= __ldg(p.part_mul + n0 / (p.units * 64));
         constexpr int kChunk = BN_OUT < 32 ? BN_OUT : 32;     // output columns per step
         uint4 res[EPI == RFK_GEMM_EPI_RESIDUAL ? BN_OUT / 8 : 1];
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                   // the row's residual arrives while the products run
@@ -1137,7 +1139,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
                 epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
-            const float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
+            float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
+            if (FOLD && EPI == kEpiHeads && p.part_mul) factor *= __ldg(p.part_mul + n0 / (p.units * kUnitCols));
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
@@ -1617,7 +1620,7 @@ static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cuda
     CUtensorMap ma, mh, mraster;
     if (!make_map_2d(&ma, f.A, p.M, p.K, p.K)) return RFK_EUNSUPPORTED;
     if (EPI == tcgemm::kEpiHeads &&
-        !make_map_heads(&mh, f.C, p.seq, p.seq, p.units / p.head_units, p.head_units * 64, p.M / p.seq, p.N / (p.units * 64), p.part_stride))
+        !make_map_heads(&mh, f.C, p.seq, p.out_seq, p.units / p.head_units, p.head_units * 64, p.M / p.seq, p.N / (p.units * 64), p.part_stride))
         return RFK_EUNSUPPORTED;
     if (p.raster && !make_map_raster(&mraster, p.raster, p.N, p.grid.bw * 4, p.M / (p.grid.bw * 4))) return RFK_EUNSUPPORTED;
     return launch_gemm_pair<E>(ma, f.W, f.W_up, p.K, p, dev, st, EPI == tcgemm::kEpiHeads ? &mh : nullptr, p.raster ? &mraster : nullptr, ss_tiles);
@@ -1629,12 +1632,13 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream)
     if (!residual && (!f.in_ss || f.in_tiles <= 0)) return RFK_EINVAL;
     const int path = g_gemm_path.load(std::memory_order_relaxed), dim = heads ? f.num_heads * f.head_dim : f.N;
     if (path == 1 || path == 3) return RFK_EUNSUPPORTED;
-    if (f.M % 64 || f.K % 256 || f.N % dim || dim % 256) return RFK_EUNSUPPORTED;
+    if ((f.M % 64 && !(heads && f.seq == f.M)) || f.K % 256 || f.N % dim || dim % 256) return RFK_EUNSUPPORTED;
     if (!aligned16(f.A) || !aligned16(f.W) || !aligned16(f.W_up) || !aligned16(f.R) || !aligned16(f.C) || !aligned16(f.raster) ||
         !aligned16(f.in_ss) || !aligned16(f.out_ss))
         return RFK_EUNSUPPORTED;
     if (!residual && f.in_tiles != f.K / 256 && f.in_tiles != f.K / 32) return RFK_EINVAL;
-    if (heads && ((f.head_dim != 64 && f.head_dim != 128) || f.seq <= 0 || f.seq % 32 || f.M % f.seq || (f.N > dim && f.part_stride < (long long)f.M * dim)))
+    if (heads && ((f.head_dim != 64 && f.head_dim != 128) || f.seq <= 0 || (f.seq % 32 && f.seq != f.M) || f.M % f.seq || (f.out_seq && (f.seq != f.M || f.out_seq < f.seq)) ||
+                  (f.N > dim && f.part_stride < (long long)f.M * dim) || f.part_stride % 8))
         return RFK_EUNSUPPORTED;
     if (f.blocks_across && (!residual || f.blocks_across % 2 || f.blocks_down % 2 || f.blocks_down <= 0 || f.M % (f.blocks_across * f.blocks_down * 16)))
         return RFK_EUNSUPPORTED;
@@ -1654,7 +1658,7 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream)
     p.raster = (__half*)f.raster;
     p.grid = tcgemm::Grid{f.blocks_across, f.blocks_down, f.shift_from, f.shift_to};
     if (heads) {
-        p.seq = p.out_seq = f.seq; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
+        p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.part_mul = f.part_mul; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
         p.part_stride = f.N > dim ? f.part_stride : (long long)f.M * dim;
     }
     const cudaStream_t st = as_stream(stream);

@@ -270,6 +270,102 @@ largest_magnitude_kernel(const __grid_constant__ GammaList list, float* __restri
     }
 }
 
+// y = half(x + r) and the sums of its squares, added as gemm_folded's epilogues do: a scene's context rows, one CTA a row of 1024 (5665 rows
+// 8.4 us, where the residual add and the cast took 16)
+__global__ void __launch_bounds__(kRmsThreads)
+context_rows_kernel(const float* __restrict__ x, const __half* __restrict__ r, __half* __restrict__ y, float* __restrict__ row_ss, int dim) {
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t at = (size_t)blockIdx.x * dim + threadIdx.x * 8;
+    float v[8], c = 0.0f;
+    ldcs_float8(x + at, v);
+    if (r) {
+        float a[8];
+        unpack8(ldcs_half8(r + at), a);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += a[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v[i] = round_half(v[i]);
+        c = fmaf(v[i], v[i], c);
+    }
+    store8(y + at, v);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    float sum = __shfl_sync(0xffffffffu, c, 0);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) sum += __shfl_sync(0xffffffffu, c, 4 * k);
+    if (lane == 0) row_ss[(size_t)blockIdx.x * (kRmsThreads / 32) + warp] = sum;
+}
+
+constexpr int kMaxKvLayers = 32;
+struct KvWeights {
+    const __half* w[2 * kMaxKvLayers];   // keys', values' of each layer
+    const float* gamma[kMaxKvLayers];
+};
+__global__ void __launch_bounds__(256)
+fold_kv_weights_kernel(const __grid_constant__ KvWeights m, __half* __restrict__ out, float* __restrict__ part_mul, int dim) {
+    __shared__ float s_max[8];
+    pdl_wait();
+    pdl_trigger();
+    const int part = blockIdx.y, tid = threadIdx.x;
+    const float* gamma = m.gamma[part >> 1];
+    float mx = 0.0f;
+    for (int i = tid; i < dim; i += 256) mx = fmaxf(mx, fabsf(gamma[i]));
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) mx = fmaxf(mx, s_max[w]);
+    const int e = (int)(__float_as_uint(mx) >> 23) + 1;   // biased exponent of the next power of two
+    const float scale = mx > 0.0f && e < 255 ? __uint_as_float((uint32_t)min(max(e, 27), 227) << 23) : 1.0f, mul = 1.0f / scale;
+    if (blockIdx.x == 0 && tid == 0) part_mul[part] = scale;
+    const int chunks = dim * (dim / 8);
+    const int col = (tid * 8) % dim;      // 256 threads walk whole rows of dim = 1024: a thread keeps its columns
+    float g[8];
+    ldg_float8(gamma + col, g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) g[i] *= mul;
+    __half* o = out + (size_t)part * dim * dim;
+#pragma unroll 4
+    for (int i = blockIdx.x * 256 + tid; i < chunks; i += gridDim.x * 256) {
+        float w[8];
+        unpack8(ldcs_half8(m.w[part] + (size_t)i * 8), w);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] *= g[j];
+        store8(o + (size_t)i * 8, w);
+    }
+}
+
+// Bound: HBM, each key once in and once out. A thread takes its chunk of a row in four heads, whose sum it reads once.
+struct KeyGammas { const float* gamma[kMaxKvLayers]; };
+__global__ void __launch_bounds__(128)
+keys_norm_kernel(__half* keys, long long layer_stride, const __grid_constant__ KeyGammas m, const float* __restrict__ row_ss, int rows, int out_seq,
+                 int num_heads, int head_dim, float inv_dim, float eps) {
+    constexpr int UN = 4;
+    pdl_wait();
+    pdl_trigger();
+    const int cpr = head_dim / 8, idx = blockIdx.x * 128 + threadIdx.x, s = idx / cpr, c = idx % cpr;
+    const int groups = num_heads / UN, layer = blockIdx.y / groups, h0 = (blockIdx.y % groups) * UN;
+    if (s >= rows) return;
+    __half* at = keys + (size_t)layer * layer_stride + ((size_t)h0 * out_seq + s) * head_dim + c * 8;
+    Half8 v[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) v[u] = ldcs_half8(at + (size_t)u * out_seq * head_dim);
+    const float4 a = __ldg(reinterpret_cast<const float4*>(row_ss) + (size_t)(2 * layer) * rows + s);
+    const float rinv = rsqrtf((((a.x + a.y) + a.z) + a.w) * inv_dim + eps);
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+        float f[8], g[8];
+        unpack8(v[u], f);
+        ldg_float8(m.gamma[layer] + (h0 + u) * head_dim + c * 8, g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = (f[i] * rinv) * g[i];
+        store8(at + (size_t)u * out_seq * head_dim, f);
+    }
+}
+
 // Any dim / any alignment: one CTA per row, scalar accesses, the row is re-read.
 template <typename TH, typename TR, typename TY, bool HAS_RES, bool WRITE_H>
 __global__ void __launch_bounds__(256)
@@ -385,6 +481,46 @@ int embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, r
     if (rows == 0) return RFK_OK;
     launch_pdl(embed_tokens_kernel, dim3(rows), dim3(kRmsThreads), 0, as_stream(stream), (const __half*)e, gamma, (const __half*)token, (__half*)x,
                row_ss, dim, eps, blocks_across, blocks_down);
+    return launch_status();
+}
+
+int context_rows(const float* x, const rfk_half* r, rfk_half* y, float* row_ss, int rows, int dim, rfk_stream_t stream) {
+    if (!x || !y || !row_ss || rows < 0) return RFK_EINVAL;
+    if (dim != 256 * (kRmsThreads / 32) || !aligned16(x) || !aligned16(r) || !aligned16(y)) return RFK_EUNSUPPORTED;
+    if (rows == 0) return RFK_OK;
+    launch_pdl(context_rows_kernel, dim3(rows), dim3(kRmsThreads), 0, as_stream(stream), x, (const __half*)r, (__half*)y, row_ss, dim);
+    return launch_status();
+}
+
+int fold_kv_weights(const rfk_half* const* k, const rfk_half* const* v, const float* const* gamma, rfk_half* out, float* part_mul, int layers, int dim,
+                    rfk_stream_t stream) {
+    if (!k || !v || !gamma || !out || !part_mul || layers <= 0) return RFK_EINVAL;
+    if (dim != 1024 || layers > kMaxKvLayers || !aligned16(out)) return RFK_EUNSUPPORTED;
+    KvWeights m{};
+    for (int i = 0; i < layers; ++i) {
+        if (!k[i] || !v[i] || !gamma[i]) return RFK_EINVAL;
+        if (!aligned16(k[i]) || !aligned16(v[i]) || !aligned16(gamma[i])) return RFK_EUNSUPPORTED;
+        m.w[2 * i] = (const __half*)k[i]; m.w[2 * i + 1] = (const __half*)v[i]; m.gamma[i] = gamma[i];
+    }
+    launch_pdl(fold_kv_weights_kernel, dim3(64, 2 * layers), dim3(256), 0, as_stream(stream), m, (__half*)out, part_mul, dim);
+    return launch_status();
+}
+
+int keys_norm(rfk_half* keys, long long layer_stride, const float* const* gamma, const float* row_ss, int layers, int rows, int out_seq, int num_heads,
+              int head_dim, float eps, rfk_stream_t stream) {
+    if (!keys || !gamma || !row_ss || layers <= 0 || rows < 0 || out_seq < rows || num_heads <= 0 || head_dim <= 0) return RFK_EINVAL;
+    if (num_heads * head_dim != 1024 || num_heads % 4 || head_dim % 8 || layers > kMaxKvLayers || !aligned16(keys) || layer_stride % 8 ||
+        !aligned16(row_ss))
+        return RFK_EUNSUPPORTED;
+    KeyGammas m{};
+    for (int i = 0; i < layers; ++i) {
+        if (!gamma[i]) return RFK_EINVAL;
+        if (!aligned16(gamma[i])) return RFK_EUNSUPPORTED;
+        m.gamma[i] = gamma[i];
+    }
+    if (rows == 0) return RFK_OK;
+    launch_pdl(keys_norm_kernel, dim3(ceil_div((long long)rows * (head_dim / 8), 128), layers * (num_heads / 4)), dim3(128), 0, as_stream(stream),
+               (__half*)keys, layer_stride, m, row_ss, rows, out_seq, num_heads, head_dim, 1.0f / (float)(num_heads * head_dim), eps);
     return launch_status();
 }
 

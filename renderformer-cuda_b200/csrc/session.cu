@@ -172,6 +172,7 @@ struct rfk_session {
     uint8_t* shift_mask = nullptr;
     // Views that end at the token map: the decoder with its norms folded into its products (decoder_layer_folded)
     bool folded = false;
+    bool folds_kv = false;                 // the keys and values of all layers from one product (see encode_kv)
     FoldedWeights fold[RFK_MAX_LAYERS] = {};
     FoldedBuffers fbuf{};
     rfk_half* x_other = nullptr;           // the residual stream's second buffer: a layer's last product reorders the rows
@@ -438,6 +439,13 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
                            cudaMemcpyDeviceToDevice) != cudaSuccess)
                 return fail((int)cudaGetLastError());
     }
+    d->folds_kv = !d->ctx->reproducible && dim == 1024 && nh % 4 == 0 && (d->hd == 64 || d->hd == 128) && model->dec_layers <= 16 &&
+                  (reinterpret_cast<uintptr_t>(scene_state) & 15u) == 0;
+    for (int i = 0; i < model->dec_layers && d->folds_kv; ++i) {
+        const auto given = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+        const rfk_cross_attn_weights& w = model->dec[i].cross_attn;
+        d->folds_kv = given(model->dec[i].kv_norm_gamma) && given(w.k_proj_w) && given(w.v_proj_w) && given(w.k_norm_gamma) && !w.k_proj_b && !w.v_proj_b;
+    }
     d->folded = d->prescale && !d->ctx->reproducible && 3 * model->dec_layers <= 96 &&
                 !((reinterpret_cast<uintptr_t>(model->ray_enc_norm) | reinterpret_cast<uintptr_t>(model->ray_map_patch_token)) & 15u);
     for (int i = 0; i < model->dec_layers && d->folded; ++i)
@@ -522,6 +530,7 @@ struct EncodeBuffers {
     float *vn_n, *tex_n;
     rfk_half *ctx16, *ctx_normed, *kv_proj;     // inside qkv, after it
     float *seq, *score;
+    rfk_half* kv_w; float *kv_mul, *kv_ss;      // folds_kv: the weights of all layers' keys and values, their scales; sums of squares, the context's last
     size_t plan(const rfk_session& d, char* base) {
         const rfk_model& m = d.m;
         const size_t Se = d.Se, N = d.N, dim = m.dim;
@@ -537,6 +546,12 @@ struct EncodeBuffers {
         c.get(&ffn, Se * std::max(dim, (size_t)m.ffn_hidden));
         score = nullptr;
         if (!(d.hd == 64 || d.hd == 128)) c.get(&score, (size_t)m.num_heads * Se * d.Se_pad);
+        kv_w = nullptr;
+        if (d.folds_kv) {
+            c.get(&kv_w, 2 * (size_t)m.dec_layers * dim * dim);
+            c.get(&kv_mul, 2 * m.dec_layers);
+            c.get(&kv_ss, (2 * (size_t)m.dec_layers + 1) * Se * 4);
+        }
         if (base) {
             const size_t piece = align_up(Se * dim, 128);   // halves, so that every piece is 256-byte aligned
             vn_emb16 = qkv;
@@ -550,6 +565,37 @@ struct EncodeBuffers {
         return c.used;
     }
 };
+
+// The cross-attention's keys and values of all decoder layers. They are 24 products of the same rows behind 12 norms that differ in their weights
+// alone: with those in the products' weights (folded anew each time, 96 MB of traffic) they are one product of 24576 columns, whose
+// tiles fill the SMs where 92 of one layer's left a third of them idle, stored head-split in the cache; then the keys' own norm in
+// place, all layers at once. 5633 triangles: 12 x 43 us (norm, product, transposing norm, product, two memsets) -> 280 (folding 21, product 190 = 1.5
+// PFLOP/s, norm 46, context rows 8), scenes of 60 triangles 735 -> 547 us in all, 1000 1275 -> 1106, 5633 5500 -> 5250. RFK_EUNSUPPORTED with nothing but work space written: layer by layer instead.
+static int encode_kv(rfk_session& d, EncodeBuffers& b, const float* ctx_ss) {
+    const rfk_model& m = d.m;
+    const rfk_stream_t s = (rfk_stream_t)d.stream;
+    const int layers = m.dec_layers, dim = m.dim, Se = d.Se, Se_pad = d.Se_pad, hd = d.hd;
+    const rfk_half *k[RFK_MAX_LAYERS], *v[RFK_MAX_LAYERS];
+    const float *gamma[RFK_MAX_LAYERS], *key_gamma[RFK_MAX_LAYERS];
+    for (int i = 0; i < layers; ++i) {
+        k[i] = m.dec[i].cross_attn.k_proj_w; v[i] = m.dec[i].cross_attn.v_proj_w;
+        gamma[i] = m.dec[i].kv_norm_gamma; key_gamma[i] = m.dec[i].cross_attn.k_norm_gamma;
+    }
+    TRY(rfk::fold_kv_weights(k, v, gamma, b.kv_w, b.kv_mul, layers, dim, s));
+    const long long slab = (long long)Se_pad * dim;
+    rfk::FoldedProduct p{};
+    p.A = b.ctx16; p.W = b.kv_w; p.C = d.kvK(0); p.M = Se; p.N = 2 * layers * dim; p.K = dim; p.in_ss = ctx_ss; p.in_tiles = dim / 256; p.in_mul = 1.0f;
+    p.eps = kEpsFp16; p.out_ss = b.kv_ss; p.ss_mask = 0x55555555; p.part_stride = slab; p.seq = Se; p.out_seq = Se_pad; p.num_heads = m.num_heads;
+    p.head_dim = hd; p.part_mul = b.kv_mul;
+    int tiles = 0;
+    TRY(rfk::gemm_folded(p, &tiles, s));
+    if (tiles != dim / 256) return RFK_EUNSUPPORTED;   // small tiles: not with this many columns
+    if (Se_pad != Se) {   // the rows behind the last key of each head
+        const size_t row = (size_t)hd * 2;
+        TRY_CUDA(cudaMemset2DAsync((char*)d.kvK(0) + Se * row, Se_pad * row, 0, (Se_pad - Se) * row, (size_t)2 * layers * m.num_heads, d.stream));
+    }
+    return rfk::keys_norm(d.kvK(0), 2 * slab, key_gamma, b.kv_ss, layers, Se, Se_pad, m.num_heads, hd, kEpsFp16, s);
+}
 
 extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const float* vn, const rfk_half* tex) {
     if (!d || !tri || !vn || !tex) return RFK_EINVAL;
@@ -591,14 +637,22 @@ extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const 
     const rfk_half* pending = nullptr;
     for (int i = 0; i < m.enc_layers; ++i) {
         const rfk_half* next = nullptr;
-        TRY(rfk_encoder_layer_forward_mixed(d->ctx, &m.enc[i], b.seq, pending, i + 1 < m.enc_layers ? &next : nullptr,
+        TRY(rfk_encoder_layer_forward_mixed(d->ctx, &m.enc[i], b.seq, pending, i + 1 < m.enc_layers || d->folds_kv ? &next : nullptr,
                                             b.temp, b.qkv, b.ffn, b.score, 1, Se, dim, nh, ffn, b.cos, b.sin, s));
         pending = next;
     }
     // context in fp16, then per decoder layer: kv-norm, K/V projections, padded head-major cache
     // (render_session.cu:377-416)
-    TRY(rfk_cast_fp32_to_fp16(b.seq, b.ctx16, (long long)Se * dim, s));
-    for (int i = 0; i < m.dec_layers; ++i) {
+    int kv = RFK_EUNSUPPORTED;
+    if (d->folds_kv) {
+        float* const ctx_ss = b.kv_ss + 2 * (size_t)m.dec_layers * Se * 4;
+        TRY(rfk::context_rows(b.seq, pending, b.ctx16, ctx_ss, Se, dim, s));
+        kv = encode_kv(*d, b, ctx_ss);
+        if (kv != RFK_OK && kv != RFK_EUNSUPPORTED) return kv;
+    } else {
+        TRY(rfk_cast_fp32_to_fp16(b.seq, b.ctx16, (long long)Se * dim, s));
+    }
+    for (int i = 0; kv != RFK_OK && i < m.dec_layers; ++i) {
         TRY(rfk_rmsnorm(b.ctx16, m.dec[i].kv_norm_gamma, b.ctx_normed, Se, dim, kEpsFp16, s));
         TRY(rfk_precompute_cross_kv(d->ctx, &m.dec[i].cross_attn, b.ctx_normed, d->kvK(i),
                                     d->kvV(i), b.kv_proj, 1, Se, Se_pad, dim, dim, nh, s));

@@ -15,7 +15,8 @@ class Product(ctypes.Structure):
     _fields_ = [(n, ctypes.c_void_p) for n in ("A", "W", "W_up", "R", "C", "raster")] + [(n, ctypes.c_int) for n in ("M", "N", "K")] + [
         ("in_ss", ctypes.c_void_p), ("in_tiles", ctypes.c_int), ("in_mul", ctypes.c_float), ("eps", ctypes.c_float), ("out_ss", ctypes.c_void_p),
         ("ss_mask", ctypes.c_int), ("part_stride", ctypes.c_longlong)] + [
-        (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "blocks_across", "blocks_down", "shift_from", "shift_to")]
+        (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "out_seq")] + [("part_mul", ctypes.c_void_p)] + [
+        (n, ctypes.c_int) for n in ("blocks_across", "blocks_down", "shift_from", "shift_to")]
 
 
 def _run(path=0, **kw):
@@ -241,3 +242,49 @@ def test_weights_changed_in_place_count_from_the_next_encoding():
     f, want = _view(other, scene, 64)
     f.close()
     assert not torch.equal(before, want) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M,pad,parts,hd", [(1, 8, 4, 64), (333, 336, 24, 128), (777, 784, 6, 64), (2665, 2672, 8, 64)])
+@pytest.mark.parametrize("path", [0, 2])
+def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts, hd, path):
+    """The keys and values of several layers: any number of rows, heads with room for more, each part its own factor, sums for every other one."""
+    rnd = _gen(M)
+    K = dim = 1024
+    heads, N = dim // hd, parts * dim
+    x, w = rnd(M, K), rnd(N, K, scale=K ** -0.5)
+    ss = x.float().square().view(M, 4, -1).sum(-1).contiguous()
+    mul = 2.0 ** -(torch.arange(parts, device="cuda") % 5).float()
+    out = torch.full((parts, heads, pad, hd), 7.0, device="cuda", dtype=torch.half)
+    sums = torch.full((parts * M * dim // 32,), float("nan"), device="cuda")
+    tiles = _run(path, A=x, W=w, C=out, M=M, N=N, K=K, in_ss=ss, in_tiles=4, in_mul=1.0, out_ss=sums, ss_mask=0x55555555, part_stride=dim * pad, seq=M,
+                 num_heads=heads, head_dim=hd, out_seq=pad, part_mul=mul)
+    assert (out[:, :, M:] == 7.0).all()
+    got = out[:, :, :M].permute(2, 0, 1, 3).reshape(M, N)
+    factor = _factor(x, 1.0)
+    for i in range(parts):
+        cols = slice(i * dim, (i + 1) * dim)
+        _near(got[:, cols], (x.float() @ w[cols].float().t()) * factor * mul[i], K)
+    s = sums[: parts * M * tiles].view(parts, M, tiles)
+    assert s[1::2].isnan().all()
+    want = got.float().square().view(M, parts, tiles, -1).sum(-1).permute(1, 0, 2)
+    assert torch.allclose(s[0::2], want[0::2], rtol=2e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("n,heads,layers", [(1, 16, 1), (60, 16, 3), (333, 8, 12), (1100, 16, 12), (2600, 8, 2)])
+def test_cache_of_all_layers_at_once_and_layer_by_layer(n, heads, layers):
+    """1024-wide rows: sessions with an image head keep one norm, two products and a transposing norm a layer; sessions without take one product."""
+    from renderformer_cuda_b200 import session
+    model = lambda dpt: session.Model.random(seed=6, dim=1024, num_heads=heads, ffn_hidden=256, enc_layers=1, dec_layers=layers, with_dpt=dpt,
+                                             dpt_features=64, dpt_out_channels=(32, 64, 128, 128))
+    scene, keys = _scene(n, n), (32 + n + 7) // 8 * 8
+    states = []
+    for dpt in (False, True):
+        s = session.RenderSession(model(dpt), n, 64)
+        for _ in range(2):   # the second time into what the first one left
+            s.encode_scene(*scene)
+        states.append(s.scene_state[: 2 * layers * keys * 1024 * 2].clone().view(torch.half).view(2 * layers, heads, keys, 1024 // heads))
+        s.close()
+    got, want = states
+    assert (got[:, :, 32 + n:] == 0).all() and torch.isfinite(got).all()
+    for i in range(2 * layers):   # (the encoder's attention may be cut along its keys without an image head)
+        assert (got[i].float() - want[i].float()).norm() <= 1.5e-3 * want[i].float().norm()
