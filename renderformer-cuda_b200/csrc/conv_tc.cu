@@ -33,24 +33,43 @@ __device__ int g_conv_tc_error = 0;  // first time-out / failure code seen by an
 namespace tcconv {
 using namespace pair_ptx;
 
-constexpr int BM = 128, BK = 64, kBoxX = 16, kBoxY = 8;
-static_assert(kBoxX * kBoxY == BM, "a CTA's rows are one box of pixels");
+constexpr int BK = 64, kBoxY = 8;
 constexpr int kThreads = 192;                    // warp 0 producer, warp 1 issuer of the products, warps 2-5 epilogue
-constexpr int kTmemCols = 512;                   // all of it: both CTAs of a pair then have the same addresses
-constexpr int kABytes = BM * BK * 2;             // 16 KB
-constexpr int kUnitBytes = 32 * 64 * 2;          // one epilogue warp's 32 pixels x 64 channels, 4 KB
-template <int BN> struct Cfg {
-    static constexpr int kWBytes = BN / 2 * BK * 2;          // this CTA's half of the weight tile
-    static constexpr int kStageBytes = kABytes + kWBytes;
-    static constexpr int kUnits = BN / 64;                   // 64-channel units per tile, one staging buffer each
+constexpr int kResidentBlocks = 2;               // blocks of 64 input channels whose weights fit beside the boxes (32 output channels)
+constexpr int kColBytes = kBoxY * BK * 2;        // a column of 8 pixels: one 8-row group of the tensor core's layout
+static_assert(kColBytes == 1024, "a tap's operand starts on the swizzle's period");
+
+// BN output channels x a box of BX x 8 pixels per CTA
+template <int BN, int BX> struct Cfg {
+    static constexpr int kRows = BX * kBoxY;
+    static_assert(kRows == 128 || (kRows == 64 && BN == 64), "the tensor core's tiles of a pair that are used here");
+    static constexpr int kHaloBytes = (BX + 2) * kColBytes;  // the box with a column of pixels on either side
+    // The ring's stages hold a halo box and the weights of its three taps, so that one barrier serves three K blocks. kResident: boxes
+    // alone, the weights come once, ahead of the first tile.
+    static constexpr bool kResident = BN == 32;
+    static constexpr int kWBytes = BN / 2 * BK * 2;          // this CTA's half of a tap's weights
+    static constexpr int kStages = BN == 128 ? 4 : BN == 32 ? 9 : kRows == 64 ? 4 : 3;
+    static constexpr int kWTiles = kResident ? 9 * kResidentBlocks : 3 * kStages;
+    static constexpr int kStageTx = 2 * (kHaloBytes + (kResident ? 0 : 3 * kWBytes));   // what a stage's barrier counts, of both CTAs
+    // An accumulator: a row's channels in the lane of that row, or, with 64 rows, the second half of them in the lane 64 further
+    static constexpr int kAccCols = kRows == 64 ? BN / 2 : BN;
+    static constexpr int kUnitCh = kAccCols < 64 ? kAccCols : 64;   // the epilogue's units: 32 pixels x kUnitCh channels, a staging buffer each
+    static constexpr int kUnitBytes = 32 * kUnitCh * 2;
+    static constexpr int kUnits = kAccCols / kUnitCh;
     static constexpr int kStagingBytes = 4 * kUnits * kUnitBytes;
-    static constexpr int kStages = BN == 256 ? 5 : 7;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 512;
-    static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
+    static constexpr int kSmemBytes = kStages * kHaloBytes + kWTiles * kWBytes + kStagingBytes + 512;
+    static constexpr int kCtas = BN == 64 ? 2 : 1;           // of an SM
+    static_assert(kCtas * (kSmemBytes + 1024) <= 227 * 1024 && kCtas * 2 * kAccCols <= 512, "shared and tensor memory of an SM");
+    // 16-byte chunk j of pixel r in a staging buffer, in the copy engine's swizzled layout (128-byte rows, or 64-byte ones)
+    static __device__ __forceinline__ uint32_t chunk(int r, int j) {
+        return kUnitCh == 64 ? staged(r, j) : (uint32_t)(r * 64 + ((j ^ ((r >> 1) & 3)) << 4));
+    }
 };
 
 struct __align__(8) Ctrl {
-    uint64_t full[7], empty[7], acc_full[2], acc_empty[2], drain;
+    uint64_t full[9], empty[9];
+    uint64_t weights;          // kResident: all of them have landed; one phase
+    uint64_t acc_full[2], acc_empty[2], drain;
     uint64_t started;          // one phase only: the products of the CTA's first K block are complete
     uint64_t res_full[4][4];   // [epilogue warp][unit]: that unit's residual box has landed
     uint32_t tmem_base;
@@ -64,23 +83,32 @@ struct Params {
     const __half* bias;
     int tiles, tiles_x, tiles_img;    // boxes in all images, per row of an image, per image
     int tiles_m, tiles_n;             // pairs of boxes, blocks of BN output channels
-    int c_in, cb;                     // input channels, blocks of 64 of them
+    int cb, c_out;                    // blocks of 64 input channels; output channels
     int rows_outside, silu, has_res, dual;
 };
 
+// boxes of pixels: the maps have the columns' pixels (y) ahead of the rows' (x), see make_map_pixels
 __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* map, int c, int x, int y, int n, uint32_t cluster_bar) {
     asm volatile(
         "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-        ::"r"(dst), "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(cluster_bar) : "memory");
+        ::"r"(dst), "l"(map), "r"(c), "r"(y), "r"(x), "r"(n), "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* map, int c, int n, int tap, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(c), "r"(n), "r"(tap), "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_3d(const void* map, int c, int n, int tap) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(c), "r"(n), "r"(tap) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int c, int x, int y, int n, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-        ::"r"(dst), "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(tc::smem_addr(bar)) : "memory");
+        ::"r"(dst), "l"(map), "r"(c), "r"(y), "r"(x), "r"(n), "r"(tc::smem_addr(bar)) : "memory");
 }
 __device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int c, int x, int y, int n) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                 ::"l"(map), "r"(src), "r"(c), "r"(x), "r"(y), "r"(n) : "memory");
+                 ::"l"(map), "r"(src), "r"(c), "r"(y), "r"(x), "r"(n) : "memory");
 }
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     __half2 h = __floats2half2_rn(lo, hi);
@@ -89,32 +117,40 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 __device__ __forceinline__ float2 unpack_half2(uint32_t w) { return __half22float2(*reinterpret_cast<__half2*>(&w)); }
 
 struct Box { int x, y, n; };   // first pixel of a CTA's box, and its image
-__device__ __forceinline__ Box box_of(const Params& p, int tile) {
+template <int BX> __device__ __forceinline__ Box box_of(const Params& p, int tile) {
     const int n = tile / p.tiles_img, r = tile - n * p.tiles_img, ty = r / p.tiles_x;
-    return {(r - ty * p.tiles_x) * kBoxX, ty * kBoxY, n};
+    return {(r - ty * p.tiles_x) * BX, ty * kBoxY, n};
 }
 
-template <int BN>
-__global__ void __launch_bounds__(kThreads, 1)
+// from one box's block of input channels and row of taps to the next one's
+__device__ __forceinline__ void step(const Params& p, int& c, int& ty) {
+    if (p.rows_outside) { if (++c == p.cb) { c = 0; ++ty; } }
+    else if (++ty == 3) { ty = 0; ++c; }
+}
+
+template <int BN, int BX>
+__global__ void __launch_bounds__(kThreads, (Cfg<BN, BX>::kCtas))
 conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r,
                     const __grid_constant__ CUtensorMap map_s, const Params p) {
-    using C = Cfg<BN>;
-    constexpr int kStages = C::kStages, kUnits = C::kUnits;
+    using C = Cfg<BN, BX>;
+    constexpr int kStages = C::kStages, kUnits = C::kUnits, kUnitBytes = C::kUnitBytes, kUnitCh = C::kUnitCh, kTmemCols = 2 * C::kAccCols < 32 ? 32 : 2 * C::kAccCols;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = tc::smem_addr(smem_raw);
     const uint32_t rank = cluster_rank();            // 0: issues the products for the pair; 1: its peer
-    unsigned char* staging = smem_raw + kStages * C::kStageBytes;
+    const uint32_t base_w = base + kStages * C::kHaloBytes;
+    unsigned char* staging = smem_raw + kStages * C::kHaloBytes + C::kWTiles * C::kWBytes;
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(staging + C::kStagingBytes);
     volatile int* abort_flag = &ctrl->abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int num_kb = 9 * p.cb;
+    const int num_boxes = 3 * p.cb;                  // halo boxes a tile: one for each row of taps and block of 64 input channels
     const int num_tiles = p.tiles_m * p.tiles_n;
     const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
     const bool aligned = (base & 1023u) == 0;        // the same in both CTAs (same kernel, same shared-memory layout)
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
+        tc::mbar_init(&ctrl->weights, 1);
         for (int a = 0; a < 2; ++a) { tc::mbar_init(&ctrl->acc_full[a], 1); tc::mbar_init(&ctrl->acc_empty[a], 8); }
         tc::mbar_init(&ctrl->drain, 1);
         tc::mbar_init(&ctrl->started, 1);
@@ -140,6 +176,13 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         return;
     }
     const uint32_t tmem_cta = ctrl->tmem_base;
+    // The weights on their way into L2 while the kernel before still runs: of a tile's boxes each pair that reads the same weights asks
+    // for its share. (A hint: what is copied below is read after the wait.)
+    if (warp == 0 && tc::elect_one()) {
+        const int nw = (first_tile / p.tiles_m) * BN + (int)rank * (BN / 2), sharing = min(p.tiles_m, tile_step);
+        for (int i = first_tile % p.tiles_m; i < num_boxes; i += sharing) tma_prefetch_3d(&map_w, i / 3 * BK, nw, i % 3 * 3);
+    }
+    __syncwarp();
     pdl_wait();      // set-up above is on-chip only; the operands are another kernel's output
     pdl_trigger();
 
@@ -148,28 +191,28 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const bool leader = tc::elect_one();
         int s = 0, par = 1, filled = 0;   // stage, parity of its previous phase, stages filled once
         bool ok = true;
+        if (C::kResident && leader && first_tile < num_tiles) {
+            const uint32_t full0 = map_to_cta(tc::smem_addr(&ctrl->weights), 0);
+            if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->weights, 2 * 9 * p.cb * C::kWBytes);
+            for (int i = 0; i < 3 * p.cb; ++i) tma_load_3d_pair(base_w + i * 3 * C::kWBytes, &map_w, i / 3 * BK, rank * (BN / 2), i % 3 * 3, full0);
+        }
         for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
-            const Box b = box_of(p, 2 * (t % p.tiles_m) + (int)rank);   // a box beyond the last one reads as zeros
-            const int nw = (t / p.tiles_m) * BN + (int)rank * (BN / 2);
-            int c = 0, ty = 0, tx = 0;    // channel block and tap of the K block
-            for (int kb = 0; kb < num_kb; ++kb) {
+            const Box b = box_of<BX>(p, 2 * (t % p.tiles_m) + (int)rank);   // a box beyond the last one reads as zeros
+            const int nw = (t / p.tiles_m) * BN + (int)rank * (BN / 2);      // channels beyond the last one too
+            int c = 0, ty = 0;            // channel block and row of taps of the box
+            for (int i = 0; i < num_boxes; ++i) {
                 if (filled == kStages) ok = tc::mbar_wait_warp(&ctrl->empty[s], par, abort_flag);
                 else ++filled;
                 if (!ok) break;
                 if (leader) {
-                    const uint32_t sA = base + s * C::kStageBytes;
                     const uint32_t full0 = map_to_cta(tc::smem_addr(&ctrl->full[s]), 0);
                     // CTA 0 announces the bytes of both CTAs' copies on its own barrier; CTA 1's may land before that: the phase
                     // cannot complete without the announcement's arrival
-                    if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->full[s], 2 * C::kStageBytes);
-                    tma_load_4d_pair(sA, &map_x, c * BK, b.x + tx - 1, b.y + ty - 1, b.n, full0);
-                    tma_load_2d_pair(sA + kABytes, &map_w, (ty * 3 + tx) * p.c_in + c * BK, nw, full0);
+                    if (rank == 0) tc::mbar_arrive_expect_tx(&ctrl->full[s], C::kStageTx);
+                    tma_load_4d_pair(base + s * C::kHaloBytes, &map_x, c * BK, b.x - 1, b.y + ty - 1, b.n, full0);
+                    if (!C::kResident) tma_load_3d_pair(base_w + s * 3 * C::kWBytes, &map_w, c * BK, nw, ty * 3, full0);
                 }
-                if (++tx == 3) {
-                    tx = 0;
-                    if (p.rows_outside) { if (++c == p.cb) { c = 0; ++ty; } }
-                    else if (++ty == 3) { ty = 0; ++c; }
-                }
+                step(p, c, ty);
                 if (++s == kStages) { s = 0; par ^= 1; }
             }
         }
@@ -178,7 +221,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else if (warp == 1) {
         // ------------------------------------------------------------ issuer of the pair's products (elected lane of CTA 0)
         if (rank == 0) {
-            constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BN, 0);
+            constexpr uint32_t idesc = tc::umma_idesc_f16(2 * C::kRows, BN, 0);
             const bool leader = tc::elect_one();
             int s = 0, par = 0, tl = 0;
             bool ok = true;
@@ -187,20 +230,28 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 if (tl >= 2) ok = wait_remote_warp(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const uint32_t d_tmem = tmem_cta + acc * BN;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                const uint32_t d_tmem = tmem_cta + acc * C::kAccCols;
+                if (C::kResident && tl == 0) ok = tc::mbar_wait_warp(&ctrl->weights, 0, abort_flag);
+                if (!ok) break;
+                int c = 0, ty = 0;            // of the box: where its weights lie, if they are resident
+                for (int i = 0; i < num_boxes; ++i) {
                     ok = tc::mbar_wait_warp(&ctrl->full[s], par, abort_flag);
                     if (!ok) break;
                     tc::tc_fence_after();
                     if (leader) {
-                        const uint32_t a_lo = tc::umma_desc_lo(base + s * C::kStageBytes);
-                        const uint32_t b_lo = tc::umma_desc_lo(base + s * C::kStageBytes + kABytes);
+                        const uint32_t w0 = base_w + (C::kResident ? c * 3 + ty : s) * (3 * C::kWBytes);
 #pragma unroll
-                        for (int ks = 0; ks < BK / 16; ++ks)
-                            umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb > 0) || (ks > 0));
+                        for (int tx = 0; tx < 3; ++tx) {
+                            const uint32_t a_lo = tc::umma_desc_lo(base + s * C::kHaloBytes + tx * kColBytes);
+                            const uint32_t b_lo = tc::umma_desc_lo(w0 + tx * C::kWBytes);
+#pragma unroll
+                            for (int ks = 0; ks < BK / 16; ++ks)
+                                umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (i > 0) || (tx > 0) || (ks > 0));
+                        }
                         umma_pair_commit(&ctrl->empty[s]);
-                        if (tl == 0 && kb == 0) umma_pair_commit(&ctrl->started);
+                        if (tl == 0 && i == 0) umma_pair_commit(&ctrl->started);
                     }
+                    step(p, c, ty);
                     if (++s == kStages) { s = 0; par ^= 1; }
                 }
                 if (ok && leader) umma_pair_commit(&ctrl->acc_full[acc]);
@@ -222,8 +273,9 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         int tl = 0;
         for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
             const int acc = tl & 1;
-            const Box b = box_of(p, 2 * (t % p.tiles_m) + (int)rank);
-            const int y0 = b.y + 2 * lane_grp, n0 = (t / p.tiles_m) * BN;   // this warp's 32 pixels: two rows of the box
+            const Box b = box_of<BX>(p, 2 * (t % p.tiles_m) + (int)rank);
+            // this warp's 32 pixels, four columns of the box, and its first channel
+            const int x0 = b.x + 4 * (lane_grp & (BX / 4 - 1)), n0 = (t / p.tiles_m) * BN + (C::kRows == 64 ? (lane_grp >> 1) * C::kAccCols : 0);
             const bool live = 2 * (t % p.tiles_m) + (int)rank < p.tiles;
             if (lane == 0) {
                 bulk_wait_read<0>();   // the previous tile's stores have read the buffers
@@ -234,7 +286,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
                     for (int u = 0; u < kUnits; ++u) {
                         tc::mbar_arrive_expect_tx(&my_res[u], kUnitBytes);
-                        tma_load_4d(stage_base + u * kUnitBytes, &map_r, n0 + u * 64, b.x, y0, b.n, &my_res[u]);
+                        tma_load_4d(stage_base + u * kUnitBytes, &map_r, n0 + u * kUnitCh, x0, b.y, b.n, &my_res[u]);
                     }
                 }
             }
@@ -242,32 +294,33 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // Lane l holds channels 2l and 2l + 1 of a unit's bias, fetched a unit ahead (each thread reading the 64 of them itself
             // was 8 us of load latencies a tile)
             const uint32_t* bias_lane = reinterpret_cast<const uint32_t*>(p.bias + n0) + lane;
-            uint32_t bias_next = p.bias ? __ldg(bias_lane) : 0;
+            const bool biased = p.bias != nullptr;
+            uint32_t bias_next = biased && n0 + 2 * lane < p.c_out ? __ldg(bias_lane) : 0;
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
-            const uint32_t t_acc = tmem_cta + lane_off + acc * BN;
+            const uint32_t t_acc = tmem_cta + lane_off + acc * C::kAccCols;
 #pragma unroll 1
             for (int u = 0; u < kUnits; ++u) {
                 const uint32_t bias_u = bias_next;
-                if (p.bias && u + 1 < kUnits) bias_next = __ldg(bias_lane + (u + 1) * 32);
+                if (biased && u + 1 < kUnits) bias_next = n0 + (u + 1) * kUnitCh + 2 * lane < p.c_out ? __ldg(bias_lane + (u + 1) * (kUnitCh / 2)) : 0;
                 unsigned char* buf = my_stage + u * kUnitBytes;
                 if (p.has_res) ok = tc::mbar_wait_warp(&my_res[u], tl & 1, abort_flag);
                 if (!ok) break;
-                uint32_t second[32];      // silu(out), if asked
+                uint32_t second[kUnitCh / 2];      // silu(out), if asked
 #pragma unroll
-                for (int hc = 0; hc < 2; ++hc) {
+                for (int hc = 0; hc < kUnitCh / 32; ++hc) {
                     uint32_t v[32], o[16];
-                    tc::tmem_ld32(t_acc + u * 64 + hc * 32, v);
+                    tc::tmem_ld32(t_acc + u * kUnitCh + hc * 32, v);
                     uint4 res[4];
                     if (p.has_res) {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) res[q] = *reinterpret_cast<const uint4*>(buf + staged(lane, hc * 4 + q));
+                        for (int q = 0; q < 4; ++q) res[q] = *reinterpret_cast<const uint4*>(buf + C::chunk(lane, hc * 4 + q));
                     }
                     tc::tc_wait_ld(v);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) o[i] = pack_half2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-                    if (p.bias) {
+                    if (biased) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float2 y = unpack_half2(o[i]), bb = unpack_half2(__shfl_sync(0xffffffffu, bias_u, hc * 16 + i));
@@ -298,25 +351,25 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                     }
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
-                        *reinterpret_cast<uint4*>(buf + staged(lane, hc * 4 + q)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                        *reinterpret_cast<uint4*>(buf + C::chunk(lane, hc * 4 + q)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                 }
                 tc::fence_proxy_async();                      // the copy engine reads what the threads just wrote
                 __syncwarp();
                 if (lane == 0 && live) {
-                    tma_store_4d(&map_o, stage_base + u * kUnitBytes, n0 + u * 64, b.x, y0, b.n);   // pixels beyond the image are clipped
+                    tma_store_4d(&map_o, stage_base + u * kUnitBytes, n0 + u * kUnitCh, x0, b.y, b.n);   // pixels beyond the image are clipped
                     bulk_commit();
                 }
                 if (p.dual) {                                 // the same buffer again, once that store has read it
                     if (lane == 0) bulk_wait_read<0>();
                     __syncwarp();
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        *reinterpret_cast<uint4*>(buf + staged(lane, q)) =
+                    for (int q = 0; q < kUnitCh / 8; ++q)
+                        *reinterpret_cast<uint4*>(buf + C::chunk(lane, q)) =
                             make_uint4(second[4 * q], second[4 * q + 1], second[4 * q + 2], second[4 * q + 3]);
                     tc::fence_proxy_async();
                     __syncwarp();
                     if (lane == 0 && live) {
-                        tma_store_4d(&map_s, stage_base + u * kUnitBytes, n0 + u * 64, b.x, y0, b.n);
+                        tma_store_4d(&map_s, stage_base + u * kUnitBytes, n0 + u * kUnitCh, x0, b.y, b.n);
                         bulk_commit();
                     }
                 }
@@ -366,69 +419,71 @@ EncodeTiledFn tensor_map_encoder() {
     return fn;
 }
 
-// fp16 tensor of 2 to 4 dimensions, innermost first, dense; boxes in the 128-byte-swizzled layout, elements outside read as zeros
-bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint32_t* box) {
+// fp16 tensor of 3 or 4 dimensions, innermost first, strides in bytes from the second on; boxes swizzled by 128 bytes (of 32 channels: by 64),
+// elements outside read as zeros
+bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+    static_assert(tcconv::BK == 64, "rows of 128 bytes, or of 64 for units of 32 channels");
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return false;
-    cuuint64_t strides[3], bytes = 2;
-    for (int i = 0; i + 1 < rank; ++i) strides[i] = bytes *= dims[i];
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// [N][H][W][C]; boxes of 64 channels x kBoxX x rows pixels of one image
-bool make_map_pixels(CUtensorMap* m, const void* base, int N, int H, int W, int C, int rows) {
-    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-    const cuuint32_t box[4] = {64, (cuuint32_t)tcconv::kBoxX, (cuuint32_t)rows, 1};
-    return make_map(m, base, 4, dims, box);
+// [N][H][W][C] as (c, y, x, n): boxes of `channels` channels x kBoxY x columns pixels of one image, a column's pixels one after the other
+bool make_map_pixels(CUtensorMap* m, const void* base, int N, int H, int W, int C, int columns, int channels) {
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)H, (cuuint64_t)W, (cuuint64_t)N};
+    const cuuint64_t strides[3] = {(cuuint64_t)2 * W * C, (cuuint64_t)2 * C, (cuuint64_t)2 * H * W * C};
+    const cuuint32_t box[4] = {(cuuint32_t)channels, (cuuint32_t)tcconv::kBoxY, (cuuint32_t)columns, 1};
+    return make_map(m, base, 4, dims, strides, box);
 }
 
-template <int BN> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+template <int BN, int BX> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.blockDim = dim3(tcconv::kThreads); cfg.dynamicSmemBytes = tcconv::Cfg<BN>::kSmemBytes; cfg.stream = st;
+    cfg.blockDim = dim3(tcconv::kThreads); cfg.dynamicSmemBytes = tcconv::Cfg<BN, BX>::kSmemBytes; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
     return cfg;
 }
 
 // CTA pairs of the kernel that the device runs at once (asked once per device; 0: it cannot place them)
-template <int BN> int resident_pairs(int dev) {
+template <int BN, int BX> int resident_pairs(int dev) {
     static std::atomic<int> asked[64];   // the answer + 1
     int n = asked[dev].load(std::memory_order_acquire);
     if (n == 0) {
         cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = pair_config<BN>(attr, nullptr);
+        cudaLaunchConfig_t cfg = pair_config<BN, BX>(attr, nullptr);
         int sms = 0, pairs = 0;
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tcconv::conv3x3_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcconv::Cfg<BN>::kSmemBytes);
+            e = cudaFuncSetAttribute(tcconv::conv3x3_pair_kernel<BN, BX>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcconv::Cfg<BN, BX>::kSmemBytes);
         cfg.gridDim = dim3(2 * std::max(1, sms / 2));
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&pairs, tcconv::conv3x3_pair_kernel<BN>, &cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&pairs, tcconv::conv3x3_pair_kernel<BN, BX>, &cfg);
         if (e != cudaSuccess) { cudaGetLastError(); pairs = 0; }
-        n = std::min(std::max(pairs, 0), sms / 2) + 1;
+        n = std::max(pairs, 0) + 1;
         asked[dev].store(n, std::memory_order_release);
     }
     return n - 1;
 }
 
-template <int BN>
-int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap& mr, const CUtensorMap& ms, const __half* w, int Cout,
+template <int BN, int BX>
+int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap& mr, const CUtensorMap& ms, const __half* w,
                 tcconv::Params p, int dev, cudaStream_t st) {
-    CUtensorMap mw;
-    const cuuint64_t dims[2] = {(cuuint64_t)9 * p.c_in, (cuuint64_t)Cout};
-    const cuuint32_t box[2] = {64, BN / 2};
-    if (!make_map(&mw, w, 2, dims, box)) return RFK_EUNSUPPORTED;
-    const int pairs = resident_pairs<BN>(dev);
+    CUtensorMap mw;   // [C_out][9][C_in] as (c_in, c_out, tap)
+    const cuuint64_t C_in = (cuuint64_t)p.cb * 64;
+    const cuuint64_t dims[3] = {C_in, (cuuint64_t)p.c_out, 9}, strides[2] = {18 * C_in, 2 * C_in};
+    const cuuint32_t box[3] = {64, BN / 2, 3};
+    if (!make_map(&mw, w, 3, dims, strides, box)) return RFK_EUNSUPPORTED;
+    const int pairs = resident_pairs<BN, BX>(dev);
     if (pairs <= 0) return RFK_EUNSUPPORTED;
-    p.tiles_n = Cout / BN;
+    p.tiles_n = ceil_div(p.c_out, BN);
     cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = pair_config<BN>(attr, st);
+    cudaLaunchConfig_t cfg = pair_config<BN, BX>(attr, st);
     cfg.gridDim = dim3(2 * std::min(p.tiles_m * p.tiles_n, pairs));
-    cudaError_t e = cudaLaunchKernelEx(&cfg, tcconv::conv3x3_pair_kernel<BN>, mx, mw, mo, mr, ms, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcconv::conv3x3_pair_kernel<BN, BX>, mx, mw, mo, mr, ms, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
@@ -436,8 +491,31 @@ int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap&
 // shapes and alignments that the kernel takes
 bool conv_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, const rfk_half* out,
                  const rfk_half* out_silu, int C_in, int C_out) {
-    return C_in % 64 == 0 && C_out % 128 == 0 && aligned16(x) && aligned16(w) && aligned16(out) && (!residual || aligned16(residual)) &&
+    return C_in % 64 == 0 && C_out % 32 == 0 && aligned16(x) && aligned16(w) && aligned16(out) && (!residual || aligned16(residual)) &&
            (!out_silu || aligned16(out_silu)) && (!bias || (reinterpret_cast<uintptr_t>(bias) & 3u) == 0);
+}
+
+// Tiles (rfk_conv3x3_nhwc_tiled's `tile`): output channels x pixels of a pair's CTA
+enum : int { kByRule = 0, k128x128 = 1, k64x128 = 2, k64x64 = 3, k32x128 = 4 };
+
+// all weights beside the ring of boxes
+bool resident_weights(int C_in, int C_out) { return C_out == 32 && C_in <= 64 * tcconv::kResidentBlocks; }
+
+// pairs of boxes of BX x kBoxY pixels
+long long box_pairs(int N, int H, int W, int BX) { return ((long long)ceil_div(W, BX) * ceil_div(H, tcconv::kBoxY) * N + 1) / 2; }
+
+int choose_tile(int N, int H, int W, int C_in, int C_out, int pairs) {
+    if (resident_weights(C_in, C_out)) return k32x128;
+    struct { int tile, bx, bn, clocks; } const kinds[] = {{k128x128, 16, 128, 260}, {k64x128, 16, 64, 177}, {k64x64, 8, 64, 125}};
+    int best = 0;
+    long long least = 0;
+    for (const auto& k : kinds) {
+        if (k.bn > 64 && C_out % k.bn) continue;
+        const long long rounds = ceil_div(box_pairs(N, H, W, k.bx) * ceil_div(C_out, k.bn), pairs);
+        const long long clocks = rounds * (9 * C_in / 64) * k.clocks + 20 * k.bn * k.bx / 8;
+        if (!best || clocks < least) { best = k.tile; least = clocks; }
+    }
+    return best;
 }
 
 }  // namespace
@@ -450,34 +528,48 @@ extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, con
     int dev = 0;
     if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out) || !tensor_map_encoder()) return 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    return (C_out % 256 == 0 ? resident_pairs<256>(dev) : resident_pairs<128>(dev)) > 0;
+    return resident_pairs<128, 16>(dev) > 0 && resident_pairs<64, 16>(dev) > 0 && resident_pairs<64, 8>(dev) > 0 && resident_pairs<32, 16>(dev) > 0;
+}
+
+extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
+                                      rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
+                                      rfk_stream_t stream) {
+    if (!x || !w || !out || N < 0 || H <= 0 || W <= 0 || C_in <= 0 || C_out <= 0) return RFK_EINVAL;
+    if (x == out || x == out_silu || out == out_silu) return RFK_EINVAL;   // a pixel is read by its neighbours' tiles
+    if (tile < kByRule || tile > k32x128 || (tile == k128x128 && C_out % 128) || (tile == k32x128 && !resident_weights(C_in, C_out))) return RFK_EINVAL;
+    if (N == 0) return RFK_OK;
+    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out)) return RFK_EUNSUPPORTED;
+    if (box_pairs(N, H, W, 8) * ceil_div(C_out, 64) > 0x1fffffffLL || 9LL * C_in > 0x7fffffffLL) return RFK_EUNSUPPORTED;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    if (tile == kByRule) {
+        const int pairs = resident_pairs<128, 16>(dev);   // one on every two SMs
+        if (pairs <= 0) return RFK_EUNSUPPORTED;
+        tile = choose_tile(N, H, W, C_in, C_out, pairs);
+    }
+    const int bx = tile == k64x64 ? 8 : 16, unit = tile == k64x64 || tile == k32x128 ? 32 : 64;
+    CUtensorMap mx, mo, mr, ms;
+    if (!make_map_pixels(&mx, x, N, H, W, C_in, bx + 2, 64) || !make_map_pixels(&mo, out, N, H, W, C_out, 4, unit) ||
+        !make_map_pixels(&mr, residual ? residual : out, N, H, W, C_out, 4, unit) ||
+        !make_map_pixels(&ms, out_silu ? out_silu : out, N, H, W, C_out, 4, unit))
+        return RFK_EUNSUPPORTED;
+    tcconv::Params p{};
+    p.bias = (const __half*)bias;
+    p.tiles_x = (int)ceil_div(W, bx); p.tiles_img = p.tiles_x * (int)ceil_div(H, tcconv::kBoxY); p.tiles = p.tiles_img * N;
+    p.tiles_m = (p.tiles + 1) / 2;
+    p.cb = C_in / 64; p.c_out = C_out;
+    p.rows_outside = rows_outside != 0; p.silu = silu != 0; p.has_res = residual != nullptr; p.dual = out_silu != nullptr;
+    const auto launch = tile == k128x128 ? launch_conv<128, 16> : tile == k64x128 ? launch_conv<64, 16> : tile == k64x64 ? launch_conv<64, 8> : launch_conv<32, 16>;
+    return launch(mx, mo, mr, ms, (const __half*)w, p, dev, as_stream(stream));
 }
 
 extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
                                 rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside,
                                 rfk_stream_t stream) {
-    if (!x || !w || !out || N < 0 || H <= 0 || W <= 0 || C_in <= 0 || C_out <= 0) return RFK_EINVAL;
-    if (x == out || x == out_silu || out == out_silu) return RFK_EINVAL;   // a pixel is read by its neighbours' tiles
-    if (N == 0) return RFK_OK;
-    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out)) return RFK_EUNSUPPORTED;
-    const long long tx = ceil_div(W, tcconv::kBoxX), ty = ceil_div(H, tcconv::kBoxY);
-    if (tx * ty * N * (C_out / 128) > 0x3fffffffLL || 9LL * C_in > 0x7fffffffLL) return RFK_EUNSUPPORTED;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return (int)e;
-    if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
-    CUtensorMap mx, mo, mr, ms;
-    if (!make_map_pixels(&mx, x, N, H, W, C_in, tcconv::kBoxY) || !make_map_pixels(&mo, out, N, H, W, C_out, 2) ||
-        !make_map_pixels(&mr, residual ? residual : out, N, H, W, C_out, 2) ||
-        !make_map_pixels(&ms, out_silu ? out_silu : out, N, H, W, C_out, 2))
-        return RFK_EUNSUPPORTED;
-    tcconv::Params p{};
-    p.bias = (const __half*)bias;
-    p.tiles_x = (int)tx; p.tiles_img = (int)(tx * ty); p.tiles = p.tiles_img * N;
-    p.tiles_m = (p.tiles + 1) / 2;
-    p.c_in = C_in; p.cb = C_in / 64;
-    p.rows_outside = rows_outside != 0; p.silu = silu != 0; p.has_res = residual != nullptr; p.dual = out_silu != nullptr;
-    return (C_out % 256 == 0 ? launch_conv<256> : launch_conv<128>)(mx, mo, mr, ms, (const __half*)w, C_out, p, dev, as_stream(stream));
+    if (C_out > 0 && C_out % 128) return x && w && out ? RFK_EUNSUPPORTED : RFK_EINVAL;
+    return rfk_conv3x3_nhwc_tiled(x, w, bias, residual, out, out_silu, N, H, W, C_in, C_out, silu, rows_outside, kByRule, stream);
 }
 
 extern "C" int rfk_conv_error(int* code, int clear) {

@@ -7,8 +7,8 @@
 //     they are (handed NCHW tensors they convert every operand on the way in and out: 69 conversion launches, 35 % of
 //     the head's time when it ran that way); a 1x1 convolution is a row-major GEMM and goes to rfk_linear, i.e. the
 //     tcgen05 projection kernel with the bias in its epilogue; the two transposed convolutions (kernel = stride) are that
-//     same GEMM followed by a depth-to-space scatter. The large 3x3 convolutions of a single view are the tcgen05 kernel of
-//     conv_tc.cu, the others library (cuDNN) calls (own_conv says where the line lies). Filters are re-laid out once, at plan time.
+//     same GEMM followed by a depth-to-space scatter. The 3x3 convolutions of a single view are the tcgen05 kernel of
+//     conv_tc.cu, those of stride 2 and of several views library (cuDNN) calls. Filters are re-laid out once, at plan time.
 //   - bias, SiLU and residual adds that follow a convolution, and the SiLU that the next residual unit starts with, are the
 //     epilogue of that kernel, or one pass behind the library (rfk_bias_act_residual_nhwc), bit-identical
 //     to the separate operators; the copy the reference's in-place SiLU forces before a residual unit is gone.
@@ -38,17 +38,16 @@ namespace {
         if (rc_ != RFK_OK) return rc_;  \
     } while (0)
 
-// Which 3x3 convolutions (stride 1) of a view the tcgen05 kernel of conv_tc.cu takes from the library: those of more than 2^31
-// multiply-adds a tap (smaller ones: 256 -> 256 channels at 128^2 20.4 / 21.1, 64^2 9.7 / 19.6), of which
-//   - maps of 256 channels whose tiles of 256 x 256 fill the pairs of SMs one and a half times, from 256 input channels up, and
-//   - every map beyond 170000 pixels, where the library's kernels take a step (256 -> 128 at 408^2 91.2 / 90.9, at 416^2 139.1 / 95.5).
-// Measured with bias and SiLU, the library and its pass / this kernel, us: 256 -> 256 at 184^2 (1.9 times) 34.5 / 31.5, 200^2 45.2 / 41.1,
-// 224^2 48.3 / 43.7, 256^2 73.5 / 56.3, 288^2 79.2 / 71.3; 512 -> 256 at 136^2 (1.04 times) 33.8 / 51.1, 160^2 (1.35) 46.9 / 51.6, 168^2 (1.57)
-// 55.0 / 52.8, 256^2 131 / 109; 64 -> 256 at 320^2 43.0 / 47.1, 448^2 83.5 / 82.6; 256 -> 128, whose narrow tiles read three quarters of the
-// operands for half the products, at 272^2 38.0 / 39.0, 320^2 54.3 / 55.4, 368^2 75.0 / 76.2, 448^2 152 / 108, 512^2 183 / 140.
+// The 3x3 convolutions (stride 1) of a head over one view run on the tcgen05 kernel of conv_tc.cu. With bias and SiLU, the library and its pass /
+// that kernel, us: 256 -> 256 at 8^2 8.1 / 5.9, 32^2 8.3 / 6.2, 64^2 9.6 / 8.6, 128^2 21 / 18, 160^2 28.1 / 23.3, 256^2 78 / 52; 512 -> 256 at 32^2
+// 11.2 / 9.2, 128^2 34.6 / 29.5; 1024 -> 256 at 8^2 16.6 / 13.7, 32^2 16.9 / 14.2, 64^2 19.2 / 19.5 (the one size of 64 where it is not the faster
+// one); 256 -> 128 at 64^2 8.6 / 6.4, 320^2 56 / 43, 512^2 183 / 107; 128 -> 32 at 64^2 6.9 / 5.3, 320^2 40 / 16, 512^2 81 / 38.
 // A head over several views keeps the library, which chooses the order of its sums anew for every batch size.
-bool own_conv(int B, int H, int W, int Cin, int Cout, int sms) {
-    if (B != 1 || (long long)H * W * Cin * Cout <= (1LL << 31)) return false;
+//
+// Those of large maps are counted (rfk_dpt_create_from's own_convolutions): of more than 2^31 multiply-adds a tap, maps of 256 channels whose
+// tiles of 256 x 256 would fill the pairs of SMs one and a half times, from 256 input channels up, and every map beyond 170000 pixels.
+bool large_map(int H, int W, int Cin, int Cout, int sms) {
+    if ((long long)H * W * Cin * Cout <= (1LL << 31)) return false;
     const long long tiles = ((long long)((H + 7) / 8) * ((W + 15) / 16) + 1) / 2 * (Cout / 256);
     return (long long)H * W > 170000 || (Cout % 256 == 0 && Cin >= 256 && 2 * tiles > 3 * (sms / 2));
 }
@@ -86,11 +85,14 @@ struct rfk_dpt {
     size_t ws_bytes = 0;
     std::vector<Step> program;
     rfk_half* out = nullptr;  // [B, out_dim, pH*ps, pW*ps]
-    int n_convs = 0, n_own = 0;      // convolutions in all, and those of the tcgen05 kernel among them
+    int n_convs = 0, n_own = 0;      // convolutions in all; those of large maps that the tcgen05 kernel of conv_tc.cu takes
+    int n_library = 0;               // those that the library takes
     bool library_only = false;
     int sms = 0;
     struct Order { int H, W, Cin, Cout, rows_outside; };
     std::vector<Order> orders;       // what order_of_sums found
+    char* scratch = nullptr;         // order_of_sums' operands, while the head is planned
+    size_t scratch_bytes = 0;
 
     rfk_half* alloc(size_t halves) {
         void* p = nullptr;
@@ -127,15 +129,18 @@ struct rfk_dpt {
     // or -1 if neither order has them, and the convolution stays with the library. An image is 10^x of what comes out here, and
     // images do not change with the kernel that makes them. Which order the library takes is its own choice per size, type of
     // kernel and version, so it is not written down here but found out: both run once on the same operands when the head is planned, once
-    // for each size of map (1 to 3 ms of a plan's 50 to 55, most of it the scratch memory). x and y are the step's own buffers,
-    // which hold nothing yet.
+    // for each size of map. x and y are the step's own buffers, which hold nothing yet.
     int order_of_sums(cudnnTensorDescriptor_t xd, cudnnFilterDescriptor_t fd, cudnnConvolutionDescriptor_t cd, cudnnTensorDescriptor_t yd,
                       cudnnConvolutionFwdAlgo_t algo, size_t ws, rfk_half* x, rfk_half* y, int H, int W, int Cin, int Cout) {
         const size_t nx = (size_t)H * W * Cin, nw = (size_t)Cout * 9 * Cin, ny = (size_t)H * W * Cout;
         const auto pad = [](size_t halves) { return (halves * sizeof(__half) + 255) / 256 * 256; };
+        const size_t bytes = pad(nw) + pad(ny) + 256 + ws;
         int found = -1;
-        char* scratch = nullptr;
-        if (cudaMalloc((void**)&scratch, pad(nw) + pad(ny) + 256 + ws) == cudaSuccess) {
+        if (bytes > scratch_bytes) {
+            free_scratch();
+            if (cudaMalloc((void**)&scratch, bytes) == cudaSuccess) scratch_bytes = bytes;
+        }
+        if (bytes <= scratch_bytes) {
             rfk_half *k = (rfk_half*)scratch, *want = (rfk_half*)(scratch + pad(nw));
             int* differ = (int*)((char*)want + pad(ny));
             const auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
@@ -147,16 +152,20 @@ struct rfk_dpt {
             for (int rows_outside = 0; ran && found < 0 && rows_outside < 2; ++rows_outside) {
                 int other = 1;
                 ran = cudaMemsetAsync(differ, 0, sizeof(int)) == cudaSuccess &&
-                      rfk_conv3x3_nhwc(x, k, nullptr, nullptr, y, nullptr, 1, H, W, Cin, Cout, 0, rows_outside, nullptr) == RFK_OK;
+                      rfk_conv3x3_nhwc_tiled(x, k, nullptr, nullptr, y, nullptr, 1, H, W, Cin, Cout, 0, rows_outside, 0, nullptr) == RFK_OK;
                 if (ran) differ_kernel<<<blocks(ny / 2), 256>>>((const unsigned*)want, (const unsigned*)y, (long long)(ny / 2), differ);
                 ran = ran && cudaMemcpy(&other, differ, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
                 if (ran && !other) found = rows_outside;
             }
-            cudaFree(scratch);
         }
         cudaGetLastError();   // whatever failed: the library serves this size
         orders.push_back({H, W, Cin, Cout, found});
         return found;
+    }
+    void free_scratch() {
+        if (scratch) cudaFree(scratch);
+        scratch = nullptr;
+        scratch_bytes = 0;
     }
 
     // o [B, Ho, Wo, Cout] = conv(in [B, H, W, Cin], weight [Cout, Cin, k, k] as the reference stores it) + bias, then SiLU
@@ -183,13 +192,12 @@ struct rfk_dpt {
         rfk_half* wk = alloc((size_t)Cout * Cin * k * k);  // [Cout, k, k, Cin]
         if (!wk) return (int)cudaErrorMemoryAllocation;
         TRY(rfk_permute_filter(weight, wk, Cout, Cin, k * k, 0, nullptr));
-        const bool may_own = !library_only && k == 3 && stride == 1 && pad == 1 && own_conv(B, H, W, Cin, Cout, sms) &&
+        const bool may_own = !library_only && k == 3 && stride == 1 && pad == 1 && B == 1 &&
                              rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout);
         const auto push_own = [&](int rows_outside) {
-            const int Bn = B;
-            ++n_own;
+            if (large_map(H, W, Cin, Cout, sms)) ++n_own;
             program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
-                return rfk_conv3x3_nhwc(in, wk, bias, residual, o, o_silu, Bn, H, W, Cin, Cout, silu, rows_outside, (rfk_stream_t)st);
+                return rfk_conv3x3_nhwc_tiled(in, wk, bias, residual, o, o_silu, 1, H, W, Cin, Cout, silu, rows_outside, 0, (rfk_stream_t)st);
             });
             return RFK_OK;
         };
@@ -216,6 +224,7 @@ struct rfk_dpt {
             if (rows_outside >= 0) return push_own(rows_outside);
         }
         ws_bytes = std::max(ws_bytes, ws);
+        ++n_library;
         rfk_dpt* self = this;
         program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
             const float one = 1.0f, zero = 0.0f;
@@ -373,6 +382,7 @@ struct rfk_dpt {
                 return rfk_permute_nhwc_to_nchw(oc2b, image, Bn, HWf, od, (rfk_stream_t)st);
             });
         }
+        free_scratch();
         if (ws_bytes) {
             if (cudaMalloc(&workspace, ws_bytes) != cudaSuccess) return (int)cudaErrorMemoryAllocation;
             owned.push_back(workspace);
@@ -388,6 +398,7 @@ extern "C" int rfk_dpt_destroy(rfk_dpt* d) {
     for (auto f : d->fdescs) cudnnDestroyFilterDescriptor(f);
     for (auto c : d->cdescs) cudnnDestroyConvolutionDescriptor(c);
     for (void* p : d->owned) cudaFree(p);
+    d->free_scratch();
     if (d->dnn) cudnnDestroy(d->dnn);
     delete d;
     return RFK_OK;
@@ -439,4 +450,5 @@ extern "C" int rfk_dpt_forward(rfk_dpt* d, const rfk_half* const* features, rfk_
 }
 
 extern "C" const rfk_half* rfk_dpt_output(rfk_dpt* d) { return d ? d->out : nullptr; }
+extern "C" int rfk_dpt_num_library_convolutions(rfk_dpt* d) { return d ? d->n_library : 0; }
 extern "C" int rfk_dpt_num_convolutions(rfk_dpt* d) { return d ? d->n_convs : 0; }

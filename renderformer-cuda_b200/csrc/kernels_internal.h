@@ -128,6 +128,9 @@ extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_
                                 rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside,
                                 rfk_stream_t stream);
 // whether it takes these operands on the current device
+extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
+                                      rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
+                                      rfk_stream_t stream);
 extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
                                        const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out);
 
