@@ -5,10 +5,12 @@
 // Reference boundary: rf::conv2d and the residual units of rf::dpt_forward, src/layers/dpt.cu:100-178, :397-409 of
 // BANANASJIM/renderformer-cuda.
 //
-// A pair of CTAs owns 256 output pixels (two boxes of 16 x 8, one per CTA) x BN output channels (256 or 128). The GEMM's rows are
-// pixels and its K index is (tap, input channel): a K block is 64 channels of one tap, and its A tile is the box of input pixels
-// shifted by the tap, which one TMA copy of a rank-4 map [n][y][x][c] brings in the tensor core's swizzled layout; pixels beyond
-// the image arrive as zeros, which is the padding. So no patch matrix exists, and the nine shifted reads of a box come from L2.
+// A pair of CTAs owns two boxes of pixels (one per CTA, 16 x 8 or 8 x 8) x BN output channels. The GEMM's rows are pixels and its K index is
+// (tap, input channel): a K block is 64 channels of one tap. The three taps of a row of taps read the same pixels but for a shift by one
+// column, so a box comes with a column on either side, once for the three of them, by one TMA copy of a rank-4 map that has a column's pixels one
+// after the other ([c][y][x][n]): 8 pixels of a column are one 8-row group of the tensor core's swizzled layout, and a tap's operand
+// starts one group further. Pixels beyond the image arrive as zeros, which is the padding. So no patch matrix exists, and a K block
+// brings 6 KB of pixels into an SM instead of the 16 that a box per tap takes.
 // Otherwise the kernel is the projection kernel's (gemm_tc.cu: pair tiles, ring of operand stages filled by per-CTA copies that
 // count on CTA 0's barrier, two accumulators so that a tile's epilogue runs under the next tile's products, staged TMA stores).
 //
@@ -16,9 +18,14 @@
 //   taps inside  for each 64 input channels: the nine taps        (its implicit-GEMM kernels)
 //   rows outside for each row of taps: for each 64 channels: the three taps of that row   (its weight-stationary kernels)
 // The caller names the order (dpt.cu finds out, size by size, which the library takes); both cost the same here.
-// Bound: tensor pipe and the operands' way from L2 (32 KB a K block and SM for 256 channels), as the projections: 1.37 PFLOP/s for
-// 256 -> 256 channels at 256 x 256 with bias and SiLU (56 us; library 61 and 12 for the pass behind it), 1.10 for 256 -> 128 at
-// 512 x 512 (140 us; 171 and 16), whose tiles of 128 channels read 24 KB a K block for half the products.
+// Bound, by the tile (a K block of a pair, clocks): 128 channels x 2 x 128 pixels 260 with few pairs at work, which is the tensor pipe's own 256, and
+// 350 with all of them, where 14 KB a K block and SM are 11 TB/s out of L2; 64 x 2 x 128 177, 64 x 2 x 64 125: the tensor core's reads of the pixels
+// from shared memory, for fewer products each. To that a launch adds 3 to 4 us, of which the last tile's epilogue is 1.4 us for each 64
+// channels x 128 pixels. us, with bias and SiLU, a box per tap and tiles of 256 channels / now: 256 -> 256 at 256 x 256 57.0 / 51.5 (1.5 PFLOP/s), at 128 x 128
+// 20.9 / 18, 64 x 64 19.6 / 8.6, 32 x 32 19.0 / 6.2; 256 -> 128 at 512 x 512 144 / 107; 1024 -> 256 at 32 x 32 49 / 14.2. Tiles of 256 channels with the boxes shared
+// were slower up to 352 x 352 (98 for 100 there; 224 x 224 42.6 for 41.0, 128 x 128 21.3 for 18), 5 percent faster at 512 x 512, beyond the maps of
+// images that a session makes, and need a ring of their own for the weights: not kept.
+// Weights of at most 128 -> 32 channels stay in shared memory (BN = 32): 320 x 320 23.0 / 16.0, 512 x 512 58 / 38 against a stream of them in tiles of 64.
 #include <algorithm>
 #include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
 #include "common.cuh"
@@ -177,7 +184,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     const uint32_t tmem_cta = ctrl->tmem_base;
     // The weights on their way into L2 while the kernel before still runs: of a tile's boxes each pair that reads the same weights asks
-    // for its share. (A hint: what is copied below is read after the wait.)
+    // for its share. A hint only: what is copied below is read after the wait. Images of 64 x 64 pixels 911 -> 896 us, 128 x 128 1137 -> 1119, 192 x 192 1443 -> 1420.
     if (warp == 0 && tc::elect_one()) {
         const int nw = (first_tile / p.tiles_m) * BN + (int)rank * (BN / 2), sharing = min(p.tiles_m, tile_step);
         for (int i = first_tile % p.tiles_m; i < num_boxes; i += sharing) tma_prefetch_3d(&map_w, i / 3 * BK, nw, i % 3 * 3);
@@ -498,12 +505,16 @@ bool conv_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, con
 // Tiles (rfk_conv3x3_nhwc_tiled's `tile`): output channels x pixels of a pair's CTA
 enum : int { kByRule = 0, k128x128 = 1, k64x128 = 2, k64x64 = 3, k32x128 = 4 };
 
-// all weights beside the ring of boxes
+// all weights beside the ring of boxes (at 64 x 64 pixels the launch is all there is: 5.3 for 4.9 in tiles of 64 x 64; 128 x 128 6.1 / 6.9 / 8.0)
 bool resident_weights(int C_in, int C_out) { return C_out == 32 && C_in <= 64 * tcconv::kResidentBlocks; }
 
 // pairs of boxes of BX x kBoxY pixels
 long long box_pairs(int N, int H, int W, int BX) { return ((long long)ceil_div(W, BX) * ceil_div(H, tcconv::kBoxY) * N + 1) / 2; }
 
+// The tile whose busiest pair is done first: it takes its tiles one after the other, a K block of each in the clocks named at the top, and
+// the last one's epilogue shows. us, tiles of 128 x 128 / 64 x 128 / 64 x 64: 256 -> 256 channels at 48^2 11.7 / 8.3 / 6.5, 56^2 11.8 / 8.5 / 9.5, 64^2 12.0 / 8.7 / 9.7,
+// 80^2 12.7 / 12.5 / 13.0, 96^2 13.3 / 13.2 / 16.2, 112^2 17.1 / 17.1 / 22.1, 128^2 17.9 / 21.6 / 25.6, 160^2 23.4 / 30.0 / 37.4; 512 -> 256 at 48^2 16.7 / 12.1 / 9.8, 64^2 17.2 / 12.6 /
+// 15.0, 80^2 18.2 / 19.7 / 20.6; 1024 -> 256 at 48^2 26.6 / 18.9 / 15.3, 64^2 28.5 / 20.1 / 25.9.
 int choose_tile(int N, int H, int W, int C_in, int C_out, int pairs) {
     if (resident_weights(C_in, C_out)) return k32x128;
     struct { int tile, bx, bn, clocks; } const kinds[] = {{k128x128, 16, 128, 260}, {k64x128, 16, 64, 177}, {k64x64, 8, 64, 125}};

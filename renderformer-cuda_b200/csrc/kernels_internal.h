@@ -127,10 +127,12 @@ extern "C" int rfk_window_attention_steps(const rfk_half* Q, const rfk_half* K, 
 extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
                                 rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside,
                                 rfk_stream_t stream);
-// whether it takes these operands on the current device
+// The same for C_out % 32 == 0, with the tile named: output channels x pixels of a CTA 128 x 128 (1; C_out % 128 == 0), 64 x 128 (2), 64 x 64 (3), 32 x 128 with
+// the weights resident (4; C_out == 32, C_in <= 128), or by the rule on sizes (0). All of them have the same bits.
 extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
                                       rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
                                       rfk_stream_t stream);
+// whether it takes these operands on the current device
 extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
                                        const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out);
 
