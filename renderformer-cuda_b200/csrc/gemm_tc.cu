@@ -164,6 +164,18 @@ __device__ __forceinline__ float square_sum(const uint32_t (&o)[16]) {
 
 // Tiled copy global -> shared of one box of a rank-2 tensor map (x innermost, in elements; x * 2 bytes
 // is always a multiple of 128 here); the bytes are counted on `bar`.
+__device__ __forceinline__ void tma_prefetch_2d(const void* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+// A product's weights on their way from device memory into L2 while the kernel before it still runs, asked for by one lane of a CTA ahead of the
+// wait: `ask` walks the K blocks of the CTA's first tile that fall to it among the tiles that read the same weights. A hint only, and L2 is where
+// writes meet: what the product reads is copied after the wait, so weights that the kernel before writes are read as it left them. A model's weights are 0.3 GB
+// a view or scene, more than L2 keeps. us without / with: encodings of 300 triangles 698 / 685, of 2500 2103 / 2073, of 5633 5337 / 5286; an image of
+// 128 x 128 1119 / 1100, of 320 x 320 2468 / 2437; a view of 512 x 512 no difference.
+template <typename Ask> __device__ __forceinline__ void prefetch_weights(bool leader, Ask ask) {
+    if (leader) ask();
+    __syncwarp();
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void* tmap, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -497,6 +509,18 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
         }
     }
+    // Folded ones have asked for their ring above: the rest, for wide tiles only (views of 128 x 128 pixels 649.0 -> 645.6 us, 192 x 192 1145.5 ->
+    // 1141.3, 256 x 256 1172.9 -> 1168.7; for every tile 64 x 64 pixels 535 -> 548).
+    if (!FOLD || kWhole)
+        prefetch_weights(warp == 0 && (kLane0 ? lane == 0 : tc::elect_one()), [&] {
+            for (int t = early + m0 / BM_; t < num_st; t += p.tiles_m) {
+#pragma unroll
+                for (int h = 0; h < kSub; ++h) {
+                    tma_prefetch_2d(&map_w0, (t * kSub + h) * BK, n0);
+                    if (kGate) tma_prefetch_2d(&map_w1, (t * kSub + h) * BK, n0);
+                }
+            }
+        });
     pdl_wait();      // set-up above is on-chip only; the operands are another kernel's output
     pdl_trigger();
 
@@ -1050,6 +1074,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         return;
     }
     const uint32_t tmem_cta = ctrl->tmem_base;
+    prefetch_weights(warp == 0 && tc::elect_one(), [&] {
+        const void* map_w = rank == 0 || (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL) ? (const void*)&map_w0 : (const void*)&map_w1;
+        const int n0 = (first_tile / p.tiles_m) * BN_OUT, nw = (EPI == RFK_GEMM_EPI_SWIGLU || rank == 0) ? n0 : n0 + BN / 2;
+        for (int kb = first_tile % p.tiles_m; kb < num_kb; kb += p.tiles_m) tma_prefetch_2d(map_w, kb * BK, nw);
+    });
     pdl_wait();      // set-up above is on-chip only; the operands are another kernel's output
     pdl_trigger();
     if (tid == 0) RFK_STAMP(1);   // prologue done (barriers, tensor memory, cluster barrier)
