@@ -413,9 +413,16 @@ namespace pair { using namespace pair_ptx; }
 // The same product on small tiles, one per CTA, for calls that do not fill the machine: a view of 256 tokens gives the pair
 // kernel below four tiles for its 74 pairs, and a 4096-wide K then runs 64 K blocks of 0.3 us one after the other. Here a
 // tile is 64 or 128 rows by 32 to 128 accumulator columns, so that there are many and each takes few operand bytes per K
-// block (one SM takes them at about 110 GB/s). K is not split: every output is summed over the K blocks in the same order
+// block (one SM takes them at about 110 GB/s). But for the sums in quarters below every output is summed over the K blocks in the same order
 // as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
 // must equal the views one by one).
+//   Sums in quarters (SUM_): of a 64-row view's product with K = 4096 a CTA takes 64 K blocks of 64 x 32 columns one after the other, 7 us
+//   of loads on 32 SMs. The sum is therefore defined as ((a + b) + c) + d of its quarters of K for views of at most 128 rows, whatever frame they are in.
+//   For few rows a cluster of four CTAs takes a quarter each; the fp32 rows go to the CTA of their quarter of the tile through the cluster's shared
+//   memory, and one warp of it finishes 32 columns. For more rows one CTA keeps the four sums in accumulators of their own. us, one sum / quarters, K = 4096,
+//   N = 1024: 64 rows 8.7 / 5.8, 128 8.7 / 6.6, 192 8.9 / 8.5, 256 9.1 / 8.6, and on single CTAs 320 9.8 / 10.1, 1024 13.8 / 13.8; a view of 64 x 64
+//   pixels 539 / 508. With K = 1024 the exchange (1.2 us, 2.3 for tiles of 128 x 64) costs more than it gains (64 rows 3.67 / 3.97), and at 256 rows a
+//   view stays as it was (648 us), so these keep one sum.
 //   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing lane and the producer's are
 //   elected ones (elect.sync). With one block per stage and lane 0's loops a K block took 0.30 us on every tile size, the cost
 //   of issuing and not of the operands; two blocks and elected lanes in loops of whole warps took the 64 x 32 tile to 0.12 us, loops of
@@ -432,10 +439,10 @@ namespace pair { using namespace pair_ptx; }
 namespace small {
 
 constexpr int kSub = 2;                  // K blocks per stage
-template <int BM_, int BN_> struct Cfg {
+template <int BM_, int BN_, bool SPLIT = false> struct Cfg {
     static constexpr int kBlockBytes = (BM_ + BN_) * BK * 2;      // operands of one K block
     static constexpr int kStageBytes = kSub * kBlockBytes;
-    static constexpr int kStages = 192 * 1024 / kStageBytes;      // 8 to 3: a lone CTA waits for memory, so as deep as fits
+    static constexpr int kStages = (SPLIT ? 180 : 192) * 1024 / kStageBytes;   // 8 to 3: a lone CTA waits for memory, so as deep as fits
     static constexpr int kSmemBytes = kStages * kStageBytes + 256;
     static_assert(kStages >= 2 && kStages <= 8 && kSmemBytes + 1024 <= 227 * 1024, "control block, shared memory of an SM");
 };
@@ -447,17 +454,29 @@ struct __align__(8) Ctrl {
 };
 static_assert(sizeof(Ctrl) <= 256, "control block");
 
-template <int EPI_, int BM_, int BN_>
+// The pieces of a split sum on their way to the CTA that adds them: [the other pieces, its own][row of its quarter of the tile][BN_ floats and 16
+// bytes, which spread the banks]
+template <int BM_, int BN_> constexpr int kHandedPitch = BN_ * 4 + 16;
+template <int BM_, int BN_> constexpr int kHandedBytes = 4 * (BM_ / 4) * kHandedPitch<BM_, BN_>;
+
+// SUM 1: one sum over K. 4: ((a + b) + c) + d over the quarters of K, each a sum of its own; kSplit: by a cluster of four CTAs with a quarter each.
+enum : int { kSplit = 8 };
+template <int EPI_, int BM_, int BN_, int SUM_ = 1>
 __global__ void __launch_bounds__(kThreads)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                      const __grid_constant__ CUtensorMap map_w1, const Params p) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & kFold) != 0;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
+    constexpr bool SPLIT = (SUM_ & kSplit) != 0;
+    constexpr int kSums = SUM_ == 4 ? 4 : 1;            // accumulators of this CTA
+    static_assert(SUM_ == 1 || (SUM_ == 4 && kSums * BN_ <= 512) || SUM_ == (4 | kSplit), "a whole sum, or one of four quarters");
+    static_assert(SUM_ == 1 || (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL), "the form that is summed in quarters");
     constexpr bool kWhole = BM_ == 128 && BN_ == 128;   // producer and issuer run their loops as whole warps
     constexpr bool kLane0 = BM_ == 128 && BN_ == 64 && (EPI == RFK_GEMM_EPI_NONE || EPI == RFK_GEMM_EPI_RESIDUAL);   // the producer is lane 0
     constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
-    constexpr int kStages = Cfg<BM_, BN_>::kStages, kStage = Cfg<BM_, BN_>::kStageBytes, kBlock = Cfg<BM_, BN_>::kBlockBytes;
+    using C = Cfg<BM_, BN_, SPLIT>;
+    constexpr int kStages = C::kStages, kStage = C::kStageBytes, kBlock = C::kBlockBytes;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = tc::smem_addr(smem_raw);
     if (base & 1023u) {  // uniform over the CTA, nothing allocated yet
@@ -467,11 +486,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + kStages * kStage);
     volatile int* abort_flag = &ctrl->abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int num_st = (p.K + kSub * BK - 1) / (kSub * BK);   // stages of K; a second block beyond K arrives as zeros
+    const int all_st = (p.K + kSub * BK - 1) / (kSub * BK);   // stages of K; a second block beyond K arrives as zeros
+    const int piece = SPLIT ? blockIdx.x & 3 : 0, num_st = SPLIT ? all_st / 4 : all_st, st0 = piece * num_st;   // this CTA's
+    const unsigned tile = SPLIT ? blockIdx.x >> 2 : blockIdx.x;
     // rows fastest, so that the tiles running together share weights; the heads form runs columns fastest, because the tiles
     // of 256 columns are one cluster
-    const int m0 = (EPI == kEpiHeads && !FOLD ? blockIdx.x / p.tiles_n : blockIdx.x % p.tiles_m) * BM_;
-    const int n0 = (EPI == kEpiHeads && !FOLD ? blockIdx.x % p.tiles_n : blockIdx.x / p.tiles_m) * BN_OUT;
+    const int m0 = (EPI == kEpiHeads && !FOLD ? tile / p.tiles_n : tile % p.tiles_m) * BM_;
+    const int n0 = (EPI == kEpiHeads && !FOLD ? tile % p.tiles_n : tile / p.tiles_m) * BN_OUT;
     const bool want_ss = EPI == kEpiHeads && p.row_ss && ((p.ss_mask >> (n0 / (p.units * 64))) & 1);   // uniform over a cluster
     bool acc_ok = false;
 
@@ -483,12 +504,16 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         tc::fence_barrier_init();
     }
     if (warp == 2) {   // beside the barriers
-        tc::tmem_alloc(&ctrl->tmem_base, BN_);
+        tc::tmem_alloc(&ctrl->tmem_base, kSums * BN_);
         tc::tmem_relinquish();
     }
     if (warp == 1 && lane == 0) {   // descriptors are kernel arguments: fetched ahead of the wait for the kernel before
         tc::prefetch_tensormap(&map_a); tc::prefetch_tensormap(&map_w0);
         if (kGate) tc::prefetch_tensormap(&map_w1);
+    }
+    if (SPLIT) {                 // met again ahead of the first store into another CTA: by then all four run
+        __syncwarp();
+        pair::cluster_arrive();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -503,7 +528,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
             for (int h = 0; h < kSub; ++h) {
                 const uint32_t sW = base + t * kStage + h * kBlock + BM_ * BK * 2;
-                const int x = (t * kSub + h) * BK;
+                const int x = ((st0 + t) * kSub + h) * BK;
                 tma_load_2d(sW, &map_w0, x, n0, &ctrl->full[t]);
                 if (kGate) tma_load_2d(sW + BN_OUT * BK * 2, &map_w1, x, n0, &ctrl->full[t]);
             }
@@ -537,7 +562,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
                     for (int h = 0; h < kSub; ++h) {
                         const uint32_t sA = base + s * kStage + h * kBlock, sW = sA + BM_ * BK * 2;
-                        const int x = (it * kSub + h) * BK;
+                        const int x = ((st0 + it) * kSub + h) * BK;
                         tma_load_2d(sA, &map_a, x, m0, &ctrl->full[s]);
                         if (it < early) continue;
                         tma_load_2d(sW, &map_w0, x, n0, &ctrl->full[s]);
@@ -559,7 +584,10 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         constexpr uint32_t idesc = tc::umma_idesc_f16(BM_, BN_, 0);  // A and B both K-major
         const bool leader = tc::elect_one();
         bool ok = true;
+        const int quarter = num_st / 4;
+        int sum = 0;
         for (int it = 0; (kWhole || leader) && it < num_st; ++it) {
+            if (kSums > 1 && it == (sum + 1) * quarter) ++sum;
             const int s = it % kStages;
             ok = kWhole ? tc::mbar_wait_warp(&ctrl->full[s], (it / kStages) & 1, abort_flag)
                         : tc::mbar_wait(&ctrl->full[s], (it / kStages) & 1, abort_flag);
@@ -572,7 +600,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     const uint32_t b_lo = tc::umma_desc_lo(base + s * kStage + h * kBlock + BM_ * BK * 2);
 #pragma unroll
                     for (int ks = 0; ks < BK / 16; ++ks)  // 16 halves = 32 bytes along a swizzled row
-                        tc::umma_f16_lo(tmem_cta, a_lo + ks * 2, b_lo + ks * 2, idesc, (it > 0) || (h > 0) || (ks > 0));
+                        tc::umma_f16_lo(kSums > 1 ? tmem_cta + sum * BN_ : tmem_cta, a_lo + ks * 2, b_lo + ks * 2, idesc,
+                                        (kSums > 1 ? it > sum * quarter : it > 0) || (h > 0) || (ks > 0));
                 }
                 tc::umma_commit(&ctrl->empty[s]);
             }
@@ -588,7 +617,9 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else {
         // ------------------------------------------------------------ epilogue, warps 2-5
         const int lane_grp = warp & 3;                        // a warp reaches tensor-memory lanes [32 * (warp % 4), +32)
-        const int row = m0 + (BM_ == 64 ? lane_grp * 16 + lane : lane_grp * 32 + lane);
+        // SPLIT: the CTA finishes the rows of one quarter of the tile, a warp 32 columns of them
+        const int row_grp = SPLIT ? piece : lane_grp, first_c = SPLIT ? (lane_grp - piece) & 3 : 0;
+        const int row = m0 + (BM_ == 64 ? row_grp * 16 + lane : row_grp * 32 + lane);
         const bool row_ok = row < p.M && (BM_ == 128 || lane < 16);
         const uint32_t t_acc = tmem_cta + ((uint32_t)(lane_grp * 32) << 16);
         __half* crow = p.C + (size_t)(row_ok ? row : 0) * p.ldc + n0;
@@ -612,16 +643,68 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const __half* rrow = p.R + (size_t)(row_ok ? row : 0) * p.ldr + n0;
 #pragma unroll
             for (int q = 0; q < BN_OUT / 8; ++q)
-                res[q] = (row_ok && n0 + q * 8 < p.N) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
+                res[q] = (row_ok && n0 + q * 8 < p.N && (!SPLIT || q / 4 == first_c)) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
         }
         acc_ok = tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag);
+        const int handed = C::kSmemBytes + (lane & (BM_ / 4 - 1)) * kHandedPitch<BM_, BN_>;   // the row's place, of the first piece
+        constexpr int kHandedPiece = (BM_ / 4) * kHandedPitch<BM_, BN_>;
+        if (SPLIT) {                                          // a warp's rows to the CTA of their quarter
+            pair::cluster_wait();
+            if (acc_ok) {
+                tc::tc_fence_after();
+                const int slot = lane_grp == piece ? 3 : piece < lane_grp ? piece : piece - 1;
+                const uint32_t to = pair::map_to_cta(base + handed + slot * kHandedPiece, lane_grp);
+#pragma unroll
+                for (int c = 0; c < BN_ / 32; ++c) {
+                    uint32_t v[32];
+                    tc::tmem_ld32(t_acc + c * 32, v);
+                    tc::tc_wait_ld(v);
+                    if (BM_ == 128 || lane < 16) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                         ::"r"(to + c * 128 + q * 16), "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3]) : "memory");
+                    }
+                }
+            }
+            __syncwarp();
+            pair::cluster_arrive();
+            pair::cluster_wait();
+        }
         if ((EPI != kEpiHeads || FOLD) && acc_ok) {
             tc::tc_fence_after();
 #pragma unroll
             for (int c = 0; c < BN_OUT / kChunk; ++c) {
                 if (n0 + c * kChunk >= p.N) break;            // uniform over the CTA: the tile's tail lies beyond N
+                if (SPLIT && c != first_c) continue;
                 uint32_t v[32], o[kChunk / 2];
-                tc::tmem_ld32(t_acc + c * 32, v);
+                if (!SPLIT) tc::tmem_ld32(t_acc + c * 32, v);
+                if (SPLIT) {                                  // ((a + b) + c) + d, whichever of them is this CTA's
+                    const float4* at = reinterpret_cast<const float4*>(smem_raw + handed + c * 128);
+                    constexpr int kPiece4 = kHandedPiece / 16;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 own = at[3 * kPiece4 + q], s0 = at[q], s1 = at[kPiece4 + q], s2 = at[2 * kPiece4 + q];
+                        const auto sum = [&](float o, float a0, float a1, float a2) {
+                            const float x1 = piece <= 1 ? o : a1, x2 = piece <= 1 ? a1 : piece == 2 ? o : a2, x3 = piece <= 2 ? a2 : o;
+                            return __float_as_uint(((a0 + x1) + x2) + x3);   // (pieces 0 and 1 either way round)
+                        };
+                        v[4 * q] = sum(own.x, s0.x, s1.x, s2.x);
+                        v[4 * q + 1] = sum(own.y, s0.y, s1.y, s2.y);
+                        v[4 * q + 2] = sum(own.z, s0.z, s1.z, s2.z);
+                        v[4 * q + 3] = sum(own.w, s0.w, s1.w, s2.w);
+                    }
+                } else if (kSums > 1) {
+#pragma unroll
+                    for (int a = 1; a < kSums; ++a) {
+                        uint32_t u[32];
+                        tc::tmem_ld32(t_acc + a * BN_ + c * 32, u);
+                        if (a == 1) tc::tc_wait_ld(v);
+                        tc::tc_wait_ld(u);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(u[i]));
+                    }
+                }
                 if (kGate) {
                     uint32_t u[32];
                     if (kChunk == 32) {
@@ -649,7 +732,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         o[i >> 1] = pack_half2(s0 * __uint_as_float(u[i]), s1 * __uint_as_float(u[i + 1]));
                     }
                 } else {
-                    tc::tc_wait_ld(v);
+                    if (SUM_ == 1) tc::tc_wait_ld(v);
                     if (p.bias) {
 #pragma unroll
                         for (int i = 0; i < kChunk; i += 2) {
@@ -706,6 +789,11 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         __syncwarp();
     }
 
+    if (SPLIT && warp < 2) {     // the other warps' share in the cluster's barriers
+        pair::cluster_wait();
+        pair::cluster_arrive();
+        pair::cluster_wait();
+    }
     if (EPI == kEpiHeads && !FOLD) {
         // ------------------------------------------------------------ epilogue of the head-split form
         // [part][group][head][seq][hd] by plain stores. The row statistic has the bits of the pair kernel's: one thread adds
@@ -787,7 +875,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     if (warp == 0) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem_cta, BN_);
+        tc::tmem_dealloc(tmem_cta, kSums * BN_);
     }
     if (tid == 0 && ctrl->abort) atomicCAS(&g_gemm_tc_error, 0, kErrTimeout);
 }
@@ -1437,41 +1525,43 @@ int heads_resident(int dev) {
     return n - 1;
 }
 
-template <int EPI_, int BM_, int BN_>
+template <int EPI_, int BM_, int BN_, int SUM_ = 1>
 int launch_gemm_small(const void* A, long long lda, const void* W, const void* W_up, long long ldw, tcgemm::Params p, int dev,
                       cudaStream_t st) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & tcgemm::kFold) != 0;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     constexpr int BN_OUT = kGate ? BN_ / 2 : BN_;
-    constexpr int smem = tcgemm::small::Cfg<BM_, BN_>::kSmemBytes;
+    constexpr bool SPLIT = (SUM_ & tcgemm::small::kSplit) != 0;
+    constexpr int smem = tcgemm::small::Cfg<BM_, BN_, SPLIT>::kSmemBytes + (SPLIT ? tcgemm::small::kHandedBytes<BM_, BN_> : 0);
+    static_assert(smem + 1024 <= 227 * 1024, "shared memory of an SM");
     CUtensorMap ma, mw0, mw1;
     if (!make_map_2d(&ma, A, p.M, p.K, lda, BM_) || !make_map_2d(&mw0, W, p.N, p.K, ldw, BN_OUT)) return RFK_EUNSUPPORTED;
     if (!kGate) mw1 = mw0;
     else if (!make_map_2d(&mw1, W_up, p.N, p.K, ldw, BN_OUT)) return RFK_EUNSUPPORTED;
     static std::atomic<bool> configured[64];
     if (!configured[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>,
+        cudaError_t e = cudaFuncSetAttribute(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_, SUM_>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured[dev].store(true, std::memory_order_release);
     }
     p.tiles_m = (p.M + BM_ - 1) / BM_;
     p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
-    const dim3 grid((unsigned)(p.tiles_m * p.tiles_n));
-    if (EPI != tcgemm::kEpiHeads || FOLD) {   // the sums of a folded form need no cluster
-        launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>, grid, dim3(tcgemm::kThreads), smem, st, ma, mw0, mw1, p);
+    const dim3 grid((unsigned)(p.tiles_m * p.tiles_n) * (SPLIT ? 4 : 1));
+    if ((EPI != tcgemm::kEpiHeads || FOLD) && !SPLIT) {   // the sums of a folded form need no cluster
+        launch_pdl(tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_, SUM_>, grid, dim3(tcgemm::kThreads), smem, st, ma, mw0, mw1, p);
         return launch_status();
     }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 256 / BN_; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = SPLIT ? 4 : 256 / BN_; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = grid; cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_>, ma, mw0, mw1, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcgemm::small::gemm_tc_small_kernel<EPI_, BM_, BN_, SUM_>, ma, mw0, mw1, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
@@ -1627,6 +1717,48 @@ static bool make_map_raster(CUtensorMap* m, const void* base, int n, int width, 
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// clusters of the split kernel that the device runs at once (asked once per device)
+template <int BM_, int BN_> static int resident_quarters(int dev) {
+    constexpr int SUM = 4 | tcgemm::small::kSplit;
+    const auto kernel = tcgemm::small::gemm_tc_small_kernel<RFK_GEMM_EPI_RESIDUAL | tcgemm::kFold, BM_, BN_, SUM>;
+    static std::atomic<int> asked[64];   // the answer + 1
+    int n = asked[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+        constexpr int smem = tcgemm::small::Cfg<BM_, BN_, true>::kSmemBytes + tcgemm::small::kHandedBytes<BM_, BN_>;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 4; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(4 * 64); cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = smem;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int clusters = 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+        if (e != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+        n = std::max(clusters, 0) + 1;
+        asked[dev].store(n, std::memory_order_release);
+    }
+    return n - 1;
+}
+
+// A residual product summed in quarters (FoldedProduct::quarters): one cluster a tile where they all run at once, else a CTA a tile with the
+// same sums
+static int launch_quarters(const FoldedProduct& f, const tcgemm::Params& p, int dev, cudaStream_t st) {
+    constexpr int E = RFK_GEMM_EPI_RESIDUAL | tcgemm::kFold, kSplit = 4 | tcgemm::small::kSplit;
+    const auto tiles = [&](int bm, int bn) { return (long long)ceil_div(p.M, bm) * ceil_div(p.N, bn); };
+    int rc = RFK_EUNSUPPORTED;
+    if (tiles(64, 32) <= resident_quarters<64, 32>(dev)) rc = launch_gemm_small<E, 64, 32, kSplit>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+    else if (tiles(64, 64) <= resident_quarters<64, 64>(dev)) rc = launch_gemm_small<E, 64, 64, kSplit>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+    else if (tiles(128, 64) <= resident_quarters<128, 64>(dev)) rc = launch_gemm_small<E, 128, 64, kSplit>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+    if (rc == RFK_OK) return rc;
+    switch (small_tile(p.M, p.N, sm_count(dev))) {
+        case 1: return launch_gemm_small<E, 64, 32, 4>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+        case 2: return launch_gemm_small<E, 64, 64, 4>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+        case 3: return launch_gemm_small<E, 128, 64, 4>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+        default: return launch_gemm_small<E, 128, 128, 4>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+    }
+}
+
 template <int EPI>
 static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cudaStream_t st, int* ss_tiles) {
     constexpr int E = EPI | tcgemm::kFold;
@@ -1636,6 +1768,8 @@ static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cuda
         int rc = RFK_EUNSUPPORTED;
         p.ss_tiles = sums;
         *ss_tiles = sums;
+        if constexpr (EPI == RFK_GEMM_EPI_RESIDUAL)
+            if (f.quarters) return launch_quarters(f, p, dev, st);
         switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
             case 1: rc = launch_gemm_small<E, 64, 32>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
             case 2: rc = launch_gemm_small<E, 64, 64>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
@@ -1672,6 +1806,7 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream)
     if (f.blocks_across && (!residual || f.blocks_across % 2 || f.blocks_down % 2 || f.blocks_down <= 0 || f.M % (f.blocks_across * f.blocks_down * 16)))
         return RFK_EUNSUPPORTED;
     if (!f.blocks_across && (f.raster || !f.C)) return RFK_EINVAL;
+    if (f.quarters && (!residual || f.K % 512)) return RFK_EUNSUPPORTED;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;

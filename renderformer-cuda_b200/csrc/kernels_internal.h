@@ -26,6 +26,7 @@ struct FoldedProduct {
     long long part_stride; int seq, num_heads, head_dim;
     int out_seq; const float* part_mul;                     // head-split: rows a head has room for (0: seq); another factor for each part, or NULL
     int blocks_across, blocks_down, shift_from, shift_to;   // 0: rows stay where they are
+    int quarters;                                           // residual: the sum over K is ((a + b) + c) + d of its quarters (K % 512 == 0), whatever M
 };
 int gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream);
 

@@ -16,7 +16,7 @@ class Product(ctypes.Structure):
         ("in_ss", ctypes.c_void_p), ("in_tiles", ctypes.c_int), ("in_mul", ctypes.c_float), ("eps", ctypes.c_float), ("out_ss", ctypes.c_void_p),
         ("ss_mask", ctypes.c_int), ("part_stride", ctypes.c_longlong)] + [
         (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "out_seq")] + [("part_mul", ctypes.c_void_p)] + [
-        (n, ctypes.c_int) for n in ("blocks_across", "blocks_down", "shift_from", "shift_to")]
+        (n, ctypes.c_int) for n in ("blocks_across", "blocks_down", "shift_from", "shift_to", "quarters")]
 
 
 def _run(path=0, **kw):
@@ -288,3 +288,41 @@ def test_cache_of_all_layers_at_once_and_layer_by_layer(n, heads, layers):
     assert (got[:, :, 32 + n:] == 0).all() and torch.isfinite(got).all()
     for i in range(2 * layers):   # (the encoder's attention may be cut along its keys without an image head)
         assert (got[i].float() - want[i].float()).norm() <= 1.5e-3 * want[i].float().norm()
+
+
+@pytest.mark.parametrize("views,h,w", [(1, 8, 8), (3, 8, 8), (1, 16, 16), (4, 16, 16), (9, 16, 16), (1, 8, 24), (21, 8, 8)])
+@pytest.mark.parametrize("N,K", [(1024, 4096), (1024, 512), (256, 1536)])
+def test_sums_in_quarters(views, h, w, N, K):
+    """A residual product whose sum over K is that of its quarters: by clusters of four for few rows, by single CTAs for many. The sums and the
+    order of their addition are the same whoever makes them: a view's rows have the bits of the frame that it shares; and they are those of four
+    products of a quarter each, which leave fp32 nowhere, up to the distance of two orders."""
+    rnd = _gen(views * 100 + h * w + K)
+    M = views * h * w
+    a, wt = rnd(M, K), rnd(N, K, scale=K ** -0.5)
+    grid = rnd(views, h, w, N)
+    r = _to_blocks(grid, 0)
+    args = dict(W=wt, N=N, K=K, blocks_across=w // 4, blocks_down=h // 4, shift_from=0, shift_to=1, quarters=1)
+    out, raster = (torch.full((M, N), float("nan"), device="cuda", dtype=torch.half) for _ in range(2))
+    sums = torch.full((M * N // 32,), float("nan"), device="cuda")
+    tiles = _run(0, A=a, R=r, C=out, raster=raster, out_ss=sums, M=M, **args)
+    _check_sums(sums, tiles, out)
+    back = _to_blocks(torch.arange(M, device="cuda", dtype=torch.float32).view(views, h, w, 1), 0).long().flatten()
+    _near(raster[back], r.float() + a.float() @ wt.float().t(), K)
+    assert torch.equal(out, _to_blocks(raster.view(views, h, w, N), 4))
+    n = h * w
+    for v in {0, views - 1}:
+        alone, alone_raster = torch.full((n, N), float("nan"), device="cuda", dtype=torch.half), torch.full((n, N), float("nan"), device="cuda", dtype=torch.half)
+        alone_sums = torch.full((n * N // 32,), float("nan"), device="cuda")
+        _run(0, A=a[v * n:(v + 1) * n], R=r[v * n:(v + 1) * n], C=alone, raster=alone_raster, out_ss=alone_sums, M=n, **args)
+        assert torch.equal(alone, out[v * n:(v + 1) * n]) and torch.equal(alone_raster, raster[v * n:(v + 1) * n])
+        assert torch.equal(alone_sums, sums.view(views, -1)[v])
+
+
+def test_sums_in_quarters_are_refused_where_they_cannot_be():
+    f = Product()
+    x = torch.zeros(64, 1024, device="cuda", dtype=torch.half)
+    lib, tiles = _abi.load("rfk.h"), ctypes.c_int()
+    for n in ("A", "W", "R", "C"):
+        setattr(f, n, x.data_ptr())
+    f.M, f.N, f.K, f.quarters = 64, 256, 256, 1
+    assert lib.rfk_gemm_folded(ctypes.byref(f), ctypes.byref(tiles), None) == -2     # RFK_EUNSUPPORTED: 256 are not four stages
