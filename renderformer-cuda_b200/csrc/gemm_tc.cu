@@ -416,13 +416,13 @@ namespace pair { using namespace pair_ptx; }
 // block (one SM takes them at about 110 GB/s). But for the sums in quarters below every output is summed over the K blocks in the same order
 // as by the other kernels and has the same bits, so that a call may move between them with its size (the views of a frame
 // must equal the views one by one).
-//   Sums in quarters (SUM_): of a 64-row view's product with K = 4096 a CTA takes 64 K blocks of 64 x 32 columns one after the other, 7 us
-//   of loads on 32 SMs. The sum is therefore defined as ((a + b) + c) + d of its quarters of K for views of at most 128 rows, whatever frame they are in.
-//   For few rows a cluster of four CTAs takes a quarter each; the fp32 rows go to the CTA of their quarter of the tile through the cluster's shared
-//   memory, and one warp of it finishes 32 columns. For more rows one CTA keeps the four sums in accumulators of their own. us, one sum / quarters, K = 4096,
-//   N = 1024: 64 rows 8.7 / 5.8, 128 8.7 / 6.6, 192 8.9 / 8.5, 256 9.1 / 8.6, and on single CTAs 320 9.8 / 10.1, 1024 13.8 / 13.8; a view of 64 x 64
-//   pixels 539 / 508. With K = 1024 the exchange (1.2 us, 2.3 for tiles of 128 x 64) costs more than it gains (64 rows 3.67 / 3.97), and at 256 rows a
-//   view stays as it was (648 us), so these keep one sum.
+//   Sums in quarters (SUM_): of a 64-row view's product with K = 4096 a CTA takes 64 K blocks of 64 x 32 columns one after the other, 7 us of loads
+//   on 32 SMs, and with 256 rows the 128 tiles take 98 MB out of L2. The sum is therefore defined as ((a + b) + c) + d of its quarters of K for views of
+//   at most 256 rows, whatever frame they are in. For few rows a cluster of four CTAs takes a quarter each, of wider tiles; the fp32 rows go to the CTA
+//   of their quarter of the tile through the cluster's shared memory, and a warp of it finishes 32 columns. For more rows one CTA keeps the four
+//   sums in accumulators of their own. us, one sum / quarters, K = 4096, N = 1024: 64 rows 8.7 / 5.6, 128 8.7 / 6.3, 192 8.9 / 7.8, 256 9.1 / 7.9, and on single
+//   CTAs 320 9.8 / 10.0, 512 10.0 / 10.2, 1024 13.8 / 13.8; a view of 64 x 64 pixels 539 / 505, of 128 x 128 648 / 637, frames of four of these 847 / 843. With
+//   K = 1024 the exchange (0.8 to 1.5 us) costs more than it gains (64 rows 3.63 / 3.87): these keep one sum.
 //   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing lane and the producer's are
 //   elected ones (elect.sync). With one block per stage and lane 0's loops a K block took 0.30 us on every tile size, the cost
 //   of issuing and not of the operands; two blocks and elected lanes in loops of whole warps took the 64 x 32 tile to 0.12 us, loops of
@@ -454,10 +454,10 @@ struct __align__(8) Ctrl {
 };
 static_assert(sizeof(Ctrl) <= 256, "control block");
 
-// The pieces of a split sum on their way to the CTA that adds them: [the other pieces, its own][row of its quarter of the tile][BN_ floats and 16
-// bytes, which spread the banks]
-template <int BM_, int BN_> constexpr int kHandedPitch = BN_ * 4 + 16;
-template <int BM_, int BN_> constexpr int kHandedBytes = 4 * (BM_ / 4) * kHandedPitch<BM_, BN_>;
+// The pieces of a split sum on their way to the CTA that adds them: [the other pieces, its own][four columns][row of its quarter of the tile][4 floats], so
+// that a warp's stores into another CTA are 512 (256) bytes on end
+template <int BM_, int BN_> constexpr int kHandedPiece = (BM_ / 4) * BN_ * 4;
+template <int BM_, int BN_> constexpr int kHandedBytes = 4 * kHandedPiece<BM_, BN_>;
 
 // SUM 1: one sum over K. 4: ((a + b) + c) + d over the quarters of K, each a sum of its own; kSplit: by a cluster of four CTAs with a quarter each.
 enum : int { kSplit = 8 };
@@ -646,14 +646,14 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 res[q] = (row_ok && n0 + q * 8 < p.N && (!SPLIT || q / 4 == first_c)) ? *reinterpret_cast<const uint4*>(rrow + q * 8) : make_uint4(0, 0, 0, 0);
         }
         acc_ok = tc::mbar_wait_warp(&ctrl->acc_full, 0, abort_flag);
-        const int handed = C::kSmemBytes + (lane & (BM_ / 4 - 1)) * kHandedPitch<BM_, BN_>;   // the row's place, of the first piece
-        constexpr int kHandedPiece = (BM_ / 4) * kHandedPitch<BM_, BN_>;
+        constexpr int kRows = BM_ / 4, kPiece = kHandedPiece<BM_, BN_>;
+        const int handed = C::kSmemBytes + (lane & (kRows - 1)) * 16;   // the row's first four columns, of the first piece
         if (SPLIT) {                                          // a warp's rows to the CTA of their quarter
             pair::cluster_wait();
             if (acc_ok) {
                 tc::tc_fence_after();
                 const int slot = lane_grp == piece ? 3 : piece < lane_grp ? piece : piece - 1;
-                const uint32_t to = pair::map_to_cta(base + handed + slot * kHandedPiece, lane_grp);
+                const uint32_t to = pair::map_to_cta(base + handed + slot * kPiece, lane_grp);
 #pragma unroll
                 for (int c = 0; c < BN_ / 32; ++c) {
                     uint32_t v[32];
@@ -663,7 +663,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(to + c * 128 + q * 16), "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3]) : "memory");
+                                         ::"r"(to + (c * 8 + q) * kRows * 16), "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3]) : "memory");
                     }
                 }
             }
@@ -680,11 +680,11 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 uint32_t v[32], o[kChunk / 2];
                 if (!SPLIT) tc::tmem_ld32(t_acc + c * 32, v);
                 if (SPLIT) {                                  // ((a + b) + c) + d, whichever of them is this CTA's
-                    const float4* at = reinterpret_cast<const float4*>(smem_raw + handed + c * 128);
-                    constexpr int kPiece4 = kHandedPiece / 16;
+                    const float4* at = reinterpret_cast<const float4*>(smem_raw + handed) + c * 8 * kRows;
+                    constexpr int kPiece4 = kPiece / 16;
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        const float4 own = at[3 * kPiece4 + q], s0 = at[q], s1 = at[kPiece4 + q], s2 = at[2 * kPiece4 + q];
+                        const float4 own = at[3 * kPiece4 + q * kRows], s0 = at[q * kRows], s1 = at[kPiece4 + q * kRows], s2 = at[2 * kPiece4 + q * kRows];
                         const auto sum = [&](float o, float a0, float a1, float a2) {
                             const float x1 = piece <= 1 ? o : a1, x2 = piece <= 1 ? a1 : piece == 2 ? o : a2, x3 = piece <= 2 ? a2 : o;
                             return __float_as_uint(((a0 + x1) + x2) + x3);   // (pieces 0 and 1 either way round)

@@ -635,7 +635,7 @@ int rfk_layers::decoder_layer_folded(rfk_ctx* ctx, const rfk_decoder_layer_weigh
     g = onto_x(b.act, w->ffn.w2, ffn_hidden);
     g.C = next; g.raster = raster; g.out_ss = next ? b.x_ss : nullptr;
     g.blocks_across = patch_w / 4; g.blocks_down = patch_h / 4; g.shift_from = shift / 4; g.shift_to = next_shift / 4;
-    g.quarters = Sq <= 128 && ffn_hidden % 512 == 0;   // by the rows of a view, not of the frame: a view has the same bits alone and in any frame
+    g.quarters = Sq <= 256 && ffn_hidden % 512 == 0;   // by the rows of a view, not of the frame: a view has the same bits alone and in any frame
     return rfk::gemm_folded(g, &b.x_tiles, stream);
 }
 
