@@ -9,8 +9,9 @@
 //   src/layers/attention.cu:476-576      swin_self_attention
 //   src/layers/transformer.cu:151-224    decoder_layer_forward_cached, encoder_layer_forward_mixed
 //
-// What is re-cut here (launches per decoder layer: ~36 in the reference, 15 here plus the
-// rotation of the cached keys, which the session runs on a parallel graph branch):
+// What is re-cut here (launches per decoder layer: ~36 in the reference, 11 here and 8 where the
+// norms are folded into their products (decoder_layer_folded), plus the rotation of the cached
+// keys, which the session runs on a parallel graph branch):
 //   - residual add + RMSNorm (+ fp16 cast) is one kernel; the FFN residual of a layer is
 //     deferred into the first norm of the next layer;
 //   - QK-RMSNorm + [B,S,H,D]->[B,H,S,D] + RoPE (+ QKV de-interleave) is one kernel;
