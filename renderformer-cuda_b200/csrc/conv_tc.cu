@@ -92,6 +92,8 @@ struct Params {
     int tiles_m, tiles_n;             // pairs of boxes, blocks of BN output channels
     int cb, c_out;                    // blocks of 64 input channels; output channels
     int rows_outside, silu, has_res, dual;
+    const __half* sum;                // ADD: [N][H][W][c_out] to which the output is added (it may be the output)
+    int H, W;
 };
 
 // boxes of pixels: the maps have the columns' pixels (y) ahead of the rows' (x), see make_map_pixels
@@ -135,7 +137,10 @@ __device__ __forceinline__ void step(const Params& p, int& c, int& ty) {
     else if (++ty == 3) { ty = 0; ++c; }
 }
 
-template <int BN, int BX>
+// ADD: the output is what the epilogue has made so far plus p.sum, whose values a thread reads itself, half a unit ahead (the staging buffers hold the
+// residual). That takes a pass over four maps (19 us at 256 x 256 x 256) out of a fusion block: an image of 512 x 512 4957 -> 4877 us,
+// of 128 x 128 1086 -> 1082, of 320 x 320 no difference. Forms without it keep their registers.
+template <int BN, int BX, bool ADD>
 __global__ void __launch_bounds__(kThreads, (Cfg<BN, BX>::kCtas))
 conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r,
@@ -284,6 +289,21 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // this warp's 32 pixels, four columns of the box, and its first channel
             const int x0 = b.x + 4 * (lane_grp & (BX / 4 - 1)), n0 = (t / p.tiles_m) * BN + (C::kRows == 64 ? (lane_grp >> 1) * C::kAccCols : 0);
             const bool live = 2 * (t % p.tiles_m) + (int)rank < p.tiles;
+            // ADD: the thread's pixel of p.sum, 32 channels of which are fetched ahead of the half unit that adds them
+            const int px = x0 + (lane >> 3), py = b.y + (lane & 7);
+            const bool inside = ADD && live && px < p.W && py < p.H;
+            const __half* sum_row = ADD ? p.sum + ((size_t)(inside ? b.n : 0) * p.H * p.W + (inside ? (size_t)py * p.W + px : 0)) * p.c_out + n0 : nullptr;
+            uint4 add[ADD ? 4 : 1];
+            const auto fetch = [&](int half) {
+                if constexpr (ADD) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int ch = half * 32 + q * 8;
+                        add[q] = inside && ch < kUnits * kUnitCh && n0 + ch < p.c_out ? *reinterpret_cast<const uint4*>(sum_row + ch) : make_uint4(0, 0, 0, 0);
+                    }
+                }
+            };
+            fetch(0);
             if (lane == 0) {
                 bulk_wait_read<0>();   // the previous tile's stores have read the buffers
                 if (p.has_res) {
@@ -348,6 +368,15 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                             const float2 y = unpack_half2(o[i]), rr = unpack_half2(rw[i]);
                             o[i] = pack_half2(y.x + rr.x, y.y + rr.y);
                         }
+                    }
+                    if constexpr (ADD) {
+                        const uint32_t* aw = reinterpret_cast<const uint32_t*>(add);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 y = unpack_half2(o[i]), aa = unpack_half2(aw[i]);
+                            o[i] = pack_half2(aa.x + y.x, aa.y + y.y);
+                        }
+                        fetch(u * (kUnitCh / 32) + hc + 1);
                     }
                     if (p.dual) {
 #pragma unroll
@@ -457,7 +486,7 @@ template <int BN, int BX> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&a
 }
 
 // CTA pairs of the kernel that the device runs at once (asked once per device; 0: it cannot place them)
-template <int BN, int BX> int resident_pairs(int dev) {
+template <int BN, int BX, bool ADD = false> int resident_pairs(int dev) {
     static std::atomic<int> asked[64];   // the answer + 1
     int n = asked[dev].load(std::memory_order_acquire);
     if (n == 0) {
@@ -466,9 +495,9 @@ template <int BN, int BX> int resident_pairs(int dev) {
         int sms = 0, pairs = 0;
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tcconv::conv3x3_pair_kernel<BN, BX>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcconv::Cfg<BN, BX>::kSmemBytes);
+            e = cudaFuncSetAttribute(tcconv::conv3x3_pair_kernel<BN, BX, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcconv::Cfg<BN, BX>::kSmemBytes);
         cfg.gridDim = dim3(2 * std::max(1, sms / 2));
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&pairs, tcconv::conv3x3_pair_kernel<BN, BX>, &cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&pairs, tcconv::conv3x3_pair_kernel<BN, BX, ADD>, &cfg);
         if (e != cudaSuccess) { cudaGetLastError(); pairs = 0; }
         n = std::max(pairs, 0) + 1;
         asked[dev].store(n, std::memory_order_release);
@@ -476,7 +505,7 @@ template <int BN, int BX> int resident_pairs(int dev) {
     return n - 1;
 }
 
-template <int BN, int BX>
+template <int BN, int BX, bool ADD = false>
 int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap& mr, const CUtensorMap& ms, const __half* w,
                 tcconv::Params p, int dev, cudaStream_t st) {
     CUtensorMap mw;   // [C_out][9][C_in] as (c_in, c_out, tap)
@@ -484,13 +513,13 @@ int launch_conv(const CUtensorMap& mx, const CUtensorMap& mo, const CUtensorMap&
     const cuuint64_t dims[3] = {C_in, (cuuint64_t)p.c_out, 9}, strides[2] = {18 * C_in, 2 * C_in};
     const cuuint32_t box[3] = {64, BN / 2, 3};
     if (!make_map(&mw, w, 3, dims, strides, box)) return RFK_EUNSUPPORTED;
-    const int pairs = resident_pairs<BN, BX>(dev);
+    const int pairs = resident_pairs<BN, BX, ADD>(dev);
     if (pairs <= 0) return RFK_EUNSUPPORTED;
     p.tiles_n = ceil_div(p.c_out, BN);
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = pair_config<BN, BX>(attr, st);
     cfg.gridDim = dim3(2 * std::min(p.tiles_m * p.tiles_n, pairs));
-    cudaError_t e = cudaLaunchKernelEx(&cfg, tcconv::conv3x3_pair_kernel<BN, BX>, mx, mw, mo, mr, ms, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tcconv::conv3x3_pair_kernel<BN, BX, ADD>, mx, mw, mo, mr, ms, p);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_status();
 }
@@ -542,14 +571,13 @@ extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, con
     return resident_pairs<128, 16>(dev) > 0 && resident_pairs<64, 16>(dev) > 0 && resident_pairs<64, 8>(dev) > 0 && resident_pairs<32, 16>(dev) > 0;
 }
 
-extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
-                                      rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
-                                      rfk_stream_t stream) {
+static int conv3x3(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, const rfk_half* sum, rfk_half* out,
+                   rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile, rfk_stream_t stream) {
     if (!x || !w || !out || N < 0 || H <= 0 || W <= 0 || C_in <= 0 || C_out <= 0) return RFK_EINVAL;
     if (x == out || x == out_silu || out == out_silu) return RFK_EINVAL;   // a pixel is read by its neighbours' tiles
     if (tile < kByRule || tile > k32x128 || (tile == k128x128 && C_out % 128) || (tile == k32x128 && !resident_weights(C_in, C_out))) return RFK_EINVAL;
     if (N == 0) return RFK_OK;
-    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out)) return RFK_EUNSUPPORTED;
+    if (!conv_serves(x, w, bias, residual, out, out_silu, C_in, C_out) || (sum && (!aligned16(sum) || resident_weights(C_in, C_out)))) return RFK_EUNSUPPORTED;
     if (box_pairs(N, H, W, 8) * ceil_div(C_out, 64) > 0x1fffffffLL || 9LL * C_in > 0x7fffffffLL) return RFK_EUNSUPPORTED;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -572,8 +600,25 @@ extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, cons
     p.tiles_m = (p.tiles + 1) / 2;
     p.cb = C_in / 64; p.c_out = C_out;
     p.rows_outside = rows_outside != 0; p.silu = silu != 0; p.has_res = residual != nullptr; p.dual = out_silu != nullptr;
-    const auto launch = tile == k128x128 ? launch_conv<128, 16> : tile == k64x128 ? launch_conv<64, 16> : tile == k64x64 ? launch_conv<64, 8> : launch_conv<32, 16>;
+    p.sum = (const __half*)sum; p.H = H; p.W = W;
+    if (sum)
+        return (tile == k128x128 ? launch_conv<128, 16, true> : tile == k64x128 ? launch_conv<64, 16, true> : launch_conv<64, 8, true>)(
+            mx, mo, mr, ms, (const __half*)w, p, dev, as_stream(stream));
+    const auto launch = tile == k128x128 ? launch_conv<128, 16, false> : tile == k64x128 ? launch_conv<64, 16, false> : tile == k64x64 ? launch_conv<64, 8, false>
+                                            : launch_conv<32, 16, false>;
     return launch(mx, mo, mr, ms, (const __half*)w, p, dev, as_stream(stream));
+}
+
+extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
+                                      rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
+                                      rfk_stream_t stream) {
+    return conv3x3(x, w, bias, residual, nullptr, out, out_silu, N, H, W, C_in, C_out, silu, rows_outside, tile, stream);
+}
+
+extern "C" int rfk_conv3x3_nhwc_add(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* sum,
+                                    rfk_half* sum_silu, int N, int H, int W, int C_in, int C_out, int rows_outside, int tile, rfk_stream_t stream) {
+    if (!sum || !sum_silu || residual == sum || residual == sum_silu) return RFK_EINVAL;
+    return conv3x3(x, w, bias, residual, sum, sum, sum_silu, N, H, W, C_in, C_out, 0, rows_outside, tile, stream);
 }
 
 extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,

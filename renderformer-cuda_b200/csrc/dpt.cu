@@ -170,9 +170,11 @@ struct rfk_dpt {
 
     // o [B, Ho, Wo, Cout] = conv(in [B, H, W, Cin], weight [Cout, Cin, k, k] as the reference stores it) + bias, then SiLU
     // if silu, then + residual if given; o_silu (3x3, may be null) = SiLU of that.
+    // sum (3x3): instead of staying in o, that result is added to sum, and *sum_silu = SiLU of the new sum, in o or, once it is read, in `in`.
     // in == nullptr: the step reads feature tap `tap` ([B, pH*pW, dim] is [B, pH, pW, dim]).
     int add_conv(const rfk_half* in, int tap, const rfk_half* weight, const rfk_half* bias, rfk_half* o, int Cin, int H, int W,
-                 int Cout, int k, int stride, int pad, bool silu = false, const rfk_half* residual = nullptr, rfk_half* o_silu = nullptr) {
+                 int Cout, int k, int stride, int pad, bool silu = false, const rfk_half* residual = nullptr, rfk_half* o_silu = nullptr,
+                 rfk_half* sum = nullptr, rfk_half** sum_silu = nullptr) {
         const int Ho = (H + 2 * pad - k) / stride + 1, Wo = (W + 2 * pad - k) / stride + 1;
         const long long rows_out = (long long)B * Ho * Wo;
         ++n_convs;
@@ -196,6 +198,13 @@ struct rfk_dpt {
                              rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout);
         const auto push_own = [&](int rows_outside) {
             if (large_map(H, W, Cin, Cout, sms)) ++n_own;
+            if (sum) {
+                *sum_silu = o;
+                program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
+                    return rfk_conv3x3_nhwc_add(in, wk, bias, residual, sum, o, 1, H, W, Cin, Cout, rows_outside, 0, (rfk_stream_t)st);
+                });
+                return RFK_OK;
+            }
             program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
                 return rfk_conv3x3_nhwc_tiled(in, wk, bias, residual, o, o_silu, 1, H, W, Cin, Cout, silu, rows_outside, 0, (rfk_stream_t)st);
             });
@@ -225,12 +234,15 @@ struct rfk_dpt {
         }
         ws_bytes = std::max(ws_bytes, ws);
         ++n_library;
+        rfk_half* const read = const_cast<rfk_half*>(in);
+        if (sum) *sum_silu = read;
         rfk_dpt* self = this;
         program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
             const float one = 1.0f, zero = 0.0f;
             DNN_TRY(cudnnSetStream(self->dnn, st));
             DNN_TRY(cudnnConvolutionForward(self->dnn, &one, xd, in, fd, wk, cd, algo, self->workspace, ws, &zero, yd, o));
             if (bias || silu || residual) TRY(rfk_bias_act_residual_nhwc(o, bias, residual, rows_out, Cout, silu, (rfk_stream_t)st));
+            if (sum) return rfk_residual_add_silu_nhwc(sum, o, read, rows_out * Cout, (rfk_stream_t)st);
             if (o_silu) return rfk_silu(o, o_silu, rows_out * Cout, (rfk_stream_t)st);
             return RFK_OK;
         });
@@ -261,12 +273,13 @@ struct rfk_dpt {
 
     // residual convolution unit (src/layers/dpt.cu:397-409): y <- conv2(silu(conv1(y))) + x, where y holds silu(x), which whatever made x
     // has left there; x is left as it was. *spare: a buffer of the same size that nothing needs any more once the unit is done.
-    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, rfk_half* y, int F, int H, int W, rfk_half** spare) {
+    // path: the result is added to it instead, and *spare = SiLU of the new path.
+    int add_rcu(const rfk_rcu_weights& r, const rfk_half* x, rfk_half* y, int F, int H, int W, rfk_half** spare, rfk_half* path = nullptr) {
         rfk_half* t = alloc((size_t)B * F * H * W);
         if (!t) return (int)cudaErrorMemoryAllocation;
         TRY(add_conv(y, -1, r.conv1_w, r.conv1_b, t, F, H, W, F, 3, 1, 1, /*silu=*/true));
-        TRY(add_conv(t, -1, r.conv2_w, r.conv2_b, y, F, H, W, F, 3, 1, 1, /*silu=*/false, /*residual=*/x));
-        *spare = t;
+        TRY(add_conv(t, -1, r.conv2_w, r.conv2_b, y, F, H, W, F, 3, 1, 1, /*silu=*/false, /*residual=*/x, nullptr, path, spare));
+        if (!path) *spare = t;
         return RFK_OK;
     }
 
@@ -279,12 +292,7 @@ struct rfk_dpt {
         const long long n = (long long)B * F * ph * pw;
         if (f.has_resconv1) {
             if (!lr) return RFK_EINVAL;
-            rfk_half* s = nullptr;
-            TRY(add_rcu(f.rcu1, lr, lr_silu, F, ph, pw, &s));
-            program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
-                return rfk_residual_add_silu_nhwc(path_in, lr_silu, s, n, (rfk_stream_t)st);
-            });
-            path_silu = s;
+            TRY(add_rcu(f.rcu1, lr, lr_silu, F, ph, pw, &path_silu, path_in));
         } else if (!path_silu) {
             rfk_half* s = alloc((size_t)n);
             if (!s) return (int)cudaErrorMemoryAllocation;

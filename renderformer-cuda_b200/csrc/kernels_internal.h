@@ -133,6 +133,11 @@ extern "C" int rfk_conv3x3_nhwc(const rfk_half* x, const rfk_half* w, const rfk_
 extern "C" int rfk_conv3x3_nhwc_tiled(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* out,
                                       rfk_half* out_silu, int N, int H, int W, int C_in, int C_out, int silu, int rows_outside, int tile,
                                       rfk_stream_t stream);
+// sum += half(half(half(conv) + bias) + residual) and sum_silu = silu(sum): a residual unit's second convolution, the sum into the path and the SiLU that
+// opens the next unit (rfk_residual_add_silu_nhwc), with the bits of the separate steps. sum and sum_silu must not be x, residual or one another; not for
+// the shapes whose weights stay resident (RFK_EUNSUPPORTED).
+extern "C" int rfk_conv3x3_nhwc_add(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual, rfk_half* sum,
+                                    rfk_half* sum_silu, int N, int H, int W, int C_in, int C_out, int rows_outside, int tile, rfk_stream_t stream);
 // whether it takes these operands on the current device
 extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, const rfk_half* bias, const rfk_half* residual,
                                        const rfk_half* out, const rfk_half* out_silu, int C_in, int C_out);

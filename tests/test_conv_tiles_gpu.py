@@ -84,6 +84,23 @@ def test_epilogues_equal_the_separate_operators(tile, N, H, W, C, K):
         assert torch.equal(got, want) and torch.equal(got_act, act)
 
 
+@pytest.mark.parametrize("tile,N,H,W,C,K", [c for c in CASES if c[0] != T32x128 and not (c[4] <= 128 and c[5] == 32)])
+def test_sum_into_the_path_equals_the_separate_operators(tile, N, H, W, C, K):
+    L = _lib()
+    L.rfk_conv3x3_nhwc_add.argtypes, L.rfk_conv3x3_nhwc_add.restype = [VP] * 6 + [ctypes.c_int] * 7 + [VP], ctypes.c_int
+    L.rfk_residual_add_silu_nhwc.argtypes, L.rfk_residual_add_silu_nhwc.restype = [VP] * 3 + [ctypes.c_longlong, VP], ctypes.c_int
+    x, w, bias, residual = _operands(N, H, W, C, K)
+    st = VP(torch.cuda.current_stream().cuda_stream)
+    path = torch.randn(N, H, W, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(H)).half()
+    for b, r in [(bias, residual), (None, None)]:
+        unit, want, want_silu = _conv(x, w, b, r, False, False, tile), path.clone(), torch.empty_like(path)
+        assert L.rfk_residual_add_silu_nhwc(_p(want), _p(unit), _p(want_silu), want.numel(), st) == 0
+        got, got_silu = path.clone(), torch.full_like(path, 7.0)
+        assert L.rfk_conv3x3_nhwc_add(_p(x), _p(w), _p(b), _p(r), _p(got), _p(got_silu), N, H, W, C, K, 0, tile, st) == 0
+        assert torch.equal(got, want) and torch.equal(got_silu, want_silu)
+    assert L.rfk_conv3x3_nhwc_add(_p(x), _p(w), None, _p(got), _p(got), _p(got_silu), N, H, W, C, K, 0, tile, st) == -1
+
+
 def test_refuses_tiles_that_do_not_take_the_shape():
     x, w, _, _ = _operands(1, 8, 8, 64, 96)
     out = torch.full((1, 8, 8, 96), 7.0, device="cuda", dtype=torch.float16)
