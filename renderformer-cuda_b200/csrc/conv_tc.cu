@@ -138,7 +138,7 @@ __device__ __forceinline__ void step(const Params& p, int& c, int& ty) {
 }
 
 // ADD: the output is what the epilogue has made so far plus p.sum, whose values a thread reads itself, half a unit ahead (the staging buffers hold the
-// residual). That takes a pass over four maps (19 us at 256 x 256 x 256) out of a fusion block: an image of 512 x 512 4957 -> 4877 us,
+// residual). That takes a pass over four maps (19 us at 256 x 256 x 256) out of a fusion block: an image of 512 x 512 4930 -> 4877 us,
 // of 128 x 128 1086 -> 1082, of 320 x 320 no difference. Forms without it keep their registers.
 template <int BN, int BX, bool ADD>
 __global__ void __launch_bounds__(kThreads, (Cfg<BN, BX>::kCtas))
