@@ -905,7 +905,6 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // CTA 1's copies count on CTA 0's barrier.
 namespace pair {
 
-constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA, of which a tile of 192 columns leaves 4 free
 // The epilogue goes through shared memory both ways: an epilogue warp owns staging buffers of 32 rows x 64 halves
 // (4 KB, the 128-byte-swizzled layout of a TMA box) for its 32 rows of the tile; it writes the finished fp16 values
 // of 64 output columns there and one lane issues a TMA tile store, so the global writes are whole 128-byte lines
@@ -919,17 +918,18 @@ constexpr int kStageBytes = kABytes + kWBoxBytes;   // 32 KB per CTA, of which a
 // a tail of N - ends in the buffer that the next one begins with, whose last store may still be reading it.)
 constexpr int kUnitCols = 64;
 constexpr int kUnitBytes = 32 * kUnitCols * 2;       // 4 KB
-// BN: accumulator columns of a tile, 256 or 192 (narrow_tile)
+// BN: accumulator columns of a tile, 256 or 192 (narrow_tile); 128 with SwiGLU (narrow_gate)
 template <int EPI_, int BN> struct Cfg {
     static constexpr int EPI = EPI_ & 7;
-    static constexpr int kUnits = (EPI == RFK_GEMM_EPI_SWIGLU) ? 2 : BN / 64;              // 64-column units per tile
+    static constexpr int kStageBytes = kABytes + (BN == 128 ? 64 * BK * 2 : kWBoxBytes);   // 32 KB per CTA, of which a tile of 192 columns leaves 4 free, or 24
+    static constexpr int kUnits = (EPI == RFK_GEMM_EPI_SWIGLU) ? BN / 128 : BN / 64;       // 64-column units per tile
     static constexpr int kBufsPerWarp = (EPI == RFK_GEMM_EPI_RESIDUAL) ? 4 : 2;
     static constexpr int kStagingBytes = 4 * kBufsPerWarp * kUnitBytes;                      // 4 epilogue warps
-    static constexpr int kStages = (EPI == RFK_GEMM_EPI_RESIDUAL) ? 5 : 6;
+    static constexpr int kStages = BN == 128 ? 8 : (EPI == RFK_GEMM_EPI_RESIDUAL) ? 5 : 6;
     static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 512;
     static_assert(kSmemBytes + 1024 <= 227 * 1024, "one CTA per SM");
 };
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8;
 
 struct __align__(8) Ctrl {
     uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], drain;
@@ -1017,7 +1017,7 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
             if (EPI == RFK_GEMM_EPI_SWIGLU) {
                 uint32_t up[32];
                 tc::tmem_ld32(t_acc + c32 * 32, v);          // gate columns
-                tc::tmem_ld32(t_acc + 128 + c32 * 32, up);   // up columns of the same hidden units
+                tc::tmem_ld32(t_acc + BN / 2 + c32 * 32, up);   // up columns of the same hidden units
                 tc::tc_wait_ld(v);
                 tc::tc_wait_ld(up);
                 if (FOLD) {
@@ -1129,8 +1129,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const __grid_constant__ CUtensorMap map_r, const Params p) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & kFold) != 0;
-    static_assert(BN == 256 || (BN == 192 && EPI != RFK_GEMM_EPI_SWIGLU), "whole 64-column units");
-    constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? 128 : BN;
+    static_assert(BN == 256 || (BN == 192 && EPI != RFK_GEMM_EPI_SWIGLU) || (BN == 128 && EPI == RFK_GEMM_EPI_SWIGLU), "whole 64-column units");
+    constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? BN / 2 : BN;
+    constexpr int kStageBytes = Cfg<EPI, BN>::kStageBytes;
     constexpr int kTxBytes = kABytes + BN / 2 * BK * 2;   // of a stage, per CTA
     constexpr int kStages = Cfg<EPI, BN>::kStages;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -1451,7 +1452,8 @@ int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUten
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = pair_config<EPI_, BN>(attr, st);
     p.tiles_m = (p.M + 2 * tcgemm::BM - 1) / (2 * tcgemm::BM);
-    if (BN != 256) p.tiles_n = (p.N + BN - 1) / BN;
+    constexpr int BN_OUT = EPI == RFK_GEMM_EPI_SWIGLU ? BN / 2 : BN;
+    p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
     const int tiles = p.tiles_m * p.tiles_n;
     cfg.gridDim = dim3(2 * std::min(tiles, pairs));
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mw0, mw1, mc, mr, p);
@@ -1601,6 +1603,21 @@ int heads_tile(int M, int N, const int* resident) {
     return 0;
 }
 
+// Gate products whose small tiles would be 128 x 128: pairs with 64 hidden units each (128 accumulator columns), if they all run at once. A pair's CTA takes 24 KB
+// a K block where a small tile takes 32, and 256 x 4096 hidden x 1024 is bound by what comes out of L2. us, small tiles / these, weights from HBM: 256 rows
+// 8.10 / 7.59, 192 rows 7.98 / 7.57; a view of 128 x 128 pixels 634 / 630, an image of it 1087 / 1077, sixteen views of 64 x 64 in frames of four 2048 / 2014,
+// an encoding of 200 triangles 604 / 595. RFK_EUNSUPPORTED: not that one.
+template <int EPI_>
+int launch_narrow_gate(const void* A, long long lda, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev, cudaStream_t st) {
+    int pairs = 0;
+    if (small_tile(p.M, 2 * p.N, sm_count(dev)) != 4) return RFK_EUNSUPPORTED;
+    const int rc = resident_pairs<EPI_, 128>(dev, &pairs);
+    if (rc != RFK_OK || (long long)ceil_div(p.M, 256) * ceil_div(p.N, 64) > pairs) return RFK_EUNSUPPORTED;
+    CUtensorMap ma, mw0, mw1;
+    if (!make_map_2d(&ma, A, p.M, p.K, lda) || !make_map_2d(&mw0, W, p.N, p.K, ldw, 64) || !make_map_2d(&mw1, W_up, p.N, p.K, ldw, 64)) return RFK_EUNSUPPORTED;
+    return launch_pair_tiles<EPI_, 128>(ma, mw0, mw1, p, dev, st, nullptr);
+}
+
 // path 0: small tiles or CTA pairs; path 2: CTA pairs; the single-CTA kernel if pairs are unavailable; path 3: that kernel
 template <int EPI>
 int launch_gemm(const void* A, long long lda, const void* W, const void* W_up, long long ldw, const tcgemm::Params& p, int dev,
@@ -1609,6 +1626,8 @@ int launch_gemm(const void* A, long long lda, const void* W, const void* W_up, l
     const int path = g_gemm_path.load(std::memory_order_relaxed);
     if (path == 0) {
         int rc = RFK_EUNSUPPORTED;
+        if constexpr (kGate) rc = launch_narrow_gate<EPI>(A, lda, W, W_up, ldw, p, dev, st);
+        if (rc != RFK_EUNSUPPORTED) return rc;
         switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
             case 1: rc = launch_gemm_small<EPI, 64, 32>(A, lda, W, W_up, ldw, p, dev, st); break;
             case 2: rc = launch_gemm_small<EPI, 64, 64>(A, lda, W, W_up, ldw, p, dev, st); break;
@@ -1784,6 +1803,8 @@ static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cuda
         *ss_tiles = sums;
         if constexpr (EPI == RFK_GEMM_EPI_RESIDUAL)
             if (f.quarters) return launch_quarters(f, p, dev, st);
+        if constexpr (kGate) rc = launch_narrow_gate<E>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st);
+        if (rc != RFK_EUNSUPPORTED) return rc;
         switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {
             case 1: rc = launch_gemm_small<E, 64, 32>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
             case 2: rc = launch_gemm_small<E, 64, 64>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st); break;
