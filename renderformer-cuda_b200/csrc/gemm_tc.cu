@@ -1792,6 +1792,17 @@ static int launch_quarters(const FoldedProduct& f, const tcgemm::Params& p, int 
     }
 }
 
+// small tiles, by the size of a product (SwiGLU aside)
+static bool folded_small(int M, int N, int dev) {
+    return g_gemm_path.load(std::memory_order_relaxed) == 0 && small_tile(M, N, sm_count(dev)) != 0;
+}
+
+bool rfk::folded_on_pairs(int M, int N) {
+    int dev = 0;
+    if (M <= 0 || N <= 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return false; }
+    return !folded_small(M, N, dev);
+}
+
 template <int EPI>
 static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cudaStream_t st, int* ss_tiles) {
     constexpr int E = EPI | tcgemm::kFold;
@@ -1824,7 +1835,7 @@ static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cuda
     return launch_gemm_pair<E>(ma, f.W, f.W_up, p.K, p, dev, st, EPI == tcgemm::kEpiHeads ? &mh : nullptr, p.raster ? &mraster : nullptr, ss_tiles);
 }
 
-int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream) {
+int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream, const FoldedMore& more) {
     const bool residual = f.R != nullptr, heads = f.num_heads > 0, gate = f.W_up != nullptr;
     if (!f.A || !f.W || (!f.C && !f.raster) || f.M <= 0 || f.N <= 0 || f.K <= 0 || residual + heads + gate != 1 || !ss_tiles) return RFK_EINVAL;
     if (!residual && (!f.in_ss || f.in_tiles <= 0)) return RFK_EINVAL;
@@ -1846,6 +1857,8 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return RFK_EUNSUPPORTED;
+    // (pairs of 192 columns write sums of 32 too: head-split products of several parts have none, see launch_gemm_pair)
+    if (more.pairs && (!heads || f.N == dim || !f.out_ss || folded_small(f.M, f.N, dev))) return RFK_EUNSUPPORTED;
     tcgemm::Params p{};
     p.C = (__half*)f.C; p.ldc = f.N; p.R = (const __half*)f.R; p.ldr = f.N;
     p.M = f.M; p.N = f.N; p.K = f.K;
@@ -1866,6 +1879,10 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream)
 }
 
 extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream) { return f ? rfk::gemm_folded(*f, ss_tiles, stream) : RFK_EINVAL; }
+extern "C" int rfk_gemm_folded_more(const rfk::FoldedProduct* f, const rfk::FoldedMore* more, int* ss_tiles, rfk_stream_t stream) {
+    return f && more ? rfk::gemm_folded(*f, ss_tiles, stream, *more) : RFK_EINVAL;
+}
+extern "C" int rfk_folded_on_pairs(int M, int N) { return rfk::folded_on_pairs(M, N); }
 
 extern "C" int rfk_gemm_heads_tile(int M, int N, const int* resident) {
     return M > 0 && N > 0 && resident ? heads_tile(M, N, resident) : RFK_EINVAL;

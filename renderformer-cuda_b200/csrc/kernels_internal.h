@@ -28,7 +28,13 @@ struct FoldedProduct {
     int blocks_across, blocks_down, shift_from, shift_to;   // 0: rows stay where they are
     int quarters;                                           // residual: the sum over K is ((a + b) + c) + d of its quarters (K % 512 == 0), whatever M
 };
-int gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream);
+struct FoldedMore {
+    int pairs;      // CTA pairs with one sum each 256 columns, which read W behind the kernel before, or RFK_EUNSUPPORTED: small tiles write one each
+                    // 32 columns, and ask for W while the kernel before may still be writing it
+};
+int gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream, const FoldedMore& more = {});
+// whether a product (SwiGLU aside) goes to the pairs of FoldedMore::pairs, by its size
+bool folded_on_pairs(int M, int N);
 
 // The tokens that enter a view's folded layers, 1024 wide (else RFK_EUNSUPPORTED): x = half(half(rmsnorm(e) * gamma) + token), with the bits of the
 // separate steps, and its rows' sums of squares row_ss [rows][4]. e is a token grid in raster order, x in the block order of gemm_folded, of
@@ -148,7 +154,9 @@ extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_ha
 extern "C" int rfk_embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
                                 int blocks_across, int blocks_down, rfk_stream_t stream);   // embed_tokens and fold_norm_weights, for their tests
 extern "C" int rfk_fold_norm_weights(const rfk_half* w, rfk_half* out, const float* gamma, float mul, int rows, int cols, rfk_stream_t stream);
-extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream);   // gemm_folded, for its test
+extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream);   // gemm_folded and folded_on_pairs, for their tests
+extern "C" int rfk_gemm_folded_more(const rfk::FoldedProduct* f, const rfk::FoldedMore* more, int* ss_tiles, rfk_stream_t stream);
+extern "C" int rfk_folded_on_pairs(int M, int N);
 // rfk_rmsnorm_residual_f16_windows for operands that the kernels before have just written (the layers' case): the same values, another
 // split of the rows (one_warp_per_row in rmsnorm.cu)
 extern "C" int rfk_rmsnorm_residual_f16_windows_in_l2(rfk_half* x, const rfk_half* r, const float* gamma, rfk_half* y, int B, int H, int W,

@@ -570,11 +570,14 @@ struct EncodeBuffers {
 // alone: with those in the products' weights (folded anew each time, 96 MB of traffic) they are one product of 24576 columns, whose
 // tiles fill the SMs where 92 of one layer's left a third of them idle, stored head-split in the cache; then the keys' own norm in
 // place, all layers at once. 5633 triangles: 12 x 43 us (norm, product, transposing norm, product, two memsets) -> 280 (folding 21, product 190 = 1.5
-// PFLOP/s, norm 46, context rows 8), scenes of 60 triangles 735 -> 547 us in all, 1000 1275 -> 1106, 5633 5500 -> 5250. RFK_EUNSUPPORTED with nothing but work space written: layer by layer instead.
+// PFLOP/s, norm 46, context rows 8), scenes of 60 triangles 735 -> 547 us in all, 1000 1275 -> 1106, 5633 5500 -> 5250. RFK_EUNSUPPORTED with nothing but work
+// space written: layer by layer instead. That is known ahead of all work where few layers and rows make a product of small tiles (up to 1152 rows of one
+// layer, 128 of nine), whose weights would be folded for too little and whose sums are more than kv_ss has room for.
 static int encode_kv(rfk_session& d, EncodeBuffers& b, const float* ctx_ss) {
     const rfk_model& m = d.m;
     const rfk_stream_t s = (rfk_stream_t)d.stream;
     const int layers = m.dec_layers, dim = m.dim, Se = d.Se, Se_pad = d.Se_pad, hd = d.hd;
+    if (!rfk::folded_on_pairs(Se, 2 * layers * dim)) return RFK_EUNSUPPORTED;
     const rfk_half *k[RFK_MAX_LAYERS], *v[RFK_MAX_LAYERS];
     const float *gamma[RFK_MAX_LAYERS], *key_gamma[RFK_MAX_LAYERS];
     for (int i = 0; i < layers; ++i) {
@@ -588,8 +591,7 @@ static int encode_kv(rfk_session& d, EncodeBuffers& b, const float* ctx_ss) {
     p.eps = kEpsFp16; p.out_ss = b.kv_ss; p.ss_mask = 0x55555555; p.part_stride = slab; p.seq = Se; p.out_seq = Se_pad; p.num_heads = m.num_heads;
     p.head_dim = hd; p.part_mul = b.kv_mul;
     int tiles = 0;
-    TRY(rfk::gemm_folded(p, &tiles, s));
-    if (tiles != dim / 256) return RFK_EUNSUPPORTED;   // small tiles: not with this many columns
+    TRY(rfk::gemm_folded(p, &tiles, s, {/*pairs=*/1}));
     if (Se_pad != Se) {   // the rows behind the last key of each head
         const size_t row = (size_t)hd * 2;
         TRY_CUDA(cudaMemset2DAsync((char*)d.kvK(0) + Se * row, Se_pad * row, 0, (Se_pad - Se) * row, (size_t)2 * layers * m.num_heads, d.stream));

@@ -270,6 +270,38 @@ def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts,
     assert torch.allclose(s[0::2], want[0::2], rtol=2e-5, atol=1e-6)
 
 
+class More(ctypes.Structure):
+    _fields_ = [("pairs", ctypes.c_int)]
+
+
+# both sides of the line, which is 148 tiles of 128 x 128 on 148 SMs: 1 layer of keys and values, 3, 9 and 12
+@pytest.mark.parametrize("M,parts,small", [(92, 6, True), (1152, 2, True), (1153, 2, False), (128, 18, True), (129, 18, False), (33, 24, False)])
+def test_sums_of_256_columns_or_nothing(M, parts, small):
+    """Whoever has room for one sum each 256 columns asks for pairs: small tiles, which write eight times as many, are refused before anything is written."""
+    lib = _abi.load("rfk.h")
+    assert lib.rfk_folded_on_pairs(M, parts * 1024) == (not small)
+    rnd = _gen(M)
+    K = dim = 1024
+    x, w = rnd(M, K), rnd(parts * dim, K, scale=K ** -0.5)
+    ss = x.float().square().view(M, 4, -1).sum(-1).contiguous()
+    out = torch.full((parts, 16, M, 64), 7.0, device="cuda", dtype=torch.half)
+    sums, n = torch.full((2 * parts * M * 4,), -1.0, device="cuda"), parts * M * 4
+    f, more, tiles = Product(), More(pairs=1), ctypes.c_int()
+    for k, v in dict(A=x, W=w, C=out, M=M, N=parts * dim, K=K, in_ss=ss, in_tiles=4, in_mul=1.0, eps=EPS, out_ss=sums, ss_mask=0x55555555,
+                     part_stride=dim * M, seq=M, num_heads=16, head_dim=64).items():
+        setattr(f, k, v.data_ptr() if torch.is_tensor(v) else v)
+    rc = lib.rfk_gemm_folded_more(ctypes.byref(f), ctypes.byref(more), ctypes.byref(tiles), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert (sums[n:] == -1.0).all()
+    if small:
+        assert rc == -2 and (sums == -1.0).all() and (out == 7.0).all()
+        return
+    assert rc == 0 and tiles.value == 4
+    got = out.permute(2, 0, 1, 3).reshape(M, parts * dim)
+    _near(got, (x.float() @ w.float().t()) * _factor(x, 1.0), K)
+    want = got.float().square().view(M, parts, 4, -1).sum(-1).permute(1, 0, 2)
+    assert torch.allclose(sums[:n].view(parts, M, 4)[0::2], want[0::2], rtol=2e-5, atol=1e-6)
+
+
 @pytest.mark.parametrize("n,heads,layers", [(1, 16, 1), (60, 16, 3), (333, 8, 12), (1100, 16, 12), (2600, 8, 2)])
 def test_cache_of_all_layers_at_once_and_layer_by_layer(n, heads, layers):
     """1024-wide rows: sessions with an image head keep one norm, two products and a transposing norm a layer; sessions without take one product."""
