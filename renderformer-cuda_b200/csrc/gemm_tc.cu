@@ -117,12 +117,16 @@ struct Params {
     int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
     const float* in_ss; int in_tiles, in_group;    // kFold: A's rows' sums of squares, how many a row, and how many of them make up 256 columns
     float in_inv_dim, in_eps, in_mul;              // the row's factor: in_mul * rsqrt(sum * in_inv_dim + in_eps)
-    const float* part_mul;                         // kEpiHeads: if not null, another factor for each part
+    const float* col_mul; int mul_units;           // kEpiHeads: if not null, another factor for each mul_units * 64 columns
     int ss_tiles;                                  // kFold: sums a row that row_ss gets, of a part
     __half* raster;                                // kFold, residual: the rows in raster order too, or alone if C is null; pitch ldc
     Grid grid;
 };
 
+// the further factor of the columns that begin at col, a multiple of 64 or inside one (kFold)
+__device__ __forceinline__ float column_factor(const Params& p, int col) {
+    return p.col_mul ? __ldg(p.col_mul + min(col, p.N - 1) / 64 / p.mul_units) : 1.0f;
+}
 // a row's factor (kFold)
 __device__ __forceinline__ float row_factor(const Params& p, int row) {
     const float* s = p.in_ss + (size_t)row * p.in_tiles;
@@ -635,8 +639,10 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 rrow2 = p.raster + (at * (p.grid.bw * 4) + bx * 4 + (row & 3)) * p.ldc + n0;
             }
         }
-        float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
-        if (FOLD && EPI == kEpiHeads && p.part_mul) factor *= __ldg(p.part_mul + n0 / (p.units * 64));
+        float factors[BN_OUT > 64 ? 2 : 1];                   // of the row, in each 64 columns
+        factors[0] = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
+        if constexpr (BN_OUT > 64) factors[1] = FOLD && EPI == kEpiHeads ? factors[0] * column_factor(p, n0 + 64) : factors[0];
+        if (FOLD && EPI == kEpiHeads) factors[0] *= column_factor(p, n0);
         constexpr int kChunk = BN_OUT < 32 ? BN_OUT : 32;     // output columns per step
         uint4 res[EPI == RFK_GEMM_EPI_RESIDUAL ? BN_OUT / 8 : 1];
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                   // the row's residual arrives while the products run
@@ -687,6 +693,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             for (int c = 0; c < BN_OUT / kChunk; ++c) {
                 if (n0 + c * kChunk >= p.N) break;            // uniform over the CTA: the tile's tail lies beyond N
                 if (SPLIT && c != first_c) continue;
+                const float factor = factors[c * kChunk / 64];
                 uint32_t v[32], o[kChunk / 2];
                 if (!SPLIT) tc::tmem_ld32(t_acc + c * 32, v);
                 if (SPLIT) {                                  // ((a + b) + c) + d, whichever of them is this CTA's
@@ -969,10 +976,10 @@ __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* ma
 
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
 // t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0. turn: the staging buffer of the
-// next store, kept from tile to tile (not with the residual epilogue).
+// next store, kept from tile to tile (not with the residual epilogue). FOLD: row_mul is the row's factor; lane u holds that of the tile's unit u.
 template <int EPI_, int BN>
-__device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, uint32_t t_acc, float factor,
-                                                     unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
+__device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, uint32_t t_acc,
+                                                     float row_mul, float unit_mul, unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
                                                      int row0, int n0, int lane, int& turn, volatile int* abort_flag) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & kFold) != 0;
@@ -999,6 +1006,7 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     for (int u = 0; u < kUnits; ++u) {
         const uint32_t bias_unit = bias_next;
         bias_next = bias_of(u + 1);
+        const float factor = FOLD && EPI == kEpiHeads ? row_mul * __shfl_sync(0xffffffffu, unit_mul, u) : row_mul;
         const int b = (EPI == RFK_GEMM_EPI_RESIDUAL) ? u : turn;
         unsigned char* buf = stage_ptr + b * kUnitBytes;
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                 // this unit's residual box has landed (also for units beyond N)
@@ -1271,14 +1279,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
                 epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
-            float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
-            if (FOLD && EPI == kEpiHeads && p.part_mul) factor *= __ldg(p.part_mul + n0 / (p.units * kUnitCols));
+            const float row_mul = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
+            const float unit_mul = FOLD && EPI == kEpiHeads ? column_factor(p, n0 + min(lane, BN_OUT / kUnitCols - 1) * kUnitCols) : 1.0f;
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(4);   // first tile's accumulator complete
-            ok = epilogue_tile_staged<EPI_, BN>(p, &map_c, &map_w1, tmem_cta + lane_off + acc * BNACC, factor, my_stage, my_res, tl & 1, row0, n0,
-                                           lane, turn, abort_flag);
+            ok = epilogue_tile_staged<EPI_, BN>(p, &map_c, &map_w1, tmem_cta + lane_off + acc * BNACC, row_mul, unit_mul, my_stage, my_res, tl & 1,
+                                                  row0, n0, lane, turn, abort_flag);
             if (!ok) break;
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(5);   // its epilogue done (stores issued)
             // every tcgen05.ld of this warp has completed: hand the accumulator back
@@ -1870,7 +1878,7 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream,
     p.raster = (__half*)f.raster;
     p.grid = tcgemm::Grid{f.blocks_across, f.blocks_down, f.shift_from, f.shift_to};
     if (heads) {
-        p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.part_mul = f.part_mul; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
+        p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.col_mul = f.part_mul; p.mul_units = p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
         p.part_stride = f.N > dim ? f.part_stride : (long long)f.M * dim;
     }
     const cudaStream_t st = as_stream(stream);

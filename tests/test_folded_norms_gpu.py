@@ -270,6 +270,25 @@ def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts,
     assert torch.allclose(s[0::2], want[0::2], rtol=2e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("M,parts", [(256, 3), (3136, 3), (4096, 2)])
+def test_factors_of_parts_without_sums(M, parts):
+    """3136 rows: pair tiles of 192 columns, which cross from one part of 512 into the next."""
+    lib = _abi.load("rfk.h")
+    assert M != 3136 or lib.rfk_gemm_pair_tile(M, parts * 512, 74) == 192
+    rnd = _gen(M + parts)
+    K, dim, hd = 512, 512, 64
+    x, w = rnd(M, K), rnd(parts * dim, K, scale=K ** -0.5)
+    ss = x.float().square().view(M, K // 256, -1).sum(-1).contiguous()
+    mul = 2.0 ** (3 * torch.arange(parts, device="cuda")).float()
+    out = torch.full((parts, 1, dim // hd, M, hd), float("nan"), device="cuda", dtype=torch.half)
+    _run(A=x, W=w, C=out, M=M, N=parts * dim, K=K, in_ss=ss, in_tiles=K // 256, in_mul=1.0, part_stride=M * dim, seq=M, num_heads=dim // hd, head_dim=hd,
+         part_mul=mul)
+    got, factor = out.permute(1, 3, 0, 2, 4).reshape(M, parts * dim), _factor(x, 1.0)
+    for i in range(parts):
+        cols = slice(i * dim, (i + 1) * dim)
+        _near(got[:, cols], (x.float() @ w[cols].float().t()) * factor * mul[i], K)
+
+
 class More(ctypes.Structure):
     _fields_ = [("pairs", ctypes.c_int)]
 
