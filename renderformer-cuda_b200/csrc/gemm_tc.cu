@@ -117,15 +117,18 @@ struct Params {
     int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
     const float* in_ss; int in_tiles, in_group;    // kFold: A's rows' sums of squares, how many a row, and how many of them make up 256 columns
     float in_inv_dim, in_eps, in_mul;              // the row's factor: in_mul * rsqrt(sum * in_inv_dim + in_eps)
-    const float* col_mul; int mul_units;           // kEpiHeads: if not null, another factor for each mul_units * 64 columns
+    const float *col_mul, *up_mul; int mul_shift;  // if not null, another factor for each 2^mul_shift columns, 64 or more (and of the up columns)
     int ss_tiles;                                  // kFold: sums a row that row_ss gets, of a part
     __half* raster;                                // kFold, residual: the rows in raster order too, or alone if C is null; pitch ldc
     Grid grid;
 };
 
 // the further factor of the columns that begin at col, a multiple of 64 or inside one (kFold)
-__device__ __forceinline__ float column_factor(const Params& p, int col) {
-    return p.col_mul ? __ldg(p.col_mul + min(col, p.N - 1) / 64 / p.mul_units) : 1.0f;
+__device__ const float g_one = 1.0f;
+__device__ __forceinline__ float column_factor(const Params& p, const float* mul, int col) {
+    float f;   // volatile: asked for where it is written, ahead of the loads that row_factor waits for, and not behind the products
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(mul ? mul + (min(col, p.N - 1) >> p.mul_shift) : &g_one));
+    return f;
 }
 // a row's factor (kFold)
 __device__ __forceinline__ float row_factor(const Params& p, int row) {
@@ -639,10 +642,18 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 rrow2 = p.raster + (at * (p.grid.bw * 4) + bx * 4 + (row & 3)) * p.ldc + n0;
             }
         }
+        constexpr bool kScaled = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL;
         float factors[BN_OUT > 64 ? 2 : 1];                   // of the row, in each 64 columns
-        factors[0] = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL && row_ok ? row_factor(p, row) : 1.0f;
-        if constexpr (BN_OUT > 64) factors[1] = FOLD && EPI == kEpiHeads ? factors[0] * column_factor(p, n0 + 64) : factors[0];
-        if (FOLD && EPI == kEpiHeads) factors[0] *= column_factor(p, n0);
+        float up_factor = 1.0f;
+        if (kScaled) {
+#pragma unroll
+            for (int i = 0; i < (BN_OUT > 64 ? 2 : 1); ++i) factors[i] = column_factor(p, p.col_mul, n0 + 64 * i);
+            if (kGate) up_factor = column_factor(p, p.up_mul, n0);
+            const float row_mul = row_ok ? row_factor(p, row) : 1.0f;
+#pragma unroll
+            for (int i = 0; i < (BN_OUT > 64 ? 2 : 1); ++i) factors[i] *= row_mul;
+            up_factor *= row_mul;
+        }
         constexpr int kChunk = BN_OUT < 32 ? BN_OUT : 32;     // output columns per step
         uint4 res[EPI == RFK_GEMM_EPI_RESIDUAL ? BN_OUT / 8 : 1];
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                   // the row's residual arrives while the products run
@@ -737,7 +748,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
                         for (int i = 0; i < kChunk; ++i) {
                             v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
-                            u[i] = __float_as_uint(__uint_as_float(u[i]) * factor);
+                            u[i] = __float_as_uint(__uint_as_float(u[i]) * up_factor);
                         }
                     }
 #pragma unroll
@@ -976,10 +987,21 @@ __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* ma
 
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
 // t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0. turn: the staging buffer of the
-// next store, kept from tile to tile (not with the residual epilogue). FOLD: row_mul is the row's factor; lane u holds that of the tile's unit u.
+// next store, kept from tile to tile (not with the residual epilogue). factors (FOLD): of the row, in each unit.
+// (Kept by the lanes, a unit each, and shuffled in the loop they cost a head-split tile 0.5 us: 1024 x 3072 x 1024 11.3, so 10.7, without any 10.6.)
+template <int EPI_, int BN> struct UnitFactors {
+    static constexpr int kUnits = Cfg<EPI_, BN>::kUnits;
+    float own[kUnits], up[(EPI_ & 7) == RFK_GEMM_EPI_SWIGLU ? kUnits : 1];
+    template <int N> static __device__ __forceinline__ float pick(const float (&f)[N], int u) {
+        float v = f[0];
+#pragma unroll
+        for (int i = 1; i < N; ++i) v = u == i ? f[i] : v;
+        return v;
+    }
+};
 template <int EPI_, int BN>
 __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, uint32_t t_acc,
-                                                     float row_mul, float unit_mul, unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
+                                                     const UnitFactors<EPI_, BN>& factors, unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity,
                                                      int row0, int n0, int lane, int& turn, volatile int* abort_flag) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & kFold) != 0;
@@ -1006,7 +1028,8 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     for (int u = 0; u < kUnits; ++u) {
         const uint32_t bias_unit = bias_next;
         bias_next = bias_of(u + 1);
-        const float factor = FOLD && EPI == kEpiHeads ? row_mul * __shfl_sync(0xffffffffu, unit_mul, u) : row_mul;
+        const float factor = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? factors.pick(factors.own, u) : 1.0f;
+        const float up_factor = FOLD && EPI == RFK_GEMM_EPI_SWIGLU ? factors.pick(factors.up, u) : 1.0f;
         const int b = (EPI == RFK_GEMM_EPI_RESIDUAL) ? u : turn;
         unsigned char* buf = stage_ptr + b * kUnitBytes;
         if (EPI == RFK_GEMM_EPI_RESIDUAL) {                 // this unit's residual box has landed (also for units beyond N)
@@ -1032,7 +1055,7 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
-                        up[i] = __float_as_uint(__uint_as_float(up[i]) * factor);
+                        up[i] = __float_as_uint(__uint_as_float(up[i]) * up_factor);
                     }
                 }
 #pragma unroll
@@ -1279,13 +1302,25 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
                 epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
             }
-            const float row_mul = FOLD && EPI != RFK_GEMM_EPI_RESIDUAL ? row_factor(p, min(row0 + lane, p.M - 1)) : 1.0f;
-            const float unit_mul = FOLD && EPI == kEpiHeads ? column_factor(p, n0 + min(lane, BN_OUT / kUnitCols - 1) * kUnitCols) : 1.0f;
+            UnitFactors<EPI_, BN> factors;
+            if (FOLD && EPI != RFK_GEMM_EPI_RESIDUAL) {
+#pragma unroll
+                for (int u = 0; u < Cfg<EPI_, BN>::kUnits; ++u) {
+                    factors.own[u] = column_factor(p, p.col_mul, n0 + u * kUnitCols);
+                    if (EPI == RFK_GEMM_EPI_SWIGLU) factors.up[u] = column_factor(p, p.up_mul, n0 + u * kUnitCols);
+                }
+                const float row_mul = row_factor(p, min(row0 + lane, p.M - 1));
+#pragma unroll
+                for (int u = 0; u < Cfg<EPI_, BN>::kUnits; ++u) {
+                    factors.own[u] *= row_mul;
+                    if (EPI == RFK_GEMM_EPI_SWIGLU) factors.up[u] *= row_mul;
+                }
+            }
             ok = tc::mbar_wait_warp(&ctrl->acc_full[acc], (tl >> 1) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(4);   // first tile's accumulator complete
-            ok = epilogue_tile_staged<EPI_, BN>(p, &map_c, &map_w1, tmem_cta + lane_off + acc * BNACC, row_mul, unit_mul, my_stage, my_res, tl & 1,
+            ok = epilogue_tile_staged<EPI_, BN>(p, &map_c, &map_w1, tmem_cta + lane_off + acc * BNACC, factors, my_stage, my_res, tl & 1,
                                                   row0, n0, lane, turn, abort_flag);
             if (!ok) break;
             if (tl == 0 && warp == 2 && lane == 0) RFK_STAMP(5);   // its epilogue done (stores issued)
@@ -1860,7 +1895,9 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream,
     if (f.blocks_across && (!residual || f.blocks_across % 2 || f.blocks_down % 2 || f.blocks_down <= 0 || f.M % (f.blocks_across * f.blocks_down * 16)))
         return RFK_EUNSUPPORTED;
     if (!f.blocks_across && (f.raster || !f.C)) return RFK_EINVAL;
+    if (f.part_mul && heads && (dim & (dim - 1))) return RFK_EUNSUPPORTED;
     if (f.quarters && (!residual || f.K % 512)) return RFK_EUNSUPPORTED;
+    if ((more.w_mul || more.w_up_mul) && (residual || f.part_mul || gate != (more.w_up_mul != nullptr) || !more.w_mul)) return RFK_EINVAL;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -1878,9 +1915,14 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream,
     p.raster = (__half*)f.raster;
     p.grid = tcgemm::Grid{f.blocks_across, f.blocks_down, f.shift_from, f.shift_to};
     if (heads) {
-        p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.col_mul = f.part_mul; p.mul_units = p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
+        p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
         p.part_stride = f.N > dim ? f.part_stride : (long long)f.M * dim;
     }
+    p.col_mul = more.w_mul ? more.w_mul : heads ? f.part_mul : nullptr;
+    p.up_mul = more.w_up_mul;
+    p.mul_shift = 6;
+    if (!more.w_mul)
+        while (1 << p.mul_shift < dim) ++p.mul_shift;
     const cudaStream_t st = as_stream(stream);
     return gate ? launch_folded<RFK_GEMM_EPI_SWIGLU>(f, p, dev, st, ss_tiles)
                 : heads ? launch_folded<tcgemm::kEpiHeads>(f, p, dev, st, ss_tiles) : launch_folded<RFK_GEMM_EPI_RESIDUAL>(f, p, dev, st, ss_tiles);

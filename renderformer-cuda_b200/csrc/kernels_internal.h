@@ -31,6 +31,7 @@ struct FoldedProduct {
 struct FoldedMore {
     int pairs;      // CTA pairs with one sum each 256 columns, which read W behind the kernel before, or RFK_EUNSUPPORTED: small tiles write one each
                     // 32 columns, and ask for W while the kernel before may still be writing it
+    const float *w_mul, *w_up_mul;   // SwiGLU and head-split: what each 64 rows of W and W_up are to be multiplied by (fold_weights); device memory, or NULL
 };
 int gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream, const FoldedMore& more = {});
 // whether a product (SwiGLU aside) goes to the pairs of FoldedMore::pairs, by its size
@@ -52,11 +53,10 @@ int fold_kv_weights(const rfk_half* const* k, const rfk_half* const* v, const fl
 int keys_norm(rfk_half* keys, long long layer_stride, const float* const* gamma, const float* row_ss, int layers, int rows, int out_seq, int num_heads,
               int head_dim, float eps, rfk_stream_t stream);
 
-// Weights for gemm_folded: out[i] = half(w[i] * gamma[i][column] * mul[i]) for up to 4 matrices [rows[i]][cols]; out[i] = the largest |gamma[i]|
-// of up to 96 vectors
-int fold_norm_weights(const rfk_half* const* w, rfk_half* const* out, const float* const* gamma, const float* mul, const int* rows, int n, int cols,
-                      rfk_stream_t stream);
-int largest_magnitudes(const float* const* gamma, int n, int dim, float* out, rfk_stream_t stream);
+// Weights for gemm_folded, 1024 wide (else RFK_EUNSUPPORTED): n matrices [rows[i]][1024], rows in whole 64s, one after the other in out as
+// half(w * gamma[i][column] / mul), where mul is a power of two for each 64 rows of them all, written to device memory
+constexpr int kMaxFolded = 64;
+int fold_weights(const rfk_half* const* w, const float* const* gamma, const int* rows, int n, int cols, rfk_half* out, float* mul, rfk_stream_t stream);
 
 // rfk_qkv_norm_rope_transpose behind gemm_heads: parts [heads][out_seq][head_dim], of which the first seq_len rows of each head are
 // normalised over the row (all heads) and, unless cos_vals is NULL, rotated in place, with that kernel's bits
@@ -152,8 +152,9 @@ extern "C" int rfk_conv3x3_nhwc_serves(const rfk_half* x, const rfk_half* w, con
 extern "C" int rfk_residual_add_silu_nhwc(rfk_half* y, const rfk_half* r, rfk_half* y_silu, long long n, rfk_stream_t stream);
 
 extern "C" int rfk_embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, rfk_half* x, float* row_ss, int rows, int dim, float eps,
-                                int blocks_across, int blocks_down, rfk_stream_t stream);   // embed_tokens and fold_norm_weights, for their tests
-extern "C" int rfk_fold_norm_weights(const rfk_half* w, rfk_half* out, const float* gamma, float mul, int rows, int cols, rfk_stream_t stream);
+                                int blocks_across, int blocks_down, rfk_stream_t stream);   // embed_tokens and fold_weights, for their tests
+extern "C" int rfk_fold_weights(const rfk_half* const* w, const float* const* gamma, const int* rows, int n, int cols, rfk_half* out, float* mul,
+                                rfk_stream_t stream);
 extern "C" int rfk_gemm_folded(const rfk::FoldedProduct* f, int* ss_tiles, rfk_stream_t stream);   // gemm_folded and folded_on_pairs, for their tests
 extern "C" int rfk_gemm_folded_more(const rfk::FoldedProduct* f, const rfk::FoldedMore* more, int* ss_tiles, rfk_stream_t stream);
 extern "C" int rfk_folded_on_pairs(int M, int N);

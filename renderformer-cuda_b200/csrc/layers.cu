@@ -601,9 +601,9 @@ int rfk_layers::decoder_layer_folded(rfk_ctx* ctx, const rfk_decoder_layer_weigh
     rfk::FoldedProduct p{};
     p.M = M;
     p.eps = kEpsFp16;
-    const auto normed = [&](const rfk_half* W, float mul, rfk_half* C, int N) {   // a product behind a norm
+    const auto normed = [&](const rfk_half* W, rfk_half* C, int N) {              // a product behind a norm
         rfk::FoldedProduct g = p;
-        g.A = x; g.W = W; g.C = C; g.N = N; g.K = dim; g.in_ss = b.x_ss; g.in_tiles = b.x_tiles; g.in_mul = mul;
+        g.A = x; g.W = W; g.C = C; g.N = N; g.K = dim; g.in_ss = b.x_ss; g.in_tiles = b.x_tiles; g.in_mul = 1.0f;
         return g;
     };
     const auto onto_x = [&](const rfk_half* A, const rfk_half* W, int K) {        // x += A W^T
@@ -613,26 +613,26 @@ int rfk_layers::decoder_layer_folded(rfk_ctx* ctx, const rfk_decoder_layer_weigh
     };
     int tiles = 0;
     // cross-attention (its query norm stays deferred: attention applies 1 / rms, the rotated keys carry the weight; the cut along the keys: see cross_attention_impl)
-    rfk::FoldedProduct g = normed(f.q, f.mul_q, b.q, dim);
+    rfk::FoldedProduct g = normed(f.q, b.q, dim);
     g.num_heads = num_heads; g.head_dim = hd; g.seq = Sq; g.out_ss = b.qk_ss; g.ss_mask = 1;
-    TRY(rfk::gemm_folded(g, &tiles, stream));
+    TRY(rfk::gemm_folded(g, &tiles, stream, {0, f.mul_q}));
     TRY(rfk::flash_attention_ex(b.q, K_rotated, V_cached, b.attn, b.qk_ss, tiles, dim, kEpsFp16, ctx->attn_ws, ctx->attn_ws_bytes,
                                 hd == 64 ? rfk::AttnCut::kBelowOneRound : rfk::AttnCut::kLastRound, v_shared, B, num_heads, Sq, Sk, n_keys, hd, 1,
                                 1.0f / sqrtf((float)hd), stream, group(tiles)));
     TRY(rfk::gemm_folded(onto_x(b.attn, w->cross_attn.out_proj_w, dim), &b.x_tiles, stream));
     // window attention
-    g = normed(f.in, f.mul_in, b.qkv, 3 * dim);
+    g = normed(f.in, b.qkv, 3 * dim);
     g.num_heads = num_heads; g.head_dim = hd; g.seq = 64; g.part_stride = (long long)M * dim; g.out_ss = b.qk_ss; g.ss_mask = 3;
-    TRY(rfk::gemm_folded(g, &tiles, stream));
+    TRY(rfk::gemm_folded(g, &tiles, stream, {0, f.mul_in}));
     const size_t part = (size_t)M * dim;
     TRY(rfk::window_attention(b.qkv, b.qkv + part, b.qkv + 2 * part, b.attn, mask, b.qk_ss, b.qk_ss + (size_t)M * tiles, tiles, w->self_attn.q_norm_gamma,
                               w->self_attn.k_norm_gamma, dim, kEpsFp16, M / 64, num_heads, 64, hd, Sq / 64, 1.0f / sqrtf((float)hd), stream,
                               group(tiles), true));
     TRY(rfk::gemm_folded(onto_x(b.attn, w->self_attn.out_proj_w, dim), &b.x_tiles, stream));
     // FFN; its result leaves in the next layer's order
-    g = normed(f.w1, f.mul_ffn, b.act, ffn_hidden);
+    g = normed(f.w1, b.act, ffn_hidden);
     g.W_up = f.w3;
-    TRY(rfk::gemm_folded(g, &tiles, stream));
+    TRY(rfk::gemm_folded(g, &tiles, stream, {0, f.mul_w1, f.mul_w3}));
     g = onto_x(b.act, w->ffn.w2, ffn_hidden);
     g.C = next; g.raster = raster; g.out_ss = next ? b.x_ss : nullptr;
     g.blocks_across = patch_w / 4; g.blocks_down = patch_h / 4; g.shift_from = shift / 4; g.shift_to = next_shift / 4;

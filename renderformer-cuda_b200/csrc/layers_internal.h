@@ -38,8 +38,8 @@ int decoder_layer_impl(rfk_ctx* ctx, const rfk_decoder_layer_weights* w, const r
 // the grid in the window order of the layer's own shift; x is read there and, where next is not NULL, written in the order of shift
 // next_shift; raster (may be NULL): the result in raster order. The mask's tokens are in row order.
 struct FoldedWeights {
-    rfk_half *q, *in, *w1, *w3;        // the products' weights with the norms' multiplied in, times 1 / mul
-    float mul_q, mul_in, mul_ffn;      // powers of two
+    rfk_half *q, *in, *w1, *w3;        // the products' weights with the norms' multiplied in,
+    float *mul_q, *mul_in, *mul_w1, *mul_w3;   // divided by these (fold_weights)
 };
 struct FoldedBuffers {                 // work space of a frame of M rows
     rfk_half *attn, *q, *qkv, *act;    // [M, dim] twice, [3 M, dim] (q may lie in it), [M, ffn_hidden]

@@ -233,40 +233,47 @@ embed_tokens_kernel(const __half* __restrict__ e, const float* __restrict__ gamm
     if (lane == 0) row_ss[(size_t)row * W + warp] = sum;
 }
 
-// Weights of the folded products (gemm_folded): out = half(w * gamma[column] * mul), a matrix a blockIdx.y
-struct FoldMatrices {
-    const __half* w[4];
-    __half* out[4];
-    const float* gamma[4];
-    float mul[4];
-    int rows[4];
+// Weights of the folded products (gemm_folded): out = half(w * gamma[column] / mul), 64 rows a CTA, one matrix after the other, with their power of two.
+// The scale lies in device memory beside the weights, where a captured graph's products find the one that they were divided by last.
+// Bound: HBM, each weight once in and once out; the 64 rows stay in registers until their scale is known.
+struct FoldList {
+    const __half* w[kMaxFolded];
+    const float* gamma[kMaxFolded];
+    int first[kMaxFolded], groups[kMaxFolded];   // of 64 rows
 };
-__global__ void __launch_bounds__(256)
-fold_weights_kernel(const __grid_constant__ FoldMatrices m, int cols) {
-    const int k = blockIdx.y;
-    const long long chunks = (long long)m.rows[k] * (cols / 8);
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < chunks; i += (long long)gridDim.x * 256) {
-        float w[8], g[8];
-        unpack8(ldg_half8(m.w[k] + i * 8), w);
-        ldg_float8(m.gamma[k] + (i * 8) % cols, g);
+constexpr int kFoldThreads = 512, kFoldCols = 1024, kFoldChunks = 64 * kFoldCols / 8 / kFoldThreads;
+__global__ void __launch_bounds__(kFoldThreads)
+fold_weights_kernel(const __grid_constant__ FoldList m, __half* __restrict__ out, float* __restrict__ mul) {
+    __shared__ float s_max[kFoldThreads / 32];
+    const int i = blockIdx.y, tid = threadIdx.x;
+    if ((int)blockIdx.x >= m.groups[i]) return;
+    const size_t group = m.first[i] + blockIdx.x;
+    const __half* w = m.w[i] + (size_t)blockIdx.x * 64 * kFoldCols + tid * 8;
+    Half8 raw[kFoldChunks];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] *= g[j] * m.mul[k];
-        store8(m.out[k] + i * 8, w);
-    }
-}
-// the largest magnitude of each of n vectors
-struct GammaList { const float* gamma[96]; };
-__global__ void __launch_bounds__(256)
-largest_magnitude_kernel(const __grid_constant__ GammaList list, float* __restrict__ out, int dim) {
-    __shared__ float part[8];
-    float m = 0.0f;
-    for (int i = threadIdx.x; i < dim; i += 256) m = fmaxf(m, fabsf(list.gamma[blockIdx.x][i]));
-    m = warp_max(m);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    for (int k = 0; k < kFoldChunks; ++k) raw[k] = ldcs_half8(w + (size_t)k * kFoldThreads * 8);
+    float g[8], mx = 0.0f;      // a thread keeps its columns: the threads walk whole rows
+    ldg_float8(m.gamma[i] + tid * 8 % kFoldCols, g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(g[j]));
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) m = fmaxf(m, part[w]);
-        out[blockIdx.x] = m;
+#pragma unroll
+    for (int k = 0; k < kFoldThreads / 32; ++k) mx = fmaxf(mx, s_max[k]);
+    const int e = (int)(__float_as_uint(mx) >> 23) + 1;   // biased exponent of the next power of two
+    const float scale = mx > 0.0f && e < 255 ? __uint_as_float((uint32_t)min(max(e, 27), 227) << 23) : 1.0f, by = 1.0f / scale;
+    if (tid == 0) mul[group] = scale;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] *= by;
+    __half* o = out + group * 64 * kFoldCols + tid * 8;
+#pragma unroll
+    for (int k = 0; k < kFoldChunks; ++k) {
+        float v[8];
+        unpack8(raw[k], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] *= g[j];
+        store8(o + (size_t)k * kFoldThreads * 8, v);
     }
 }
 
@@ -524,24 +531,19 @@ int keys_norm(rfk_half* keys, long long layer_stride, const float* const* gamma,
     return launch_status();
 }
 
-int fold_norm_weights(const rfk_half* const* w, rfk_half* const* out, const float* const* gamma, const float* mul, const int* rows, int n, int cols,
-                      rfk_stream_t stream) {
-    if (!w || !out || !gamma || !mul || !rows || n < 1 || n > 4 || cols <= 0 || cols % 8) return RFK_EINVAL;
-    FoldMatrices m{};
+int fold_weights(const rfk_half* const* w, const float* const* gamma, const int* rows, int n, int cols, rfk_half* out, float* mul, rfk_stream_t stream) {
+    if (!w || !gamma || !rows || !out || !mul || n < 1 || cols <= 0) return RFK_EINVAL;
+    if (cols != kFoldCols || n > kMaxFolded || !aligned16(out)) return RFK_EUNSUPPORTED;
+    FoldList m{};
+    int groups = 0, most = 0;
     for (int i = 0; i < n; ++i) {
-        if (!w[i] || !out[i] || !gamma[i] || rows[i] < 0) return RFK_EINVAL;
-        if (!aligned16(w[i]) || !aligned16(out[i]) || !aligned16(gamma[i])) return RFK_EUNSUPPORTED;
-        m.w[i] = (const __half*)w[i]; m.out[i] = (__half*)out[i]; m.gamma[i] = gamma[i]; m.mul[i] = mul[i]; m.rows[i] = rows[i];
+        if (!w[i] || !gamma[i] || rows[i] <= 0) return RFK_EINVAL;
+        if (!aligned16(w[i]) || !aligned16(gamma[i]) || rows[i] % 64) return RFK_EUNSUPPORTED;
+        m.w[i] = (const __half*)w[i]; m.gamma[i] = gamma[i]; m.first[i] = groups; m.groups[i] = rows[i] / 64;
+        groups += m.groups[i];
+        most = std::max(most, m.groups[i]);
     }
-    fold_weights_kernel<<<dim3(2 * kNumSMs, n), 256, 0, as_stream(stream)>>>(m, cols);
-    return launch_status();
-}
-
-int largest_magnitudes(const float* const* gamma, int n, int dim, float* out, rfk_stream_t stream) {
-    if (!gamma || !out || n < 1 || n > 96 || dim <= 0) return RFK_EINVAL;
-    GammaList list{};
-    for (int i = 0; i < n; ++i) list.gamma[i] = gamma[i];
-    largest_magnitude_kernel<<<n, 256, 0, as_stream(stream)>>>(list, out, dim);
+    fold_weights_kernel<<<dim3(most, n), kFoldThreads, 0, as_stream(stream)>>>(m, (__half*)out, mul);
     return launch_status();
 }
 
@@ -554,8 +556,9 @@ extern "C" int rfk_embed_tokens(const rfk_half* e, const float* gamma, const rfk
     return embed_tokens(e, gamma, token, x, row_ss, rows, dim, eps, blocks_across, blocks_down, stream);
 }
 
-extern "C" int rfk_fold_norm_weights(const rfk_half* w, rfk_half* out, const float* gamma, float mul, int rows, int cols, rfk_stream_t stream) {
-    return fold_norm_weights(&w, &out, &gamma, &mul, &rows, 1, cols, stream);
+extern "C" int rfk_fold_weights(const rfk_half* const* w, const float* const* gamma, const int* rows, int n, int cols, rfk_half* out, float* mul,
+                                rfk_stream_t stream) {
+    return fold_weights(w, gamma, rows, n, cols, out, mul, stream);
 }
 
 extern "C" int rfk_norm_pair_add(const rfk_half* a, const float* gamma_a, const rfk_half* b, const float* gamma_b, const rfk_half* c,

@@ -176,7 +176,8 @@ struct rfk_session {
     FoldedWeights fold[RFK_MAX_LAYERS] = {};
     FoldedBuffers fbuf{};
     rfk_half* x_other = nullptr;           // the residual stream's second buffer: a layer's last product reorders the rows
-    float* fold_max = nullptr;
+    rfk_half* fold_w = nullptr;            // what fold[] points into
+    float* fold_mul = nullptr;
     rfk_half* dft[kSlots][4] = {};  // the four decoder feature taps of each frame slot
     rfk_dpt_weights dptw{};          // copy of the model's DPT record (if any)
     rfk_dpt* dpt = nullptr;          // planned image head; null: the view ends at the token map
@@ -311,34 +312,23 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
     return RFK_OK;
 }
 
-// The weights of the folded products. The norms' weights are scaled by a power of two to below one first, so that a product of two stays in
-// fp16's range wherever the matrix was; the products' row factors take it back.
+// The weights of the folded products and their scales, where a captured graph finds them: nothing of them is an argument of a launch.
 int rfk_session::fold_weights() {
-    const int n = 3 * m.dec_layers, dim = m.dim;
-    std::vector<const float*> gamma(n);
-    for (int i = 0; i < m.dec_layers; ++i) {
-        gamma[3 * i] = m.dec[i].query_norm_gamma;
-        gamma[3 * i + 1] = m.dec[i].self_attn_norm_gamma;
-        gamma[3 * i + 2] = m.dec[i].ffn_norm_gamma;
-    }
-    TRY(rfk::largest_magnitudes(gamma.data(), n, dim, fold_max, (rfk_stream_t)stream));
-    std::vector<float> mul(n);
-    TRY_CUDA(cudaMemcpyAsync(mul.data(), fold_max, n * sizeof(float), cudaMemcpyDeviceToHost, stream));
-    TRY_CUDA(cudaStreamSynchronize(stream));
-    for (float& v : mul) {
-        int e = 0;
-        if (std::isfinite(v) && v > 0.0f) std::frexp(v, &e);
-        v = std::ldexp(1.0f, std::min(std::max(e, -100), 100));
-    }
-    for (int i = 0; i < m.dec_layers; ++i) {
-        FoldedWeights& f = fold[i];
-        f.mul_q = mul[3 * i]; f.mul_in = mul[3 * i + 1]; f.mul_ffn = mul[3 * i + 2];
-        const rfk_half* w[4] = {m.dec[i].cross_attn.q_proj_w, m.dec[i].self_attn.in_proj_w, m.dec[i].ffn.w1, m.dec[i].ffn.w3};
-        rfk_half* out[4] = {f.q, f.in, f.w1, f.w3};
-        const float* g[4] = {gamma[3 * i], gamma[3 * i + 1], gamma[3 * i + 2], gamma[3 * i + 2]};
-        const float by[4] = {1.0f / f.mul_q, 1.0f / f.mul_in, 1.0f / f.mul_ffn, 1.0f / f.mul_ffn};
-        const int rows[4] = {dim, 3 * dim, m.ffn_hidden, m.ffn_hidden};
-        TRY(rfk::fold_norm_weights(w, out, g, by, rows, 4, dim, (rfk_stream_t)stream));
+    constexpr int kLayers = rfk::kMaxFolded / 4;   // a launch
+    const int dim = m.dim, ffn = m.ffn_hidden;
+    for (int first = 0; first < m.dec_layers; first += kLayers) {
+        const rfk_half* w[rfk::kMaxFolded];
+        const float* gamma[rfk::kMaxFolded];
+        int rows[rfk::kMaxFolded], n = 0;
+        const auto add = [&](const rfk_half* weights, const float* norm, int r) { w[n] = weights; gamma[n] = norm; rows[n++] = r; };
+        for (int i = first; i < std::min(first + kLayers, m.dec_layers); ++i) {
+            const rfk_decoder_layer_weights& d = m.dec[i];
+            add(d.cross_attn.q_proj_w, d.query_norm_gamma, dim);
+            add(d.self_attn.in_proj_w, d.self_attn_norm_gamma, 3 * dim);
+            add(d.ffn.w1, d.ffn_norm_gamma, ffn);
+            add(d.ffn.w3, d.ffn_norm_gamma, ffn);
+        }
+        TRY(rfk::fold_weights(w, gamma, rows, n, dim, fold[first].q, fold[first].mul_q, (rfk_stream_t)stream));
     }
     return RFK_OK;
 }
@@ -446,19 +436,21 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
         const rfk_cross_attn_weights& w = model->dec[i].cross_attn;
         d->folds_kv = given(model->dec[i].kv_norm_gamma) && given(w.k_proj_w) && given(w.v_proj_w) && given(w.k_norm_gamma) && !w.k_proj_b && !w.v_proj_b;
     }
-    d->folded = d->prescale && !d->ctx->reproducible && 3 * model->dec_layers <= 96 &&
+    d->folded = d->prescale && !d->ctx->reproducible &&
                 !((reinterpret_cast<uintptr_t>(model->ray_enc_norm) | reinterpret_cast<uintptr_t>(model->ray_map_patch_token)) & 15u);
     for (int i = 0; i < model->dec_layers && d->folded; ++i)
         d->folded = layer_folds(model->dec[i], nP, dim, nh, ffn, d->pH, d->pW, ws, model->shift_size);
     if (d->folded) {
-        const size_t rows = V * nP, per_layer = (size_t)4 * dim * dim + (size_t)2 * ffn * dim;
-        rfk_half* weights = nullptr;
-        if ((rc = d->alloc(&weights, model->dec_layers * per_layer))) return fail(rc);
-        for (int i = 0; i < model->dec_layers; ++i, weights += per_layer)
-            d->fold[i] = FoldedWeights{weights, weights + (size_t)dim * dim, weights + (size_t)4 * dim * dim,
-                                       weights + (size_t)4 * dim * dim + (size_t)ffn * dim, 1.0f, 1.0f, 1.0f};
+        const size_t rows = V * nP, layer_rows = 4 * (size_t)dim + 2 * (size_t)ffn;   // in whole 64s
+        ALLOC(fold_w, model->dec_layers * layer_rows * dim);
+        ALLOC(fold_mul, model->dec_layers * layer_rows / 64);
+        for (int i = 0; i < model->dec_layers; ++i) {
+            const size_t at[4] = {i * layer_rows, i * layer_rows + dim, i * layer_rows + 4 * dim, i * layer_rows + 4 * dim + ffn};
+            const auto weights = [&](int k) { return d->fold_w + at[k] * dim; };
+            const auto mul = [&](int k) { return d->fold_mul + at[k] / 64; };
+            d->fold[i] = FoldedWeights{weights(0), weights(1), weights(2), weights(3), mul(0), mul(1), mul(2), mul(3)};
+        }
         ALLOC(x_other, rows * dim);
-        ALLOC(fold_max, 3 * model->dec_layers);
         ALLOC(fbuf.x_ss, rows * dim / 32);
         ALLOC(fbuf.qk_ss, rows * dim / 16);
         d->fbuf.attn = d->temp;

@@ -167,15 +167,27 @@ def test_tokens_that_enter_folded_layers(views, h, w):
     _check_sums(ss, 4, x)
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 8), (33, 264), (3072, 1024)])
-def test_folded_weights(rows, cols):
-    rnd = _gen(rows)
-    w, gamma = rnd(rows, cols), rnd(cols).float()
-    out = torch.empty_like(w)
-    p = lambda t: ctypes.c_void_p(t.data_ptr())
-    assert _abi.load("rfk.h").rfk_fold_norm_weights(p(w), p(out), p(gamma), ctypes.c_float(0.25), rows, cols,
-                                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
-    assert torch.equal(out, (w.float() * (gamma * 0.25)).half())
+def _fold(weights, gammas):
+    """rfk_fold_weights of matrices [rows][1024]: the folded rows and what each 64 of them were divided by."""
+    n, rows = len(weights), sum(w.shape[0] for w in weights)
+    out, mul = torch.empty(rows, 1024, device="cuda", dtype=torch.half), torch.full((rows // 64,), float("nan"), device="cuda")
+    table = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])
+    rc = _abi.load("rfk.h").rfk_fold_weights(table(weights), table(gammas), (ctypes.c_int * n)(*[w.shape[0] for w in weights]), n, 1024,
+                                             ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(mul.data_ptr()),
+                                             ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    return out, mul
+
+
+@pytest.mark.parametrize("rows", [(64,), (1024, 3072, 256, 256), (64, 192) * 32])
+def test_folded_weights(rows):
+    rnd = _gen(len(rows))
+    w = [rnd(r, 1024) for r in rows]
+    gamma = [rnd(1024).float() * 2.0 ** (3 * (i % 9) - 12) for i in range(len(rows))]
+    out, mul = _fold(w, gamma)
+    assert (mul.log2() == mul.log2().round()).all()
+    product = torch.cat([a.float() * g for a, g in zip(w, gamma)])
+    assert torch.equal(out, (product / mul.repeat_interleave(64)[:, None]).half())
 
 
 def _scene(n, seed):
@@ -244,6 +256,28 @@ def test_weights_changed_in_place_count_from_the_next_encoding():
     assert not torch.equal(before, want) and torch.equal(got, want)
 
 
+@pytest.mark.parametrize("heads,res,use_graph", [(16, 64, True), (8, 128, True), (16, 192, True), (16, 64, False)])
+def test_norm_weights_changed_across_powers_of_two(heads, res, use_graph):
+    """The scales that are taken out of the weights are not part of a captured view: norm weights 8, 1/16 and 37 times as large."""
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=3, dim=1024, num_heads=heads, ffn_hidden=512, enc_layers=1, dec_layers=2)
+    scene = _scene(60, 1)
+    s, before = _view(model, scene, res, use_graph=use_graph)
+    before = before.clone()
+    for i in range(2):
+        for k, by in (("query_norm", 8.0), ("self_attn_norm", 1 / 16), ("ffn_norm", 37.0)):
+            model.t[f"dec{i}.{k}"].mul_(by)
+    s.encode_scene(*scene)
+    c2w = torch.eye(4)
+    c2w[2, 3] = 3.0
+    s.render_frame(c2w, 0.7)
+    got = s.download().clone()
+    s.close()
+    f, want = _view(model, scene, res, use_graph=use_graph)
+    f.close()
+    assert not torch.equal(before, want) and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M,pad,parts,hd", [(1, 8, 4, 64), (333, 336, 24, 128), (777, 784, 6, 64), (2665, 2672, 8, 64)])
 @pytest.mark.parametrize("path", [0, 2])
 def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts, hd, path):
@@ -290,7 +324,7 @@ def test_factors_of_parts_without_sums(M, parts):
 
 
 class More(ctypes.Structure):
-    _fields_ = [("pairs", ctypes.c_int)]
+    _fields_ = [("pairs", ctypes.c_int), ("w_mul", ctypes.c_void_p), ("w_up_mul", ctypes.c_void_p)]
 
 
 # both sides of the line, which is 148 tiles of 128 x 128 on 148 SMs: 1 layer of keys and values, 3, 9 and 12
