@@ -117,7 +117,7 @@ struct Params {
     int seq, out_seq, units, head_units, ss_mask;  // kEpiHeads: rows per group, 64-column units per part and per head, parts that get row_ss
     const float* in_ss; int in_tiles, in_group;    // kFold: A's rows' sums of squares, how many a row, and how many of them make up 256 columns
     float in_inv_dim, in_eps, in_mul;              // the row's factor: in_mul * rsqrt(sum * in_inv_dim + in_eps)
-    const float *col_mul, *up_mul; int mul_shift;  // if not null, another factor for each 2^mul_shift columns, 64 or more (and of the up columns)
+    const float *col_mul, *up_mul;                 // if not null, another factor for each 64 columns (and of the up columns)
     int ss_tiles;                                  // kFold: sums a row that row_ss gets, of a part
     __half* raster;                                // kFold, residual: the rows in raster order too, or alone if C is null; pitch ldc
     Grid grid;
@@ -127,7 +127,7 @@ struct Params {
 __device__ const float g_one = 1.0f;
 __device__ __forceinline__ float column_factor(const Params& p, const float* mul, int col) {
     float f;   // volatile: asked for where it is written, ahead of the loads that row_factor waits for, and not behind the products
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(mul ? mul + (min(col, p.N - 1) >> p.mul_shift) : &g_one));
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(mul ? mul + min(col, p.N - 1) / 64 : &g_one));
     return f;
 }
 // a row's factor (kFold)
@@ -1895,9 +1895,8 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream,
     if (f.blocks_across && (!residual || f.blocks_across % 2 || f.blocks_down % 2 || f.blocks_down <= 0 || f.M % (f.blocks_across * f.blocks_down * 16)))
         return RFK_EUNSUPPORTED;
     if (!f.blocks_across && (f.raster || !f.C)) return RFK_EINVAL;
-    if (f.part_mul && heads && (dim & (dim - 1))) return RFK_EUNSUPPORTED;
     if (f.quarters && (!residual || f.K % 512)) return RFK_EUNSUPPORTED;
-    if ((more.w_mul || more.w_up_mul) && (residual || f.part_mul || gate != (more.w_up_mul != nullptr) || !more.w_mul)) return RFK_EINVAL;
+    if ((more.w_mul || more.w_up_mul) && (residual || gate != (more.w_up_mul != nullptr) || !more.w_mul)) return RFK_EINVAL;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -1918,11 +1917,8 @@ int rfk::gemm_folded(const FoldedProduct& f, int* ss_tiles, rfk_stream_t stream,
         p.seq = f.seq; p.out_seq = f.out_seq ? f.out_seq : f.seq; p.units = dim / 64; p.head_units = f.head_dim / 64; p.ss_mask = f.ss_mask;
         p.part_stride = f.N > dim ? f.part_stride : (long long)f.M * dim;
     }
-    p.col_mul = more.w_mul ? more.w_mul : heads ? f.part_mul : nullptr;
+    p.col_mul = more.w_mul;
     p.up_mul = more.w_up_mul;
-    p.mul_shift = 6;
-    if (!more.w_mul)
-        while (1 << p.mul_shift < dim) ++p.mul_shift;
     const cudaStream_t st = as_stream(stream);
     return gate ? launch_folded<RFK_GEMM_EPI_SWIGLU>(f, p, dev, st, ss_tiles)
                 : heads ? launch_folded<tcgemm::kEpiHeads>(f, p, dev, st, ss_tiles) : launch_folded<RFK_GEMM_EPI_RESIDUAL>(f, p, dev, st, ss_tiles);

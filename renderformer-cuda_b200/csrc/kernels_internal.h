@@ -24,7 +24,7 @@ struct FoldedProduct {
     const float* in_ss; int in_tiles; float in_mul, eps;    // SwiGLU and head-split: a row's factor is in_mul / sqrt(mean square + eps)
     float* out_ss; int ss_mask;                             // head-split: parts that get sums
     long long part_stride; int seq, num_heads, head_dim;
-    int out_seq; const float* part_mul;                     // head-split: rows a head has room for (0: seq); another factor for each part, or NULL
+    int out_seq;                                            // head-split: rows a head has room for (0: seq)
     int blocks_across, blocks_down, shift_from, shift_to;   // 0: rows stay where they are
     int quarters;                                           // residual: the sum over K is ((a + b) + c) + d of its quarters (K % 512 == 0), whatever M
 };
@@ -44,17 +44,15 @@ int embed_tokens(const rfk_half* e, const float* gamma, const rfk_half* token, r
                  int blocks_across, int blocks_down, rfk_stream_t stream);
 
 // The keys and values of several layers from one set of rows (1024 wide, else RFK_EUNSUPPORTED): y = half(x + r) with its rows' sums of squares
-// row_ss [rows][4] (r may be NULL); the weights [2 * layers][1024][1024], keys' and values' in turn, with each layer's norm weight multiplied in and
-// divided by part_mul [2 * layers], a power of two; and the keys' own norm, in place on [layers] slabs [head][out_seq][head_dim], layer_stride apart,
+// row_ss [rows][4] (r may be NULL); and the keys' own norm, in place on [layers] slabs [head][out_seq][head_dim], layer_stride apart,
 // with sums row_ss [2 * layers][rows][4] of which the keys' are read
 int context_rows(const float* x, const rfk_half* r, rfk_half* y, float* row_ss, int rows, int dim, rfk_stream_t stream);
-int fold_kv_weights(const rfk_half* const* k, const rfk_half* const* v, const float* const* gamma, rfk_half* out, float* part_mul, int layers, int dim,
-                    rfk_stream_t stream);
 int keys_norm(rfk_half* keys, long long layer_stride, const float* const* gamma, const float* row_ss, int layers, int rows, int out_seq, int num_heads,
               int head_dim, float eps, rfk_stream_t stream);
 
 // Weights for gemm_folded, 1024 wide (else RFK_EUNSUPPORTED): n matrices [rows[i]][1024], rows in whole 64s, one after the other in out as
-// half(w * gamma[i][column] / mul), where mul is a power of two for each 64 rows of them all, written to device memory
+// half(w * gamma[i][column] / mul), where mul is a power of two for each 64 rows of them all, written to device memory: their largest product
+// comes to between 2^13 and 2^14
 constexpr int kMaxFolded = 64;
 int fold_weights(const rfk_half* const* w, const float* const* gamma, const int* rows, int n, int cols, rfk_half* out, float* mul, rfk_stream_t stream);
 

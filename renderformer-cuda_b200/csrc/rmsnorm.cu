@@ -21,6 +21,7 @@
 // stores of finished ones. The W partial sums meet through 16 bytes of shared memory.
 #include "common.cuh"
 #include "kernels_internal.h"
+#include "tc_pair.cuh"
 
 namespace rfk {
 
@@ -233,46 +234,67 @@ embed_tokens_kernel(const __half* __restrict__ e, const float* __restrict__ gamm
     if (lane == 0) row_ss[(size_t)row * W + warp] = sum;
 }
 
-// Weights of the folded products (gemm_folded): out = half(w * gamma[column] / mul), 64 rows a CTA, one matrix after the other, with their power of two.
-// The scale lies in device memory beside the weights, where a captured graph's products find the one that they were divided by last.
-// Bound: HBM, each weight once in and once out; the 64 rows stay in registers until their scale is known.
+// Weights of the folded products (gemm_folded): out = half(w * gamma[column] / mul), one matrix after the other, each 64 rows with a power of two of theirs.
+// The scale lies in device memory beside the weights, where a captured graph's products find the one that they were divided by last. It is that of
+// the largest product and not of the norm's weights: a product that is 2^27 times smaller still has all its bits, where a small norm
+// weight that holds down a large channel would otherwise leave products below 2^-14, which have fewer (512 x 1024 x 1024, W of 0.02 n, norm weights
+// exp(a n), channels inversely as large, error against 64 bits, separate norm / the norm's weights brought below 1 / this:
+// a = 1.5 2.1e-4 / 7.8e-4 / 2.1e-4, a = 2 2.1e-4 / 1.4e-2 / 2.1e-4). 2^14 leaves two bits below fp16's largest; the sums are fp32.
+// Bound: HBM, each weight once in and once out; the rows stay in registers until their scale is known. A cluster of two CTAs with 32 rows each, two of them an
+// SM, loads while another stores: twelve layers' weights (302 MB in, 302 out) 106 us, 5.7 TB/s; 64 rows a CTA 132, 256 threads a CTA 123.
 struct FoldList {
     const __half* w[kMaxFolded];
     const float* gamma[kMaxFolded];
     int first[kMaxFolded], groups[kMaxFolded];   // of 64 rows
 };
-constexpr int kFoldThreads = 512, kFoldCols = 1024, kFoldChunks = 64 * kFoldCols / 8 / kFoldThreads;
-__global__ void __launch_bounds__(kFoldThreads)
+constexpr int kFoldThreads = 512, kFoldCols = 1024, kFoldRows = 32, kFoldChunks = kFoldRows * kFoldCols / 8 / kFoldThreads;
+__global__ void __cluster_dims__(2) __launch_bounds__(kFoldThreads, 2)
 fold_weights_kernel(const __grid_constant__ FoldList m, __half* __restrict__ out, float* __restrict__ mul) {
-    __shared__ float s_max[kFoldThreads / 32];
-    const int i = blockIdx.y, tid = threadIdx.x;
-    if ((int)blockIdx.x >= m.groups[i]) return;
-    const size_t group = m.first[i] + blockIdx.x;
-    const __half* w = m.w[i] + (size_t)blockIdx.x * 64 * kFoldCols + tid * 8;
+    __shared__ float s_max[kFoldThreads / 32], s_half[2];
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.y, tid = threadIdx.x, part = blockIdx.x & 1;
+    if ((int)blockIdx.x >= 2 * m.groups[i]) return;   // both CTAs of a cluster
+    pair_ptx::cluster_arrive();                       // met ahead of the store into the other CTA: by then it runs
+    const size_t at = (size_t)blockIdx.x * kFoldRows * kFoldCols + tid * 8;
+    const __half* w = m.w[i] + at;
     Half8 raw[kFoldChunks];
 #pragma unroll
     for (int k = 0; k < kFoldChunks; ++k) raw[k] = ldcs_half8(w + (size_t)k * kFoldThreads * 8);
     float g[8], mx = 0.0f;      // a thread keeps its columns: the threads walk whole rows
     ldg_float8(m.gamma[i] + tid * 8 % kFoldCols, g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(g[j]));
-    mx = warp_max(mx);
-    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kFoldThreads / 32; ++k) mx = fmaxf(mx, s_max[k]);
-    const int e = (int)(__float_as_uint(mx) >> 23) + 1;   // biased exponent of the next power of two
-    const float scale = mx > 0.0f && e < 255 ? __uint_as_float((uint32_t)min(max(e, 27), 227) << 23) : 1.0f, by = 1.0f / scale;
-    if (tid == 0) mul[group] = scale;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) g[j] *= by;
-    __half* o = out + group * 64 * kFoldCols + tid * 8;
-#pragma unroll
     for (int k = 0; k < kFoldChunks; ++k) {
         float v[8];
         unpack8(raw[k], v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] *= g[j];
+        for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j] * g[j]));
+    }
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
+    __syncthreads();
+    pair_ptx::cluster_wait();
+    if (tid < 2) {              // into both CTAs
+        for (int k = 0; k < kFoldThreads / 32; ++k) mx = fmaxf(mx, s_max[k]);
+        const uint32_t to = pair_ptx::map_to_cta(tc::smem_addr(&s_half[part]), tid);
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(mx) : "memory");
+    }
+    __syncwarp();
+    pair_ptx::cluster_arrive();
+    pair_ptx::cluster_wait();
+    mx = fmaxf(s_half[0], s_half[1]);
+    const int e = (int)(__float_as_uint(mx) >> 23) + 1;   // biased exponent of the next power of two; 255, 256: not finite
+    const float scale = mx > 0.0f && e < 255 ? __uint_as_float((uint32_t)min(max(e - 14, 27), 227) << 23) : 1.0f, by = 1.0f / scale;
+    if (tid == 0 && part == 0) mul[m.first[i] + (blockIdx.x >> 1)] = scale;
+    __half* o = out + (size_t)m.first[i] * 64 * kFoldCols + at;
+#pragma unroll
+    for (int k = 0; k < kFoldChunks; ++k) {
+        float v[8];
+        uint32_t* q = reinterpret_cast<uint32_t*>(&raw[k]);
+        asm volatile("" : "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]));   // unpacked anew: all of them in fp32 are more than the registers
+        unpack8(raw[k], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (v[j] * g[j]) * by;
         store8(o + (size_t)k * kFoldThreads * 8, v);
     }
 }
@@ -308,42 +330,6 @@ context_rows_kernel(const float* __restrict__ x, const __half* __restrict__ r, _
 }
 
 constexpr int kMaxKvLayers = 32;
-struct KvWeights {
-    const __half* w[2 * kMaxKvLayers];   // keys', values' of each layer
-    const float* gamma[kMaxKvLayers];
-};
-__global__ void __launch_bounds__(256)
-fold_kv_weights_kernel(const __grid_constant__ KvWeights m, __half* __restrict__ out, float* __restrict__ part_mul, int dim) {
-    __shared__ float s_max[8];
-    pdl_wait();
-    pdl_trigger();
-    const int part = blockIdx.y, tid = threadIdx.x;
-    const float* gamma = m.gamma[part >> 1];
-    float mx = 0.0f;
-    for (int i = tid; i < dim; i += 256) mx = fmaxf(mx, fabsf(gamma[i]));
-    mx = warp_max(mx);
-    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
-    __syncthreads();
-    for (int w = 0; w < 8; ++w) mx = fmaxf(mx, s_max[w]);
-    const int e = (int)(__float_as_uint(mx) >> 23) + 1;   // biased exponent of the next power of two
-    const float scale = mx > 0.0f && e < 255 ? __uint_as_float((uint32_t)min(max(e, 27), 227) << 23) : 1.0f, mul = 1.0f / scale;
-    if (blockIdx.x == 0 && tid == 0) part_mul[part] = scale;
-    const int chunks = dim * (dim / 8);
-    const int col = (tid * 8) % dim;      // 256 threads walk whole rows of dim = 1024: a thread keeps its columns
-    float g[8];
-    ldg_float8(gamma + col, g);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) g[i] *= mul;
-    __half* o = out + (size_t)part * dim * dim;
-#pragma unroll 4
-    for (int i = blockIdx.x * 256 + tid; i < chunks; i += gridDim.x * 256) {
-        float w[8];
-        unpack8(ldcs_half8(m.w[part] + (size_t)i * 8), w);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] *= g[j];
-        store8(o + (size_t)i * 8, w);
-    }
-}
 
 // Bound: HBM, each key once in and once out. A thread takes its chunk of a row in four heads, whose sum it reads once.
 struct KeyGammas { const float* gamma[kMaxKvLayers]; };
@@ -499,20 +485,6 @@ int context_rows(const float* x, const rfk_half* r, rfk_half* y, float* row_ss, 
     return launch_status();
 }
 
-int fold_kv_weights(const rfk_half* const* k, const rfk_half* const* v, const float* const* gamma, rfk_half* out, float* part_mul, int layers, int dim,
-                    rfk_stream_t stream) {
-    if (!k || !v || !gamma || !out || !part_mul || layers <= 0) return RFK_EINVAL;
-    if (dim != 1024 || layers > kMaxKvLayers || !aligned16(out)) return RFK_EUNSUPPORTED;
-    KvWeights m{};
-    for (int i = 0; i < layers; ++i) {
-        if (!k[i] || !v[i] || !gamma[i]) return RFK_EINVAL;
-        if (!aligned16(k[i]) || !aligned16(v[i]) || !aligned16(gamma[i])) return RFK_EUNSUPPORTED;
-        m.w[2 * i] = (const __half*)k[i]; m.w[2 * i + 1] = (const __half*)v[i]; m.gamma[i] = gamma[i];
-    }
-    launch_pdl(fold_kv_weights_kernel, dim3(64, 2 * layers), dim3(256), 0, as_stream(stream), m, (__half*)out, part_mul, dim);
-    return launch_status();
-}
-
 int keys_norm(rfk_half* keys, long long layer_stride, const float* const* gamma, const float* row_ss, int layers, int rows, int out_seq, int num_heads,
               int head_dim, float eps, rfk_stream_t stream) {
     if (!keys || !gamma || !row_ss || layers <= 0 || rows < 0 || out_seq < rows || num_heads <= 0 || head_dim <= 0) return RFK_EINVAL;
@@ -543,7 +515,7 @@ int fold_weights(const rfk_half* const* w, const float* const* gamma, const int*
         groups += m.groups[i];
         most = std::max(most, m.groups[i]);
     }
-    fold_weights_kernel<<<dim3(most, n), kFoldThreads, 0, as_stream(stream)>>>(m, (__half*)out, mul);
+    launch_pdl(fold_weights_kernel, dim3(2 * most, n), dim3(kFoldThreads), 0, as_stream(stream), m, (__half*)out, mul);
     return launch_status();
 }
 

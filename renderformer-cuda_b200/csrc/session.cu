@@ -148,6 +148,8 @@ std::vector<uint8_t> build_window_mask(int rows, int cols, int ws, int shift) {
 
 }  // namespace
 
+constexpr int kMaxFoldedKv = 16;   // decoder layers whose keys and values are one product (encode_kv): as many as ss_mask has bits for
+
 struct rfk_session {
     rfk_model m{};
     int N = 0, res = 0, Se = 0, Se_pad = 0, pH = 0, pW = 0, nP = 0, hd = 0, flags = 0;
@@ -429,7 +431,7 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
                            cudaMemcpyDeviceToDevice) != cudaSuccess)
                 return fail((int)cudaGetLastError());
     }
-    d->folds_kv = !d->ctx->reproducible && dim == 1024 && nh % 4 == 0 && (d->hd == 64 || d->hd == 128) && model->dec_layers <= 16 &&
+    d->folds_kv = !d->ctx->reproducible && dim == 1024 && nh % 4 == 0 && (d->hd == 64 || d->hd == 128) && model->dec_layers <= kMaxFoldedKv &&
                   (reinterpret_cast<uintptr_t>(scene_state) & 15u) == 0;
     for (int i = 0; i < model->dec_layers && d->folds_kv; ++i) {
         const auto given = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
@@ -541,7 +543,7 @@ struct EncodeBuffers {
         kv_w = nullptr;
         if (d.folds_kv) {
             c.get(&kv_w, 2 * (size_t)m.dec_layers * dim * dim);
-            c.get(&kv_mul, 2 * m.dec_layers);
+            c.get(&kv_mul, 2 * m.dec_layers * (dim / 64));
             c.get(&kv_ss, (2 * (size_t)m.dec_layers + 1) * Se * 4);
         }
         if (base) {
@@ -559,9 +561,9 @@ struct EncodeBuffers {
 };
 
 // The cross-attention's keys and values of all decoder layers. They are 24 products of the same rows behind 12 norms that differ in their weights
-// alone: with those in the products' weights (folded anew each time, 96 MB of traffic) they are one product of 24576 columns, whose
+// alone: with those in the products' weights (folded anew each time, 100 MB of traffic) they are one product of 24576 columns, whose
 // tiles fill the SMs where 92 of one layer's left a third of them idle, stored head-split in the cache; then the keys' own norm in
-// place, all layers at once. 5633 triangles: 12 x 43 us (norm, product, transposing norm, product, two memsets) -> 280 (folding 21, product 190 = 1.5
+// place, all layers at once. 5633 triangles: 12 x 43 us (norm, product, transposing norm, product, two memsets) -> 280 (folding 24, product 190 = 1.5
 // PFLOP/s, norm 46, context rows 8), scenes of 60 triangles 735 -> 547 us in all, 1000 1275 -> 1106, 5633 5500 -> 5250. RFK_EUNSUPPORTED with nothing but work
 // space written: layer by layer instead. That is known ahead of all work where few layers and rows make a product of small tiles (up to 1152 rows of one
 // layer, 128 of nine), whose weights would be folded for too little and whose sums are more than kv_ss has room for.
@@ -570,20 +572,23 @@ static int encode_kv(rfk_session& d, EncodeBuffers& b, const float* ctx_ss) {
     const rfk_stream_t s = (rfk_stream_t)d.stream;
     const int layers = m.dec_layers, dim = m.dim, Se = d.Se, Se_pad = d.Se_pad, hd = d.hd;
     if (!rfk::folded_on_pairs(Se, 2 * layers * dim)) return RFK_EUNSUPPORTED;
-    const rfk_half *k[RFK_MAX_LAYERS], *v[RFK_MAX_LAYERS];
-    const float *gamma[RFK_MAX_LAYERS], *key_gamma[RFK_MAX_LAYERS];
+    const rfk_half* w[2 * kMaxFoldedKv];
+    const float *gamma[2 * kMaxFoldedKv], *key_gamma[kMaxFoldedKv];
+    int rows[2 * kMaxFoldedKv];
     for (int i = 0; i < layers; ++i) {
-        k[i] = m.dec[i].cross_attn.k_proj_w; v[i] = m.dec[i].cross_attn.v_proj_w;
-        gamma[i] = m.dec[i].kv_norm_gamma; key_gamma[i] = m.dec[i].cross_attn.k_norm_gamma;
+        w[2 * i] = m.dec[i].cross_attn.k_proj_w; w[2 * i + 1] = m.dec[i].cross_attn.v_proj_w;
+        gamma[2 * i] = gamma[2 * i + 1] = m.dec[i].kv_norm_gamma;
+        rows[2 * i] = rows[2 * i + 1] = dim;
+        key_gamma[i] = m.dec[i].cross_attn.k_norm_gamma;
     }
-    TRY(rfk::fold_kv_weights(k, v, gamma, b.kv_w, b.kv_mul, layers, dim, s));
+    TRY(rfk::fold_weights(w, gamma, rows, 2 * layers, dim, b.kv_w, b.kv_mul, s));
     const long long slab = (long long)Se_pad * dim;
     rfk::FoldedProduct p{};
     p.A = b.ctx16; p.W = b.kv_w; p.C = d.kvK(0); p.M = Se; p.N = 2 * layers * dim; p.K = dim; p.in_ss = ctx_ss; p.in_tiles = dim / 256; p.in_mul = 1.0f;
     p.eps = kEpsFp16; p.out_ss = b.kv_ss; p.ss_mask = 0x55555555; p.part_stride = slab; p.seq = Se; p.out_seq = Se_pad; p.num_heads = m.num_heads;
-    p.head_dim = hd; p.part_mul = b.kv_mul;
+    p.head_dim = hd;
     int tiles = 0;
-    TRY(rfk::gemm_folded(p, &tiles, s, {/*pairs=*/1}));
+    TRY(rfk::gemm_folded(p, &tiles, s, {/*pairs=*/1, b.kv_mul}));
     if (Se_pad != Se) {   // the rows behind the last key of each head
         const size_t row = (size_t)hd * 2;
         TRY_CUDA(cudaMemset2DAsync((char*)d.kvK(0) + Se * row, Se_pad * row, 0, (Se_pad - Se) * row, (size_t)2 * layers * m.num_heads, d.stream));

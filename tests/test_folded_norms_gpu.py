@@ -15,20 +15,23 @@ class Product(ctypes.Structure):
     _fields_ = [(n, ctypes.c_void_p) for n in ("A", "W", "W_up", "R", "C", "raster")] + [(n, ctypes.c_int) for n in ("M", "N", "K")] + [
         ("in_ss", ctypes.c_void_p), ("in_tiles", ctypes.c_int), ("in_mul", ctypes.c_float), ("eps", ctypes.c_float), ("out_ss", ctypes.c_void_p),
         ("ss_mask", ctypes.c_int), ("part_stride", ctypes.c_longlong)] + [
-        (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "out_seq")] + [("part_mul", ctypes.c_void_p)] + [
-        (n, ctypes.c_int) for n in ("blocks_across", "blocks_down", "shift_from", "shift_to", "quarters")]
+        (n, ctypes.c_int) for n in ("seq", "num_heads", "head_dim", "out_seq", "blocks_across", "blocks_down", "shift_from", "shift_to", "quarters")]
 
 
-def _run(path=0, **kw):
+class More(ctypes.Structure):
+    _fields_ = [("pairs", ctypes.c_int), ("w_mul", ctypes.c_void_p), ("w_up_mul", ctypes.c_void_p)]
+
+
+def _run(path=0, w_mul=None, **kw):
     lib = _abi.load("rfk.h")
-    f = Product()
+    f, more = Product(), More(w_mul=w_mul.data_ptr() if w_mul is not None else None)
     f.eps = EPS
     for k, v in kw.items():
         setattr(f, k, v.data_ptr() if torch.is_tensor(v) else v)
     tiles = ctypes.c_int()
     assert lib.rfk_gemm_set_path(path) == 0
     try:
-        rc = lib.rfk_gemm_folded(ctypes.byref(f), ctypes.byref(tiles), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        rc = lib.rfk_gemm_folded_more(ctypes.byref(f), ctypes.byref(more), ctypes.byref(tiles), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     finally:
         lib.rfk_gemm_set_path(0)
     assert rc == 0
@@ -187,7 +190,29 @@ def test_folded_weights(rows):
     out, mul = _fold(w, gamma)
     assert (mul.log2() == mul.log2().round()).all()
     product = torch.cat([a.float() * g for a, g in zip(w, gamma)])
+    largest = (product.abs().view(-1, 64 * 1024).amax(1) / mul).log2()
+    assert (largest >= 13).all() and (largest <= 14).all()
     assert torch.equal(out, (product / mul.repeat_interleave(64)[:, None]).half())
+
+
+@pytest.mark.parametrize("spread", [0.0, 1.0, 1.5, 2.0, "half"])
+@pytest.mark.parametrize("M", [64, 512, 4096])
+def test_norm_weights_that_hold_down_large_channels(M, spread):
+    """Weight x norm weight keeps the bits of an fp16 value however far norm weights lie apart. Each product has one operand rounded (2^-11 of it at most,
+    2^-11 / sqrt 3 in the mean of squares, for a mantissa anywhere in its binade less), and so has the result: 4e-4 of the result's norm."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    N = K = 1024
+    gamma = torch.where(torch.arange(K, device="cuda") % 2 == 0, 1.0, 0.001) if spread == "half" else torch.exp(spread * n(K))
+    w, x = (0.02 * n(N, K)).half(), (n(M, K) / gamma).half()
+    f, mul = _fold([w], [gamma])
+    ss = x.float().square().view(M, 4, -1).sum(-1).contiguous()
+    out = torch.empty(1, 16, M, 64, device="cuda", dtype=torch.half)
+    _run(A=x, W=f, C=out, M=M, N=N, K=K, in_ss=ss, in_tiles=4, in_mul=1.0, part_stride=M * N, seq=M, num_heads=16, head_dim=64, w_mul=mul)
+    xd = x.double()
+    want = (xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + EPS) * gamma.double()) @ w.double().t()
+    got = out[0].permute(1, 0, 2).reshape(M, N).double()
+    assert (got - want).norm() <= 4e-4 * want.norm()
 
 
 def _scene(n, seed):
@@ -291,7 +316,7 @@ def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts,
     out = torch.full((parts, heads, pad, hd), 7.0, device="cuda", dtype=torch.half)
     sums = torch.full((parts * M * dim // 32,), float("nan"), device="cuda")
     tiles = _run(path, A=x, W=w, C=out, M=M, N=N, K=K, in_ss=ss, in_tiles=4, in_mul=1.0, out_ss=sums, ss_mask=0x55555555, part_stride=dim * pad, seq=M,
-                 num_heads=heads, head_dim=hd, out_seq=pad, part_mul=mul)
+                 num_heads=heads, head_dim=hd, out_seq=pad, w_mul=mul.repeat_interleave(dim // 64))
     assert (out[:, :, M:] == 7.0).all()
     got = out[:, :, :M].permute(2, 0, 1, 3).reshape(M, N)
     factor = _factor(x, 1.0)
@@ -316,15 +341,11 @@ def test_factors_of_parts_without_sums(M, parts):
     mul = 2.0 ** (3 * torch.arange(parts, device="cuda")).float()
     out = torch.full((parts, 1, dim // hd, M, hd), float("nan"), device="cuda", dtype=torch.half)
     _run(A=x, W=w, C=out, M=M, N=parts * dim, K=K, in_ss=ss, in_tiles=K // 256, in_mul=1.0, part_stride=M * dim, seq=M, num_heads=dim // hd, head_dim=hd,
-         part_mul=mul)
+         w_mul=mul.repeat_interleave(dim // 64))
     got, factor = out.permute(1, 3, 0, 2, 4).reshape(M, parts * dim), _factor(x, 1.0)
     for i in range(parts):
         cols = slice(i * dim, (i + 1) * dim)
         _near(got[:, cols], (x.float() @ w[cols].float().t()) * factor * mul[i], K)
-
-
-class More(ctypes.Structure):
-    _fields_ = [("pairs", ctypes.c_int), ("w_mul", ctypes.c_void_p), ("w_up_mul", ctypes.c_void_p)]
 
 
 # both sides of the line, which is 148 tiles of 128 x 128 on 148 SMs: 1 layer of keys and values, 3, 9 and 12
