@@ -322,7 +322,8 @@ size_t rfk_scene_state_bytes(const rfk_model* model, int n_tris);
  * The weights stay the caller's and are read where they lie, except that a session keeps copies, laid out for its kernels, of an image head's
  * filters and of the cross-attention's query norms (taken when it is created) and, where it ends at the token map and rows are 1024
  * wide, of the decoder's products behind a norm with the norm's weight multiplied in (24 MB a layer at 4096 hidden; taken by
- * rfk_session_finalize, and again by every rfk_session_encode_scene after that).
+ * rfk_session_finalize, and again by every rfk_session_encode_scene or rfk_session_finalize after that: weights that change in
+ * place count in a session from its next call of either, also in one that shares its scene state with the session that encodes).
  * replaces the allocation half of rf::RenderSession::create — src/pipeline/render_session.cu:258-295,418-462 */
 int rfk_session_create(const rfk_model* model, int n_tris, int img_res, void* scene_state,
                        int flags, rfk_session** out);
@@ -348,7 +349,8 @@ int rfk_session_encode_scene(rfk_session* s, const float* tri, const float* vn,
                              const rfk_half* tex);
 
 /* Builds the per-session constants (query RoPE tables, shift mask), runs one warm-up view and
- * captures the per-view CUDA graph. Call after the scene state is complete on this device.
+ * captures the per-view CUDA graph. Call after the scene state is complete on this device. On a session that is finalized it
+ * takes the session's copies of weights anew (rfk_session_create) and does nothing else. Synchronises at the end.
  * replaces render_session.cu:430-495 */
 int rfk_session_finalize(rfk_session* s);
 

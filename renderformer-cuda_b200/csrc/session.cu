@@ -676,7 +676,12 @@ static int check_attention_error() {
 
 extern "C" int rfk_session_finalize(rfk_session* d) {
     if (!d) return RFK_EINVAL;
-    if (d->finalized) return RFK_OK;
+    if (d->finalized) {
+        if (!d->folded) return RFK_OK;
+        TRY(d->fold_weights());   // should the weights be others now: this session may not be the one that encodes
+        TRY_CUDA(cudaStreamSynchronize(d->stream));
+        return RFK_OK;
+    }
     const rfk_model& m = d->m;
     std::vector<uint8_t> mask = build_window_mask(d->pH, d->pW, m.window_size, m.shift_size);
     TRY_CUDA(cudaMemcpy(d->shift_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice));

@@ -309,6 +309,7 @@ class RenderSession:
                                                                            tex.data_ptr()))
 
     def finalize(self):
+        """Captures the per-view graph; on a finalized session it takes the session's copies of the model's weights anew."""
         torch.cuda.synchronize()
         _check("rfk_session_finalize", _lib().rfk_session_finalize(self.h))
 
@@ -487,7 +488,7 @@ class ViewScheduler:
 
     def load_scene(self, tri=None, vn=None, tex=None, src: int = 0):
         """Rank `src` passes the scene tensors and runs the encoder; every rank receives the
-        scene state. Returns the broadcast time in ms (device events, this rank)."""
+        scene state, and every session takes its copies of the weights anew. Returns the broadcast time in ms (device events, this rank)."""
         if self.rank == src:
             self.encode_scene(tri, vn, tex)
         self.broadcast_scene(src)

@@ -303,6 +303,39 @@ def test_norm_weights_changed_across_powers_of_two(heads, res, use_graph):
     assert not torch.equal(before, want) and torch.equal(got, want)
 
 
+@pytest.mark.parametrize("views_per_frame", [1, 2])
+def test_every_session_of_a_scheduler_takes_changed_weights(views_per_frame):
+    """Two sessions share the scene state that one of them encodes; after load_scene both render with the weights as they are then."""
+    from renderformer_cuda_b200 import session
+    dims = dict(dim=1024, num_heads=16, ffn_hidden=512, enc_layers=1, dec_layers=2)
+    model, other = (session.Model.random(seed=k, **dims) for k in (3, 4))
+    scene, n = _scene(60, 1), 4 * views_per_frame
+    c2w = torch.eye(4).repeat(n, 1, 1)
+    c2w[:, 2, 3] = 3.0 + 0.1 * torch.arange(n)
+    fov, out = torch.full((n,), 0.7), torch.empty(n, 64, 1024, dtype=torch.half).pin_memory()
+    def render(s):
+        assert s.render(c2w, fov, out) == list(range(n))
+        return out.clone()
+    new = lambda m: session.ViewScheduler(m, 60, 64, streams_per_gpu=2, views_per_frame=views_per_frame)
+    s = new(model)
+    s.load_scene(*scene)
+    before = render(s)
+    for k, t in model.t.items():   # all but the query norms of the cross-attention, which a session takes over when it is made
+        if k.endswith("cq_norm"):
+            other.t[k].copy_(t)
+        else:
+            t.copy_(other.t[k])
+    s.load_scene(*scene)
+    got = render(s)
+    s.close()
+    f = new(other)
+    f.load_scene(*scene)
+    want = render(f)
+    f.close()
+    for v in range(n):
+        assert not torch.equal(before[v], want[v]) and torch.equal(got[v], want[v]), v
+
+
 @pytest.mark.parametrize("M,pad,parts,hd", [(1, 8, 4, 64), (333, 336, 24, 128), (777, 784, 6, 64), (2665, 2672, 8, 64)])
 @pytest.mark.parametrize("path", [0, 2])
 def test_parts_with_factors_of_their_own_and_room_behind_the_rows(M, pad, parts, hd, path):
