@@ -321,7 +321,7 @@ size_t rfk_scene_state_bytes(const rfk_model* model, int n_tris);
  * Allocates every per-view buffer; runs nothing.
  * The weights stay the caller's and are read where they lie, except that a session keeps copies, laid out for its kernels, of an image head's
  * filters and of the cross-attention's query norms (taken when it is created) and, where it ends at the token map and rows are 1024
- * wide, of the decoder's products behind a norm with the norm's weight multiplied in (24 MB a layer at 4096 hidden; taken by
+ * wide, of the decoder's products behind a norm with the norm's weight multiplied in (24 MB a layer at 4096 hidden, if they fit; taken by
  * rfk_session_finalize, and again by every rfk_session_encode_scene or rfk_session_finalize after that: weights that change in
  * place count in a session from its next call of either, also in one that shares its scene state with the session that encodes).
  * replaces the allocation half of rf::RenderSession::create — src/pipeline/render_session.cu:258-295,418-462 */

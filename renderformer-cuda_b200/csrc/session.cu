@@ -215,6 +215,12 @@ struct rfk_session {
         return RFK_OK;
     }
 
+    void release(void* p) {
+        owned.erase(std::remove(owned.begin(), owned.end(), p), owned.end());
+        cudaFree(p);
+    }
+    void alloc_folded();
+    void drop_folded();
     int fold_weights();
     int render_view(const float* pinned_cam, rfk_half* result_out, rfk_half* const* taps_out, float* image_out);
 };
@@ -312,6 +318,33 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
         TRY(rfk_post_elu_pow10(rfk_dpt_output(dpt), image_out, (long long)V * dptw.out_dim * res * res, 1e-3f, s));
     }
     return RFK_OK;
+}
+
+// The buffers of the folded layers, 300 MB at the published sizes. They come last: where a session fits only without them, it keeps separate norms.
+void rfk_session::alloc_folded() {
+    const size_t rows = (size_t)V * nP, dim = m.dim, ffn_rows = m.ffn_hidden, layer_rows = 4 * dim + 2 * ffn_rows;   // of weights, in whole 64s
+    if (alloc(&fold_w, m.dec_layers * layer_rows * dim) || alloc(&fold_mul, m.dec_layers * layer_rows / 64) || alloc(&x_other, rows * dim) ||
+        alloc(&fbuf.x_ss, rows * dim / 32) || alloc(&fbuf.qk_ss, rows * dim / 16))
+        return drop_folded();
+    for (int i = 0; i < m.dec_layers; ++i) {
+        const size_t at[4] = {i * layer_rows, i * layer_rows + dim, i * layer_rows + 4 * dim, i * layer_rows + 4 * dim + ffn_rows};
+        const auto weights = [&](int k) { return fold_w + at[k] * dim; };
+        const auto mul = [&](int k) { return fold_mul + at[k] / 64; };
+        fold[i] = FoldedWeights{weights(0), weights(1), weights(2), weights(3), mul(0), mul(1), mul(2), mul(3)};
+    }
+    fbuf.attn = temp;
+    fbuf.q = fbuf.qkv = proj;
+    fbuf.act = qkv;
+}
+
+// ... and without them; not once a captured view uses them
+void rfk_session::drop_folded() {
+    cudaGetLastError();
+    for (void* p : {(void*)fold_w, (void*)fold_mul, (void*)x_other, (void*)fbuf.x_ss, (void*)fbuf.qk_ss})
+        if (p) release(p);
+    fold_w = x_other = nullptr;
+    fold_mul = fbuf.x_ss = fbuf.qk_ss = nullptr;
+    folded = false;
 }
 
 // The weights of the folded products and their scales, where a captured graph finds them: nothing of them is an argument of a launch.
@@ -442,23 +475,6 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
                 !((reinterpret_cast<uintptr_t>(model->ray_enc_norm) | reinterpret_cast<uintptr_t>(model->ray_map_patch_token)) & 15u);
     for (int i = 0; i < model->dec_layers && d->folded; ++i)
         d->folded = layer_folds(model->dec[i], nP, dim, nh, ffn, d->pH, d->pW, ws, model->shift_size);
-    if (d->folded) {
-        const size_t rows = V * nP, layer_rows = 4 * (size_t)dim + 2 * (size_t)ffn;   // in whole 64s
-        ALLOC(fold_w, model->dec_layers * layer_rows * dim);
-        ALLOC(fold_mul, model->dec_layers * layer_rows / 64);
-        for (int i = 0; i < model->dec_layers; ++i) {
-            const size_t at[4] = {i * layer_rows, i * layer_rows + dim, i * layer_rows + 4 * dim, i * layer_rows + 4 * dim + ffn};
-            const auto weights = [&](int k) { return d->fold_w + at[k] * dim; };
-            const auto mul = [&](int k) { return d->fold_mul + at[k] / 64; };
-            d->fold[i] = FoldedWeights{weights(0), weights(1), weights(2), weights(3), mul(0), mul(1), mul(2), mul(3)};
-        }
-        ALLOC(x_other, rows * dim);
-        ALLOC(fbuf.x_ss, rows * dim / 32);
-        ALLOC(fbuf.qk_ss, rows * dim / 16);
-        d->fbuf.attn = d->temp;
-        d->fbuf.q = d->fbuf.qkv = d->proj;
-        d->fbuf.act = d->qkv;
-    }
     const bool fused_attention = d->hd == 64 || d->hd == 128;  // rfk_flash_attention serves these
     if (!fused_attention) ALLOC(score, V * nh * nP * Se_pad);
     if (!(ws * ws == 64 && d->hd == 64)) ALLOC(self_score, V * nWin * nh * ws * ws * ws * ws);
@@ -471,6 +487,7 @@ extern "C" int rfk_session_create_batched(const rfk_model* model, int n_tris, in
         if ((rc = rfk_dpt_create(d->ctx, &d->dptw, views_per_frame, dim, d->pH, d->pW, model->patch_size, &d->dpt))) return fail(rc);
     }
 #undef ALLOC
+    if (d->folded) d->alloc_folded();
     const float id[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
     if (cudaMemcpy(d->id_c2w, id, sizeof(id), cudaMemcpyHostToDevice) != cudaSuccess) return fail((int)cudaGetLastError());
     *out = d;
@@ -605,7 +622,14 @@ extern "C" int rfk_session_encode_scene(rfk_session* d, const float* tri, const 
     cudaStream_t st = d->stream;
     rfk_stream_t s = (rfk_stream_t)st;
     EncodeBuffers b{};
-    if (!d->encode_block) TRY(d->alloc(&d->encode_block, b.plan(*d, nullptr)));
+    while (!d->encode_block) {   // where it does not fit: without the folded weights, the encoding's or the views'
+        const int rc = d->alloc(&d->encode_block, b.plan(*d, nullptr));
+        if (rc == RFK_OK) break;
+        if (d->folds_kv) d->folds_kv = false;
+        else if (d->folded && !d->finalized) d->drop_folded();
+        else return rc;
+        cudaGetLastError();
+    }
     b.plan(*d, d->encode_block);
 
     scene_inputs_kernel<<<blocks_for((long long)N * std::max(9, C)), 256, 0, st>>>(

@@ -303,6 +303,28 @@ def test_norm_weights_changed_across_powers_of_two(heads, res, use_graph):
     assert not torch.equal(before, want) and torch.equal(got, want)
 
 
+def test_sessions_fit_where_they_fit_without_folded_weights():
+    """150 MB less than a session takes are left, of which 302 MB are folded weights: it keeps separate norms, and renders."""
+    from renderformer_cuda_b200 import session
+    model = session.Model.random(seed=3, dim=1024, num_heads=16, ffn_hidden=4096, enc_layers=1, dec_layers=12)
+    scene, mb = _scene(60, 1), 1 << 20
+    free = lambda: torch.cuda.mem_get_info()[0]
+    torch.cuda.empty_cache()
+    s, want = _view(model, scene, 64)     # whatever is loaded and kept once, and how much a session takes
+    few, want = s.kernels_per_view, want.clone()
+    with_all = free()
+    s.close()
+    took = free() - with_all
+    assert took > 450 * mb
+    taken = torch.empty(free() - took + 150 * mb, dtype=torch.uint8, device="cuda")
+    s, got = _view(model, scene, 64)
+    assert s.kernels_per_view > few
+    s.close()
+    del taken
+    torch.cuda.empty_cache()
+    assert (got.float() - want.float()).norm() <= 3e-3 * want.float().norm()
+
+
 @pytest.mark.parametrize("views_per_frame", [1, 2])
 def test_every_session_of_a_scheduler_takes_changed_weights(views_per_frame):
     """Two sessions share the scene state that one of them encodes; after load_scene both render with the weights as they are then."""
