@@ -127,7 +127,7 @@ struct Params {
 __device__ const float g_one = 1.0f;
 __device__ __forceinline__ float column_factor(const Params& p, const float* mul, int col) {
     float f;   // volatile: asked for where it is written, ahead of the loads that row_factor waits for, and not behind the products
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(mul ? mul + min(col, p.N - 1) / 64 : &g_one));
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(mul ? mul + (min(col, p.N - 1) >> 6) : &g_one));
     return f;
 }
 // a row's factor (kFold)
@@ -427,7 +427,7 @@ namespace pair { using namespace pair_ptx; }
 //   on 32 SMs, and with 256 rows the 128 tiles take 98 MB out of L2. The sum is therefore defined as ((a + b) + c) + d of its quarters of K for views of
 //   at most 256 rows, whatever frame they are in. For few rows a cluster of four CTAs takes a quarter each, of wider tiles; the fp32 rows go to the CTA
 //   of their quarter of the tile through the cluster's shared memory, and a warp of it finishes 32 columns. For more rows one CTA keeps the four
-//   sums in accumulators of their own. us, one sum / quarters, K = 4096, N = 1024: 64 rows 8.7 / 5.6, 128 8.7 / 6.3, 192 8.9 / 7.8, 256 9.1 / 7.9, and on single
+//   sums in accumulators of their own, and for more than a round of those the pair kernel makes them (kSumThreads). us, one sum / quarters, K = 4096, N = 1024: 64 rows 8.7 / 5.6, 128 8.7 / 6.3, 192 8.9 / 7.8, 256 9.1 / 7.9, and on single
 //   CTAs 320 9.8 / 10.0, 512 10.0 / 10.2, 1024 13.8 / 13.8; a view of 64 x 64 pixels 539 / 505, of 128 x 128 648 / 637, frames of four of these 847 / 843. With
 //   K = 1024 the exchange (0.8 to 1.5 us) costs more than it gains (64 rows 3.63 / 3.87): these keep one sum.
 //   A stage is two K blocks: one wait, one announcement and one commit for eight products. The issuing lane and the producer's are
@@ -973,17 +973,43 @@ __device__ __forceinline__ void tma_store_5d(const void* tmap, uint32_t src_smem
 }
 // Residual epilogue, before the tile's accumulator is waited for: bring the warp's residual rows of the whole tile
 // into its four staging buffers. Lane 0 only. The buffers were last read by the TMA stores of the previous tile.
-template <int EPI, int BN>
+template <int EPI, int UNITS>
 __device__ __forceinline__ void epilogue_prefetch_residual(const CUtensorMap* map_r, uint32_t stage_base, uint64_t* res_full,
                                                            int row0, int n0) {
     if (EPI != RFK_GEMM_EPI_RESIDUAL) return;
     bulk_wait_read<0>();
 #pragma unroll
-    for (int u = 0; u < Cfg<EPI, BN>::kUnits; ++u) {   // units beyond N are loaded too (all zeros): every barrier sees one phase per tile
+    for (int u = 0; u < UNITS; ++u) {   // units beyond N are loaded too (all zeros): every barrier sees one phase per tile
         tc::mbar_arrive_expect_tx(&res_full[u], kUnitBytes);
         tma_load_2d(stage_base + u * kUnitBytes, map_r, n0 + u * kUnitCols, row0, &res_full[u]);
     }
 }
+
+// FOLD, residual: where a warp's 32 rows go
+struct RowPlaces {
+    int ss_row;        // the lane's sums of squares
+    int block[2][3];   // view and place of the warp's two blocks, if rows move
+    __device__ __forceinline__ RowPlaces(const Params& p, int row0, int lane) : ss_row(row0 + lane), block{} {
+        if (!p.grid.bw) return;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) p.grid.block((row0 >> 4) + h, block[h][0], block[h][1], block[h][2]);
+        const int h = lane >> 4;
+        ss_row = p.grid.next(h ? block[1][0] : block[0][0], h ? block[1][1] : block[0][1], h ? block[1][2] : block[0][2]) * 16 + (lane & 15);
+    }
+    // one lane: a unit's stores from its buffer
+    __device__ __forceinline__ void store(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, uint32_t buf, int col, int row0) const {
+        if (!p.grid.bw) {
+            tma_store_2d(map_c, buf, col, row0);   // rows >= M, columns >= N are clipped
+        } else if (row0 < p.M) {                   // two blocks of 16 rows; M is a whole number of them, 32 at a time
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t src = buf + h * (kUnitBytes / 2);
+                if (p.C) tma_store_2d(map_c, src, col, p.grid.next(block[h][0], block[h][1], block[h][2]) * 16);
+                if (p.raster) tma_store_3d(map_raster, src, col, block[h][2] * 4, (block[h][0] * p.grid.bh + block[h][1]) * 4);
+            }
+        }
+    }
+};
 
 // One epilogue warp, one tile: accumulator rows [lane] -> (bias / residual / gate) -> fp16 -> staging buffer -> TMA store.
 // t_acc: tensor-memory address of the thread's accumulator row; row0: global row of the warp's lane 0. turn: the staging buffer of the
@@ -1009,13 +1035,9 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     const uint32_t stage_base = tc::smem_addr(stage_ptr);
     uint32_t v[32];
     float ss = 0.0f;   // kEpiHeads: this row's sum of squares over the tile
-    int ss_row = row0 + lane, block[2][3] = {};   // FOLD, residual: where the row's sums go; view and place of the warp's two blocks
-    if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && p.grid.bw) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) p.grid.block((row0 >> 4) + h, block[h][0], block[h][1], block[h][2]);
-        const int h = lane >> 4;
-        ss_row = p.grid.next(h ? block[1][0] : block[0][0], h ? block[1][1] : block[0][1], h ? block[1][2] : block[0][2]) * 16 + (lane & 15);
-    }
+    constexpr bool kPlaced = FOLD && EPI == RFK_GEMM_EPI_RESIDUAL;
+    const RowPlaces places = kPlaced ? RowPlaces(p, row0, lane) : RowPlaces(Params{}, row0, lane);
+    const int ss_row = places.ss_row;
     // Lane l holds columns 2l and 2l + 1 of a unit's bias, fetched a unit ahead. Each thread reading all 64 of them, one load's latency after the other, was
     // 2.5 us a tile: 262144 x 256 x 256 90.7 -> 57.5 us (54.7 without a bias), 65536 x 256 x 256 25.4 -> 15.8, 4096 x 1024 x 1024 13.4 -> 11.0, x 192 9.1 -> 6.7.
     constexpr bool kBiased = !FOLD && (EPI == RFK_GEMM_EPI_NONE || EPI == RFK_GEMM_EPI_RESIDUAL);
@@ -1126,17 +1148,8 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
                 const int g = (n0 + u * kUnitCols) / kUnitCols;   // 64-column unit over all parts
                 tma_store_5d(map_c, stage_base + b * kUnitBytes, (g % p.head_units) * kUnitCols, row0 % p.seq,
                              (g % p.units) / p.head_units, row0 / p.seq, g / p.units);
-            } else if (FOLD && EPI == RFK_GEMM_EPI_RESIDUAL && p.grid.bw) {   // two blocks of 16 rows; M is a whole number of them, 32 at a time
-                if (row0 < p.M) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t src = stage_base + b * kUnitBytes + h * (kUnitBytes / 2);
-                        if (p.C)
-                            tma_store_2d(map_c, src, n0 + u * kUnitCols, p.grid.next(block[h][0], block[h][1], block[h][2]) * 16);
-                        if (p.raster)
-                            tma_store_3d(map_raster, src, n0 + u * kUnitCols, block[h][2] * 4, (block[h][0] * p.grid.bh + block[h][1]) * 4);
-                    }
-                }
+            } else if (kPlaced) {
+                places.store(p, map_c, map_raster, stage_base + b * kUnitBytes, n0 + u * kUnitCols, row0);
             } else {
                 tma_store_2d(map_c, stage_base + b * kUnitBytes, n0 + u * kUnitCols, row0);   // rows >= M, columns >= N are clipped
             }
@@ -1153,14 +1166,70 @@ __device__ __forceinline__ bool epilogue_tile_staged(const Params& p, const CUte
     return true;
 }
 
-template <int EPI_, int BN>
-__global__ void __launch_bounds__(kThreads, 1)
+// Sums in quarters of K (small tiles have the definition) for frames of many small views: each quarter is an accumulation of its own in the two accumulators in
+// turn, and eight epilogue warps add them up in registers, 128 columns of a row a thread, under the next quarter's products. (Four accumulators of 128
+// columns would read 24 KB a K block for half the products; small tiles, which read as much as this for half, were what such frames had.) us, small
+// tiles in rounds / this / one sum on pairs, K = 4096, N = 1024: 2560 rows 34.8 / 31.0 / 24.0 (192 columns a tile), 4096 37.8 / 32.2 / 29.8, 8192 80.9 / 62.3 / 57.6,
+// 16384 196 / 130 / 122; 2304, the most that small tiles take in one round, 19.7 there.
+constexpr int kSumThreads = 64 + 8 * 32;   // ten warps, three on a scheduler: 168 registers a thread, of which the sums take 128
+// 16 columns of the warp's rows, and the wait for them (tc::tmem_ld32 and tc::tc_wait_ld for fewer registers)
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+template <int SUM> constexpr int kPairThreads = SUM == 4 ? kSumThreads : kThreads;
+// One of those warps, one tile: the sums of its 32 rows x 128 columns -> residual -> fp16 -> staging buffers -> TMA stores, and squares
+__device__ __forceinline__ bool epilogue_sums(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_raster, const float (&sum)[128],
+                                              unsigned char* stage_ptr, uint64_t* res_full, uint32_t res_parity, int row0, int n0, int lane,
+                                              volatile int* abort_flag) {
+    const uint32_t stage_base = tc::smem_addr(stage_ptr);
+    const RowPlaces places(p, row0, lane);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        unsigned char* buf = stage_ptr + u * kUnitBytes;
+        if (!tc::mbar_wait_warp(&res_full[u], res_parity, abort_flag)) return false;
+#pragma unroll
+        for (int hc = 0; hc < 2; ++hc) {
+            uint32_t o[16];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 res = *reinterpret_cast<const uint4*>(buf + staged(lane, hc * 4 + q));
+                const uint32_t rw[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 rr = unpack_half2(rw[i]);
+                    const int c = u * 64 + hc * 32 + q * 8 + 2 * i;
+                    o[4 * q + i] = pack_half2(sum[c] + rr.x, sum[c + 1] + rr.y);
+                }
+            }
+            if (p.row_ss && row0 + lane < p.M) p.row_ss[(size_t)places.ss_row * p.ss_tiles + (n0 >> 5) + u * 2 + hc] = square_sum(o);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(buf + staged(lane, hc * 4 + q)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        }
+        tc::fence_proxy_async();                            // the copy engine reads what the threads just wrote
+        __syncwarp();
+        if (lane == 0) {
+            places.store(p, map_c, map_raster, stage_base + u * kUnitBytes, n0 + u * kUnitCols, row0);
+            bulk_commit();
+        }
+    }
+    return true;
+}
+
+// SUM: one sum over K, or four of its quarters
+template <int EPI_, int BN, int SUM = 1>
+__global__ void __launch_bounds__(kPairThreads<SUM>, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0,
                     const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_c,
                     const __grid_constant__ CUtensorMap map_r, const Params p) {
     constexpr int EPI = EPI_ & 7;
     constexpr bool FOLD = (EPI_ & kFold) != 0;
     static_assert(BN == 256 || (BN == 192 && EPI != RFK_GEMM_EPI_SWIGLU) || (BN == 128 && EPI == RFK_GEMM_EPI_SWIGLU), "whole 64-column units");
+    static_assert(SUM == 1 || (SUM == 4 && BN == 256 && FOLD && EPI == RFK_GEMM_EPI_RESIDUAL), "the form that is summed in quarters");
     constexpr int BN_OUT = (EPI == RFK_GEMM_EPI_SWIGLU) ? BN / 2 : BN;
     constexpr int kStageBytes = Cfg<EPI, BN>::kStageBytes;
     constexpr int kTxBytes = kABytes + BN / 2 * BK * 2;   // of a stage, per CTA
@@ -1181,7 +1250,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { tc::mbar_init(&ctrl->full[s], 1); tc::mbar_init(&ctrl->empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { tc::mbar_init(&ctrl->acc_full[a], 1); tc::mbar_init(&ctrl->acc_empty[a], 8); }
+        for (int a = 0; a < 2; ++a) { tc::mbar_init(&ctrl->acc_full[a], 1); tc::mbar_init(&ctrl->acc_empty[a], (kPairThreads<SUM> - 64) / 16); }   // a warp of both CTAs each
         tc::mbar_init(&ctrl->drain, 1);
         tc::mbar_init(&ctrl->started, 1);
         for (int w = 0; w < 4; ++w)
@@ -1252,30 +1321,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // us, lane 0 / elected lane: 4096 x 1024 x 4096 + residual 27.9 / 26.4, w1|w3 + SwiGLU 48.1 / 46.1, 3072 x 1024 20.5 / 20.2.
         if (rank == 0 && tc::elect_one()) {
             constexpr uint32_t idesc = tc::umma_idesc_f16(2 * BM, BN, 0);
-            int it = 0, tl = 0;
+            const int sum_kb = SUM == 1 ? num_kb : num_kb / SUM;
+            int it = 0, tl = 0;   // tl: accumulations, SUM a tile
             bool ok = true;
-            for (int t = first_tile; ok && t < num_tiles; t += tile_step, ++tl) {
-                const int acc = tl & 1;
-                if (tl >= 2) ok = wait_remote(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after();
-                const uint32_t d_tmem = tmem_cta + acc * BNACC;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % kStages;
-                    ok = wait(&ctrl->full[s], (it / kStages) & 1);
+            for (int t = first_tile; ok && t < num_tiles; t += tile_step) {
+                for (int q = 0; q < SUM; ++q, ++tl) {
+                    const int acc = tl & 1;
+                    if (tl >= 2) ok = wait_remote(&ctrl->acc_empty[acc], ((tl >> 1) + 1) & 1, abort_flag);
                     if (!ok) break;
-                    if (it == 0) RFK_STAMP(2);   // first K block has landed
                     tc::tc_fence_after();
-                    const uint32_t a_lo = tc::umma_desc_lo(base + s * kStageBytes);
-                    const uint32_t b_lo = tc::umma_desc_lo(base + s * kStageBytes + kABytes);
+                    const uint32_t d_tmem = tmem_cta + acc * BNACC;
+                    for (int kb = 0; kb < sum_kb; ++kb, ++it) {
+                        const int s = it % kStages;
+                        ok = wait(&ctrl->full[s], (it / kStages) & 1);
+                        if (!ok) break;
+                        if (it == 0) RFK_STAMP(2);   // first K block has landed
+                        tc::tc_fence_after();
+                        const uint32_t a_lo = tc::umma_desc_lo(base + s * kStageBytes);
+                        const uint32_t b_lo = tc::umma_desc_lo(base + s * kStageBytes + kABytes);
 #pragma unroll
-                    for (int ks = 0; ks < BK / 16; ++ks)
-                        umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb > 0) || (ks > 0));
-                    umma_pair_commit(&ctrl->empty[s]);
-                    if (EPI == RFK_GEMM_EPI_RESIDUAL && it == 0) umma_pair_commit(&ctrl->started);
+                        for (int ks = 0; ks < BK / 16; ++ks)
+                            umma_pair_f16_lo(d_tmem, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb > 0) || (ks > 0));
+                        umma_pair_commit(&ctrl->empty[s]);
+                        if (EPI == RFK_GEMM_EPI_RESIDUAL && it == 0) umma_pair_commit(&ctrl->started);
+                    }
+                    if (!ok) break;
+                    umma_pair_commit(&ctrl->acc_full[acc]);
+                    if (tl == 0) RFK_STAMP(3);       // all products of the first tile issued
                 }
-                if (ok) umma_pair_commit(&ctrl->acc_full[acc]);
-                if (tl == 0) RFK_STAMP(3);       // all products of the first tile issued
             }
             if (*abort_flag) {
                 umma_pair_commit(&ctrl->drain);
@@ -1284,11 +1357,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
     } else {
-        // ------------------------------------------------------------ epilogue, warps 2-5 of both CTAs
+        // ------------------------------------------------------------ epilogue, warps 2-5 of both CTAs (2-9: 6-9 take a tile's second half of columns)
         const int lane_grp = warp & 3;                        // a warp reaches tensor-memory lanes [32 * (warp % 4), +32)
         const uint32_t lane_off = (uint32_t)(lane_grp * 32) << 16;
-        unsigned char* my_stage = staging + lane_grp * Cfg<EPI, BN>::kBufsPerWarp * kUnitBytes;
-        uint64_t* my_res = ctrl->res_full[lane_grp];
+        const int unit0 = SUM == 4 ? (warp - 2) / 4 * 2 : 0;  // first unit
+        unsigned char* my_stage = staging + (lane_grp * Cfg<EPI, BN>::kBufsPerWarp + unit0) * kUnitBytes;
+        uint64_t* my_res = ctrl->res_full[lane_grp] + unit0;
         int tl = 0, turn = 0;
         for (int t = first_tile; t < num_tiles; t += tile_step, ++tl) {
             const bool last = t + tile_step >= num_tiles;
@@ -1300,7 +1374,36 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // (a multicast commit): issued at kernel start they delay the first operand tiles by ~0.5 us. The barrier has one
                 // phase, so a warp that comes late cannot miss it; empty[0] goes on to other phases.
                 if (EPI == RFK_GEMM_EPI_RESIDUAL && tl == 0) tc::mbar_wait(&ctrl->started, 0, abort_flag);
-                epilogue_prefetch_residual<EPI, BN>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0);
+                epilogue_prefetch_residual<EPI, SUM == 4 ? 2 : Cfg<EPI, BN>::kUnits>(&map_r, tc::smem_addr(my_stage), my_res, row0, n0 + unit0 * kUnitCols);
+            }
+            if constexpr (SUM == 4) {
+                float sum[128];
+#pragma unroll 1
+                for (int q = 0; q < 4; ++q) {
+                    const int n = 4 * tl + q, a = n & 1;
+                    ok = tc::mbar_wait_warp(&ctrl->acc_full[a], (n >> 1) & 1, abort_flag);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        uint32_t v[16];
+                        tmem_ld16(tmem_cta + lane_off + a * BNACC + unit0 * kUnitCols + c * 16, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) sum[c * 16 + i] = q == 0 ? __uint_as_float(v[i]) : sum[c * 16 + i] + __uint_as_float(v[i]);
+                    }
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (last && q == 3) {   // nobody waits for the last one, see below
+                        cluster_arrive();
+                        left = true;
+                    } else if (lane == 0) {
+                        remote_arrive(map_to_cta(tc::smem_addr(&ctrl->acc_empty[a]), 0));
+                    }
+                }
+                if (!ok) break;
+                ok = epilogue_sums(p, &map_c, &map_w1, sum, my_stage, my_res, tl & 1, row0, n0 + unit0 * kUnitCols, lane, abort_flag);
+                if (!ok) break;
+                continue;
             }
             UnitFactors<EPI_, BN> factors;
             if (FOLD && EPI != RFK_GEMM_EPI_RESIDUAL) {
@@ -1436,27 +1539,27 @@ int sm_count(int dev) {
 
 std::atomic<int> g_pair_clusters[64];  // CTA pairs the device can run at once, per device (0 not asked yet, -1 none)
 
-template <int EPI, int BN> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+template <int EPI, int BN, int SUM = 1> cudaLaunchConfig_t pair_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_pdl in common.cuh
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.blockDim = dim3(tcgemm::kThreads); cfg.dynamicSmemBytes = tcgemm::pair::Cfg<EPI, BN>::kSmemBytes; cfg.stream = st;
+    cfg.blockDim = dim3(tcgemm::pair::kPairThreads<SUM>); cfg.dynamicSmemBytes = tcgemm::pair::Cfg<EPI, BN>::kSmemBytes; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
     return cfg;
 }
 
 // *pairs: how many CTA pairs of this form the device runs at once (asked once per device and form; every form takes a whole SM a CTA);
 // RFK_EUNSUPPORTED where it cannot co-schedule pairs.
-template <int EPI, int BN>
+template <int EPI, int BN, int SUM = 1>
 int resident_pairs(int dev, int* pairs) {
     static std::atomic<bool> configured[64];
     int nc = g_pair_clusters[dev].load(std::memory_order_acquire);
     if (nc == 0 || !configured[dev].load(std::memory_order_acquire)) {
-        constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI, BN>;
+        constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI, BN, SUM>;
         cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = pair_config<EPI, BN>(attr, nullptr);
+        cudaLaunchConfig_t cfg = pair_config<EPI, BN, SUM>(attr, nullptr);
         cfg.numAttrs = 1;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
         if (e != cudaSuccess) return (int)e;
@@ -1477,11 +1580,11 @@ int resident_pairs(int dev, int* pairs) {
 }
 
 // CTA-pair kernel: clusters of two; returns RFK_EUNSUPPORTED (nothing launched) when the device cannot co-schedule pairs
-template <int EPI_, int BN>
+template <int EPI_, int BN, int SUM = 1>
 int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUtensorMap& mw1, tcgemm::Params p, int dev,
                       cudaStream_t st, const CUtensorMap* heads_map) {
     constexpr int EPI = EPI_ & 7;
-    constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI_, BN>;
+    constexpr auto kernel = tcgemm::pair::gemm_tc_pair_kernel<EPI_, BN, SUM>;
     // tile maps of the output (stores) and of the residual (loads): boxes of 32 rows x 64 columns, one per epilogue warp
     CUtensorMap mc, mr;
     if (heads_map) mc = *heads_map;
@@ -1490,10 +1593,10 @@ int launch_pair_tiles(const CUtensorMap& ma, const CUtensorMap& mw0, const CUten
                      EPI == RFK_GEMM_EPI_RESIDUAL ? p.ldr : p.ldc, 32))
         return RFK_EUNSUPPORTED;
     int pairs = 0;
-    const int rc = resident_pairs<EPI_, BN>(dev, &pairs);
+    const int rc = resident_pairs<EPI_, BN, SUM>(dev, &pairs);
     if (rc != RFK_OK) return rc;
     cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = pair_config<EPI_, BN>(attr, st);
+    cudaLaunchConfig_t cfg = pair_config<EPI_, BN, SUM>(attr, st);
     p.tiles_m = (p.M + 2 * tcgemm::BM - 1) / (2 * tcgemm::BM);
     constexpr int BN_OUT = EPI == RFK_GEMM_EPI_SWIGLU ? BN / 2 : BN;
     p.tiles_n = (p.N + BN_OUT - 1) / BN_OUT;
@@ -1793,6 +1896,11 @@ static bool make_map_raster(CUtensorMap* m, const void* base, int n, int width, 
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// small tiles, by the size of a product (SwiGLU aside)
+static bool folded_small(int M, int N, int dev) {
+    return g_gemm_path.load(std::memory_order_relaxed) == 0 && small_tile(M, N, sm_count(dev)) != 0;
+}
+
 // clusters of the split kernel that the device runs at once (asked once per device)
 template <int BM_, int BN_> static int resident_quarters(int dev) {
     constexpr int SUM = 4 | tcgemm::small::kSplit;
@@ -1818,9 +1926,18 @@ template <int BM_, int BN_> static int resident_quarters(int dev) {
 }
 
 // A residual product summed in quarters (FoldedProduct::quarters): one cluster a tile where they all run at once, else a CTA a tile with the
-// same sums
+// same sums where those do, else CTA pairs
 static int launch_quarters(const FoldedProduct& f, const tcgemm::Params& p, int dev, cudaStream_t st) {
     constexpr int E = RFK_GEMM_EPI_RESIDUAL | tcgemm::kFold, kSplit = 4 | tcgemm::small::kSplit;
+    if (!folded_small(p.M, p.N, dev)) {
+        CUtensorMap ma, mw, mraster;
+        if (!make_map_2d(&ma, f.A, p.M, p.K, p.K) || !make_map_2d(&mw, f.W, p.N, p.K, p.K) ||
+            (p.raster && !make_map_raster(&mraster, p.raster, p.N, p.grid.bw * 4, p.M / (p.grid.bw * 4))))
+            return RFK_EUNSUPPORTED;
+        const int rc = launch_pair_tiles<E, 256, 4>(ma, mw, p.raster ? mraster : mw, p, dev, st, nullptr);
+        if (rc != RFK_EUNSUPPORTED || g_gemm_path.load(std::memory_order_relaxed) == 2) return rc;
+        return launch_gemm_small<E, 128, 128, 4>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
+    }
     const auto tiles = [&](int bm, int bn) { return (long long)ceil_div(p.M, bm) * ceil_div(p.N, bn); };
     int rc = RFK_EUNSUPPORTED;
     if (tiles(64, 32) <= resident_quarters<64, 32>(dev)) rc = launch_gemm_small<E, 64, 32, kSplit>(f.A, p.K, f.W, nullptr, p.K, p, dev, st);
@@ -1835,11 +1952,6 @@ static int launch_quarters(const FoldedProduct& f, const tcgemm::Params& p, int 
     }
 }
 
-// small tiles, by the size of a product (SwiGLU aside)
-static bool folded_small(int M, int N, int dev) {
-    return g_gemm_path.load(std::memory_order_relaxed) == 0 && small_tile(M, N, sm_count(dev)) != 0;
-}
-
 bool rfk::folded_on_pairs(int M, int N) {
     int dev = 0;
     if (M <= 0 || N <= 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return false; }
@@ -1851,12 +1963,12 @@ static int launch_folded(const FoldedProduct& f, tcgemm::Params p, int dev, cuda
     constexpr int E = EPI | tcgemm::kFold;
     constexpr bool kGate = EPI == RFK_GEMM_EPI_SWIGLU;
     const int sums = (EPI == tcgemm::kEpiHeads ? p.units * 64 : p.N) / 32;
+    p.ss_tiles = sums;
+    *ss_tiles = sums;
+    if constexpr (EPI == RFK_GEMM_EPI_RESIDUAL)
+        if (f.quarters) return launch_quarters(f, p, dev, st);
     if (g_gemm_path.load(std::memory_order_relaxed) == 0) {
         int rc = RFK_EUNSUPPORTED;
-        p.ss_tiles = sums;
-        *ss_tiles = sums;
-        if constexpr (EPI == RFK_GEMM_EPI_RESIDUAL)
-            if (f.quarters) return launch_quarters(f, p, dev, st);
         if constexpr (kGate) rc = launch_narrow_gate<E>(f.A, p.K, f.W, f.W_up, p.K, p, dev, st);
         if (rc != RFK_EUNSUPPORTED) return rc;
         switch (small_tile(p.M, kGate ? 2 * p.N : p.N, sm_count(dev))) {

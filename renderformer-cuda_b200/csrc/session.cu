@@ -323,8 +323,8 @@ int rfk_session::render_view(const float* pinned_cam, rfk_half* result_out, rfk_
 // The buffers of the folded layers, 300 MB at the published sizes. They come last: where a session fits only without them, it keeps separate norms.
 void rfk_session::alloc_folded() {
     const size_t rows = (size_t)V * nP, dim = m.dim, ffn_rows = m.ffn_hidden, layer_rows = 4 * dim + 2 * ffn_rows;   // of weights, in whole 64s
-    if (alloc(&fold_w, m.dec_layers * layer_rows * dim) || alloc(&fold_mul, m.dec_layers * layer_rows / 64) || alloc(&x_other, rows * dim) ||
-        alloc(&fbuf.x_ss, rows * dim / 32) || alloc(&fbuf.qk_ss, rows * dim / 16))
+    if (alloc(&x_other, rows * dim) || alloc(&fbuf.x_ss, rows * dim / 32) || alloc(&fbuf.qk_ss, rows * dim / 16) ||
+        alloc(&fold_w, m.dec_layers * layer_rows * dim) || alloc(&fold_mul, m.dec_layers * layer_rows / 64))
         return drop_folded();
     for (int i = 0; i < m.dec_layers; ++i) {
         const size_t at[4] = {i * layer_rows, i * layer_rows + dim, i * layer_rows + 4 * dim, i * layer_rows + 4 * dim + ffn_rows};

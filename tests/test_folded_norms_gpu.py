@@ -451,10 +451,11 @@ def test_cache_of_all_layers_at_once_and_layer_by_layer(n, heads, layers):
         assert (got[i].float() - want[i].float()).norm() <= 1.5e-3 * want[i].float().norm()
 
 
-@pytest.mark.parametrize("views,h,w", [(1, 8, 8), (3, 8, 8), (1, 16, 16), (4, 16, 16), (9, 16, 16), (1, 8, 24), (21, 8, 8)])
+@pytest.mark.parametrize("views,h,w", [(1, 8, 8), (3, 8, 8), (1, 16, 16), (4, 16, 16), (9, 16, 16), (1, 8, 24), (21, 8, 8), (41, 8, 8), (17, 16, 16), (150, 8, 8)])
 @pytest.mark.parametrize("N,K", [(1024, 4096), (1024, 512), (256, 1536)])
 def test_sums_in_quarters(views, h, w, N, K):
-    """A residual product whose sum over K is that of its quarters: by clusters of four for few rows, by single CTAs for many. The sums and the
+    """A residual product whose sum over K is that of its quarters: by clusters of four for few rows, by single CTAs for more, by pairs for many (41 views of
+    64 rows: pair tiles with a tail of rows; 150: several tiles a pair, and pairs with 256 columns too). The sums and the
     order of their addition are the same whoever makes them: a view's rows have the bits of the frame that it shares; and they are those of four
     products of a quarter each, which leave fp32 nowhere, up to the distance of two orders."""
     rnd = _gen(views * 100 + h * w + K)
@@ -471,7 +472,13 @@ def test_sums_in_quarters(views, h, w, N, K):
     _near(raster[back], r.float() + a.float() @ wt.float().t(), K)
     assert torch.equal(out, _to_blocks(raster.view(views, h, w, N), 4))
     n = h * w
-    for v in {0, views - 1}:
+    if (views, h) in ((1, 8), (3, 8), (4, 16)):   # pairs whatever the size
+        again, again_raster, again_sums = torch.empty_like(out), torch.empty_like(raster), torch.empty_like(sums)
+        assert _run(2, A=a, R=r, C=again, raster=again_raster, out_ss=again_sums, M=M, **args) == tiles
+        assert torch.equal(again, out) and torch.equal(again_raster, raster) and torch.equal(again_sums, sums)
+        _run(2, A=a, W=wt, R=r, C=again, M=M, N=N, K=K, quarters=1)   # rows where they are, without sums
+        assert torch.equal(again, raster[back])
+    for v in {0, views // 2, views - 1}:
         alone, alone_raster = torch.full((n, N), float("nan"), device="cuda", dtype=torch.half), torch.full((n, N), float("nan"), device="cuda", dtype=torch.half)
         alone_sums = torch.full((n * N // 32,), float("nan"), device="cuda")
         _run(0, A=a[v * n:(v + 1) * n], R=r[v * n:(v + 1) * n], C=alone, raster=alone_raster, out_ss=alone_sums, M=n, **args)
