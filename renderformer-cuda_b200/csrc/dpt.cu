@@ -43,14 +43,6 @@ namespace {
 // 11.2 / 9.2, 128^2 34.6 / 29.5; 1024 -> 256 at 8^2 16.6 / 13.7, 32^2 16.9 / 14.2, 64^2 19.2 / 19.5 (the one size of 64 where it is not the faster
 // one); 256 -> 128 at 64^2 8.6 / 6.4, 320^2 56 / 43, 512^2 183 / 107; 128 -> 32 at 64^2 6.9 / 5.3, 320^2 40 / 16, 512^2 81 / 38.
 // A head over several views keeps the library, which chooses the order of its sums anew for every batch size.
-//
-// Those of large maps are counted (rfk_dpt_create_from's own_convolutions): of more than 2^31 multiply-adds a tap, maps of 256 channels whose
-// tiles of 256 x 256 would fill the pairs of SMs one and a half times, from 256 input channels up, and every map beyond 170000 pixels.
-bool large_map(int H, int W, int Cin, int Cout, int sms) {
-    if ((long long)H * W * Cin * Cout <= (1LL << 31)) return false;
-    const long long tiles = ((long long)((H + 7) / 8) * ((W + 15) / 16) + 1) / 2 * (Cout / 256);
-    return (long long)H * W > 170000 || (Cout % 256 == 0 && Cin >= 256 && 2 * tiles > 3 * (sms / 2));
-}
 
 // Operands of the plan's comparison of the two (order_of_sums): fp16 in [-1, 1), a hash of the position
 __global__ void fill_hashed_kernel(__half* p, long long n, unsigned seed) {
@@ -85,10 +77,9 @@ struct rfk_dpt {
     size_t ws_bytes = 0;
     std::vector<Step> program;
     rfk_half* out = nullptr;  // [B, out_dim, pH*ps, pW*ps]
-    int n_convs = 0, n_own = 0;      // convolutions in all; those of large maps that the tcgen05 kernel of conv_tc.cu takes
+    int n_convs = 0, n_own = 0;      // convolutions in all; those that the tcgen05 kernel of conv_tc.cu takes
     int n_library = 0;               // those that the library takes
     bool library_only = false;
-    int sms = 0;
     struct Order { int H, W, Cin, Cout, rows_outside; };
     std::vector<Order> orders;       // what order_of_sums found
     char* scratch = nullptr;         // order_of_sums' operands, while the head is planned
@@ -197,7 +188,7 @@ struct rfk_dpt {
         const bool may_own = !library_only && k == 3 && stride == 1 && pad == 1 && B == 1 &&
                              rfk_conv3x3_nhwc_serves(in, wk, bias, residual, o, o_silu, Cin, Cout);
         const auto push_own = [&](int rows_outside) {
-            if (large_map(H, W, Cin, Cout, sms)) ++n_own;
+            ++n_own;
             if (sum) {
                 *sum_silu = o;
                 program.push_back([=](const rfk_half* const*, cudaStream_t st) -> int {
@@ -425,11 +416,6 @@ extern "C" int rfk_dpt_create_from(rfk_ctx* ctx, const rfk_dpt_weights* w, int B
     rfk_dpt* d = new rfk_dpt();
     d->ctx = ctx; d->w = *w; d->B = B; d->dim = dim; d->pH = patch_h; d->pW = patch_w; d->ps = patch_size;
     d->library_only = library_only != 0;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        delete d;
-        return (int)cudaGetLastError();
-    }
     if (cudnnCreate(&d->dnn) != CUDNN_STATUS_SUCCESS) { delete d; return 2000; }
     const int rc = d->build();
     if (rc != RFK_OK) { rfk_dpt_destroy(d); return rc; }

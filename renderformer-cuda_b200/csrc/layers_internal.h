@@ -56,7 +56,7 @@ bool layer_folds(const rfk_decoder_layer_weights& w, int Sq, int dim, int num_he
 }  // namespace rfk_layers
 
 // rfk_dpt_create, with every 3x3 convolution left to the library if library_only, for the tests that compare the two;
-// *own_convolutions (may be NULL) = how many of large maps the tcgen05 kernel took (large_map in dpt.cu).
+// *own_convolutions (may be NULL) = how many convolutions the tcgen05 kernel took.
 extern "C" int rfk_dpt_create_from(rfk_ctx* ctx, const rfk_dpt_weights* w, int B, int dim, int patch_h, int patch_w, int patch_size,
                                    int library_only, int* own_convolutions, rfk_dpt** out);
 // how many convolutions of a head the library takes: those of stride 2, all of a head over several views, and those whose order of

@@ -128,8 +128,8 @@ def _plan(L, ctx, model, B, pH, pW, library_only):
 @pytest.mark.parametrize("pH,pW,F,B", [(48, 48, 256, 1), (52, 52, 256, 1), (64, 64, 256, 1), (72, 72, 256, 1), (33, 128, 256, 1), (40, 40, 512, 1),
                                        (52, 52, 256, 2), (16, 16, 256, 1)])
 def test_heads_have_the_bits_of_the_library_convolutions(pH, pW, F, B):
-    """Whole heads, the large convolutions of a view on the kernel and all of them with the library: maps whose order of sums the
-    library changes from one size to the next, oblong ones, more features, images above 512 pixels. Several views and small maps
+    """Whole heads, the convolutions of a view on the kernel and all of them with the library: maps whose order of sums the
+    library changes from one size to the next, oblong ones, more features, images above 512 pixels, small ones. Several views
     stay with the library."""
     from renderformer_cuda_b200 import session
     L = _abi.load("rfk_layers.h")
@@ -141,7 +141,7 @@ def test_heads_have_the_bits_of_the_library_convolutions(pH, pW, F, B):
     images = []
     for library_only in (0, 1):
         dpt, own = _plan(L, ctx, model, B, pH, pW, library_only)
-        assert (own > 0) == (not library_only and B == 1 and pH > 16)
+        assert (own > 0) == (not library_only and B == 1)
         image = torch.full((B, 3, pH * 8, pW * 8), 7.0, device="cuda", dtype=torch.float16)
         for _ in range(2):   # the buffers of the first pass are those of the second
             assert L.rfk_dpt_forward(dpt, taps, VP(image.data_ptr()), _stream()) == 0
@@ -152,18 +152,19 @@ def test_heads_have_the_bits_of_the_library_convolutions(pH, pW, F, B):
     ctx.close()
 
 
-@pytest.mark.parametrize("p,own", [(40, 0), (48, 5), (52, 6), (64, 6), (72, 6)])
-def test_convolutions_that_leave_the_library(p, own):
-    """Those that gain by it: the five on the map of four times the grid from 184 pixels up, the one at full resolution beyond 170000
-    pixels; not that one of a 320 x 320 image, nor 512 -> 256 channels at 144 x 144 (81 tiles on 74 pairs)."""
+@pytest.mark.parametrize("p", [8, 24, 40, 48, 52, 64, 72])
+def test_convolutions_that_leave_the_library(p):
+    """All 3 x 3 convolutions of one view but the one of stride 2: four in front of the fusion blocks, two a residual unit of which three blocks have two
+    and one has one, two at full resolution. At 24 x 24 tokens the library adds one of them in an order that the kernel does not have."""
     from renderformer_cuda_b200 import session
     model = session.Model.random(seed=3, dim=64, num_heads=1, ffn_hidden=64, enc_layers=0, dec_layers=1, with_dpt=True, dpt_features=256,
                                  dpt_out_channels=(256, 512, 1024, 1024))
     L, ctx = _abi.load("rfk_layers.h"), session.Ctx()
     dpt, n = _plan(L, ctx, model, 1, p, p, 0)
+    left = L.rfk_dpt_num_library_convolutions(dpt)
     L.rfk_dpt_destroy(dpt)
     ctx.close()
-    assert n == own
+    assert n + left == 4 + 2 * (3 * 2 + 1) + 2 + 1 and left == (2 if p == 24 else 1)
 
 
 def test_a_head_holds_no_copies_beside_its_maps():
