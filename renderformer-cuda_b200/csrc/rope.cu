@@ -302,6 +302,14 @@ static int launch_rope(const T* src0, T* dst0, const T* src1, T* dst1, const __h
         return RFK_EINVAL;
     if (rows_total < seq_len || src_rows < rows_total || dst_rows < rows_total) return RFK_EINVAL;
     if (batch == 0 || rows_total == 0) return RFK_OK;
+    if constexpr (NT == 2) {
+        if (dst0 == dst1) {   // one tensor given twice is rotated twice: the second time from what the first has left
+            const int rc = launch_rope<T, 1>(src0, dst0, nullptr, nullptr, cos_vals, sin_vals, batch, num_heads, seq_len, rows_total, head_dim, src_rows, dst_rows, st,
+                                             src_bstride, dst_bstride, tab_bstride, col_scale, scale_bstride);
+            return rc != RFK_OK ? rc : launch_rope<T, 1>(src1, dst1, nullptr, nullptr, cos_vals, sin_vals, batch, num_heads, seq_len, rows_total, head_dim,
+                                                         src_rows, dst_rows, st, src_bstride, dst_bstride, tab_bstride, col_scale, scale_bstride);
+        }
+    }
     const bool vec = head_dim % 16 == 0 && aligned16(src0) && aligned16(dst0) &&
                      (NT == 1 || (aligned16(src1) && aligned16(dst1))) && aligned16(cos_vals) &&
                      aligned16(sin_vals) && src_bstride % 8 == 0 && dst_bstride % 8 == 0 &&

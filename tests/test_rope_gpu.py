@@ -63,3 +63,17 @@ def test_rows_behind_the_sequence_are_copied():
     ops.rope_one_oop(src, dst, cos, sin, 2, 4, 33, 64, 40, 40, True)
     _near(dst[:, :, :33], _rotated(src[:, :, :33], cos[:, None], sin[:, None]))
     assert torch.equal(dst[:, :, 33:], src[:, :, 33:])
+
+
+@pytest.mark.parametrize("hd", [24, 64])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_one_tensor_given_twice_is_rotated_twice(hd, dtype):
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    x = torch.randn(2, 3, 70, hd, device="cuda", generator=g).to(dtype)
+    cos, sin = (torch.randn(2, 70, hd, device="cuda", generator=g).half() for _ in range(2))
+    both, one = (ops.apply_rope, ops.apply_rope_one) if dtype == torch.float16 else (ops.apply_rope_f32, ops.apply_rope_one_f32)
+    got, want = x.clone(), x.clone()
+    both(got, got, cos, sin, 2, 3, 70, hd)
+    for _ in range(2):
+        one(want, cos, sin, 2, 3, 70, hd)
+    assert torch.equal(got, want)
