@@ -169,8 +169,6 @@ __device__ __forceinline__ float square_sum(const uint32_t (&o)[16]) {
     return (c[0] + c[1]) + (c[2] + c[3]);
 }
 
-// Tiled copy global -> shared of one box of a rank-2 tensor map (x innermost, in elements; x * 2 bytes
-// is always a multiple of 128 here); the bytes are counted on `bar`.
 __device__ __forceinline__ void tma_prefetch_2d(const void* map, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
@@ -183,6 +181,8 @@ template <typename Ask> __device__ __forceinline__ void prefetch_weights(bool le
     if (leader) ask();
     __syncwarp();
 }
+// Tiled copy global -> shared of one box of a rank-2 tensor map (x innermost, in elements; x * 2 bytes
+// is always a multiple of 128 here); the bytes are counted on `bar`.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void* tmap, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -438,8 +438,9 @@ namespace pair { using namespace pair_ptx; }
 //   tensor pipe alone would take 0.05 us a block). 128 x 128 tiles keep whole warps: 2304 x 1024 x 4096 16.9 / 17.6, 1600 x 1024 x 4096
 //   16.4 / 17.4. The 128 x 64 tile's producer is lane 0 with the plain and residual epilogues (elected / lane 0, issuer elected in both: 2779 x 384 x
 //   4096 13.2 / 12.6, 1115 x 1024 x 4096 12.2 / 11.5, x 1024 4.87 / 4.88) and an elected lane with the others (SwiGLU 1024 x 512 x 1024 5.09 /
-//   5.70, head-split 1024 x 1024 x 4096 12.0 / 12.3). Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two, and
-//   weights asked for ahead of the kernel's wait for its predecessor, changed nothing or cost (320 x 320 views +4 %).
+//   5.70, head-split 1024 x 1024 x 4096 12.0 / 12.3). Half the ring costs 7 % (the copies in flight cover their latency); one copy per operand and stage instead of two changed
+//   nothing. Weights copied ahead of the kernel's wait for its predecessor gain where norms are folded (below); with separate norms they changed nothing or
+//   cost (320 x 320 views +4 %), and only the prefetch into L2 is left there.
 //   BM 64: the accumulator's row r is tensor-memory lane 32 * (r / 16) + r % 16, half the lanes of each warp's quarter.
 //   SwiGLU: the first BN / 2 accumulator columns are gate columns, the others the up columns of the same hidden units.
 // The epilogue's threads store their own rows: a tile row is 32 to 256 bytes, one to eight whole sectors.
@@ -526,7 +527,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem_cta = ctrl->tmem_base;
-    // A folded layer's weights are nobody's output: a ring of them is asked for ahead of the wait for the kernel before (a view of 64 x 64 pixels 579 ->
+    // A folded layer's weights are no output of the kernel before (gemm_folded's callers see to it, or ask for pairs): a ring of them is asked for ahead of the wait for it (a view of 64 x 64 pixels 579 ->
     // 542 us, 128 x 128 658 -> 645, 320 x 320 1469 -> 1449; half a ring 556, 647, 1459).
     const int early = FOLD ? min(kStages, num_st) : 0;
     if (FOLD && warp == 0 && (kLane0 ? lane == 0 : tc::elect_one())) {

@@ -15,7 +15,8 @@ int gemm_heads(const rfk_half* A, long long lda, const rfk_half* W, long long ld
 // [N, K] with the norm's weight multiplied in. One of: W_up (SwiGLU, C [M, N]), num_heads > 0 (head-split, C as gemm_heads'), R (C = R + A W^T).
 // out_ss (may be NULL; residual and head-split): the sums of squares of the rows written, *ss_tiles a row (of a part). A residual product's
 // rows may be the 4 x 4 blocks of a token grid in window order, of a grid shifted by shift_from blocks; they are then written in the order
-// of a grid shifted by shift_to blocks (C, with out_ss) and in raster order (raster), each where it is not NULL; C is then not R.
+// of a grid shifted by shift_to blocks (C, with out_ss) and in raster order (raster), each where it is not NULL; C is then not R. W is not written by the
+// kernel right ahead in the stream, unless FoldedMore::pairs is asked for.
 // RFK_EUNSUPPORTED: shapes or a device that these kernels do not serve, nothing launched.
 struct FoldedProduct {
     const rfk_half *A, *W, *W_up, *R;

@@ -579,8 +579,8 @@ int rfk_layers::decoder_layer_impl(
     return RFK_OK;
 }
 
-// 1024 columns: four sums of squares a row, one 16-byte load, and CTAs of one row (embed_tokens); narrower rows leave less to gain than the launches that
-// are left, and keep their separate norms.
+// 1024 columns: what embed_tokens, fold_weights and the grouped sums of the attention are written for, and the models have; gemm_folded itself takes any multiple
+// of 256. Other widths keep their separate norms, and the bits of the public layer calls; what folding them would gain is not measured.
 bool rfk_layers::layer_folds(const rfk_decoder_layer_weights& w, int Sq, int dim, int num_heads, int ffn_hidden, int patch_h, int patch_w,
                              int window_size, int shift_size) {
     const auto given = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };

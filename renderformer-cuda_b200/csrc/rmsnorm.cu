@@ -238,8 +238,8 @@ embed_tokens_kernel(const __half* __restrict__ e, const float* __restrict__ gamm
 // The scale lies in device memory beside the weights, where a captured graph's products find the one that they were divided by last. It is that of
 // the largest product and not of the norm's weights: a product that is 2^27 times smaller still has all its bits, where a small norm
 // weight that holds down a large channel would otherwise leave products below 2^-14, which have fewer (512 x 1024 x 1024, W of 0.02 n, norm weights
-// exp(a n), channels inversely as large, error against 64 bits, separate norm / the norm's weights brought below 1 / this:
-// a = 1.5 2.1e-4 / 7.8e-4 / 2.1e-4, a = 2 2.1e-4 / 1.4e-2 / 2.1e-4). 2^14 leaves two bits below fp16's largest; the sums are fp32.
+// exp(a n), channels inversely as large, error against 64 bits, separate norm / the norm's weights brought below 1 / this: a = 1 2.9e-4 / 3.2e-4 / 2.9e-4,
+// 1.5 2.9e-4 / 3.5e-3 / 2.9e-4, 2 2.9e-4 / 6.9e-2 / 2.9e-4). 2^14 leaves two bits below fp16's largest; the sums are fp32.
 // Bound: HBM, each weight once in and once out; the rows stay in registers until their scale is known. A cluster of two CTAs with 32 rows each, two of them an
 // SM, loads while another stores: twelve layers' weights (302 MB in, 302 out) 106 us, 5.7 TB/s; 64 rows a CTA 132, 256 threads a CTA 123.
 struct FoldList {

@@ -532,7 +532,7 @@ struct Carver {
     }
 };
 
-// Work buffers of the scene encoding. They are one block that the session keeps (174 MB at 5633 triangles): 19 cudaMalloc
+// Work buffers of the scene encoding. They are one block that the session keeps (177 MB at 5633 triangles, and 53 MB of folded weights and sums): 19 cudaMalloc
 // and as many cudaFree a call, and the host work above, took 6.7 of 12.7 ms (5633 triangles; now 6.0). The embeddings and the K/V
 // projections lie in the layers' qkv buffer, which is idle before the first and after the last encoder layer.
 struct EncodeBuffers {
